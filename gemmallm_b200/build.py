@@ -1,16 +1,19 @@
-"""Build libmoe_b200.so in-tree with nvcc for sm_100a.
+"""Build libmoe_b200.so in-tree with nvcc for sm_100a, and the host extension
+_host.so (csrc/host/, C++ against the installed torch and libmoe_b200.so).
 
     python -m gemmallm_b200.build [--force] [--verbose]
 
 nvcc cross-compiles without a GPU. Objects go to gemmallm_b200/csrc/_build/,
-the library to gemmallm_b200/libmoe_b200.so (git-ignored, built artefact).
+the libraries to gemmallm_b200/ (git-ignored, built artefacts).
 """
 from __future__ import annotations
 
 import os
+import importlib.util
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -18,6 +21,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = CSRC / "_build"
 LIB = PKG / "libmoe_b200.so"
+HOST_SRC = CSRC / "host" / "host.cpp"
+HOST_LIB = PKG / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -48,7 +53,7 @@ def _stale(target: Path, deps: list[Path]) -> bool:
 def build(force: bool = False, verbose: bool = False) -> Path:
     nvcc = _nvcc()
     OBJ.mkdir(exist_ok=True)
-    headers = sorted(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "moe_b200.h"]
+    headers = sorted(CSRC.glob("*.cuh")) + [CSRC / "internal.h", PKG.parent / "include" / "moe_b200.h"]
     jobs = []
     objs = []
     for src in sources():
@@ -77,7 +82,29 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link of libmoe_b200.so failed")
+    build_host(force, verbose)
     return LIB
+
+
+def build_host(force: bool = False, verbose: bool = False) -> Path:
+    """The modules' native host path: one C++ file against torch's headers, linked to
+    libmoe_b200.so next to it."""
+    deps = [HOST_SRC, CSRC / "internal.h", PKG.parent / "include" / "moe_b200.h"]
+    if not force and not _stale(HOST_LIB, deps):
+        return HOST_LIB
+    torch_dir = Path(next(iter(importlib.util.find_spec("torch").submodule_search_locations)))
+    cuda = Path(_nvcc()).resolve().parent.parent
+    includes = [torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include",
+                sysconfig.get_paths()["include"], cuda / "include"]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{i}" for i in includes),
+           str(HOST_SRC), "-o", str(HOST_LIB), f"-L{torch_dir / 'lib'}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+           "-ltorch_python", "-lc10", "-lc10_cuda", f"-L{PKG}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError("build of _host.so failed")
+    return HOST_LIB
 
 
 if __name__ == "__main__":

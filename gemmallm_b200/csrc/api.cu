@@ -5,6 +5,7 @@
 #include <stdio.h>
 #include <string.h>
 #include "common.cuh"
+#include "internal.h"
 
 namespace moe {
 
@@ -405,6 +406,28 @@ int moe_b200_forward(const void* x, const void* Wg, const void* bg, const void* 
                      const void* residual, const void* norm_weight, const void* norm_bias,
                      float norm_eps, int64_t N, int d, int f, int E, int k, int dtype, int flags,
                      void* workspace, size_t workspace_bytes, void* out, void* stream) {
+  return forward_into(x, Wg, bg, plan, residual, norm_weight, norm_bias, norm_eps, N, d, f, E, k, dtype,
+                      flags, workspace, workspace_bytes, out, nullptr, stream);
+}
+
+int moe_b200_read_status(const int32_t* status, int32_t* h_status, void* stream) {
+  if (!status || !h_status) return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  MOE_CUDA_CHECK(cudaMemcpyAsync(h_status, status, 16 * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                 (cudaStream_t)stream));
+  MOE_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));
+  return h_status[0];
+}
+
+}  // extern "C"
+
+namespace moe {
+
+// moe_b200_forward with the load-balancing loss written to `aux` (nullptr: the workspace's own word),
+// so that a caller who hands the loss on as a tensor of its own needs no copy of it.
+int forward_into(const void* x, const void* Wg, const void* bg, const void* plan, const void* residual,
+                 const void* norm_weight, const void* norm_bias, float norm_eps, int64_t N, int d, int f,
+                 int E, int k, int dtype, int flags, void* workspace, size_t workspace_bytes, void* out,
+                 float* aux, void* stream) {
   int rc = check_shape(N, d, f, E, k, dtype);
   if (rc) return rc;
   if (!workspace) return set_error(MOE_B200_ERR_NULL, "workspace is NULL");
@@ -423,7 +446,7 @@ int moe_b200_forward(const void* x, const void* Wg, const void* bg, const void* 
   float* w = reinterpret_cast<float*>(ws + off[MOE_B200_WS_W]);
   float* psum_part = reinterpret_cast<float*>(ws + off[MOE_B200_WS_PSUM_PART]);
   float* psum = reinterpret_cast<float*>(ws + off[MOE_B200_WS_PSUM]);
-  float* aux = reinterpret_cast<float*>(ws + off[MOE_B200_WS_AUX]);
+  if (aux == nullptr) aux = reinterpret_cast<float*>(ws + off[MOE_B200_WS_AUX]);
   int32_t* scratch = reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_SCRATCH]);
   int32_t* cnt_slot = reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_CNT_SLOT]);
   int32_t* offsets = reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_OFFSETS]);
@@ -451,7 +474,9 @@ int moe_b200_forward(const void* x, const void* Wg, const void* bg, const void* 
                          rows_supported(N * k, E);
   const bool counters = small_n || rows_path;
   // status words, and the completion counters behind them where a kernel uses them, in one memset
-  if (!(counters && (flags & MOE_B200_FLAG_WS_CLEAN)))
+  // (a caller that keeps the region clean needs none at any size: kernels write the status words
+  // only when something failed)
+  if (!(flags & MOE_B200_FLAG_WS_CLEAN))
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
   const bool front = (small_n || rows_path) &&
@@ -519,12 +544,4 @@ int moe_b200_forward(const void* x, const void* Wg, const void* bg, const void* 
   return moe_b200_combine(y, row_of, w, residual, N, d, k, dtype, out, stream);
 }
 
-int moe_b200_read_status(const int32_t* status, int32_t* h_status, void* stream) {
-  if (!status || !h_status) return set_error(MOE_B200_ERR_NULL, "NULL argument");
-  MOE_CUDA_CHECK(cudaMemcpyAsync(h_status, status, 16 * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                 (cudaStream_t)stream));
-  MOE_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));
-  return h_status[0];
-}
-
-}  // extern "C"
+}  // namespace moe

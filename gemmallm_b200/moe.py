@@ -15,6 +15,7 @@ import torch.nn as nn
 
 from . import _cabi
 from ._cabi import lib, check
+from . import _host
 
 _DTYPES = {torch.float32: _cabi.F32, torch.bfloat16: _cabi.BF16}
 
@@ -32,6 +33,29 @@ def _stream(device: torch.device) -> int:
 
 _LORA_NAMES = ("gate_and_up", "down", "lora_gate_and_up_a", "lora_gate_and_up_b", "lora_down_a",
                "lora_down_b")
+
+
+def _expert_watch(ex, fine_tuning: bool) -> list:
+    """(dictionary, key) of everything in an expert's module tree that a prepared call uses: the
+    Linears, then weight and bias of each in the order of _LORA_NAMES."""
+    names = _LORA_NAMES if fine_tuning else _LORA_NAMES[:2]
+    watch = [(ex._modules, n) for n in names]
+    for n in names:
+        watch += [(getattr(ex, n)._parameters, "weight"), (getattr(ex, n)._parameters, "bias")]
+    return watch
+
+
+def _lora_jobs(ex, merged, first: int) -> list:
+    """The two merges of an expert for the native path: indices of weight, bias, a.weight, a.bias,
+    b.weight, b.bias among the watched parameters (the expert's twelve start at ``first``), then
+    scale, shape and the merged buffers."""
+    jobs = []
+    for lin, a, b, out, i in ((ex.gate_and_up, ex.lora_gate_and_up_a, ex.lora_gate_and_up_b, merged.gate_and_up, 0),
+                              (ex.down, ex.lora_down_a, ex.lora_down_b, merged.down, 1)):
+        w, la, lb = first + 2 * i, first + 4 + 4 * i, first + 6 + 4 * i
+        jobs.append((w, w + 1, la, la + 1, lb, lb + 1, float(ex.lora_scale), lin.out_features, lin.in_features,
+                     a.out_features, out.weight.data_ptr(), out.bias.data_ptr()))
+    return jobs
 
 
 class _MergedExpert:
@@ -216,6 +240,8 @@ class FeedForward(nn.Module):
         self._plan = _Plan()
         self._plan_ft = _Plan()
         self._lora = _MergedLora()
+        # native calls prepared for the last number of rows: plain, and with the LoRA branches merged
+        self._native, self._native_ft = _host.Ffn(), _host.Ffn()
         self._offsets = None   # ((rows, device), int32 [0, rows]) of the last call
         self._tws = None
         self._tws_key = None
@@ -310,23 +336,31 @@ class FeedForward(nn.Module):
                 for lin in (self.lora_gate_and_up_a, self.lora_gate_and_up_b, self.lora_down_a, self.lora_down_b):
                     params += [lin.weight, lin.bias]
             return _FfnTrainFn.apply(self, tensor, seed, bool(fine_tuning), *params)
+        native = self._native_ft if fine_tuning else self._native
+        y = native.forward(tensor)
+        return self._forward_prepared(tensor, bool(fine_tuning), native) if y is None else y
+
+    def _forward_prepared(self, tensor, fine_tuning: bool, native):
+        """The forward of a call that differs from the one ``native`` was bound for: prepares plan,
+        offsets and merged weights, runs, and binds the result."""
         dtype = _dtype_code(tensor)
         shape = tensor.shape
-        x = tensor.reshape(-1, shape[-1]).contiguous()
-        M, d, f = x.shape[0], self.hidden_size, self.d_ff
-        dev = x.device
+        x, M, dev, offsets = self._rows(tensor)
+        d, f = self.hidden_size, self.d_ff
         with torch.cuda.device(dev):
             plan = (self._plan_ft if fine_tuning else self._plan).get(
                 self._lora.get([self], dtype, dev) if fine_tuning else [self], d, f, dtype, dev)
-            if self._offsets is None or self._offsets[0] != (M, str(dev)):
-                self._offsets = ((M, str(dev)), torch.tensor([0, M], dtype=torch.int32, device=dev))
-            offsets = self._offsets[1]
             status = torch.zeros(16, dtype=torch.int32, device=dev)
             h = torch.empty(M, f, dtype=x.dtype, device=dev)
             y = torch.empty(M, d, dtype=x.dtype, device=dev)
             check(lib.moe_b200_experts(x.data_ptr(), offsets.data_ptr(), plan, M, d, f, 1, dtype, 0,
                                        h.data_ptr(), y.data_ptr(), status.data_ptr(), _stream(dev)),
                   "experts")
+        native.unbind()
+        watch = _expert_watch(self, fine_tuning)
+        if x.shape[-1] == d and all(name in table for table, name in watch):
+            jobs = _lora_jobs(self, self._lora.merged[0], 0) if fine_tuning else None
+            native.bind(watch, jobs, plan, offsets, status, M, d, f, dtype, dev.index)
         return y.reshape(shape)
 
 
@@ -360,7 +394,30 @@ class MOE(nn.Module):
         self._tws = None
         self._tws_key = None
         self._train_gen = 0
-        self.last = None  # views into the workspace of the most recent call
+        self._last_seed = None
+        # native calls prepared for the last input size: plain, and with the LoRA branches merged
+        self._native, self._native_ft = _host.Block(), _host.Block()
+
+    @property
+    def last(self) -> dict | None:
+        """Views into the workspace of the most recent call (None before the first): logits, idx,
+        w, cnt_slot, offsets, psum, row_of, status; after a training forward also its seed."""
+        if self._ws is None:
+            return None
+        N, E, k = self._ws_key[0], self.num_experts, self.top_k
+        views = {
+            "logits": self._view("logits", torch.float32, (N, E)),
+            "idx": self._view("idx", torch.int32, (N, k)),
+            "w": self._view("w", torch.float32, (N, k)),
+            "cnt_slot": self._view("cnt_slot", torch.int32, (k, E)),
+            "offsets": self._view("offsets", torch.int32, (E + 1,)),
+            "psum": self._view("psum", torch.float32, (E,)),
+            "row_of": self._view("row_of", torch.int32, (N, k)),
+            "status": self._view("status", torch.int32, (16,)),
+        }
+        if self._last_seed is not None:
+            views["seed"] = self._last_seed
+        return views
 
     # -- workspace ---------------------------------------------------------
     def _workspace(self, N: int, dtype: int, device: torch.device):
@@ -368,12 +425,18 @@ class MOE(nn.Module):
         if key != self._ws_key:
             d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
             nbytes = _cabi.workspace_bytes(N, d, f, E, k, dtype)
-            # zeroed: the small-N kernels keep their counters in the status region and leave
-            # them zero after every call (FLAG_WS_CLEAN below)
-            buf = torch.zeros(nbytes + 1024, dtype=torch.uint8, device=device)
+            buf = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
             base = (buf.data_ptr() + 1023) & ~1023
             self._ws = (buf, base, nbytes, _cabi.workspace_layout(N, d, f, E, k, dtype))
             self._ws_key = key
+            self._native.unbind()
+            self._native_ft.unbind()
+            # the small-N kernels keep their counters in the status region and leave them zero
+            # after every call (FLAG_WS_CLEAN below); everything else is written before it is
+            # read, except for what a call without tokens leaves as it is
+            if N == 0:
+                buf.zero_()
+            self._view("status", torch.int32, (_cabi.READY_OFFSET + _cabi.READY_INTS,)).zero_()
         return self._ws
 
     def _view(self, name: str, dtype: torch.dtype, shape) -> torch.Tensor:
@@ -416,6 +479,16 @@ class MOE(nn.Module):
                     for lin in (ex.lora_gate_and_up_a, ex.lora_gate_and_up_b, ex.lora_down_a, ex.lora_down_b):
                         params += [lin.weight, lin.bias]
             return _TrainFn.apply(self, tensor, residual, seed, bool(fine_tuning), *params)
+        native = self._native_ft if fine_tuning else self._native
+        self._last_seed = None
+        done = native.forward(tensor, residual, norm)
+        if done is None:
+            done = self._forward_prepared(tensor, bool(fine_tuning), residual, norm, native)
+        return done
+
+    def _forward_prepared(self, tensor, fine_tuning: bool, residual, norm, native):
+        """The forward of a call that differs from the one ``native`` was bound for: checks the
+        arguments, prepares plan, workspace and merged weights, runs, and binds the result."""
         dtype = _dtype_code(tensor)
         shape = tensor.shape
         d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
@@ -451,18 +524,28 @@ class MOE(nn.Module):
             check(lib.moe_b200_forward(x.data_ptr(), gw.data_ptr(), gb.data_ptr(), plan, res_ptr,
                                        nw, nb, eps, N, d, f, E, k, dtype, _cabi.FLAG_WS_CLEAN, base, nbytes,
                                        out.data_ptr(), _stream(dev)), "forward")
-        self.last = {
-            "logits": self._view("logits", torch.float32, (N, E)),
-            "idx": self._view("idx", torch.int32, (N, k)),
-            "w": self._view("w", torch.float32, (N, k)),
-            "cnt_slot": self._view("cnt_slot", torch.int32, (k, E)),
-            "offsets": self._view("offsets", torch.int32, (E + 1,)),
-            "psum": self._view("psum", torch.float32, (E,)),
-            "row_of": self._view("row_of", torch.int32, (N, k)),
-            "status": self._view("status", torch.int32, (16,)),
-        }
         aux = self._view("aux", torch.float32, (1,))[0].clone()
+        self._bind(native, fine_tuning, plan, N, dtype, dev)
         return out.reshape(shape), aux
+
+    def _bind(self, native, fine_tuning: bool, plan: int, N: int, dtype: int, dev: torch.device) -> None:
+        """Hand the prepared call to the native path, with everything in the module tree it depends
+        on. Trees that do not hold their parameters under the usual names stay on the Python path."""
+        d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
+        native.unbind()
+        watch = [(self._modules, "gate"), (self._modules, "experts"),
+                 (self.gate._parameters, "weight"), (self.gate._parameters, "bias")]
+        for name, ex in self.experts._modules.items():
+            watch.append((self.experts._modules, name))
+            watch += _expert_watch(ex, fine_tuning)
+        jobs = None
+        if fine_tuning:
+            jobs = [job for e, (ex, mg) in enumerate(zip(self.experts, self._lora.merged))
+                    for job in _lora_jobs(ex, mg, 2 + 12 * e)]
+        if len(self.experts) != E or any(name not in table for table, name in watch):
+            return
+        buf, base, nbytes, _ = self._ws
+        native.bind(watch, jobs, plan, buf, base, nbytes, N, d, f, E, k, dtype, dev.index)
 
     # -- training mode -------------------------------------------------------
     def _train_workspace(self, N: int, dtype: int, device: torch.device):
@@ -516,17 +599,7 @@ class MOE(nn.Module):
                 N, d, f, E, k, dtype, float(self.experts[0].dropout.p), seed, base, nbytes, tbase, tbytes,
                 out.data_ptr(), _stream(dev)), "forward_train")
         self._train_gen += 1
-        self.last = {
-            "logits": self._view("logits", torch.float32, (N, E)),
-            "idx": self._view("idx", torch.int32, (N, k)),
-            "w": self._view("w", torch.float32, (N, k)),
-            "cnt_slot": self._view("cnt_slot", torch.int32, (k, E)),
-            "offsets": self._view("offsets", torch.int32, (E + 1,)),
-            "psum": self._view("psum", torch.float32, (E,)),
-            "row_of": self._view("row_of", torch.int32, (N, k)),
-            "status": self._view("status", torch.int32, (16,)),
-            "seed": seed,
-        }
+        self._last_seed = seed
         aux = self._view("aux", torch.float32, (1,))[0].clone()
         return out.reshape(shape), aux
 
@@ -574,9 +647,9 @@ class MOE(nn.Module):
     def device_status(self) -> int:
         """Status word of the most recent call (0 = ok); synchronises. A non-zero status is
         returned once: the status region is zeroed again so that later calls start clean."""
-        if not self.last:
+        if self._ws is None:
             return 0
-        code = int(self.last["status"][0].item())
+        code = int(self._view("status", torch.int32, (16,))[0].item())
         if code != 0:
             self._view("status", torch.int32, (_cabi.READY_OFFSET + _cabi.READY_INTS,)).zero_()
         return code
