@@ -134,7 +134,8 @@ def workspace_layout(N: int, d: int, f: int, E: int, k: int, dtype: int) -> dict
 
 
 TWS_NAMES = ("gu", "pair_of", "koff", "dy", "dh", "dxs", "w1t", "w2t", "tmaps", "xt", "ht", "dyt", "dgut",
-             "dl", "dw", "ones", "dwg_f32", "dxr", "g_wg", "g_bg", "g_w1", "g_b1", "g_w2", "g_b2")
+             "dl", "dw", "ones", "dwg_f32", "dxr", "g_wg", "g_bg", "g_w1", "g_b1", "g_w2", "g_b2", "mask",
+             "col_part")
 
 
 def train_workspace_layout(N: int, d: int, f: int, E: int, k: int, dtype: int) -> dict[str, int]:

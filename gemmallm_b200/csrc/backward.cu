@@ -1,36 +1,20 @@
 // Backward pass of the block (the reference trains through MOE.forward with torch.autograd:
 // loss.backward() in train.py:140-141 reaches model.py:200-276 and 173-190). The two input
 // gradients and the two weight gradients of the expert Linears are grouped products on the
-// tcgen05 kernel of experts_tc2.cu; this file holds what surrounds them, all HBM-bound:
+// tcgen05 kernel of experts_tc2.cu, whose epilogue also takes dh back through dropout, product and
+// GELU; this file holds what surrounds them, all HBM-bound:
 //
 //   combine_bwd      dy[r] = w[pair] * dOut[token], dw[pair] = dOut[token] . y[r]   (model.py:271)
 //   router_bwd       dw -> d(renormalised scores) -> d(softmax) -> dlogits, plus the gradient
 //                    of the load-balancing loss through the mean probabilities
 //                    (model.py:207-223; the counts of model.py:213 carry no gradient)
 //   router_bwd_wx    dWg = dlogits^T x, dbg = sum dlogits, dx += dlogits Wg       (model.py:206)
-//   geglu_bwd        through dropout, the product and the tanh-GELU                (model.py:180-183)
-//   transposes       W -> W^T per expert (input gradients contract over the output features);
-//                    activations [rows, C] -> [C, padded rows] with every expert's rows starting
-//                    at a multiple of 64 and zero fill (weight gradients contract over rows)
 //   colsum           bias gradients per expert
 #include "common.cuh"
-#include "philox.cuh"
 
 namespace moe {
 
 namespace {
-
-// koff[e+1] = koff[e] + round_up(rows of e, 64)
-__global__ void pad_offsets_kernel(const int32_t* __restrict__ offsets, int E, int32_t* __restrict__ koff) {
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    koff[0] = 0;
-    for (int e = 0; e < E; ++e) {
-      acc += (offsets[e + 1] - offsets[e] + 63) & ~63;
-      koff[e + 1] = acc;
-    }
-  }
-}
 
 __global__ void pair_of_kernel(const int32_t* __restrict__ row_of, int64_t M, int32_t* __restrict__ pair_of) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -75,8 +59,8 @@ combine_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* 
 __global__ void __launch_bounds__(256)
 router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ idx,
                   const float* __restrict__ w, const float* __restrict__ dw,
-                  const int32_t* __restrict__ cnt0, float grad_aux, int64_t N, int E, int k,
-                  float* __restrict__ dl) {
+                  const int32_t* __restrict__ cnt0, float grad_aux_host, const float* __restrict__ grad_aux_dev,
+                  int64_t N, int E, int k, float* __restrict__ dl) {
   const int64_t t = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= N) return;
@@ -103,6 +87,7 @@ router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ 
   // total of the chosen probabilities and sum_i dw_i w_i (every lane computes them: k <= 8)
   float total = 0.f, dww = 0.f;
   for (int j = 0; j < k; ++j) dww = fmaf(dw[t * k + j], w[t * k + j], dww);
+  const float grad_aux = grad_aux_dev != nullptr ? __ldg(grad_aux_dev) : grad_aux_host;
   const float aux_c = grad_aux * (float)E / ((float)N * (float)N);
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
@@ -212,160 +197,46 @@ __global__ void fill_f32_kernel(float* __restrict__ p, int64_t n, float v) {
   if (i < n) p[i] = v;
 }
 
-// In place over gu [M, 2f]: (g, u) -> (dg, du), given dh [M, f] (gradient of the dropped h):
-//   dhe = dh * mask * scale;  du = dhe * gelu(g);  dg = dhe * u * gelu'(g)
-//   gelu(g) = 0.5 g (1 + t), t = tanh(b (g + a g^3)), gelu'(g) = 0.5 (1 + t) + 0.5 g (1 - t^2) b (1 + 3 a g^2)
+// Partial column sums: one block per 256-row tile of an expert (tiles counted over the experts in
+// order, as the grouped products count them) and 64 columns; eight threads cover a row's 128 bytes,
+// 32 such groups take every 32nd row, eight loads in flight each.
 __global__ void __launch_bounds__(256)
-geglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* __restrict__ gu,
-                 const int32_t* __restrict__ pair_of, int64_t M, int f, uint32_t thresh, float scale,
-                 uint32_t seed_lo, uint32_t seed_hi) {
-  const int pieces = f >> 3;
-  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= M * pieces) return;
-  const int64_t r = item / pieces;
-  const int c = (int)(item - r * pieces) << 3;
-  float dv[8], g[8], u[8], dg[8], du[8];
-  load8(dh + r * f + c, dv);
-  load8(gu + r * 2 * f + c, g);
-  load8(gu + r * 2 * f + f + c, u);
-  if (thresh != 0u) {
-    const uint32_t pair = (uint32_t)pair_of[r];
-#pragma unroll
-    for (int b4 = 0; b4 < 2; ++b4) {
-      const uint4 rn = philox4x32_10((uint32_t)(c >> 2) + b4, pair, seed_lo, seed_hi);
-      const uint32_t wv[4] = {rn.x, rn.y, rn.z, rn.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) dv[b4 * 4 + i] = wv[i] >= thresh ? dv[b4 * 4 + i] * scale : 0.f;
-    }
-  }
-  const float kB = 0.7978845608028654f, kA = 0.044715f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float x = g[i];
-    const float t = tanhf(kB * (x + kA * x * x * x));
-    const float gelu = 0.5f * x * (1.f + t);
-    const float dgelu = 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * kB * (1.f + 3.f * kA * x * x);
-    du[i] = dv[i] * gelu;
-    dg[i] = dv[i] * u[i] * dgelu;
-  }
-  store8(gu + r * 2 * f + c, dg);
-  store8(gu + r * 2 * f + f + c, du);
-}
-
-// 64 x 64 tile transpose with 16-byte global accesses on both sides: rows r < rows_valid of
-// `src` (row pitch C elements, columns [c0, c0 + 64)) become columns of `dst`:
-// dst[(c0 + c) * ldd + i] = src[i][c0 + c], zero where i >= rows_valid. Positions i >= k_valid of
-// dst do not exist and are not written. Shared memory holds the tile as 32-bit words (two
-// neighbouring columns), 33 words per row; a thread then reads one word of eight consecutive
-// rows and splits them into the two columns' 16-byte pieces.
-__device__ __forceinline__ void transpose_tile64(const __nv_bfloat16* __restrict__ src, int rows_valid,
-                                                 int C, int c0, __nv_bfloat16* __restrict__ dst,
-                                                 int64_t ldd, int k_valid, uint32_t (&tile)[64 * 33]) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    const int p = tid + s * 256;
-    const int i = p >> 3, pc = p & 7;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (i < rows_valid && c0 + pc * 8 < C)
-      v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)i * C + c0 + pc * 8));
-    uint32_t* t4 = &tile[i * 33 + pc * 4];
-    t4[0] = v.x; t4[1] = v.y; t4[2] = v.z; t4[3] = v.w;
-  }
-  __syncthreads();
-  const int kp = tid & 7, cp = tid >> 3;     // eight rows kp*8.., columns 2cp and 2cp + 1
-  uint32_t w[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) w[q] = tile[(kp * 8 + q) * 33 + cp];
-  uint4 lo, hi;
-  lo.x = __byte_perm(w[0], w[1], 0x5410); hi.x = __byte_perm(w[0], w[1], 0x7632);
-  lo.y = __byte_perm(w[2], w[3], 0x5410); hi.y = __byte_perm(w[2], w[3], 0x7632);
-  lo.z = __byte_perm(w[4], w[5], 0x5410); hi.z = __byte_perm(w[4], w[5], 0x7632);
-  lo.w = __byte_perm(w[6], w[7], 0x5410); hi.w = __byte_perm(w[6], w[7], 0x7632);
-  if (kp * 8 < k_valid) {
-    const int c = c0 + 2 * cp;
-    if (c < C) *reinterpret_cast<uint4*>(dst + (size_t)(2 * cp) * ldd + kp * 8) = lo;
-    if (c + 1 < C) *reinterpret_cast<uint4*>(dst + (size_t)(2 * cp + 1) * ldd + kp * 8) = hi;
-  }
-}
-
-// dst[e] [C, R] = src[e] [R, C] transposed (R, C multiples of 8); one block per 64 x 64 tile.
-__global__ void __launch_bounds__(256)
-transpose_weight_kernel(const void* const* __restrict__ src_ptrs, int R, int C,
-                        __nv_bfloat16* __restrict__ dst) {
-  __shared__ uint32_t tile[64 * 33];
-  const int e = blockIdx.z;
-  const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(src_ptrs[e]);
-  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-  const int rows = R - r0 < 64 ? R - r0 : 64;
-  transpose_tile64(src + (size_t)r0 * C, rows, C, c0,
-                   dst + (size_t)e * R * C + (size_t)c0 * R + r0, R, rows, tile);
-}
-
-// dst [C, Kpad]: column koff[e] + j holds row offsets[e] + j of src [M, C] for j < rows of e,
-// zero for the padding up to koff[e+1]. One block per 64 padded columns x 64 source columns.
-__global__ void __launch_bounds__(256)
-transpose_pad_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ offsets,
-                     const int32_t* __restrict__ koff, int E, int C, int64_t Kpad,
-                     __nv_bfloat16* __restrict__ dst) {
-  __shared__ uint32_t tile[64 * 33];
-  __shared__ int s_row0, s_rows;
-  const int k0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
+colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ offsets, int E, int C,
+              float* __restrict__ part) {
+  __shared__ float s_part[32][65];
+  __shared__ int s_row0, s_row1;
   if (threadIdx.x == 0) {
-    int row0 = 0, rows = 0;
-    if (k0 < koff[E]) {
-      int lo = 0, hi = E;   // last e with koff[e] <= k0
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (koff[mid] <= k0) lo = mid; else hi = mid;
+    int tile = blockIdx.y, r0 = 0, r1 = 0;
+    for (int e = 0; e < E; ++e) {
+      const int beg = offsets[e], end = offsets[e + 1], tiles = (end - beg + 255) / 256;
+      if (tile < tiles) {
+        r0 = beg + tile * 256;
+        r1 = min(end, r0 + 256);
+        break;
       }
-      const int within = k0 - koff[lo];
-      const int n = offsets[lo + 1] - offsets[lo];
-      row0 = offsets[lo] + within;
-      rows = n - within < 0 ? 0 : (n - within > 64 ? 64 : n - within);
+      tile -= tiles;
     }
-    s_row0 = row0;
-    s_rows = rows;
+    s_row0 = r0;
+    s_row1 = r1;
   }
   __syncthreads();
-  transpose_tile64(src + (size_t)s_row0 * C, s_rows, C, c0, dst + (size_t)c0 * Kpad + k0, Kpad, 64, tile);
-}
-
-// db[e][c] = sum over the expert's rows of src[r][c] (C a multiple of 8). One block per (expert,
-// 64 columns): eight threads cover a row's 128 bytes, 32 such groups take rows r, r + 32, ...
-// with four 16-byte loads in flight each; the 32 partial sums of a column are added in order.
-__global__ void __launch_bounds__(256)
-colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ offsets, int C,
-              __nv_bfloat16* __restrict__ db) {
-  __shared__ float part[32][65];
-  const int e = blockIdx.y;
+  const int r0 = s_row0, r1 = s_row1;
+  if (r0 == r1) return;      // behind the last tile
   const int pc = threadIdx.x & 7, lane_r = threadIdx.x >> 3;
   const int c = blockIdx.x * 64 + pc * 8;
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
   if (c < C) {
-    const int r1 = offsets[e + 1];
-    int r = offsets[e] + lane_r;
-    const uint4* base = reinterpret_cast<const uint4*>(src + c);
-    const size_t pitch = (size_t)C >> 3;     // 16-byte pieces per row
-    for (; r + 96 < r1; r += 128) {
-      uint4 v[4];
+    uint4 v[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = __ldg(base + (size_t)(r + 32 * u) * pitch);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          acc[2 * i] += bf16_lo(w[i]);
-          acc[2 * i + 1] += bf16_hi(w[i]);
-        }
-      }
+    for (int q = 0; q < 8; ++q) {
+      const int r = r0 + lane_r + 32 * q;
+      v[q] = r < r1 ? __ldg(reinterpret_cast<const uint4*>(src + (size_t)r * C + c)) : make_uint4(0, 0, 0, 0);
     }
-    for (; r < r1; r += 32) {
-      const uint4 v = __ldg(base + (size_t)r * pitch);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const uint32_t w[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         acc[2 * i] += bf16_lo(w[i]);
@@ -374,15 +245,48 @@ colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) part[lane_r][pc * 8 + i] = acc[i];
+  for (int i = 0; i < 8; ++i) s_part[lane_r][pc * 8 + i] = acc[i];
   __syncthreads();
   if (threadIdx.x < 64) {
     const int col = blockIdx.x * 64 + threadIdx.x;
     if (col < C) {
       float sum = 0.f;
-      for (int q = 0; q < 32; ++q) sum += part[q][threadIdx.x];
-      db[(size_t)e * C + col] = __float2bfloat16_rn(sum);
+#pragma unroll
+      for (int q = 0; q < 32; ++q) sum += s_part[q][threadIdx.x];
+      part[(size_t)blockIdx.y * C + col] = sum;
     }
+  }
+}
+
+// db[e][c] = sum of the expert's slots of part (`slots` per 256-row tile), in order: eight groups of
+// 32 threads take every eighth slot.
+__global__ void __launch_bounds__(256)
+colsum_finish_kernel(const float* __restrict__ part, int slots, const int32_t* __restrict__ offsets, int C,
+                     __nv_bfloat16* __restrict__ db) {
+  __shared__ float s_sum[8][33];
+  __shared__ int s_first, s_count;
+  const int e = blockIdx.y;
+  if (threadIdx.x == 0) {
+    int first = 0;
+    for (int i = 0; i < e; ++i) first += (offsets[i + 1] - offsets[i] + 255) / 256;
+    s_first = first * slots;
+    s_count = (offsets[e + 1] - offsets[e] + 255) / 256 * slots;
+  }
+  __syncthreads();
+  const int col = blockIdx.x * 32 + (threadIdx.x & 31), grp = threadIdx.x >> 5;
+  float sum = 0.f;
+  if (col < C) {
+    const float* p = part + (size_t)s_first * C + col;
+#pragma unroll 4
+    for (int i = grp; i < s_count; i += 8) sum += p[(size_t)i * C];
+  }
+  s_sum[grp][threadIdx.x & 31] = sum;
+  __syncthreads();
+  if (threadIdx.x < 32 && col < C) {
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t += s_sum[q][threadIdx.x];
+    db[(size_t)e * C + col] = __float2bfloat16_rn(t);
   }
 }
 
@@ -393,12 +297,6 @@ unsigned blocks_for(int64_t n, int per) { return (unsigned)((n + per - 1) / per)
 int launch_pair_of(const int32_t* row_of, int64_t M, int32_t* pair_of, cudaStream_t s) {
   if (M == 0) return 0;
   pair_of_kernel<<<blocks_for(M, 256), 256, 0, s>>>(row_of, M, pair_of);
-  MOE_CUDA_CHECK(cudaGetLastError());
-  return 0;
-}
-
-int launch_pad_offsets(const int32_t* offsets, int E, int32_t* koff, cudaStream_t s) {
-  pad_offsets_kernel<<<1, 32, 0, s>>>(offsets, E, koff);
   MOE_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
@@ -414,11 +312,11 @@ int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, 
 }
 
 int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, const float* dw,
-                      const int32_t* cnt0, float grad_aux, const void* x, const void* Wg, int64_t N,
-                      int d, int E, int k, float* dl, float* dWg_f32, float* dbg_f32, void* dWg,
+                      const int32_t* cnt0, float grad_aux, const float* grad_aux_dev, const void* x, const void* Wg,
+                      int64_t N, int d, int E, int k, float* dl, float* dWg_f32, float* dbg_f32, void* dWg,
                       void* dbg, void* dxr, cudaStream_t s) {
   if (N == 0) return 0;
-  router_bwd_kernel<<<blocks_for(N, 8), 256, 0, s>>>(logits, idx, w, dw, cnt0, grad_aux, N, E, k, dl);
+  router_bwd_kernel<<<blocks_for(N, 8), 256, 0, s>>>(logits, idx, w, dw, cnt0, grad_aux, grad_aux_dev, N, E, k, dl);
   MOE_CUDA_CHECK(cudaGetLastError());
   MOE_CUDA_CHECK(cudaMemsetAsync(dWg_f32, 0, sizeof(float) * (size_t)E * d, s));
   MOE_CUDA_CHECK(cudaMemsetAsync(dbg_f32, 0, sizeof(float) * (size_t)E, s));
@@ -435,9 +333,11 @@ int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, c
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(Wg), dl, N, d, E,
       (int)per, dWg_f32, dbg_f32, static_cast<__nv_bfloat16*>(dxr));
   MOE_CUDA_CHECK(cudaGetLastError());
-  f32_to_bf16_kernel<<<blocks_for((int64_t)E * d, 256), 256, 0, s>>>(dWg_f32, (int64_t)E * d,
+  if (dWg != nullptr)
+    f32_to_bf16_kernel<<<blocks_for((int64_t)E * d, 256), 256, 0, s>>>(dWg_f32, (int64_t)E * d,
                                                                        static_cast<__nv_bfloat16*>(dWg));
-  f32_to_bf16_kernel<<<blocks_for(E, 256), 256, 0, s>>>(dbg_f32, E, static_cast<__nv_bfloat16*>(dbg));
+  if (dbg != nullptr)
+    f32_to_bf16_kernel<<<blocks_for(E, 256), 256, 0, s>>>(dbg_f32, E, static_cast<__nv_bfloat16*>(dbg));
   MOE_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
@@ -456,37 +356,21 @@ int launch_fill_f32(float* p, int64_t n, float v, cudaStream_t s) {
   return 0;
 }
 
-int launch_geglu_bwd(const void* dh, void* gu, const int32_t* pair_of, int64_t M, int f,
-                     uint32_t thresh, float scale, uint32_t seed_lo, uint32_t seed_hi, cudaStream_t s) {
-  if (M == 0) return 0;
-  geglu_bwd_kernel<<<blocks_for(M * (f >> 3), 256), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(gu), pair_of, M, f, thresh,
-      scale, seed_lo, seed_hi);
+int launch_colsum_finish(const float* part, int slots, const int32_t* offsets, int E, int C, void* db,
+                         cudaStream_t s) {
+  colsum_finish_kernel<<<dim3((C + 31) / 32, E), 256, 0, s>>>(part, slots, offsets, C,
+                                                             static_cast<__nv_bfloat16*>(db));
   MOE_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
 
-int launch_transpose_weights(const void* const* src_ptrs, int E, int R, int C, void* dst, cudaStream_t s) {
-  transpose_weight_kernel<<<dim3((C + 63) / 64, (R + 63) / 64, E), 256, 0, s>>>(
-      src_ptrs, R, C, static_cast<__nv_bfloat16*>(dst));
+int launch_colsum(const void* src, const int32_t* offsets, int64_t M, int E, int C, float* part, void* db,
+                  cudaStream_t s) {
+  const unsigned tiles = blocks_for(M, 256) + (unsigned)E;    // at least as many as there are
+  colsum_kernel<<<dim3((C + 63) / 64, tiles), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(src), offsets, E, C,
+                                                            part);
   MOE_CUDA_CHECK(cudaGetLastError());
-  return 0;
-}
-
-int launch_transpose_pad(const void* src, const int32_t* offsets, const int32_t* koff, int E, int C,
-                         int64_t Kpad, void* dst, cudaStream_t s) {
-  if (Kpad == 0) return 0;
-  transpose_pad_kernel<<<dim3((unsigned)(Kpad / 64), (C + 63) / 64), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(src), offsets, koff, E, C, Kpad, static_cast<__nv_bfloat16*>(dst));
-  MOE_CUDA_CHECK(cudaGetLastError());
-  return 0;
-}
-
-int launch_colsum(const void* src, const int32_t* offsets, int E, int C, void* db, cudaStream_t s) {
-  colsum_kernel<<<dim3((C + 63) / 64, E), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(src),
-                                                        offsets, C, static_cast<__nv_bfloat16*>(db));
-  MOE_CUDA_CHECK(cudaGetLastError());
-  return 0;
+  return launch_colsum_finish(part, 1, offsets, E, C, db, s);
 }
 
 }  // namespace moe

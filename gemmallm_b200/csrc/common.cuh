@@ -129,6 +129,11 @@ __device__ __forceinline__ float tanh_approx(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float exp2f_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __device__ __forceinline__ float gelu_tanh_fast(float g) {
   const float kBeta = 0.7978845608028654f;
   float g2 = g * g;
@@ -241,9 +246,13 @@ struct EpScatter {
 // what the backward pass needs): the pre-activations gate/up with their biases go to
 // gu [M, 2f] (columns [0,f) gate, [f,2f) up), and h is multiplied by the dropout mask of its
 // (token, slot) pair: element (pair, c) is kept iff its Philox word (philox.cuh) is >= thresh,
-// and scaled by `scale` = 1 / (1 - p).
+// and scaled by `scale` = 1 / (1 - p). The backward pass reads the mask back and replaces gu by
+// its gradient; col_part receives the column sums of that gradient, one row per 128-row half
+// of a 256-row tile (tiles counted over the experts in order).
 struct TrainArgs {
   __nv_bfloat16* gu;
+  uint8_t* mask;            // [M, f / 8] one bit per element of h, set = kept
+  float* col_part;          // [2 * m-tiles, 2f], backward only
   const int32_t* pair_of;   // [M] token * k + slot of every sorted row
   uint32_t thresh;          // p * 2^32; 0 keeps everything
   float scale;
@@ -275,16 +284,15 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
                        int f, int E, void* h, void* y, const EpScatter* sc, int32_t* status,
                        cudaStream_t s, const TrainArgs* train = nullptr, const EpSync* ep_wait = nullptr,
                        const EpSync* ep_signal = nullptr);
-// One grouped product out[rows of e] = A[rows of e] . B_e^T (+ bias_e), B_e given by the e-th
-// tensor map of tmaps_b ([Nout, K] row-major, 128-row boxes); bias may be nullptr.
-int launch_grouped_rows(const void* A, int64_t M, int K, const void* tmaps_b, const int32_t* offsets,
-                        const void* const* bias, int E, int Nout, void* out, int32_t* status,
-                        cudaStream_t s);
-// Grouped over the contraction index: out_e [Ra, Rb] = At[:, K_e] . Bt[:, K_e]^T for the column
-// ranges K_e = [koff[e], koff[e+1]) (multiples of 64) of At [Ra, Kpad] and Bt [Rb, Kpad];
-// out [E][Ra][Rb]. Experts with an empty range are skipped (their slice is left untouched).
-int launch_grouped_cols(const void* At, const void* Bt, int64_t Kpad, int Ra, int Rb,
-                        const int32_t* koff, void* out, int E, int32_t* status, cudaStream_t s);
+// Input gradient of a grouped Linear: out[rows of e] = A[rows of e] . B_e, B_e [K, Nout] row-major, given by
+// the e-th tensor map of tmaps_b (64-row boxes). With geglu_bwd the product is dh (Nout = f) and is not
+// stored: the epilogue carries it back to gu (see TrainArgs).
+int launch_grouped_dx(const void* A, int64_t M, int K, const void* tmaps_b, const int32_t* offsets, int E, int Nout,
+                      void* out, const TrainArgs* geglu_bwd, int32_t* status, cudaStream_t s);
+// Weight gradients: out_e [Ra, Rb] = A[rows of e]^T . B[rows of e], A [M, Ra], B [M, Rb]; zeros for experts
+// without rows.
+int launch_grouped_wgrad(const void* A, const void* B, int64_t M, int Ra, int Rb, const int32_t* offsets, void* out,
+                         int E, int32_t* status, cudaStream_t s);
 int64_t ep_scratch_ints(int64_t N, int EV, int E);
 int launch_ep_begin(uint32_t* epoch, uint32_t* done_counter, int32_t* status, int32_t* scratch, int EV,
                     int E, cudaStream_t s);
@@ -339,20 +347,17 @@ int launch_experts_gemv(const void* perm, const int32_t* offsets, const void* pl
 
 // ---- backward.cu ----
 int launch_pair_of(const int32_t* row_of, int64_t M, int32_t* pair_of, cudaStream_t s);
-int launch_pad_offsets(const int32_t* offsets, int E, int32_t* koff, cudaStream_t s);
 int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, const float* w,
                        int64_t M, int d, int k, void* dy, float* dw, cudaStream_t s);
 int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, const float* dw,
-                      const int32_t* cnt0, float grad_aux, const void* x, const void* Wg, int64_t N,
-                      int d, int E, int k, float* dl, float* dWg_f32, float* dbg_f32, void* dWg,
+                      const int32_t* cnt0, float grad_aux, const float* grad_aux_dev, const void* x, const void* Wg,
+                      int64_t N, int d, int E, int k, float* dl, float* dWg_f32, float* dbg_f32, void* dWg,
                       void* dbg, void* dxr, cudaStream_t s);
 int launch_fill_f32(float* p, int64_t n, float v, cudaStream_t s);
 int launch_iota(int32_t* p, int64_t n, cudaStream_t s);
-int launch_geglu_bwd(const void* dh, void* gu, const int32_t* pair_of, int64_t M, int f,
-                     uint32_t thresh, float scale, uint32_t seed_lo, uint32_t seed_hi, cudaStream_t s);
-int launch_transpose_weights(const void* const* src_ptrs, int E, int R, int C, void* dst, cudaStream_t s);
-int launch_transpose_pad(const void* src, const int32_t* offsets, const int32_t* koff, int E, int C,
-                         int64_t Kpad, void* dst, cudaStream_t s);
-int launch_colsum(const void* src, const int32_t* offsets, int E, int C, void* db, cudaStream_t s);
+// Bias gradients: column sums of src [M, C] over every expert's rows; part as TrainArgs::col_part.
+int launch_colsum(const void* src, const int32_t* offsets, int64_t M, int E, int C, float* part, void* db,
+                  cudaStream_t s);
+int launch_colsum_finish(const float* part, int slots, const int32_t* offsets, int E, int C, void* db, cudaStream_t s);
 
 }  // namespace moe

@@ -19,10 +19,16 @@
 // Math and epilogue (tc_epilogue.cuh): reference model.py:174,180-184.
 //
 // The same kernel serves the backward pass (the reference trains through this block with
-// torch.autograd, train.py:140): the input gradients are two more row-grouped products
-// against transposed weights; the weight gradients dW_e = dY_e^T X_e contract over an
-// expert's rows, so there (COLS) a group is a range of the contraction index of two
-// transposed activation buffers and every expert has the same output tiles.
+// torch.autograd, train.py:140). The input gradients are two more row-grouped products whose
+// weights are read as they lie in memory: their rows are the contraction index there, so the B
+// operand is MN-major in shared memory (B_MN; 64 x 64 boxes, see make_smem_desc_mn) and no
+// transposed copy of the weights is made. The weight gradients dW_e = dY_e^T X_e (COLS) contract
+// over an expert's rows: both operands are MN-major tiles of the activation buffers, a group is
+// a range of rows, and every expert has the same output tiles. An expert's last 64-row block holds
+// rows of the next expert; an eleventh warp (the "fixer") waits for such a block itself, zeroes
+// those rows in shared memory up to the next multiple of 16, which is where the products of that
+// block stop, and passes the stage on. (Only there do the two CTAs arrive on a common barrier: an
+// arrival across the pair for every block halved the rate, 680 instead of 1280 TFLOP/s.)
 #include <cuda.h>
 #include "common.cuh"
 #include "tc_ptx.cuh"
@@ -39,29 +45,61 @@ constexpr int BM = 128;           // rows per CTA = TMEM lanes
 constexpr int kPairRows = 256;    // rows per tile (both CTAs)
 constexpr int BK = 64;
 constexpr int BN = 256;
-constexpr int kStages = 6;
+constexpr int kMaxStages = 6;
 constexpr int kABytes = BM * BK * 2;         // 16 KiB: this CTA's rows
 constexpr int kBBytes = (BN / 2) * BK * 2;   // 16 KiB: this CTA's half of the weight tile
 constexpr int kStageBytes = kABytes + kBBytes;
-constexpr int kThreads = 320;   // TMA warp, MMA warp, 8 epilogue warps
 constexpr int kTmemCols = 2 * BN;
+constexpr int kHalfTile = 64 * BK * 2;   // one 64 x 64 box of an MN-major operand: 8 KiB
+
+// What a launch computes. Rows of A are grouped by expert except in kWgrad.
+enum Kind {
+  kGeglu,        // h = gelu(x Wg^T + bg) * (x Wu^T + bu)
+  kGegluTrain,   // the same with dropout, keeping pre-activations and mask (TrainArgs)
+  kPlain,        // y = h W2^T + b2
+  kScatter,      // the same into the token owners' buffers (expert parallelism)
+  kDx,           // out = A B, B [K, Nout] as it lies in memory
+  kDhGeglu,      // dh = dy W2 as kDx, then back through dropout, product and GELU in the epilogue
+  kWgrad         // out_e [Ra, Nout] = A[rows of e]^T B[rows of e]
+};
+template <int KIND>
+struct Traits {
+  static constexpr bool GEGLU = KIND == kGeglu || KIND == kGegluTrain;
+  static constexpr bool COLS = KIND == kWgrad;
+  static constexpr bool A_MN = COLS;
+  static constexpr bool B_MN = KIND == kDx || KIND == kDhGeglu || COLS;
+  // The training epilogues do 20 to 40 instructions per accumulator element (Philox, GELU and its
+  // derivative): eight warps cannot issue them in the time of a tile's products, sixteen can.
+  static constexpr int kEpiWarps = KIND == kGegluTrain || KIND == kDhGeglu ? 16 : 8;
+  static constexpr int kThreads = 64 + 32 * kEpiWarps + (COLS ? 32 : 0);
+  static constexpr int kStgWarp = KIND == kGegluTrain ? kStg32Bytes : kStgBytes;
+  static constexpr int kStages = KIND == kDhGeglu ? 5 : 6;   // its staging areas take a stage's room
+  static constexpr int kColBytes = KIND == kDhGeglu ? 4 * 2 * BN * 4 : 0;   // column sums, four lane quadrants
+};
 // M = 256 across the pair: M/16 at bit 24
 constexpr uint32_t kIdesc2 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                              ((256u >> 4) << 24);
 
 struct Control {
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
+  uint64_t full[kMaxStages];
+  uint64_t empty[kMaxStages];
+  uint64_t tail[kMaxStages];   // COLS: this CTA's half of a block that has to be cut has arrived
+  uint64_t peer_cut[kMaxStages];   // COLS, even CTA: the odd CTA's half has been cut
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   int abort;
   int tile_start[kMaxExperts + 1];
   int offsets[kMaxExperts + 1];
-  alignas(16) uint8_t stage_out[8][kStgBytes];  // one staging area per epilogue warp
 };
 
-constexpr size_t kSmemBytes = 1024 + (size_t)kStages * kStageBytes + sizeof(Control);
+// [stages][Control][staging area of every epilogue warp][column sums]
+constexpr size_t kControlBytes = (sizeof(Control) + 15) & ~(size_t)15;
+template <int KIND>
+constexpr size_t smem_bytes() {
+  using T = Traits<KIND>;
+  return 1024 + (size_t)T::kStages * kStageBytes + kControlBytes + (size_t)T::kEpiWarps * T::kStgWarp + T::kColBytes;
+}
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -101,27 +139,74 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uin
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// mbar_wait for a barrier the peer CTA arrives on
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* abort_flag, int32_t* status,
+                                                  int where) {
+  const unsigned long long t0 = global_ns();
+  for (uint32_t it = 1;; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((it & 255u) == 0) {
+      if (*reinterpret_cast<volatile int*>(abort_flag)) return false;
+      if (global_ns() - t0 > kWaitLimitNs) {
+        *reinterpret_cast<volatile int*>(abort_flag) = 1;
+        atomicMax(&status[0], MOE_B200_DEV_TIMEOUT);
+        status[1] = where;
+        status[2] = (int)blockIdx.x;
+        return false;
+      }
+    }
+  }
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster)
                : "memory");
 }
 
+// Barrier of `threads` threads (all of them in whole warps) that also tells whether all of them agree.
+__device__ __forceinline__ bool barrier_and(int id, int threads, bool ok) {
+  int all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.s32 p, %3, 0;\n\t"
+      "barrier.cta.red.and.pred q, %1, %2, p;\n\t"
+      "selp.s32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"(id), "r"(threads), "r"((int)ok)
+      : "memory");
+  return all != 0;
+}
+
 // COLS = false: groups are row ranges [offsets[e], offsets[e+1]) of A; B_e = tmap_b[e]; K fixed.
-// COLS = true : groups are ranges [offsets[e], offsets[e+1]) (multiples of 64) of the contraction
-//               index; A has Ra rows, B (one map, tmap_bc) has Nout rows; out [E][Ra][Nout].
-template <bool GEGLU, bool SCATTER, bool TRAIN, bool COLS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+// COLS = true : groups are the same row ranges, contracted over; A has Ra columns, B (one map,
+//               tmap_bc) has Nout columns; out [E][Ra][Nout], zero for experts without rows.
+template <int KIND>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Traits<KIND>::kThreads, 1)
 grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                         const __grid_constant__ CUtensorMap tmap_bc,
-                        const CUtensorMap* __restrict__ tmap_b,  // [E], 128-row boxes
+                        const CUtensorMap* __restrict__ tmap_b,  // [E], 128-row (B_MN: 64-row) boxes
                         const int32_t* __restrict__ offsets,
                         const void* const* __restrict__ bias_ptrs, int E, int K, int Nout,
                         __nv_bfloat16* __restrict__ out, const EpScatter sc, const TrainArgs tr,
                         const EpSync sy, int Ra, int32_t* __restrict__ status) {
+  using T = Traits<KIND>;
+  constexpr bool GEGLU = T::GEGLU, COLS = T::COLS, A_MN = T::A_MN, B_MN = T::B_MN;
+  constexpr int kStages = T::kStages, kEpiWarps = T::kEpiWarps;
+  constexpr uint32_t kIdesc = kIdesc2 | (A_MN ? 1u << 15 : 0u) | (B_MN ? 1u << 16 : 0u);
+  // descriptor step of one K = 16 product: 32 bytes along a row, or sixteen 128-byte rows
+  constexpr uint64_t kStepA = A_MN ? 16 * 128 / 16 : 2, kStepB = B_MN ? 16 * 128 / 16 : 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~(uintptr_t)1023);
   Control* ctl = reinterpret_cast<Control*>(smem + (size_t)kStages * kStageBytes);
+  uint8_t* stage_out = smem + (size_t)kStages * kStageBytes + kControlBytes;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -134,8 +219,13 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int m_tiles_cols = (Ra + kPairRows - 1) / kPairRows;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&ctl->tmem_full[a], 1); mbar_init(&ctl->tmem_empty[a], 16); }
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&ctl->full[s], 1);
+      mbar_init(&ctl->empty[s], 1);
+      mbar_init(&ctl->tail[s], 1);
+      mbar_init(&ctl->peer_cut[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) { mbar_init(&ctl->tmem_full[a], 1); mbar_init(&ctl->tmem_empty[a], 2 * kEpiWarps); }
     ctl->abort = 0;
   }
   if (warp == 1) {
@@ -160,8 +250,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       ctl->tile_start[e] = acc;
       const int end = offsets[e + 1];
       ctl->offsets[e + 1] = end;
-      acc += COLS ? (end > beg ? m_tiles_cols * n_tiles : 0)
-                  : ((end - beg + kPairRows - 1) / kPairRows) * n_tiles;
+      acc += (COLS ? m_tiles_cols : (end - beg + kPairRows - 1) / kPairRows) * n_tiles;
       beg = end;
     }
     ctl->tile_start[E] = arrived ? acc : 0;   // a peer never arrived: nothing to do
@@ -191,16 +280,34 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                                : nt * kTileN + (int)cta * (BN / 2);
         const CUtensorMap* tb = COLS ? &tmap_bc : tmap_b + e;
         const int k0 = COLS ? ctl->offsets[e] : 0;
-        const int k_blocks = COLS ? (ctl->offsets[e + 1] - k0) / BK : k_blocks_rows;
+        const int k_rows = COLS ? ctl->offsets[e + 1] - k0 : 0;
+        const int k_blocks = COLS ? (k_rows + BK - 1) / BK : k_blocks_rows;
         for (int kb = 0; kb < k_blocks; ++kb) {
           {
             if (!mbar_wait(&ctl->empty[stage], phase ^ 1u, &ctl->abort, status, 31)) { ok = false; break; }
           }
           uint8_t* sa = smem + (size_t)stage * kStageBytes;
           const uint32_t full0 = map_to_cta(smem_u32(&ctl->full[stage]), 0);
-          if (cta == 0) mbar_expect_tx(&ctl->full[stage], 2 * kStageBytes);
-          tma_load_2d_pair(sa, &tmap_a, full0, k0 + kb * BK, row0);
-          tma_load_2d_pair(sa + kABytes, tb, full0, k0 + kb * BK, brow);
+          uint32_t bar = full0;
+          if (COLS && (kb + 1) * BK > k_rows) {
+            mbar_expect_tx(&ctl->tail[stage], kStageBytes);     // the fixer passes it on
+            bar = map_to_cta(smem_u32(&ctl->tail[stage]), cta);
+          } else if (cta == 0) {
+            mbar_expect_tx(&ctl->full[stage], 2 * kStageBytes);
+          }
+          const int kc = k0 + kb * BK;
+          if (A_MN) {
+            tma_load_2d_pair(sa, &tmap_a, bar, row0, kc);
+            tma_load_2d_pair(sa + kHalfTile, &tmap_a, bar, row0 + 64, kc);
+          } else {
+            tma_load_2d_pair(sa, &tmap_a, bar, kc, row0);
+          }
+          if (B_MN) {
+            tma_load_2d_pair(sa + kABytes, tb, bar, brow, kc);
+            tma_load_2d_pair(sa + kABytes + kHalfTile, tb, bar, brow + 64, kc);
+          } else {
+            tma_load_2d_pair(sa + kABytes, tb, bar, kc, brow);
+          }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -214,13 +321,15 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       int it = 0;
       int e = 0;
       bool ok = true;
-      for (int t = pair; ok && t < total_tiles; t += num_pairs, ++it) {
-        const int a = it & 1;
-        int k_blocks = k_blocks_rows;
+      for (int t = pair; ok && t < total_tiles; t += num_pairs) {
+        int k_blocks = k_blocks_rows, k_rows = 0;
         if (COLS) {
           while (t >= ctl->tile_start[e + 1]) ++e;
-          k_blocks = (ctl->offsets[e + 1] - ctl->offsets[e]) / BK;
+          k_rows = ctl->offsets[e + 1] - ctl->offsets[e];
+          k_blocks = (k_rows + BK - 1) / BK;
+          if (k_blocks == 0) continue;     // nothing to add up: the epilogue stores zeros
         }
+        const int a = it & 1;
         {
           if (!mbar_wait(&ctl->tmem_empty[a], acc_phase ^ 1u, &ctl->abort, status, 32)) { ok = false; break; }
         }
@@ -232,12 +341,14 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + (size_t)stage * kStageBytes);
-          const uint64_t adesc = make_smem_desc(sa);
-          const uint64_t bdesc = make_smem_desc(sa + kABytes);
+          const uint64_t adesc = A_MN ? make_smem_desc_mn(sa) : make_smem_desc(sa);
+          const uint64_t bdesc = B_MN ? make_smem_desc_mn(sa + kABytes) : make_smem_desc(sa + kABytes);
+          const int left = COLS ? k_rows - kb * BK : BK;    // rows of this expert in the block
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk)
-            tc_mma_pair(tmem_d, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), kIdesc2,
-                        (kb | kk) != 0 ? 1u : 0u);
+            if (!COLS || kk * 16 < left)
+              tc_mma_pair(tmem_d, adesc + (uint64_t)kk * kStepA, bdesc + (uint64_t)kk * kStepB, kIdesc,
+                          (kb | kk) != 0 ? 1u : 0u);
           // the stage is free in both CTAs once these MMAs have read it
           const uint32_t e_local = smem_u32(&ctl->empty[stage]);
           tc_commit_pair(map_to_cta(e_local, 0));
@@ -249,41 +360,106 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         tc_commit_pair(map_to_cta(f_local, 0));
         tc_commit_pair(map_to_cta(f_local, 1));
         if (a == 1) acc_phase ^= 1u;
+        ++it;
       }
     }
+  } else if (COLS && warp == 2 + kEpiWarps) {
+    // ---------------- fixer: blocks that run past the expert's last row ----------------
+    int blocks = 0;             // K blocks of this CTA's tiles so far
+    uint32_t parity = 0;        // bit s: parity of the next use of tail[s]
+    int e = 0;
+    for (int t = pair; t < total_tiles; t += num_pairs) {
+      while (t >= ctl->tile_start[e + 1]) ++e;
+      const int k_rows = ctl->offsets[e + 1] - ctl->offsets[e];
+      const int k_blocks = (k_rows + BK - 1) / BK;
+      const int left = k_rows - (k_blocks - 1) * BK;        // rows of the last block, 1 .. 64
+      blocks = (blocks + k_blocks) % kStages;
+      if (k_blocks == 0 || left == BK) continue;
+      const int s = (blocks + kStages - 1) % kStages;       // the stage of the last block
+      if (!mbar_wait(&ctl->tail[s], (parity >> s) & 1u, &ctl->abort, status, 35)) break;
+      uint8_t* sa = smem + (size_t)s * kStageBytes;
+      // rows [left, next multiple of 16) of the four 64 x 64 boxes; a row is 128 bytes
+      const int pieces = (((left + 15) & ~15) - left) * 8;
+      for (int i = lane; i < 4 * pieces; i += 32) {
+        const int box = i / pieces, p = i - box * pieces;
+        *reinterpret_cast<uint4*>(sa + box * kHalfTile + (size_t)left * 128 + p * 16) = make_uint4(0, 0, 0, 0);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (cta == 1) {
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->peer_cut[s]), 0));
+      } else {
+        if (!mbar_wait_cluster(&ctl->peer_cut[s], (parity >> s) & 1u, &ctl->abort, status, 36)) break;
+        if (lane == 0) mbar_arrive(&ctl->full[s]);
+      }
+      parity ^= 1u << s;
+    }
   } else {
-    // ---------------- epilogue: 8 warps per CTA, one accumulator row per thread ----------------
+    // ---------------- epilogue: one accumulator row per thread ----------------
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;  // two warps per TMEM lane quadrant split the columns
+    const int part = (warp - 2) >> 2;  // the warps of a TMEM lane quadrant split the columns
     const int r = quad * 32 + lane;
+    uint8_t* stg = stage_out + (warp - 2) * T::kStgWarp;
     uint32_t acc_phase = 0;
     int it = 0;
     int e = 0;
     bool ok = true;
-    for (int t = pair; ok && t < total_tiles; t += num_pairs, ++it) {
+    for (int t = pair; ok && t < total_tiles; t += num_pairs) {
       while (t >= ctl->tile_start[e + 1]) ++e;
       const int local = t - ctl->tile_start[e];
       const int mt = local / n_tiles, nt = local - mt * n_tiles;
-      const int row = (COLS ? 0 : ctl->offsets[e]) + mt * kPairRows + (int)cta * BM + r;
-      const bool row_ok = COLS ? row < Ra : row < ctl->offsets[e + 1];
+      const int row_end = COLS ? Ra : ctl->offsets[e + 1];
+      const int row_cta = (COLS ? 0 : ctl->offsets[e]) + mt * kPairRows + (int)cta * BM;
+      const int row_warp = row_cta + quad * 32;
+      const int rows = min(32, row_end - row_warp);   // rows of this warp to store (may be negative)
       const int n0 = nt * kTileN;
       const __nv_bfloat16* bias =
           bias_ptrs != nullptr ? static_cast<const __nv_bfloat16*>(bias_ptrs[e]) : nullptr;
       __nv_bfloat16* out_e = COLS ? out + (size_t)e * Ra * Nout : out;
-      const int a = it & 1;
-      {
-        if (!mbar_wait(&ctl->tmem_full[a], acc_phase, &ctl->abort, status, 34)) { ok = false; break; }
+      if (COLS && ctl->offsets[e + 1] == ctl->offsets[e]) {
+        store_zero_tile(out_e, row_warp, rows, Nout, n0 + part * 128, lane);
+        continue;
       }
+      const int a = it & 1;
+      GegluBwd gb;
+      if constexpr (KIND == kDhGeglu)     // its inputs are requested before the products are awaited
+        gb.start(tr, row_warp, rows, Nout, n0 + part * 64, lane);
+      ok = mbar_wait(&ctl->tmem_full[a], acc_phase, &ctl->abort, status, 34);
+      if (KIND != kDhGeglu && !ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN);
-      store_tile<GEGLU, SCATTER, TRAIN>(taddr, row, row_ok, n0, Nout, bias, out_e, sc, tr,
-                                        ctl->stage_out[warp - 2], lane, half);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->tmem_empty[a]), 0));
+      auto release = [&]() {     // this warp has read its part of the accumulator
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->tmem_empty[a]), 0));
+      };
+      if constexpr (KIND == kGegluTrain) {
+        store_tile_train(taddr, row_warp, rows, n0, Nout, bias, out_e, tr, stg, lane, part);
+        release();
+      } else if constexpr (KIND == kDhGeglu) {
+        float* s_col = reinterpret_cast<float*>(stage_out + kEpiWarps * T::kStgWarp);
+        if (ok) gb.finish(taddr + part * 64, stg, s_col + quad * 2 * BN + part * 64, BN, release);
+        // column sums of this CTA's 128 rows: the four lane quadrants in order. A warp whose wait
+        // ran out still comes to the barrier, and all leave together.
+        ok = barrier_and(1, 32 * kEpiWarps, ok);
+        if (!ok) break;
+        const int c = (int)threadIdx.x - 64;
+        const int col = n0 + (c & (BN - 1));
+        if (col < Nout) {
+          const float sum = (s_col[c] + s_col[2 * BN + c]) + (s_col[4 * BN + c] + s_col[6 * BN + c]);
+          const int64_t slot = (int64_t)(ctl->tile_start[e] / n_tiles + mt) * 2 + (int)cta;
+          tr.col_part[slot * 2 * Nout + (c >= BN ? Nout : 0) + col] = sum;
+        }
+        barrier_and(1, 32 * kEpiWarps, true);
+      } else {
+        store_tile<GEGLU, KIND == kScatter>(taddr, row_cta + r, row_cta + r < row_end, n0, Nout, bias, out_e, sc, stg,
+                                            lane, part);
+        release();
+      }
       if (a == 1) acc_phase ^= 1u;
+      ++it;
     }
-    if (SCATTER) __threadfence_system();
+    if (KIND == kScatter) __threadfence_system();
   }
   // expert-parallel down pass: the last CTA to get here tells every rank that this rank's
   // outputs have been stored
@@ -306,15 +482,17 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
 }
 
-template <bool GEGLU, bool SCATTER, bool TRAIN, bool COLS>
+template <int KIND>
 int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_bc, const void* tmap_b, const int32_t* offsets,
                 const void* const* bias, int E, int K, int Nout, void* out, const EpScatter& sc,
                 const TrainArgs& tr, const EpSync& sy, int Ra, int32_t* status, int sms, cudaStream_t s) {
   static PerDeviceOnce once;
-  auto fn = grouped_gemm_tc2_kernel<GEGLU, SCATTER, TRAIN, COLS>;
-  int rc = ensure_dynamic_smem(once, fn, kSmemBytes);
+  auto fn = grouped_gemm_tc2_kernel<KIND>;
+  constexpr size_t smem = smem_bytes<KIND>();
+  static_assert(smem <= 227 * 1024, "shared memory of one CTA");
+  int rc = ensure_dynamic_smem(once, fn, smem);
   if (rc) return rc;
-  MOE_CUDA_CHECK(launch_pdl(fn, dim3(sms & ~1), dim3(kThreads), kSmemBytes, s, tm_a, tm_bc,
+  MOE_CUDA_CHECK(launch_pdl(fn, dim3(sms & ~1), dim3(Traits<KIND>::kThreads), smem, s, tm_a, tm_bc,
                             static_cast<const CUtensorMap*>(tmap_b), offsets, bias, E, K, Nout,
                             static_cast<__nv_bfloat16*>(out), sc, tr, sy, Ra, status));
   return 0;
@@ -344,22 +522,19 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
   const EpSync& sy1 = ep_wait != nullptr ? *ep_wait : nosync;
   const EpSync& sy2 = ep_signal != nullptr ? *ep_signal : nosync;
   if (train != nullptr)
-    rc = launch_pair<true, false, true, false>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, *train,
-                                               sy1, 0, status, sms, s);
+    rc = launch_pair<kGegluTrain>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, *train, sy1, 0, status,
+                                  sms, s);
   else
-    rc = launch_pair<true, false, false, false>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, eval,
-                                                sy1, 0, status, sms, s);
+    rc = launch_pair<kGeglu>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, eval, sy1, 0, status, sms, s);
   if (rc) return rc;
   if (sc != nullptr)
-    return launch_pair<false, true, false, false>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, nullptr, *sc,
-                                                  eval, sy2, 0, status, sms, s);
-  return launch_pair<false, false, false, false>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, y, none, eval,
-                                                 sy2, 0, status, sms, s);
+    return launch_pair<kScatter>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, nullptr, *sc, eval, sy2, 0, status,
+                                 sms, s);
+  return launch_pair<kPlain>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, y, none, eval, sy2, 0, status, sms, s);
 }
 
-int launch_grouped_rows(const void* A, int64_t M, int K, const void* tmaps_b, const int32_t* offsets,
-                        const void* const* bias, int E, int Nout, void* out, int32_t* status,
-                        cudaStream_t s) {
+int launch_grouped_dx(const void* A, int64_t M, int K, const void* tmaps_b, const int32_t* offsets, int E, int Nout,
+                      void* out, const TrainArgs* geglu_bwd, int32_t* status, cudaStream_t s) {
   if (M == 0 || E == 0) return 0;
   alignas(64) CUtensorMap tm_a;
   int rc = encode_tmap_2d(&tm_a, A, (uint64_t)M, (uint64_t)K, BM);
@@ -370,17 +545,20 @@ int launch_grouped_rows(const void* A, int64_t M, int K, const void* tmaps_b, co
   const EpScatter none = {};
   const TrainArgs eval = {};
   const EpSync nosync = {};
-  return launch_pair<false, false, false, false>(tm_a, tm_a, tmaps_b, offsets, bias, E, K, Nout, out, none,
-                                                 eval, nosync, 0, status, sms, s);
+  if (geglu_bwd != nullptr)
+    return launch_pair<kDhGeglu>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, nullptr, none, *geglu_bwd,
+                                 nosync, 0, status, sms, s);
+  return launch_pair<kDx>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, out, none, eval, nosync, 0, status, sms,
+                          s);
 }
 
-int launch_grouped_cols(const void* At, const void* Bt, int64_t Kpad, int Ra, int Rb,
-                        const int32_t* koff, void* out, int E, int32_t* status, cudaStream_t s) {
-  if (Kpad == 0 || E == 0) return 0;
+int launch_grouped_wgrad(const void* A, const void* B, int64_t M, int Ra, int Rb, const int32_t* offsets, void* out,
+                         int E, int32_t* status, cudaStream_t s) {
+  if (M == 0 || E == 0) return 0;
   alignas(64) CUtensorMap tm_a, tm_b;
-  int rc = encode_tmap_2d(&tm_a, At, (uint64_t)Ra, (uint64_t)Kpad, BM);
+  int rc = encode_tmap_2d(&tm_a, A, (uint64_t)M, (uint64_t)Ra, BK);
   if (rc) return rc;
-  rc = encode_tmap_2d(&tm_b, Bt, (uint64_t)Rb, (uint64_t)Kpad, BM);
+  rc = encode_tmap_2d(&tm_b, B, (uint64_t)M, (uint64_t)Rb, BK);
   if (rc) return rc;
   int sms = 0;
   rc = sm_count(&sms);
@@ -388,8 +566,8 @@ int launch_grouped_cols(const void* At, const void* Bt, int64_t Kpad, int Ra, in
   const EpScatter none = {};
   const TrainArgs eval = {};
   const EpSync nosync = {};
-  return launch_pair<false, false, false, true>(tm_a, tm_b, nullptr, koff, nullptr, E, 0, Rb, out,
-                                                none, eval, nosync, Ra, status, sms, s);
+  return launch_pair<kWgrad>(tm_a, tm_b, nullptr, offsets, nullptr, E, 0, Rb, out, none, eval, nosync, Ra, status,
+                             sms, s);
 }
 
 }  // namespace moe

@@ -12,4 +12,28 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
                  int E, int k, int dtype, int flags, void* workspace, size_t workspace_bytes, void* out,
                  float* aux, void* stream);
 
+// Where the gradients of a backward pass go; nullptr: not wanted, and its kernels are not launched.
+struct TrainGrads {
+  void* x;                   // [N, d]
+  void *wg, *bg;             // router [E, d], [E]
+  void *w1, *b1, *w2, *b2;   // experts [E, 2f, d], [E, 2f], [E, d, f], [E, d]
+};
+
+// moe_b200_forward_train with the load-balancing loss written to `aux` (nullptr: the workspace's word).
+int forward_train_into(const void* x, const void* Wg, const void* bg, const void* plan, const void* residual,
+                       int64_t N, int d, int f, int E, int k, int dtype, float dropout_p, uint64_t seed,
+                       void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes, void* out,
+                       float* aux, void* stream);
+// moe_b200_backward with the gradients written where the caller wants them and the loss's gradient read
+// from device memory (grad_aux_dev, when not nullptr, instead of grad_aux).
+int backward_into(const void* x, const void* Wg, const void* plan, const void* grad_out, float grad_aux,
+                  const float* grad_aux_dev, int64_t N, int d, int f, int E, int k, int dtype, float dropout_p,
+                  uint64_t seed, void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes,
+                  const TrainGrads& grads, void* stream);
+// moe_b200_experts_backward likewise (grads.wg and grads.bg are not used).
+int experts_backward_into(const void* x_sorted, const void* h, const int32_t* offsets, const void* plan,
+                          const void* grad_y, int64_t M, int d, int f, int E, float dropout_p, uint64_t seed,
+                          void* train_ws, size_t train_ws_bytes, const TrainGrads& grads, int32_t* status,
+                          void* stream);
+
 }  // namespace moe

@@ -120,6 +120,19 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
   return desc;
 }
 
+// The same for an MN-major tile (the contraction index runs down the rows): boxes of 64 elements
+// (128 bytes) x 64 rows, neighbouring boxes along M or N 8192 bytes apart (LBO), 8-row groups
+// 1024 bytes apart (SBO).
+__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t saddr) {
+  uint64_t desc = 0;
+  desc |= (uint64_t)((saddr & 0x3ffffu) >> 4);
+  desc |= (uint64_t)(8192 >> 4) << 16;
+  desc |= (uint64_t)(1024 >> 4) << 32;
+  desc |= (uint64_t)1 << 46;
+  desc |= (uint64_t)2 << 61;
+  return desc;
+}
+
 // Instruction descriptor: fp32 accumulate (bit 4), bf16 x bf16 (bits 7, 10), both
 // operands K-major, N/8 at bit 17, M/16 at bit 24 (M = 128).
 __host__ __device__ constexpr uint32_t make_idesc(int n) {

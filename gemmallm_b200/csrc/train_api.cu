@@ -2,9 +2,8 @@
 // dropout on h and the tensors the backward pass needs (reference model.py:164,183 under
 // .train()), and the backward pass itself (what torch.autograd derives for model.py:200-276
 // and 173-190 when the reference trains, train.py:140-141).
-#include <cuda.h>
-#include <string.h>
 #include "common.cuh"
+#include "internal.h"
 
 namespace moe {
 namespace {
@@ -21,25 +20,13 @@ int train_check(int64_t N, int d, int f, int E, int k, int dtype, float p) {
   return 0;
 }
 
-int64_t padded_rows(int64_t M, int E) { return ((M + 63) & ~(int64_t)63) + (int64_t)64 * E; }
-
 void tws_layout(int64_t N, int d, int f, int E, int k, size_t* off, size_t* total) {
   const size_t M = (size_t)N * k;
-  const size_t Kp = (size_t)padded_rows((int64_t)M, E);
-  size_t sizes[MOE_B200_TWS_NUM];
+  size_t sizes[MOE_B200_TWS_NUM] = {};
   sizes[MOE_B200_TWS_GU] = M * 2 * f * 2;
   sizes[MOE_B200_TWS_PAIR_OF] = M * sizeof(int32_t);
-  sizes[MOE_B200_TWS_KOFF] = (size_t)(E + 1) * sizeof(int32_t);
   sizes[MOE_B200_TWS_DY] = M * d * 2;
-  sizes[MOE_B200_TWS_DH] = M * f * 2;
   sizes[MOE_B200_TWS_DXS] = M * d * 2;
-  sizes[MOE_B200_TWS_W1T] = (size_t)E * d * 2 * f * 2;
-  sizes[MOE_B200_TWS_W2T] = (size_t)E * f * d * 2;
-  sizes[MOE_B200_TWS_TMAPS] = (size_t)2 * E * 128;
-  sizes[MOE_B200_TWS_XT] = (size_t)d * Kp * 2;
-  sizes[MOE_B200_TWS_HT] = (size_t)f * Kp * 2;
-  sizes[MOE_B200_TWS_DYT] = (size_t)d * Kp * 2;
-  sizes[MOE_B200_TWS_DGUT] = (size_t)2 * f * Kp * 2;
   sizes[MOE_B200_TWS_DL] = (size_t)N * E * sizeof(float);
   sizes[MOE_B200_TWS_DW] = M * sizeof(float);
   sizes[MOE_B200_TWS_ONES] = M * sizeof(float);
@@ -51,6 +38,11 @@ void tws_layout(int64_t N, int d, int f, int E, int k, size_t* off, size_t* tota
   sizes[MOE_B200_TWS_G_B1] = (size_t)E * 2 * f * 2;
   sizes[MOE_B200_TWS_G_W2] = (size_t)E * d * f * 2;
   sizes[MOE_B200_TWS_G_B2] = (size_t)E * d * 2;
+  sizes[MOE_B200_TWS_MASK] = M * (f / 8);
+  // one row per 128-row half of a 256-row tile for dg and du; the sums of dy take less
+  const size_t tiles = (M + 255) / 256 + E;
+  const size_t cols = (size_t)4 * f > (size_t)d ? (size_t)4 * f : (size_t)d;
+  sizes[MOE_B200_TWS_COL_PART] = tiles * cols * sizeof(float);
   size_t pos = 0;
   for (int i = 0; i < MOE_B200_TWS_NUM; ++i) {
     off[i] = pos;
@@ -62,6 +54,8 @@ void tws_layout(int64_t N, int d, int f, int E, int k, size_t* off, size_t* tota
 TrainArgs train_args(char* tws, const size_t* to, float p, uint64_t seed) {
   TrainArgs tr;
   tr.gu = reinterpret_cast<__nv_bfloat16*>(tws + to[MOE_B200_TWS_GU]);
+  tr.mask = reinterpret_cast<uint8_t*>(tws + to[MOE_B200_TWS_MASK]);
+  tr.col_part = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_COL_PART]);
   tr.pair_of = reinterpret_cast<const int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]);
   const double t = (double)p * 4294967296.0;
   tr.thresh = p <= 0.f ? 0u : (uint32_t)(t >= 4294967295.0 ? 4294967295.0 : t);
@@ -71,55 +65,44 @@ TrainArgs train_args(char* tws, const size_t* to, float p, uint64_t seed) {
   return tr;
 }
 
-// Backward of the grouped expert feed-forward (model.py:174-184) on sorted rows: given dy (gradient
-// of y, in the training workspace), h (the dropped h of the forward), the saved pre-activations and
-// the sorted inputs, writes dxs (gradient of the sorted inputs) and the four parameter gradients.
-int experts_backward(const void* perm, const void* h, const int32_t* offsets, const void* plan,
-                     int64_t M, int d, int f, int E, const TrainArgs& tr, char* tws, const size_t* to,
-                     int32_t* status, cudaStream_t s) {
-  const int64_t Kp = padded_rows(M, E);
+// Backward of the grouped expert feed-forward (model.py:174-184) on sorted rows: given dy (gradient of y),
+// h (the dropped h of the forward), the saved pre-activations and the sorted inputs, writes g.x (gradient of the
+// sorted inputs) and the four parameter gradients.
+int experts_backward(const void* perm, const void* h, const int32_t* offsets, const void* plan, const void* dy,
+                     int64_t M, int d, int f, int E, const TrainArgs& tr, const TrainGrads& g, int32_t* status,
+                     cudaStream_t s) {
   const PlanView pv = plan_view(plan, E);
-  int32_t* koff = reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_KOFF]);
-  void* gu = tws + to[MOE_B200_TWS_GU];
-  void* dy = tws + to[MOE_B200_TWS_DY];
-  void* dh = tws + to[MOE_B200_TWS_DH];
-  void* dxs = tws + to[MOE_B200_TWS_DXS];
-  const char* tmaps = tws + to[MOE_B200_TWS_TMAPS];
-  // experts without rows get no tile in the weight-gradient products
-  MOE_CUDA_CHECK(cudaMemsetAsync(tws + to[MOE_B200_TWS_G_W1], 0, (size_t)E * 2 * f * d * 2, s));
-  MOE_CUDA_CHECK(cudaMemsetAsync(tws + to[MOE_B200_TWS_G_W2], 0, (size_t)E * d * f * 2, s));
-  int rc = launch_pad_offsets(offsets, E, koff, s);
+  int rc;
+  // down Linear (model.py:184): db2 = column sums of dy, dW2 = dy^T h, dh = dy W2; the last one goes back
+  // through dropout, product and GELU (model.py:180-183) in its epilogue: (g, u) -> (dg, du) in place
+  if (g.b2 != nullptr) {
+    rc = launch_colsum(dy, offsets, M, E, d, tr.col_part, g.b2, s);
+    if (rc) return rc;
+  }
+  if (g.w2 != nullptr) {
+    rc = launch_grouped_wgrad(dy, h, M, d, f, offsets, g.w2, E, status, s);
+    if (rc) return rc;
+  }
+  if (g.x == nullptr && g.w1 == nullptr && g.b1 == nullptr) return 0;
+  rc = launch_grouped_dx(dy, M, d, pv.tmap_W2_dec, offsets, E, f, nullptr, &tr, status, s);
   if (rc) return rc;
-  // down Linear (model.py:184): dh = dy W2, dW2 = dy^T h, db2 = column sums of dy
-  rc = launch_transpose_weights(pv.W2, E, d, f, tws + to[MOE_B200_TWS_W2T], s);
-  if (rc) return rc;
-  rc = launch_grouped_rows(dy, M, d, tmaps + (size_t)128 * E, offsets, nullptr, E, f, dh, status, s);
-  if (rc) return rc;
-  rc = launch_transpose_pad(dy, offsets, koff, E, d, Kp, tws + to[MOE_B200_TWS_DYT], s);
-  if (rc) return rc;
-  rc = launch_transpose_pad(h, offsets, koff, E, f, Kp, tws + to[MOE_B200_TWS_HT], s);
-  if (rc) return rc;
-  rc = launch_grouped_cols(tws + to[MOE_B200_TWS_DYT], tws + to[MOE_B200_TWS_HT], Kp, d, f, koff,
-                           tws + to[MOE_B200_TWS_G_W2], E, status, s);
-  if (rc) return rc;
-  rc = launch_colsum(dy, offsets, E, d, tws + to[MOE_B200_TWS_G_B2], s);
-  if (rc) return rc;
-  // dropout, product and GELU (model.py:180-183): (g, u) -> (dg, du) in place
-  rc = launch_geglu_bwd(dh, gu, tr.pair_of, M, f, tr.thresh, tr.scale, tr.seed_lo, tr.seed_hi, s);
-  if (rc) return rc;
-  // gate_and_up Linear (model.py:174): dx = dgu W1, dW1 = dgu^T x, db1 = column sums of dgu
-  rc = launch_transpose_weights(pv.W1, E, 2 * f, d, tws + to[MOE_B200_TWS_W1T], s);
-  if (rc) return rc;
-  rc = launch_grouped_rows(gu, M, 2 * f, tmaps, offsets, nullptr, E, d, dxs, status, s);
-  if (rc) return rc;
-  rc = launch_transpose_pad(gu, offsets, koff, E, 2 * f, Kp, tws + to[MOE_B200_TWS_DGUT], s);
-  if (rc) return rc;
-  rc = launch_transpose_pad(perm, offsets, koff, E, d, Kp, tws + to[MOE_B200_TWS_XT], s);
-  if (rc) return rc;
-  rc = launch_grouped_cols(tws + to[MOE_B200_TWS_DGUT], tws + to[MOE_B200_TWS_XT], Kp, 2 * f, d, koff,
-                           tws + to[MOE_B200_TWS_G_W1], E, status, s);
-  if (rc) return rc;
-  return launch_colsum(gu, offsets, E, 2 * f, tws + to[MOE_B200_TWS_G_B1], s);
+  // gate_and_up Linear (model.py:174): db1 = column sums of dgu, dx = dgu W1, dW1 = dgu^T x
+  if (g.b1 != nullptr) {
+    rc = launch_colsum_finish(tr.col_part, 2, offsets, E, 2 * f, g.b1, s);
+    if (rc) return rc;
+  }
+  if (g.x != nullptr) {
+    rc = launch_grouped_dx(tr.gu, M, 2 * f, pv.tmap_W1_dec, offsets, E, d, g.x, nullptr, status, s);
+    if (rc) return rc;
+  }
+  if (g.w1 == nullptr) return 0;
+  return launch_grouped_wgrad(tr.gu, perm, M, 2 * f, d, offsets, g.w1, E, status, s);
+}
+
+// the gradient regions of the training workspace
+TrainGrads own_grads(char* tws, const size_t* to, void* grad_x) {
+  return TrainGrads{grad_x, tws + to[MOE_B200_TWS_G_WG], tws + to[MOE_B200_TWS_G_BG], tws + to[MOE_B200_TWS_G_W1],
+                    tws + to[MOE_B200_TWS_G_B1], tws + to[MOE_B200_TWS_G_W2], tws + to[MOE_B200_TWS_G_B2]};
 }
 
 }  // namespace
@@ -155,32 +138,78 @@ int moe_b200_train_setup(int64_t N, int d, int f, int E, int k, int dtype, void*
   if (train_ws_bytes < total) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
   if ((uintptr_t)train_ws & 1023) return set_error(MOE_B200_ERR_ALIGN, "training workspace must be 1024-byte aligned");
   char* tws = static_cast<char*>(train_ws);
-  cudaStream_t s = (cudaStream_t)stream;
-  // tensor maps of the transposed weight buffers (their addresses never change)
-  const size_t nmaps = (size_t)2 * E;
-  unsigned char* maps = static_cast<unsigned char*>(aligned_alloc(128, nmaps * 128));
-  if (!maps) return set_error(MOE_B200_ERR_WORKSPACE, "out of host memory");
-  for (int e = 0; e < E && rc == 0; ++e) {
-    rc = encode_tmap_2d(maps + 128 * (size_t)e, tws + to[MOE_B200_TWS_W1T] + (size_t)e * d * 2 * f * 2,
-                        (uint64_t)d, (uint64_t)2 * f, 128);
-    if (rc == 0)
-      rc = encode_tmap_2d(maps + 128 * (size_t)(E + e), tws + to[MOE_B200_TWS_W2T] + (size_t)e * f * d * 2,
-                          (uint64_t)f, (uint64_t)d, 128);
-  }
-  if (rc == 0) {
-    cudaError_t ce = cudaMemcpyAsync(tws + to[MOE_B200_TWS_TMAPS], maps, nmaps * 128, cudaMemcpyHostToDevice, s);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
-    if (ce != cudaSuccess) rc = cuda_error(ce, "upload of the tensor maps");
-  }
-  free(maps);
-  if (rc) return rc;
-  return launch_fill_f32(reinterpret_cast<float*>(tws + to[MOE_B200_TWS_ONES]), N * (int64_t)k, 1.0f, s);
+  return launch_fill_f32(reinterpret_cast<float*>(tws + to[MOE_B200_TWS_ONES]), N * (int64_t)k, 1.0f, (cudaStream_t)stream);
 }
 
 int moe_b200_forward_train(const void* x, const void* Wg, const void* bg, const void* plan,
                            const void* residual, int64_t N, int d, int f, int E, int k, int dtype,
                            float dropout_p, uint64_t seed, void* workspace, size_t workspace_bytes,
                            void* train_ws, size_t train_ws_bytes, void* out, void* stream) {
+  return forward_train_into(x, Wg, bg, plan, residual, N, d, f, E, k, dtype, dropout_p, seed, workspace,
+                            workspace_bytes, train_ws, train_ws_bytes, out, nullptr, stream);
+}
+
+int moe_b200_backward(const void* x, const void* Wg, const void* plan, const void* grad_out,
+                      float grad_aux, int64_t N, int d, int f, int E, int k, int dtype,
+                      float dropout_p, uint64_t seed, void* workspace, size_t workspace_bytes,
+                      void* train_ws, size_t train_ws_bytes, void* grad_x, void* stream) {
+  int rc = train_check(N, d, f, E, k, dtype, dropout_p);
+  if (rc) return rc;
+  if (!train_ws) return set_error(MOE_B200_ERR_NULL, "workspace is NULL");
+  if (N > 0 && !grad_x) return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  size_t to[MOE_B200_TWS_NUM], ttotal;
+  tws_layout(N, d, f, E, k, to, &ttotal);
+  return backward_into(x, Wg, plan, grad_out, grad_aux, nullptr, N, d, f, E, k, dtype, dropout_p, seed, workspace,
+                       workspace_bytes, train_ws, train_ws_bytes,
+                       own_grads(static_cast<char*>(train_ws), to, grad_x), stream);
+}
+
+// ---- the expert feed-forward alone (the reference's dense FeedForward, model.py:154-190, is one
+// group; any grouping by offsets works) ----
+
+int moe_b200_experts_train(const void* x_sorted, const int32_t* offsets, const void* plan, int64_t M,
+                           int d, int f, int E, float dropout_p, uint64_t seed, void* train_ws,
+                           size_t train_ws_bytes, void* h, void* y, int32_t* status, void* stream) {
+  int rc = train_check(M, d, f, E, 1, MOE_B200_BF16, dropout_p);
+  if (rc) return rc;
+  if (M == 0) return 0;
+  if (!x_sorted || !offsets || !plan || !train_ws || !h || !y || !status)
+    return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  size_t to[MOE_B200_TWS_NUM], ttotal;
+  tws_layout(M, d, f, E, 1, to, &ttotal);
+  if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
+  if ((uintptr_t)train_ws & 1023) return set_error(MOE_B200_ERR_ALIGN, "training workspace must be 1024-byte aligned");
+  char* tws = static_cast<char*>(train_ws);
+  cudaStream_t s = (cudaStream_t)stream;
+  // row r is pair r: the dropout mask of element (r, c) depends on the row's position only
+  rc = launch_iota(reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]), M, s);
+  if (rc) return rc;
+  const TrainArgs tr = train_args(tws, to, dropout_p, seed);
+  return launch_experts_tc2(x_sorted, offsets, plan, M, d, f, E, h, y, nullptr, status, s, &tr);
+}
+
+int moe_b200_experts_backward(const void* x_sorted, const void* h, const int32_t* offsets,
+                              const void* plan, const void* grad_y, int64_t M, int d, int f, int E,
+                              float dropout_p, uint64_t seed, void* train_ws, size_t train_ws_bytes,
+                              void* grad_x, int32_t* status, void* stream) {
+  int rc = train_check(M, d, f, E, 1, MOE_B200_BF16, dropout_p);
+  if (rc) return rc;
+  if (M == 0) return 0;
+  if (!train_ws || !grad_x) return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  size_t to[MOE_B200_TWS_NUM], ttotal;
+  tws_layout(M, d, f, E, 1, to, &ttotal);
+  return experts_backward_into(x_sorted, h, offsets, plan, grad_y, M, d, f, E, dropout_p, seed, train_ws,
+                               train_ws_bytes, own_grads(static_cast<char*>(train_ws), to, grad_x), status, stream);
+}
+
+}  // extern "C"
+
+namespace moe {
+
+int forward_train_into(const void* x, const void* Wg, const void* bg, const void* plan, const void* residual,
+                       int64_t N, int d, int f, int E, int k, int dtype, float dropout_p, uint64_t seed,
+                       void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes, void* out,
+                       float* aux, void* stream) {
   int rc = train_check(N, d, f, E, k, dtype, dropout_p);
   if (rc) return rc;
   if (!workspace || !train_ws) return set_error(MOE_B200_ERR_NULL, "workspace is NULL");
@@ -216,7 +245,8 @@ int moe_b200_forward_train(const void* x, const void* Wg, const void* bg, const 
   rc = moe_b200_dispatch(x, idx, N, d, E, k, dtype, reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_SCRATCH]),
                          reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_CNT_SLOT]), offsets, row_of, perm,
                          psum_part, reinterpret_cast<float*>(ws + off[MOE_B200_WS_PSUM]),
-                         reinterpret_cast<float*>(ws + off[MOE_B200_WS_AUX]), status, stream);
+                         aux != nullptr ? aux : reinterpret_cast<float*>(ws + off[MOE_B200_WS_AUX]), status,
+                         stream);
   if (rc) return rc;
   rc = launch_pair_of(row_of, M, reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]), s);
   if (rc) return rc;
@@ -226,10 +256,10 @@ int moe_b200_forward_train(const void* x, const void* Wg, const void* bg, const 
   return moe_b200_combine(y, row_of, w, residual, N, d, k, dtype, out, stream);
 }
 
-int moe_b200_backward(const void* x, const void* Wg, const void* plan, const void* grad_out,
-                      float grad_aux, int64_t N, int d, int f, int E, int k, int dtype,
-                      float dropout_p, uint64_t seed, void* workspace, size_t workspace_bytes,
-                      void* train_ws, size_t train_ws_bytes, void* grad_x, void* stream) {
+int backward_into(const void* x, const void* Wg, const void* plan, const void* grad_out, float grad_aux,
+                  const float* grad_aux_dev, int64_t N, int d, int f, int E, int k, int dtype, float dropout_p,
+                  uint64_t seed, void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes,
+                  const TrainGrads& grads, void* stream) {
   int rc = train_check(N, d, f, E, k, dtype, dropout_p);
   if (rc) return rc;
   if (!workspace || !train_ws) return set_error(MOE_B200_ERR_NULL, "workspace is NULL");
@@ -241,14 +271,13 @@ int moe_b200_backward(const void* x, const void* Wg, const void* plan, const voi
   tws_layout(N, d, f, E, k, to, &ttotal);
   if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
   if (N == 0) return 0;
-  if (!x || !Wg || !plan || !grad_out || !grad_x) return set_error(MOE_B200_ERR_NULL, "NULL argument");
-  if (!aligned16(grad_out) || !aligned16(grad_x) || !aligned16(x))
+  if (!x || !Wg || !plan || !grad_out) return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  if (!aligned16(grad_out) || !aligned16(grads.x) || !aligned16(x))
     return set_error(MOE_B200_ERR_ALIGN, "buffers must be 16-byte aligned");
   char* ws = static_cast<char*>(workspace);
   char* tws = static_cast<char*>(train_ws);
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t M = N * k;
-  const int64_t Kp = padded_rows(M, E);
   int32_t* status = reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_STATUS]);
   const float* logits = reinterpret_cast<const float*>(ws + off[MOE_B200_WS_LOGITS]);
   const int32_t* idx = reinterpret_cast<const int32_t*>(ws + off[MOE_B200_WS_IDX]);
@@ -259,81 +288,48 @@ int moe_b200_backward(const void* x, const void* Wg, const void* plan, const voi
   const void* perm = ws + off[MOE_B200_WS_PERM];
   const void* h = ws + off[MOE_B200_WS_H];
   const void* y = ws + off[MOE_B200_WS_Y];
-  const int32_t* pair_of = reinterpret_cast<const int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]);
-  int32_t* koff = reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_KOFF]);
-  void* gu = tws + to[MOE_B200_TWS_GU];
   void* dy = tws + to[MOE_B200_TWS_DY];
-  void* dh = tws + to[MOE_B200_TWS_DH];
   void* dxs = tws + to[MOE_B200_TWS_DXS];
-  void* w1t = tws + to[MOE_B200_TWS_W1T];
-  void* w2t = tws + to[MOE_B200_TWS_W2T];
-  const char* tmaps = tws + to[MOE_B200_TWS_TMAPS];
   float* dl = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DL]);
   float* dw = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DW]);
   const float* ones = reinterpret_cast<const float*>(tws + to[MOE_B200_TWS_ONES]);
   float* dwg32 = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DWG_F32]);
   void* dxr = tws + to[MOE_B200_TWS_DXR];
-  const PlanView pv = plan_view(plan, E);
   const TrainArgs tr = train_args(tws, to, dropout_p, seed);
 
   // combine (model.py:271) and router (model.py:206-223)
-  rc = launch_combine_bwd(grad_out, y, pair_of, w, M, d, k, dy, dw, s);
+  rc = launch_combine_bwd(grad_out, y, tr.pair_of, w, M, d, k, dy, dw, s);
   if (rc) return rc;
-  rc = launch_router_bwd(logits, idx, w, dw, cnt_slot, grad_aux, x, Wg, N, d, E, k, dl, dwg32,
-                         dwg32 + (size_t)E * d, tws + to[MOE_B200_TWS_G_WG], tws + to[MOE_B200_TWS_G_BG],
-                         dxr, s);
-  if (rc) return rc;
+  if (grads.x != nullptr || grads.wg != nullptr || grads.bg != nullptr) {
+    rc = launch_router_bwd(logits, idx, w, dw, cnt_slot, grad_aux, grad_aux_dev, x, Wg, N, d, E, k, dl, dwg32,
+                           dwg32 + (size_t)E * d, grads.wg, grads.bg, dxr, s);
+    if (rc) return rc;
+  }
   // the experts (model.py:174-184)
-  rc = experts_backward(perm, h, offsets, plan, M, d, f, E, tr, tws, to, status, s);
-  if (rc) return rc;
+  TrainGrads eg = grads;
+  eg.x = grads.x != nullptr ? dxs : nullptr;
+  rc = experts_backward(perm, h, offsets, plan, dy, M, d, f, E, tr, eg, status, s);
+  if (rc || grads.x == nullptr) return rc;
   // gather (model.py:248-253) and the router's share: dx[t] = sum_j dxs[row_of[t,j]] + dxr[t]
-  return launch_combine(dxs, row_of, ones, dxr, N, d, k, dtype, grad_x, s);
+  return launch_combine(dxs, row_of, ones, dxr, N, d, k, dtype, grads.x, s);
 }
 
-// ---- the expert feed-forward alone (the reference's dense FeedForward, model.py:154-190, is one
-// group; any grouping by offsets works) ----
-
-int moe_b200_experts_train(const void* x_sorted, const int32_t* offsets, const void* plan, int64_t M,
-                           int d, int f, int E, float dropout_p, uint64_t seed, void* train_ws,
-                           size_t train_ws_bytes, void* h, void* y, int32_t* status, void* stream) {
+int experts_backward_into(const void* x_sorted, const void* h, const int32_t* offsets, const void* plan,
+                          const void* grad_y, int64_t M, int d, int f, int E, float dropout_p, uint64_t seed,
+                          void* train_ws, size_t train_ws_bytes, const TrainGrads& grads, int32_t* status,
+                          void* stream) {
   int rc = train_check(M, d, f, E, 1, MOE_B200_BF16, dropout_p);
   if (rc) return rc;
   if (M == 0) return 0;
-  if (!x_sorted || !offsets || !plan || !train_ws || !h || !y || !status)
+  if (!x_sorted || !h || !offsets || !plan || !grad_y || !train_ws || !status)
     return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  if (!aligned16(x_sorted) || !aligned16(h) || !aligned16(grad_y) || !aligned16(grads.x))
+    return set_error(MOE_B200_ERR_ALIGN, "buffers must be 16-byte aligned");
   size_t to[MOE_B200_TWS_NUM], ttotal;
   tws_layout(M, d, f, E, 1, to, &ttotal);
   if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
-  if ((uintptr_t)train_ws & 1023) return set_error(MOE_B200_ERR_ALIGN, "training workspace must be 1024-byte aligned");
-  char* tws = static_cast<char*>(train_ws);
-  cudaStream_t s = (cudaStream_t)stream;
-  // row r is pair r: the dropout mask of element (r, c) depends on the row's position only
-  rc = launch_iota(reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]), M, s);
-  if (rc) return rc;
-  const TrainArgs tr = train_args(tws, to, dropout_p, seed);
-  return launch_experts_tc2(x_sorted, offsets, plan, M, d, f, E, h, y, nullptr, status, s, &tr);
+  const TrainArgs tr = train_args(static_cast<char*>(train_ws), to, dropout_p, seed);
+  return experts_backward(x_sorted, h, offsets, plan, grad_y, M, d, f, E, tr, grads, status, (cudaStream_t)stream);
 }
 
-int moe_b200_experts_backward(const void* x_sorted, const void* h, const int32_t* offsets,
-                              const void* plan, const void* grad_y, int64_t M, int d, int f, int E,
-                              float dropout_p, uint64_t seed, void* train_ws, size_t train_ws_bytes,
-                              void* grad_x, int32_t* status, void* stream) {
-  int rc = train_check(M, d, f, E, 1, MOE_B200_BF16, dropout_p);
-  if (rc) return rc;
-  if (M == 0) return 0;
-  if (!x_sorted || !h || !offsets || !plan || !grad_y || !train_ws || !grad_x || !status)
-    return set_error(MOE_B200_ERR_NULL, "NULL argument");
-  size_t to[MOE_B200_TWS_NUM], ttotal;
-  tws_layout(M, d, f, E, 1, to, &ttotal);
-  if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
-  char* tws = static_cast<char*>(train_ws);
-  cudaStream_t s = (cudaStream_t)stream;
-  const TrainArgs tr = train_args(tws, to, dropout_p, seed);
-  MOE_CUDA_CHECK(cudaMemcpyAsync(tws + to[MOE_B200_TWS_DY], grad_y, (size_t)M * d * 2, cudaMemcpyDeviceToDevice, s));
-  rc = experts_backward(x_sorted, h, offsets, plan, M, d, f, E, tr, tws, to, status, s);
-  if (rc) return rc;
-  MOE_CUDA_CHECK(cudaMemcpyAsync(grad_x, tws + to[MOE_B200_TWS_DXS], (size_t)M * d * 2, cudaMemcpyDeviceToDevice, s));
-  return 0;
-}
-
-}  // extern "C"
+}  // namespace moe

@@ -411,15 +411,15 @@ int moe_b200_attention(const void* qkv, const void* gate, const float* pos_emb, 
  * that forward and its backward pass for bf16. Both work on the block's ordinary
  * workspace (which the forward fills and the backward reads: call the backward before
  * the next forward on the same workspace) plus a training workspace for the saved
- * pre-activations, the transposed operands and the parameter gradients. */
+ * pre-activations, the dropout mask and the parameter gradients. */
 enum {
   MOE_B200_TWS_GU = 0,   /* bf16 [N*k, 2f] gate/up pre-activations; (dg, du) after the backward */
   MOE_B200_TWS_PAIR_OF,  /* int32 [N*k]    token * k + slot of every sorted row */
-  MOE_B200_TWS_KOFF,     /* int32 [E+1]    expert starts, each padded to a multiple of 64 */
+  MOE_B200_TWS_KOFF,     /* empty, as DH, W1T .. DGUT below: the products read their operands as
+                          * they lie in memory and dh never leaves the chip */
   MOE_B200_TWS_DY, MOE_B200_TWS_DH, MOE_B200_TWS_DXS,   /* gradients of y, h, sorted x */
-  MOE_B200_TWS_W1T, MOE_B200_TWS_W2T,                   /* transposed weights [E][d][2f], [E][f][d] */
-  MOE_B200_TWS_TMAPS,    /* tensor maps of W1T[e], W2T[e] (moe_b200_train_setup) */
-  MOE_B200_TWS_XT, MOE_B200_TWS_HT, MOE_B200_TWS_DYT, MOE_B200_TWS_DGUT, /* [cols][padded rows] */
+  MOE_B200_TWS_W1T, MOE_B200_TWS_W2T, MOE_B200_TWS_TMAPS,
+  MOE_B200_TWS_XT, MOE_B200_TWS_HT, MOE_B200_TWS_DYT, MOE_B200_TWS_DGUT,
   MOE_B200_TWS_DL,       /* float [N,E]   gradient of the router logits */
   MOE_B200_TWS_DW,       /* float [N,k]   gradient of the renormalised scores */
   MOE_B200_TWS_ONES,     /* float [N,k]   ones (moe_b200_train_setup) */
@@ -432,13 +432,14 @@ enum {
   MOE_B200_TWS_G_B1,     /* [E,2f]     experts.e.gate_and_up.bias */
   MOE_B200_TWS_G_W2,     /* [E,d,f]    experts.e.down.weight */
   MOE_B200_TWS_G_B2,     /* [E,d]      experts.e.down.bias */
+  MOE_B200_TWS_MASK,     /* uint8 [N*k, f/8] dropout mask of h, one bit per element */
+  MOE_B200_TWS_COL_PART, /* float      partial column sums of the bias gradients */
   MOE_B200_TWS_NUM
 };
 size_t moe_b200_train_workspace_bytes(int64_t N, int d, int f, int E, int k, int dtype);
 int moe_b200_train_workspace_layout(int64_t N, int d, int f, int E, int k, int dtype,
                                     size_t* h_offsets);
-/* Once per training workspace (synchronous): tensor maps of its transposed-weight
- * buffers, constants. */
+/* Once per training workspace: constants. */
 int moe_b200_train_setup(int64_t N, int d, int f, int E, int k, int dtype, void* train_ws,
                          size_t train_ws_bytes, void* stream);
 

@@ -260,3 +260,48 @@ def test_dense_feedforward_fine_tuning_trains_the_lora_tensors(cuda_device):
     for name, short in LORA_NAMES:
         close(getattr(ff, name).weight.grad, lora[short + "_w"].grad, 4e-2, f"grad {name}.weight")
         close(getattr(ff, name).bias.grad, lora[short + "_b"].grad, 4e-2, f"grad {name}.bias")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 63, 64, 65, 129, 255, 257])
+def test_weight_gradients_at_the_edges_of_a_block_of_rows(cuda_device, rows):
+    """The weight-gradient product contracts over the rows in blocks of 64 (sixteen at a time) and cuts the last
+    block; the input-gradient product works on 256-row tiles: gradients around those sizes, d and f that are no
+    multiples of 64. bf16 products of bf16 operands with fp32 sums: relative 3e-2 as in the tests above."""
+    from gemmallm_b200 import FeedForward
+    d, f = 72, 136
+    g = torch.Generator().manual_seed(rows)
+    ff = FeedForward(d, dropout_ratio=0.25, d_ff=f).to(device=cuda_device, dtype=DT).train()
+    with torch.no_grad():
+        for prm in ff.parameters():
+            prm.copy_(synthetic.round_to(torch.randn(prm.shape, generator=g) * 0.1, DT))
+    x = synthetic.round_to(torch.randn(rows, d, generator=g), DT)
+    grad_y = synthetic.round_to(torch.randn(rows, d, generator=g), DT)
+    xd = x.to(DT).to(cuda_device).requires_grad_(True)
+    (ff(xd).float() * grad_y.to(cuda_device)).sum().backward()
+    torch.cuda.synchronize()
+    mult = torch.from_numpy(philox_ref.dropout_multiplier(rows, f, 0.25, ff.last_seed))
+    params = (ff.gate_and_up.weight, ff.gate_and_up.bias, ff.down.weight, ff.down.bias)
+    leaves = [t.clone().requires_grad_(True) for t in (x, *(p.detach().float().cpu() for p in params))]
+    (moe_oracle.expert_ffn(*leaves, h_mask=mult) * grad_y).sum().backward()
+    for got, ref, what in zip((xd, *params), leaves, ("x", "w1", "b1", "w2", "b2")):
+        close(got.grad, ref.grad, 3e-2, f"grad {what}")
+
+
+@pytest.mark.gpu
+def test_experts_without_tokens_get_zero_gradients(cuda_device):
+    d, E, f, k = 64, 8, 128, 2
+    m, _ = make_block(d, E, f, k, 0.1, cuda_device, seed=9)
+    with torch.no_grad():
+        m.gate.bias[3:] = -100.0
+    m.train()
+    x = torch.randn(1, 40, d, generator=torch.Generator().manual_seed(1)).to(DT).to(cuda_device)
+    for _ in range(2):
+        m.zero_grad(set_to_none=True)
+        m(x)[0].float().square().sum().backward()
+    torch.cuda.synchronize()
+    assert m.device_status() == 0 and m.last["cnt_slot"].sum(0)[3:].eq(0).all()
+    for e, ex in enumerate(m.experts):
+        for p in (ex.gate_and_up.weight, ex.gate_and_up.bias, ex.down.weight, ex.down.bias):
+            assert torch.isfinite(p.grad).all()
+            assert bool((p.grad != 0).any()) == (e < 3 and bool(m.last["cnt_slot"].sum(0)[e] > 0))
