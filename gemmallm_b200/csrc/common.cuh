@@ -310,7 +310,8 @@ int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
                        cudaStream_t s, int* xch = nullptr, int* counter = nullptr,
                        int32_t* status = nullptr);
-int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
+                   uint32_t box_cols = 64);
 int sm_count(int* sms);
 int decode_splits(int f);
 int decode_spec_rows(int64_t N);

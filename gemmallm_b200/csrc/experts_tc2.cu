@@ -68,14 +68,21 @@ struct Traits {
   static constexpr bool COLS = KIND == kWgrad;
   static constexpr bool A_MN = COLS;
   static constexpr bool B_MN = KIND == kDx || KIND == kDhGeglu || COLS;
-  // The training epilogues do 20 to 40 instructions per accumulator element (Philox, GELU and its
-  // derivative): eight warps cannot issue them in the time of a tile's products, sixteen can.
+  // The training epilogues do 10 to 20 instructions per accumulator element and move as much again as the
+  // products' operands: sixteen warps, and further ones for what does not need the accumulator.
   static constexpr int kEpiWarps = KIND == kGegluTrain || KIND == kDhGeglu ? 16 : 8;
-  static constexpr int kThreads = 64 + 32 * kEpiWarps + (COLS ? 32 : 0);
-  static constexpr int kStgWarp = KIND == kGegluTrain ? kStg32Bytes : kStgBytes;
-  static constexpr int kStages = KIND == kDhGeglu ? 5 : 6;   // its staging areas take a stage's room
-  static constexpr int kColBytes = KIND == kDhGeglu ? 4 * 2 * BN * 4 : 0;   // column sums, four lane quadrants
+  static constexpr int kHelpers = KIND == kGegluTrain ? 4 : (KIND == kDhGeglu || COLS ? 1 : 0);
+  static constexpr int kThreads = 64 + 32 * (kEpiWarps + kHelpers);
+  // (kGegluTrain at 16384 tokens, d 1024, f 4096: 149 / 126 / 116 us above the inference pass with 3 / 4 / 5
+  // stages, so one box per epilogue warp and a fifth stage instead of two boxes)
+  static constexpr int kStages = KIND == kGegluTrain ? 5 : (KIND == kDhGeglu ? 4 : 6);
+  // room behind the stages (boxes want 1 KiB alignment): a box for each epilogue warp, or two chunks of gate and up
+  static constexpr int kBoxes = KIND == kGegluTrain ? 16 * kBoxBytes : (KIND == kDhGeglu ? 2 * 2 * GegluBwd::kBoxBytes : 0);
+  // and behind Control: staging of the epilogue warps; biases and mask bits; column sums of the lane quadrants
+  static constexpr int kExtra =
+      KIND == kGegluTrain ? 16 * 256 + 2 * BM * 16 : (KIND == kDhGeglu ? 4 * 2 * BN * 4 : 8 * kStgBytes);
 };
+
 // M = 256 across the pair: M/16 at bit 24
 constexpr uint32_t kIdesc2 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                              ((256u >> 4) << 24);
@@ -85,6 +92,8 @@ struct Control {
   uint64_t empty[kMaxStages];
   uint64_t tail[kMaxStages];   // COLS: this CTA's half of a block that has to be cut has arrived
   uint64_t peer_cut[kMaxStages];   // COLS, even CTA: the odd CTA's half has been cut
+  uint64_t aux_full[2];    // kGegluTrain: mask bits of a tile drawn; kDhGeglu: a chunk of gate and up values there
+  uint64_t aux_empty[2];   // kGegluTrain: they have been read; kDhGeglu: replaced by their gradients
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
@@ -93,12 +102,12 @@ struct Control {
   int offsets[kMaxExperts + 1];
 };
 
-// [stages][Control][staging area of every epilogue warp][column sums]
+// [stages][boxes][Control][extra]
 constexpr size_t kControlBytes = (sizeof(Control) + 15) & ~(size_t)15;
 template <int KIND>
 constexpr size_t smem_bytes() {
   using T = Traits<KIND>;
-  return 1024 + (size_t)T::kStages * kStageBytes + kControlBytes + (size_t)T::kEpiWarps * T::kStgWarp + T::kColBytes;
+  return 1024 + (size_t)T::kStages * kStageBytes + T::kBoxes + kControlBytes + T::kExtra;
 }
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -169,6 +178,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster)
                : "memory");
 }
+// The same without ordering this thread's earlier writes before it: a release at cluster scope waits for
+// all of the warp's global stores, and an epilogue warp that only hands its accumulator back (whose
+// reads tcgen05.wait::ld has completed) publishes nothing.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t bar_cluster) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
+}
 
 // Barrier of `threads` threads (all of them in whole warps) that also tells whether all of them agree.
 __device__ __forceinline__ bool barrier_and(int id, int threads, bool ok) {
@@ -191,6 +206,8 @@ template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Traits<KIND>::kThreads, 1)
 grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                         const __grid_constant__ CUtensorMap tmap_bc,
+                        const __grid_constant__ CUtensorMap tmap_h,    // kGegluTrain: h, 32 x 32 boxes
+                        const __grid_constant__ CUtensorMap tmap_gu,   // training: gu
                         const CUtensorMap* __restrict__ tmap_b,  // [E], 128-row (B_MN: 64-row) boxes
                         const int32_t* __restrict__ offsets,
                         const void* const* __restrict__ bias_ptrs, int E, int K, int Nout,
@@ -205,8 +222,9 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~(uintptr_t)1023);
-  Control* ctl = reinterpret_cast<Control*>(smem + (size_t)kStages * kStageBytes);
-  uint8_t* stage_out = smem + (size_t)kStages * kStageBytes + kControlBytes;
+  uint8_t* boxes = smem + (size_t)kStages * kStageBytes;
+  Control* ctl = reinterpret_cast<Control*>(boxes + T::kBoxes);
+  uint8_t* extra = boxes + T::kBoxes + kControlBytes;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -225,7 +243,12 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       mbar_init(&ctl->tail[s], 1);
       mbar_init(&ctl->peer_cut[s], 1);
     }
-    for (int a = 0; a < 2; ++a) { mbar_init(&ctl->tmem_full[a], 1); mbar_init(&ctl->tmem_empty[a], 2 * kEpiWarps); }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&ctl->tmem_full[a], 1);
+      mbar_init(&ctl->tmem_empty[a], 2 * kEpiWarps);
+      mbar_init(&ctl->aux_full[a], KIND == kGegluTrain ? T::kHelpers : 1);
+      mbar_init(&ctl->aux_empty[a], kEpiWarps);
+    }
     ctl->abort = 0;
   }
   if (warp == 1) {
@@ -394,16 +417,74 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       }
       parity ^= 1u << s;
     }
+  } else if (KIND == kGegluTrain && warp >= 2 + kEpiWarps) {
+    // ---------------- dropout mask: four warps, 32 rows of the tile each ----------------
+    int it = 0, e = 0;
+    for (int t = pair; tr.thresh != 0u && t < total_tiles; t += num_pairs, ++it) {
+      while (t >= ctl->tile_start[e + 1]) ++e;
+      const int local = t - ctl->tile_start[e];
+      const int mt = local / n_tiles, nt = local - mt * n_tiles;
+      const int row_cta = ctl->offsets[e] + mt * kPairRows + (int)cta * BM;
+      const int a = it & 1;
+      if (!mbar_wait(&ctl->aux_empty[a], ((uint32_t)(it >> 1) & 1u) ^ 1u, &ctl->abort, status, 37)) break;
+      uint32_t* s_mask = reinterpret_cast<uint32_t*>(extra + kEpiWarps * 256) + a * BM * 4;
+      const int rl = (warp - 2 - kEpiWarps) * 32 + lane;
+      draw_mask(tr, row_cta + rl, row_cta + rl < ctl->offsets[e + 1], nt * kTileN, Nout, s_mask + rl * 4);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->aux_full[a]);
+    }
+  } else if (KIND == kDhGeglu && warp == 2 + kEpiWarps) {
+    // ---------------- gate and up values: two chunks ahead, stored again as gradients ----------------
+    if (lane == 0) {
+      struct Place { int col, row; bool boxes; } place[2];
+      int ci = 0, e = 0;
+      auto put_back = [&](int b, int use) {      // use: how many times the buffer has been filled before
+        if (!mbar_wait(&ctl->aux_empty[b], (uint32_t)use & 1u, &ctl->abort, status, 38)) return false;
+        const Place& p = place[b];
+        if (p.boxes) {
+          uint8_t* box = boxes + b * 2 * GegluBwd::kBoxBytes;
+          tma_store_2d(&tmap_gu, box, p.col, p.row);
+          tma_store_2d(&tmap_gu, box + GegluBwd::kBoxBytes, Nout + p.col, p.row);
+        }
+        bulk_commit();
+        return true;
+      };
+      bool ok = true;
+      for (int t = pair; ok && t < total_tiles; t += num_pairs) {
+        while (t >= ctl->tile_start[e + 1]) ++e;
+        const int local = t - ctl->tile_start[e];
+        const int mt = local / n_tiles, nt = local - mt * n_tiles;
+        const int row_cta = ctl->offsets[e] + mt * kPairRows + (int)cta * BM;
+        const bool rows_full = ctl->offsets[e + 1] - row_cta >= BM;
+        for (int c = 0; ok && c < BN / GegluBwd::kChunk; ++c, ++ci) {
+          const int b = ci & 1;
+          const int col = nt * kTileN + c * GegluBwd::kChunk;
+          if (ci >= 2) {
+            ok = put_back(b, (ci >> 1) - 1);
+            bulk_wait_read<0>();
+            if (!ok) break;
+          }
+          // a box must lie inside gate or up: the last columns of an odd width are stored by the epilogue
+          place[b] = Place{col, row_cta, rows_full && col + GegluBwd::kChunk <= Nout};
+          uint8_t* box = boxes + b * 2 * GegluBwd::kBoxBytes;
+          mbar_expect_tx(&ctl->aux_full[b], 2 * GegluBwd::kBoxBytes);
+          tma_load_2d(box, &tmap_gu, &ctl->aux_full[b], col, row_cta);
+          tma_load_2d(box + GegluBwd::kBoxBytes, &tmap_gu, &ctl->aux_full[b], Nout + col, row_cta);
+        }
+      }
+      for (int q = ci > 2 ? ci - 2 : 0; ok && q < ci; ++q) ok = put_back(q & 1, q >> 1);
+      bulk_wait_all();
+    }
   } else {
     // ---------------- epilogue: one accumulator row per thread ----------------
     const int quad = warp & 3;
     const int part = (warp - 2) >> 2;  // the warps of a TMEM lane quadrant split the columns
     const int r = quad * 32 + lane;
-    uint8_t* stg = stage_out + (warp - 2) * T::kStgWarp;
     uint32_t acc_phase = 0;
     int it = 0;
     int e = 0;
     bool ok = true;
+    BoxOut box{boxes + (warp - 2) * kBoxBytes};    // kGegluTrain
     for (int t = pair; ok && t < total_tiles; t += num_pairs) {
       while (t >= ctl->tile_start[e + 1]) ++e;
       const int local = t - ctl->tile_start[e];
@@ -421,9 +502,14 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         continue;
       }
       const int a = it & 1;
-      GegluBwd gb;
-      if constexpr (KIND == kDhGeglu)     // its inputs are requested before the products are awaited
-        gb.start(tr, row_warp, rows, Nout, n0 + part * 64, lane);
+      float* s_bias = reinterpret_cast<float*>(extra + (warp - 2) * 256);
+      if constexpr (KIND == kGegluTrain) GegluTrain::start(n0, Nout, bias, s_bias, lane, part);
+      uint32_t keep[4];
+      if constexpr (KIND == kDhGeglu) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          keep[c] = GegluBwd::mask_bits(tr, row_warp + lane, lane < rows, n0 + c * 64 + part * 16, Nout);
+      }
       ok = mbar_wait(&ctl->tmem_full[a], acc_phase, &ctl->abort, status, 34);
       if (KIND != kDhGeglu && !ok) break;
       tc_fence_after();
@@ -431,14 +517,44 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       auto release = [&]() {     // this warp has read its part of the accumulator
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&ctl->tmem_empty[a]), 0));
+        if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&ctl->tmem_empty[a]), 0));
       };
       if constexpr (KIND == kGegluTrain) {
-        store_tile_train(taddr, row_warp, rows, n0, Nout, bias, out_e, tr, stg, lane, part);
-        release();
+        uint32_t bits = 0xffffffffu;
+        if (tr.thresh != 0u) {
+          ok = mbar_wait(&ctl->aux_full[a], acc_phase, &ctl->abort, status, 39);
+          if (!ok) break;
+          bits = reinterpret_cast<const uint32_t*>(extra + kEpiWarps * 256)[(a * BM + r) * 4 + part];
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->aux_empty[a]);
+        }
+        GegluTrain::finish(taddr, row_warp, rows, n0, Nout, out_e, tr, &tmap_h, &tmap_gu, s_bias, bits, box, lane, part,
+                           release);
       } else if constexpr (KIND == kDhGeglu) {
-        float* s_col = reinterpret_cast<float*>(stage_out + kEpiWarps * T::kStgWarp);
-        if (ok) gb.finish(taddr + part * 64, stg, s_col + quad * 2 * BN + part * 64, BN, release);
+        float* s_col = reinterpret_cast<float*>(extra);
+#pragma unroll 1
+        for (int c = 0; ok && c < 4; ++c) {
+          const int b = c & 1;
+          // two uses of either buffer per tile
+          ok = mbar_wait(&ctl->aux_full[b], (uint32_t)(c >> 1), &ctl->abort, status, 40);
+          if (!ok) break;
+          const int n = n0 + c * 64 + part * 16;
+          uint32_t v[16];
+          tc_ld16(taddr + c * 64 + part * 16, v);
+          tc_ld_wait();
+          if (c == 3) release();
+          const bool as_boxes = row_end - row_cta >= BM && n0 + c * 64 + 64 <= Nout;
+          __nv_bfloat16* direct = as_boxes ? nullptr : tr.gu + (int64_t)(row_warp + lane) * 2 * Nout + n;
+          uint32_t bits = keep[0];
+          bits = c == 1 ? keep[1] : bits;
+          bits = c == 2 ? keep[2] : bits;
+          bits = c == 3 ? keep[3] : bits;
+          GegluBwd::chunk(v, boxes + b * 2 * GegluBwd::kBoxBytes, bits, tr.scale, lane < rows, direct, Nout, Nout - n,
+                          s_col + quad * 2 * BN + c * 64 + part * 16, BN, quad, part, lane);
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ctl->aux_empty[b]);
+        }
         // column sums of this CTA's 128 rows: the four lane quadrants in order. A warp whose wait
         // ran out still comes to the barrier, and all leave together.
         ok = barrier_and(1, 32 * kEpiWarps, ok);
@@ -452,13 +568,13 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         barrier_and(1, 32 * kEpiWarps, true);
       } else {
-        store_tile<GEGLU, KIND == kScatter>(taddr, row_cta + r, row_cta + r < row_end, n0, Nout, bias, out_e, sc, stg,
-                                            lane, part);
-        release();
+        store_tile<GEGLU, KIND == kScatter>(taddr, row_cta + r, row_cta + r < row_end, n0, Nout, bias, out_e, sc,
+                                            extra + (warp - 2) * kStgBytes, lane, part, release);
       }
       if (a == 1) acc_phase ^= 1u;
       ++it;
     }
+    if (KIND == kGegluTrain && lane == 0) bulk_wait_all();
     if (KIND == kScatter) __threadfence_system();
   }
   // expert-parallel down pass: the last CTA to get here tells every rank that this rank's
@@ -485,7 +601,8 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
 template <int KIND>
 int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_bc, const void* tmap_b, const int32_t* offsets,
                 const void* const* bias, int E, int K, int Nout, void* out, const EpScatter& sc,
-                const TrainArgs& tr, const EpSync& sy, int Ra, int32_t* status, int sms, cudaStream_t s) {
+                const TrainArgs& tr, const EpSync& sy, int Ra, int32_t* status, int sms, cudaStream_t s,
+                const CUtensorMap* tm_h = nullptr, const CUtensorMap* tm_gu = nullptr) {
   static PerDeviceOnce once;
   auto fn = grouped_gemm_tc2_kernel<KIND>;
   constexpr size_t smem = smem_bytes<KIND>();
@@ -493,6 +610,7 @@ int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_bc, const void* t
   int rc = ensure_dynamic_smem(once, fn, smem);
   if (rc) return rc;
   MOE_CUDA_CHECK(launch_pdl(fn, dim3(sms & ~1), dim3(Traits<KIND>::kThreads), smem, s, tm_a, tm_bc,
+                            tm_h != nullptr ? *tm_h : tm_a, tm_gu != nullptr ? *tm_gu : tm_a,
                             static_cast<const CUtensorMap*>(tmap_b), offsets, bias, E, K, Nout,
                             static_cast<__nv_bfloat16*>(out), sc, tr, sy, Ra, status));
   return 0;
@@ -521,11 +639,17 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
   const EpSync nosync = {};
   const EpSync& sy1 = ep_wait != nullptr ? *ep_wait : nosync;
   const EpSync& sy2 = ep_signal != nullptr ? *ep_signal : nosync;
-  if (train != nullptr)
+  if (train != nullptr) {
+    alignas(64) CUtensorMap tm_hb, tm_gu;
+    rc = encode_tmap_2d(&tm_hb, h, rows, (uint64_t)f, 32, 32);
+    if (rc) return rc;
+    rc = encode_tmap_2d(&tm_gu, train->gu, rows, (uint64_t)2 * f, 32, 32);
+    if (rc) return rc;
     rc = launch_pair<kGegluTrain>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, *train, sy1, 0, status,
-                                  sms, s);
-  else
+                                  sms, s, &tm_hb, &tm_gu);
+  } else {
     rc = launch_pair<kGeglu>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, eval, sy1, 0, status, sms, s);
+  }
   if (rc) return rc;
   if (sc != nullptr)
     return launch_pair<kScatter>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, nullptr, *sc, eval, sy2, 0, status,
@@ -545,9 +669,13 @@ int launch_grouped_dx(const void* A, int64_t M, int K, const void* tmaps_b, cons
   const EpScatter none = {};
   const TrainArgs eval = {};
   const EpSync nosync = {};
-  if (geglu_bwd != nullptr)
+  if (geglu_bwd != nullptr) {
+    alignas(64) CUtensorMap tm_gu;
+    rc = encode_tmap_2d(&tm_gu, geglu_bwd->gu, (uint64_t)M, (uint64_t)2 * Nout, BM);
+    if (rc) return rc;
     return launch_pair<kDhGeglu>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, nullptr, none, *geglu_bwd,
-                                 nosync, 0, status, sms, s);
+                                 nosync, 0, status, sms, s, nullptr, &tm_gu);
+  }
   return launch_pair<kDx>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, out, none, eval, nosync, 0, status, sms,
                           s);
 }

@@ -16,7 +16,6 @@
 
 namespace moe {
 
-int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
 namespace {
 

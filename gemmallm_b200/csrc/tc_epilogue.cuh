@@ -58,11 +58,12 @@ __device__ __forceinline__ uint4 pack8(const float (&o)[8]) {
 //   plain  : 256 outputs per row, 128 per warp (two passes); bias may be nullptr (none)
 //   SCATTER: plain, but the row goes to sc.ret_y[meta >> 24] + (meta & 0xffffff) * Nout
 //            (the token owner's buffer, possibly on another GPU)
-template <bool GEGLU, bool SCATTER>
+//   release(): called once the warp has read its part of the accumulator
+template <bool GEGLU, bool SCATTER, typename Release>
 __device__ __forceinline__ void store_tile(uint32_t taddr, int row, bool row_ok, int n0, int Nout,
                                            const __nv_bfloat16* __restrict__ bias,
                                            __nv_bfloat16* __restrict__ out, const EpScatter& sc,
-                                           uint8_t* stg, int lane, int half) {
+                                           uint8_t* stg, int lane, int half, Release release) {
   constexpr int BN = 256;
   constexpr int kTileN = GEGLU ? BN / 2 : BN;
   constexpr int kPasses = kTileN / 128;        // 64-column passes per warp
@@ -89,6 +90,7 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, int row, bool row_ok,
         uint32_t u[32];
         tc_ld32(taddr + BN / 2 + c * 32, u);
         tc_ld_wait();
+        if (hc == 1 && p == kPasses - 1) release();
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int n = n0 + c * 32 + q * 8;
@@ -110,6 +112,7 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, int row, bool row_ok,
         }
       } else {
         tc_ld_wait();
+        if (hc == 1 && p == kPasses - 1) release();
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int n = n0 + c * 32 + q * 8;
@@ -161,193 +164,200 @@ __device__ __forceinline__ void flush32(const uint4 (&packed)[4], __nv_bfloat16*
   }
 }
 
+// Output boxes of 32 rows x 32 columns of an epilogue warp whose 32 rows all exist: written to the
+// warp's buffer (64-byte swizzle: 16-byte piece c of row r lies at c ^ (r / 2 mod 4)) and stored by TMA,
+// about a fifth of the instructions of flush32 and no wait for the memory.
+constexpr int kBoxBytes = 32 * 64;
+struct BoxOut {
+  uint8_t* buf;
+  __device__ __forceinline__ void put(const uint4 (&packed)[4], const void* tmap, int col, int row, int lane) {
+    if (lane == 0) bulk_wait_read<0>();      // the store before this one has read the buffer
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<uint4*>(buf + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4)) = packed[q];
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(tmap, buf, col, row);
+      bulk_commit();
+    }
+  }
+};
+
 // GEGLU pass in training mode (TrainArgs in common.cuh), 16 epilogue warps: this one takes output
 // columns [32 part, 32 part + 32) of its 32 rows. The gate/up pre-activations are kept for the backward
-// pass, h gets its dropout mask, and the mask itself is kept as one bit per element, so that the
-// backward pass does not run Philox again.
-__device__ __forceinline__ void store_tile_train(uint32_t taddr, int row_warp, int rows, int n0, int Nout,
-                                                 const __nv_bfloat16* __restrict__ bias,
-                                                 __nv_bfloat16* __restrict__ out, const TrainArgs& tr, uint8_t* stg,
-                                                 int lane, int part) {
-  const int n = n0 + part * 32;
-  const int cols = Nout - n;
-  const int64_t row = row_warp + lane;
-  const bool row_ok = lane < rows;
-  const uint32_t pair = row_ok ? (uint32_t)__ldg(&tr.pair_of[row]) : 0u;
-  uint32_t g[32], u[32];
-  tc_ld32(taddr + part * 32, g);
-  tc_ld32(taddr + 128 + part * 32, u);
-  tc_ld_wait();
-  uint4 ph[4], pg[4], pu[4];
-  uint32_t keep = 0xffffffffu;
+// pass and h gets its dropout mask: s_mask[row][part], bits drawn by four other warps while the products of the
+// tile run (draw_mask). start() fetches the biases into this warp's 64 floats of shared memory before the
+// products are awaited.
+struct GegluTrain {
+  __device__ __forceinline__ static void start(int n0, int Nout, const __nv_bfloat16* __restrict__ bias, float* s_bias,
+                                               int lane, int part) {
+    const int n = n0 + part * 32 + lane;
+    const float bg = n < Nout ? __bfloat162float(__ldg(bias + n)) : 0.f;
+    const float bu = n < Nout ? __bfloat162float(__ldg(bias + Nout + n)) : 0.f;
+    __syncwarp();
+    s_bias[lane] = bg;
+    s_bias[32 + lane] = bu;
+    __syncwarp();
+  }
+  template <typename Release>
+  __device__ __forceinline__ static void finish(uint32_t taddr, int row_warp, int rows, int n0, int Nout,
+                                                __nv_bfloat16* __restrict__ out, const TrainArgs& tr,
+                                                const void* tmap_h, const void* tmap_gu, const float* s_bias,
+                                                uint32_t keep, BoxOut& box, int lane, int part, Release release) {
+    const int n = n0 + part * 32;
+    const int cols = Nout - n;
+    uint4 ph[4], pg[4], pu[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    float gv[8], uv[8], o[8];
-    if (q * 8 < cols) {
-      load8_ldg(bias + n + q * 8, gv);
-      load8_ldg(bias + Nout + n + q * 8, uv);
-    } else {
+    for (int hc = 0; hc < 2; ++hc) {      // 16 columns at a time: fewer registers, more warps
+      uint32_t g[16], u[16];
+      tc_ld16(taddr + part * 32 + hc * 16, g);
+      tc_ld16(taddr + 128 + part * 32 + hc * 16, u);
+      tc_ld_wait();
+      if (hc == 1) release();
 #pragma unroll
-      for (int i = 0; i < 8; ++i) gv[i] = uv[i] = 0.f;
-    }
+      for (int q = 0; q < 2; ++q) {
+        const int c = hc * 16 + q * 8;
+        float gv[8], uv[8], o[8];
+        load8(s_bias + c, gv);
+        load8(s_bias + 32 + c, uv);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      gv[i] += __uint_as_float(g[q * 8 + i]);
-      uv[i] += __uint_as_float(u[q * 8 + i]);
-      o[i] = gelu_tanh_fast(gv[i]) * uv[i];
-    }
-    pg[q] = pack8(gv);
-    pu[q] = pack8(uv);
-    if (tr.thresh != 0u) {
-#pragma unroll
-      for (int b4 = 0; b4 < 2; ++b4) {
-        const uint4 r = philox4x32_10((uint32_t)((n + q * 8) >> 2) + b4, pair, tr.seed_lo, tr.seed_hi);
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const bool kept = w[i] >= tr.thresh;
-          o[b4 * 4 + i] = kept ? o[b4 * 4 + i] * tr.scale : 0.f;
-          if (!kept) keep &= ~(1u << (q * 8 + b4 * 4 + i));
+        for (int i = 0; i < 8; ++i) {
+          gv[i] += __uint_as_float(g[q * 8 + i]);
+          uv[i] += __uint_as_float(u[q * 8 + i]);
+          const float hv = gelu_tanh_fast(gv[i]) * uv[i];
+          o[i] = (keep >> (c + i)) & 1u ? hv * tr.scale : 0.f;
         }
+        pg[c / 8] = pack8(gv);
+        pu[c / 8] = pack8(uv);
+        ph[c / 8] = pack8(o);
       }
     }
-    ph[q] = pack8(o);
-  }
-  if (tr.thresh != 0u && row_ok) {
-    uint8_t* m = tr.mask + row * (Nout >> 3) + (n >> 3);
-    if ((Nout & 31) == 0) {
-      *reinterpret_cast<uint32_t*>(m) = keep;
-    } else {
-      for (int q = 0; q < 4 && q * 8 < cols; ++q) m[q] = (uint8_t)(keep >> (q * 8));
+    if (rows >= 32 && cols >= 32) {
+      box.put(ph, tmap_h, n, row_warp, lane);
+      box.put(pg, tmap_gu, n, row_warp, lane);
+      box.put(pu, tmap_gu, Nout + n, row_warp, lane);
+    } else {       // the expert's last rows, or the last columns of an odd width
+      if (lane == 0) bulk_wait_read<0>();
+      __syncwarp();
+      flush32(ph, out + (int64_t)row_warp * Nout + n, Nout, rows, cols, box.buf, lane);
+      flush32(pg, tr.gu + (int64_t)row_warp * 2 * Nout + n, 2 * (int64_t)Nout, rows, cols, box.buf, lane);
+      flush32(pu, tr.gu + (int64_t)row_warp * 2 * Nout + Nout + n, 2 * (int64_t)Nout, rows, cols, box.buf, lane);
     }
   }
-  flush32(ph, out + (int64_t)row_warp * Nout + n, Nout, rows, cols, stg, lane);
-  flush32(pg, tr.gu + (int64_t)row_warp * 2 * Nout + n, 2 * (int64_t)Nout, rows, cols, stg, lane);
-  flush32(pu, tr.gu + (int64_t)row_warp * 2 * Nout + Nout + n, 2 * (int64_t)Nout, rows, cols, stg, lane);
+};
+
+// The dropout mask of one row's 128 columns from n0 (bit i of word w: column n0 + 32 w + i, set = kept), to
+// shared memory for the epilogue and to global memory for the backward pass.
+__device__ __forceinline__ void draw_mask(const TrainArgs& tr, int64_t row, bool row_ok, int n0, int Nout,
+                                          uint32_t* s_row) {
+  const uint32_t pair = row_ok ? (uint32_t)__ldg(&tr.pair_of[row]) : 0u;
+  uint32_t w[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    uint32_t keep = 0u;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const uint4 r = philox4x32_10((uint32_t)((n0 >> 2) + p * 8 + b), pair, tr.seed_lo, tr.seed_hi);
+      keep |= (r.x >= tr.thresh ? 1u : 0u) << (4 * b) | (r.y >= tr.thresh ? 2u : 0u) << (4 * b) |
+              (r.z >= tr.thresh ? 4u : 0u) << (4 * b) | (r.w >= tr.thresh ? 8u : 0u) << (4 * b);
+    }
+    w[p] = keep;
+  }
+  *reinterpret_cast<uint4*>(s_row) = make_uint4(w[0], w[1], w[2], w[3]);
+  if (row_ok) {
+    uint8_t* m = tr.mask + row * (Nout >> 3) + (n0 >> 3);
+    if ((Nout & 127) == 0) {
+      *reinterpret_cast<uint4*>(m) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+      for (int q = 0; q < 16 && n0 + q * 8 < Nout; ++q) m[q] = (uint8_t)(w[q >> 2] >> ((q & 3) * 8));
+    }
+  }
 }
 
-// Epilogue of dh = dy W2 in the backward pass (model.py:180-183), 16 epilogue warps, this one for 64
-// columns of its 32 rows: dh is rounded to bf16 and staged so that a lane owns eight neighbouring columns
-// of a row, whose gate/up pre-activations (and mask bits) it reads and whose gradients it writes in 128-byte
-// runs of eight lanes:
+// Epilogue of dh = dy W2 in the backward pass (model.py:180-183), 16 epilogue warps, one accumulator row per
+// thread, back through dropout, product and GELU in place over the pre-activations gu:
 //   dhe = dh * mask * scale;  du = dhe * gelu(g);  dg = dhe * u * gelu'(g)
 //   with s = 1 / (1 + exp(-2 z)), z = b (g + a g^3):  gelu(g) = g s,
 //   gelu'(g) = s + 2 g s (1 - s) b (1 + 3 a g^2)       (0.5 (1 + tanh z) = s)
-// in place over gu. It also sums dg and du over its rows (the bias gradient of gate_and_up).
+// The tile is worked on in chunks of 64 columns: another warp (gu_warp in the kernel) brings a chunk of gate and up
+// values (two boxes of 128 rows x 64 columns, 128-byte swizzle) to shared memory two chunks ahead, the epilogue
+// replaces them by their gradients there, and the boxes are stored again. (With the loads issued by the epilogue
+// warps themselves, however far ahead registers allowed, their latency made the kernel 2.3 times as long.)
+// This warp takes columns [16 part, 16 part + 16) of the chunk for its 32 rows; it also sums dg and du over the
+// rows (the bias gradient of gate_and_up) into s_col[0..15] and s_col[du_off ..].
 struct GegluBwd {
-  uint4 g[4], u[4];      // pre-activations of 16 rows: rows i*4 + lane/8, columns 8 (lane % 8) ..
-  uint32_t m[4];
-  __nv_bfloat16* gp;     // row lane/8, this lane's columns
-  const uint8_t* mp;
-  int64_t f;
-  int rows, lane;
-  bool col_ok, masked;
-  float scale;
-
-  __device__ __forceinline__ void fetch(int hr) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int rr = hr * 16 + i * 4 + (lane >> 3);
-      g[i] = u[i] = make_uint4(0, 0, 0, 0);
-      m[i] = 0xffu;
-      if (col_ok && rr < rows) {
-        const __nv_bfloat16* p = gp + (hr * 16 + i * 4) * 2 * f;
-        g[i] = *reinterpret_cast<const uint4*>(p);
-        u[i] = *reinterpret_cast<const uint4*>(p + f);
-        if (masked) m[i] = mp[(hr * 16 + i * 4) * (f >> 3)];
-      }
-    }
+  static constexpr int kChunk = 64;
+  static constexpr int kBoxBytes = 128 * 128;
+  __device__ __forceinline__ static uint32_t mask_bits(const TrainArgs& tr, int64_t row, bool row_ok, int n, int f) {
+    if (tr.thresh == 0u) return 0xffffu;
+    if (!row_ok || n >= f) return 0u;
+    const uint8_t* m = tr.mask + row * (f >> 3) + (n >> 3);
+    if ((f & 15) == 0) return *reinterpret_cast<const uint16_t*>(m);
+    return n + 8 < f ? (uint32_t)m[0] | (uint32_t)m[1] << 8 : (uint32_t)m[0];
   }
-  __device__ __forceinline__ void start(const TrainArgs& tr, int row_warp, int rows_, int Nout, int n, int lane_) {
-    lane = lane_;
-    rows = rows_;
-    f = Nout;
-    scale = tr.scale;
-    masked = tr.thresh != 0u;
-    const int c = n + (lane & 7) * 8;
-    col_ok = c < Nout;
-    const int64_t row = row_warp + (lane >> 3);
-    gp = tr.gu + row * 2 * f + c;
-    mp = tr.mask + row * (f >> 3) + (c >> 3);
-    fetch(0);
-  }
-  // taddr: this warp's 64 columns; s_col: where the column sums go, du's `du_off` floats behind dg's
-  template <typename Release>
-  __device__ __forceinline__ void finish(uint32_t taddr, uint8_t* stg, float* s_col, int du_off, Release release) {
-    uint4 dh[8];
+  // v: dh of this row's 16 columns; box: the chunk's gate box in shared memory, the up box behind it.
+  // direct: the row's place in gu for a chunk that cannot be stored as boxes, else nullptr; cols: columns that exist
+  __device__ __forceinline__ static void chunk(const uint32_t (&v)[16], uint8_t* box, uint32_t keep, float scale,
+                                               bool row_ok, __nv_bfloat16* direct, int f, int cols, float* s_col,
+                                               int du_off, int quad, int part, int lane) {
+    float dg[16], du[16];
+    const int r = quad * 32 + lane;
 #pragma unroll
-    for (int hc = 0; hc < 2; ++hc) {
-      uint32_t v[32];
-      tc_ld32(taddr + hc * 32, v);
-      tc_ld_wait();
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float o[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(v[q * 8 + i]);
-        dh[hc * 4 + q] = pack8(o);
-      }
-    }
-    release();
-    float cg[8], cu[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) cg[i] = cu[i] = 0.f;
-#pragma unroll
-    for (int hr = 0; hr < 2; ++hr) {
-      if ((lane >> 4) == hr) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *reinterpret_cast<uint4*>(stg + (lane & 15) * kStgPitch + q * 16) = dh[q];
-      }
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int rl = i * 4 + (lane >> 3);
-        if (col_ok && hr * 16 + rl < rows) {
-          const uint4 dv4 = *reinterpret_cast<const uint4*>(stg + rl * kStgPitch + (lane & 7) * 16);
-          const uint32_t dw[4] = {dv4.x, dv4.y, dv4.z, dv4.w};
-          const uint32_t gw[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
-          const uint32_t uw[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
-          float dg[8], du[8];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            float dv = (c & 1) ? bf16_hi(dw[c >> 1]) : bf16_lo(dw[c >> 1]);
-            const float x = (c & 1) ? bf16_hi(gw[c >> 1]) : bf16_lo(gw[c >> 1]);
-            const float uv = (c & 1) ? bf16_hi(uw[c >> 1]) : bf16_lo(uw[c >> 1]);
-            if (masked) dv = ((m[i] >> c) & 1u) ? dv * scale : 0.f;
-            constexpr float kB = 0.7978845608028654f, kA = 0.044715f, kL = -2.f * 1.4426950408889634f;
-            const float x2 = x * x;
-            const float s = __fdividef(1.f, 1.f + exp2f_fast(x * fmaf(kL * kB * kA, x2, kL * kB)));
-            const float gs = x * s;
-            const float dgelu = fmaf(fmaf(-gs, s, gs), fmaf(6.f * kA * kB, x2, 2.f * kB), s);
-            du[c] = dv * gs;
-            dg[c] = dv * uv * dgelu;
-            cg[c] += dg[c];
-            cu[c] += du[c];
-          }
-          __nv_bfloat16* p = gp + (hr * 16 + i * 4) * 2 * f;
-          *reinterpret_cast<uint4*>(p) = pack8(dg);
-          *reinterpret_cast<uint4*>(p + f) = pack8(du);
-        }
-      }
-      __syncwarp();
-      if (hr == 0) fetch(1);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-#pragma unroll
-      for (int o = 8; o <= 16; o <<= 1) {
-        cg[i] += __shfl_xor_sync(0xffffffffu, cg[i], o);
-        cu[i] += __shfl_xor_sync(0xffffffffu, cu[i], o);
-      }
-    }
-    if (lane < 8) {
+    for (int j = 0; j < 2; ++j) {
+      uint4* gp = reinterpret_cast<uint4*>(box + r * 128 + (((part * 2 + j) ^ (r & 7)) << 4));
+      uint4* up = gp + kBoxBytes / 16;
+      const uint4 g4 = *gp, u4 = *up;
+      const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w};
+      const uint32_t uw[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        s_col[lane * 8 + i] = cg[i];
-        s_col[du_off + lane * 8 + i] = cu[i];
+        constexpr float kB = 0.7978845608028654f, kA = 0.044715f, kL = -2.f * 1.4426950408889634f;
+        const int c = j * 8 + i;
+        const float dv = (keep >> c) & 1u ? __uint_as_float(v[c]) * scale : 0.f;
+        const float x = (i & 1) ? bf16_hi(gw[i >> 1]) : bf16_lo(gw[i >> 1]);
+        const float uv = (i & 1) ? bf16_hi(uw[i >> 1]) : bf16_lo(uw[i >> 1]);
+        const float x2 = x * x;
+        const float s = __fdividef(1.f, 1.f + exp2f_fast(x * fmaf(kL * kB * kA, x2, kL * kB)));
+        const float gs = x * s;
+        const float dgelu = fmaf(fmaf(-gs, s, gs), fmaf(6.f * kA * kB, x2, 2.f * kB), s);
+        du[c] = row_ok ? dv * gs : 0.f;
+        dg[c] = row_ok ? dv * uv * dgelu : 0.f;
+      }
+      const uint4 og = make_uint4(pack_bf16x2(dg[j * 8], dg[j * 8 + 1]), pack_bf16x2(dg[j * 8 + 2], dg[j * 8 + 3]),
+                                  pack_bf16x2(dg[j * 8 + 4], dg[j * 8 + 5]), pack_bf16x2(dg[j * 8 + 6], dg[j * 8 + 7]));
+      const uint4 ou = make_uint4(pack_bf16x2(du[j * 8], du[j * 8 + 1]), pack_bf16x2(du[j * 8 + 2], du[j * 8 + 3]),
+                                  pack_bf16x2(du[j * 8 + 4], du[j * 8 + 5]), pack_bf16x2(du[j * 8 + 6], du[j * 8 + 7]));
+      if (direct == nullptr) {
+        *gp = og;
+        *up = ou;
+      } else if (row_ok && j * 8 < cols) {
+        *reinterpret_cast<uint4*>(direct + j * 8) = og;
+        *reinterpret_cast<uint4*>(direct + f + j * 8) = ou;
       }
     }
+    // sums over the 32 lanes, each step keeping half of the 32 values: lane l ends with one of them
+    float t[32];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      t[i] = dg[i];
+      t[16 + i] = du[i];
+    }
+    int first = 0;
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      const bool upper = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (i < o) {
+          const float give = upper ? t[i] : t[o + i];
+          const float mine = upper ? t[o + i] : t[i];
+          t[i] = mine + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      if (upper) first += o;
+    }
+    s_col[(first & 15) + (first >= 16 ? du_off : 0)] = t[0];
   }
 };
 
