@@ -7,8 +7,9 @@
 //   combine_bwd      dy[r] = w[pair] * dOut[token], dw[pair] = dOut[token] . y[r]   (model.py:271)
 //   router_bwd       dw -> d(renormalised scores) -> d(softmax) -> dlogits, plus the gradient
 //                    of the load-balancing loss through the mean probabilities
-//                    (model.py:207-223; the counts of model.py:213 carry no gradient)
-//   router_bwd_wx    dWg = dlogits^T x, dbg = sum dlogits, dx += dlogits Wg       (model.py:206)
+//                    (model.py:207-223; the counts of model.py:213 carry no gradient), and in the
+//                    same pass dWg = dlogits^T x, dbg = sum dlogits                 (model.py:206)
+//   combine_dx       dx[t] = the sum of its rows' gradients + dlogits[t] Wg    (model.py:248-253, 206)
 //   colsum           bias gradients per expert
 #include "common.cuh"
 
@@ -52,34 +53,30 @@ combine_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* 
   if (lane == 0) dw[p] = dot;
 }
 
-// One warp per token; lane e handles experts e, e+32, ...
+// Gradient of a token's logits by one warp; lane l holds experts l, l + 32, ... (PER of them).
 //   w_j = v_j / total, v_j = p[idx_j]:  dv_j = (dw_j - sum_i dw_i w_i) / total
 //   aux = E * sum_e mean_n p[n,e] * cnt0_e / N:  dp[e] += grad_aux * E * cnt0_e / N^2
 //   dl[e] = p[e] * (dp[e] - sum_e' p[e'] dp[e'])
-__global__ void __launch_bounds__(256)
-router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ idx,
-                  const float* __restrict__ w, const float* __restrict__ dw,
-                  const int32_t* __restrict__ cnt0, float grad_aux_host, const float* __restrict__ grad_aux_dev,
-                  int64_t N, int E, int k, float* __restrict__ dl) {
-  const int64_t t = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (t >= N) return;
-  constexpr int kPer = kMaxExperts / 32;
-  float l[kPer], p[kPer], dp[kPer];
+template <int PER>
+__device__ __forceinline__ void token_dlogits(const float* __restrict__ logits, const int32_t* __restrict__ idx,
+                                              const float* __restrict__ w, const float* __restrict__ dw,
+                                              const int32_t* __restrict__ cnt0, float aux_c, int64_t t, int E, int k,
+                                              int lane, float (&dl)[PER]) {
+  float p[PER], dp[PER];
   float m = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) {
+  for (int i = 0; i < PER; ++i) {
     const int e = lane + 32 * i;
-    l[i] = e < E ? logits[t * E + e] : -INFINITY;
-    m = fmaxf(m, l[i]);
+    p[i] = e < E ? logits[t * E + e] : -INFINITY;
+    m = fmaxf(m, p[i]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) {
+  for (int i = 0; i < PER; ++i) {
     const int e = lane + 32 * i;
-    p[i] = e < E ? expf(l[i] - m) : 0.f;
+    p[i] = e < E ? expf(p[i] - m) : 0.f;
     sum += p[i];
   }
 #pragma unroll
@@ -87,10 +84,8 @@ router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ 
   // total of the chosen probabilities and sum_i dw_i w_i (every lane computes them: k <= 8)
   float total = 0.f, dww = 0.f;
   for (int j = 0; j < k; ++j) dww = fmaf(dw[t * k + j], w[t * k + j], dww);
-  const float grad_aux = grad_aux_dev != nullptr ? __ldg(grad_aux_dev) : grad_aux_host;
-  const float aux_c = grad_aux * (float)E / ((float)N * (float)N);
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) {
+  for (int i = 0; i < PER; ++i) {
     const int e = lane + 32 * i;
     p[i] = p[i] / sum;
     dp[i] = e < E ? aux_c * (float)cnt0[e] : 0.f;
@@ -100,7 +95,7 @@ router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ 
     const int e = idx[t * k + j];
     float v = 0.f;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i)
+    for (int i = 0; i < PER; ++i)
       if (i == (e >> 5)) v = p[i];
     total += __shfl_sync(0xffffffffu, v, e & 31);
   }
@@ -109,92 +104,172 @@ router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ 
     const float dv = (dw[t * k + j] - dww) / total;
     if ((e & 31) == lane) {
 #pragma unroll
-      for (int i = 0; i < kPer; ++i)
+      for (int i = 0; i < PER; ++i)
         if (i == (e >> 5)) dp[i] += dv;
     }
   }
   float pdp = 0.f;
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) pdp = fmaf(p[i], dp[i], pdp);
+  for (int i = 0; i < PER; ++i) pdp = fmaf(p[i], dp[i], pdp);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) pdp += __shfl_xor_sync(0xffffffffu, pdp, o);
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) {
-    const int e = lane + 32 * i;
-    if (e < E) dl[t * E + e] = p[i] * (dp[i] - pdp);
+  for (int i = 0; i < PER; ++i) dl[i] = p[i] * (dp[i] - pdp);
+}
+
+constexpr int kDlTokens = 32;    // tokens of a step
+constexpr int kDlExperts = 8;    // experts of a block's accumulators
+constexpr int kDlCols = 1024;    // columns of a block, four per thread
+
+// grid: (column blocks, token ranges, expert groups). Every block forms the logits' gradients of its tokens (the
+// first column block and expert group store them) and the products of its eight experts with its columns of
+// x; the partial sums of a token range go to part [range][E][d] and part_b [range][E] (no atomics: the same
+// result every time). What bounds it is one pass over x.
+template <int PER>
+__global__ void __launch_bounds__(256)
+router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ idx,
+                  const float* __restrict__ w, const float* __restrict__ dw,
+                  const int32_t* __restrict__ cnt0, float grad_aux_host, const float* __restrict__ grad_aux_dev,
+                  const __nv_bfloat16* __restrict__ x, int64_t N, int d, int E, int k, int tokens_per_block,
+                  float* __restrict__ dl_out, float* __restrict__ part, float* __restrict__ part_b) {
+  __shared__ float s_dl[kDlTokens][kDlExperts];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int e0 = blockIdx.z * kDlExperts;
+  const int c = blockIdx.x * kDlCols + tid * 4;
+  const int64_t t_begin = (int64_t)blockIdx.y * tokens_per_block;
+  const int64_t t_end = min(t_begin + tokens_per_block, N);
+  const float grad_aux = grad_aux_dev != nullptr ? __ldg(grad_aux_dev) : grad_aux_host;
+  const float aux_c = grad_aux * (float)E / ((float)N * (float)N);
+  const bool store_dl = blockIdx.x == 0 && blockIdx.z == 0;
+  float acc[kDlExperts][4];
+#pragma unroll
+  for (int i = 0; i < kDlExperts; ++i)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[i][q] = 0.f;
+  float bsum = 0.f;
+  for (int64_t t0 = t_begin; t0 < t_end; t0 += kDlTokens) {
+    const int nt = (int)min((int64_t)kDlTokens, t_end - t0);
+    __syncthreads();
+    for (int tl = warp; tl < nt; tl += 8) {
+      float dl[PER];
+      token_dlogits<PER>(logits, idx, w, dw, cnt0, aux_c, t0 + tl, E, k, lane, dl);
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int e = lane + 32 * i;
+        if (e < E && store_dl) dl_out[(t0 + tl) * E + e] = dl[i];
+        if (e >= e0 && e < e0 + kDlExperts) s_dl[tl][e - e0] = e < E ? dl[i] : 0.f;
+      }
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && tid < kDlExperts)
+      for (int tl = 0; tl < nt; ++tl) bsum += s_dl[tl][tid];
+    if (c < d) {
+      const uint2* xp = reinterpret_cast<const uint2*>(x + t0 * d + c);
+      const size_t pitch = (size_t)d >> 2;
+      for (int tb = 0; tb < nt; tb += 8) {
+        uint2 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = tb + u < nt ? __ldg(xp + (size_t)(tb + u) * pitch) : make_uint2(0, 0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (tb + u < nt) {
+            const float xv[4] = {bf16_lo(v[u].x), bf16_hi(v[u].x), bf16_lo(v[u].y), bf16_hi(v[u].y)};
+            const float4 ga = *reinterpret_cast<const float4*>(&s_dl[tb + u][0]);
+            const float4 gb = *reinterpret_cast<const float4*>(&s_dl[tb + u][4]);
+            const float g[kDlExperts] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+#pragma unroll
+            for (int i = 0; i < kDlExperts; ++i)
+#pragma unroll
+              for (int q = 0; q < 4; ++q) acc[i][q] = fmaf(g[i], xv[q], acc[i][q]);
+          }
+      }
+    }
+  }
+  if (c < d) {
+#pragma unroll
+    for (int i = 0; i < kDlExperts; ++i)
+      if (e0 + i < E)
+        *reinterpret_cast<float4*>(part + ((size_t)blockIdx.y * E + e0 + i) * d + c) =
+            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  }
+  if (blockIdx.x == 0 && tid < kDlExperts && e0 + tid < E) part_b[(size_t)blockIdx.y * E + e0 + tid] = bsum;
+}
+
+// out[i] = sum over `ranges` of part[r][i], in order; eight groups of 32 threads take every eighth.
+__global__ void __launch_bounds__(256)
+router_bwd_finish_kernel(const float* __restrict__ part, const float* __restrict__ part_b, int ranges, int64_t n,
+                         int E, __nv_bfloat16* __restrict__ dWg, __nv_bfloat16* __restrict__ dbg) {
+  __shared__ float s_sum[8][33];
+  const int grp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool bias = blockIdx.x == gridDim.x - 1;
+  for (int64_t i0 = bias ? 0 : (int64_t)blockIdx.x * 32; i0 < (bias ? (int64_t)E : n); i0 += bias ? 32 : n) {
+    const float* p = bias ? part_b : part;
+    const int64_t len = bias ? (int64_t)E : n, i = i0 + lane;
+    float sum = 0.f;
+    if (i < len) {
+#pragma unroll 4
+      for (int r = grp; r < ranges; r += 8) sum += p[(size_t)r * len + i];
+    }
+    s_sum[grp][lane] = sum;
+    __syncthreads();
+    if (threadIdx.x < 32 && i < len) {
+      float t = 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) t += s_sum[q][lane];
+      __nv_bfloat16* out = bias ? dbg : dWg;
+      if (out != nullptr) out[i] = __float2bfloat16_rn(t);
+    }
+    __syncthreads();
   }
 }
 
-// dWg[e][c] += sum_t dl[t][e] x[t][c] (fp32 atomics into a zeroed buffer), dbg[e] += sum_t dl[t][e],
-// dxr[t][c] = sum_e dl[t][e] Wg[e][c]. A block owns 256 columns and a range of tokens; experts in
-// groups of 32 (E > 32 re-reads the token range from L2).
+// dx[t] = sum_j dxs[row_of[t, j]] + sum_e dl[t, e] Wg[e]; a thread takes eight columns of four tokens, so that a
+// piece of Wg is used four times.
 __global__ void __launch_bounds__(256)
-router_bwd_wx_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ Wg,
-                     const float* __restrict__ dl, int64_t N, int d, int E, int tokens_per_block,
-                     float* __restrict__ dWg, float* __restrict__ dbg,
-                     __nv_bfloat16* __restrict__ dxr) {
-  __shared__ float s_dl[64][33];
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  const int64_t t_begin = (int64_t)blockIdx.y * tokens_per_block;
-  const int64_t t_end = t_begin + tokens_per_block < N ? t_begin + tokens_per_block : N;
-  const bool col_ok = c < d;
-  for (int e0 = 0; e0 < E; e0 += 32) {
-    const int ne = E - e0 < 32 ? E - e0 : 32;
-    float acc[32], wg[32];
+combine_dx_kernel(const __nv_bfloat16* __restrict__ dxs, const int32_t* __restrict__ row_of,
+                  const float* __restrict__ dl, const __nv_bfloat16* __restrict__ Wg, int64_t N, int d, int E, int k,
+                  __nv_bfloat16* __restrict__ dx) {
+  constexpr int kTok = 4;
+  const int pieces = d >> 3;
+  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t0 = item / pieces * kTok;
+  const int c = (int)(item % pieces) << 3;
+  pdl_wait();
+  if (t0 >= N) return;
+  float acc[kTok][8];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      acc[i] = 0.f;
-      wg[i] = (col_ok && i < ne) ? __bfloat162float(Wg[(size_t)(e0 + i) * d + c]) : 0.f;
-    }
-    float bsum = 0.f;   // thread i < ne of column block 0 sums dl[:, e0 + i]
-    for (int64_t t0 = t_begin; t0 < t_end; t0 += 64) {
-      const int nt = (int)(t_end - t0 < 64 ? t_end - t0 : 64);
-      __syncthreads();
-      for (int i = threadIdx.x; i < 64 * 32; i += 256) {
-        const int tl = i >> 5, el = i & 31;
-        s_dl[tl][el] = (tl < nt && el < ne) ? dl[(t0 + tl) * E + e0 + el] : 0.f;
+  for (int u = 0; u < kTok; ++u) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[u][i] = 0.f;
+    if (t0 + u < N)
+      for (int j = 0; j < k; ++j) {
+        const int row = row_of[(t0 + u) * k + j];
+        if (row < 0) continue;
+        float v[8];
+        load8(dxs + (int64_t)row * d + c, v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[u][i] += v[i];
       }
-      __syncthreads();
-      if (blockIdx.x == 0 && (int)threadIdx.x < ne)
-        for (int tl = 0; tl < nt; ++tl) bsum += s_dl[tl][threadIdx.x];
-      if (col_ok) {
-        for (int tl = 0; tl < nt; ++tl) {
-          const float xv = __bfloat162float(x[(t0 + tl) * d + c]);
-          float dx = 0.f;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float g = s_dl[tl][i];
-            acc[i] = fmaf(g, xv, acc[i]);
-            dx = fmaf(g, wg[i], dx);
-          }
-          // more than 32 experts: the sum over expert groups passes through the bf16 buffer
-          // (one extra rounding per group of 32 experts)
-          float prev = e0 == 0 ? 0.f : __bfloat162float(dxr[(t0 + tl) * d + c]);
-          dxr[(t0 + tl) * d + c] = __float2bfloat16_rn(prev + dx);
-        }
-      }
-    }
-    if (col_ok)
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (i < ne) atomicAdd(&dWg[(size_t)(e0 + i) * d + c], acc[i]);
-    if (blockIdx.x == 0 && (int)threadIdx.x < ne) atomicAdd(&dbg[e0 + threadIdx.x], bsum);
   }
+  for (int e = 0; e < E; ++e) {
+    float wv[8];
+    load8_ldg(Wg + (size_t)e * d + c, wv);
+#pragma unroll
+    for (int u = 0; u < kTok; ++u)
+      if (t0 + u < N) {
+        const float g = __ldg(&dl[(t0 + u) * E + e]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[u][i] = fmaf(g, wv[i], acc[u][i]);
+      }
+  }
+#pragma unroll
+  for (int u = 0; u < kTok; ++u)
+    if (t0 + u < N) store8(dx + (t0 + u) * d + c, acc[u]);
 }
 
 __global__ void iota_kernel(int32_t* __restrict__ p, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = (int32_t)i;
-}
-
-__global__ void f32_to_bf16_kernel(const float* __restrict__ src, int64_t n, __nv_bfloat16* __restrict__ dst) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = __float2bfloat16_rn(src[i]);
-}
-
-__global__ void fill_f32_kernel(float* __restrict__ p, int64_t n, float v) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
 }
 
 // Partial column sums: one block per 256-row tile of an expert (tiles counted over the experts in
@@ -311,47 +386,56 @@ int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, 
   return 0;
 }
 
+// Token ranges of router_bwd_kernel: about two blocks per SM, their partial sums at most 16 MB.
+static int64_t router_bwd_tokens(int64_t N, int d, int E) {
+  const int64_t groups = (int64_t)((d + kDlCols - 1) / kDlCols) * ((E + kDlExperts - 1) / kDlExperts);
+  int64_t ranges = (2 * kNumSMs + groups - 1) / groups;
+  const int64_t most = ((int64_t)16 << 20) / ((int64_t)E * d * 4);
+  if (ranges > most) ranges = most;
+  if (ranges < 1) ranges = 1;
+  const int64_t per = (N + ranges - 1) / ranges;
+  return (per + kDlTokens - 1) / kDlTokens * kDlTokens;
+}
+
+int64_t router_bwd_scratch_floats(int64_t N, int d, int E) {
+  const int64_t per = router_bwd_tokens(N > 0 ? N : 1, d, E);
+  return (N + per - 1) / per * ((int64_t)E * d + E);
+}
+
 int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, const float* dw,
-                      const int32_t* cnt0, float grad_aux, const float* grad_aux_dev, const void* x, const void* Wg,
-                      int64_t N, int d, int E, int k, float* dl, float* dWg_f32, float* dbg_f32, void* dWg,
-                      void* dbg, void* dxr, cudaStream_t s) {
+                      const int32_t* cnt0, float grad_aux, const float* grad_aux_dev, const void* x,
+                      int64_t N, int d, int E, int k, float* dl, float* scratch, void* dWg, void* dbg, cudaStream_t s) {
   if (N == 0) return 0;
-  router_bwd_kernel<<<blocks_for(N, 8), 256, 0, s>>>(logits, idx, w, dw, cnt0, grad_aux, grad_aux_dev, N, E, k, dl);
+  const int64_t per = router_bwd_tokens(N, d, E);
+  const int64_t ranges = (N + per - 1) / per;
+  float* part_b = scratch + (size_t)ranges * E * d;
+  auto fn = E <= 32 ? router_bwd_kernel<1> : (E <= 64 ? router_bwd_kernel<2> : router_bwd_kernel<kMaxExperts / 32>);
+  const dim3 grid((d + kDlCols - 1) / kDlCols, (unsigned)ranges, (E + kDlExperts - 1) / kDlExperts);
+  fn<<<grid, 256, 0, s>>>(logits, idx, w, dw, cnt0, grad_aux, grad_aux_dev, static_cast<const __nv_bfloat16*>(x), N, d,
+                          E, k, (int)per, dl, scratch, part_b);
   MOE_CUDA_CHECK(cudaGetLastError());
-  MOE_CUDA_CHECK(cudaMemsetAsync(dWg_f32, 0, sizeof(float) * (size_t)E * d, s));
-  MOE_CUDA_CHECK(cudaMemsetAsync(dbg_f32, 0, sizeof(float) * (size_t)E, s));
-  // about two token ranges per SM column block
-  int sms = 0;
-  int rc = sm_count(&sms);
-  if (rc) return rc;
-  const int col_blocks = (d + 255) / 256;
-  int64_t ranges = (2 * (int64_t)sms + col_blocks - 1) / col_blocks;
-  int64_t per = (N + ranges - 1) / ranges;
-  per = (per + 63) / 64 * 64;
-  ranges = (N + per - 1) / per;
-  router_bwd_wx_kernel<<<dim3(col_blocks, (unsigned)ranges), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(Wg), dl, N, d, E,
-      (int)per, dWg_f32, dbg_f32, static_cast<__nv_bfloat16*>(dxr));
+  if (dWg == nullptr && dbg == nullptr) return 0;
+  const int64_t n = (int64_t)E * d;
+  router_bwd_finish_kernel<<<blocks_for(n, 32) + 1, 256, 0, s>>>(scratch, part_b, (int)ranges, n, E,
+                                                                static_cast<__nv_bfloat16*>(dWg),
+                                                                static_cast<__nv_bfloat16*>(dbg));
   MOE_CUDA_CHECK(cudaGetLastError());
-  if (dWg != nullptr)
-    f32_to_bf16_kernel<<<blocks_for((int64_t)E * d, 256), 256, 0, s>>>(dWg_f32, (int64_t)E * d,
-                                                                       static_cast<__nv_bfloat16*>(dWg));
-  if (dbg != nullptr)
-    f32_to_bf16_kernel<<<blocks_for(E, 256), 256, 0, s>>>(dbg_f32, E, static_cast<__nv_bfloat16*>(dbg));
-  MOE_CUDA_CHECK(cudaGetLastError());
+  return 0;
+}
+
+int launch_combine_dx(const void* dxs, const int32_t* row_of, const float* dl, const void* Wg, int64_t N, int d, int E,
+                      int k, void* dx, cudaStream_t s) {
+  if (N == 0) return 0;
+  const int64_t items = (N + 3) / 4 * (d >> 3);
+  MOE_CUDA_CHECK(launch_pdl(combine_dx_kernel, dim3(blocks_for(items, 256)), dim3(256), 0, s,
+                            static_cast<const __nv_bfloat16*>(dxs), row_of, dl, static_cast<const __nv_bfloat16*>(Wg),
+                            N, d, E, k, static_cast<__nv_bfloat16*>(dx)));
   return 0;
 }
 
 int launch_iota(int32_t* p, int64_t n, cudaStream_t s) {
   if (n == 0) return 0;
   iota_kernel<<<blocks_for(n, 256), 256, 0, s>>>(p, n);
-  MOE_CUDA_CHECK(cudaGetLastError());
-  return 0;
-}
-
-int launch_fill_f32(float* p, int64_t n, float v, cudaStream_t s) {
-  if (n == 0) return 0;
-  fill_f32_kernel<<<blocks_for(n, 256), 256, 0, s>>>(p, n, v);
   MOE_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

@@ -350,15 +350,24 @@ int launch_experts_gemv(const void* perm, const int32_t* offsets, const void* pl
 int launch_pair_of(const int32_t* row_of, int64_t M, int32_t* pair_of, cudaStream_t s);
 int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, const float* w,
                        int64_t M, int d, int k, void* dy, float* dw, cudaStream_t s);
+int64_t router_bwd_scratch_floats(int64_t N, int d, int E);
 int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, const float* dw,
-                      const int32_t* cnt0, float grad_aux, const float* grad_aux_dev, const void* x, const void* Wg,
-                      int64_t N, int d, int E, int k, float* dl, float* dWg_f32, float* dbg_f32, void* dWg,
-                      void* dbg, void* dxr, cudaStream_t s);
-int launch_fill_f32(float* p, int64_t n, float v, cudaStream_t s);
+                      const int32_t* cnt0, float grad_aux, const float* grad_aux_dev, const void* x,
+                      int64_t N, int d, int E, int k, float* dl, float* scratch, void* dWg, void* dbg, cudaStream_t s);
+int launch_combine_dx(const void* dxs, const int32_t* row_of, const float* dl, const void* Wg, int64_t N, int d, int E,
+                      int k, void* dx, cudaStream_t s);
 int launch_iota(int32_t* p, int64_t n, cudaStream_t s);
 // Bias gradients: column sums of src [M, C] over every expert's rows; part as TrainArgs::col_part.
 int launch_colsum(const void* src, const int32_t* offsets, int64_t M, int E, int C, float* part, void* db,
                   cudaStream_t s);
 int launch_colsum_finish(const float* part, int slots, const int32_t* offsets, int E, int C, void* db, cudaStream_t s);
+
+// ---- lora_bwd.cu ----
+// LoRA gradients of both Linears of every expert (index 0: gate_and_up, 1: down) from the sorted activations and
+// their gradients; tab [2][E][3] device pointers A, a, B; g [E, out] gradients of the merged biases.
+int launch_lora_grads(const void* const* tab, const void* x, const void* dgu, const void* h, const void* dy,
+                      const int32_t* offsets, int64_t M, int d, int f, int E, int rank, float scale, float* scratch,
+                      const void* const (&g)[2], void* const (&dA)[2], void* const (&da)[2], void* const (&dB)[2],
+                      void* const (&db)[2], cudaStream_t s);
 
 }  // namespace moe

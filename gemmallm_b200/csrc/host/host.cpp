@@ -13,8 +13,12 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -167,6 +171,223 @@ class LoraJobs {
   std::vector<LoraJob> jobs_;
 };
 
+// ---- training -----------------------------------------------------------------------------------
+// The forward of a module under .train() as one autograd node, without Python on either way: the node keeps
+// what its backward needs (the prepared call, the input, the call's seed) and hands every gradient that is wanted
+// a place of its own, so that nothing is copied out of a workspace afterwards.
+
+using torch::autograd::Edge;
+using torch::autograd::edge_list;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+// What a prepared training call works on; shared by the module and the nodes of its calls.
+struct TrainCall {
+  Tensor ws, tws, offsets, status, lora_tab;    // buffers kept alive
+  const void* plan = nullptr;
+  void *ws_base = nullptr, *tws_base = nullptr;
+  size_t ws_bytes = 0, tws_bytes = 0;
+  int64_t N = 0;
+  int d = 0, f = 0, E = 0, k = 0, device = 0, rank = 0;
+  double lora_scale = 0.0;
+  int64_t gen = 0;          // number of forwards: a backward must belong to the last one
+};
+
+uint64_t draw_seed() {      // torch's CPU generator, as torch.randint(0, 2**62, (1,)) in Python
+  return (uint64_t)at::randint((int64_t)1 << 62, {1}, at::TensorOptions().dtype(at::kLong)).item<int64_t>();
+}
+
+void check_rc(int rc, const char* what) {
+  if (rc != 0)
+    throw std::runtime_error(std::string(what) + " failed with code " + std::to_string(rc) + ": " +
+                             moe_b200_last_error_string());
+}
+
+// Gradients of the experts' parameters: per expert w1, b1, w2, b2 and, with LoRA, weight and bias of
+// gate_and_up a, b and down a, b; `wanted(i)` says whether the i-th of them (counted over the experts) is.
+struct ExpertGrads {
+  Tensor w1, b1, w2, b2, scratch;
+  Tensor dA[2], da[2], dB[2], db[2];
+  int per = 4;
+
+  template <typename Wanted>
+  moe::LoraGrads prepare(const TrainCall& c, int64_t M, const at::TensorOptions& opt, moe::TrainGrads* g, Wanted wanted) {
+    const int64_t E = c.E, d = c.d, f = c.f;
+    per = c.rank > 0 ? 12 : 4;
+    bool need[12] = {};
+    for (int64_t e = 0; e < E; ++e)
+      for (int i = 0; i < per; ++i) need[i] |= wanted(e * per + i);
+    bool lora = false;
+    for (int i = 4; i < per; ++i) lora |= need[i];
+    if (need[0]) w1 = at::empty({E, 2 * f, d}, opt);
+    if (need[1] || lora) b1 = at::empty({E, 2 * f}, opt);
+    if (need[2]) w2 = at::empty({E, d, f}, opt);
+    if (need[3] || lora) b2 = at::empty({E, d}, opt);
+    auto ptr = [](Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
+    g->w1 = ptr(w1);
+    g->b1 = ptr(b1);
+    g->w2 = ptr(w2);
+    g->b2 = ptr(b2);
+    moe::LoraGrads lg = {};
+    if (lora) {
+      const int64_t in[2] = {d, f}, out[2] = {2 * f, d}, r = c.rank;
+      scratch = at::empty({(int64_t)moe::lora_grads_scratch_floats(M, c.d, c.f, c.E, c.rank)}, opt.dtype(at::kFloat));
+      lg.tab = static_cast<const void* const*>(c.lora_tab.const_data_ptr());
+      lg.rank = c.rank;
+      lg.scale = (float)c.lora_scale;
+      lg.scratch = scratch.data_ptr<float>();
+      for (int l = 0; l < 2; ++l) {
+        dA[l] = at::empty({E, r, in[l]}, opt);
+        da[l] = at::empty({E, r}, opt);
+        dB[l] = at::empty({E, out[l], r}, opt);
+        db[l] = at::empty({E, out[l]}, opt);
+        lg.dA[l] = dA[l].data_ptr();
+        lg.da[l] = da[l].data_ptr();
+        lg.dB[l] = dB[l].data_ptr();
+        lg.db[l] = db[l].data_ptr();
+      }
+    }
+    return lg;
+  }
+  template <typename Wanted>
+  void collect(int64_t E, variable_list* out, size_t first, Wanted wanted) {
+    Tensor* all[12] = {&w1, &b1, &w2, &b2, &dA[0], &da[0], &dB[0], &db[0], &dA[1], &da[1], &dB[1], &db[1]};
+    for (int64_t e = 0; e < E; ++e)
+      for (int i = 0; i < per; ++i)
+        if (wanted(e * per + i)) (*out)[first + e * per + i] = all[i]->select(0, e);
+  }
+};
+
+Tensor output_grad(const Tensor& g, const Tensor& like) {
+  if (!g.defined()) return at::zeros_like(like);
+  return g.to(like.scalar_type()).contiguous();
+}
+
+void check_generation(const TrainCall& c, int64_t gen) {
+  if (c.gen != gen)
+    throw std::runtime_error("this module ran another training forward before the backward of this one: its "
+                             "workspace holds the later call's tensors");
+}
+
+// inputs: x, residual (an empty edge without one), gate weight, gate bias, the experts' parameters
+struct BlockBackward : public Node {
+  std::shared_ptr<TrainCall> call;
+  SavedVariable x;
+  Tensor gate_w;
+  int64_t gen = 0;
+  uint64_t seed = 0;
+  double p = 0.0;
+
+  std::string name() const override { return "MOEBackward"; }
+  void release_variables() override { x.reset_data(); }
+  variable_list apply(variable_list&& grads) override {
+    const TrainCall& c = *call;
+    check_generation(c, gen);
+    at::AutoGradMode no_grad(false);
+    const Tensor xv = x.unpack();
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)c.device);
+    void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c.device).stream();
+    const Tensor go = output_grad(grads[0], xv);
+    Tensor aux = grads[1];
+    if (aux.defined()) aux = aux.to(xv.options().dtype(at::kFloat)).contiguous();
+    variable_list out(next_edges().size());
+    const auto opt = xv.options();
+    moe::TrainGrads g = {};
+    Tensor gx, gwg, gbg;
+    if (task_should_compute_output(0)) gx = at::empty(xv.sizes(), opt);
+    if (task_should_compute_output(2)) gwg = at::empty({c.E, c.d}, opt);
+    if (task_should_compute_output(3)) gbg = at::empty({c.E}, opt);
+    g.x = gx.defined() ? gx.data_ptr() : nullptr;
+    g.wg = gwg.defined() ? gwg.data_ptr() : nullptr;
+    g.bg = gbg.defined() ? gbg.data_ptr() : nullptr;
+    auto wanted = [&](int64_t i) { return task_should_compute_output(4 + (size_t)i); };
+    ExpertGrads eg;
+    const moe::LoraGrads lg = eg.prepare(c, c.N * c.k, opt, &g, wanted);
+    if (c.N > 0) {
+      check_rc(moe::backward_into(xv.const_data_ptr(), gate_w.const_data_ptr(), c.plan, go.const_data_ptr(), 0.f,
+                                  aux.defined() ? aux.const_data_ptr<float>() : nullptr, c.N, c.d, c.f, c.E, c.k,
+                                  MOE_B200_BF16, (float)p, seed, c.ws_base, c.ws_bytes, c.tws_base, c.tws_bytes, g,
+                                  lg.tab != nullptr ? &lg : nullptr, stream),
+               "backward");
+    } else {
+      for (Tensor* t : {&gwg, &gbg, &eg.w1, &eg.b1, &eg.w2, &eg.b2, &eg.dA[0], &eg.da[0], &eg.dB[0], &eg.db[0], &eg.dA[1],
+                        &eg.da[1], &eg.dB[1], &eg.db[1]})
+        if (t->defined()) t->zero_();
+    }
+    out[0] = gx;
+    if (task_should_compute_output(1)) out[1] = grads[0].defined() ? grads[0] : go;
+    out[2] = gwg;
+    out[3] = gbg;
+    eg.collect(c.E, &out, 4, wanted);
+    return out;
+  }
+};
+
+// inputs: x, the parameters
+struct FfnBackward : public Node {
+  std::shared_ptr<TrainCall> call;
+  SavedVariable x;
+  Tensor h;
+  int64_t gen = 0;
+  uint64_t seed = 0;
+  double p = 0.0;
+
+  std::string name() const override { return "FeedForwardBackward"; }
+  void release_variables() override {
+    x.reset_data();
+    h.reset();
+  }
+  variable_list apply(variable_list&& grads) override {
+    const TrainCall& c = *call;
+    check_generation(c, gen);
+    at::AutoGradMode no_grad(false);
+    const Tensor xv = x.unpack();
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)c.device);
+    void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c.device).stream();
+    const Tensor go = output_grad(grads[0], xv);
+    variable_list out(next_edges().size());
+    const auto opt = xv.options();
+    moe::TrainGrads g = {};
+    Tensor gx;
+    if (task_should_compute_output(0)) gx = at::empty(xv.sizes(), opt);
+    g.x = gx.defined() ? gx.data_ptr() : nullptr;
+    auto wanted = [&](int64_t i) { return task_should_compute_output(1 + (size_t)i); };
+    ExpertGrads eg;
+    const moe::LoraGrads lg = eg.prepare(c, c.N, opt, &g, wanted);
+    if (c.N > 0) {
+      check_rc(moe::experts_backward_into(xv.const_data_ptr(), h.const_data_ptr(), c.offsets.const_data_ptr<int32_t>(),
+                                          c.plan, go.const_data_ptr(), c.N, c.d, c.f, 1, (float)p, seed, c.tws_base,
+                                          c.tws_bytes, g, lg.tab != nullptr ? &lg : nullptr,
+                                          c.status.data_ptr<int32_t>(), stream),
+               "experts_backward");
+    } else {
+      for (Tensor* t : {&eg.w1, &eg.b1, &eg.w2, &eg.b2, &eg.dA[0], &eg.da[0], &eg.dB[0], &eg.db[0], &eg.dA[1], &eg.da[1],
+                        &eg.dB[1], &eg.db[1]})
+        if (t->defined()) t->zero_();
+    }
+    out[0] = gx;
+    eg.collect(1, &out, 1, wanted);
+    return out;
+  }
+};
+
+// Edges of a call's inputs; false when none of them wants a gradient (or gradients are off).
+class Edges {
+ public:
+  void add(const Tensor& t) {
+    any_ |= t.requires_grad();
+    list_.push_back(torch::autograd::impl::gradient_edge(t));
+  }
+  void add_empty() { list_.emplace_back(); }
+  bool wanted() const { return any_ && at::GradMode::is_enabled(); }
+  edge_list take() { return std::move(list_); }
+
+ private:
+  edge_list list_;
+  bool any_ = false;
+};
+
 at::ScalarType scalar_of(int dtype) { return dtype == MOE_B200_BF16 ? at::kBFloat16 : at::kFloat; }
 
 // ---- the Mixture-of-Experts block ------------------------------------------------------------
@@ -176,6 +397,7 @@ struct Block {
   WatchList* watch;       // [0], [1]: the router's weight and bias, then the experts' tensors
   LoraJobs* lora;
   Tensor* workspace;
+  std::shared_ptr<TrainCall>* train;
   const void* plan;
   void* ws_base;
   size_t ws_bytes;
@@ -219,6 +441,7 @@ PyObject* block_new(PyTypeObject* type, PyObject*, PyObject*) {
   self->watch = new WatchList();
   self->lora = new LoraJobs();
   self->workspace = new Tensor();
+  self->train = new std::shared_ptr<TrainCall>();
   return reinterpret_cast<PyObject*>(self);
 }
 
@@ -228,6 +451,7 @@ void block_dealloc(PyObject* o) {
   delete self->watch;
   delete self->lora;
   delete self->workspace;
+  delete self->train;
   type->tp_free(o);
   Py_DECREF(type);
 }
@@ -270,7 +494,39 @@ PyObject* block_unbind(PyObject* o, PyObject*) {
   Block* self = reinterpret_cast<Block*>(o);
   self->watch->clear();
   *self->workspace = Tensor();
+  self->train->reset();
   Py_RETURN_NONE;
+}
+
+// bind_train(training workspace, base, bytes, LoRA pointer table or None, rank, scale): after bind()
+PyObject* block_bind_train(PyObject* o, PyObject* args) {
+  HANDLE_TH_ERRORS
+  Block* self = reinterpret_cast<Block*>(o);
+  PyObject *tws, *tab;
+  unsigned long long base, bytes;
+  int rank;
+  double scale;
+  if (!PyArg_ParseTuple(args, "OKKOid", &tws, &base, &bytes, &tab, &rank, &scale)) return nullptr;
+  auto c = std::make_shared<TrainCall>();
+  c->ws = *self->workspace;
+  c->tws = THPVariable_Unpack(tws);
+  if (tab != Py_None) c->lora_tab = THPVariable_Unpack(tab);
+  c->plan = self->plan;
+  c->ws_base = self->ws_base;
+  c->ws_bytes = self->ws_bytes;
+  c->tws_base = reinterpret_cast<void*>(base);
+  c->tws_bytes = (size_t)bytes;
+  c->N = self->N;
+  c->d = self->d;
+  c->f = self->f;
+  c->E = self->E;
+  c->k = self->k;
+  c->device = self->device;
+  c->rank = rank;
+  c->lora_scale = scale;
+  *self->train = std::move(c);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
 }
 
 // a contiguous tensor of the bound device, dtype and row width with n rows
@@ -323,12 +579,101 @@ PyObject* block_forward(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// train(tensor, residual or None, dropout p, parameters or None) -> (out, loss, seed), or None: prepare again.
+// Without a list the parameters are the watched ones.
+PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  Block* self = reinterpret_cast<Block*>(o);
+  if (nargs != 4) {
+    PyErr_SetString(PyExc_TypeError, "train(tensor, residual, p, parameters)");
+    return nullptr;
+  }
+  if (*self->train == nullptr || !THPVariable_Check(args[0])) Py_RETURN_NONE;
+  const std::shared_ptr<TrainCall> c = *self->train;
+  const Tensor& x = THPVariable_Unpack(args[0]);
+  if (!rows_match(x, c->device, MOE_B200_BF16, c->d, c->N)) Py_RETURN_NONE;
+  const bool has_res = args[1] != Py_None;
+  if (has_res && !THPVariable_Check(args[1])) Py_RETURN_NONE;
+  Tensor res;
+  if (has_res) {
+    res = THPVariable_Unpack(args[1]);
+    if (!rows_match(res, c->device, MOE_B200_BF16, c->d, c->N) || res.sizes() != x.sizes()) Py_RETURN_NONE;
+  }
+  const double p = PyFloat_AsDouble(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  Edges edges;
+  edges.add(x);
+  if (has_res) edges.add(res); else edges.add_empty();
+  Tensor gate_w, gate_b;
+  if (args[3] == Py_None) {
+    if (self->watch->empty() || !self->watch->unchanged()) Py_RETURN_NONE;
+    gate_w = self->watch->param(0);
+    gate_b = self->watch->param(1);
+    for (int i = 0; i < self->watch->num_params(); ++i) edges.add(self->watch->param(i));
+  } else {
+    const Py_ssize_t n = PyList_Size(args[3]);
+    if (n < 2) {
+      PyErr_SetString(PyExc_TypeError, "parameters must be a list");
+      return nullptr;
+    }
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      PyObject* v = PyList_GET_ITEM(args[3], i);
+      if (!THPVariable_Check(v)) {
+        PyErr_SetString(PyExc_TypeError, "parameters must be tensors");
+        return nullptr;
+      }
+      edges.add(THPVariable_Unpack(v));
+    }
+    gate_w = THPVariable_Unpack(PyList_GET_ITEM(args[3], 0));
+    gate_b = THPVariable_Unpack(PyList_GET_ITEM(args[3], 1));
+  }
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)c->device);
+  void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c->device).stream();
+  if (args[3] == Py_None) {
+    const int rc = self->lora->refresh(*self->watch, MOE_B200_BF16, stream);
+    if (rc != 0) return fail(rc, "lora_merge");
+  }
+  const uint64_t seed = draw_seed();
+  Tensor out, aux;
+  {
+    at::AutoGradMode no_grad(false);
+    out = at::empty(x.sizes(), x.options());
+    aux = c->N > 0 ? at::empty({}, x.options().dtype(at::kFloat)) : at::zeros({}, x.options().dtype(at::kFloat));
+    const int rc = moe::forward_train_into(
+        x.const_data_ptr(), gate_w.const_data_ptr(), gate_b.const_data_ptr(), c->plan,
+        has_res ? res.const_data_ptr() : nullptr, c->N, c->d, c->f, c->E, c->k, MOE_B200_BF16, (float)p, seed, c->ws_base,
+        c->ws_bytes, c->tws_base, c->tws_bytes, out.data_ptr(), aux.data_ptr<float>(), stream);
+    if (rc != 0) return fail(rc, "forward_train");
+  }
+  ++c->gen;
+  if (edges.wanted()) {
+    auto node = std::shared_ptr<BlockBackward>(new BlockBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(edges.take());
+    node->call = c;
+    node->gen = c->gen;
+    node->seed = seed;
+    node->p = p;
+    node->gate_w = gate_w.detach();
+    node->x = SavedVariable(x, false);
+    torch::autograd::set_history({out, aux}, node);
+  }
+  PyObject* t = PyTuple_New(3);
+  if (t == nullptr) return nullptr;
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(out)));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(aux)));
+  PyTuple_SET_ITEM(t, 2, PyLong_FromUnsignedLongLong(seed));
+  return t;
+  END_HANDLE_TH_ERRORS
+}
+
 // a copy or an unpickled module starts unbound
 PyObject* fresh_reduce(PyObject* o, PyObject*) { return Py_BuildValue("O()", (PyObject*)Py_TYPE(o)); }
 
 PyMethodDef block_methods[] = {
     {"bind", block_bind, METH_VARARGS, nullptr},
     {"unbind", block_unbind, METH_NOARGS, nullptr},
+    {"bind_train", block_bind_train, METH_VARARGS, nullptr},
+    {"train", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(block_train)), METH_FASTCALL, nullptr},
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(block_forward)), METH_FASTCALL, nullptr},
     {"__reduce__", fresh_reduce, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr}};
@@ -346,6 +691,7 @@ struct Ffn {
   LoraJobs* lora;
   Tensor* offsets;        // int32 [0, M]
   Tensor* status;         // int32 [16], written only when a wait inside a kernel ran out
+  std::shared_ptr<TrainCall>* train;
   const void* plan;
   int64_t M;
   int d, f, dtype, device;
@@ -358,6 +704,7 @@ PyObject* ffn_new(PyTypeObject* type, PyObject*, PyObject*) {
   self->lora = new LoraJobs();
   self->offsets = new Tensor();
   self->status = new Tensor();
+  self->train = new std::shared_ptr<TrainCall>();
   return reinterpret_cast<PyObject*>(self);
 }
 
@@ -368,6 +715,7 @@ void ffn_dealloc(PyObject* o) {
   delete self->lora;
   delete self->offsets;
   delete self->status;
+  delete self->train;
   type->tp_free(o);
   Py_DECREF(type);
 }
@@ -405,7 +753,106 @@ PyObject* ffn_bind(PyObject* o, PyObject* args) {
 
 PyObject* ffn_unbind(PyObject* o, PyObject*) {
   reinterpret_cast<Ffn*>(o)->watch->clear();
+  reinterpret_cast<Ffn*>(o)->train->reset();
   Py_RETURN_NONE;
+}
+
+// bind_train(training workspace, base, bytes, LoRA pointer table or None, rank, scale): after bind()
+PyObject* ffn_bind_train(PyObject* o, PyObject* args) {
+  HANDLE_TH_ERRORS
+  Ffn* self = reinterpret_cast<Ffn*>(o);
+  PyObject *tws, *tab;
+  unsigned long long base, bytes;
+  int rank;
+  double scale;
+  if (!PyArg_ParseTuple(args, "OKKOid", &tws, &base, &bytes, &tab, &rank, &scale)) return nullptr;
+  auto c = std::make_shared<TrainCall>();
+  c->tws = THPVariable_Unpack(tws);
+  c->offsets = *self->offsets;
+  c->status = *self->status;
+  if (tab != Py_None) c->lora_tab = THPVariable_Unpack(tab);
+  c->plan = self->plan;
+  c->tws_base = reinterpret_cast<void*>(base);
+  c->tws_bytes = (size_t)bytes;
+  c->N = self->M;
+  c->d = self->d;
+  c->f = self->f;
+  c->E = 1;
+  c->k = 1;
+  c->device = self->device;
+  c->rank = rank;
+  c->lora_scale = scale;
+  *self->train = std::move(c);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// train(tensor, dropout p, parameters or None) -> (y, seed), or None: prepare again
+PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  Ffn* self = reinterpret_cast<Ffn*>(o);
+  if (nargs != 3) {
+    PyErr_SetString(PyExc_TypeError, "train(tensor, p, parameters)");
+    return nullptr;
+  }
+  if (*self->train == nullptr || !THPVariable_Check(args[0])) Py_RETURN_NONE;
+  const std::shared_ptr<TrainCall> c = *self->train;
+  const Tensor& x = THPVariable_Unpack(args[0]);
+  if (!rows_match(x, c->device, MOE_B200_BF16, c->d, c->N)) Py_RETURN_NONE;
+  const double p = PyFloat_AsDouble(args[1]);
+  if (PyErr_Occurred()) return nullptr;
+  Edges edges;
+  edges.add(x);
+  if (args[2] == Py_None) {
+    if (self->watch->empty() || !self->watch->unchanged()) Py_RETURN_NONE;
+    for (int i = 0; i < self->watch->num_params(); ++i) edges.add(self->watch->param(i));
+  } else {
+    const Py_ssize_t n = PyList_Size(args[2]);
+    if (n < 0) return nullptr;
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      PyObject* v = PyList_GET_ITEM(args[2], i);
+      if (!THPVariable_Check(v)) {
+        PyErr_SetString(PyExc_TypeError, "parameters must be tensors");
+        return nullptr;
+      }
+      edges.add(THPVariable_Unpack(v));
+    }
+  }
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)c->device);
+  void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c->device).stream();
+  if (args[2] == Py_None) {
+    const int rc = self->lora->refresh(*self->watch, MOE_B200_BF16, stream);
+    if (rc != 0) return fail(rc, "lora_merge");
+  }
+  const uint64_t seed = draw_seed();
+  Tensor h, y;
+  {
+    at::AutoGradMode no_grad(false);
+    h = at::empty({c->N, c->f}, x.options());
+    y = at::empty(x.sizes(), x.options());
+    const int rc = moe_b200_experts_train(x.const_data_ptr(), c->offsets.const_data_ptr<int32_t>(), c->plan, c->N, c->d,
+                                          c->f, 1, (float)p, seed, c->tws_base, c->tws_bytes, h.data_ptr(), y.data_ptr(),
+                                          c->status.data_ptr<int32_t>(), stream);
+    if (rc != 0) return fail(rc, "experts_train");
+  }
+  ++c->gen;
+  if (edges.wanted()) {
+    auto node = std::shared_ptr<FfnBackward>(new FfnBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(edges.take());
+    node->call = c;
+    node->gen = c->gen;
+    node->seed = seed;
+    node->p = p;
+    node->h = std::move(h);
+    node->x = SavedVariable(x, false);
+    torch::autograd::set_history(y, node);
+  }
+  PyObject* t = PyTuple_New(2);
+  if (t == nullptr) return nullptr;
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(y)));
+  PyTuple_SET_ITEM(t, 1, PyLong_FromUnsignedLongLong(seed));
+  return t;
+  END_HANDLE_TH_ERRORS
 }
 
 // forward(tensor) -> y, or None: prepare again
@@ -436,6 +883,8 @@ PyObject* ffn_forward(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
 PyMethodDef ffn_methods[] = {
     {"bind", ffn_bind, METH_VARARGS, nullptr},
     {"unbind", ffn_unbind, METH_NOARGS, nullptr},
+    {"bind_train", ffn_bind_train, METH_VARARGS, nullptr},
+    {"train", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(ffn_train)), METH_FASTCALL, nullptr},
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(ffn_forward)), METH_FASTCALL, nullptr},
     {"__reduce__", fresh_reduce, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr}};

@@ -19,6 +19,17 @@ struct TrainGrads {
   void *w1, *b1, *w2, *b2;   // experts [E, 2f, d], [E, 2f], [E, d, f], [E, d]
 };
 
+// LoRA gradients of both Linears (0: gate_and_up, 1: down) of all experts; the bias gradients b1 and b2 of
+// TrainGrads are needed with them.
+struct LoraGrads {
+  const void* const* tab;    // device [2][E][3]: A, a, B of every expert
+  int rank;
+  float scale;
+  float* scratch;            // lora_grads_scratch_floats() floats
+  void *dA[2], *da[2], *dB[2], *db[2];   // [E, rank, in], [E, rank], [E, out, rank], [E, out]
+};
+size_t lora_grads_scratch_floats(int64_t M, int d, int f, int E, int rank);
+
 // moe_b200_forward_train with the load-balancing loss written to `aux` (nullptr: the workspace's word).
 int forward_train_into(const void* x, const void* Wg, const void* bg, const void* plan, const void* residual,
                        int64_t N, int d, int f, int E, int k, int dtype, float dropout_p, uint64_t seed,
@@ -29,11 +40,11 @@ int forward_train_into(const void* x, const void* Wg, const void* bg, const void
 int backward_into(const void* x, const void* Wg, const void* plan, const void* grad_out, float grad_aux,
                   const float* grad_aux_dev, int64_t N, int d, int f, int E, int k, int dtype, float dropout_p,
                   uint64_t seed, void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes,
-                  const TrainGrads& grads, void* stream);
+                  const TrainGrads& grads, const LoraGrads* lora, void* stream);
 // moe_b200_experts_backward likewise (grads.wg and grads.bg are not used).
 int experts_backward_into(const void* x_sorted, const void* h, const int32_t* offsets, const void* plan,
                           const void* grad_y, int64_t M, int d, int f, int E, float dropout_p, uint64_t seed,
-                          void* train_ws, size_t train_ws_bytes, const TrainGrads& grads, int32_t* status,
-                          void* stream);
+                          void* train_ws, size_t train_ws_bytes, const TrainGrads& grads, const LoraGrads* lora,
+                          int32_t* status, void* stream);
 
 }  // namespace moe

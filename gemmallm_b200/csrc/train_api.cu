@@ -29,9 +29,7 @@ void tws_layout(int64_t N, int d, int f, int E, int k, size_t* off, size_t* tota
   sizes[MOE_B200_TWS_DXS] = M * d * 2;
   sizes[MOE_B200_TWS_DL] = (size_t)N * E * sizeof(float);
   sizes[MOE_B200_TWS_DW] = M * sizeof(float);
-  sizes[MOE_B200_TWS_ONES] = M * sizeof(float);
-  sizes[MOE_B200_TWS_DWG_F32] = ((size_t)E * d + E) * sizeof(float);
-  sizes[MOE_B200_TWS_DXR] = (size_t)N * d * 2;
+  sizes[MOE_B200_TWS_DWG_F32] = (size_t)router_bwd_scratch_floats(N, d, E) * sizeof(float);
   sizes[MOE_B200_TWS_G_WG] = (size_t)E * d * 2;
   sizes[MOE_B200_TWS_G_BG] = (size_t)E * 2;
   sizes[MOE_B200_TWS_G_W1] = (size_t)E * 2 * f * d * 2;
@@ -69,8 +67,8 @@ TrainArgs train_args(char* tws, const size_t* to, float p, uint64_t seed) {
 // h (the dropped h of the forward), the saved pre-activations and the sorted inputs, writes g.x (gradient of the
 // sorted inputs) and the four parameter gradients.
 int experts_backward(const void* perm, const void* h, const int32_t* offsets, const void* plan, const void* dy,
-                     int64_t M, int d, int f, int E, const TrainArgs& tr, const TrainGrads& g, int32_t* status,
-                     cudaStream_t s) {
+                     int64_t M, int d, int f, int E, const TrainArgs& tr, const TrainGrads& g, const LoraGrads* lora,
+                     int32_t* status, cudaStream_t s) {
   const PlanView pv = plan_view(plan, E);
   int rc;
   // down Linear (model.py:184): db2 = column sums of dy, dW2 = dy^T h, dh = dy W2; the last one goes back
@@ -83,12 +81,19 @@ int experts_backward(const void* perm, const void* h, const int32_t* offsets, co
     rc = launch_grouped_wgrad(dy, h, M, d, f, offsets, g.w2, E, status, s);
     if (rc) return rc;
   }
-  if (g.x == nullptr && g.w1 == nullptr && g.b1 == nullptr) return 0;
+  if (g.x == nullptr && g.w1 == nullptr && g.b1 == nullptr) return 0;   // (LoRA gradients need b1)
   rc = launch_grouped_dx(dy, M, d, pv.tmap_W2_dec, offsets, E, f, nullptr, &tr, status, s);
   if (rc) return rc;
   // gate_and_up Linear (model.py:174): db1 = column sums of dgu, dx = dgu W1, dW1 = dgu^T x
   if (g.b1 != nullptr) {
     rc = launch_colsum_finish(tr.col_part, 2, offsets, E, 2 * f, g.b1, s);
+    if (rc) return rc;
+  }
+  if (lora != nullptr) {
+    if (g.b1 == nullptr || g.b2 == nullptr) return set_error(MOE_B200_ERR_NULL, "LoRA gradients need b1 and b2");
+    const void* const gb[2] = {g.b1, g.b2};
+    rc = launch_lora_grads(lora->tab, perm, tr.gu, h, dy, offsets, M, d, f, E, lora->rank, lora->scale, lora->scratch,
+                           gb, lora->dA, lora->da, lora->dB, lora->db, s);
     if (rc) return rc;
   }
   if (g.x != nullptr) {
@@ -137,8 +142,8 @@ int moe_b200_train_setup(int64_t N, int d, int f, int E, int k, int dtype, void*
   tws_layout(N, d, f, E, k, to, &total);
   if (train_ws_bytes < total) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
   if ((uintptr_t)train_ws & 1023) return set_error(MOE_B200_ERR_ALIGN, "training workspace must be 1024-byte aligned");
-  char* tws = static_cast<char*>(train_ws);
-  return launch_fill_f32(reinterpret_cast<float*>(tws + to[MOE_B200_TWS_ONES]), N * (int64_t)k, 1.0f, (cudaStream_t)stream);
+  (void)stream;
+  return 0;
 }
 
 int moe_b200_forward_train(const void* x, const void* Wg, const void* bg, const void* plan,
@@ -161,7 +166,7 @@ int moe_b200_backward(const void* x, const void* Wg, const void* plan, const voi
   tws_layout(N, d, f, E, k, to, &ttotal);
   return backward_into(x, Wg, plan, grad_out, grad_aux, nullptr, N, d, f, E, k, dtype, dropout_p, seed, workspace,
                        workspace_bytes, train_ws, train_ws_bytes,
-                       own_grads(static_cast<char*>(train_ws), to, grad_x), stream);
+                       own_grads(static_cast<char*>(train_ws), to, grad_x), nullptr, stream);
 }
 
 // ---- the expert feed-forward alone (the reference's dense FeedForward, model.py:154-190, is one
@@ -199,7 +204,8 @@ int moe_b200_experts_backward(const void* x_sorted, const void* h, const int32_t
   size_t to[MOE_B200_TWS_NUM], ttotal;
   tws_layout(M, d, f, E, 1, to, &ttotal);
   return experts_backward_into(x_sorted, h, offsets, plan, grad_y, M, d, f, E, dropout_p, seed, train_ws,
-                               train_ws_bytes, own_grads(static_cast<char*>(train_ws), to, grad_x), status, stream);
+                               train_ws_bytes, own_grads(static_cast<char*>(train_ws), to, grad_x), nullptr, status,
+                               stream);
 }
 
 }  // extern "C"
@@ -259,7 +265,7 @@ int forward_train_into(const void* x, const void* Wg, const void* bg, const void
 int backward_into(const void* x, const void* Wg, const void* plan, const void* grad_out, float grad_aux,
                   const float* grad_aux_dev, int64_t N, int d, int f, int E, int k, int dtype, float dropout_p,
                   uint64_t seed, void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes,
-                  const TrainGrads& grads, void* stream) {
+                  const TrainGrads& grads, const LoraGrads* lora, void* stream) {
   int rc = train_check(N, d, f, E, k, dtype, dropout_p);
   if (rc) return rc;
   if (!workspace || !train_ws) return set_error(MOE_B200_ERR_NULL, "workspace is NULL");
@@ -292,32 +298,30 @@ int backward_into(const void* x, const void* Wg, const void* plan, const void* g
   void* dxs = tws + to[MOE_B200_TWS_DXS];
   float* dl = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DL]);
   float* dw = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DW]);
-  const float* ones = reinterpret_cast<const float*>(tws + to[MOE_B200_TWS_ONES]);
   float* dwg32 = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DWG_F32]);
-  void* dxr = tws + to[MOE_B200_TWS_DXR];
   const TrainArgs tr = train_args(tws, to, dropout_p, seed);
 
   // combine (model.py:271) and router (model.py:206-223)
   rc = launch_combine_bwd(grad_out, y, tr.pair_of, w, M, d, k, dy, dw, s);
   if (rc) return rc;
   if (grads.x != nullptr || grads.wg != nullptr || grads.bg != nullptr) {
-    rc = launch_router_bwd(logits, idx, w, dw, cnt_slot, grad_aux, grad_aux_dev, x, Wg, N, d, E, k, dl, dwg32,
-                           dwg32 + (size_t)E * d, grads.wg, grads.bg, dxr, s);
+    rc = launch_router_bwd(logits, idx, w, dw, cnt_slot, grad_aux, grad_aux_dev, x, N, d, E, k, dl, dwg32, grads.wg,
+                           grads.bg, s);
     if (rc) return rc;
   }
   // the experts (model.py:174-184)
   TrainGrads eg = grads;
   eg.x = grads.x != nullptr ? dxs : nullptr;
-  rc = experts_backward(perm, h, offsets, plan, dy, M, d, f, E, tr, eg, status, s);
+  rc = experts_backward(perm, h, offsets, plan, dy, M, d, f, E, tr, eg, lora, status, s);
   if (rc || grads.x == nullptr) return rc;
-  // gather (model.py:248-253) and the router's share: dx[t] = sum_j dxs[row_of[t,j]] + dxr[t]
-  return launch_combine(dxs, row_of, ones, dxr, N, d, k, dtype, grads.x, s);
+  // gather (model.py:248-253) and the router's share
+  return launch_combine_dx(dxs, row_of, dl, Wg, N, d, E, k, grads.x, s);
 }
 
 int experts_backward_into(const void* x_sorted, const void* h, const int32_t* offsets, const void* plan,
                           const void* grad_y, int64_t M, int d, int f, int E, float dropout_p, uint64_t seed,
-                          void* train_ws, size_t train_ws_bytes, const TrainGrads& grads, int32_t* status,
-                          void* stream) {
+                          void* train_ws, size_t train_ws_bytes, const TrainGrads& grads, const LoraGrads* lora,
+                          int32_t* status, void* stream) {
   int rc = train_check(M, d, f, E, 1, MOE_B200_BF16, dropout_p);
   if (rc) return rc;
   if (M == 0) return 0;
@@ -329,7 +333,8 @@ int experts_backward_into(const void* x_sorted, const void* h, const int32_t* of
   tws_layout(M, d, f, E, 1, to, &ttotal);
   if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
   const TrainArgs tr = train_args(static_cast<char*>(train_ws), to, dropout_p, seed);
-  return experts_backward(x_sorted, h, offsets, plan, grad_y, M, d, f, E, tr, grads, status, (cudaStream_t)stream);
+  return experts_backward(x_sorted, h, offsets, plan, grad_y, M, d, f, E, tr, grads, lora, status,
+                          (cudaStream_t)stream);
 }
 
 }  // namespace moe

@@ -112,23 +112,18 @@ class _MergedLora:
         return self.merged
 
 
-def _lora_grads(ex, g_w1, g_b1, g_w2, g_b2):
-    """Gradients of an expert's four LoRA Linears (weight, bias each, in the order
-    gate_and_up a, b, down a, b) from the gradients G = dL/dW', g = dL/db' of its two merged
-    Linears W' = W + s B A, b' = b + s (B a + b_lora) (model.py:175-179,185-189):
-    dL/dA = s B^T G, dL/da = s B^T g, dL/dB = s (G A^T + g a^T), dL/db_lora = s g."""
-    out = []
-    s = float(ex.lora_scale)
-    with torch.no_grad():
-        for G, g, a, b in ((g_w1, g_b1, ex.lora_gate_and_up_a, ex.lora_gate_and_up_b),
-                           (g_w2, g_b2, ex.lora_down_a, ex.lora_down_b)):
-            Gf, gf = G.float(), g.float()
-            Af, af, Bf = a.weight.float(), a.bias.float(), b.weight.float()
-            dA = (Bf.t() @ Gf).mul_(s)
-            da = (Bf.t() @ gf).mul_(s)
-            dB = (Gf @ Af.t()).addr_(gf, af).mul_(s)
-            out += [dA.to(G.dtype), da.to(G.dtype), dB.to(G.dtype), (gf * s).to(G.dtype)]
-    return out
+def _lora_table(experts, dev) -> torch.Tensor:
+    """Device table of the LoRA tensors' addresses, [2 Linears][experts][A, a, B], for their gradients."""
+    rows = [[p.data_ptr() for p in (a.weight, a.bias, b.weight)]
+            for pair in (("lora_gate_and_up_a", "lora_gate_and_up_b"), ("lora_down_a", "lora_down_b"))
+            for a, b in ((getattr(ex, pair[0]), getattr(ex, pair[1])) for ex in experts)]
+    return torch.tensor(rows, dtype=torch.int64).to(dev)
+
+
+def _expert_params(ex, fine_tuning: bool) -> list:
+    """The tensors an expert's gradients belong to, in the order of _LORA_NAMES."""
+    return [p for n in (_LORA_NAMES if fine_tuning else _LORA_NAMES[:2])
+            for p in (getattr(ex, n).weight, getattr(ex, n).bias)]
 
 
 class _Plan:
@@ -165,55 +160,6 @@ class _Plan:
         return self.base
 
 
-class _TrainFn(torch.autograd.Function):
-    """MOE.forward in training mode as one autograd node: moe_b200_forward_train /
-    moe_b200_backward (dropout on h, model.py:183; gradients of model.py:200-276)."""
-
-    @staticmethod
-    def forward(ctx, module, x, residual, seed, fine_tuning, *params):
-        out, aux = module._forward_train(x, residual, seed, fine_tuning)
-        ctx.module, ctx.seed, ctx.gen = module, seed, module._train_gen
-        ctx.fine_tuning = fine_tuning
-        ctx.has_residual = residual is not None
-        ctx.save_for_backward(x)
-        return out, aux
-
-    @staticmethod
-    def backward(ctx, grad_out, grad_aux):
-        m = ctx.module
-        if ctx.gen != m._train_gen:
-            raise RuntimeError("this block ran another training forward before the backward of this "
-                               "one: its workspace holds the later call's tensors")
-        (x,) = ctx.saved_tensors
-        grads = m._backward_train(x, grad_out.contiguous(), float(grad_aux), ctx.seed, ctx.fine_tuning)
-        grad_x = grads.pop(0)
-        grad_res = grad_out if ctx.has_residual else None
-        return (None, grad_x, grad_res, None, None, *grads)
-
-
-class _FfnTrainFn(torch.autograd.Function):
-    """FeedForward.forward in training mode as one autograd node (moe_b200_experts_train /
-    moe_b200_experts_backward: dropout on h, model.py:183; gradients of model.py:173-184)."""
-
-    @staticmethod
-    def forward(ctx, module, x, seed, fine_tuning, *params):
-        y, h = module._forward_train(x, seed, fine_tuning)
-        ctx.module, ctx.seed, ctx.gen = module, seed, module._train_gen
-        ctx.fine_tuning = fine_tuning
-        ctx.save_for_backward(x, h)
-        return y
-
-    @staticmethod
-    def backward(ctx, grad_y):
-        m = ctx.module
-        if ctx.gen != m._train_gen:
-            raise RuntimeError("this module ran another training forward before the backward of this "
-                               "one: its training workspace holds the later call's tensors")
-        x, h = ctx.saved_tensors
-        (grad_x,) = m._backward_train(x, h, grad_y.contiguous(), ctx.seed, ctx.fine_tuning)
-        return (None, grad_x, None, None, *m._last_param_grads)
-
-
 class FeedForward(nn.Module):
     """GeGLU feed-forward expert; mirrors reference model.py:154-190.
 
@@ -242,12 +188,18 @@ class FeedForward(nn.Module):
         self._lora = _MergedLora()
         # native calls prepared for the last number of rows: plain, and with the LoRA branches merged
         self._native, self._native_ft = _host.Ffn(), _host.Ffn()
+        self._native_train, self._native_train_ft = _host.Ffn(), _host.Ffn()
         self._offsets = None   # ((rows, device), int32 [0, rows]) of the last call
         self._tws = None
         self._tws_key = None
-        self._train_gen = 0
-        self._last_param_grads = None
         self.last_seed = None
+
+    def _rows(self, tensor):
+        x = tensor.reshape(-1, tensor.shape[-1]).contiguous()
+        M, dev = x.shape[0], x.device
+        if self._offsets is None or self._offsets[0] != (M, str(dev)):
+            self._offsets = ((M, str(dev)), torch.tensor([0, M], dtype=torch.int32, device=dev))
+        return x, M, dev, self._offsets[1]
 
     # -- training mode (bf16): dropout on h and a backward pass -----------------
     def _train_ws(self, M: int, device: torch.device):
@@ -257,67 +209,40 @@ class FeedForward(nn.Module):
             nbytes = lib.moe_b200_train_workspace_bytes(M, d, f, 1, 1, _cabi.BF16)
             if nbytes == 0:
                 raise _cabi.MoeB200Error(lib.moe_b200_last_error_string().decode())
-            buf = torch.zeros(nbytes + 1024, dtype=torch.uint8, device=device)
+            buf = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
             base = (buf.data_ptr() + 1023) & ~1023
             check(lib.moe_b200_train_setup(M, d, f, 1, 1, _cabi.BF16, base, nbytes, _stream(device)), "train_setup")
-            self._tws = (buf, base, nbytes, _cabi.train_workspace_layout(M, d, f, 1, 1, _cabi.BF16))
+            self._tws = (buf, base, nbytes)
             self._tws_key = key
+            self._native_train.unbind()
+            self._native_train_ft.unbind()
         return self._tws
 
-    def _tws_view(self, name: str, shape) -> torch.Tensor:
-        buf, base, _, layout = self._tws
-        start = base - buf.data_ptr() + layout[name]
-        n = 2
-        for s in shape:
-            n *= s
-        return buf[start:start + n].view(torch.bfloat16).view(*shape)
-
-    def _rows(self, tensor):
-        x = tensor.reshape(-1, tensor.shape[-1]).contiguous()
-        M, dev = x.shape[0], x.device
-        if self._offsets is None or self._offsets[0] != (M, str(dev)):
-            self._offsets = ((M, str(dev)), torch.tensor([0, M], dtype=torch.int32, device=dev))
-        return x, M, dev, self._offsets[1]
-
-    def _train_plan(self, fine_tuning: bool, d, f, dev):
-        if fine_tuning:
-            return self._plan_ft.get(self._lora.get([self], _cabi.BF16, dev), d, f, _cabi.BF16, dev)
-        return self._plan.get([self], d, f, _cabi.BF16, dev)
-
-    def _forward_train(self, tensor, seed: int, fine_tuning: bool = False):
-        x, M, dev, offsets = self._rows(tensor)
+    def _prepare_train(self, tensor, fine_tuning: bool, native):
+        """Training forward of a call that differs from the one ``native`` was bound for: prepares plan,
+        workspace and merged weights, binds them and runs."""
         d, f = self.hidden_size, self.d_ff
-        h = torch.empty(M, f, dtype=x.dtype, device=dev)
-        y = torch.empty(M, d, dtype=x.dtype, device=dev)
-        with torch.cuda.device(dev):
-            plan = self._train_plan(fine_tuning, d, f, dev)
-            _, tbase, tbytes, _ = self._train_ws(M, dev)
-            status = torch.zeros(16, dtype=torch.int32, device=dev)
-            check(lib.moe_b200_experts_train(x.data_ptr(), offsets.data_ptr(), plan, M, d, f, 1,
-                                             float(self.dropout.p), seed, tbase, tbytes, h.data_ptr(),
-                                             y.data_ptr(), status.data_ptr(), _stream(dev)), "experts_train")
-        self._train_gen += 1
-        self.last_seed = seed
-        return y.reshape(tensor.shape), h
-
-    def _backward_train(self, tensor, h, grad_y, seed: int, fine_tuning: bool = False):
+        if tensor.shape[-1] != d:
+            raise ValueError(f"last dimension {tensor.shape[-1]} != hidden_size {d}")
         x, M, dev, offsets = self._rows(tensor)
-        d, f = self.hidden_size, self.d_ff
-        g = grad_y.reshape(-1, d).contiguous().to(x.dtype)
-        grad_x = torch.empty_like(x)
         with torch.cuda.device(dev):
-            plan = self._train_plan(fine_tuning, d, f, dev)
-            _, tbase, tbytes, _ = self._train_ws(M, dev)
+            if fine_tuning:
+                plan = self._plan_ft.get(self._lora.get([self], _cabi.BF16, dev), d, f, _cabi.BF16, dev)
+            else:
+                plan = self._plan.get([self], d, f, _cabi.BF16, dev)
+            buf, tbase, tbytes = self._train_ws(M, dev)
             status = torch.zeros(16, dtype=torch.int32, device=dev)
-            check(lib.moe_b200_experts_backward(x.data_ptr(), h.data_ptr(), offsets.data_ptr(), plan, g.data_ptr(),
-                                                M, d, f, 1, float(self.dropout.p), seed, tbase, tbytes,
-                                                grad_x.data_ptr(), status.data_ptr(), _stream(dev)),
-                  "experts_backward")
-        self._last_param_grads = [self._tws_view("g_w1", (2 * f, d)).clone(), self._tws_view("g_b1", (2 * f,)).clone(),
-                                  self._tws_view("g_w2", (d, f)).clone(), self._tws_view("g_b2", (d,)).clone()]
-        if fine_tuning:
-            self._last_param_grads += _lora_grads(self, *self._last_param_grads[:4])
-        return [grad_x.reshape(tensor.shape)]
+            watch = _expert_watch(self, fine_tuning)
+            usual = all(name in table for table, name in watch)
+            jobs = _lora_jobs(self, self._lora.merged[0], 0) if fine_tuning and usual else None
+            native.unbind()
+            native.bind(watch if usual else [], jobs, plan, offsets, status, M, d, f, _cabi.BF16, dev.index)
+            table = _lora_table([self], dev) if fine_tuning else None
+            native.bind_train(buf, tbase, tbytes, table, self.lora_down_a.out_features if fine_tuning else 0,
+                              float(self.lora_scale))
+            # the tensors themselves, wherever the module tree keeps them
+            y, seed = native.train(x, float(self.dropout.p), _expert_params(self, fine_tuning))
+        return y.reshape(tensor.shape), seed
 
     def forward(self, tensor: torch.Tensor, fine_tuning: bool = False) -> torch.Tensor:
         """y = down(gelu_tanh(gate) * up) for every row, through the grouped
@@ -330,12 +255,12 @@ class FeedForward(nn.Module):
         if self.training and (torch.is_grad_enabled() or self.dropout.p > 0):
             if tensor.dtype != torch.bfloat16:
                 raise NotImplementedError("training mode computes in bfloat16")
-            seed = int(torch.randint(0, 2 ** 62, (1,), dtype=torch.int64).item())
-            params = [self.gate_and_up.weight, self.gate_and_up.bias, self.down.weight, self.down.bias]
-            if fine_tuning:
-                for lin in (self.lora_gate_and_up_a, self.lora_gate_and_up_b, self.lora_down_a, self.lora_down_b):
-                    params += [lin.weight, lin.bias]
-            return _FfnTrainFn.apply(self, tensor, seed, bool(fine_tuning), *params)
+            native = self._native_train_ft if fine_tuning else self._native_train
+            done = native.train(tensor, self.dropout.p, None)
+            if done is None:
+                done = self._prepare_train(tensor, bool(fine_tuning), native)
+            y, self.last_seed = done
+            return y
         native = self._native_ft if fine_tuning else self._native
         y = native.forward(tensor)
         return self._forward_prepared(tensor, bool(fine_tuning), native) if y is None else y
@@ -393,10 +318,10 @@ class MOE(nn.Module):
         self._ws_key = None
         self._tws = None
         self._tws_key = None
-        self._train_gen = 0
         self._last_seed = None
         # native calls prepared for the last input size: plain, and with the LoRA branches merged
         self._native, self._native_ft = _host.Block(), _host.Block()
+        self._native_train, self._native_train_ft = _host.Block(), _host.Block()
 
     @property
     def last(self) -> dict | None:
@@ -429,8 +354,8 @@ class MOE(nn.Module):
             base = (buf.data_ptr() + 1023) & ~1023
             self._ws = (buf, base, nbytes, _cabi.workspace_layout(N, d, f, E, k, dtype))
             self._ws_key = key
-            self._native.unbind()
-            self._native_ft.unbind()
+            for native in (self._native, self._native_ft, self._native_train, self._native_train_ft):
+                native.unbind()
             # the small-N kernels keep their counters in the status region and leave them zero
             # after every call (FLAG_WS_CLEAN below); everything else is written before it is
             # read, except for what a call without tokens leaves as it is
@@ -470,15 +395,12 @@ class MOE(nn.Module):
                                           "apply the LayerNorm in front of the block")
             if tensor.dtype != torch.bfloat16:
                 raise NotImplementedError("training mode computes in bfloat16")
-            seed = int(torch.randint(0, 2 ** 62, (1,), dtype=torch.int64).item())   # torch's CPU generator
-            params = [self.gate.weight, self.gate.bias]
-            for ex in self.experts:
-                params += [ex.gate_and_up.weight, ex.gate_and_up.bias, ex.down.weight, ex.down.bias]
-            if fine_tuning:
-                for ex in self.experts:
-                    for lin in (ex.lora_gate_and_up_a, ex.lora_gate_and_up_b, ex.lora_down_a, ex.lora_down_b):
-                        params += [lin.weight, lin.bias]
-            return _TrainFn.apply(self, tensor, residual, seed, bool(fine_tuning), *params)
+            native = self._native_train_ft if fine_tuning else self._native_train
+            done = native.train(tensor, residual, self.experts[0].dropout.p, None)
+            if done is None:
+                done = self._prepare_train(tensor, residual, bool(fine_tuning), native)
+            out, aux, self._last_seed = done
+            return out, aux
         native = self._native_ft if fine_tuning else self._native
         self._last_seed = None
         done = native.forward(tensor, residual, norm)
@@ -528,54 +450,51 @@ class MOE(nn.Module):
         self._bind(native, fine_tuning, plan, N, dtype, dev)
         return out.reshape(shape), aux
 
-    def _bind(self, native, fine_tuning: bool, plan: int, N: int, dtype: int, dev: torch.device) -> None:
-        """Hand the prepared call to the native path, with everything in the module tree it depends
-        on. Trees that do not hold their parameters under the usual names stay on the Python path."""
-        d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
-        native.unbind()
+    def _watch(self, fine_tuning: bool) -> list:
+        """Everything in the module tree a prepared call depends on; empty for trees that do not hold
+        their parameters under the usual names (those calls are prepared every time)."""
         watch = [(self._modules, "gate"), (self._modules, "experts"),
                  (self.gate._parameters, "weight"), (self.gate._parameters, "bias")]
         for name, ex in self.experts._modules.items():
             watch.append((self.experts._modules, name))
             watch += _expert_watch(ex, fine_tuning)
+        usual = len(self.experts) == self.num_experts and all(name in table for table, name in watch)
+        return watch if usual else []
+
+    def _bind(self, native, fine_tuning: bool, plan: int, N: int, dtype: int, dev: torch.device) -> None:
+        """Hand the prepared call to the native path."""
+        d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
+        native.unbind()
+        watch = self._watch(fine_tuning)
         jobs = None
-        if fine_tuning:
+        if fine_tuning and watch:
             jobs = [job for e, (ex, mg) in enumerate(zip(self.experts, self._lora.merged))
                     for job in _lora_jobs(ex, mg, 2 + 12 * e)]
-        if len(self.experts) != E or any(name not in table for table, name in watch):
-            return
         buf, base, nbytes, _ = self._ws
         native.bind(watch, jobs, plan, buf, base, nbytes, N, d, f, E, k, dtype, dev.index)
 
     # -- training mode -------------------------------------------------------
-    def _train_workspace(self, N: int, dtype: int, device: torch.device):
-        key = (N, dtype, str(device))
+    def _train_workspace(self, N: int, device: torch.device):
+        key = (N, str(device))
         if key != self._tws_key:
             d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
-            nbytes = lib.moe_b200_train_workspace_bytes(N, d, f, E, k, dtype)
+            nbytes = lib.moe_b200_train_workspace_bytes(N, d, f, E, k, _cabi.BF16)
             if nbytes == 0:
                 raise _cabi.MoeB200Error(lib.moe_b200_last_error_string().decode())
-            buf = torch.zeros(nbytes + 1024, dtype=torch.uint8, device=device)
+            buf = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
             base = (buf.data_ptr() + 1023) & ~1023
-            check(lib.moe_b200_train_setup(N, d, f, E, k, dtype, base, nbytes, _stream(device)), "train_setup")
-            self._tws = (buf, base, nbytes, _cabi.train_workspace_layout(N, d, f, E, k, dtype))
+            check(lib.moe_b200_train_setup(N, d, f, E, k, _cabi.BF16, base, nbytes, _stream(device)), "train_setup")
+            self._tws = (buf, base, nbytes)
             self._tws_key = key
+            self._native_train.unbind()
+            self._native_train_ft.unbind()
         return self._tws
 
-    def _tws_view(self, name: str, shape) -> torch.Tensor:
-        buf, base, _, layout = self._tws
-        start = base - buf.data_ptr() + layout[name]
-        n = 2
-        for s in shape:
-            n *= s
-        return buf[start:start + n].view(torch.bfloat16).view(*shape)
-
-    def _train_plan(self, fine_tuning: bool, d, f, dtype, dev):
-        if fine_tuning:
-            return self._plan_ft.get(self._lora.get(list(self.experts), dtype, dev), d, f, dtype, dev)
-        return self._plan.get(self.experts, d, f, dtype, dev)
-
-    def _forward_train(self, tensor, residual, seed: int, fine_tuning: bool = False):
+    def _prepare_train(self, tensor, residual, fine_tuning: bool, native):
+        """Training forward of a call that differs from the one ``native`` was bound for: checks the arguments,
+        prepares plan, workspaces and merged weights, binds them and runs. Gradients: the kernels run on the merged
+        weights W' = W + s B A, b' = b + s (B a + b_lora) (model.py:175-179,185-189), whose gradients are the
+        base Linear's own; the LoRA tensors' follow from the same activations (csrc/lora_bwd.cu)."""
         dtype = _dtype_code(tensor)
         shape = tensor.shape
         d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
@@ -584,65 +503,28 @@ class MOE(nn.Module):
         x = tensor.reshape(-1, d).contiguous()
         N = x.shape[0]
         dev = x.device
-        res_ptr = None
         if residual is not None:
             if residual.shape != shape or residual.dtype != tensor.dtype or residual.device != dev:
                 raise ValueError("residual must match the input's shape, dtype and device")
-            res_ptr = residual.reshape(-1, d).contiguous().data_ptr()
-        out = torch.empty_like(x)
+            residual = residual.reshape(-1, d).contiguous()
         with torch.cuda.device(dev):
-            plan = self._train_plan(fine_tuning, d, f, dtype, dev)
-            _, base, nbytes, _ = self._workspace(N, dtype, dev)
-            _, tbase, tbytes, _ = self._train_workspace(N, dtype, dev)
-            check(lib.moe_b200_forward_train(
-                x.data_ptr(), self.gate.weight.data_ptr(), self.gate.bias.data_ptr(), plan, res_ptr,
-                N, d, f, E, k, dtype, float(self.experts[0].dropout.p), seed, base, nbytes, tbase, tbytes,
-                out.data_ptr(), _stream(dev)), "forward_train")
-        self._train_gen += 1
-        self._last_seed = seed
-        aux = self._view("aux", torch.float32, (1,))[0].clone()
-        return out.reshape(shape), aux
-
-    def _backward_train(self, tensor, grad_out, grad_aux: float, seed: int, fine_tuning: bool = False):
-        """[grad_x, grad gate.weight, grad gate.bias, then per expert the gradients of
-        gate_and_up.weight, gate_and_up.bias, down.weight, down.bias; with ``fine_tuning`` then
-        per expert those of the four LoRA Linears (weight, bias each)].
-
-        With ``fine_tuning`` the kernels run on the merged weights W' = W + s B A,
-        b' = b + s (B a + b_lora) (model.py:175-179,185-189), so what they return for a Linear
-        is G = dL/dW' = dL/dW and g = dL/db' = dL/db; _lora_grads forms the LoRA tensors'
-        gradients from them: four small products per Linear on the gradient the grouped
-        kernel already produced."""
-        dtype = _dtype_code(tensor)
-        shape = tensor.shape
-        d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
-        x = tensor.reshape(-1, d).contiguous()
-        N = x.shape[0]
-        dev = x.device
-        g = grad_out.reshape(-1, d).contiguous()
-        if g.dtype != tensor.dtype:
-            g = g.to(tensor.dtype)
-        grad_x = torch.empty_like(x)
-        with torch.cuda.device(dev):
-            plan = self._train_plan(fine_tuning, d, f, dtype, dev)
-            _, base, nbytes, _ = self._workspace(N, dtype, dev)
-            _, tbase, tbytes, _ = self._train_workspace(N, dtype, dev)
-            check(lib.moe_b200_backward(
-                x.data_ptr(), self.gate.weight.data_ptr(), plan, g.data_ptr(), grad_aux, N, d, f, E, k, dtype,
-                float(self.experts[0].dropout.p), seed, base, nbytes, tbase, tbytes, grad_x.data_ptr(),
-                _stream(dev)), "backward")
-        # copies: the workspace is overwritten by the next backward
-        grads = [grad_x.reshape(shape), self._tws_view("g_wg", (E, d)).clone(), self._tws_view("g_bg", (E,)).clone()]
-        g_w1 = self._tws_view("g_w1", (E, 2 * f, d)).clone()
-        g_b1 = self._tws_view("g_b1", (E, 2 * f)).clone()
-        g_w2 = self._tws_view("g_w2", (E, d, f)).clone()
-        g_b2 = self._tws_view("g_b2", (E, d)).clone()
-        for e in range(E):
-            grads += [g_w1[e], g_b1[e], g_w2[e], g_b2[e]]
-        if fine_tuning:
-            for e, ex in enumerate(self.experts):
-                grads += _lora_grads(ex, g_w1[e], g_b1[e], g_w2[e], g_b2[e])
-        return grads
+            if fine_tuning:
+                plan = self._plan_ft.get(self._lora.get(list(self.experts), dtype, dev), d, f, dtype, dev)
+            else:
+                plan = self._plan.get(self.experts, d, f, dtype, dev)
+            self._workspace(N, dtype, dev)
+            buf, tbase, tbytes = self._train_workspace(N, dev)
+            self._bind(native, fine_tuning, plan, N, dtype, dev)
+            table = _lora_table(self.experts, dev) if fine_tuning else None
+            ex = self.experts[0]
+            native.bind_train(buf, tbase, tbytes, table, ex.lora_down_a.out_features if fine_tuning else 0,
+                              float(ex.lora_scale))
+            # the tensors themselves, wherever the module tree keeps them
+            params = [self.gate.weight, self.gate.bias]
+            for ex in self.experts:
+                params += _expert_params(ex, fine_tuning)
+            out, aux, seed = native.train(x, residual, float(self.experts[0].dropout.p), params)
+        return out.reshape(shape), aux, seed
 
     def device_status(self) -> int:
         """Status word of the most recent call (0 = ok); synchronises. A non-zero status is

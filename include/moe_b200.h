@@ -415,16 +415,16 @@ int moe_b200_attention(const void* qkv, const void* gate, const float* pos_emb, 
 enum {
   MOE_B200_TWS_GU = 0,   /* bf16 [N*k, 2f] gate/up pre-activations; (dg, du) after the backward */
   MOE_B200_TWS_PAIR_OF,  /* int32 [N*k]    token * k + slot of every sorted row */
-  MOE_B200_TWS_KOFF,     /* empty, as DH, W1T .. DGUT below: the products read their operands as
-                          * they lie in memory and dh never leaves the chip */
+  MOE_B200_TWS_KOFF,     /* empty, as DH, W1T .. DGUT, ONES and DXR below: the products read their
+                          * operands as they lie in memory and dh never leaves the chip */
   MOE_B200_TWS_DY, MOE_B200_TWS_DH, MOE_B200_TWS_DXS,   /* gradients of y, h, sorted x */
   MOE_B200_TWS_W1T, MOE_B200_TWS_W2T, MOE_B200_TWS_TMAPS,
   MOE_B200_TWS_XT, MOE_B200_TWS_HT, MOE_B200_TWS_DYT, MOE_B200_TWS_DGUT,
   MOE_B200_TWS_DL,       /* float [N,E]   gradient of the router logits */
   MOE_B200_TWS_DW,       /* float [N,k]   gradient of the renormalised scores */
-  MOE_B200_TWS_ONES,     /* float [N,k]   ones (moe_b200_train_setup) */
-  MOE_B200_TWS_DWG_F32,  /* float [E*d + E] accumulators of the gate gradients */
-  MOE_B200_TWS_DXR,      /* bf16 [N,d]    the router's share of grad_x */
+  MOE_B200_TWS_ONES,
+  MOE_B200_TWS_DWG_F32,  /* float         partial sums of the gate gradients */
+  MOE_B200_TWS_DXR,
   /* results of moe_b200_backward, bf16: */
   MOE_B200_TWS_G_WG,     /* [E,d]      gradient of gate.weight */
   MOE_B200_TWS_G_BG,     /* [E]        gate.bias */
@@ -439,7 +439,7 @@ enum {
 size_t moe_b200_train_workspace_bytes(int64_t N, int d, int f, int E, int k, int dtype);
 int moe_b200_train_workspace_layout(int64_t N, int d, int f, int E, int k, int dtype,
                                     size_t* h_offsets);
-/* Once per training workspace: constants. */
+/* Once per training workspace (checks it; nothing in it has to be prepared any more). */
 int moe_b200_train_setup(int64_t N, int d, int f, int E, int k, int dtype, void* train_ws,
                          size_t train_ws_bytes, void* stream);
 
