@@ -251,7 +251,7 @@ int moe_b200_experts(const void* perm, const int32_t* offsets, const void* plan,
   if (dtype == MOE_B200_BF16)
     return launch_experts_tc2(perm, offsets, plan, M, d, f, E, h, y, nullptr, status,
                               (cudaStream_t)stream);
-  return launch_experts_simt(perm, offsets, plan, M, d, f, E, dtype, h, y, (cudaStream_t)stream);
+  return launch_experts_simt(perm, offsets, plan, M, d, f, E, h, y, (cudaStream_t)stream);
 }
 
 int moe_b200_rows_splits(int64_t M, int d, int f, int E) { return M > 0 && f >= 8 && d >= 8 && E >= 1 ? rows_splits(M, d, f, E) : 0; }

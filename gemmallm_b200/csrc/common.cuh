@@ -274,7 +274,7 @@ int launch_norm_fold(const void* Wg, const void* bg, const void* gamma, const vo
 int launch_layernorm_rows(const void* x, const void* gamma, const void* beta, float eps, int64_t N,
                           int d, int dtype, void* out, float* stats, cudaStream_t s);
 int launch_experts_simt(const void* perm, const int32_t* offsets, const void* plan, int64_t M,
-                        int d, int f, int E, int dtype, void* h, void* y, cudaStream_t s);
+                        int d, int f, int E, void* h, void* y, cudaStream_t s);
 int launch_combine(const void* y, const int32_t* row_of, const float* w, const void* residual,
                    int64_t N, int d, int k, int dtype, void* out, cudaStream_t s,
                    const EpSync* ep_wait = nullptr, int32_t* status = nullptr);

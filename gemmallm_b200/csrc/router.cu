@@ -2,8 +2,8 @@
 // Cover reference model.py:206-223 (gate Linear, F.softmax, topk, score
 // renormalisation) and the per-expert probability sums of model.py:215.
 //
-// HBM-bound: x [N,d] is read once; Wg [E,d] stays in L1/L2. A block of four
-// warps owns 64 consecutive tokens.
+// HBM-bound: x [N,d] is read once; Wg [E,d] stays in L1/L2. A block (fp32: a
+// cluster of eight) owns 64 consecutive tokens.
 //   bf16: router_mma_kernel. Each warp owns 16 tokens and forms their logits
 //     with mma.sync m16n8k16 (bf16 products are exact in fp32, accumulation in
 //     fp32). Operands go from global memory straight into fragment registers
@@ -15,7 +15,10 @@
 //     Then four lanes per token do softmax / top-k over a quarter of the E logits each.
 //   fp32: router_kernel. CUDA-core FMA (TF32 would perturb the logits), four
 //     tokens x eight experts per warp pass, warp-shuffle reductions, softmax and
-//     top-k with one expert slice per lane.
+//     top-k with one expert slice per lane. Latency bounds it at the few hundred tokens fp32
+//     is used with: four tokens a warp over a cluster of eight blocks, whose probability sums
+//     meet in shared memory, where one block of four warps took sixteen tokens a warp in turn
+//     (512 tokens, d 512, 8 experts, nothing in L2: 62 -> 22 us).
 // With the caller's LayerNorm folded in (NORM, norm.cu): Wg is the folded weight
 // Wn = Wg * gamma, the same pass over x also forms sum(x - x0) and sum((x - x0)^2)
 // per row (x0 = the row's first element: a shift that keeps the one-pass variance
@@ -28,24 +31,28 @@ namespace moe {
 namespace {
 
 constexpr int kWarps = 4;
-constexpr int kTokPerWarp = kRouterTokensPerBlock / kWarps;  // 16
+// fp32: a cluster of eight two-warp blocks owns the 64 tokens, four tokens a warp
+constexpr int kF32Cluster = 8;
+constexpr int kF32Warps = 2;
+constexpr int kTokPerBlockF32 = kRouterTokensPerBlock / kF32Cluster;   // 8
+constexpr int kTokPerWarp = kTokPerBlockF32 / kF32Warps;               // 4
 constexpr int kTokGroup = 4;
 constexpr int kExpGroup = 8;
 
 template <typename T>
-__global__ void __launch_bounds__(kWarps * 32)
+__global__ void __cluster_dims__(kF32Cluster, 1, 1) __launch_bounds__(kF32Warps * 32)
 router_kernel(const T* __restrict__ x, const T* __restrict__ Wg, const T* __restrict__ bg,
               int64_t N, int d, int E, int k, float* __restrict__ out_logits,
               int32_t* __restrict__ out_idx, float* __restrict__ out_w,
               float* __restrict__ psum_part, const float* __restrict__ norm_c, float eps,
               float* __restrict__ stats) {
   extern __shared__ float smem[];
-  float* s_logits = smem;                                     // [64][E]
-  float* s_psum = smem + (size_t)kRouterTokensPerBlock * E;   // [kWarps][E]
+  float* s_logits = smem;                                     // [8][E]
+  float* s_psum = smem + (size_t)kTokPerBlockF32 * E;         // [kF32Warps][E]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int64_t tok_block0 = (int64_t)blockIdx.x * kRouterTokensPerBlock;
+  const int64_t tok_block0 = (int64_t)blockIdx.x * kTokPerBlockF32;
   const int64_t tok_warp0 = tok_block0 + warp * kTokPerWarp;
 
   // ---- logits ------------------------------------------------------------
@@ -224,19 +231,32 @@ router_kernel(const T* __restrict__ x, const T* __restrict__ Wg, const T* __rest
     }
   }
 
-  // ---- per-block probability sums, fixed order --------------------------
+  // ---- probability sums of the cluster's 64 tokens, four-token groups in token order ----
 #pragma unroll
   for (int i = 0; i < kPerLane; ++i) {
     int e = lane + 32 * i;
     if (e < E) s_psum[warp * E + e] = psum_local[i];
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    float s = 0.f;
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (blockIdx.x % kF32Cluster == 0) {
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+      float s = 0.f;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) s += s_psum[w * E + e];
-    psum_part[(size_t)blockIdx.x * E + e] = s;
+      for (int c = 0; c < kF32Cluster; ++c)
+#pragma unroll
+        for (int w = 0; w < kF32Warps; ++w) {
+          uint32_t addr = (uint32_t)__cvta_generic_to_shared(s_psum + w * E + e), remote;
+          float v;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(c));
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+          s += v;
+        }
+      psum_part[(size_t)(blockIdx.x / kF32Cluster) * E + e] = s;
+    }
   }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // the sums have been read
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 
@@ -602,13 +622,13 @@ int launch_router(const void* x, const void* Wg, const void* bg, int64_t N, int 
   if (dtype == MOE_B200_BF16 && norm_c == nullptr && status != nullptr && router_tc_supported(N, d, E, k))
     return launch_router_tc(x, Wg, bg, N, d, E, k, out_logits, out_idx, out_w, psum_part, status, s);
   const int64_t blocks = (N + kRouterTokensPerBlock - 1) / kRouterTokensPerBlock;
-  const size_t smem = sizeof(float) * (size_t)(kRouterTokensPerBlock + kWarps) * E;
+  const size_t smem = sizeof(float) * (size_t)(kTokPerBlockF32 + kF32Warps) * E;
   if (dtype == MOE_B200_BF16) {
     if (norm_c != nullptr)
       return launch_mma_nt<true>(x, Wg, bg, N, d, E, k, out_logits, out_idx, out_w, psum_part, norm_c, eps, stats, s);
     return launch_mma_nt<false>(x, Wg, bg, N, d, E, k, out_logits, out_idx, out_w, psum_part, nullptr, 0.f, nullptr, s);
   }
-  router_kernel<float><<<(unsigned)blocks, kWarps * 32, smem, s>>>(
+  router_kernel<float><<<(unsigned)blocks * kF32Cluster, kF32Warps * 32, smem, s>>>(
       static_cast<const float*>(x), static_cast<const float*>(Wg), static_cast<const float*>(bg),
       N, d, E, k, out_logits, out_idx, out_w, psum_part, norm_c, eps, stats);
   MOE_CUDA_CHECK(cudaGetLastError());

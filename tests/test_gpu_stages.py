@@ -208,6 +208,22 @@ def test_experts_fp32(cuda_device, rows, d, f):
     assert (y.cpu() - y_ref).abs().max() <= 1e-4
 
 
+# edges of the fp32 tiles: 4 and 8 rows (short products), 32 (a warp's rows), 64 (a block's); widths that are no
+# multiple of 32, 64 or 128; K split over a cluster of up to eight blocks, with ranges that end early
+@pytest.mark.parametrize("rows,d,f", [([1, 4, 5, 8, 9, 0, 31], 72, 200), ([64, 65, 32, 33], 264, 136), ([2], 1024, 2056),
+                                      ([129, 0, 0, 1], 2056, 8)])
+def test_experts_fp32_tile_edges(cuda_device, rows, d, f):
+    params, x, offsets = expert_inputs(rows, d, f, torch.float32, seed=3 * len(rows) + d)
+    dp = helpers.device_params(params, torch.float32, cuda_device)
+    plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
+    h, y, status = helpers.experts(x.to(cuda_device), offsets.to(cuda_device), plan)
+    assert status.cpu()[0] == 0
+    h_ref, y_ref = oracle_experts({n: t.double() for n, t in params.items()}, x.double(), offsets)
+    # sums of at most 2056 fp32 products: a few ulp (2^-24) times the square root of their number
+    assert (h.cpu().double() - h_ref).norm() <= 2e-6 * h_ref.norm()
+    assert (y.cpu().double() - y_ref).norm() <= 4e-6 * y_ref.norm()
+
+
 @pytest.mark.parametrize("rows,d,f", EXPERT_CASES)
 def test_experts_bf16(cuda_device, rows, d, f):
     params, x, offsets = expert_inputs(rows, d, f, torch.bfloat16, seed=len(rows) + d)
