@@ -5,15 +5,16 @@
 // (model.py:226-253), and finishes the load-balancing loss (model.py:213-216).
 //
 // HBM-bound: x [N,d] is read once and written k times with 16-byte accesses.
-// Tokens are cut into chunks of 64; every block owns one contiguous range of
-// chunks (the first nchunk mod gridDim blocks one chunk more than the rest) in
-// both phases. Phase 1 counts experts per chunk and per block into scratch.
-// After a grid barrier every block sums the per-block counts (gridDim * E
-// numbers: all of them for the expert offsets, those of earlier blocks for its
-// base), then for each of its chunks ranks the (token, slot) pairs in token
-// order and copies the rows, the loads of one batch of rows in flight while
-// the batch before it is stored. Rows of one expert therefore stay in token
-// order whatever the grid size.
+// Tokens are cut into chunks of at most 64, of the size that gives every block of
+// a full grid the same number of chunks (chunk_tokens below); every block owns one
+// contiguous range of chunks in both phases. The rows of its first chunk are
+// requested before anything else: they depend on nothing. Phase 1 counts experts
+// per block into scratch. After a grid barrier every block sums the per-block
+// counts (gridDim * E numbers: all of them for the expert offsets, those of
+// earlier blocks for its base), then for each of its chunks ranks the (token,
+// slot) pairs in token order and copies the rows, the loads of two batches of rows
+// in flight while the one before them is stored. Rows of one expert therefore stay
+// in token order whatever the grid size.
 // With the caller's LayerNorm folded in (norm_stats != nullptr, see norm.cu) a row is
 // copied as (x - mean) * rstd * gamma + beta, with (mean, rstd) from the router
 // (reference model.py:311-312).
@@ -31,7 +32,15 @@ constexpr int kThreads = 256;
 constexpr int kChunk = kDispatchChunk;
 constexpr int kScratchHeader = 32;  // ints: [0] = blocks finished
 
-__host__ __device__ inline int64_t num_chunks(int64_t N) { return (N + kChunk - 1) / kChunk; }
+// Tokens per chunk for a grid of at most `grid` blocks: as few rounds of chunks as chunks of 64 would
+// take, evened out over the grid, and no block with fewer than four tokens. 16384 tokens on 296 blocks are
+// 293 chunks of 56, where 256 chunks of 64 left 40 SMs with half the rows of the others; 512 tokens are
+// 128 blocks instead of 8 (fp32, d 512: 27 -> 14 us with the early loads).
+inline int chunk_tokens(int64_t N, int64_t grid) {
+  const int64_t rounds = (N + kChunk * grid - 1) / (kChunk * grid);
+  const int64_t per = rounds > 0 ? (N + grid * rounds - 1) / (grid * rounds) : 1;
+  return (int)(per < 4 ? 4 : per);
+}
 
 // chunks [first, first + count) of block b out of G
 __device__ inline void chunk_range(int64_t nchunk, int G, int b, int64_t& first, int64_t& count) {
@@ -48,10 +57,10 @@ dispatch_kernel(const T* __restrict__ x, const int32_t* __restrict__ idx, int64_
                 const float* __restrict__ psum_part, int64_t router_blocks,
                 float* __restrict__ psum, float* __restrict__ aux, int32_t* __restrict__ status,
                 const float* __restrict__ norm_stats, const T* __restrict__ gamma,
-                const T* __restrict__ beta) {
+                const T* __restrict__ beta, int chunk) {
   cg::grid_group grid = cg::this_grid();
   extern __shared__ int s_int[];
-  int* s_hist = s_int;             // [E]  chunk histogram, later totals
+  int* s_hist = s_int;             // [E]  totals
   int* s_base = s_hist + E;        // [E]  rows of earlier chunks per expert
   int* s_off = s_base + E;         // [E+1]
   int* s_run = s_off + E + 1;      // [E]  running rank inside the chunk
@@ -62,41 +71,58 @@ dispatch_kernel(const T* __restrict__ x, const int32_t* __restrict__ idx, int64_
 
   const int tid = threadIdx.x;
   const int G = gridDim.x;
-  const int64_t nchunk = num_chunks(N);
+  const int64_t nchunk = (N + chunk - 1) / chunk;
   int32_t* done = scratch;
-  int32_t* chunk_cnt = scratch + kScratchHeader;     // [nchunk][E]
-  int32_t* blk_slot = chunk_cnt + nchunk * E;        // [G][k][E]
+  int32_t* blk_slot = scratch + kScratchHeader;      // [G][k][E]
   int32_t* blk_cnt = blk_slot + (size_t)kNumSMs * 2 * k * E;   // [G][E]
   int64_t c_first, c_count;
   chunk_range(nchunk, G, blockIdx.x, c_first, c_count);
 
+  // rows of a chunk: its 16-byte pieces are spread over the block, kInFlight loads per thread and batch;
+  // each piece is stored once per slot
+  const int warp = tid >> 5, lane = tid & 31;
+  constexpr int kVec = 16 / (int)sizeof(T);
+  constexpr int kInFlight = 8;
+  constexpr int kBatch = kThreads * kInFlight;
+  const int pieces = d / kVec;
+  int64_t t0 = c_first * chunk;
+  int ntok = c_count > 0 ? (int)((N - t0) < chunk ? (N - t0) : chunk) : 0;
+  int items = ntok * pieces;
+  auto load = [&](uint4 (&v)[kInFlight], int i0) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + t0 * d);
+#pragma unroll
+    for (int u = 0; u < kInFlight; ++u) {
+      const int i = i0 + u * kThreads;
+      if (i < items) v[u] = __ldg(src + i);
+    }
+  };
+  uint4 va[kInFlight], vb[kInFlight];
+  load(va, tid);
+  load(vb, tid + kBatch);
+
   // ---- phase 1: histograms -----------------------------------------------
   for (int i = tid; i < k * E; i += kThreads) s_slot[i] = 0;
-  for (int e = tid; e < E; e += kThreads) s_base[e] = 0;   // this block's total per expert
   if (blockIdx.x == 0 && tid == 0) *done = 0;
-  for (int64_t c = c_first; c < c_first + c_count; ++c) {
-    for (int e = tid; e < E; e += kThreads) s_hist[e] = 0;
-    __syncthreads();
-    const int64_t t0 = c * kChunk;
-    const int ntok = (int)((N - t0) < kChunk ? (N - t0) : kChunk);
-    for (int p = tid; p < ntok * k; p += kThreads) {
-      int e = idx[t0 * k + p];
+  __syncthreads();
+  {
+    const int64_t t_end = (c_first + c_count) * chunk < N ? (c_first + c_count) * chunk : N;
+    const int npair = (int)(t_end - t0) * k;
+    for (int p = tid; p < npair; p += kThreads) {
+      const int e = idx[t0 * k + p];
       if ((unsigned)e >= (unsigned)E) {
         atomicMax(&status[0], MOE_B200_DEV_BAD_INDEX);
         continue;
       }
-      atomicAdd(&s_hist[e], 1);
       atomicAdd(&s_slot[(p % k) * E + e], 1);
     }
-    __syncthreads();
-    for (int e = tid; e < E; e += kThreads) {
-      chunk_cnt[c * E + e] = s_hist[e];
-      s_base[e] += s_hist[e];
-    }
-    __syncthreads();
   }
+  __syncthreads();
   for (int i = tid; i < k * E; i += kThreads) blk_slot[(size_t)blockIdx.x * k * E + i] = s_slot[i];
-  for (int e = tid; e < E; e += kThreads) blk_cnt[(size_t)blockIdx.x * E + e] = s_base[e];
+  for (int e = tid; e < E; e += kThreads) {
+    int sum = 0;
+    for (int j = 0; j < k; ++j) sum += s_slot[j * E + e];
+    blk_cnt[(size_t)blockIdx.x * E + e] = sum;
+  }
 
   grid.sync();
 
@@ -159,28 +185,8 @@ dispatch_kernel(const T* __restrict__ x, const int32_t* __restrict__ idx, int64_
     for (int e = tid; e <= E; e += kThreads) offsets[e] = s_off[e];
 
   // ---- phase 2: rank and copy ---------------------------------------------
-  const int warp = tid >> 5, lane = tid & 31;
-  constexpr int kVec = 16 / (int)sizeof(T);
-  constexpr int kInFlight = 8;
-  constexpr int kBatch = kThreads * kInFlight;
-  const int pieces = d / kVec;
   for (int64_t c = c_first; c < c_first + c_count; ++c) {
-    const int64_t t0 = c * kChunk;
-    const int ntok = (int)((N - t0) < kChunk ? (N - t0) : kChunk);
     const int npair = ntok * k;
-    // rows: the chunk's 16-byte pieces are spread over the block, kInFlight loads per
-    // thread and batch; each piece is stored once per slot. The first batch is
-    // requested before the ranks are known, every later one before the batch in
-    // front of it is stored.
-    const int items = ntok * pieces;
-    const uint4* src = reinterpret_cast<const uint4*>(x + t0 * d);
-    auto load = [&](uint4 (&v)[kInFlight], int i0) {
-#pragma unroll
-      for (int u = 0; u < kInFlight; ++u) {
-        const int i = i0 + u * kThreads;
-        if (i < items) v[u] = __ldg(src + i);
-      }
-    };
     auto store = [&](uint4 (&v)[kInFlight], int i0) {
 #pragma unroll
       for (int u = 0; u < kInFlight; ++u) {
@@ -206,8 +212,6 @@ dispatch_kernel(const T* __restrict__ x, const int32_t* __restrict__ idx, int64_
         }
       }
     };
-    uint4 va[kInFlight], vb[kInFlight];
-    load(va, tid);
     if (warp == 0) {
       for (int e = lane; e < E; e += 32) s_run[e] = 0;
       __syncwarp();
@@ -232,19 +236,22 @@ dispatch_kernel(const T* __restrict__ x, const int32_t* __restrict__ idx, int64_
       }
     }
     __syncthreads();
-    for (int i0 = tid;;) {
-      const int i1 = i0 + kBatch;
-      if (i1 < items) load(vb, i1);
+    for (int i0 = tid; i0 < items;) {
+      const int i1 = i0 + kBatch, i2 = i1 + kBatch, i3 = i2 + kBatch;
       store(va, i0);
-      if (i1 >= items) break;
-      i0 = i1 + kBatch;
-      if (i0 < items) load(va, i0);
-      store(vb, i1);
-      if (i0 >= items) break;
+      if (i2 < items) load(va, i2);
+      if (i1 < items) store(vb, i1);
+      if (i3 < items) load(vb, i3);
+      i0 = i2;
     }
+    t0 += ntok;
+    ntok = c + 1 < c_first + c_count ? (int)((N - t0) < chunk ? (N - t0) : chunk) : 0;
+    items = ntok * pieces;
+    load(va, tid);
+    load(vb, tid + kBatch);
     __syncthreads();
     // this chunk's rows precede the next chunk's
-    for (int e = tid; e < E; e += kThreads) s_base[e] += chunk_cnt[c * E + e];
+    for (int e = tid; e < E; e += kThreads) s_base[e] += s_run[e];
     __syncthreads();
   }
 
@@ -296,7 +303,9 @@ dispatch_kernel(const T* __restrict__ x, const int32_t* __restrict__ idx, int64_
 }  // namespace
 
 int64_t dispatch_scratch_ints(int64_t N, int E, int k) {
-  return kScratchHeader + num_chunks(N) * E + (int64_t)kNumSMs * 2 * k * E + (int64_t)kNumSMs * 2 * E;
+  // (the kernel uses the header and the counts of at most 2 * kNumSMs blocks; callers' buffers keep the size
+  // they have always had)
+  return kScratchHeader + (N + kChunk - 1) / kChunk * E + (int64_t)kNumSMs * 2 * k * E + (int64_t)kNumSMs * 2 * E;
 }
 
 int launch_dispatch(const void* x, const int32_t* idx, int64_t N, int d, int E, int k, int dtype,
@@ -317,7 +326,8 @@ int launch_dispatch(const void* x, const int32_t* idx, int64_t N, int d, int E, 
   per_sm = per_sm < 1 ? 1 : (per_sm > 2 ? 2 : per_sm);
   int64_t grid = (int64_t)sms * per_sm;
   if (grid > (int64_t)kNumSMs * 2) grid = (int64_t)kNumSMs * 2;
-  int64_t nchunk = num_chunks(N);
+  int chunk = chunk_tokens(N, grid);
+  int64_t nchunk = (N + chunk - 1) / chunk;
   if (nchunk < 1) nchunk = 1;
   if (grid > nchunk) grid = nchunk;
   int64_t router_blocks = (N + kRouterTokensPerBlock - 1) / kRouterTokensPerBlock;
@@ -325,7 +335,7 @@ int launch_dispatch(const void* x, const int32_t* idx, int64_t N, int d, int E, 
                   (void*)&E,        (void*)&k,       (void*)&scratch, (void*)&cnt_slot,
                   (void*)&offsets,  (void*)&row_of,  (void*)&perm,    (void*)&psum_part,
                   (void*)&router_blocks, (void*)&psum, (void*)&aux,   (void*)&status,
-                  (void*)&norm_stats, (void*)&gamma, (void*)&beta};
+                  (void*)&norm_stats, (void*)&gamma, (void*)&beta,  (void*)&chunk};
   MOE_CUDA_CHECK(cudaLaunchCooperativeKernel(fn, dim3((unsigned)grid), dim3(kThreads), args, smem, s));
   return 0;
 }
