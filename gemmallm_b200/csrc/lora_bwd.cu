@@ -84,22 +84,38 @@ lora_rows_kernel(const Jobs jobs, const int32_t* __restrict__ offsets, int E, in
   const bool is_b = (job & 1) != 0;
   const __nv_bfloat16* W =
       static_cast<const __nv_bfloat16*>(jobs.tab[((size_t)(job >> 1) * E + e) * 3 + (is_b ? 2 : 0)]);
-  for (int i = tid; i < kRank * kRange / 8; i += 256) {
-    const int r = i / (kRange / 8), k = (i - r * (kRange / 8)) * 8;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (n0 + r < rank && k < klen) {
-      if (!is_b) {
-        v = __ldg(reinterpret_cast<const uint4*>(W + (size_t)(n0 + r) * C + k0 + k));
-      } else {
-        uint16_t h[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          h[q] = __ldg(reinterpret_cast<const unsigned short*>(W) + (size_t)(k0 + k + q) * rank + n0 + r);
-        v = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16,
-                       h[6] | (uint32_t)h[7] << 16);
-      }
+  if (!is_b) {
+    for (int i = tid; i < kRank * kRange / 8; i += 256) {
+      const int r = i / (kRange / 8), k = (i - r * (kRange / 8)) * 8;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (n0 + r < rank && k < klen) v = __ldg(reinterpret_cast<const uint4*>(W + (size_t)(n0 + r) * C + k0 + k));
+      *reinterpret_cast<uint4*>(s_w + r * kWPitch + k) = v;
     }
-    *reinterpret_cast<uint4*>(s_w + r * kWPitch + k) = v;
+  } else {
+    // a thread takes whole rows of B, 16 ranks of one k (32 contiguous bytes where rows allow 16-byte loads), and
+    // a warp's stores of one rank are 64 contiguous bytes (with k along the lanes of the loads, a sector for
+    // every two bytes, this kernel took 38 instead of 15 us at 1632 rows, d 1024, f 4096)
+    const bool wide = rank % 8 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
+#pragma unroll
+    for (int u = 0; u < kRange / 256; ++u) {
+      const int k = tid + u * 256;
+      uint4 v[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+      if (k < klen) {
+        const __nv_bfloat16* row = W + (size_t)(k0 + k) * rank + n0;
+        if (wide) {
+          v[0] = __ldg(reinterpret_cast<const uint4*>(row));
+          if (n0 + 8 < rank) v[1] = __ldg(reinterpret_cast<const uint4*>(row) + 1);
+        } else {
+          unsigned short* h = reinterpret_cast<unsigned short*>(v);
+#pragma unroll
+          for (int r = 0; r < kRank; ++r)
+            if (n0 + r < rank) h[r] = __ldg(reinterpret_cast<const unsigned short*>(row) + r);
+        }
+      }
+      const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(v);
+#pragma unroll
+      for (int r = 0; r < kRank; ++r) s_w[r * kWPitch + k] = h[r];
+    }
   }
   __syncthreads();
   // warp = 16 rows x half of the range; the contraction index inside 32 elements is permuted alike for both sides
