@@ -517,3 +517,35 @@ def test_layernorm_stage_entry_points(cuda_device, N, d, E, k, dtype):
     ro = row_of.cpu().long()
     for j in range(k):
         assert (perm.float().cpu()[ro[:, j]] - xn).abs().max() <= rtol * scale
+
+
+# query heads of one KV head over several blocks (few sequences) and in one block; contexts at the edges of the
+# 16-token tiles; a position table at an address that is no multiple of 16; masks with -inf, with none
+@pytest.mark.parametrize("B,S,H,KV,masked,shift", [(1, 37, 16, 1, True, 0), (1, 1, 16, 1, True, 0), (3, 16, 6, 2, False, 1),
+                                                   (2, 17, 4, 4, True, 0), (400, 48, 3, 1, True, 0),
+                                                   (300, 15, 2, 1, False, 3), (1, 128, 5, 1, True, 0)])
+def test_attention_core(cuda_device, B, S, H, KV, masked, shift):
+    hd, g = 64, torch.Generator().manual_seed(B + S)
+    qkv = synthetic.round_to(torch.randn(B, S, H + 2 * KV, hd, generator=g), torch.bfloat16)
+    gate = synthetic.round_to(torch.randn(B, S, H, generator=g), torch.bfloat16)
+    table = torch.randn(S, 2 * hd, generator=g)
+    mask = torch.full((S, S), float("-inf")).triu(1) if masked else None
+    table_d = torch.empty(S * 2 * hd + shift, device=cuda_device)[shift:].view(S, 2 * hd)
+    table_d.copy_(table)
+    mask_d = None if mask is None else mask.to(cuda_device)
+    qkv_d, gate_d = qkv.bfloat16().to(cuda_device), gate.bfloat16().to(cuda_device)
+    out = torch.empty(B, S, H * hd, dtype=torch.bfloat16, device=cuda_device)
+    check(lib.moe_b200_attention(qkv_d.data_ptr(), gate_d.data_ptr(), table_d.data_ptr(),
+                                 None if mask is None else mask_d.data_ptr(), B, S, H, KV, hd, hd ** -0.5,
+                                 out.data_ptr(), helpers.stream(cuda_device)), "attention")
+    swap = lambda t: t.view(*t.shape[:-1], hd // 2, 2).flip(-1).flatten(-2)
+    rope = lambda t: t * table[:, None, :hd] + swap(t) * table[:, None, hd:]
+    q, kk, v = qkv.split((H, KV, KV), dim=2)
+    q, kk, v = rope(q), rope(kk).repeat_interleave(H // KV, 2), v.repeat_interleave(H // KV, 2)
+    scores = torch.einsum("bshd,bthd->bhst", q, kk) * hd ** -0.5
+    probs = torch.softmax(scores if mask is None else scores + mask, dim=-1)
+    want = (torch.einsum("bhst,bthd->bshd", probs, v) * torch.sigmoid(gate)[..., None]).flatten(2)
+    # rotated q and k are rounded to bf16, 2^-9 relative each, which moves scores (of about 2) by about 2^-8 and
+    # probabilities by as much of themselves; probabilities and outputs are rounded once more: about 2^-7 in the
+    # 2-norm, twice that allowed
+    assert (out.float().cpu() - want).norm() <= 2 ** -6 * want.norm()
