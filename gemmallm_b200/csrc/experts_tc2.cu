@@ -29,6 +29,13 @@
 // those rows in shared memory up to the next multiple of 16, which is where the products of that
 // block stop, and passes the stage on. (Only there do the two CTAs arrive on a common barrier: an
 // arrival across the pair for every block halved the rate, 680 instead of 1280 TFLOP/s.)
+//
+// SPLIT > 1 (kPlain, kDx): products of few tiles and a long contraction. A tile of 256 x 256 takes 0.39 us per
+// 64 of K however few of them run (the tensor pipe's own rate: 1630 TFLOP/s if all 74 pairs had one), so 28 tiles
+// of K = 4096 left 46 pairs idle for 27 us. SPLIT pairs in one cluster take a range of K each, put their fp32
+// accumulators into shared memory (the stages are free by then: a cluster has one tile) and each adds up and
+// stores 256 / SPLIT columns, in the order of the ranges. (128-column tiles instead gained nothing: a product of
+// half the columns takes the same time.)
 #include <cuda.h>
 #include "common.cuh"
 #include "tc_ptx.cuh"
@@ -50,6 +57,7 @@ constexpr int kABytes = BM * BK * 2;         // 16 KiB: this CTA's rows
 constexpr int kBBytes = (BN / 2) * BK * 2;   // 16 KiB: this CTA's half of the weight tile
 constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kTmemCols = 2 * BN;
+constexpr int kPartPitch = BN + 4;       // SPLIT: floats per row of a partial tile in shared memory
 constexpr int kHalfTile = 64 * BK * 2;   // one 64 x 64 box of an MN-major operand: 8 KiB
 
 // What a launch computes. Rows of A are grouped by expert except in kWgrad.
@@ -202,8 +210,8 @@ __device__ __forceinline__ bool barrier_and(int id, int threads, bool ok) {
 // COLS = false: groups are row ranges [offsets[e], offsets[e+1]) of A; B_e = tmap_b[e]; K fixed.
 // COLS = true : groups are the same row ranges, contracted over; A has Ra columns, B (one map,
 //               tmap_bc) has Nout columns; out [E][Ra][Nout], zero for experts without rows.
-template <int KIND>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Traits<KIND>::kThreads, 1)
+template <int KIND, int SPLIT>
+__global__ void __launch_bounds__(Traits<KIND>::kThreads, 1)
 grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                         const __grid_constant__ CUtensorMap tmap_bc,
                         const __grid_constant__ CUtensorMap tmap_h,    // kGegluTrain: h, 32 x 32 boxes
@@ -228,12 +236,20 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t cta = cluster_ctarank();   // 0 = even CTA: issues the MMAs, owns full/tmem_empty
-  const int pair = blockIdx.x >> 1;
-  const int num_pairs = gridDim.x >> 1;
+  static_assert(SPLIT == 1 || KIND == kPlain || KIND == kDx, "kinds with a split form");
+  static_assert(SPLIT == 1 || BM * kPartPitch * 4 <= kStages * kStageBytes, "the partial tile reuses the stages");
+  const uint32_t rank = cluster_ctarank();
+  const uint32_t cta = rank & 1u;           // 0 = even CTA: issues the MMAs, owns full/tmem_empty
+  const uint32_t lead = SPLIT > 1 ? rank & ~1u : 0u;      // the pair's even CTA
+  // the tiles of this pair: t = pair, pair + num_pairs, ... (SPLIT: of its cluster, one tile at most)
+  const int pair = blockIdx.x / (2 * SPLIT);
+  const int num_pairs = gridDim.x / (2 * SPLIT);
   constexpr int kTileN = GEGLU ? BN / 2 : BN;
   const int n_tiles = (Nout + kTileN - 1) / kTileN;
-  const int k_blocks_rows = (K + BK - 1) / BK;
+  const int k_blocks_all = (K + BK - 1) / BK;
+  const int k_blocks_per = (k_blocks_all + SPLIT - 1) / SPLIT;
+  const int kb_first = SPLIT > 1 ? (int)(rank >> 1) * k_blocks_per : 0;       // this pair's range of K
+  const int k_blocks_rows = min(k_blocks_per, k_blocks_all - kb_first);
   const int m_tiles_cols = (Ra + kPairRows - 1) / kPairRows;
 
   if (threadIdx.x == 0) {
@@ -310,15 +326,15 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
             if (!mbar_wait(&ctl->empty[stage], phase ^ 1u, &ctl->abort, status, 31)) { ok = false; break; }
           }
           uint8_t* sa = smem + (size_t)stage * kStageBytes;
-          const uint32_t full0 = map_to_cta(smem_u32(&ctl->full[stage]), 0);
+          const uint32_t full0 = map_to_cta(smem_u32(&ctl->full[stage]), lead);
           uint32_t bar = full0;
           if (COLS && (kb + 1) * BK > k_rows) {
             mbar_expect_tx(&ctl->tail[stage], kStageBytes);     // the fixer passes it on
-            bar = map_to_cta(smem_u32(&ctl->tail[stage]), cta);
+            bar = map_to_cta(smem_u32(&ctl->tail[stage]), rank);
           } else if (cta == 0) {
             mbar_expect_tx(&ctl->full[stage], 2 * kStageBytes);
           }
-          const int kc = k0 + kb * BK;
+          const int kc = k0 + (kb_first + kb) * BK;
           if (A_MN) {
             tma_load_2d_pair(sa, &tmap_a, bar, row0, kc);
             tma_load_2d_pair(sa + kHalfTile, &tmap_a, bar, row0 + 64, kc);
@@ -374,14 +390,14 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                           (kb | kk) != 0 ? 1u : 0u);
           // the stage is free in both CTAs once these MMAs have read it
           const uint32_t e_local = smem_u32(&ctl->empty[stage]);
-          tc_commit_pair(map_to_cta(e_local, 0));
-          tc_commit_pair(map_to_cta(e_local, 1));
+          tc_commit_pair(map_to_cta(e_local, lead));
+          tc_commit_pair(map_to_cta(e_local, lead + 1));
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         const uint32_t f_local = smem_u32(&ctl->tmem_full[a]);
-        tc_commit_pair(map_to_cta(f_local, 0));
-        tc_commit_pair(map_to_cta(f_local, 1));
+        tc_commit_pair(map_to_cta(f_local, lead));
+        tc_commit_pair(map_to_cta(f_local, lead + 1));
         if (a == 1) acc_phase ^= 1u;
         ++it;
       }
@@ -517,7 +533,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       auto release = [&]() {     // this warp has read its part of the accumulator
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&ctl->tmem_empty[a]), 0));
+        if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&ctl->tmem_empty[a]), lead));
       };
       if constexpr (KIND == kGegluTrain) {
         uint32_t bits = 0xffffffffu;
@@ -567,6 +583,17 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tr.col_part[slot * 2 * Nout + (c >= BN ? Nout : 0) + col] = sum;
         }
         barrier_and(1, 32 * kEpiWarps, true);
+      } else if constexpr (SPLIT > 1) {
+        float* mine = reinterpret_cast<float*>(smem) + r * kPartPitch + part * (BN / 2);
+#pragma unroll 1
+        for (int c = 0; c < BN / 2; c += 32) {
+          uint32_t v[32];
+          tc_ld32(taddr + part * (BN / 2) + c, v);
+          tc_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 32; q += 4)
+            *reinterpret_cast<uint4*>(mine + c + q) = make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+        }
       } else {
         store_tile<GEGLU, KIND == kScatter>(taddr, row_cta + r, row_cta + r < row_end, n0, Nout, bias, out_e, sc,
                                             extra + (warp - 2) * kStgBytes, lane, part, release);
@@ -576,6 +603,45 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
     if (KIND == kGegluTrain && lane == 0) bulk_wait_all();
     if (KIND == kScatter) __threadfence_system();
+  }
+  if constexpr (SPLIT > 1) {
+    __syncwarp();
+    cluster_sync();       // the partial tiles of all ranges are there (or a wait ran out, and the status says so)
+    if (pair < total_tiles) {
+      int e = 0;
+      while (pair >= ctl->tile_start[e + 1]) ++e;
+      const int local = pair - ctl->tile_start[e];
+      const int mt = local / n_tiles, nt = local - mt * n_tiles;
+      const int row_cta = ctl->offsets[e] + mt * kPairRows + (int)cta * BM;
+      const int rows = min(BM, ctl->offsets[e + 1] - row_cta);
+      const __nv_bfloat16* bias = bias_ptrs != nullptr ? static_cast<const __nv_bfloat16*>(bias_ptrs[e]) : nullptr;
+      constexpr int kPieces = BN / SPLIT / 8;          // of eight columns, per row
+      const int c0 = (int)(rank >> 1) * (BN / SPLIT);
+      for (int i = threadIdx.x; i < rows * kPieces; i += T::kThreads) {
+        const int rr = i / kPieces, c = c0 + (i % kPieces) * 8, n = nt * kTileN + c;
+        if (n >= Nout) continue;
+        const uint32_t at = smem_u32(smem) + (uint32_t)(rr * kPartPitch + c) * 4;
+        float o[8] = {};
+#pragma unroll
+        for (int q = 0; q < SPLIT; ++q) {
+          const uint32_t from = map_to_cta(at, 2 * q + cta);
+          float4 v0, v1;
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v0.x), "=f"(v0.y), "=f"(v0.z), "=f"(v0.w) : "r"(from) : "memory");
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v1.x), "=f"(v1.y), "=f"(v1.z), "=f"(v1.w) : "r"(from + 16) : "memory");
+          o[0] += v0.x; o[1] += v0.y; o[2] += v0.z; o[3] += v0.w;
+          o[4] += v1.x; o[5] += v1.y; o[6] += v1.z; o[7] += v1.w;
+        }
+        if (bias != nullptr) {
+          float b[8];
+          load8_ldg(bias + n, b);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) o[q] += b[q];
+        }
+        store8(out + (int64_t)(row_cta + rr) * Nout + n, o);
+      }
+    }
   }
   // expert-parallel down pass: the last CTA to get here tells every rank that this rank's
   // outputs have been stored
@@ -598,22 +664,42 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
 }
 
-template <int KIND>
+// SPLIT > 1: max_tiles is an upper bound of the launch's tiles, one cluster each (those without one leave).
+template <int KIND, int SPLIT = 1>
 int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_bc, const void* tmap_b, const int32_t* offsets,
                 const void* const* bias, int E, int K, int Nout, void* out, const EpScatter& sc,
                 const TrainArgs& tr, const EpSync& sy, int Ra, int32_t* status, int sms, cudaStream_t s,
-                const CUtensorMap* tm_h = nullptr, const CUtensorMap* tm_gu = nullptr) {
+                const CUtensorMap* tm_h = nullptr, const CUtensorMap* tm_gu = nullptr, int64_t max_tiles = 0) {
   static PerDeviceOnce once;
-  auto fn = grouped_gemm_tc2_kernel<KIND>;
+  auto fn = grouped_gemm_tc2_kernel<KIND, SPLIT>;
   constexpr size_t smem = smem_bytes<KIND>();
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
   int rc = ensure_dynamic_smem(once, fn, smem);
   if (rc) return rc;
-  MOE_CUDA_CHECK(launch_pdl(fn, dim3(sms & ~1), dim3(Traits<KIND>::kThreads), smem, s, tm_a, tm_bc,
-                            tm_h != nullptr ? *tm_h : tm_a, tm_gu != nullptr ? *tm_gu : tm_a,
-                            static_cast<const CUtensorMap*>(tmap_b), offsets, bias, E, K, Nout,
-                            static_cast<__nv_bfloat16*>(out), sc, tr, sy, Ra, status));
+  const unsigned grid = SPLIT > 1 ? (unsigned)max_tiles * 2 * SPLIT : (unsigned)(sms & ~1);
+  MOE_CUDA_CHECK(launch_pdl_cluster(fn, dim3(grid), dim3(Traits<KIND>::kThreads), 2 * SPLIT, smem, s, tm_a, tm_bc,
+                                    tm_h != nullptr ? *tm_h : tm_a, tm_gu != nullptr ? *tm_gu : tm_a,
+                                    static_cast<const CUtensorMap*>(tmap_b), offsets, bias, E, K, Nout,
+                                    static_cast<__nv_bfloat16*>(out), sc, tr, sy, Ra, status));
   return 0;
+}
+
+// How many pairs share a tile of a row-grouped product: as many as the tiles leave idle, where each still has a
+// range of eight blocks of K or more. The host does not know the routing: every expert that can have rows is taken
+// to end in half a tile. The tiles must fit in one round of clusters, and clusters stay inside a group of SMs: 32
+// clusters of four CTAs and 12 of eight did, 36 and 16 did not. The feed-forward with E 1, d 1024, f 4096, without
+// and with the split (us, nothing in L2): 1 row 48 / 32, 512 rows (8 tiles, four ranges) 50 / 40, 1024 rows (16 tiles)
+// 58 / 62 with four ranges, 1100 rows (20 tiles, two ranges) 63 / 54, 2048 (32 tiles) 73 / 64, 2304 (36) 73 / 83.
+int k_splits(int64_t M, int E, int K, int Nout) {
+  const int64_t n_tiles = (Nout + BN - 1) / BN;
+  const int64_t tiles = ((M + kPairRows - 1) / kPairRows + (E > 1 ? (M < E ? M : E) / 2 : 0)) * n_tiles;
+  const int kb = (K + BK - 1) / BK;
+  if (tiles <= 12 && kb >= 32) return 4;
+  if (tiles <= 32 && kb >= 16) return 2;
+  return 1;
+}
+int64_t max_tiles(int64_t M, int E, int Nout) {
+  return ((M + kPairRows - 1) / kPairRows + (M < E ? M : E)) * ((Nout + BN - 1) / BN);
 }
 
 }  // namespace
@@ -654,6 +740,13 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
   if (sc != nullptr)
     return launch_pair<kScatter>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, nullptr, *sc, eval, sy2, 0, status,
                                  sms, s);
+  const int split = ep_signal == nullptr && M > 0 ? k_splits(M, E, f, d) : 1;
+  if (split == 4)
+    return launch_pair<kPlain, 4>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, y, none, eval, sy2, 0, status, sms,
+                                  s, nullptr, nullptr, max_tiles(M, E, d));
+  if (split == 2)
+    return launch_pair<kPlain, 2>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, y, none, eval, sy2, 0, status, sms,
+                                  s, nullptr, nullptr, max_tiles(M, E, d));
   return launch_pair<kPlain>(tm_h, tm_h, pv.tmap_W2, offsets, pv.b2, E, f, d, y, none, eval, sy2, 0, status, sms, s);
 }
 
@@ -676,6 +769,13 @@ int launch_grouped_dx(const void* A, int64_t M, int K, const void* tmaps_b, cons
     return launch_pair<kDhGeglu>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, nullptr, none, *geglu_bwd,
                                  nosync, 0, status, sms, s, nullptr, &tm_gu);
   }
+  const int split = k_splits(M, E, K, Nout);
+  if (split == 4)
+    return launch_pair<kDx, 4>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, out, none, eval, nosync, 0, status,
+                               sms, s, nullptr, nullptr, max_tiles(M, E, Nout));
+  if (split == 2)
+    return launch_pair<kDx, 2>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, out, none, eval, nosync, 0, status,
+                               sms, s, nullptr, nullptr, max_tiles(M, E, Nout));
   return launch_pair<kDx>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, out, none, eval, nosync, 0, status, sms,
                           s);
 }

@@ -224,6 +224,22 @@ def test_experts_fp32_tile_edges(cuda_device, rows, d, f):
     assert (y.cpu().double() - y_ref).norm() <= 4e-6 * y_ref.norm()
 
 
+# the down product with its contraction split over the pairs of a cluster: four and two ranges, the last one shorter,
+# K that is no multiple of 64, a last tile of 8 columns, odd CTAs without rows, an expert without rows; 33 tiles: none
+@pytest.mark.parametrize("rows,d,f", [([700], 1024, 2056), ([300, 1, 0, 40], 520, 1032), ([2048], 1024, 1024),
+                                      ([1], 64, 2048), ([2049], 1024, 1024)])
+def test_experts_bf16_split_contraction(cuda_device, rows, d, f):
+    params, x, offsets = expert_inputs(rows, d, f, torch.bfloat16, seed=rows[0] + d)
+    dp = helpers.device_params(params, torch.bfloat16, cuda_device)
+    plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
+    h, y, status = helpers.experts(x.to(torch.bfloat16).to(cuda_device), offsets.to(cuda_device), plan)
+    assert status.cpu()[0] == 0
+    h_ref, y_ref = oracle_experts(params, x, offsets)
+    # h and y are rounded to bf16 once each (2^-9 relative) and h enters the sums of y: within 2^-7 in the 2-norm
+    assert (h.float().cpu() - h_ref).norm() <= 2 ** -7 * h_ref.norm()
+    assert (y.float().cpu() - y_ref).norm() <= 2 ** -7 * y_ref.norm()
+
+
 @pytest.mark.parametrize("rows,d,f", EXPERT_CASES)
 def test_experts_bf16(cuda_device, rows, d, f):
     params, x, offsets = expert_inputs(rows, d, f, torch.bfloat16, seed=len(rows) + d)

@@ -266,7 +266,8 @@ def test_dense_feedforward_fine_tuning_trains_the_lora_tensors(cuda_device):
 @pytest.mark.parametrize("rank,rows,f", [(5, 65, 520), (8, 129, 136), (24, 300, 1032)])
 def test_lora_gradients_at_other_ranks(cuda_device, rank, rows, f):
     """LoRA weights whose rows allow 16-byte loads (ranks that are multiples of 8) and those that do not, one and two
-    rank steps of 16, contraction ranges of 512 that end early. Tolerance as in the test above: bf16 activations and
+    rank steps of 16, contraction ranges of 512 that end early; dx = dgu W with its contraction over 2 f in one, two and
+    four ranges. Tolerance as in the test above: bf16 activations and
     gradients, fp32 sums."""
     from gemmallm_b200 import FeedForward
     d, g = 72, torch.Generator().manual_seed(rank)
@@ -276,13 +277,15 @@ def test_lora_gradients_at_other_ranks(cuda_device, rank, rows, f):
             prm.copy_(synthetic.round_to(torch.randn(prm.shape, generator=g) * 0.05, DT))
     x = synthetic.round_to(torch.randn(rows, d, generator=g), DT)
     grad_y = synthetic.round_to(torch.randn(rows, d, generator=g), DT)
-    (ff(x.to(DT).to(cuda_device).view(1, rows, d), fine_tuning=True).float() * grad_y.to(cuda_device)).sum().backward()
+    xd, xl = x.to(DT).to(cuda_device).requires_grad_(True), x.clone().requires_grad_(True)
+    (ff(xd.view(1, rows, d), fine_tuning=True).float() * grad_y.to(cuda_device)).sum().backward()
     cpu = lambda t: t.detach().float().cpu().requires_grad_(True)
     lora = {"scale": ff.lora_scale}
     for name, short in LORA_NAMES:
         lora[short + "_w"], lora[short + "_b"] = cpu(getattr(ff, name).weight), cpu(getattr(ff, name).bias)
     base = [cpu(ff.gate_and_up.weight), cpu(ff.gate_and_up.bias), cpu(ff.down.weight), cpu(ff.down.bias)]
-    (moe_oracle.expert_ffn(x, *base, lora, None) * grad_y).sum().backward()
+    (moe_oracle.expert_ffn(xl, *base, lora, None) * grad_y).sum().backward()
+    close(xd.grad, xl.grad, 3e-2, "grad x")
     for name, short in LORA_NAMES:
         close(getattr(ff, name).weight.grad, lora[short + "_w"].grad, 4e-2, f"grad {name}.weight")
         close(getattr(ff, name).bias.grad, lora[short + "_b"].grad, 4e-2, f"grad {name}.bias")
