@@ -472,6 +472,11 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   // between the decode and the prefill sizes: the streaming kernel on the sorted rows
   const bool rows_path = dtype == MOE_B200_BF16 && !small_n && N * k <= kRowsPathMaxRows &&
                          rows_supported(N * k, E);
+  // ... of which those with 192 rows an expert or more, as long as the down product is one round of 256 x 256
+  // tiles, take the prefill products behind the single-launch front: the streaming kernel reads an expert's weights
+  // once per 128 rows and is bound by L2 there. Experts and combine, d 1024, f 4096, 8 experts (us, streaming /
+  // tiles): 1024 rows 79 / 81, 1536 88 / 83, 2346 109 / 101, 3072 117 / 101, 4096 (two rounds) 134 / 157
+  const bool tiles = rows_path && tiles_at_row_counts(N * k, d, E);
   const bool counters = small_n || rows_path;
   // status words, and the completion counters behind them where a kernel uses them, in one memset
   // (a caller that keeps the region clean needs none at any size: kernels write the status words
@@ -531,7 +536,7 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
     return moe_b200_combine_decode(part, decode_splits(f), N * k, row_of, idx, w, plan, E, residual,
                                    N, d, k, out, stream);
   }
-  if (rows_path) {
+  if (rows_path && !tiles) {
     const int ks = rows_splits(N * k, d, f, E);
     rc = launch_experts_tc_rows(perm, offsets, plan, N * k, d, f, E, ks, h, part,
                                 status + MOE_B200_READY_OFFSET, status, s);

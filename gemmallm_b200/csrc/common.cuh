@@ -294,6 +294,8 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
                        int f, int E, void* h, void* y, const EpScatter* sc, int32_t* status,
                        cudaStream_t s, const TrainArgs* train = nullptr, const EpSync* ep_wait = nullptr,
                        const EpSync* ep_signal = nullptr);
+// Whether a call between the decode and the prefill sizes (M sorted rows) is better off with launch_experts_tc2.
+bool tiles_at_row_counts(int64_t M, int d, int E);
 // Input gradient of a grouped Linear: out[rows of e] = A[rows of e] . B_e, B_e [K, Nout] row-major, given by
 // the e-th tensor map of tmaps_b (64-row boxes). With geglu_bwd the product is dh (Nout = f) and is not
 // stored: the epilogue carries it back to gu (see TrainArgs).

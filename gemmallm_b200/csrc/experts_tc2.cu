@@ -704,6 +704,11 @@ int64_t max_tiles(int64_t M, int E, int Nout) {
 
 }  // namespace
 
+bool tiles_at_row_counts(int64_t M, int d, int E) {
+  const int64_t tiles = ((M + kPairRows - 1) / kPairRows + E / 2) * ((d + BN - 1) / BN);
+  return M >= (int64_t)192 * E && tiles <= kNumSMs / 2;
+}
+
 int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d,
                        int f, int E, void* h, void* y, const EpScatter* sc, int32_t* status,
                        cudaStream_t s, const TrainArgs* train, const EpSync* ep_wait,

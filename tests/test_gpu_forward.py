@@ -107,6 +107,21 @@ def test_empty_expert_and_one_hot_expert(cuda_device, dtype):
     assert last["cnt_slot"][1].tolist() == [0, N, 0, 0, 0, 0, 0, 0]
 
 
+# where calls of up to 4096 rows leave the streaming kernel for the prefill products: 192 rows an expert, and the tiles
+# of the down product in one round (74); 1534 and 1536 rows, an uneven routing, and 4096 rows of too many tiles
+@pytest.mark.parametrize("N,d,bias0", [(767, 264, 0.0), (768, 264, 0.0), (1000, 72, 2.0), (2048, 1024, 0.0)])
+def test_between_streaming_and_prefill(cuda_device, N, d, bias0):
+    E, f, k = 8, 136, 2
+    params = helpers.rounded_params(synthetic.make_params(d, E, f, seed=N), torch.bfloat16)
+    params["w1"] *= 2.0
+    params["gate_b"][0] = bias0
+    x = synthetic.round_to(synthetic.make_input(N, d, seed=N + 1), torch.bfloat16)
+    res = synthetic.round_to(synthetic.make_input(N, d, seed=N + 2), torch.bfloat16)
+    m = build(params, d, E, f, k, torch.bfloat16, cuda_device)
+    for _ in range(2):
+        check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device, residual=res)
+
+
 def test_c0_full_size_fp32(cuda_device):
     wl = synthetic.WORKLOADS["c0"]
     pins = json.loads((GOLDEN / "routing_pins.json").read_text())["c0"]
