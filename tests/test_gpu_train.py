@@ -134,6 +134,14 @@ LORA_NAMES = (("lora_gate_and_up_a", "gu_a"), ("lora_gate_and_up_b", "gu_b"),
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,k", [(37, 2), (38, 2), (39, 3)])
+def test_backward_of_token_counts_that_are_no_multiple_of_four(cuda_device, N, k):
+    """The gather of the input gradient takes four tokens a thread, with two slots all of them at once: same comparison
+    and tolerance as above."""
+    test_backward_matches_autograd_on_the_oracle(cuda_device, N, 72, 8, 136, k, 0.1)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("N,d,E,f,k,p", [(600, 128, 8, 256, 2, 0.1), (900, 256, 4, 264, 2, 0.0)])
 def test_fine_tuning_trains_the_lora_tensors(cuda_device, N, d, E, f, k, p):
     """fine_tuning=True under .train() (what the reference's fine-tuning loop runs,
