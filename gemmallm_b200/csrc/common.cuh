@@ -298,9 +298,9 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
 bool tiles_at_row_counts(int64_t M, int d, int E);
 // Input gradient of a grouped Linear: out[rows of e] = A[rows of e] . B_e, B_e [K, Nout] row-major, given by
 // the e-th tensor map of tmaps_b (64-row boxes). With geglu_bwd the product is dh (Nout = f) and is not
-// stored: the epilogue carries it back to gu (see TrainArgs).
+// stored: the epilogue carries it back to gu (see TrainArgs); round_dh rounds it to bf16 in between.
 int launch_grouped_dx(const void* A, int64_t M, int K, const void* tmaps_b, const int32_t* offsets, int E, int Nout,
-                      void* out, const TrainArgs* geglu_bwd, int32_t* status, cudaStream_t s);
+                      void* out, const TrainArgs* geglu_bwd, bool round_dh, int32_t* status, cudaStream_t s);
 // Weight gradients: out_e [Ra, Rb] = A[rows of e]^T . B[rows of e], A [M, Ra], B [M, Rb]; zeros for experts
 // without rows.
 int launch_grouped_wgrad(const void* A, const void* B, int64_t M, int Ra, int Rb, const int32_t* offsets, void* out,
@@ -375,11 +375,10 @@ int launch_colsum(const void* src, const int32_t* offsets, int64_t M, int E, int
 int launch_colsum_finish(const float* part, int slots, const int32_t* offsets, int E, int C, void* db, cudaStream_t s);
 
 // ---- lora_bwd.cu ----
-// LoRA gradients of both Linears of every expert (index 0: gate_and_up, 1: down) from the sorted activations and
-// their gradients; tab [2][E][3] device pointers A, a, B; g [E, out] gradients of the merged biases.
-int launch_lora_grads(const void* const* tab, const void* x, const void* dgu, const void* h, const void* dy,
-                      const int32_t* offsets, int64_t M, int d, int f, int E, int rank, float scale, float* scratch,
-                      const void* const (&g)[2], void* const (&dA)[2], void* const (&da)[2], void* const (&dB)[2],
-                      void* const (&db)[2], cudaStream_t s);
+// LoRA gradients of both Linears (index 0: gate_and_up, 1: down) of every expert from the gradients of their merged
+// weights G [E, out, in] and biases g [E, out]; tab [2][E][3] device pointers A, a, B.
+int launch_lora_grads(const void* const* tab, int d, int f, int E, int rank, float scale, float* scratch,
+                      const void* const (&G)[2], const void* const (&g)[2], void* const (&dA)[2], void* const (&da)[2],
+                      void* const (&dB)[2], void* const (&db)[2], cudaStream_t s);
 
 }  // namespace moe

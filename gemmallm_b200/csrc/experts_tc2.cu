@@ -68,27 +68,29 @@ enum Kind {
   kScatter,      // the same into the token owners' buffers (expert parallelism)
   kDx,           // out = A B, B [K, Nout] as it lies in memory
   kDhGeglu,      // dh = dy W2 as kDx, then back through dropout, product and GELU in the epilogue
+  kDhGegluBf16,  // the same with dh rounded to bf16 and the column sums over rounded values (LoRA steps)
   kWgrad         // out_e [Ra, Nout] = A[rows of e]^T B[rows of e]
 };
 template <int KIND>
 struct Traits {
   static constexpr bool GEGLU = KIND == kGeglu || KIND == kGegluTrain;
   static constexpr bool COLS = KIND == kWgrad;
+  static constexpr bool DH = KIND == kDhGeglu || KIND == kDhGegluBf16;
   static constexpr bool A_MN = COLS;
-  static constexpr bool B_MN = KIND == kDx || KIND == kDhGeglu || COLS;
+  static constexpr bool B_MN = KIND == kDx || DH || COLS;
   // The training epilogues do 10 to 20 instructions per accumulator element and move as much again as the
   // products' operands: sixteen warps, and further ones for what does not need the accumulator.
-  static constexpr int kEpiWarps = KIND == kGegluTrain || KIND == kDhGeglu ? 16 : 8;
-  static constexpr int kHelpers = KIND == kGegluTrain ? 4 : (KIND == kDhGeglu || COLS ? 1 : 0);
+  static constexpr int kEpiWarps = KIND == kGegluTrain || DH ? 16 : 8;
+  static constexpr int kHelpers = KIND == kGegluTrain ? 4 : (DH || COLS ? 1 : 0);
   static constexpr int kThreads = 64 + 32 * (kEpiWarps + kHelpers);
   // (kGegluTrain at 16384 tokens, d 1024, f 4096: 149 / 126 / 116 us above the inference pass with 3 / 4 / 5
   // stages, so one box per epilogue warp and a fifth stage instead of two boxes)
-  static constexpr int kStages = KIND == kGegluTrain ? 5 : (KIND == kDhGeglu ? 4 : 6);
+  static constexpr int kStages = KIND == kGegluTrain ? 5 : (DH ? 4 : 6);
   // room behind the stages (boxes want 1 KiB alignment): a box for each epilogue warp, or two chunks of gate and up
-  static constexpr int kBoxes = KIND == kGegluTrain ? 16 * kBoxBytes : (KIND == kDhGeglu ? 2 * 2 * GegluBwd::kBoxBytes : 0);
+  static constexpr int kBoxes = KIND == kGegluTrain ? 16 * kBoxBytes : (DH ? 2 * 2 * GegluBwd::kBoxBytes : 0);
   // and behind Control: staging of the epilogue warps; biases and mask bits; column sums of the lane quadrants
   static constexpr int kExtra =
-      KIND == kGegluTrain ? 16 * 256 + 2 * BM * 16 : (KIND == kDhGeglu ? 4 * 2 * BN * 4 : 8 * kStgBytes);
+      KIND == kGegluTrain ? 16 * 256 + 2 * BM * 16 : (DH ? 4 * 2 * BN * 4 : 8 * kStgBytes);
 };
 
 // M = 256 across the pair: M/16 at bit 24
@@ -449,7 +451,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->aux_full[a]);
     }
-  } else if (KIND == kDhGeglu && warp == 2 + kEpiWarps) {
+  } else if (T::DH && warp == 2 + kEpiWarps) {
     // ---------------- gate and up values: two chunks ahead, stored again as gradients ----------------
     if (lane == 0) {
       struct Place { int col, row; bool boxes; } place[2];
@@ -521,13 +523,13 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       float* s_bias = reinterpret_cast<float*>(extra + (warp - 2) * 256);
       if constexpr (KIND == kGegluTrain) GegluTrain::start(n0, Nout, bias, s_bias, lane, part);
       uint32_t keep[4];
-      if constexpr (KIND == kDhGeglu) {
+      if constexpr (T::DH) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           keep[c] = GegluBwd::mask_bits(tr, row_warp + lane, lane < rows, n0 + c * 64 + part * 16, Nout);
       }
       ok = mbar_wait(&ctl->tmem_full[a], acc_phase, &ctl->abort, status, 34);
-      if (KIND != kDhGeglu && !ok) break;
+      if (!T::DH && !ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN);
       auto release = [&]() {     // this warp has read its part of the accumulator
@@ -546,7 +548,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
         GegluTrain::finish(taddr, row_warp, rows, n0, Nout, out_e, tr, &tmap_h, &tmap_gu, s_bias, bits, box, lane, part,
                            release);
-      } else if constexpr (KIND == kDhGeglu) {
+      } else if constexpr (T::DH) {
         float* s_col = reinterpret_cast<float*>(extra);
 #pragma unroll 1
         for (int c = 0; ok && c < 4; ++c) {
@@ -565,7 +567,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           bits = c == 1 ? keep[1] : bits;
           bits = c == 2 ? keep[2] : bits;
           bits = c == 3 ? keep[3] : bits;
-          GegluBwd::chunk(v, boxes + b * 2 * GegluBwd::kBoxBytes, bits, tr.scale, lane < rows, direct, Nout, Nout - n,
+          GegluBwd::chunk<KIND == kDhGegluBf16>(v, boxes + b * 2 * GegluBwd::kBoxBytes, bits, tr.scale, lane < rows, direct, Nout, Nout - n,
                           s_col + quad * 2 * BN + c * 64 + part * 16, BN, quad, part, lane);
           fence_async_smem();
           __syncwarp();
@@ -756,7 +758,7 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
 }
 
 int launch_grouped_dx(const void* A, int64_t M, int K, const void* tmaps_b, const int32_t* offsets, int E, int Nout,
-                      void* out, const TrainArgs* geglu_bwd, int32_t* status, cudaStream_t s) {
+                      void* out, const TrainArgs* geglu_bwd, bool round_dh, int32_t* status, cudaStream_t s) {
   if (M == 0 || E == 0) return 0;
   alignas(64) CUtensorMap tm_a;
   int rc = encode_tmap_2d(&tm_a, A, (uint64_t)M, (uint64_t)K, BM);
@@ -771,6 +773,9 @@ int launch_grouped_dx(const void* A, int64_t M, int K, const void* tmaps_b, cons
     alignas(64) CUtensorMap tm_gu;
     rc = encode_tmap_2d(&tm_gu, geglu_bwd->gu, (uint64_t)M, (uint64_t)2 * Nout, BM);
     if (rc) return rc;
+    if (round_dh)
+      return launch_pair<kDhGegluBf16>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, nullptr, none, *geglu_bwd,
+                                       nosync, 0, status, sms, s, nullptr, &tm_gu);
     return launch_pair<kDhGeglu>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, nullptr, none, *geglu_bwd,
                                  nosync, 0, status, sms, s, nullptr, &tm_gu);
   }

@@ -212,7 +212,7 @@ struct ExpertGrads {
   int per = 4;
 
   template <typename Wanted>
-  moe::LoraGrads prepare(const TrainCall& c, int64_t M, const at::TensorOptions& opt, moe::TrainGrads* g, Wanted wanted) {
+  moe::LoraGrads prepare(const TrainCall& c, const at::TensorOptions& opt, moe::TrainGrads* g, Wanted wanted) {
     const int64_t E = c.E, d = c.d, f = c.f;
     per = c.rank > 0 ? 12 : 4;
     bool need[12] = {};
@@ -220,9 +220,9 @@ struct ExpertGrads {
       for (int i = 0; i < per; ++i) need[i] |= wanted(e * per + i);
     bool lora = false;
     for (int i = 4; i < per; ++i) lora |= need[i];
-    if (need[0]) w1 = at::empty({E, 2 * f, d}, opt);
+    if (need[0] || lora) w1 = at::empty({E, 2 * f, d}, opt);
     if (need[1] || lora) b1 = at::empty({E, 2 * f}, opt);
-    if (need[2]) w2 = at::empty({E, d, f}, opt);
+    if (need[2] || lora) w2 = at::empty({E, d, f}, opt);
     if (need[3] || lora) b2 = at::empty({E, d}, opt);
     auto ptr = [](Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
     g->w1 = ptr(w1);
@@ -232,7 +232,7 @@ struct ExpertGrads {
     moe::LoraGrads lg = {};
     if (lora) {
       const int64_t in[2] = {d, f}, out[2] = {2 * f, d}, r = c.rank;
-      scratch = at::empty({(int64_t)moe::lora_grads_scratch_floats(M, c.d, c.f, c.E, c.rank)}, opt.dtype(at::kFloat));
+      scratch = at::empty({(int64_t)moe::lora_grads_scratch_floats(c.d, c.f, c.E, c.rank)}, opt.dtype(at::kFloat));
       lg.tab = static_cast<const void* const*>(c.lora_tab.const_data_ptr());
       lg.rank = c.rank;
       lg.scale = (float)c.lora_scale;
@@ -303,7 +303,7 @@ struct BlockBackward : public Node {
     g.bg = gbg.defined() ? gbg.data_ptr() : nullptr;
     auto wanted = [&](int64_t i) { return task_should_compute_output(4 + (size_t)i); };
     ExpertGrads eg;
-    const moe::LoraGrads lg = eg.prepare(c, c.N * c.k, opt, &g, wanted);
+    const moe::LoraGrads lg = eg.prepare(c, opt, &g, wanted);
     if (c.N > 0) {
       check_rc(moe::backward_into(xv.const_data_ptr(), gate_w.const_data_ptr(), c.plan, go.const_data_ptr(), 0.f,
                                   aux.defined() ? aux.const_data_ptr<float>() : nullptr, c.N, c.d, c.f, c.E, c.k,
@@ -354,7 +354,7 @@ struct FfnBackward : public Node {
     g.x = gx.defined() ? gx.data_ptr() : nullptr;
     auto wanted = [&](int64_t i) { return task_should_compute_output(1 + (size_t)i); };
     ExpertGrads eg;
-    const moe::LoraGrads lg = eg.prepare(c, c.N, opt, &g, wanted);
+    const moe::LoraGrads lg = eg.prepare(c, opt, &g, wanted);
     if (c.N > 0) {
       check_rc(moe::experts_backward_into(xv.const_data_ptr(), h.const_data_ptr(), c.offsets.const_data_ptr<int32_t>(),
                                           c.plan, go.const_data_ptr(), c.N, c.d, c.f, 1, (float)p, seed, c.tws_base,

@@ -298,7 +298,9 @@ struct GegluBwd {
     return n + 8 < f ? (uint32_t)m[0] | (uint32_t)m[1] << 8 : (uint32_t)m[0];
   }
   // v: dh of this row's 16 columns; box: the chunk's gate box in shared memory, the up box behind it.
-  // direct: the row's place in gu for a chunk that cannot be stored as boxes, else nullptr; cols: columns that exist
+  // direct: the row's place in gu for a chunk that cannot be stored as boxes, else nullptr; cols: columns that exist;
+  // ROUND: dh is rounded to bf16 first, and the sums take the rounded dg and du (lora_bwd.cu says why)
+  template <bool ROUND>
   __device__ __forceinline__ static void chunk(const uint32_t (&v)[16], uint8_t* box, uint32_t keep, float scale,
                                                bool row_ok, __nv_bfloat16* direct, int f, int cols, float* s_col,
                                                int du_off, int quad, int part, int lane) {
@@ -315,7 +317,9 @@ struct GegluBwd {
       for (int i = 0; i < 8; ++i) {
         constexpr float kB = 0.7978845608028654f, kA = 0.044715f, kL = -2.f * 1.4426950408889634f;
         const int c = j * 8 + i;
-        const float dv = (keep >> c) & 1u ? __uint_as_float(v[c]) * scale : 0.f;
+        float dh = __uint_as_float(v[c]);
+        if (ROUND) dh = __bfloat162float(__float2bfloat16_rn(dh));
+        const float dv = (keep >> c) & 1u ? dh * scale : 0.f;
         const float x = (i & 1) ? bf16_hi(gw[i >> 1]) : bf16_lo(gw[i >> 1]);
         const float uv = (i & 1) ? bf16_hi(uw[i >> 1]) : bf16_lo(uw[i >> 1]);
         const float x2 = x * x;
@@ -329,6 +333,14 @@ struct GegluBwd {
                                   pack_bf16x2(dg[j * 8 + 4], dg[j * 8 + 5]), pack_bf16x2(dg[j * 8 + 6], dg[j * 8 + 7]));
       const uint4 ou = make_uint4(pack_bf16x2(du[j * 8], du[j * 8 + 1]), pack_bf16x2(du[j * 8 + 2], du[j * 8 + 3]),
                                   pack_bf16x2(du[j * 8 + 4], du[j * 8 + 5]), pack_bf16x2(du[j * 8 + 6], du[j * 8 + 7]));
+      if (ROUND) {
+        const uint32_t ogw[4] = {og.x, og.y, og.z, og.w}, ouw[4] = {ou.x, ou.y, ou.z, ou.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          dg[j * 8 + i] = (i & 1) ? bf16_hi(ogw[i >> 1]) : bf16_lo(ogw[i >> 1]);
+          du[j * 8 + i] = (i & 1) ? bf16_hi(ouw[i >> 1]) : bf16_lo(ouw[i >> 1]);
+        }
+      }
       if (direct == nullptr) {
         *gp = og;
         *up = ou;

@@ -81,27 +81,28 @@ int experts_backward(const void* perm, const void* h, const int32_t* offsets, co
     rc = launch_grouped_wgrad(dy, h, M, d, f, offsets, g.w2, E, status, s);
     if (rc) return rc;
   }
-  if (g.x == nullptr && g.w1 == nullptr && g.b1 == nullptr) return 0;   // (LoRA gradients need b1)
-  rc = launch_grouped_dx(dy, M, d, pv.tmap_W2_dec, offsets, E, f, nullptr, &tr, status, s);
+  if (g.x == nullptr && g.w1 == nullptr && g.b1 == nullptr) return 0;   // (LoRA gradients need w1)
+  rc = launch_grouped_dx(dy, M, d, pv.tmap_W2_dec, offsets, E, f, nullptr, &tr, lora != nullptr, status, s);
   if (rc) return rc;
   // gate_and_up Linear (model.py:174): db1 = column sums of dgu, dx = dgu W1, dW1 = dgu^T x
   if (g.b1 != nullptr) {
     rc = launch_colsum_finish(tr.col_part, 2, offsets, E, 2 * f, g.b1, s);
     if (rc) return rc;
   }
-  if (lora != nullptr) {
-    if (g.b1 == nullptr || g.b2 == nullptr) return set_error(MOE_B200_ERR_NULL, "LoRA gradients need b1 and b2");
-    const void* const gb[2] = {g.b1, g.b2};
-    rc = launch_lora_grads(lora->tab, perm, tr.gu, h, dy, offsets, M, d, f, E, lora->rank, lora->scale, lora->scratch,
-                           gb, lora->dA, lora->da, lora->dB, lora->db, s);
-    if (rc) return rc;
-  }
   if (g.x != nullptr) {
-    rc = launch_grouped_dx(tr.gu, M, 2 * f, pv.tmap_W1_dec, offsets, E, d, g.x, nullptr, status, s);
+    rc = launch_grouped_dx(tr.gu, M, 2 * f, pv.tmap_W1_dec, offsets, E, d, g.x, nullptr, false, status, s);
     if (rc) return rc;
   }
-  if (g.w1 == nullptr) return 0;
-  return launch_grouped_wgrad(tr.gu, perm, M, 2 * f, d, offsets, g.w1, E, status, s);
+  if (g.w1 != nullptr) {
+    rc = launch_grouped_wgrad(tr.gu, perm, M, 2 * f, d, offsets, g.w1, E, status, s);
+    if (rc) return rc;
+  }
+  if (lora == nullptr) return 0;
+  if (!g.w1 || !g.b1 || !g.w2 || !g.b2) return set_error(MOE_B200_ERR_NULL, "LoRA gradients need those of the merged weights");
+  const void* const G[2] = {g.w1, g.w2};
+  const void* const gb[2] = {g.b1, g.b2};
+  return launch_lora_grads(lora->tab, d, f, E, lora->rank, lora->scale, lora->scratch, G, gb, lora->dA, lora->da, lora->dB,
+                           lora->db, s);
 }
 
 // the gradient regions of the training workspace

@@ -494,7 +494,7 @@ class MOE(nn.Module):
         """Training forward of a call that differs from the one ``native`` was bound for: checks the arguments,
         prepares plan, workspaces and merged weights, binds them and runs. Gradients: the kernels run on the merged
         weights W' = W + s B A, b' = b + s (B a + b_lora) (model.py:175-179,185-189), whose gradients are the
-        base Linear's own; the LoRA tensors' follow from the same activations (csrc/lora_bwd.cu)."""
+        base Linear's own; the LoRA tensors' are formed from them (csrc/lora_bwd.cu)."""
         dtype = _dtype_code(tensor)
         shape = tensor.shape
         d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k

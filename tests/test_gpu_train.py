@@ -342,3 +342,51 @@ def test_experts_without_tokens_get_zero_gradients(cuda_device):
         for p in (ex.gate_and_up.weight, ex.gate_and_up.bias, ex.down.weight, ex.down.bias):
             assert torch.isfinite(p.grad).all()
             assert bool((p.grad != 0).any()) == (e < 3 and bool(m.last["cnt_slot"].sum(0)[e] > 0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,d,f,rank", [(300, 136, 264, 16), (64, 72, 520, 5), (1632, 256, 1032, 24)])
+def test_lora_step_keeps_its_rounding_points(cuda_device, rows, d, f, rank):
+    """A LoRA step rounds to bf16 where a step through the merged weights' own gradients does: pre-activations, dh, dg and
+    du, and G = dL/dW', from which the LoRA gradients are formed (an SGD step on them feeds the next pass, so other
+    rounding points drift apart from step to step). The same arithmetic in 64 bits with these roundings gives what the
+    kernels give, but for values that lie at a rounding boundary: a sum's fp32 error (about 2^-20 of it) and that of the
+    GELU's exponential (2^-21) turn less than one value in 200 of bf16's 2^-8, below 3e-4 of a 2-norm, and pass through at
+    most two further products. Without the rounding of dh the gradients differ by 3.6e-3."""
+    from gemmallm_b200 import FeedForward
+    g = torch.Generator().manual_seed(rows)
+    ff = FeedForward(d, dropout_ratio=0.0, d_ff=f, lora_rank=rank).to(device=cuda_device, dtype=DT).train()
+    with torch.no_grad():
+        for prm in ff.parameters():
+            prm.copy_(synthetic.round_to(torch.randn(prm.shape, generator=g) * 0.05, DT))
+    x = synthetic.round_to(torch.randn(rows, d, generator=g), DT)
+    dy = synthetic.round_to(torch.randn(rows, d, generator=g), DT)
+    xd = x.to(DT).to(cuda_device).requires_grad_(True)
+    ff(xd, fine_tuning=True).backward(dy.to(DT).to(cuda_device))
+    cpu = lambda t: t.detach().cpu().double()
+    bf = lambda t: t.to(DT).double()
+    s = ff.lora_scale
+    lins = [tuple(cpu(t) for lin in (w, a, b) for t in (lin.weight, lin.bias))
+            for w, a, b in ((ff.gate_and_up, ff.lora_gate_and_up_a, ff.lora_gate_and_up_b),
+                            (ff.down, ff.lora_down_a, ff.lora_down_b))]
+    (w1, b1), (w2, _) = [(bf(W + s * B @ A), bf(b + s * (B @ a + bl))) for W, b, A, a, B, bl in lins]
+    x, dy = x.double(), dy.double()
+    z, u = bf(x @ w1.t() + b1).split(f, dim=1)
+    beta, alpha = 0.7978845608028654, 0.044715
+    t = torch.tanh(beta * (z + alpha * z ** 3))
+    dgelu = 0.5 * (1 + t) + 0.5 * z * (1 - t * t) * beta * (1 + 3 * alpha * z * z)
+    dh = bf(dy @ w2)
+    dgu = bf(torch.cat((dh * u * dgelu, dh * 0.5 * z * (1 + t)), dim=1))
+    off = lambda got, ref: float((cpu(got) - ref).norm() / ref.norm())
+    assert off(xd.grad, bf(dgu @ w1)) <= 1e-3
+    assert off(ff.gate_and_up.weight.grad, bf(dgu.t() @ x)) <= 1e-3
+    assert off(ff.gate_and_up.bias.grad, bf(dgu.sum(0))) <= 1e-3
+    assert off(ff.down.bias.grad, bf(dy.sum(0))) <= 1e-3
+    # the LoRA gradients from the kernels' own G and g: one rounding behind fp32 sums
+    for (_, _, A, a, B, _), w, la, lb in zip(lins, (ff.gate_and_up, ff.down), (ff.lora_gate_and_up_a, ff.lora_down_a),
+                                             (ff.lora_gate_and_up_b, ff.lora_down_b)):
+        G, gb = cpu(w.weight.grad), cpu(w.bias.grad)
+        assert off(la.weight.grad, bf(s * B.t() @ G)) <= 5e-4
+        assert off(la.bias.grad, bf(s * B.t() @ gb)) <= 1e-3        # a few values: one at a boundary counts more
+        assert off(lb.weight.grad, bf(s * (G @ A.t() + torch.outer(gb, a)))) <= 5e-4
+        assert off(lb.bias.grad, bf(s * gb)) == 0.0
