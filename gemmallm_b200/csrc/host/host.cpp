@@ -8,6 +8,11 @@
 // for every call that differs from it in any way, and the Python side then prepares again.
 // What is bound is found changed by identity: the module tree's own dictionaries must still hold
 // the same submodules and parameters, and every parameter the same storage.
+//
+// Lifetime: a bound call owns every buffer whose address it has (plan, workspaces, merged weights): the Python side may
+// replace its own, and the parameters may leave and come back (weights exchanged for an evaluation) with the binding
+// still in place. The parameters themselves it does not own, so that moving a module away frees them; an autograd node
+// does, from its forward to its backward, because the plan that it will use has their addresses.
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -59,36 +64,26 @@ class WatchList {
  public:
   ~WatchList() { clear(); }
   void clear() {
-    for (Watch& w : items_) {
+    std::vector<Watch> old;
+    old.swap(items_);
+    params_.clear();
+    for (Watch& w : old) {
       Py_DECREF(w.dict);
       Py_DECREF(w.key);
       Py_DECREF(w.value);
     }
-    items_.clear();
-    params_.clear();
   }
-  // seq: a list of (dict, key) pairs; tensors become parameters, in order
+  // seq: a list of (dict, key) pairs; tensors become parameters, in order. Nothing is bound after an error.
   bool bind(PyObject* seq) {
-    clear();
-    const Py_ssize_t n = PyList_Size(seq);
-    if (n < 0) return false;
-    items_.reserve(n);
-    for (Py_ssize_t i = 0; i < n; ++i) {
-      PyObject *dict, *key;
-      if (!PyArg_ParseTuple(PyList_GET_ITEM(seq, i), "O!O", &PyDict_Type, &dict, &key)) return false;
-      PyObject* v = PyDict_GetItemWithError(dict, key);
-      if (v == nullptr) {
-        if (!PyErr_Occurred()) PyErr_SetObject(PyExc_KeyError, key);
-        return false;
-      }
-      Py_INCREF(dict);
-      Py_INCREF(key);
-      Py_INCREF(v);
-      const bool tensor = THPVariable_Check(v);
-      items_.push_back(Watch{dict, key, v, tensor ? THPVariable_Unpack(v).const_data_ptr() : nullptr});
-      if (tensor) params_.push_back((int)items_.size() - 1);
+    bool ok = false;
+    try {
+      ok = fill(seq);
+    } catch (...) {      // a parameter without an address
+      clear();
+      throw;
     }
-    return true;
+    if (!ok) clear();
+    return ok;
   }
   bool unchanged() const {
     for (const Watch& w : items_) {
@@ -105,6 +100,28 @@ class WatchList {
   bool empty() const { return items_.empty(); }
 
  private:
+  bool fill(PyObject* seq) {
+    clear();
+    const Py_ssize_t n = PyList_Size(seq);
+    if (n < 0) return false;
+    items_.reserve(n);
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      PyObject *dict, *key;
+      if (!PyArg_ParseTuple(PyList_GET_ITEM(seq, i), "O!O", &PyDict_Type, &dict, &key)) return false;
+      PyObject* v = PyDict_GetItemWithError(dict, key);
+      if (v == nullptr) {
+        if (!PyErr_Occurred()) PyErr_SetObject(PyExc_KeyError, key);
+        return false;
+      }
+      const bool tensor = THPVariable_Check(v);
+      items_.push_back(Watch{dict, key, v, tensor ? THPVariable_Unpack(v).const_data_ptr() : nullptr});
+      Py_INCREF(dict);
+      Py_INCREF(key);
+      Py_INCREF(v);
+      if (tensor) params_.push_back((int)items_.size() - 1);
+    }
+    return true;
+  }
   std::vector<Watch> items_;
   std::vector<int> params_;
 };
@@ -182,9 +199,25 @@ using torch::autograd::Node;
 using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 
+bool tensor_list(PyObject* seq, std::vector<Tensor>* out) {
+  out->clear();
+  const Py_ssize_t n = PyList_Size(seq);
+  if (n < 0) return false;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* t = PyList_GET_ITEM(seq, i);
+    if (!THPVariable_Check(t)) {
+      PyErr_SetString(PyExc_TypeError, "buffers must be tensors");
+      return false;
+    }
+    out->push_back(THPVariable_Unpack(t));
+  }
+  return true;
+}
+
 // What a prepared training call works on; shared by the module and the nodes of its calls.
 struct TrainCall {
   Tensor ws, tws, offsets, status, lora_tab;    // buffers kept alive
+  std::vector<Tensor> owned;                    // plan and merged weights likewise
   const void* plan = nullptr;
   void *ws_base = nullptr, *tws_base = nullptr;
   size_t ws_bytes = 0, tws_bytes = 0;
@@ -275,12 +308,16 @@ struct BlockBackward : public Node {
   std::shared_ptr<TrainCall> call;
   SavedVariable x;
   Tensor gate_w;
+  std::vector<c10::Storage> weights;    // of the parameters whose addresses the plan has
   int64_t gen = 0;
   uint64_t seed = 0;
   double p = 0.0;
 
   std::string name() const override { return "MOEBackward"; }
-  void release_variables() override { x.reset_data(); }
+  void release_variables() override {
+    x.reset_data();
+    weights.clear();
+  }
   variable_list apply(variable_list&& grads) override {
     const TrainCall& c = *call;
     check_generation(c, gen);
@@ -329,6 +366,7 @@ struct FfnBackward : public Node {
   std::shared_ptr<TrainCall> call;
   SavedVariable x;
   Tensor h;
+  std::vector<c10::Storage> weights;
   int64_t gen = 0;
   uint64_t seed = 0;
   double p = 0.0;
@@ -337,6 +375,7 @@ struct FfnBackward : public Node {
   void release_variables() override {
     x.reset_data();
     h.reset();
+    weights.clear();
   }
   variable_list apply(variable_list&& grads) override {
     const TrainCall& c = *call;
@@ -372,9 +411,13 @@ struct FfnBackward : public Node {
   }
 };
 
-// Edges of a call's inputs; false when none of them wants a gradient (or gradients are off).
+// Edges of a call's inputs, and the storages of those that are parameters.
 class Edges {
  public:
+  void add_param(const Tensor& t) {
+    add(t);
+    weights_.push_back(t.storage());
+  }
   void add(const Tensor& t) {
     any_ |= t.requires_grad();
     list_.push_back(torch::autograd::impl::gradient_edge(t));
@@ -382,9 +425,11 @@ class Edges {
   void add_empty() { list_.emplace_back(); }
   bool wanted() const { return any_ && at::GradMode::is_enabled(); }
   edge_list take() { return std::move(list_); }
+  std::vector<c10::Storage> take_weights() { return std::move(weights_); }
 
  private:
   edge_list list_;
+  std::vector<c10::Storage> weights_;
   bool any_ = false;
 };
 
@@ -397,6 +442,7 @@ struct Block {
   WatchList* watch;       // [0], [1]: the router's weight and bias, then the experts' tensors
   LoraJobs* lora;
   Tensor* workspace;
+  std::vector<Tensor>* owned;     // plan and merged weights
   std::shared_ptr<TrainCall>* train;
   const void* plan;
   void* ws_base;
@@ -441,6 +487,7 @@ PyObject* block_new(PyTypeObject* type, PyObject*, PyObject*) {
   self->watch = new WatchList();
   self->lora = new LoraJobs();
   self->workspace = new Tensor();
+  self->owned = new std::vector<Tensor>();
   self->train = new std::shared_ptr<TrainCall>();
   return reinterpret_cast<PyObject*>(self);
 }
@@ -451,27 +498,28 @@ void block_dealloc(PyObject* o) {
   delete self->watch;
   delete self->lora;
   delete self->workspace;
+  delete self->owned;
   delete self->train;
   type->tp_free(o);
   Py_DECREF(type);
 }
 
-// bind(watch, lora or None, plan, workspace tensor, base, bytes, N, d, f, E, k, dtype, device index)
+// bind(watch, lora or None, plan, owned buffers, workspace tensor, base, bytes, N, d, f, E, k, dtype, device index)
 PyObject* block_bind(PyObject* o, PyObject* args) {
   HANDLE_TH_ERRORS
   Block* self = reinterpret_cast<Block*>(o);
-  PyObject *watch, *lora, *ws;
+  PyObject *watch, *lora, *owned, *ws;
   unsigned long long plan, base, bytes;
   long long N;
   int d, f, E, k, dtype, device;
-  if (!PyArg_ParseTuple(args, "O!OKOKKLiiiiii", &PyList_Type, &watch, &lora, &plan, &ws, &base, &bytes, &N, &d, &f,
+  if (!PyArg_ParseTuple(args, "O!OKO!OKKLiiiiii", &PyList_Type, &watch, &lora, &plan, &PyList_Type, &owned, &ws, &base, &bytes, &N, &d, &f,
                         &E, &k, &dtype, &device))
     return nullptr;
   if (!THPVariable_Check(ws)) {
     PyErr_SetString(PyExc_TypeError, "workspace must be a tensor");
     return nullptr;
   }
-  if (!self->watch->bind(watch) || !self->lora->bind(lora, *self->watch)) {
+  if (!tensor_list(owned, self->owned) || !self->watch->bind(watch) || !self->lora->bind(lora, *self->watch)) {
     self->watch->clear();
     return nullptr;
   }
@@ -494,6 +542,7 @@ PyObject* block_unbind(PyObject* o, PyObject*) {
   Block* self = reinterpret_cast<Block*>(o);
   self->watch->clear();
   *self->workspace = Tensor();
+  self->owned->clear();
   self->train->reset();
   Py_RETURN_NONE;
 }
@@ -509,6 +558,7 @@ PyObject* block_bind_train(PyObject* o, PyObject* args) {
   if (!PyArg_ParseTuple(args, "OKKOid", &tws, &base, &bytes, &tab, &rank, &scale)) return nullptr;
   auto c = std::make_shared<TrainCall>();
   c->ws = *self->workspace;
+  c->owned = *self->owned;
   c->tws = THPVariable_Unpack(tws);
   if (tab != Py_None) c->lora_tab = THPVariable_Unpack(tab);
   c->plan = self->plan;
@@ -609,7 +659,7 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     if (self->watch->empty() || !self->watch->unchanged()) Py_RETURN_NONE;
     gate_w = self->watch->param(0);
     gate_b = self->watch->param(1);
-    for (int i = 0; i < self->watch->num_params(); ++i) edges.add(self->watch->param(i));
+    for (int i = 0; i < self->watch->num_params(); ++i) edges.add_param(self->watch->param(i));
   } else {
     const Py_ssize_t n = PyList_Size(args[3]);
     if (n < 2) {
@@ -622,7 +672,7 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
         PyErr_SetString(PyExc_TypeError, "parameters must be tensors");
         return nullptr;
       }
-      edges.add(THPVariable_Unpack(v));
+      edges.add_param(THPVariable_Unpack(v));
     }
     gate_w = THPVariable_Unpack(PyList_GET_ITEM(args[3], 0));
     gate_b = THPVariable_Unpack(PyList_GET_ITEM(args[3], 1));
@@ -649,6 +699,7 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   if (edges.wanted()) {
     auto node = std::shared_ptr<BlockBackward>(new BlockBackward(), torch::autograd::deleteNode);
     node->set_next_edges(edges.take());
+    node->weights = edges.take_weights();
     node->call = c;
     node->gen = c->gen;
     node->seed = seed;
@@ -689,6 +740,7 @@ struct Ffn {
   PyObject_HEAD
   WatchList* watch;
   LoraJobs* lora;
+  std::vector<Tensor>* owned;   // plan and merged weights
   Tensor* offsets;        // int32 [0, M]
   Tensor* status;         // int32 [16], written only when a wait inside a kernel ran out
   std::shared_ptr<TrainCall>* train;
@@ -702,6 +754,7 @@ PyObject* ffn_new(PyTypeObject* type, PyObject*, PyObject*) {
   if (self == nullptr) return nullptr;
   self->watch = new WatchList();
   self->lora = new LoraJobs();
+  self->owned = new std::vector<Tensor>();
   self->offsets = new Tensor();
   self->status = new Tensor();
   self->train = new std::shared_ptr<TrainCall>();
@@ -713,6 +766,7 @@ void ffn_dealloc(PyObject* o) {
   PyTypeObject* type = Py_TYPE(o);
   delete self->watch;
   delete self->lora;
+  delete self->owned;
   delete self->offsets;
   delete self->status;
   delete self->train;
@@ -720,22 +774,22 @@ void ffn_dealloc(PyObject* o) {
   Py_DECREF(type);
 }
 
-// bind(watch, lora or None, plan, offsets, status, M, d, f, dtype, device index)
+// bind(watch, lora or None, plan, owned buffers, offsets, status, M, d, f, dtype, device index)
 PyObject* ffn_bind(PyObject* o, PyObject* args) {
   HANDLE_TH_ERRORS
   Ffn* self = reinterpret_cast<Ffn*>(o);
-  PyObject *watch, *lora, *offsets, *status;
+  PyObject *watch, *lora, *owned, *offsets, *status;
   unsigned long long plan;
   long long M;
   int d, f, dtype, device;
-  if (!PyArg_ParseTuple(args, "O!OKOOLiiii", &PyList_Type, &watch, &lora, &plan, &offsets, &status, &M, &d, &f,
+  if (!PyArg_ParseTuple(args, "O!OKO!OOLiiii", &PyList_Type, &watch, &lora, &plan, &PyList_Type, &owned, &offsets, &status, &M, &d, &f,
                         &dtype, &device))
     return nullptr;
   if (!THPVariable_Check(offsets) || !THPVariable_Check(status)) {
     PyErr_SetString(PyExc_TypeError, "offsets and status must be tensors");
     return nullptr;
   }
-  if (!self->watch->bind(watch) || !self->lora->bind(lora, *self->watch)) {
+  if (!tensor_list(owned, self->owned) || !self->watch->bind(watch) || !self->lora->bind(lora, *self->watch)) {
     self->watch->clear();
     return nullptr;
   }
@@ -752,8 +806,10 @@ PyObject* ffn_bind(PyObject* o, PyObject* args) {
 }
 
 PyObject* ffn_unbind(PyObject* o, PyObject*) {
-  reinterpret_cast<Ffn*>(o)->watch->clear();
-  reinterpret_cast<Ffn*>(o)->train->reset();
+  Ffn* self = reinterpret_cast<Ffn*>(o);
+  self->watch->clear();
+  self->owned->clear();
+  self->train->reset();
   Py_RETURN_NONE;
 }
 
@@ -768,6 +824,7 @@ PyObject* ffn_bind_train(PyObject* o, PyObject* args) {
   if (!PyArg_ParseTuple(args, "OKKOid", &tws, &base, &bytes, &tab, &rank, &scale)) return nullptr;
   auto c = std::make_shared<TrainCall>();
   c->tws = THPVariable_Unpack(tws);
+  c->owned = *self->owned;
   c->offsets = *self->offsets;
   c->status = *self->status;
   if (tab != Py_None) c->lora_tab = THPVariable_Unpack(tab);
@@ -805,7 +862,7 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   edges.add(x);
   if (args[2] == Py_None) {
     if (self->watch->empty() || !self->watch->unchanged()) Py_RETURN_NONE;
-    for (int i = 0; i < self->watch->num_params(); ++i) edges.add(self->watch->param(i));
+    for (int i = 0; i < self->watch->num_params(); ++i) edges.add_param(self->watch->param(i));
   } else {
     const Py_ssize_t n = PyList_Size(args[2]);
     if (n < 0) return nullptr;
@@ -815,7 +872,7 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
         PyErr_SetString(PyExc_TypeError, "parameters must be tensors");
         return nullptr;
       }
-      edges.add(THPVariable_Unpack(v));
+      edges.add_param(THPVariable_Unpack(v));
     }
   }
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)c->device);
@@ -839,6 +896,7 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   if (edges.wanted()) {
     auto node = std::shared_ptr<FfnBackward>(new FfnBackward(), torch::autograd::deleteNode);
     node->set_next_edges(edges.take());
+    node->weights = edges.take_weights();
     node->call = c;
     node->gen = c->gen;
     node->seed = seed;

@@ -111,6 +111,9 @@ class _MergedLora:
             self.key = key
         return self.merged
 
+    def buffers(self) -> list:
+        return [t for mg in self.merged for lin in (mg.gate_and_up, mg.down) for t in (lin.weight, lin.bias)]
+
 
 def _lora_table(experts, dev) -> torch.Tensor:
     """Device table of the LoRA tensors' addresses, [2 Linears][experts][A, a, B], for their gradients."""
@@ -201,6 +204,10 @@ class FeedForward(nn.Module):
             self._offsets = ((M, str(dev)), torch.tensor([0, M], dtype=torch.int32, device=dev))
         return x, M, dev, self._offsets[1]
 
+    def _owned(self, fine_tuning: bool) -> list:
+        """Buffers whose addresses a bound call has, besides workspaces: the plan and the merged weights."""
+        return [self._plan_ft.buf, *self._lora.buffers()] if fine_tuning else [self._plan.buf]
+
     # -- training mode (bf16): dropout on h and a backward pass -----------------
     def _train_ws(self, M: int, device: torch.device):
         key = (M, str(device))
@@ -236,7 +243,8 @@ class FeedForward(nn.Module):
             usual = all(name in table for table, name in watch)
             jobs = _lora_jobs(self, self._lora.merged[0], 0) if fine_tuning and usual else None
             native.unbind()
-            native.bind(watch if usual else [], jobs, plan, offsets, status, M, d, f, _cabi.BF16, dev.index)
+            native.bind(watch if usual else [], jobs, plan, self._owned(fine_tuning), offsets, status, M, d, f, _cabi.BF16,
+                        dev.index)
             table = _lora_table([self], dev) if fine_tuning else None
             native.bind_train(buf, tbase, tbytes, table, self.lora_down_a.out_features if fine_tuning else 0,
                               float(self.lora_scale))
@@ -285,7 +293,7 @@ class FeedForward(nn.Module):
         watch = _expert_watch(self, fine_tuning)
         if x.shape[-1] == d and all(name in table for table, name in watch):
             jobs = _lora_jobs(self, self._lora.merged[0], 0) if fine_tuning else None
-            native.bind(watch, jobs, plan, offsets, status, M, d, f, dtype, dev.index)
+            native.bind(watch, jobs, plan, self._owned(fine_tuning), offsets, status, M, d, f, dtype, dev.index)
         return y.reshape(shape)
 
 
@@ -471,7 +479,8 @@ class MOE(nn.Module):
             jobs = [job for e, (ex, mg) in enumerate(zip(self.experts, self._lora.merged))
                     for job in _lora_jobs(ex, mg, 2 + 12 * e)]
         buf, base, nbytes, _ = self._ws
-        native.bind(watch, jobs, plan, buf, base, nbytes, N, d, f, E, k, dtype, dev.index)
+        owned = [self._plan_ft.buf, *self._lora.buffers()] if fine_tuning else [self._plan.buf]
+        native.bind(watch, jobs, plan, owned, buf, base, nbytes, N, d, f, E, k, dtype, dev.index)
 
     # -- training mode -------------------------------------------------------
     def _train_workspace(self, N: int, device: torch.device):

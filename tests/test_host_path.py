@@ -1,0 +1,162 @@
+"""The modules' native host path (csrc/host/host.cpp): calls bound to a prepared state, in sequences of calls that
+change that state. What a sequence gives is compared with the same last call on a module built afresh from the same
+parameters, which has nothing to remember: the kernels are the same, so the results are equal bit for bit."""
+import gc
+import weakref
+
+import pytest
+import torch
+
+from gemmallm_b200 import MOE, FeedForward, _host
+
+DT = torch.bfloat16
+D, F, E, RANK = 64, 128, 4, 16
+
+
+def build(kind, dev, seed=0, rank=RANK, p=0.1):
+    torch.manual_seed(seed)
+    m = (MOE(D, num_experts=E, d_ff=F, dropout_ratio=p, lora_rank=rank, device="cuda") if kind == "moe"
+         else FeedForward(D, d_ff=F, dropout_ratio=p, lora_rank=rank))
+    return m.to(device=dev, dtype=DT)
+
+
+def fresh_copy(m, kind, dev, **kw):
+    new = build(kind, dev, **kw)
+    new.load_state_dict(m.state_dict())
+    return new
+
+
+def rows(n, dev, seed=1):
+    return torch.randn(n, D, generator=torch.Generator().manual_seed(seed)).to(DT).to(dev)
+
+
+def forward(m, x, fine_tuning=False, **kw):
+    out = m(x, fine_tuning=fine_tuning, **kw)
+    return out if isinstance(out, tuple) else (out,)
+
+
+def train_step(m, x, fine_tuning=False, mask_seed=5):
+    """Output and every gradient of one training step."""
+    m.train()
+    x = x.detach().clone().requires_grad_(True)
+    for p in m.parameters():
+        p.grad = None
+    torch.manual_seed(mask_seed)
+    out = forward(m, x, fine_tuning)
+    sum((o.float() ** 2).sum() for o in out).backward()
+    return [*(o.detach() for o in out), x.grad, *(p.grad for p in m.parameters() if p.grad is not None)]
+
+
+def same(got, want):
+    assert len(got) == len(want)
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b), f"tensor {i}: {float((a.float() - b.float()).abs().max())}"
+
+
+KINDS = ["moe", "ffn"]
+
+
+# ---- who owns what a bound call has the address of --------------------------------------------
+
+@pytest.mark.parametrize("train", [False, True])
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_bound_call_owns_its_buffers(kind, train):
+    """Plan, merged weights and workspaces belong to the binding until it is released, whatever the Python side drops."""
+    table = {"weight": torch.zeros(1), "bias": torch.zeros(1)}
+    watch = [(table, "weight"), (table, "bias")]
+    buffers = [torch.zeros(8, dtype=torch.uint8) for _ in range(4)]
+    refs = [weakref.ref(t) for t in buffers]
+    if kind == "moe":
+        native = _host.Block()
+        native.bind(watch, None, 0, buffers[:2], buffers[2], 0, 0, 1, D, F, E, 2, 1, 0)
+    else:
+        native = _host.Ffn()
+        native.bind(watch, None, 0, buffers[:2], buffers[2], buffers[2], 1, D, F, 1, 0)
+    if train:
+        native.bind_train(buffers[3], 0, 0, None, 0, 1.0)
+    else:
+        del refs[3]
+    del buffers
+    gc.collect()
+    assert all(r() is not None for r in refs)
+    native.unbind()
+    gc.collect()
+    assert refs[0]() is None and refs[1]() is None
+
+
+def test_nothing_is_bound_after_an_error():
+    table = {"weight": torch.zeros(1)}
+    native = _host.Ffn()
+    status = torch.zeros(16, dtype=torch.int32)
+    with pytest.raises(KeyError):
+        native.bind([(table, "weight"), (table, "bias")], None, 0, [status], status, status, 1, D, F, 1, 0)
+    assert native.forward(torch.zeros(1, D, dtype=DT)) is None
+
+
+def exchange(params, others):
+    for p, q in zip(params, others):
+        p.data, q.data = q.data, p.data
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fine_tuning", [False])
+@pytest.mark.parametrize("kind", KINDS)
+def test_weights_exchanged_for_an_evaluation_and_back(cuda_device, kind, fine_tuning):
+    """Averaged weights by .data for an evaluation: the training call bound before it is right afterwards."""
+    m, x = build(kind, cuda_device), rows(48, cuda_device)
+    averaged = [torch.empty_like(p).normal_(0, 0.1) for p in m.parameters()]
+    for _ in range(3):
+        train_step(m, x, fine_tuning)
+    with torch.no_grad():
+        exchange(list(m.parameters()), averaged)
+        m.eval()
+        for _ in range(3):
+            got = forward(m, x, fine_tuning)
+        fresh = fresh_copy(m, kind, cuda_device).eval()
+        same(got, forward(fresh, x, fine_tuning))
+        exchange(list(m.parameters()), averaged)
+    for p in averaged:
+        p.fill_(float("nan"))
+    want = train_step(fresh_copy(m, kind, cuda_device), x, fine_tuning)
+    same(train_step(m, x, fine_tuning), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fine_tuning", [False, True])
+@pytest.mark.parametrize("kind", KINDS)
+def test_backward_after_the_module_and_its_weights_are_gone(cuda_device, kind, fine_tuning):
+    """Between forward and backward a node keeps everything it reads: plan, weights, merged weights, workspaces."""
+    x = rows(48, cuda_device)
+    xs, grads = [], []
+    for drop in (False, True):
+        m = build(kind, cuda_device).train().requires_grad_(False)
+        xd = x.clone().requires_grad_(True)
+        for i in range(2):       # prepared, then bound
+            torch.manual_seed(i)
+            out = forward(m, xd, fine_tuning)
+        if drop:
+            del m
+            gc.collect()
+            junk = [torch.full((1 << 20,), float("nan"), device=cuda_device) for _ in range(8)]
+        out[0].float().sum().backward()
+        torch.cuda.synchronize()
+        xs.append(out[0].detach())
+        grads.append(xd.grad)
+    del junk
+    assert torch.equal(xs[0], xs[1]) and torch.equal(grads[0], grads[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_module_that_ran_can_be_freed(cuda_device, kind):
+    m, x = build(kind, cuda_device), rows(48, cuda_device)
+    for fine_tuning in (False, True):
+        for _ in range(2):
+            train_step(m, x, fine_tuning)
+            with torch.no_grad():
+                forward(m.eval(), x, fine_tuning)
+    ref = weakref.ref(m)
+    weight = weakref.ref(next(m.parameters()))
+    del m
+    gc.collect()
+    assert ref() is None and weight() is None
