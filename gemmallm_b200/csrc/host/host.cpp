@@ -214,6 +214,37 @@ bool tensor_list(PyObject* seq, std::vector<Tensor>* out) {
   return true;
 }
 
+// Number of forwards on a training workspace, of all bindings that share it: a backward must belong to the last.
+struct Generation {
+  PyObject_HEAD
+  std::shared_ptr<int64_t>* count;
+};
+
+PyObject* generation_new(PyTypeObject* type, PyObject*, PyObject*) {
+  Generation* self = reinterpret_cast<Generation*>(type->tp_alloc(type, 0));
+  if (self == nullptr) return nullptr;
+  self->count = new std::shared_ptr<int64_t>(std::make_shared<int64_t>(0));
+  return reinterpret_cast<PyObject*>(self);
+}
+
+void generation_dealloc(PyObject* o) {
+  PyTypeObject* type = Py_TYPE(o);
+  delete reinterpret_cast<Generation*>(o)->count;
+  type->tp_free(o);
+  Py_DECREF(type);
+}
+
+PyTypeObject* g_generation_type = nullptr;
+
+bool read_generation(PyObject* o, std::shared_ptr<int64_t>* out) {
+  if (!PyObject_TypeCheck(o, g_generation_type)) {
+    PyErr_SetString(PyExc_TypeError, "generation must be a Generation");
+    return false;
+  }
+  *out = *reinterpret_cast<Generation*>(o)->count;
+  return true;
+}
+
 // What a prepared training call works on; shared by the module and the nodes of its calls.
 struct TrainCall {
   Tensor ws, tws, offsets, status, lora_tab;    // buffers kept alive
@@ -224,7 +255,7 @@ struct TrainCall {
   int64_t N = 0;
   int d = 0, f = 0, E = 0, k = 0, device = 0, rank = 0;
   double lora_scale = 0.0;
-  int64_t gen = 0;          // number of forwards: a backward must belong to the last one
+  std::shared_ptr<int64_t> gen;
 };
 
 uint64_t draw_seed() {      // torch's CPU generator, as torch.randint(0, 2**62, (1,)) in Python
@@ -298,7 +329,7 @@ Tensor output_grad(const Tensor& g, const Tensor& like) {
 }
 
 void check_generation(const TrainCall& c, int64_t gen) {
-  if (c.gen != gen)
+  if (*c.gen != gen)
     throw std::runtime_error("this module ran another training forward before the backward of this one: its "
                              "workspace holds the later call's tensors");
 }
@@ -547,16 +578,17 @@ PyObject* block_unbind(PyObject* o, PyObject*) {
   Py_RETURN_NONE;
 }
 
-// bind_train(training workspace, base, bytes, LoRA pointer table or None, rank, scale): after bind()
+// bind_train(training workspace, base, bytes, LoRA pointer table or None, rank, scale, generation): after bind()
 PyObject* block_bind_train(PyObject* o, PyObject* args) {
   HANDLE_TH_ERRORS
   Block* self = reinterpret_cast<Block*>(o);
-  PyObject *tws, *tab;
+  PyObject *tws, *tab, *gen;
   unsigned long long base, bytes;
   int rank;
   double scale;
-  if (!PyArg_ParseTuple(args, "OKKOid", &tws, &base, &bytes, &tab, &rank, &scale)) return nullptr;
+  if (!PyArg_ParseTuple(args, "OKKOidO", &tws, &base, &bytes, &tab, &rank, &scale, &gen)) return nullptr;
   auto c = std::make_shared<TrainCall>();
+  if (!read_generation(gen, &c->gen)) return nullptr;
   c->ws = *self->workspace;
   c->owned = *self->owned;
   c->tws = THPVariable_Unpack(tws);
@@ -695,13 +727,13 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
         c->ws_bytes, c->tws_base, c->tws_bytes, out.data_ptr(), aux.data_ptr<float>(), stream);
     if (rc != 0) return fail(rc, "forward_train");
   }
-  ++c->gen;
+  ++*c->gen;
   if (edges.wanted()) {
     auto node = std::shared_ptr<BlockBackward>(new BlockBackward(), torch::autograd::deleteNode);
     node->set_next_edges(edges.take());
     node->weights = edges.take_weights();
     node->call = c;
-    node->gen = c->gen;
+    node->gen = *c->gen;
     node->seed = seed;
     node->p = p;
     node->gate_w = gate_w.detach();
@@ -813,16 +845,17 @@ PyObject* ffn_unbind(PyObject* o, PyObject*) {
   Py_RETURN_NONE;
 }
 
-// bind_train(training workspace, base, bytes, LoRA pointer table or None, rank, scale): after bind()
+// bind_train(training workspace, base, bytes, LoRA pointer table or None, rank, scale, generation): after bind()
 PyObject* ffn_bind_train(PyObject* o, PyObject* args) {
   HANDLE_TH_ERRORS
   Ffn* self = reinterpret_cast<Ffn*>(o);
-  PyObject *tws, *tab;
+  PyObject *tws, *tab, *gen;
   unsigned long long base, bytes;
   int rank;
   double scale;
-  if (!PyArg_ParseTuple(args, "OKKOid", &tws, &base, &bytes, &tab, &rank, &scale)) return nullptr;
+  if (!PyArg_ParseTuple(args, "OKKOidO", &tws, &base, &bytes, &tab, &rank, &scale, &gen)) return nullptr;
   auto c = std::make_shared<TrainCall>();
+  if (!read_generation(gen, &c->gen)) return nullptr;
   c->tws = THPVariable_Unpack(tws);
   c->owned = *self->owned;
   c->offsets = *self->offsets;
@@ -892,13 +925,13 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
                                           c->status.data_ptr<int32_t>(), stream);
     if (rc != 0) return fail(rc, "experts_train");
   }
-  ++c->gen;
+  ++*c->gen;
   if (edges.wanted()) {
     auto node = std::shared_ptr<FfnBackward>(new FfnBackward(), torch::autograd::deleteNode);
     node->set_next_edges(edges.take());
     node->weights = edges.take_weights();
     node->call = c;
-    node->gen = c->gen;
+    node->gen = *c->gen;
     node->seed = seed;
     node->p = p;
     node->h = std::move(h);
@@ -946,6 +979,13 @@ PyMethodDef ffn_methods[] = {
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(ffn_forward)), METH_FASTCALL, nullptr},
     {"__reduce__", fresh_reduce, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr}};
+PyMethodDef generation_methods[] = {{"__reduce__", fresh_reduce, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyType_Slot generation_slots[] = {{Py_tp_new, reinterpret_cast<void*>(generation_new)},
+                                  {Py_tp_dealloc, reinterpret_cast<void*>(generation_dealloc)},
+                                  {Py_tp_methods, generation_methods},
+                                  {0, nullptr}};
+PyType_Spec generation_spec = {"gemmallm_b200._host.Generation", sizeof(Generation), 0, Py_TPFLAGS_DEFAULT, generation_slots};
+
 PyType_Slot ffn_slots[] = {{Py_tp_new, reinterpret_cast<void*>(ffn_new)},
                            {Py_tp_dealloc, reinterpret_cast<void*>(ffn_dealloc)},
                            {Py_tp_methods, ffn_methods},
@@ -954,11 +994,15 @@ PyType_Spec ffn_spec = {"gemmallm_b200._host.Ffn", sizeof(Ffn), 0, Py_TPFLAGS_DE
 
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
 
-bool add_type(PyObject* m, const char* name, PyType_Spec* spec) {
+bool add_type(PyObject* m, const char* name, PyType_Spec* spec, PyTypeObject** keep = nullptr) {
   PyObject* t = PyType_FromSpec(spec);
   if (t == nullptr) return false;
   const int rc = PyModule_AddObjectRef(m, name, t);
-  Py_DECREF(t);
+  if (keep != nullptr && rc == 0) {
+    *keep = reinterpret_cast<PyTypeObject*>(t);      // for the life of the process
+  } else {
+    Py_DECREF(t);
+  }
   return rc == 0;
 }
 
@@ -971,7 +1015,8 @@ PyMODINIT_FUNC PyInit__host(void) {
   s_bias = PyUnicode_InternFromString("bias");
   s_parameters = PyUnicode_InternFromString("_parameters");
   s_eps = PyUnicode_InternFromString("eps");
-  if (!add_type(m, "Block", &block_spec) || !add_type(m, "Ffn", &ffn_spec)) {
+  if (!add_type(m, "Block", &block_spec) || !add_type(m, "Ffn", &ffn_spec) ||
+      !add_type(m, "Generation", &generation_spec, &g_generation_type)) {
     Py_DECREF(m);
     return nullptr;
   }

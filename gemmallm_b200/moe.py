@@ -195,6 +195,7 @@ class FeedForward(nn.Module):
         self._offsets = None   # ((rows, device), int32 [0, rows]) of the last call
         self._tws = None
         self._tws_key = None
+        self._generation = None   # counts the forwards on _tws
         self.last_seed = None
 
     def _rows(self, tensor):
@@ -220,6 +221,7 @@ class FeedForward(nn.Module):
             base = (buf.data_ptr() + 1023) & ~1023
             check(lib.moe_b200_train_setup(M, d, f, 1, 1, _cabi.BF16, base, nbytes, _stream(device)), "train_setup")
             self._tws = (buf, base, nbytes)
+            self._generation = _host.Generation()
             self._tws_key = key
             self._native_train.unbind()
             self._native_train_ft.unbind()
@@ -247,7 +249,7 @@ class FeedForward(nn.Module):
                         dev.index)
             table = _lora_table([self], dev) if fine_tuning else None
             native.bind_train(buf, tbase, tbytes, table, self.lora_down_a.out_features if fine_tuning else 0,
-                              float(self.lora_scale))
+                              float(self.lora_scale), self._generation)
             # the tensors themselves, wherever the module tree keeps them
             y, seed = native.train(x, float(self.dropout.p), _expert_params(self, fine_tuning))
         return y.reshape(tensor.shape), seed
@@ -326,6 +328,7 @@ class MOE(nn.Module):
         self._ws_key = None
         self._tws = None
         self._tws_key = None
+        self._generation = None   # counts the forwards on _tws
         self._last_seed = None
         # native calls prepared for the last input size: plain, and with the LoRA branches merged
         self._native, self._native_ft = _host.Block(), _host.Block()
@@ -494,6 +497,7 @@ class MOE(nn.Module):
             base = (buf.data_ptr() + 1023) & ~1023
             check(lib.moe_b200_train_setup(N, d, f, E, k, _cabi.BF16, base, nbytes, _stream(device)), "train_setup")
             self._tws = (buf, base, nbytes)
+            self._generation = _host.Generation()
             self._tws_key = key
             self._native_train.unbind()
             self._native_train_ft.unbind()
@@ -527,7 +531,7 @@ class MOE(nn.Module):
             table = _lora_table(self.experts, dev) if fine_tuning else None
             ex = self.experts[0]
             native.bind_train(buf, tbase, tbytes, table, ex.lora_down_a.out_features if fine_tuning else 0,
-                              float(ex.lora_scale))
+                              float(ex.lora_scale), self._generation)
             # the tensors themselves, wherever the module tree keeps them
             params = [self.gate.weight, self.gate.bias]
             for ex in self.experts:

@@ -73,7 +73,7 @@ def test_a_bound_call_owns_its_buffers(kind, train):
         native = _host.Ffn()
         native.bind(watch, None, 0, buffers[:2], buffers[2], buffers[2], 1, D, F, 1, 0)
     if train:
-        native.bind_train(buffers[3], 0, 0, None, 0, 1.0)
+        native.bind_train(buffers[3], 0, 0, None, 0, 1.0, _host.Generation())
     else:
         del refs[3]
     del buffers
@@ -160,3 +160,53 @@ def test_a_module_that_ran_can_be_freed(cuda_device, kind):
     del m
     gc.collect()
     assert ref() is None and weight() is None
+
+
+# ---- a backward belongs to the last training forward of its module ---------------------------
+
+def other_layout(x):
+    """The same values in a tensor that is not contiguous."""
+    return x.t().contiguous().t()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("what", ["fine_tuning", "not contiguous", "no_grad"])
+def test_a_second_forward_before_the_backward_is_refused(cuda_device, kind, what):
+    m = build(kind, cuda_device).train()
+    x1, x2 = rows(48, cuda_device, 1), rows(48, cuda_device, 2)
+    for _ in range(2):          # every form of the call prepared and bound
+        for ft in (False, True):
+            forward(m, x1.clone().requires_grad_(True), ft)[0].sum().backward()
+    if what == "not contiguous":
+        x1, x2 = other_layout(x1), other_layout(x2)
+    first = forward(m, x1.requires_grad_(True))[0]
+    if what == "no_grad":
+        with torch.no_grad():
+            forward(m, x2)
+    else:
+        forward(m, x2, what == "fine_tuning")
+    with pytest.raises(RuntimeError, match="another training forward"):
+        first.sum().backward()
+    # and the module is usable afterwards
+    same(train_step(m, x2), train_step(fresh_copy(m, kind, cuda_device), x2))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_forwards_of_two_sizes_before_their_backwards(cuda_device, kind):
+    """Another number of rows has workspaces of its own: both backwards are right, in either order."""
+    m = build(kind, cuda_device).train().requires_grad_(False)
+    xs = [rows(n, cuda_device, n).requires_grad_(True) for n in (48, 32)]
+    want = []
+    for x in xs:
+        torch.manual_seed(3)
+        want += torch.autograd.grad(forward(m, x)[0].float().square().sum(), x)
+    for order in ((0, 1), (1, 0)):
+        outs = []
+        for x in xs:
+            torch.manual_seed(3)
+            outs.append(forward(m, x)[0])
+        for i in order:
+            (g,) = torch.autograd.grad(outs[i].float().square().sum(), xs[i])
+            assert torch.equal(g, want[i])
