@@ -11,7 +11,7 @@
 //
 // Lifetime: a bound call owns every buffer whose address it has (plan, workspaces, merged weights): the Python side may
 // replace its own, and the parameters may leave and come back (weights exchanged for an evaluation) with the binding
-// still in place. The parameters themselves it does not own, so that moving a module away frees them; an autograd node
+// still in place. Of merged weights there is one record of what they hold, kept with them. The parameters themselves it does not own, so that moving a module away frees them; an autograd node
 // does, from its forward to its backward, because the plan that it will use has their addresses.
 #include <Python.h>
 #include <ATen/ATen.h>
@@ -23,8 +23,12 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <algorithm>
 #include <memory>
+#include <mutex>
 #include <string>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 #include "../../../include/moe_b200.h"
@@ -126,67 +130,201 @@ class WatchList {
   std::vector<int> params_;
 };
 
-// A Linear with its LoRA pair, merged again whenever one of the six tensors was written since
-// (torch's version counters): indices of weight, bias, a.weight, a.bias, b.weight, b.bias.
-struct LoraJob {
-  int p[6];
-  int64_t version[6];
-  double scale;
-  int out_f, in_f, rank;
-  void* out_w;
-  void* out_b;
+bool tensor_list(PyObject* seq, std::vector<Tensor>* out) {
+  out->clear();
+  const Py_ssize_t n = PyList_Size(seq);
+  if (n < 0) return false;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* t = PyList_GET_ITEM(seq, i);
+    if (!THPVariable_Check(t)) {
+      PyErr_SetString(PyExc_TypeError, "a list of tensors is needed");
+      return false;
+    }
+    out->push_back(THPVariable_Unpack(t));
+  }
+  return true;
+}
+
+bool float_list(PyObject* seq, std::vector<double>* out) {
+  out->clear();
+  const Py_ssize_t n = PyList_Size(seq);
+  if (n < 0) return false;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    out->push_back(PyFloat_AsDouble(PyList_GET_ITEM(seq, i)));
+    if (PyErr_Occurred()) return false;
+  }
+  return true;
+}
+
+// A parameter as a call finds it: its address, the storage that keeps it alive, and torch's version counter.
+struct Held {
+  c10::Storage storage;
+  const void* data;
+  c10::VariableVersion version;
+  explicit Held(const Tensor& t)
+      : storage(t.storage()), data(t.const_data_ptr()), version(t.unsafeGetTensorImpl()->version_counter()) {}
 };
 
-class LoraJobs {
+// Merged copies W' = W + s B A, b' = b + s (B a + b_lora) of the two Linears of a list of experts, and the one record of
+// what they hold: addresses, versions and scale of the last merge. Every call that reads them, bound or not, forward
+// or backward, compares its own parameters with that record first, so that adapters that were exchanged in between, by
+// whichever call, are merged again. Parameters are counted as in moe.py: twelve an expert.
+class Merged {
  public:
-  bool bind(PyObject* seq, const WatchList& w) {
-    jobs_.clear();
-    if (seq == Py_None) return true;
+  bool fill(PyObject* seq) {
     const Py_ssize_t n = PyList_Size(seq);
     if (n < 0) return false;
     for (Py_ssize_t i = 0; i < n; ++i) {
-      LoraJob j;
-      unsigned long long ow, ob;
-      if (!PyArg_ParseTuple(PyList_GET_ITEM(seq, i), "iiiiiidiiiKK", &j.p[0], &j.p[1], &j.p[2], &j.p[3], &j.p[4],
-                            &j.p[5], &j.scale, &j.out_f, &j.in_f, &j.rank, &ow, &ob))
+      Job j;
+      PyObject *w, *b;
+      if (!PyArg_ParseTuple(PyList_GET_ITEM(seq, i), "iiiOO", &j.out_f, &j.in_f, &j.rank, &w, &b)) return false;
+      if (!THPVariable_Check(w) || !THPVariable_Check(b)) {
+        PyErr_SetString(PyExc_TypeError, "merged weights must be tensors");
         return false;
-      j.out_w = reinterpret_cast<void*>(ow);
-      j.out_b = reinterpret_cast<void*>(ob);
-      for (int q = 0; q < 6; ++q) {
-        if (j.p[q] < 0 || j.p[q] >= w.num_params()) {
-          PyErr_SetString(PyExc_IndexError, "parameter index");
-          return false;
-        }
-        j.version[q] = (int64_t)w.param(j.p[q])._version();
       }
-      jobs_.push_back(j);
+      j.w = THPVariable_Unpack(w);
+      j.b = THPVariable_Unpack(b);
+      jobs_.push_back(std::move(j));
     }
     return true;
   }
-  int refresh(const WatchList& w, int dtype, void* stream) {
-    for (LoraJob& j : jobs_) {
-      bool stale = false;
+  size_t num_params() const { return jobs_.size() * 6; }
+  // param(i) -> (address, version) of the i-th parameter; scale of every expert
+  template <typename Param>
+  int refresh(Param param, const std::vector<double>& scales, int dtype, void* stream) {
+    const std::lock_guard<std::mutex> lock(mutex_);      // a backward runs on another thread
+    for (size_t i = 0; i < jobs_.size(); ++i) {
+      Job& j = jobs_[i];
+      const size_t first = i / 2 * 12, l = i % 2;
+      // weight, bias, a.weight, a.bias, b.weight, b.bias
+      const size_t at[6] = {first + 2 * l, first + 2 * l + 1, first + 4 + 4 * l, first + 5 + 4 * l, first + 6 + 4 * l,
+                            first + 7 + 4 * l};
+      const void* data[6];
+      int64_t version[6];
+      bool same = j.valid && j.scale == scales[i / 2];
       for (int q = 0; q < 6; ++q) {
-        const int64_t v = (int64_t)w.param(j.p[q])._version();
-        stale |= v != j.version[q];
-        j.version[q] = v;
+        std::tie(data[q], version[q]) = param(at[q]);
+        same = same && data[q] == j.data[q] && version[q] == j.version[q];
       }
-      if (!stale) continue;
-      const int rc = moe_b200_lora_merge(
-          w.param(j.p[0]).const_data_ptr(), w.param(j.p[1]).const_data_ptr(), w.param(j.p[2]).const_data_ptr(),
-          w.param(j.p[3]).const_data_ptr(), w.param(j.p[4]).const_data_ptr(), w.param(j.p[5]).const_data_ptr(),
-          (float)j.scale, j.out_f, j.in_f, j.rank, dtype, j.out_w, j.out_b, stream);
-      if (rc != 0) {
-        j.version[0] = -1;
-        return rc;
-      }
+      if (same) continue;
+      j.valid = false;
+      const int rc = moe_b200_lora_merge(data[0], data[1], data[2], data[3], data[4], data[5], (float)scales[i / 2],
+                                         j.out_f, j.in_f, j.rank, dtype, j.w.data_ptr(), j.b.data_ptr(), stream);
+      if (rc != 0) return rc;
+      std::copy(data, data + 6, j.data);
+      std::copy(version, version + 6, j.version);
+      j.scale = scales[i / 2];
+      j.valid = true;
     }
     return 0;
   }
 
  private:
-  std::vector<LoraJob> jobs_;
+  struct Job {
+    Tensor w, b;
+    int out_f = 0, in_f = 0, rank = 0;
+    bool valid = false;
+    const void* data[6];
+    int64_t version[6];
+    double scale = 0.0;
+  };
+  std::vector<Job> jobs_;
+  std::mutex mutex_;
 };
+
+// What a bound call has of it; nothing without LoRA branches.
+struct MergedUse {
+  std::shared_ptr<Merged> merged;
+  std::vector<double> scales;
+  size_t first = 0;       // place of the first expert's parameters among the call's
+
+  int refresh(const WatchList& w, int dtype, void* stream) const {
+    if (merged == nullptr) return 0;
+    return merged->refresh(
+        [&](size_t i) {
+          const Tensor& t = w.param((int)(first + i));
+          return std::make_pair(t.const_data_ptr(), (int64_t)t._version());
+        },
+        scales, dtype, stream);
+  }
+  int refresh(const std::vector<Held>& h, int dtype, void* stream) const {
+    if (merged == nullptr) return 0;
+    return merged->refresh(
+        [&](size_t i) { return std::make_pair(h[first + i].data, (int64_t)h[first + i].version.current_version()); }, scales,
+        dtype, stream);
+  }
+};
+
+struct MergedObject {
+  PyObject_HEAD
+  std::shared_ptr<Merged>* merged;
+};
+
+PyTypeObject* g_merged_type = nullptr;
+
+// Merged([(out, in, rank, W', b')]): gate_and_up and down of every expert
+PyObject* merged_new(PyTypeObject* type, PyObject* args, PyObject*) {
+  HANDLE_TH_ERRORS
+  PyObject* jobs;
+  if (!PyArg_ParseTuple(args, "O!", &PyList_Type, &jobs)) return nullptr;
+  auto m = std::make_shared<Merged>();
+  if (!m->fill(jobs)) return nullptr;
+  MergedObject* self = reinterpret_cast<MergedObject*>(type->tp_alloc(type, 0));
+  if (self == nullptr) return nullptr;
+  self->merged = new std::shared_ptr<Merged>(std::move(m));
+  return reinterpret_cast<PyObject*>(self);
+  END_HANDLE_TH_ERRORS
+}
+
+void merged_dealloc(PyObject* o) {
+  PyTypeObject* type = Py_TYPE(o);
+  delete reinterpret_cast<MergedObject*>(o)->merged;
+  type->tp_free(o);
+  Py_DECREF(type);
+}
+
+// refresh(parameters, scales, dtype, device index)
+PyObject* merged_refresh(PyObject* o, PyObject* args) {
+  HANDLE_TH_ERRORS
+  PyObject *params, *scales;
+  int dtype, device;
+  if (!PyArg_ParseTuple(args, "O!O!ii", &PyList_Type, &params, &PyList_Type, &scales, &dtype, &device)) return nullptr;
+  Merged& m = **reinterpret_cast<MergedObject*>(o)->merged;
+  std::vector<Tensor> t;
+  std::vector<double> s;
+  if (!tensor_list(params, &t) || !float_list(scales, &s)) return nullptr;
+  if (t.size() != m.num_params() || s.size() * 12 != t.size()) {
+    PyErr_SetString(PyExc_ValueError, "twelve parameters and a scale for every expert");
+    return nullptr;
+  }
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+  const int rc = m.refresh(
+      [&](size_t i) { return std::make_pair(t[i].const_data_ptr(), (int64_t)t[i]._version()); }, s, dtype, stream);
+  if (rc != 0) return fail(rc, "lora_merge");
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// (merged or None, scales) of a bind(); `params`: how many parameters the call has, the first expert's at `first`
+bool read_merged(PyObject* merged, PyObject* scales, size_t first, size_t params, MergedUse* out) {
+  *out = MergedUse();
+  if (merged == Py_None) return true;
+  if (!PyObject_TypeCheck(merged, g_merged_type)) {
+    PyErr_SetString(PyExc_TypeError, "merged must be a Merged");
+    return false;
+  }
+  if (!float_list(scales, &out->scales)) return false;
+  out->merged = *reinterpret_cast<MergedObject*>(merged)->merged;
+  out->first = first;
+  // params is 0 for a module tree that cannot be watched: its calls never refresh from the watched parameters
+  if (out->scales.size() * 12 != out->merged->num_params() ||
+      (params != 0 && params != first + out->merged->num_params())) {
+    PyErr_SetString(PyExc_ValueError, "twelve parameters and a scale for every expert");
+    return false;
+  }
+  return true;
+}
 
 // ---- training -----------------------------------------------------------------------------------
 // The forward of a module under .train() as one autograd node, without Python on either way: the node keeps
@@ -198,21 +336,6 @@ using torch::autograd::edge_list;
 using torch::autograd::Node;
 using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
-
-bool tensor_list(PyObject* seq, std::vector<Tensor>* out) {
-  out->clear();
-  const Py_ssize_t n = PyList_Size(seq);
-  if (n < 0) return false;
-  for (Py_ssize_t i = 0; i < n; ++i) {
-    PyObject* t = PyList_GET_ITEM(seq, i);
-    if (!THPVariable_Check(t)) {
-      PyErr_SetString(PyExc_TypeError, "buffers must be tensors");
-      return false;
-    }
-    out->push_back(THPVariable_Unpack(t));
-  }
-  return true;
-}
 
 // Number of forwards on a training workspace, of all bindings that share it: a backward must belong to the last.
 struct Generation {
@@ -248,7 +371,8 @@ bool read_generation(PyObject* o, std::shared_ptr<int64_t>* out) {
 // What a prepared training call works on; shared by the module and the nodes of its calls.
 struct TrainCall {
   Tensor ws, tws, offsets, status, lora_tab;    // buffers kept alive
-  std::vector<Tensor> owned;                    // plan and merged weights likewise
+  std::vector<Tensor> owned;                    // the plan likewise
+  MergedUse lora;
   const void* plan = nullptr;
   void *ws_base = nullptr, *tws_base = nullptr;
   size_t ws_bytes = 0, tws_bytes = 0;
@@ -339,7 +463,7 @@ struct BlockBackward : public Node {
   std::shared_ptr<TrainCall> call;
   SavedVariable x;
   Tensor gate_w;
-  std::vector<c10::Storage> weights;    // of the parameters whose addresses the plan has
+  std::vector<Held> weights;    // the parameters whose addresses the plan has
   int64_t gen = 0;
   uint64_t seed = 0;
   double p = 0.0;
@@ -373,6 +497,7 @@ struct BlockBackward : public Node {
     ExpertGrads eg;
     const moe::LoraGrads lg = eg.prepare(c, opt, &g, wanted);
     if (c.N > 0) {
+      check_rc(c.lora.refresh(weights, MOE_B200_BF16, stream), "lora_merge");
       check_rc(moe::backward_into(xv.const_data_ptr(), gate_w.const_data_ptr(), c.plan, go.const_data_ptr(), 0.f,
                                   aux.defined() ? aux.const_data_ptr<float>() : nullptr, c.N, c.d, c.f, c.E, c.k,
                                   MOE_B200_BF16, (float)p, seed, c.ws_base, c.ws_bytes, c.tws_base, c.tws_bytes, g,
@@ -397,7 +522,7 @@ struct FfnBackward : public Node {
   std::shared_ptr<TrainCall> call;
   SavedVariable x;
   Tensor h;
-  std::vector<c10::Storage> weights;
+  std::vector<Held> weights;
   int64_t gen = 0;
   uint64_t seed = 0;
   double p = 0.0;
@@ -426,6 +551,7 @@ struct FfnBackward : public Node {
     ExpertGrads eg;
     const moe::LoraGrads lg = eg.prepare(c, opt, &g, wanted);
     if (c.N > 0) {
+      check_rc(c.lora.refresh(weights, MOE_B200_BF16, stream), "lora_merge");
       check_rc(moe::experts_backward_into(xv.const_data_ptr(), h.const_data_ptr(), c.offsets.const_data_ptr<int32_t>(),
                                           c.plan, go.const_data_ptr(), c.N, c.d, c.f, 1, (float)p, seed, c.tws_base,
                                           c.tws_bytes, g, lg.tab != nullptr ? &lg : nullptr,
@@ -442,12 +568,12 @@ struct FfnBackward : public Node {
   }
 };
 
-// Edges of a call's inputs, and the storages of those that are parameters.
+// Edges of a call's inputs, and those of them that are parameters.
 class Edges {
  public:
   void add_param(const Tensor& t) {
     add(t);
-    weights_.push_back(t.storage());
+    weights_.emplace_back(t);
   }
   void add(const Tensor& t) {
     any_ |= t.requires_grad();
@@ -456,11 +582,11 @@ class Edges {
   void add_empty() { list_.emplace_back(); }
   bool wanted() const { return any_ && at::GradMode::is_enabled(); }
   edge_list take() { return std::move(list_); }
-  std::vector<c10::Storage> take_weights() { return std::move(weights_); }
+  std::vector<Held> take_weights() { return std::move(weights_); }
 
  private:
   edge_list list_;
-  std::vector<c10::Storage> weights_;
+  std::vector<Held> weights_;
   bool any_ = false;
 };
 
@@ -471,9 +597,9 @@ at::ScalarType scalar_of(int dtype) { return dtype == MOE_B200_BF16 ? at::kBFloa
 struct Block {
   PyObject_HEAD
   WatchList* watch;       // [0], [1]: the router's weight and bias, then the experts' tensors
-  LoraJobs* lora;
+  MergedUse* lora;
   Tensor* workspace;
-  std::vector<Tensor>* owned;     // plan and merged weights
+  std::vector<Tensor>* owned;     // the plan
   std::shared_ptr<TrainCall>* train;
   const void* plan;
   void* ws_base;
@@ -516,7 +642,7 @@ PyObject* block_new(PyTypeObject* type, PyObject*, PyObject*) {
   Block* self = reinterpret_cast<Block*>(type->tp_alloc(type, 0));
   if (self == nullptr) return nullptr;
   self->watch = new WatchList();
-  self->lora = new LoraJobs();
+  self->lora = new MergedUse();
   self->workspace = new Tensor();
   self->owned = new std::vector<Tensor>();
   self->train = new std::shared_ptr<TrainCall>();
@@ -535,22 +661,23 @@ void block_dealloc(PyObject* o) {
   Py_DECREF(type);
 }
 
-// bind(watch, lora or None, plan, owned buffers, workspace tensor, base, bytes, N, d, f, E, k, dtype, device index)
+// bind(watch, merged or None, scales, plan, owned buffers, workspace tensor, base, bytes, N, d, f, E, k, dtype, device index)
 PyObject* block_bind(PyObject* o, PyObject* args) {
   HANDLE_TH_ERRORS
   Block* self = reinterpret_cast<Block*>(o);
-  PyObject *watch, *lora, *owned, *ws;
+  PyObject *watch, *merged, *scales, *owned, *ws;
   unsigned long long plan, base, bytes;
   long long N;
   int d, f, E, k, dtype, device;
-  if (!PyArg_ParseTuple(args, "O!OKO!OKKLiiiiii", &PyList_Type, &watch, &lora, &plan, &PyList_Type, &owned, &ws, &base, &bytes, &N, &d, &f,
+  if (!PyArg_ParseTuple(args, "O!OOKO!OKKLiiiiii", &PyList_Type, &watch, &merged, &scales, &plan, &PyList_Type, &owned, &ws, &base, &bytes, &N, &d, &f,
                         &E, &k, &dtype, &device))
     return nullptr;
   if (!THPVariable_Check(ws)) {
     PyErr_SetString(PyExc_TypeError, "workspace must be a tensor");
     return nullptr;
   }
-  if (!tensor_list(owned, self->owned) || !self->watch->bind(watch) || !self->lora->bind(lora, *self->watch)) {
+  if (!tensor_list(owned, self->owned) || !self->watch->bind(watch) ||
+      !read_merged(merged, scales, 2, (size_t)self->watch->num_params(), self->lora)) {
     self->watch->clear();
     return nullptr;
   }
@@ -574,6 +701,7 @@ PyObject* block_unbind(PyObject* o, PyObject*) {
   self->watch->clear();
   *self->workspace = Tensor();
   self->owned->clear();
+  *self->lora = MergedUse();
   self->train->reset();
   Py_RETURN_NONE;
 }
@@ -591,6 +719,7 @@ PyObject* block_bind_train(PyObject* o, PyObject* args) {
   if (!read_generation(gen, &c->gen)) return nullptr;
   c->ws = *self->workspace;
   c->owned = *self->owned;
+  c->lora = *self->lora;
   c->tws = THPVariable_Unpack(tws);
   if (tab != Py_None) c->lora_tab = THPVariable_Unpack(tab);
   c->plan = self->plan;
@@ -771,8 +900,8 @@ PyType_Spec block_spec = {"gemmallm_b200._host.Block", sizeof(Block), 0, Py_TPFL
 struct Ffn {
   PyObject_HEAD
   WatchList* watch;
-  LoraJobs* lora;
-  std::vector<Tensor>* owned;   // plan and merged weights
+  MergedUse* lora;
+  std::vector<Tensor>* owned;   // the plan
   Tensor* offsets;        // int32 [0, M]
   Tensor* status;         // int32 [16], written only when a wait inside a kernel ran out
   std::shared_ptr<TrainCall>* train;
@@ -785,7 +914,7 @@ PyObject* ffn_new(PyTypeObject* type, PyObject*, PyObject*) {
   Ffn* self = reinterpret_cast<Ffn*>(type->tp_alloc(type, 0));
   if (self == nullptr) return nullptr;
   self->watch = new WatchList();
-  self->lora = new LoraJobs();
+  self->lora = new MergedUse();
   self->owned = new std::vector<Tensor>();
   self->offsets = new Tensor();
   self->status = new Tensor();
@@ -806,22 +935,23 @@ void ffn_dealloc(PyObject* o) {
   Py_DECREF(type);
 }
 
-// bind(watch, lora or None, plan, owned buffers, offsets, status, M, d, f, dtype, device index)
+// bind(watch, merged or None, scales, plan, owned buffers, offsets, status, M, d, f, dtype, device index)
 PyObject* ffn_bind(PyObject* o, PyObject* args) {
   HANDLE_TH_ERRORS
   Ffn* self = reinterpret_cast<Ffn*>(o);
-  PyObject *watch, *lora, *owned, *offsets, *status;
+  PyObject *watch, *merged, *scales, *owned, *offsets, *status;
   unsigned long long plan;
   long long M;
   int d, f, dtype, device;
-  if (!PyArg_ParseTuple(args, "O!OKO!OOLiiii", &PyList_Type, &watch, &lora, &plan, &PyList_Type, &owned, &offsets, &status, &M, &d, &f,
+  if (!PyArg_ParseTuple(args, "O!OOKO!OOLiiii", &PyList_Type, &watch, &merged, &scales, &plan, &PyList_Type, &owned, &offsets, &status, &M, &d, &f,
                         &dtype, &device))
     return nullptr;
   if (!THPVariable_Check(offsets) || !THPVariable_Check(status)) {
     PyErr_SetString(PyExc_TypeError, "offsets and status must be tensors");
     return nullptr;
   }
-  if (!tensor_list(owned, self->owned) || !self->watch->bind(watch) || !self->lora->bind(lora, *self->watch)) {
+  if (!tensor_list(owned, self->owned) || !self->watch->bind(watch) ||
+      !read_merged(merged, scales, 0, (size_t)self->watch->num_params(), self->lora)) {
     self->watch->clear();
     return nullptr;
   }
@@ -841,6 +971,7 @@ PyObject* ffn_unbind(PyObject* o, PyObject*) {
   Ffn* self = reinterpret_cast<Ffn*>(o);
   self->watch->clear();
   self->owned->clear();
+  *self->lora = MergedUse();
   self->train->reset();
   Py_RETURN_NONE;
 }
@@ -858,6 +989,7 @@ PyObject* ffn_bind_train(PyObject* o, PyObject* args) {
   if (!read_generation(gen, &c->gen)) return nullptr;
   c->tws = THPVariable_Unpack(tws);
   c->owned = *self->owned;
+  c->lora = *self->lora;
   c->offsets = *self->offsets;
   c->status = *self->status;
   if (tab != Py_None) c->lora_tab = THPVariable_Unpack(tab);
@@ -979,6 +1111,13 @@ PyMethodDef ffn_methods[] = {
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(ffn_forward)), METH_FASTCALL, nullptr},
     {"__reduce__", fresh_reduce, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr}};
+PyMethodDef merged_methods[] = {{"refresh", merged_refresh, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyType_Slot merged_slots[] = {{Py_tp_new, reinterpret_cast<void*>(merged_new)},
+                              {Py_tp_dealloc, reinterpret_cast<void*>(merged_dealloc)},
+                              {Py_tp_methods, merged_methods},
+                              {0, nullptr}};
+PyType_Spec merged_spec = {"gemmallm_b200._host.Merged", sizeof(MergedObject), 0, Py_TPFLAGS_DEFAULT, merged_slots};
+
 PyMethodDef generation_methods[] = {{"__reduce__", fresh_reduce, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyType_Slot generation_slots[] = {{Py_tp_new, reinterpret_cast<void*>(generation_new)},
                                   {Py_tp_dealloc, reinterpret_cast<void*>(generation_dealloc)},
@@ -1016,7 +1155,8 @@ PyMODINIT_FUNC PyInit__host(void) {
   s_parameters = PyUnicode_InternFromString("_parameters");
   s_eps = PyUnicode_InternFromString("eps");
   if (!add_type(m, "Block", &block_spec) || !add_type(m, "Ffn", &ffn_spec) ||
-      !add_type(m, "Generation", &generation_spec, &g_generation_type)) {
+      !add_type(m, "Generation", &generation_spec, &g_generation_type) ||
+      !add_type(m, "Merged", &merged_spec, &g_merged_type)) {
     Py_DECREF(m);
     return nullptr;
   }

@@ -45,19 +45,6 @@ def _expert_watch(ex, fine_tuning: bool) -> list:
     return watch
 
 
-def _lora_jobs(ex, merged, first: int) -> list:
-    """The two merges of an expert for the native path: indices of weight, bias, a.weight, a.bias,
-    b.weight, b.bias among the watched parameters (the expert's twelve start at ``first``), then
-    scale, shape and the merged buffers."""
-    jobs = []
-    for lin, a, b, out, i in ((ex.gate_and_up, ex.lora_gate_and_up_a, ex.lora_gate_and_up_b, merged.gate_and_up, 0),
-                              (ex.down, ex.lora_down_a, ex.lora_down_b, merged.down, 1)):
-        w, la, lb = first + 2 * i, first + 4 + 4 * i, first + 6 + 4 * i
-        jobs.append((w, w + 1, la, la + 1, lb, lb + 1, float(ex.lora_scale), lin.out_features, lin.in_features,
-                     a.out_features, out.weight.data_ptr(), out.bias.data_ptr()))
-    return jobs
-
-
 class _MergedExpert:
     """An expert's two Linears with the LoRA branch folded in (moe_b200_lora_merge):
     W' = W + s * B A and b' = b + s * (B a + b_lora), which makes
@@ -74,25 +61,21 @@ class _MergedExpert:
         self.gate_and_up = self._Lin(torch.empty_like(ex.gate_and_up.weight), torch.empty_like(ex.gate_and_up.bias))
         self.down = self._Lin(torch.empty_like(ex.down.weight), torch.empty_like(ex.down.bias))
 
-    def refresh(self, ex, dtype: int, stream: int) -> None:
-        for lin, a, b, out in ((ex.gate_and_up, ex.lora_gate_and_up_a, ex.lora_gate_and_up_b, self.gate_and_up),
-                               (ex.down, ex.lora_down_a, ex.lora_down_b, self.down)):
-            check(lib.moe_b200_lora_merge(
-                lin.weight.data_ptr(), lin.bias.data_ptr(), a.weight.data_ptr(), a.bias.data_ptr(),
-                b.weight.data_ptr(), b.bias.data_ptr(), float(ex.lora_scale), lin.out_features,
-                lin.in_features, a.out_features, dtype, out.weight.data_ptr(), out.bias.data_ptr(),
-                stream), "lora_merge")
-
 
 class _MergedLora:
     """Merged copies of a list of experts, refreshed only when one of their twelve tensors
     was replaced or written since the last call (data pointer and torch's version counter),
     so that a fine_tuning=True forward on unchanged parameters launches no merge kernel and
-    rebuilds no plan."""
+    rebuilds no plan. What the copies hold is recorded in ``native``, with the copies, for every
+    call that reads them (csrc/host/host.cpp). A copy of this object starts empty."""
 
     def __init__(self):
-        self.key = None
+        self.shapes = None
         self.merged = None
+        self.native = None
+
+    def __reduce__(self):
+        return (_MergedLora, ())
 
     def get(self, experts, dtype: int, device: torch.device):
         params = [p for ex in experts for n in _LORA_NAMES
@@ -101,18 +84,17 @@ class _MergedLora:
             if p.device != device or _dtype_code(p) != dtype or not p.is_contiguous():
                 raise ValueError("expert and LoRA parameters must be contiguous and share the "
                                  "input's device and dtype")
-        shape_key = (dtype, str(device), tuple(tuple(p.shape) for p in params))
-        key = (shape_key, tuple((p.data_ptr(), p._version) for p in params))
-        if self.key is None or self.key[0] != shape_key:
+        shapes = (dtype, str(device), tuple(tuple(p.shape) for p in params))
+        if shapes != self.shapes:
             self.merged = [_MergedExpert(ex) for ex in experts]
-        if key != self.key:
-            for ex, mg in zip(experts, self.merged):
-                mg.refresh(ex, dtype, _stream(device))
-            self.key = key
+            self.native = _host.Merged([
+                (lin.out_features, lin.in_features, a.out_features, out.weight, out.bias)
+                for ex, mg in zip(experts, self.merged)
+                for lin, a, out in ((ex.gate_and_up, ex.lora_gate_and_up_a, mg.gate_and_up),
+                                    (ex.down, ex.lora_down_a, mg.down))])
+            self.shapes = shapes
+        self.native.refresh(params, [float(ex.lora_scale) for ex in experts], dtype, device.index)
         return self.merged
-
-    def buffers(self) -> list:
-        return [t for mg in self.merged for lin in (mg.gate_and_up, mg.down) for t in (lin.weight, lin.bias)]
 
 
 def _lora_table(experts, dev) -> torch.Tensor:
@@ -205,9 +187,12 @@ class FeedForward(nn.Module):
             self._offsets = ((M, str(dev)), torch.tensor([0, M], dtype=torch.int32, device=dev))
         return x, M, dev, self._offsets[1]
 
-    def _owned(self, fine_tuning: bool) -> list:
-        """Buffers whose addresses a bound call has, besides workspaces: the plan and the merged weights."""
-        return [self._plan_ft.buf, *self._lora.buffers()] if fine_tuning else [self._plan.buf]
+    def _plan_of(self, fine_tuning: bool) -> _Plan:
+        return self._plan_ft if fine_tuning else self._plan
+
+    def _bound(self, fine_tuning: bool):
+        """Merged weights and scales of a call that is bound."""
+        return (self._lora.native, [float(self.lora_scale)]) if fine_tuning else (None, [])
 
     # -- training mode (bf16): dropout on h and a backward pass -----------------
     def _train_ws(self, M: int, device: torch.device):
@@ -243,10 +228,9 @@ class FeedForward(nn.Module):
             status = torch.zeros(16, dtype=torch.int32, device=dev)
             watch = _expert_watch(self, fine_tuning)
             usual = all(name in table for table, name in watch)
-            jobs = _lora_jobs(self, self._lora.merged[0], 0) if fine_tuning and usual else None
             native.unbind()
-            native.bind(watch if usual else [], jobs, plan, self._owned(fine_tuning), offsets, status, M, d, f, _cabi.BF16,
-                        dev.index)
+            native.bind(watch if usual else [], *self._bound(fine_tuning), plan, [self._plan_of(fine_tuning).buf],
+                        offsets, status, M, d, f, _cabi.BF16, dev.index)
             table = _lora_table([self], dev) if fine_tuning else None
             native.bind_train(buf, tbase, tbytes, table, self.lora_down_a.out_features if fine_tuning else 0,
                               float(self.lora_scale), self._generation)
@@ -294,8 +278,8 @@ class FeedForward(nn.Module):
         native.unbind()
         watch = _expert_watch(self, fine_tuning)
         if x.shape[-1] == d and all(name in table for table, name in watch):
-            jobs = _lora_jobs(self, self._lora.merged[0], 0) if fine_tuning else None
-            native.bind(watch, jobs, plan, self._owned(fine_tuning), offsets, status, M, d, f, dtype, dev.index)
+            native.bind(watch, *self._bound(fine_tuning), plan, [self._plan_of(fine_tuning).buf], offsets, status, M, d, f,
+                        dtype, dev.index)
         return y.reshape(shape)
 
 
@@ -477,13 +461,10 @@ class MOE(nn.Module):
         d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
         native.unbind()
         watch = self._watch(fine_tuning)
-        jobs = None
-        if fine_tuning and watch:
-            jobs = [job for e, (ex, mg) in enumerate(zip(self.experts, self._lora.merged))
-                    for job in _lora_jobs(ex, mg, 2 + 12 * e)]
+        merged, scales, owner = ((self._lora.native, [float(ex.lora_scale) for ex in self.experts], self._plan_ft)
+                                 if fine_tuning else (None, [], self._plan))
         buf, base, nbytes, _ = self._ws
-        owned = [self._plan_ft.buf, *self._lora.buffers()] if fine_tuning else [self._plan.buf]
-        native.bind(watch, jobs, plan, owned, buf, base, nbytes, N, d, f, E, k, dtype, dev.index)
+        native.bind(watch, merged, scales, plan, [owner.buf], buf, base, nbytes, N, d, f, E, k, dtype, dev.index)
 
     # -- training mode -------------------------------------------------------
     def _train_workspace(self, N: int, device: torch.device):

@@ -68,10 +68,10 @@ def test_a_bound_call_owns_its_buffers(kind, train):
     refs = [weakref.ref(t) for t in buffers]
     if kind == "moe":
         native = _host.Block()
-        native.bind(watch, None, 0, buffers[:2], buffers[2], 0, 0, 1, D, F, E, 2, 1, 0)
+        native.bind(watch, None, [], 0, buffers[:2], buffers[2], 0, 0, 1, D, F, E, 2, 1, 0)
     else:
         native = _host.Ffn()
-        native.bind(watch, None, 0, buffers[:2], buffers[2], buffers[2], 1, D, F, 1, 0)
+        native.bind(watch, None, [], 0, buffers[:2], buffers[2], buffers[2], 1, D, F, 1, 0)
     if train:
         native.bind_train(buffers[3], 0, 0, None, 0, 1.0, _host.Generation())
     else:
@@ -89,7 +89,7 @@ def test_nothing_is_bound_after_an_error():
     native = _host.Ffn()
     status = torch.zeros(16, dtype=torch.int32)
     with pytest.raises(KeyError):
-        native.bind([(table, "weight"), (table, "bias")], None, 0, [status], status, status, 1, D, F, 1, 0)
+        native.bind([(table, "weight"), (table, "bias")], None, [], 0, [status], status, status, 1, D, F, 1, 0)
     assert native.forward(torch.zeros(1, D, dtype=DT)) is None
 
 
@@ -99,7 +99,7 @@ def exchange(params, others):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("fine_tuning", [False])
+@pytest.mark.parametrize("fine_tuning", [False, True])
 @pytest.mark.parametrize("kind", KINDS)
 def test_weights_exchanged_for_an_evaluation_and_back(cuda_device, kind, fine_tuning):
     """Averaged weights by .data for an evaluation: the training call bound before it is right afterwards."""
@@ -210,3 +210,91 @@ def test_forwards_of_two_sizes_before_their_backwards(cuda_device, kind):
         for i in order:
             (g,) = torch.autograd.grad(outs[i].float().square().sum(), xs[i])
             assert torch.equal(g, want[i])
+
+
+# ---- merged weights: one record of what they hold ----------------------------------------------
+
+def adapters(m):
+    return [p for n, p in m.named_parameters() if "lora" in n]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [48, 20])
+@pytest.mark.parametrize("kind", KINDS)
+def test_adapters_exchanged_for_an_evaluation_and_back(cuda_device, kind, size):
+    """.data moves no version counter: what the merged weights hold is told by addresses and versions together."""
+    m, x, other = build(kind, cuda_device), rows(48, cuda_device), rows(size, cuda_device, 2)
+    adapters_b = [torch.empty_like(p).normal_(0, 0.3) for p in adapters(m)]
+    for _ in range(2):
+        train_step(m, x, True)
+    for _ in range(2):
+        with torch.no_grad():
+            exchange(adapters(m), adapters_b)
+            got = forward(m.eval(), other, True)
+            same(got, forward(fresh_copy(m, kind, cuda_device).eval(), other, True))
+            exchange(adapters(m), adapters_b)
+        want = train_step(fresh_copy(m, kind, cuda_device), x, True)
+        same(train_step(m, x, True), want)
+
+
+@pytest.mark.gpu
+def test_adapters_of_another_rank_for_an_evaluation(cuda_device):
+    """Adapters of rank 8 and back: the merged buffers of the bound training call belong to it."""
+    m, x = build("ffn", cuda_device), rows(48, cuda_device)
+    small = build("ffn", cuda_device, seed=3, rank=8)
+    names = ("lora_gate_and_up_a", "lora_gate_and_up_b", "lora_down_a", "lora_down_b")
+
+    def swap():
+        for n in names:
+            a, b = getattr(m, n), getattr(small, n)
+            setattr(m, n, b), setattr(small, n, a)
+    for _ in range(2):
+        train_step(m, x, True)
+    swap()
+    with torch.no_grad():
+        got = forward(m.eval(), x, True)
+    fresh = fresh_copy(m, "ffn", cuda_device, rank=8).eval()
+    fresh.lora_scale = m.lora_scale
+    with torch.no_grad():
+        same(got, forward(fresh, x, True))
+    swap()
+    gc.collect()
+    want = train_step(fresh_copy(m, "ffn", cuda_device), x, True)
+    same(train_step(m, x, True), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_adapters_exchanged_between_forward_and_backward(cuda_device, kind):
+    """An evaluation with other adapters in between merges them into the same buffers: the backward merges its own again.
+    (Another number of rows: the block's workspace holds the training forward's tensors.)"""
+    m, x, other = build(kind, cuda_device), rows(48, cuda_device), rows(20, cuda_device, 2)
+    want = train_step(fresh_copy(m, kind, cuda_device), x, True)
+    adapters_b = [torch.empty_like(p).normal_(0, 0.3) for p in adapters(m)]
+    for _ in range(2):
+        train_step(m, x, True)
+    m.train()
+    for p in m.parameters():
+        p.grad = None
+    xd = x.clone().requires_grad_(True)
+    torch.manual_seed(5)
+    out = forward(m, xd, True)
+    with torch.no_grad():
+        exchange(adapters(m), adapters_b)
+        forward(m.eval(), other, True)
+        exchange(adapters(m), adapters_b)
+    sum((o.float() ** 2).sum() for o in out).backward()
+    same([*(o.detach() for o in out), xd.grad, *(p.grad for p in m.parameters() if p.grad is not None)], want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_adapters_written_in_place(cuda_device, kind):
+    m, x = build(kind, cuda_device), rows(48, cuda_device)
+    for i in range(3):
+        want = train_step(fresh_copy(m, kind, cuda_device), x, True)
+        same(train_step(m, x, True), want)
+        with torch.no_grad():
+            same(forward(m.eval(), x, True), forward(fresh_copy(m, kind, cuda_device).eval(), x, True))
+            for p in adapters(m):
+                p.mul_(1.25)
