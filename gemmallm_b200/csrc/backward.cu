@@ -25,14 +25,16 @@ __global__ void pair_of_kernel(const int32_t* __restrict__ row_of, int64_t M, in
   }
 }
 
-// One warp per sorted row.
+// One warp per sorted row. Rows behind the last expert's (pairs whose router index was out of range, such as those of
+// a token with NaN logits, have none) belong to no pair, and pair_of says nothing about them.
 __global__ void __launch_bounds__(256)
 combine_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y,
-                   const int32_t* __restrict__ pair_of, const float* __restrict__ w, int64_t M, int d,
-                   int k, __nv_bfloat16* __restrict__ dy, float* __restrict__ dw) {
+                   const int32_t* __restrict__ pair_of, const int32_t* __restrict__ offsets, int E,
+                   const float* __restrict__ w, int64_t M, int d, int k, __nv_bfloat16* __restrict__ dy,
+                   float* __restrict__ dw) {
   const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (r >= M) return;
+  if (r >= M || r >= offsets[E]) return;
   const int p = pair_of[r];
   const int64_t t = p / k;
   const float wp = w[p];
@@ -402,12 +404,12 @@ int launch_pair_of(const int32_t* row_of, int64_t M, int32_t* pair_of, cudaStrea
   return 0;
 }
 
-int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, const float* w,
-                       int64_t M, int d, int k, void* dy, float* dw, cudaStream_t s) {
+int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, const int32_t* offsets, int E,
+                       const float* w, int64_t M, int d, int k, void* dy, float* dw, cudaStream_t s) {
   if (M == 0) return 0;
   combine_bwd_kernel<<<blocks_for(M, 8), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(y), pair_of, w, M, d,
-      k, static_cast<__nv_bfloat16*>(dy), dw);
+      static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(y), pair_of, offsets, E, w,
+      M, d, k, static_cast<__nv_bfloat16*>(dy), dw);
   MOE_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

@@ -360,8 +360,8 @@ int launch_experts_gemv(const void* perm, const int32_t* offsets, const void* pl
 
 // ---- backward.cu ----
 int launch_pair_of(const int32_t* row_of, int64_t M, int32_t* pair_of, cudaStream_t s);
-int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, const float* w,
-                       int64_t M, int d, int k, void* dy, float* dw, cudaStream_t s);
+int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, const int32_t* offsets, int E,
+                       const float* w, int64_t M, int d, int k, void* dy, float* dw, cudaStream_t s);
 int64_t router_bwd_scratch_floats(int64_t N, int d, int E);
 int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, const float* dw,
                       const int32_t* cnt0, float grad_aux, const float* grad_aux_dev, const void* x,

@@ -303,7 +303,7 @@ int backward_into(const void* x, const void* Wg, const void* plan, const void* g
   const TrainArgs tr = train_args(tws, to, dropout_p, seed);
 
   // combine (model.py:271) and router (model.py:206-223)
-  rc = launch_combine_bwd(grad_out, y, tr.pair_of, w, M, d, k, dy, dw, s);
+  rc = launch_combine_bwd(grad_out, y, tr.pair_of, offsets, E, w, M, d, k, dy, dw, s);
   if (rc) return rc;
   if (grads.x != nullptr || grads.wg != nullptr || grads.bg != nullptr) {
     rc = launch_router_bwd(logits, idx, w, dw, cnt_slot, grad_aux, grad_aux_dev, x, N, d, E, k, dl, dwg32, grads.wg,

@@ -298,3 +298,37 @@ def test_adapters_written_in_place(cuda_device, kind):
             same(forward(m.eval(), x, True), forward(fresh_copy(m, kind, cuda_device).eval(), x, True))
             for p in adapters(m):
                 p.mul_(1.25)
+
+
+# ---- what a new workspace holds ------------------------------------------------------------------
+
+@pytest.mark.gpu
+def test_training_with_tokens_that_have_no_expert(cuda_device):
+    """A token of NaN has no expert and no sorted row: the step reports it and gives the other tokens' gradients,
+    whatever the new workspaces held (0x7f bytes here: as an index of a pair, far outside)."""
+    m, x = build("moe", cuda_device, p=0.0), rows(200, cuda_device)
+    m.train()
+    with torch.no_grad():
+        x[[3, 77, 199]] = float("nan")
+    clean = torch.ones(200, dtype=torch.bool, device=cuda_device)
+    clean[[3, 77, 199]] = False
+    junk = [torch.full((1 << 24,), 0x7F, dtype=torch.uint8, device=cuda_device) for _ in range(4)]
+    del junk
+    xd = x.clone().requires_grad_(True)
+    out, _ = m(xd)
+    grad = torch.zeros_like(out)
+    grad[clean] = 1.0
+    out.backward(grad)
+    torch.cuda.synchronize()
+    assert m.device_status() != 0
+    assert torch.isfinite(out[clean]).all() and torch.isfinite(xd.grad[clean]).all()
+    assert all(torch.isfinite(p.grad).all() for n, p in m.named_parameters() if p.grad is not None and "gate." not in n)
+    # the clean tokens' part is what the same step without the others gives
+    only = fresh_copy(m, "moe", cuda_device, p=0.0).train()
+    xo = x[clean].clone().requires_grad_(True)
+    oo, _ = only(xo)
+    oo.backward(torch.ones_like(oo))
+    assert torch.equal(out[clean], oo)
+    for (n, p), q in zip(m.named_parameters(), only.parameters()):
+        if p.grad is not None and "experts" in n:
+            assert (p.grad.float() - q.grad.float()).norm() <= 1e-3 * q.grad.float().norm(), n
