@@ -577,17 +577,22 @@ class Edges {
   }
   void add(const Tensor& t) {
     any_ |= t.requires_grad();
+    tangent_ |= t._fw_grad(0).defined();
     list_.push_back(torch::autograd::impl::gradient_edge(t));
   }
   void add_empty() { list_.emplace_back(); }
   bool wanted() const { return any_ && at::GradMode::is_enabled(); }
+  // The node has no forward-mode derivative: a call on dual tensors would lose their tangents.
+  void refuse_tangents() const {
+    TORCH_CHECK_NOT_IMPLEMENTED(!tangent_, "training mode has no forward-mode derivative (jvp)");
+  }
   edge_list take() { return std::move(list_); }
   std::vector<Held> take_weights() { return std::move(weights_); }
 
  private:
   edge_list list_;
   std::vector<Held> weights_;
-  bool any_ = false;
+  bool any_ = false, tangent_ = false;
 };
 
 at::ScalarType scalar_of(int dtype) { return dtype == MOE_B200_BF16 ? at::kBFloat16 : at::kFloat; }
@@ -838,6 +843,7 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     gate_w = THPVariable_Unpack(PyList_GET_ITEM(args[3], 0));
     gate_b = THPVariable_Unpack(PyList_GET_ITEM(args[3], 1));
   }
+  edges.refuse_tangents();
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)c->device);
   void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c->device).stream();
   if (args[3] == Py_None) {
@@ -1040,6 +1046,7 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
       edges.add_param(THPVariable_Unpack(v));
     }
   }
+  edges.refuse_tangents();
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)c->device);
   void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c->device).stream();
   if (args[2] == Py_None) {

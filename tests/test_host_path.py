@@ -332,3 +332,23 @@ def test_training_with_tokens_that_have_no_expert(cuda_device):
     for (n, p), q in zip(m.named_parameters(), only.parameters()):
         if p.grad is not None and "experts" in n:
             assert (p.grad.float() - q.grad.float()).norm() <= 1e-3 * q.grad.float().norm(), n
+
+
+# ---- what an autograd function in Python refused, kept or passed on --------------------------------
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_forward_mode_derivatives_are_refused(cuda_device, kind):
+    import torch.autograd.forward_ad as fw
+    m, x = build(kind, cuda_device).train(), rows(48, cuda_device)
+    for _ in range(3):           # unbound, then bound
+        with fw.dual_level():
+            with pytest.raises(NotImplementedError):
+                m(fw.make_dual(x, torch.ones_like(x)))
+            with torch.no_grad(), pytest.raises(NotImplementedError):
+                m(fw.make_dual(x, torch.ones_like(x)))
+        train_step(m, x)
+    for transform in (lambda f: torch.func.grad(lambda z: f(z).float().sum())(x), lambda f: torch.func.vmap(f)(x[None]),
+                      lambda f: torch.func.jvp(f, (x,), (torch.ones_like(x),))):
+        with pytest.raises(RuntimeError):
+            transform(lambda z: forward(m, z)[0])
