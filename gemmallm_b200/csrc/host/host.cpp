@@ -22,6 +22,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <algorithm>
 #include <memory>
@@ -805,6 +806,7 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     return nullptr;
   }
   if (*self->train == nullptr || !THPVariable_Check(args[0])) Py_RETURN_NONE;
+  if (args[3] == Py_None && torch::jit::tracer::isTracing()) Py_RETURN_NONE;
   const std::shared_ptr<TrainCall> c = *self->train;
   const Tensor& x = THPVariable_Unpack(args[0]);
   if (!rows_match(x, c->device, MOE_B200_BF16, c->d, c->N)) Py_RETURN_NONE;
@@ -1024,6 +1026,8 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     return nullptr;
   }
   if (*self->train == nullptr || !THPVariable_Check(args[0])) Py_RETURN_NONE;
+  // (under a tracer the module takes a way that the tracer sees)
+  if (args[2] == Py_None && torch::jit::tracer::isTracing()) Py_RETURN_NONE;
   const std::shared_ptr<TrainCall> c = *self->train;
   const Tensor& x = THPVariable_Unpack(args[0]);
   if (!rows_match(x, c->device, MOE_B200_BF16, c->d, c->N)) Py_RETURN_NONE;

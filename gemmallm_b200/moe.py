@@ -145,6 +145,26 @@ class _Plan:
         return self.base
 
 
+class _TracedFfn(torch.autograd.Function):
+    """FeedForward's training forward as torch.jit.trace can record it, a Python operator: the native call's own graph
+    stays inside, and every run of the traced function draws a mask."""
+
+    @staticmethod
+    def forward(ctx, module, tensor, fine_tuning, *params):
+        with torch.enable_grad():
+            x = tensor.detach().requires_grad_(tensor.requires_grad)
+            y, _ = module._prepare_train(x, fine_tuning, module._native_train_ft if fine_tuning else module._native_train)
+        ctx.graph = y, [t for t in (x, *params) if t.requires_grad], [t.requires_grad for t in (x, *params)]
+        return y.detach()
+
+    @staticmethod
+    def backward(ctx, grad):
+        y, inputs, wanted = ctx.graph
+        grads = iter(torch.autograd.grad(y, inputs, grad, retain_graph=True))
+        gx, *gp = [next(grads) if w else None for w in wanted]
+        return (None, gx, None, *gp)
+
+
 class FeedForward(nn.Module):
     """GeGLU feed-forward expert; mirrors reference model.py:154-190.
 
@@ -251,6 +271,8 @@ class FeedForward(nn.Module):
                 raise NotImplementedError("training mode computes in bfloat16")
             native = self._native_train_ft if fine_tuning else self._native_train
             done = native.train(tensor, self.dropout.p, None)
+            if done is None and torch.jit.is_tracing():
+                return _TracedFfn.apply(self, tensor, bool(fine_tuning), *_expert_params(self, fine_tuning))
             if done is None:
                 done = self._prepare_train(tensor, bool(fine_tuning), native)
             y, self.last_seed = done
@@ -392,6 +414,8 @@ class MOE(nn.Module):
                 raise NotImplementedError("training mode computes in bfloat16")
             native = self._native_train_ft if fine_tuning else self._native_train
             done = native.train(tensor, residual, self.experts[0].dropout.p, None)
+            if done is None and torch.jit.is_tracing():
+                raise RuntimeError("the block's training forward cannot be traced")
             if done is None:
                 done = self._prepare_train(tensor, residual, bool(fine_tuning), native)
             out, aux, self._last_seed = done

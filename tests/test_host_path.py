@@ -352,3 +352,30 @@ def test_forward_mode_derivatives_are_refused(cuda_device, kind):
                       lambda f: torch.func.jvp(f, (x,), (torch.ones_like(x),))):
         with pytest.raises(RuntimeError):
             transform(lambda z: forward(m, z)[0])
+
+
+@pytest.mark.gpu
+def test_traced_training_forward(cuda_device):
+    """torch.jit.trace of the feed-forward in training mode (no dropout, so that runs agree) computes and has gradients;
+    the block's was refused and is."""
+    m, x = build("ffn", cuda_device, p=0.0).train(), rows(48, cuda_device)
+    for _ in range(2):
+        train_step(m, x)
+    traced = torch.jit.trace(m, (x,), check_trace=False)
+    other = rows(48, cuda_device, 2)
+    want = train_step(fresh_copy(m, "ffn", cuda_device, p=0.0), other)
+    same(_traced_step(traced, m, other), want)
+    block = build("moe", cuda_device).train()
+    for _ in range(2):
+        train_step(block, x)
+        with pytest.raises(RuntimeError):
+            torch.jit.trace(block, (x,), check_trace=False)
+
+
+def _traced_step(traced, m, x):
+    for p in m.parameters():
+        p.grad = None
+    x = x.clone().requires_grad_(True)
+    y = traced(x)
+    (y.float() ** 2).sum().backward()
+    return [y.detach(), x.grad, *(p.grad for p in m.parameters() if p.grad is not None)]
