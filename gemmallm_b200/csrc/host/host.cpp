@@ -760,7 +760,7 @@ PyObject* block_forward(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     PyErr_SetString(PyExc_TypeError, "forward(tensor, residual, norm)");
     return nullptr;
   }
-  if (self->watch->empty() || !THPVariable_Check(args[0])) Py_RETURN_NONE;
+  if (self->watch->empty() || !THPVariable_CheckExact(args[0])) Py_RETURN_NONE;    // the result is of the input's class
   const Tensor& x = THPVariable_Unpack(args[0]);
   if (self->N <= 0 || !rows_match(x, self->device, self->dtype, self->d, self->N)) Py_RETURN_NONE;
   const void* res = nullptr;
@@ -806,6 +806,7 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     return nullptr;
   }
   if (*self->train == nullptr || !THPVariable_Check(args[0])) Py_RETURN_NONE;
+  if (args[3] == Py_None && !THPVariable_CheckExact(args[0])) Py_RETURN_NONE;    // the result is of the input's class
   if (args[3] == Py_None && torch::jit::tracer::isTracing()) Py_RETURN_NONE;
   const std::shared_ptr<TrainCall> c = *self->train;
   const Tensor& x = THPVariable_Unpack(args[0]);

@@ -542,6 +542,8 @@ class MOE(nn.Module):
             for ex in self.experts:
                 params += _expert_params(ex, fine_tuning)
             out, aux, seed = native.train(x, residual, float(self.experts[0].dropout.p), params)
+        if type(tensor) not in (torch.Tensor, nn.Parameter):
+            out = out.as_subclass(type(tensor))
         return out.reshape(shape), aux, seed
 
     def device_status(self) -> int:

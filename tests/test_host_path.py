@@ -379,3 +379,14 @@ def _traced_step(traced, m, x):
     y = traced(x)
     (y.float() ** 2).sum().backward()
     return [y.detach(), x.grad, *(p.grad for p in m.parameters() if p.grad is not None)]
+
+
+@pytest.mark.gpu
+def test_the_block_keeps_the_class_of_its_input(cuda_device):
+    class Rows(torch.Tensor):
+        pass
+    m, x = build("moe", cuda_device, p=0.0), rows(48, cuda_device)
+    for module in (m.train(), m.eval()):
+        for _ in range(3):
+            assert type(module(x)[0]) is torch.Tensor and type(module(x.as_subclass(Rows))[0]) is Rows
+            assert torch.equal(module(x)[0], module(x.as_subclass(Rows))[0])
