@@ -453,6 +453,14 @@ Tensor output_grad(const Tensor& g, const Tensor& like) {
   return g.to(like.scalar_type()).contiguous();
 }
 
+// A saved tensor of N rows of `cols`, whatever hooks made of it in between.
+Tensor unpacked(const SavedVariable& v, const TrainCall& c, int64_t cols) {
+  Tensor t = v.unpack();
+  TORCH_CHECK(t.is_cuda() && t.device().index() == c.device && t.scalar_type() == at::kBFloat16 && t.numel() == c.N * cols,
+              "a saved tensor came back with another size, dtype or device");
+  return t.contiguous();
+}
+
 void check_generation(const TrainCall& c, int64_t gen) {
   if (*c.gen != gen)
     throw std::runtime_error("this module ran another training forward before the backward of this one: its "
@@ -478,7 +486,7 @@ struct BlockBackward : public Node {
     const TrainCall& c = *call;
     check_generation(c, gen);
     at::AutoGradMode no_grad(false);
-    const Tensor xv = x.unpack();
+    const Tensor xv = unpacked(x, c, c.d);
     c10::cuda::CUDAGuard guard((c10::DeviceIndex)c.device);
     void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c.device).stream();
     const Tensor go = output_grad(grads[0], xv);
@@ -521,8 +529,7 @@ struct BlockBackward : public Node {
 // inputs: x, the parameters
 struct FfnBackward : public Node {
   std::shared_ptr<TrainCall> call;
-  SavedVariable x;
-  Tensor h;
+  SavedVariable x, h;
   std::vector<Held> weights;
   int64_t gen = 0;
   uint64_t seed = 0;
@@ -531,14 +538,14 @@ struct FfnBackward : public Node {
   std::string name() const override { return "FeedForwardBackward"; }
   void release_variables() override {
     x.reset_data();
-    h.reset();
+    h.reset_data();
     weights.clear();
   }
   variable_list apply(variable_list&& grads) override {
     const TrainCall& c = *call;
     check_generation(c, gen);
     at::AutoGradMode no_grad(false);
-    const Tensor xv = x.unpack();
+    const Tensor xv = unpacked(x, c, c.d), hv = unpacked(h, c, c.f);
     c10::cuda::CUDAGuard guard((c10::DeviceIndex)c.device);
     void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c.device).stream();
     const Tensor go = output_grad(grads[0], xv);
@@ -553,7 +560,7 @@ struct FfnBackward : public Node {
     const moe::LoraGrads lg = eg.prepare(c, opt, &g, wanted);
     if (c.N > 0) {
       check_rc(c.lora.refresh(weights, MOE_B200_BF16, stream), "lora_merge");
-      check_rc(moe::experts_backward_into(xv.const_data_ptr(), h.const_data_ptr(), c.offsets.const_data_ptr<int32_t>(),
+      check_rc(moe::experts_backward_into(xv.const_data_ptr(), hv.const_data_ptr(), c.offsets.const_data_ptr<int32_t>(),
                                           c.plan, go.const_data_ptr(), c.N, c.d, c.f, 1, (float)p, seed, c.tws_base,
                                           c.tws_bytes, g, lg.tab != nullptr ? &lg : nullptr,
                                           c.status.data_ptr<int32_t>(), stream),
@@ -1078,8 +1085,8 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     node->gen = *c->gen;
     node->seed = seed;
     node->p = p;
-    node->h = std::move(h);
     node->x = SavedVariable(x, false);
+    node->h = SavedVariable(h, false);
     torch::autograd::set_history(y, node);
   }
   PyObject* t = PyTuple_New(2);

@@ -390,3 +390,24 @@ def test_the_block_keeps_the_class_of_its_input(cuda_device):
         for _ in range(3):
             assert type(module(x)[0]) is torch.Tensor and type(module(x.as_subclass(Rows))[0]) is Rows
             assert torch.equal(module(x)[0], module(x.as_subclass(Rows))[0])
+
+
+@pytest.mark.gpu
+def test_saved_tensor_hooks_see_what_is_saved(cuda_device):
+    """Input and, for the feed-forward, h: moved to the host and back between forward and backward."""
+    from torch.autograd.graph import saved_tensors_hooks
+    for kind, shapes in (("moe", [(48, D)]), ("ffn", [(48, D), (48, F)])):
+        m, x = build(kind, cuda_device), rows(48, cuda_device)
+        want = train_step(fresh_copy(m, kind, cuda_device), x)
+        for _ in range(3):
+            seen = []
+            m.train()
+            for p in m.parameters():
+                p.grad = None
+            xd = x.clone().requires_grad_(True)
+            torch.manual_seed(5)
+            with saved_tensors_hooks(lambda t: (seen.append(tuple(t.shape)), t.cpu())[1], lambda t: t.to(cuda_device)):
+                out = forward(m, xd)
+            assert seen == shapes
+            sum((o.float() ** 2).sum() for o in out).backward()
+            same([*(o.detach() for o in out), xd.grad, *(p.grad for p in m.parameters() if p.grad is not None)], want)
