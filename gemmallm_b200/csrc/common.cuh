@@ -375,10 +375,10 @@ int launch_colsum(const void* src, const int32_t* offsets, int64_t M, int E, int
 int launch_colsum_finish(const float* part, int slots, const int32_t* offsets, int E, int C, void* db, cudaStream_t s);
 
 // ---- lora_bwd.cu ----
-// LoRA gradients of both Linears (index 0: gate_and_up, 1: down) of every expert from the gradients of their merged
-// weights G [E, out, in] and biases g [E, out]; tab [2][E][3] device pointers A, a, B.
-int launch_lora_grads(const void* const* tab, int d, int f, int E, int rank, float scale, float* scratch,
-                      const void* const (&G)[2], const void* const (&g)[2], void* const (&dA)[2], void* const (&da)[2],
-                      void* const (&dB)[2], void* const (&db)[2], cudaStream_t s);
+// LoRA gradients of both Linears (index 0: gate_and_up, 1: down) of a run of the E experts from the gradients of all
+// their merged weights G [E, out, in] and biases g [E, out]; tab [2][E][3] device pointers A, a, B.
+struct LoraRun;
+int launch_lora_grads(const void* const* tab, int d, int f, int E, const LoraRun& run, float* scratch,
+                      const void* const (&G)[2], const void* const (&g)[2], cudaStream_t s);
 
 }  // namespace moe

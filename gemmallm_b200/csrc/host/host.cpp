@@ -7,7 +7,7 @@
 // merged LoRA weights) and bind() the result; forward() answers from what is bound, or returns None
 // for every call that differs from it in any way, and the Python side then prepares again.
 // What is bound is found changed by identity: the module tree's own dictionaries must still hold
-// the same submodules and parameters, and every parameter the same storage.
+// the same submodules, parameters and plain attributes (scales, slots), and every parameter the same storage.
 //
 // Lifetime: a bound call owns every buffer whose address it has (plan, workspaces, merged weights): the Python side may
 // replace its own, and the parameters may leave and come back (weights exchanged for an evaluation) with the binding
@@ -62,7 +62,7 @@ struct Watch {
   PyObject* dict;
   PyObject* key;
   PyObject* value;
-  const void* data;      // parameters: storage address; nullptr for submodules
+  const void* data;      // parameters: storage address; nullptr for submodules and plain attributes
 };
 
 class WatchList {
@@ -99,6 +99,14 @@ class WatchList {
       if (w.data != nullptr && THPVariable_Unpack(w.value).const_data_ptr() != w.data) return false;
     }
     return true;
+  }
+  int traverse(visitproc visit, void* arg) const {
+    for (const Watch& w : items_) {
+      Py_VISIT(w.dict);
+      Py_VISIT(w.key);
+      Py_VISIT(w.value);
+    }
+    return 0;
   }
   const Tensor& param(int i) const { return THPVariable_Unpack(items_[params_[i]].value); }
   int num_params() const { return (int)params_.size(); }
@@ -378,8 +386,8 @@ struct TrainCall {
   void *ws_base = nullptr, *tws_base = nullptr;
   size_t ws_bytes = 0, tws_bytes = 0;
   int64_t N = 0;
-  int d = 0, f = 0, E = 0, k = 0, device = 0, rank = 0;
-  double lora_scale = 0.0;
+  int d = 0, f = 0, E = 0, k = 0, device = 0;
+  std::vector<int> ranks;      // of gate_and_up and down of every expert; empty without LoRA branches
   std::shared_ptr<int64_t> gen;
 };
 
@@ -397,54 +405,73 @@ void check_rc(int rc, const char* what) {
 // gate_and_up a, b and down a, b; `wanted(i)` says whether the i-th of them (counted over the experts) is.
 struct ExpertGrads {
   Tensor w1, b1, w2, b2, scratch;
-  Tensor dA[2], da[2], dB[2], db[2];
+  std::vector<Tensor> lora;      // eight an expert
+  moe::LoraGrads lora_args = {};
   int per = 4;
 
+  // the arguments of the pass; LoRA gradients are wanted if lora_args.tab is set
   template <typename Wanted>
-  moe::LoraGrads prepare(const TrainCall& c, const at::TensorOptions& opt, moe::TrainGrads* g, Wanted wanted) {
+  void prepare(const TrainCall& c, const at::TensorOptions& opt, moe::TrainGrads* g, Wanted wanted) {
     const int64_t E = c.E, d = c.d, f = c.f;
-    per = c.rank > 0 ? 12 : 4;
+    per = c.ranks.empty() ? 4 : 12;
     bool need[12] = {};
     for (int64_t e = 0; e < E; ++e)
       for (int i = 0; i < per; ++i) need[i] |= wanted(e * per + i);
-    bool lora = false;
-    for (int i = 4; i < per; ++i) lora |= need[i];
-    if (need[0] || lora) w1 = at::empty({E, 2 * f, d}, opt);
-    if (need[1] || lora) b1 = at::empty({E, 2 * f}, opt);
-    if (need[2] || lora) w2 = at::empty({E, d, f}, opt);
-    if (need[3] || lora) b2 = at::empty({E, d}, opt);
+    bool with_lora = false;
+    for (int i = 4; i < per; ++i) with_lora |= need[i];
+    if (need[0] || with_lora) w1 = at::empty({E, 2 * f, d}, opt);
+    if (need[1] || with_lora) b1 = at::empty({E, 2 * f}, opt);
+    if (need[2] || with_lora) w2 = at::empty({E, d, f}, opt);
+    if (need[3] || with_lora) b2 = at::empty({E, d}, opt);
     auto ptr = [](Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
     g->w1 = ptr(w1);
     g->b1 = ptr(b1);
     g->w2 = ptr(w2);
     g->b2 = ptr(b2);
-    moe::LoraGrads lg = {};
-    if (lora) {
-      const int64_t in[2] = {d, f}, out[2] = {2 * f, d}, r = c.rank;
-      scratch = at::empty({(int64_t)moe::lora_grads_scratch_floats(c.d, c.f, c.E, c.rank)}, opt.dtype(at::kFloat));
-      lg.tab = static_cast<const void* const*>(c.lora_tab.const_data_ptr());
-      lg.rank = c.rank;
-      lg.scale = (float)c.lora_scale;
-      lg.scratch = scratch.data_ptr<float>();
+    if (!with_lora) return;
+    // experts of one rank and scale, which is all of them unless someone replaced some, in one run
+    bool alike = true;
+    for (int64_t e = 1; e < E; ++e)
+      alike = alike && c.ranks[2 * e] == c.ranks[0] && c.ranks[2 * e + 1] == c.ranks[1] && c.lora.scales[e] == c.lora.scales[0];
+    const int64_t ne = alike ? E : 1;
+    lora.resize(8 * E);
+    size_t floats = 0;
+    const int64_t in[2] = {d, f}, out[2] = {2 * f, d};
+    for (int64_t e0 = 0; e0 < E; e0 += ne) {
+      moe::LoraRun run = {};
+      run.first = (int)e0;
+      run.count = (int)ne;
+      run.scale = (float)c.lora.scales[e0];
       for (int l = 0; l < 2; ++l) {
-        dA[l] = at::empty({E, r, in[l]}, opt);
-        da[l] = at::empty({E, r}, opt);
-        dB[l] = at::empty({E, out[l], r}, opt);
-        db[l] = at::empty({E, out[l]}, opt);
-        lg.dA[l] = dA[l].data_ptr();
-        lg.da[l] = da[l].data_ptr();
-        lg.dB[l] = dB[l].data_ptr();
-        lg.db[l] = db[l].data_ptr();
+        const int64_t r = run.rank[l] = c.ranks[2 * e0 + l];
+        Tensor t[4] = {at::empty({ne, r, in[l]}, opt), at::empty({ne, r}, opt), at::empty({ne, out[l], r}, opt),
+                       at::empty({ne, out[l]}, opt)};
+        run.dA[l] = t[0].data_ptr();
+        run.da[l] = t[1].data_ptr();
+        run.dB[l] = t[2].data_ptr();
+        run.db[l] = t[3].data_ptr();
+        for (int64_t e = 0; e < ne; ++e)
+          for (int q = 0; q < 4; ++q) lora[(e0 + e) * 8 + l * 4 + q] = t[q].select(0, e);
       }
+      floats = std::max(floats, moe::lora_grads_scratch_floats(c.d, c.f, run));
+      lora_args.runs.push_back(run);
     }
-    return lg;
+    scratch = at::empty({(int64_t)floats}, opt.dtype(at::kFloat));
+    lora_args.tab = static_cast<const void* const*>(c.lora_tab.const_data_ptr());
+    lora_args.scratch = scratch.data_ptr<float>();
+  }
+  const moe::LoraGrads* lora_grads() const { return lora_args.tab != nullptr ? &lora_args : nullptr; }
+  void zero() {
+    for (Tensor* t : {&w1, &b1, &w2, &b2})
+      if (t->defined()) t->zero_();
+    for (Tensor& t : lora) t.zero_();
   }
   template <typename Wanted>
   void collect(int64_t E, variable_list* out, size_t first, Wanted wanted) {
-    Tensor* all[12] = {&w1, &b1, &w2, &b2, &dA[0], &da[0], &dB[0], &db[0], &dA[1], &da[1], &dB[1], &db[1]};
+    Tensor* base[4] = {&w1, &b1, &w2, &b2};
     for (int64_t e = 0; e < E; ++e)
       for (int i = 0; i < per; ++i)
-        if (wanted(e * per + i)) (*out)[first + e * per + i] = all[i]->select(0, e);
+        if (wanted(e * per + i)) (*out)[first + e * per + i] = i < 4 ? base[i]->select(0, e) : lora[e * 8 + i - 4];
   }
 };
 
@@ -504,18 +531,18 @@ struct BlockBackward : public Node {
     g.bg = gbg.defined() ? gbg.data_ptr() : nullptr;
     auto wanted = [&](int64_t i) { return task_should_compute_output(4 + (size_t)i); };
     ExpertGrads eg;
-    const moe::LoraGrads lg = eg.prepare(c, opt, &g, wanted);
+    eg.prepare(c, opt, &g, wanted);
     if (c.N > 0) {
       check_rc(c.lora.refresh(weights, MOE_B200_BF16, stream), "lora_merge");
       check_rc(moe::backward_into(xv.const_data_ptr(), gate_w.const_data_ptr(), c.plan, go.const_data_ptr(), 0.f,
                                   aux.defined() ? aux.const_data_ptr<float>() : nullptr, c.N, c.d, c.f, c.E, c.k,
                                   MOE_B200_BF16, (float)p, seed, c.ws_base, c.ws_bytes, c.tws_base, c.tws_bytes, g,
-                                  lg.tab != nullptr ? &lg : nullptr, stream),
+                                  eg.lora_grads(), stream),
                "backward");
     } else {
-      for (Tensor* t : {&gwg, &gbg, &eg.w1, &eg.b1, &eg.w2, &eg.b2, &eg.dA[0], &eg.da[0], &eg.dB[0], &eg.db[0], &eg.dA[1],
-                        &eg.da[1], &eg.dB[1], &eg.db[1]})
+      for (Tensor* t : {&gwg, &gbg})
         if (t->defined()) t->zero_();
+      eg.zero();
     }
     out[0] = gx;
     if (task_should_compute_output(1)) out[1] = grads[0].defined() ? grads[0] : go;
@@ -557,24 +584,34 @@ struct FfnBackward : public Node {
     g.x = gx.defined() ? gx.data_ptr() : nullptr;
     auto wanted = [&](int64_t i) { return task_should_compute_output(1 + (size_t)i); };
     ExpertGrads eg;
-    const moe::LoraGrads lg = eg.prepare(c, opt, &g, wanted);
+    eg.prepare(c, opt, &g, wanted);
     if (c.N > 0) {
       check_rc(c.lora.refresh(weights, MOE_B200_BF16, stream), "lora_merge");
       check_rc(moe::experts_backward_into(xv.const_data_ptr(), hv.const_data_ptr(), c.offsets.const_data_ptr<int32_t>(),
                                           c.plan, go.const_data_ptr(), c.N, c.d, c.f, 1, (float)p, seed, c.tws_base,
-                                          c.tws_bytes, g, lg.tab != nullptr ? &lg : nullptr,
-                                          c.status.data_ptr<int32_t>(), stream),
+                                          c.tws_bytes, g, eg.lora_grads(), c.status.data_ptr<int32_t>(), stream),
                "experts_backward");
     } else {
-      for (Tensor* t : {&eg.w1, &eg.b1, &eg.w2, &eg.b2, &eg.dA[0], &eg.da[0], &eg.dB[0], &eg.db[0], &eg.dA[1], &eg.da[1],
-                        &eg.dB[1], &eg.db[1]})
-        if (t->defined()) t->zero_();
+      eg.zero();
     }
     out[0] = gx;
     eg.collect(1, &out, 1, wanted);
     return out;
   }
 };
+
+// Two ranks for every expert that `lora` merges.
+bool read_ranks(PyObject* seq, const MergedUse& lora, std::vector<int>* out) {
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(seq); ++i) {
+    out->push_back((int)PyLong_AsLong(PyList_GET_ITEM(seq, i)));
+    if (PyErr_Occurred()) return false;
+  }
+  if (out->size() != 2 * lora.scales.size()) {
+    PyErr_SetString(PyExc_ValueError, "two ranks for every expert");
+    return false;
+  }
+  return true;
+}
 
 // Edges of a call's inputs, and those of them that are parameters.
 class Edges {
@@ -662,7 +699,22 @@ PyObject* block_new(PyTypeObject* type, PyObject*, PyObject*) {
   return reinterpret_cast<PyObject*>(self);
 }
 
+// The watched tree of a module holds the module's own dictionary, and that the binding.
+int block_traverse(PyObject* o, visitproc visit, void* arg) {
+  Py_VISIT(Py_TYPE(o));
+  const WatchList* w = reinterpret_cast<Block*>(o)->watch;
+  return w != nullptr ? w->traverse(visit, arg) : 0;
+}
+
+PyObject* block_unbind(PyObject* o, PyObject*);
+
+int block_clear(PyObject* o) {
+  Py_XDECREF(block_unbind(o, nullptr));
+  return 0;
+}
+
 void block_dealloc(PyObject* o) {
+  PyObject_GC_UnTrack(o);
   Block* self = reinterpret_cast<Block*>(o);
   PyTypeObject* type = Py_TYPE(o);
   delete self->watch;
@@ -719,20 +771,18 @@ PyObject* block_unbind(PyObject* o, PyObject*) {
   Py_RETURN_NONE;
 }
 
-// bind_train(training workspace, base, bytes, LoRA pointer table or None, rank, scale, generation): after bind()
+// bind_train(training workspace, base, bytes, LoRA pointer table or None, ranks, generation): after bind()
 PyObject* block_bind_train(PyObject* o, PyObject* args) {
   HANDLE_TH_ERRORS
   Block* self = reinterpret_cast<Block*>(o);
-  PyObject *tws, *tab, *gen;
+  PyObject *tws, *tab, *ranks, *gen;
   unsigned long long base, bytes;
-  int rank;
-  double scale;
-  if (!PyArg_ParseTuple(args, "OKKOidO", &tws, &base, &bytes, &tab, &rank, &scale, &gen)) return nullptr;
+  if (!PyArg_ParseTuple(args, "OKKOO!O", &tws, &base, &bytes, &tab, &PyList_Type, &ranks, &gen)) return nullptr;
   auto c = std::make_shared<TrainCall>();
-  if (!read_generation(gen, &c->gen)) return nullptr;
+  c->lora = *self->lora;
+  if (!read_generation(gen, &c->gen) || !read_ranks(ranks, c->lora, &c->ranks)) return nullptr;
   c->ws = *self->workspace;
   c->owned = *self->owned;
-  c->lora = *self->lora;
   c->tws = THPVariable_Unpack(tws);
   if (tab != Py_None) c->lora_tab = THPVariable_Unpack(tab);
   c->plan = self->plan;
@@ -746,8 +796,6 @@ PyObject* block_bind_train(PyObject* o, PyObject* args) {
   c->E = self->E;
   c->k = self->k;
   c->device = self->device;
-  c->rank = rank;
-  c->lora_scale = scale;
   *self->train = std::move(c);
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
@@ -907,9 +955,12 @@ PyMethodDef block_methods[] = {
     {nullptr, nullptr, 0, nullptr}};
 PyType_Slot block_slots[] = {{Py_tp_new, reinterpret_cast<void*>(block_new)},
                              {Py_tp_dealloc, reinterpret_cast<void*>(block_dealloc)},
+                             {Py_tp_traverse, reinterpret_cast<void*>(block_traverse)},
+                             {Py_tp_clear, reinterpret_cast<void*>(block_clear)},
                              {Py_tp_methods, block_methods},
                              {0, nullptr}};
-PyType_Spec block_spec = {"gemmallm_b200._host.Block", sizeof(Block), 0, Py_TPFLAGS_DEFAULT, block_slots};
+PyType_Spec block_spec = {"gemmallm_b200._host.Block", sizeof(Block), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC,
+                          block_slots};
 
 // ---- the dense feed-forward ------------------------------------------------------------------
 
@@ -938,7 +989,21 @@ PyObject* ffn_new(PyTypeObject* type, PyObject*, PyObject*) {
   return reinterpret_cast<PyObject*>(self);
 }
 
+int ffn_traverse(PyObject* o, visitproc visit, void* arg) {
+  Py_VISIT(Py_TYPE(o));
+  const WatchList* w = reinterpret_cast<Ffn*>(o)->watch;
+  return w != nullptr ? w->traverse(visit, arg) : 0;
+}
+
+PyObject* ffn_unbind(PyObject* o, PyObject*);
+
+int ffn_clear(PyObject* o) {
+  Py_XDECREF(ffn_unbind(o, nullptr));
+  return 0;
+}
+
 void ffn_dealloc(PyObject* o) {
+  PyObject_GC_UnTrack(o);
   Ffn* self = reinterpret_cast<Ffn*>(o);
   PyTypeObject* type = Py_TYPE(o);
   delete self->watch;
@@ -992,20 +1057,18 @@ PyObject* ffn_unbind(PyObject* o, PyObject*) {
   Py_RETURN_NONE;
 }
 
-// bind_train(training workspace, base, bytes, LoRA pointer table or None, rank, scale, generation): after bind()
+// bind_train(training workspace, base, bytes, LoRA pointer table or None, ranks, generation): after bind()
 PyObject* ffn_bind_train(PyObject* o, PyObject* args) {
   HANDLE_TH_ERRORS
   Ffn* self = reinterpret_cast<Ffn*>(o);
-  PyObject *tws, *tab, *gen;
+  PyObject *tws, *tab, *ranks, *gen;
   unsigned long long base, bytes;
-  int rank;
-  double scale;
-  if (!PyArg_ParseTuple(args, "OKKOidO", &tws, &base, &bytes, &tab, &rank, &scale, &gen)) return nullptr;
+  if (!PyArg_ParseTuple(args, "OKKOO!O", &tws, &base, &bytes, &tab, &PyList_Type, &ranks, &gen)) return nullptr;
   auto c = std::make_shared<TrainCall>();
-  if (!read_generation(gen, &c->gen)) return nullptr;
+  c->lora = *self->lora;
+  if (!read_generation(gen, &c->gen) || !read_ranks(ranks, c->lora, &c->ranks)) return nullptr;
   c->tws = THPVariable_Unpack(tws);
   c->owned = *self->owned;
-  c->lora = *self->lora;
   c->offsets = *self->offsets;
   c->status = *self->status;
   if (tab != Py_None) c->lora_tab = THPVariable_Unpack(tab);
@@ -1018,8 +1081,6 @@ PyObject* ffn_bind_train(PyObject* o, PyObject* args) {
   c->E = 1;
   c->k = 1;
   c->device = self->device;
-  c->rank = rank;
-  c->lora_scale = scale;
   *self->train = std::move(c);
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
@@ -1146,9 +1207,11 @@ PyType_Spec generation_spec = {"gemmallm_b200._host.Generation", sizeof(Generati
 
 PyType_Slot ffn_slots[] = {{Py_tp_new, reinterpret_cast<void*>(ffn_new)},
                            {Py_tp_dealloc, reinterpret_cast<void*>(ffn_dealloc)},
+                           {Py_tp_traverse, reinterpret_cast<void*>(ffn_traverse)},
+                           {Py_tp_clear, reinterpret_cast<void*>(ffn_clear)},
                            {Py_tp_methods, ffn_methods},
                            {0, nullptr}};
-PyType_Spec ffn_spec = {"gemmallm_b200._host.Ffn", sizeof(Ffn), 0, Py_TPFLAGS_DEFAULT, ffn_slots};
+PyType_Spec ffn_spec = {"gemmallm_b200._host.Ffn", sizeof(Ffn), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC, ffn_slots};
 
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
 

@@ -3,6 +3,7 @@
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
+#include <vector>
 
 namespace moe {
 
@@ -19,16 +20,19 @@ struct TrainGrads {
   void *w1, *b1, *w2, *b2;   // experts [E, 2f, d], [E, 2f], [E, d, f], [E, d]
 };
 
-// LoRA gradients of both Linears (0: gate_and_up, 1: down) of all experts; they are formed from w1, b1, w2 and b2 of
-// TrainGrads, which are needed with them.
+// LoRA gradients of both Linears (0: gate_and_up, 1: down); they are formed from w1, b1, w2 and b2 of TrainGrads,
+// which are needed with them. A run: experts [first, first + count) of the same ranks and scale.
+struct LoraRun {
+  int first, count, rank[2];
+  float scale;
+  void *dA[2], *da[2], *dB[2], *db[2];   // [count, rank, in], [count, rank], [count, out, rank], [count, out]
+};
 struct LoraGrads {
   const void* const* tab;    // device [2][E][3]: A, a, B of every expert
-  int rank;
-  float scale;
-  float* scratch;            // lora_grads_scratch_floats() floats
-  void *dA[2], *da[2], *dB[2], *db[2];   // [E, rank, in], [E, rank], [E, out, rank], [E, out]
+  float* scratch;            // as many floats as the largest run asks for
+  std::vector<LoraRun> runs;
 };
-size_t lora_grads_scratch_floats(int d, int f, int E, int rank);
+size_t lora_grads_scratch_floats(int d, int f, const LoraRun& run);
 
 // moe_b200_forward_train with the load-balancing loss written to `aux` (nullptr: the workspace's word).
 int forward_train_into(const void* x, const void* Wg, const void* bg, const void* plan, const void* residual,

@@ -13,7 +13,9 @@
 //   lora_finish_kernel  sums over ranges and segments in order, the bias terms, scale, rounding
 // (A step of the dense feed-forward at 1632 rows, d 1024, f 4096: 277 us, 246 us from the activations.)
 // Products of bf16 are exact in fp32 and all sums are fp32, so the only rounding behind G is that of the results.
+#include <algorithm>
 #include "common.cuh"
+#include "internal.h"
 
 namespace moe {
 
@@ -234,15 +236,15 @@ lora_finish_kernel(const __grid_constant__ Jobs jobs, float scale) {
 }
 
 // Sizes of both Linears and their places in the scratch buffer; returns its floats.
-size_t lay_out(Jobs* jobs, int d, int f, int E, int rank, float* scratch) {
+size_t lay_out(Jobs* jobs, int d, int f, const LoraRun& run, float* scratch) {
   size_t at = 0;
-  jobs->E = E;
+  const int E = jobs->E = run.count;
   for (int l = 0; l < 2; ++l) {
     Linear& L = jobs->lin[l];
     L.out = l == 0 ? 2 * f : d;
     L.in = l == 0 ? d : f;
-    L.rank = rank;
-    L.R = (rank + kRank - 1) / kRank * kRank;
+    L.rank = run.rank[l];
+    L.R = (L.rank + kRank - 1) / kRank * kRank;
     L.row_tiles = (L.out + kRowTile - 1) / kRowTile;
     L.ranges = (L.in + kRange - 1) / kRange;
     L.segs = (L.out + kSegRows - 1) / kSegRows;
@@ -259,25 +261,25 @@ size_t lay_out(Jobs* jobs, int d, int f, int E, int rank, float* scratch) {
 
 }  // namespace
 
-size_t lora_grads_scratch_floats(int d, int f, int E, int rank) {
+size_t lora_grads_scratch_floats(int d, int f, const LoraRun& run) {
   Jobs jobs = {};
-  return lay_out(&jobs, d, f, E, rank, nullptr);
+  return lay_out(&jobs, d, f, run, nullptr);
 }
 
-int launch_lora_grads(const void* const* tab, int d, int f, int E, int rank, float scale, float* scratch,
-                      const void* const (&G)[2], const void* const (&g)[2], void* const (&dA)[2], void* const (&da)[2],
-                      void* const (&dB)[2], void* const (&db)[2], cudaStream_t s) {
+int launch_lora_grads(const void* const* tab, int d, int f, int all, const LoraRun& run, float* scratch,
+                      const void* const (&G)[2], const void* const (&g)[2], cudaStream_t s) {
   Jobs jobs = {};
-  lay_out(&jobs, d, f, E, rank, scratch);
+  lay_out(&jobs, d, f, run, scratch);
+  const int E = run.count;
   for (int l = 0; l < 2; ++l) {
     Linear& L = jobs.lin[l];
-    L.tab = tab + (size_t)l * E * 3;
-    L.G = static_cast<const __nv_bfloat16*>(G[l]);
-    L.g = static_cast<const __nv_bfloat16*>(g[l]);
-    L.dA = static_cast<__nv_bfloat16*>(dA[l]);
-    L.da = static_cast<__nv_bfloat16*>(da[l]);
-    L.dB = static_cast<__nv_bfloat16*>(dB[l]);
-    L.db = static_cast<__nv_bfloat16*>(db[l]);
+    L.tab = tab + ((size_t)l * all + run.first) * 3;
+    L.G = static_cast<const __nv_bfloat16*>(G[l]) + (size_t)run.first * L.out * L.in;
+    L.g = static_cast<const __nv_bfloat16*>(g[l]) + (size_t)run.first * L.out;
+    L.dA = static_cast<__nv_bfloat16*>(run.dA[l]);
+    L.da = static_cast<__nv_bfloat16*>(run.da[l]);
+    L.dB = static_cast<__nv_bfloat16*>(run.dB[l]);
+    L.db = static_cast<__nv_bfloat16*>(run.db[l]);
   }
   const Linear &a = jobs.lin[0], &b = jobs.lin[1];
   const unsigned steps = (unsigned)((a.R > b.R ? a.R : b.R) / kRank);
@@ -289,8 +291,9 @@ int launch_lora_grads(const void* const* tab, int d, int f, int E, int rank, flo
   jobs.first[1] = jobs.first[0] + (unsigned)(b.segs * b.col_tiles * E);
   lora_cols_kernel<<<dim3(jobs.first[1], steps), 256, 0, s>>>(jobs);
   MOE_CUDA_CHECK(cudaGetLastError());
-  const int64_t widest = (int64_t)(2 * f > d ? 2 * f : d) * rank;
-  lora_finish_kernel<<<dim3((unsigned)((widest + 255) / 256), 4, (unsigned)E), 256, 0, s>>>(jobs, scale);
+  int64_t widest = 0;
+  for (const Linear& L : jobs.lin) widest = std::max(widest, (int64_t)std::max(L.out, L.in) * L.rank);
+  lora_finish_kernel<<<dim3((unsigned)((widest + 255) / 256), 4, (unsigned)E), 256, 0, s>>>(jobs, run.scale);
   MOE_CUDA_CHECK(cudaGetLastError());
   return 0;
 }

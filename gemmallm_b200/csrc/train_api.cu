@@ -101,8 +101,11 @@ int experts_backward(const void* perm, const void* h, const int32_t* offsets, co
   if (!g.w1 || !g.b1 || !g.w2 || !g.b2) return set_error(MOE_B200_ERR_NULL, "LoRA gradients need those of the merged weights");
   const void* const G[2] = {g.w1, g.w2};
   const void* const gb[2] = {g.b1, g.b2};
-  return launch_lora_grads(lora->tab, d, f, E, lora->rank, lora->scale, lora->scratch, G, gb, lora->dA, lora->da, lora->dB,
-                           lora->db, s);
+  for (const LoraRun& run : lora->runs) {
+    rc = launch_lora_grads(lora->tab, d, f, E, run, lora->scratch, G, gb, s);
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 // the gradient regions of the training workspace

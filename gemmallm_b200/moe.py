@@ -37,11 +37,13 @@ _LORA_NAMES = ("gate_and_up", "down", "lora_gate_and_up_a", "lora_gate_and_up_b"
 
 def _expert_watch(ex, fine_tuning: bool) -> list:
     """(dictionary, key) of everything in an expert's module tree that a prepared call uses: the
-    Linears, then weight and bias of each in the order of _LORA_NAMES."""
+    Linears, weight and bias of each in the order of _LORA_NAMES, and the scale of the LoRA branches."""
     names = _LORA_NAMES if fine_tuning else _LORA_NAMES[:2]
     watch = [(ex._modules, n) for n in names]
     for n in names:
         watch += [(getattr(ex, n)._parameters, "weight"), (getattr(ex, n)._parameters, "bias")]
+    if fine_tuning:
+        watch.append((ex.__dict__, "lora_scale"))
     return watch
 
 
@@ -103,6 +105,10 @@ def _lora_table(experts, dev) -> torch.Tensor:
             for pair in (("lora_gate_and_up_a", "lora_gate_and_up_b"), ("lora_down_a", "lora_down_b"))
             for a, b in ((getattr(ex, pair[0]), getattr(ex, pair[1])) for ex in experts)]
     return torch.tensor(rows, dtype=torch.int64).to(dev)
+
+
+def _lora_ranks(experts) -> list:
+    return [a.out_features for ex in experts for a in (ex.lora_gate_and_up_a, ex.lora_down_a)]
 
 
 def _expert_params(ex, fine_tuning: bool) -> list:
@@ -252,8 +258,7 @@ class FeedForward(nn.Module):
             native.bind(watch if usual else [], *self._bound(fine_tuning), plan, [self._plan_of(fine_tuning).buf],
                         offsets, status, M, d, f, _cabi.BF16, dev.index)
             table = _lora_table([self], dev) if fine_tuning else None
-            native.bind_train(buf, tbase, tbytes, table, self.lora_down_a.out_features if fine_tuning else 0,
-                              float(self.lora_scale), self._generation)
+            native.bind_train(buf, tbase, tbytes, table, _lora_ranks([self]) if fine_tuning else [], self._generation)
             # the tensors themselves, wherever the module tree keeps them
             y, seed = native.train(x, float(self.dropout.p), _expert_params(self, fine_tuning))
         return y.reshape(tensor.shape), seed
@@ -346,7 +351,7 @@ class MOE(nn.Module):
         w, cnt_slot, offsets, psum, row_of, status; after a training forward also its seed."""
         if self._ws is None:
             return None
-        N, E, k = self._ws_key[0], self.num_experts, self.top_k
+        N, _, _, E, k = self._ws_key
         views = {
             "logits": self._view("logits", torch.float32, (N, E)),
             "idx": self._view("idx", torch.int32, (N, k)),
@@ -363,9 +368,9 @@ class MOE(nn.Module):
 
     # -- workspace ---------------------------------------------------------
     def _workspace(self, N: int, dtype: int, device: torch.device):
-        key = (N, dtype, str(device))
+        d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
+        key = (N, dtype, str(device), E, k)
         if key != self._ws_key:
-            d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
             nbytes = _cabi.workspace_bytes(N, d, f, E, k, dtype)
             buf = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
             base = (buf.data_ptr() + 1023) & ~1023
@@ -472,7 +477,7 @@ class MOE(nn.Module):
     def _watch(self, fine_tuning: bool) -> list:
         """Everything in the module tree a prepared call depends on; empty for trees that do not hold
         their parameters under the usual names (those calls are prepared every time)."""
-        watch = [(self._modules, "gate"), (self._modules, "experts"),
+        watch = [(self.__dict__, "top_k"), (self.__dict__, "num_experts"), (self._modules, "gate"), (self._modules, "experts"),
                  (self.gate._parameters, "weight"), (self.gate._parameters, "bias")]
         for name, ex in self.experts._modules.items():
             watch.append((self.experts._modules, name))
@@ -492,9 +497,9 @@ class MOE(nn.Module):
 
     # -- training mode -------------------------------------------------------
     def _train_workspace(self, N: int, device: torch.device):
-        key = (N, str(device))
+        d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
+        key = (N, str(device), E, k)
         if key != self._tws_key:
-            d, f, E, k = self.hidden_size, self.d_ff, self.num_experts, self.top_k
             nbytes = lib.moe_b200_train_workspace_bytes(N, d, f, E, k, _cabi.BF16)
             if nbytes == 0:
                 raise _cabi.MoeB200Error(lib.moe_b200_last_error_string().decode())
@@ -534,9 +539,7 @@ class MOE(nn.Module):
             buf, tbase, tbytes = self._train_workspace(N, dev)
             self._bind(native, fine_tuning, plan, N, dtype, dev)
             table = _lora_table(self.experts, dev) if fine_tuning else None
-            ex = self.experts[0]
-            native.bind_train(buf, tbase, tbytes, table, ex.lora_down_a.out_features if fine_tuning else 0,
-                              float(ex.lora_scale), self._generation)
+            native.bind_train(buf, tbase, tbytes, table, _lora_ranks(self.experts) if fine_tuning else [], self._generation)
             # the tensors themselves, wherever the module tree keeps them
             params = [self.gate.weight, self.gate.bias]
             for ex in self.experts:

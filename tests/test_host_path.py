@@ -73,7 +73,7 @@ def test_a_bound_call_owns_its_buffers(kind, train):
         native = _host.Ffn()
         native.bind(watch, None, [], 0, buffers[:2], buffers[2], buffers[2], 1, D, F, 1, 0)
     if train:
-        native.bind_train(buffers[3], 0, 0, None, 0, 1.0, _host.Generation())
+        native.bind_train(buffers[3], 0, 0, None, [], _host.Generation())
     else:
         del refs[3]
     del buffers
@@ -411,3 +411,69 @@ def test_saved_tensor_hooks_see_what_is_saved(cuda_device):
             assert seen == shapes
             sum((o.float() ** 2).sum() for o in out).backward()
             same([*(o.detach() for o in out), xd.grad, *(p.grad for p in m.parameters() if p.grad is not None)], want)
+
+
+# ---- plain attributes are read by every call -----------------------------------------------------
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_lora_scale_set_between_calls(cuda_device, kind):
+    m, x = build(kind, cuda_device), rows(48, cuda_device)
+    for scale in (2.0, 0.5, 2.0):
+        for ex in (m.experts if kind == "moe" else [m]):
+            ex.lora_scale = scale
+        new = fresh_copy(m, kind, cuda_device)
+        for ex in (new.experts if kind == "moe" else [new]):
+            ex.lora_scale = scale
+        want = train_step(new, x, True)
+        for _ in range(3):
+            same(train_step(m, x, True), want)
+        with torch.no_grad():
+            want = forward(new.eval(), x, True)
+            for _ in range(3):
+                same(forward(m.eval(), x, True), want)
+
+
+@pytest.mark.gpu
+def test_slots_set_between_calls(cuda_device):
+    m, x = build("moe", cuda_device), rows(48, cuda_device)
+    for k in (2, 1, 3, 2):
+        m.top_k = k
+        new = fresh_copy(m, "moe", cuda_device)
+        new.top_k = k
+        want = train_step(new, x)
+        for _ in range(3):
+            same(train_step(m, x), want)
+        with torch.no_grad():
+            want = forward(new.eval(), x)
+            for _ in range(3):
+                same(forward(m.eval(), x), want)
+        assert m.last["idx"].shape == (48, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["ranks", "scales"])
+def test_experts_with_ranks_and_scales_of_their_own(cuda_device, what):
+    """Replaced adapters: every expert's, and each of its Linears', at a rank of its own. The gradients follow from those of
+    the merged weights (one rounding behind fp32 sums)."""
+    torch.manual_seed(0)
+    m, x = build("moe", cuda_device, p=0.0), rows(200, cuda_device)
+    for e, ex in enumerate(m.experts):
+        if what == "scales":
+            ex.lora_scale = 0.5 + e
+            continue
+        ra, rb = (4, 16, 33, 8)[e], (16, 5, 16, 24)[e]
+        ex.lora_gate_and_up_a, ex.lora_gate_and_up_b = torch.nn.Linear(D, ra), torch.nn.Linear(ra, 2 * F)
+        ex.lora_down_a, ex.lora_down_b = torch.nn.Linear(F, rb), torch.nn.Linear(rb, D)
+    m.to(device=cuda_device, dtype=DT)
+    for _ in range(3):
+        train_step(m, x, True)
+        for ex in m.experts:
+            for w, a, b in ((ex.gate_and_up, ex.lora_gate_and_up_a, ex.lora_gate_and_up_b),
+                            (ex.down, ex.lora_down_a, ex.lora_down_b)):
+                G, g, A, av, B = (t.detach().cpu().double() for t in (w.weight.grad, w.bias.grad, a.weight, a.bias, b.weight))
+                s = ex.lora_scale
+                for got, ref in ((a.weight.grad, s * B.t() @ G), (b.weight.grad, s * (G @ A.t() + torch.outer(g, av))),
+                                 (a.bias.grad, s * B.t() @ g), (b.bias.grad, s * g)):
+                    ref = ref.to(DT).double()
+                    assert (got.cpu().double() - ref).norm() <= 1e-3 * ref.norm()
