@@ -44,6 +44,7 @@ PyObject* s_weight = nullptr;
 PyObject* s_bias = nullptr;
 PyObject* s_parameters = nullptr;
 PyObject* s_eps = nullptr;
+PyObject* s_normalized_shape = nullptr;
 
 PyObject* fail(int rc, const char* what) {
   if (g_error == nullptr) {
@@ -658,8 +659,15 @@ struct Block {
   int d, f, E, k, dtype, device;
 };
 
-// The caller's LayerNorm: false when it is not an affine one over d elements of the call's dtype.
+// The caller's LayerNorm: false when it is not an affine one over d elements of the call's dtype. (normalized_shape is
+// what tells it from other norms with d weights, which would be taken for one otherwise.)
 bool read_norm(PyObject* norm, int d, int dtype, int device, const void** w, const void** b, double* eps) {
+  PyObject* shape = PyObject_GetAttr(norm, s_normalized_shape);
+  if (shape == nullptr) return false;
+  const bool over_d = PyTuple_Check(shape) && PyTuple_GET_SIZE(shape) == 1 && PyLong_Check(PyTuple_GET_ITEM(shape, 0)) &&
+                      PyLong_AsLong(PyTuple_GET_ITEM(shape, 0)) == d;
+  Py_DECREF(shape);
+  if (!over_d) return false;
   PyObject* dict = PyObject_GetAttr(norm, s_parameters);
   if (dict == nullptr) return false;
   bool ok = false;
@@ -1236,6 +1244,7 @@ PyMODINIT_FUNC PyInit__host(void) {
   s_bias = PyUnicode_InternFromString("bias");
   s_parameters = PyUnicode_InternFromString("_parameters");
   s_eps = PyUnicode_InternFromString("eps");
+  s_normalized_shape = PyUnicode_InternFromString("normalized_shape");
   if (!add_type(m, "Block", &block_spec) || !add_type(m, "Ffn", &ffn_spec) ||
       !add_type(m, "Generation", &generation_spec, &g_generation_type) ||
       !add_type(m, "Merged", &merged_spec, &g_merged_type)) {

@@ -477,3 +477,19 @@ def test_experts_with_ranks_and_scales_of_their_own(cuda_device, what):
                                  (a.bias.grad, s * B.t() @ g), (b.bias.grad, s * g)):
                     ref = ref.to(DT).double()
                     assert (got.cpu().double() - ref).norm() <= 1e-3 * ref.norm()
+
+
+@pytest.mark.gpu
+def test_only_a_layernorm_is_folded_in(cuda_device):
+    """Norms with as many weights that are none, on a call that is bound for a LayerNorm."""
+    m, x = build("moe", cuda_device).eval(), rows(48, cuda_device)
+    put = lambda norm: norm.to(device=cuda_device, dtype=DT)
+    ln = put(torch.nn.LayerNorm(D))
+    with torch.no_grad():
+        want = fresh_copy(m, "moe", cuda_device).eval()(x, norm=ln)
+        for _ in range(3):
+            same(m(x, norm=ln), want)
+            for norm in (torch.nn.GroupNorm(8, D), torch.nn.BatchNorm1d(D), torch.nn.LayerNorm((48, D)),
+                         torch.nn.LayerNorm(D, elementwise_affine=False), torch.nn.LayerNorm(D, bias=False)):
+                with pytest.raises((ValueError, AttributeError)):
+                    m(x, norm=put(norm))
