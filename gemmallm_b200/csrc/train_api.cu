@@ -331,14 +331,27 @@ int experts_backward_into(const void* x_sorted, const void* h, const int32_t* of
   if (M == 0) return 0;
   if (!x_sorted || !h || !offsets || !plan || !grad_y || !train_ws || !status)
     return set_error(MOE_B200_ERR_NULL, "NULL argument");
-  if (!aligned16(x_sorted) || !aligned16(h) || !aligned16(grad_y) || !aligned16(grads.x))
-    return set_error(MOE_B200_ERR_ALIGN, "buffers must be 16-byte aligned");
+  if (!aligned16(x_sorted) || !aligned16(h)) return set_error(MOE_B200_ERR_ALIGN, "x and h must be 16-byte aligned");
   size_t to[MOE_B200_TWS_NUM], ttotal;
   tws_layout(M, d, f, E, 1, to, &ttotal);
   if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
-  const TrainArgs tr = train_args(static_cast<char*>(train_ws), to, dropout_p, seed);
-  return experts_backward(x_sorted, h, offsets, plan, grad_y, M, d, f, E, tr, grads, lora, status,
-                          (cudaStream_t)stream);
+  char* tws = static_cast<char*>(train_ws);
+  cudaStream_t s = (cudaStream_t)stream;
+  const TrainArgs tr = train_args(tws, to, dropout_p, seed);
+  // gradients come as they come (a slice of a concatenation starts anywhere): those that TMA and 16-byte accesses cannot
+  // take go through the workspace
+  const size_t bytes = (size_t)M * d * 2;
+  const void* dy = grad_y;
+  if (!aligned16(grad_y)) {
+    MOE_CUDA_CHECK(cudaMemcpyAsync(tws + to[MOE_B200_TWS_DY], grad_y, bytes, cudaMemcpyDeviceToDevice, s));
+    dy = tws + to[MOE_B200_TWS_DY];
+  }
+  TrainGrads eg = grads;
+  if (!aligned16(grads.x)) eg.x = tws + to[MOE_B200_TWS_DXS];
+  rc = experts_backward(x_sorted, h, offsets, plan, dy, M, d, f, E, tr, eg, lora, status, s);
+  if (rc) return rc;
+  if (eg.x != grads.x) MOE_CUDA_CHECK(cudaMemcpyAsync(grads.x, eg.x, bytes, cudaMemcpyDeviceToDevice, s));
+  return 0;
 }
 
 }  // namespace moe

@@ -493,3 +493,27 @@ def test_only_a_layernorm_is_folded_in(cuda_device):
                          torch.nn.LayerNorm(D, elementwise_affine=False), torch.nn.LayerNorm(D, bias=False)):
                 with pytest.raises((ValueError, AttributeError)):
                     m(x, norm=put(norm))
+
+
+@pytest.mark.gpu
+def test_output_gradients_at_any_address(cuda_device):
+    """A gradient that starts two bytes behind a 16-byte boundary, as a slice of a concatenation does: the feed-forward
+    takes it, the block refuses it."""
+    x = rows(48, cuda_device)
+    g = torch.randn(48, D, generator=torch.Generator().manual_seed(4)).to(DT).to(cuda_device)
+    shifted = torch.zeros(48 * D + 8, dtype=DT, device=cuda_device)[1:1 + 48 * D].view(48, D)
+    shifted.copy_(g)
+    for kind in KINDS:
+        m, got = build(kind, cuda_device, p=0.0).train(), []
+        for grad in (g, shifted):
+            xd = x.clone().requires_grad_(True)
+            out = forward(m, xd)[0]
+            if kind == "moe" and grad is shifted:
+                with pytest.raises(RuntimeError):
+                    out.backward(grad)
+                continue
+            m.zero_grad(set_to_none=True)
+            out.backward(grad)
+            got.append([xd.grad, *(p.grad for p in m.parameters() if p.grad is not None)])
+        if kind == "ffn":
+            same(*got)
