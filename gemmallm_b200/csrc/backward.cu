@@ -300,8 +300,8 @@ __global__ void iota_kernel(int32_t* __restrict__ p, int64_t n) {
   if (i < n) p[i] = (int32_t)i;
 }
 
-// Partial column sums: one block per 256-row tile of an expert (tiles counted over the experts in
-// order, as the grouped products count them) and 64 columns; eight threads cover a row's 128 bytes,
+// Partial column sums: one block per 256-row tile of an expert (blockIdx.x, which alone counts beyond 65535: tiles over
+// the experts in order, as the grouped products count them) and 64 columns (blockIdx.y); eight threads cover a row's 128 bytes,
 // 32 such groups take every 32nd row, eight loads in flight each.
 __global__ void __launch_bounds__(256)
 colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ offsets, int E, int C,
@@ -309,7 +309,7 @@ colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__
   __shared__ float s_part[32][65];
   __shared__ int s_row0, s_row1;
   if (threadIdx.x == 0) {
-    int tile = blockIdx.y, r0 = 0, r1 = 0;
+    int tile = blockIdx.x, r0 = 0, r1 = 0;
     for (int e = 0; e < E; ++e) {
       const int beg = offsets[e], end = offsets[e + 1], tiles = (end - beg + 255) / 256;
       if (tile < tiles) {
@@ -326,7 +326,7 @@ colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__
   const int r0 = s_row0, r1 = s_row1;
   if (r0 == r1) return;      // behind the last tile
   const int pc = threadIdx.x & 7, lane_r = threadIdx.x >> 3;
-  const int c = blockIdx.x * 64 + pc * 8;
+  const int c = blockIdx.y * 64 + pc * 8;
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -351,12 +351,12 @@ colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__
   for (int i = 0; i < 8; ++i) s_part[lane_r][pc * 8 + i] = acc[i];
   __syncthreads();
   if (threadIdx.x < 64) {
-    const int col = blockIdx.x * 64 + threadIdx.x;
+    const int col = blockIdx.y * 64 + threadIdx.x;
     if (col < C) {
       float sum = 0.f;
 #pragma unroll
       for (int q = 0; q < 32; ++q) sum += s_part[q][threadIdx.x];
-      part[(size_t)blockIdx.y * C + col] = sum;
+      part[(size_t)blockIdx.x * C + col] = sum;
     }
   }
 }
@@ -479,7 +479,7 @@ int launch_colsum_finish(const float* part, int slots, const int32_t* offsets, i
 int launch_colsum(const void* src, const int32_t* offsets, int64_t M, int E, int C, float* part, void* db,
                   cudaStream_t s) {
   const unsigned tiles = blocks_for(M, 256) + (unsigned)E;    // at least as many as there are
-  colsum_kernel<<<dim3((C + 63) / 64, tiles), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(src), offsets, E, C,
+  colsum_kernel<<<dim3(tiles, (C + 63) / 64), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(src), offsets, E, C,
                                                             part);
   MOE_CUDA_CHECK(cudaGetLastError());
   return launch_colsum_finish(part, 1, offsets, E, C, db, s);

@@ -390,3 +390,20 @@ def test_lora_step_keeps_its_rounding_points(cuda_device, rows, d, f, rank):
         assert off(la.bias.grad, bf(s * B.t() @ gb)) <= 1e-3        # a few values: one at a boundary counts more
         assert off(lb.weight.grad, bf(s * (G @ A.t() + torch.outer(gb, a)))) <= 5e-4
         assert off(lb.bias.grad, bf(s * gb)) == 0.0
+
+
+@pytest.mark.gpu
+def test_bias_gradients_of_more_row_tiles_than_a_grid_dimension(cuda_device):
+    """65536 tiles of 256 rows: tiles lie along the grid dimension that goes beyond 65535. Rows of ones and a gradient that is
+    one in the last row alone (the other rows' sums are zero and exact)."""
+    from gemmallm_b200 import FeedForward
+    rows, d, f = 65535 * 256 + 1, 8, 8
+    torch.manual_seed(0)
+    ff = FeedForward(d, dropout_ratio=0.0, d_ff=f).to(device=cuda_device, dtype=DT).train()
+    x = torch.ones(rows, d, dtype=DT, device=cuda_device).requires_grad_(True)
+    y = ff(x)
+    grad = torch.zeros_like(y)
+    grad[-1] = 1.0
+    y.backward(grad)
+    assert torch.equal(ff.down.bias.grad, torch.ones_like(ff.down.bias))
+    assert (x.grad[:-1] == 0).all() and (x.grad[-1] != 0).any() and (ff.gate_and_up.bias.grad != 0).any()
