@@ -479,9 +479,8 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   const bool tiles = rows_path && tiles_at_row_counts(N * k, d, E);
   const bool counters = small_n || rows_path;
   // status words, and the completion counters behind them where a kernel uses them, in one memset
-  // (a caller that keeps the region clean needs none at any size: kernels write the status words
-  // only when something failed)
-  if (!(flags & MOE_B200_FLAG_WS_CLEAN))
+  // (above these sizes a call always clears the status words: they are those of the most recent call)
+  if (!(counters && (flags & MOE_B200_FLAG_WS_CLEAN)))
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
   const bool front = (small_n || rows_path) &&

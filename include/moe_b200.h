@@ -62,8 +62,8 @@ enum {
    * (MOE_B200_WS_STATUS, status words and counters) is all zero on entry: it was
    * zeroed once, and every call on this workspace since then has ended with
    * device status 0 (such calls leave the region zero). Saves the memset in
-   * front of the first kernel, which, for calls of up to 4096 rows, then overlaps
-   * the tail of the kernel before it. After a non-zero device status the region
+   * front of the first kernel of calls of up to 4096 rows, which then overlaps
+   * the tail of the kernel before it; larger calls clear the status words anyway. After a non-zero device status the region
    * has to be zeroed again by the caller. */
   MOE_B200_FLAG_WS_CLEAN = 1
 };

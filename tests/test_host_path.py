@@ -517,3 +517,22 @@ def test_output_gradients_at_any_address(cuda_device):
             got.append([xd.grad, *(p.grad for p in m.parameters() if p.grad is not None)])
         if kind == "ffn":
             same(*got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_device_status_is_that_of_the_last_large_call(cuda_device, dtype):
+    """An error that nobody asked for does not stay with the calls after it."""
+    m = build("moe", cuda_device).to(dtype).eval()
+    good = torch.randn(3000, D, generator=torch.Generator().manual_seed(1)).to(device=cuda_device, dtype=dtype)
+    bad = good.clone()
+    bad[7] = float("nan")
+    with torch.no_grad():
+        for _ in range(2):
+            m(good)
+            assert m.device_status() == 0
+            m(bad)
+            m(good)
+            assert m.device_status() == 0
+            m(bad)
+            assert m.device_status() != 0
