@@ -396,10 +396,15 @@ uint64_t draw_seed() {      // torch's CPU generator, as torch.randint(0, 2**62,
   return (uint64_t)at::randint((int64_t)1 << 62, {1}, at::TensorOptions().dtype(at::kLong)).item<int64_t>();
 }
 
+// From a backward pass, on a thread that does not hold the GIL: the same MoeB200Error.
 void check_rc(int rc, const char* what) {
-  if (rc != 0)
-    throw std::runtime_error(std::string(what) + " failed with code " + std::to_string(rc) + ": " +
-                             moe_b200_last_error_string());
+  if (rc == 0) return;
+  const PyGILState_STATE gil = PyGILState_Ensure();
+  python_error e;
+  fail(rc, what);
+  e.persist();
+  PyGILState_Release(gil);
+  throw e;
 }
 
 // Gradients of the experts' parameters: per expert w1, b1, w2, b2 and, with LoRA, weight and bias of

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from gemmallm_b200 import MOE, FeedForward, _host
+from gemmallm_b200._cabi import MoeB200Error
 
 DT = torch.bfloat16
 D, F, E, RANK = 64, 128, 4, 16
@@ -509,7 +510,7 @@ def test_output_gradients_at_any_address(cuda_device):
             xd = x.clone().requires_grad_(True)
             out = forward(m, xd)[0]
             if kind == "moe" and grad is shifted:
-                with pytest.raises(RuntimeError):
+                with pytest.raises(MoeB200Error, match="backward failed with code -3: buffers must be 16-byte aligned"):
                     out.backward(grad)
                 continue
             m.zero_grad(set_to_none=True)
