@@ -171,7 +171,29 @@ class _TracedFfn(torch.autograd.Function):
         return (None, gx, None, *gp)
 
 
-class FeedForward(nn.Module):
+class _Calls(nn.Module):
+    """A module with state that belongs to its calls (plans, workspaces, bound calls: addresses of this object's own
+    tensors). A copy of the module, by copy, pickle or replication, starts without any."""
+
+    _CALL_STATE: tuple = ()
+
+    def _reset_calls(self) -> None:
+        raise NotImplementedError
+
+    def __getstate__(self):
+        return {n: v for n, v in self.__dict__.items() if n not in self._CALL_STATE}
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        self._reset_calls()
+
+    def _replicate_for_data_parallel(self):
+        replica = super()._replicate_for_data_parallel()
+        replica._reset_calls()
+        return replica
+
+
+class FeedForward(_Calls):
     """GeGLU feed-forward expert; mirrors reference model.py:154-190.
 
     ``gate_and_up`` maps d -> 2f (rows [0,f) gate, rows [f,2f) up), ``down`` maps
@@ -194,6 +216,13 @@ class FeedForward(nn.Module):
         self.lora_gate_and_up_b = nn.Linear(lora_rank, f * 2)
         self.lora_down_a = nn.Linear(f, lora_rank)
         self.lora_down_b = nn.Linear(lora_rank, hidden_size)
+        self.last_seed = None
+        self._reset_calls()
+
+    _CALL_STATE = ("_plan", "_plan_ft", "_lora", "_native", "_native_ft", "_native_train", "_native_train_ft", "_offsets",
+                   "_tws", "_tws_key", "_generation")
+
+    def _reset_calls(self) -> None:
         self._plan = _Plan()
         self._plan_ft = _Plan()
         self._lora = _MergedLora()
@@ -204,7 +233,6 @@ class FeedForward(nn.Module):
         self._tws = None
         self._tws_key = None
         self._generation = None   # counts the forwards on _tws
-        self.last_seed = None
 
     def _rows(self, tensor):
         x = tensor.reshape(-1, tensor.shape[-1]).contiguous()
@@ -310,7 +338,7 @@ class FeedForward(nn.Module):
         return y.reshape(shape)
 
 
-class MOE(nn.Module):
+class MOE(_Calls):
     """Mixture-of-experts feed-forward block; mirrors reference model.py:192-276.
 
     Same positional/keyword arguments as the reference constructor
@@ -332,6 +360,12 @@ class MOE(nn.Module):
         self.hidden_size = hidden_size
         self.d_ff = self.experts[0].d_ff
         self.top_k = top_k
+        self._reset_calls()
+
+    _CALL_STATE = ("_plan", "_plan_ft", "_lora", "_native", "_native_ft", "_native_train", "_native_train_ft", "_ws",
+                   "_ws_key", "_tws", "_tws_key", "_generation", "_last_seed")
+
+    def _reset_calls(self) -> None:
         self._plan = _Plan()
         self._plan_ft = _Plan()
         self._lora = _MergedLora()

@@ -537,3 +537,40 @@ def test_device_status_is_that_of_the_last_large_call(cuda_device, dtype):
             assert m.device_status() == 0
             m(bad)
             assert m.device_status() != 0
+
+
+# ---- copies ----------------------------------------------------------------------------------------
+
+def test_copies_hold_no_state_of_calls():
+    import copy
+    import pickle
+    for kind in KINDS:
+        m = MOE(D, num_experts=E, d_ff=F) if kind == "moe" else FeedForward(D, d_ff=F)
+        m._tws, m._tws_key = (torch.zeros(4), 4711, 16), (48, "cpu")
+        for new in (copy.deepcopy(m), copy.copy(m), pickle.loads(pickle.dumps(m))):
+            assert new._tws is None and new._tws_key is None and new._native is not m._native and new._plan is not m._plan
+            assert all(torch.equal(a, b) for a, b in zip(new.state_dict().values(), m.state_dict().values()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fine_tuning", [False, True])
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_copy_of_a_module_that_ran(cuda_device, kind, fine_tuning):
+    """Forwards and backwards of the module and its copy in turn: each has its own workspaces."""
+    import copy
+    m, x, z = build(kind, cuda_device), rows(48, cuda_device, 1), rows(48, cuda_device, 2)
+    want = [train_step(fresh_copy(m, kind, cuda_device), t, fine_tuning) for t in (x, z)]
+    for _ in range(2):
+        train_step(m, x, fine_tuning)
+    new = copy.deepcopy(m)
+    for _ in range(3):
+        outs, xs = [], []
+        for module, t in ((m, x), (new, z)):
+            for p in module.parameters():
+                p.grad = None
+            xs.append(t.clone().requires_grad_(True))
+            torch.manual_seed(5)
+            outs.append(forward(module.train(), xs[-1], fine_tuning))
+        for module, out, xd, ref in zip((m, new), outs, xs, want):
+            sum((o.float() ** 2).sum() for o in out).backward()
+            same([*(o.detach() for o in out), xd.grad, *(p.grad for p in module.parameters() if p.grad is not None)], ref)
