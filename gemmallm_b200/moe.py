@@ -171,6 +171,22 @@ class _TracedFfn(torch.autograd.Function):
         return (None, gx, None, *gp)
 
 
+class _Asked:
+    """How often the last call, plain and with LoRA branches, has had to be prepared. Binding a call to the native path
+    costs about as much as it saves one call, so it is done the second, fourth, eighth ... time: not for a size seen once
+    (generation without a cache has another length with every token), and seldom for calls that find the
+    binding unusable."""
+
+    def __init__(self):
+        self.last = {}
+
+    def bind_now(self, fine_tuning: bool, key) -> bool:
+        was, count = self.last.get(fine_tuning, (None, 0))
+        count = count + 1 if was == key else 1
+        self.last[fine_tuning] = (key, count)
+        return count > 1 and count & (count - 1) == 0
+
+
 class _Calls(nn.Module):
     """A module with state that belongs to its calls (plans, workspaces, bound calls: addresses of this object's own
     tensors). A copy of the module, by copy, pickle or replication, starts without any."""
@@ -219,10 +235,11 @@ class FeedForward(_Calls):
         self.last_seed = None
         self._reset_calls()
 
-    _CALL_STATE = ("_plan", "_plan_ft", "_lora", "_native", "_native_ft", "_native_train", "_native_train_ft", "_offsets",
-                   "_tws", "_tws_key", "_generation")
+    _CALL_STATE = ("_calls", "_plan", "_plan_ft", "_lora", "_native", "_native_ft", "_native_train", "_native_train_ft",
+                   "_offsets", "_tws", "_tws_key", "_generation")
 
     def _reset_calls(self) -> None:
+        self._calls = _Asked()
         self._plan = _Plan()
         self._plan_ft = _Plan()
         self._lora = _MergedLora()
@@ -273,6 +290,10 @@ class FeedForward(_Calls):
         if tensor.shape[-1] != d:
             raise ValueError(f"last dimension {tensor.shape[-1]} != hidden_size {d}")
         x, M, dev, offsets = self._rows(tensor)
+        if not tensor.is_contiguous():
+            done = native.train(x, self.dropout.p, None)
+            if done is not None:
+                return done[0].reshape(tensor.shape), done[1]
         with torch.cuda.device(dev):
             if fine_tuning:
                 plan = self._plan_ft.get(self._lora.get([self], _cabi.BF16, dev), d, f, _cabi.BF16, dev)
@@ -321,6 +342,10 @@ class FeedForward(_Calls):
         shape = tensor.shape
         x, M, dev, offsets = self._rows(tensor)
         d, f = self.hidden_size, self.d_ff
+        if not tensor.is_contiguous():
+            y = native.forward(x)          # bound for these rows, contiguous
+            if y is not None:
+                return y.reshape(shape)
         with torch.cuda.device(dev):
             plan = (self._plan_ft if fine_tuning else self._plan).get(
                 self._lora.get([self], dtype, dev) if fine_tuning else [self], d, f, dtype, dev)
@@ -330,6 +355,8 @@ class FeedForward(_Calls):
             check(lib.moe_b200_experts(x.data_ptr(), offsets.data_ptr(), plan, M, d, f, 1, dtype, 0,
                                        h.data_ptr(), y.data_ptr(), status.data_ptr(), _stream(dev)),
                   "experts")
+        if not self._calls.bind_now(fine_tuning, (M, dtype, str(dev))):
+            return y.reshape(shape)
         native.unbind()
         watch = _expert_watch(self, fine_tuning)
         if x.shape[-1] == d and all(name in table for table, name in watch):
@@ -362,10 +389,11 @@ class MOE(_Calls):
         self.top_k = top_k
         self._reset_calls()
 
-    _CALL_STATE = ("_plan", "_plan_ft", "_lora", "_native", "_native_ft", "_native_train", "_native_train_ft", "_ws",
-                   "_ws_key", "_tws", "_tws_key", "_generation", "_last_seed")
+    _CALL_STATE = ("_calls", "_plan", "_plan_ft", "_lora", "_native", "_native_ft", "_native_train", "_native_train_ft",
+                   "_ws", "_ws_key", "_tws", "_tws_key", "_generation", "_last_seed")
 
     def _reset_calls(self) -> None:
+        self._calls = _Asked()
         self._plan = _Plan()
         self._plan_ft = _Plan()
         self._lora = _MergedLora()
@@ -478,6 +506,7 @@ class MOE(_Calls):
         N = x.shape[0]
         dev = x.device
         res_ptr = None
+        as_it_lies = tensor.is_contiguous() and (residual is None or residual.is_contiguous())
         if residual is not None:
             if residual.shape != shape or residual.dtype != tensor.dtype or residual.device != dev:
                 raise ValueError("residual must match the input's shape, dtype and device")
@@ -486,6 +515,10 @@ class MOE(_Calls):
         gw, gb = self.gate.weight, self.gate.bias
         if gw.device != dev or _dtype_code(gw) != dtype:
             raise ValueError("gate parameters must share the input's device and dtype")
+        if not as_it_lies:
+            done = native.forward(x, residual, norm)      # bound for these rows, contiguous
+            if done is not None:
+                return done[0].reshape(shape), done[1]
         nw = nb = None
         eps = 0.0
         if norm is not None:
@@ -505,7 +538,8 @@ class MOE(_Calls):
                                        nw, nb, eps, N, d, f, E, k, dtype, _cabi.FLAG_WS_CLEAN, base, nbytes,
                                        out.data_ptr(), _stream(dev)), "forward")
         aux = self._view("aux", torch.float32, (1,))[0].clone()
-        self._bind(native, fine_tuning, plan, N, dtype, dev)
+        if self._calls.bind_now(fine_tuning, (N, dtype, str(dev))):
+            self._bind(native, fine_tuning, plan, N, dtype, dev)
         return out.reshape(shape), aux
 
     def _watch(self, fine_tuning: bool) -> list:
@@ -560,10 +594,15 @@ class MOE(_Calls):
         x = tensor.reshape(-1, d).contiguous()
         N = x.shape[0]
         dev = x.device
+        as_it_lies = tensor.is_contiguous() and (residual is None or residual.is_contiguous())
         if residual is not None:
             if residual.shape != shape or residual.dtype != tensor.dtype or residual.device != dev:
                 raise ValueError("residual must match the input's shape, dtype and device")
             residual = residual.reshape(-1, d).contiguous()
+        if not as_it_lies:
+            done = native.train(x, residual, self.experts[0].dropout.p, None)
+            if done is not None:
+                return done[0].reshape(shape), done[1], done[2]
         with torch.cuda.device(dev):
             if fine_tuning:
                 plan = self._plan_ft.get(self._lora.get(list(self.experts), dtype, dev), d, f, dtype, dev)

@@ -574,3 +574,50 @@ def test_a_copy_of_a_module_that_ran(cuda_device, kind, fine_tuning):
         for module, out, xd, ref in zip((m, new), outs, xs, want):
             sum((o.float() ** 2).sum() for o in out).backward()
             same([*(o.detach() for o in out), xd.grad, *(p.grad for p in module.parameters() if p.grad is not None)], ref)
+
+
+# ---- what is bound, and when ------------------------------------------------------------------------
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_a_call_is_bound_when_it_comes_again(cuda_device, kind):
+    m = build(kind, cuda_device).eval()
+    bound = lambda x: (m._native.forward(x, None, None) if kind == "moe" else m._native.forward(x)) is not None
+    with torch.no_grad():
+        for n in (1, 2, 3, 48, 4):
+            x = rows(n, cuda_device)
+            same(forward(m, x), forward(fresh_copy(m, kind, cuda_device).eval(), x))
+            assert not bound(x)
+        forward(m, x)
+        assert bound(x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_inputs_that_are_not_contiguous_take_the_bound_call(cuda_device, kind):
+    m, x = build(kind, cuda_device), rows(48, cuda_device)
+    z = other_layout(x)
+    assert not z.is_contiguous()
+    want = train_step(fresh_copy(m, kind, cuda_device), x)
+    train_step(m, z)
+    prepare = m._plan.get
+    m._plan.get = None           # from here on nothing is prepared
+    for _ in range(2):
+        xd = z.detach().requires_grad_(True)
+        for p in m.parameters():
+            p.grad = None
+        torch.manual_seed(5)
+        out = forward(m.train(), xd)
+        sum((o.float() ** 2).sum() for o in out).backward()
+        same([*(o.detach() for o in out), xd.grad, *(p.grad for p in m.parameters() if p.grad is not None)], want)
+    m._plan.get = prepare
+    with torch.no_grad():
+        want = forward(fresh_copy(m, kind, cuda_device).eval(), x)
+        for _ in range(2):
+            same(forward(m.eval(), z), want)
+        m._plan.get = None
+        for _ in range(2):
+            same(forward(m, z), want)
+            if kind == "moe":
+                same(forward(m, z, residual=z), forward(m, x, residual=x))
+                same(forward(m, x, residual=z), forward(m, x, residual=x))
