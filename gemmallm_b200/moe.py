@@ -411,7 +411,7 @@ class MOE(_Calls):
     def last(self) -> dict | None:
         """Views into the workspace of the most recent call (None before the first): logits, idx,
         w, cnt_slot, offsets, psum, row_of, status; after a training forward also its seed."""
-        if self._ws is None:
+        if self._ws is None or self._last_seed is False:
             return None
         N, _, _, E, k = self._ws_key
         views = {
@@ -427,6 +427,12 @@ class MOE(_Calls):
         if self._last_seed is not None:
             views["seed"] = self._last_seed
         return views
+
+    @last.setter
+    def last(self, value) -> None:
+        if value is not None:
+            raise ValueError("last can be cleared, not set")
+        self._last_seed = False       # until the next call
 
     # -- workspace ---------------------------------------------------------
     def _workspace(self, N: int, dtype: int, device: torch.device):
@@ -625,7 +631,7 @@ class MOE(_Calls):
     def device_status(self) -> int:
         """Status word of the most recent call (0 = ok); synchronises. A non-zero status is
         returned once: the status region is zeroed again so that later calls start clean."""
-        if self._ws is None:
+        if self._ws is None or self._last_seed is False:
             return 0
         code = int(self._view("status", torch.int32, (16,))[0].item())
         if code != 0:

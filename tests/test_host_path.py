@@ -621,3 +621,20 @@ def test_inputs_that_are_not_contiguous_take_the_bound_call(cuda_device, kind):
             if kind == "moe":
                 same(forward(m, z, residual=z), forward(m, x, residual=x))
                 same(forward(m, x, residual=z), forward(m, x, residual=x))
+
+
+@pytest.mark.gpu
+def test_the_last_call_can_be_cleared(cuda_device):
+    m, x = build("moe", cuda_device).eval(), rows(48, cuda_device)
+    assert m.last is None
+    for train in (False, True):
+        m.train(train)
+        for _ in range(3):
+            with torch.no_grad():
+                m(x)
+            kept = m.last
+            assert kept["idx"].shape == (48, 2) and ("seed" in kept) == train
+            m.last = None
+            assert m.last is None and m.device_status() == 0
+            with pytest.raises(ValueError):
+                m.last = {}
