@@ -90,9 +90,11 @@ def build_host(force: bool = False, verbose: bool = False) -> Path:
     """The modules' native host path: one C++ file against torch's headers, linked to
     libmoe_b200.so next to it."""
     deps = [HOST_SRC, CSRC / "internal.h", PKG.parent / "include" / "moe_b200.h"]
-    if not force and not _stale(HOST_LIB, deps):
-        return HOST_LIB
     torch_dir = Path(next(iter(importlib.util.find_spec("torch").submodule_search_locations)))
+    # a library built against another torch's headers must not be loaded next to this one, whatever the files' dates
+    stamp, version = OBJ / "host_torch_version", (torch_dir / "version.py").read_text()
+    if not force and not _stale(HOST_LIB, deps) and stamp.exists() and stamp.read_text() == version:
+        return HOST_LIB
     cuda = Path(_nvcc()).resolve().parent.parent
     includes = [torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include",
                 sysconfig.get_paths()["include"], cuda / "include"]
@@ -104,6 +106,8 @@ def build_host(force: bool = False, verbose: bool = False) -> Path:
         sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
     if r.returncode != 0:
         raise RuntimeError("build of _host.so failed")
+    OBJ.mkdir(exist_ok=True)
+    stamp.write_text(version)
     return HOST_LIB
 
 

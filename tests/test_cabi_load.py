@@ -91,3 +91,23 @@ def test_small_and_mid_size_entry_points_check_their_arguments():
     assert tiny(4, 1024, 4096, 33, 2) == -7
     assert tiny(4, 1024, 4096, 8, 2, out=None) == -1
     assert tiny(4, 1024, 4096, 8, 2, x=a + 8) == -3
+
+
+def test_host_extension_is_rebuilt_for_another_torch(tmp_path, monkeypatch):
+    """Same sources, same dates: what counts besides them is the torch it was built against."""
+    from gemmallm_b200 import build
+    calls = []
+
+    def compile_(cmd, **kw):
+        calls.append(cmd)
+        (tmp_path / "_host.so").touch()
+        return type("R", (), {"returncode": 0, "stdout": "", "stderr": ""})()
+    monkeypatch.setattr(build, "OBJ", tmp_path)
+    monkeypatch.setattr(build, "HOST_LIB", tmp_path / "_host.so")
+    monkeypatch.setattr(build.subprocess, "run", compile_)
+    for _ in range(2):
+        build.build_host()
+    assert len(calls) == 1
+    (tmp_path / "host_torch_version").write_text("another")
+    build.build_host()
+    assert len(calls) == 2
