@@ -7,7 +7,9 @@
 // merged LoRA weights) and bind() the result; forward() answers from what is bound, or returns None
 // for every call that differs from it in any way, and the Python side then prepares again.
 // What is bound is found changed by identity: the module tree's own dictionaries must still hold
-// the same submodules, parameters and plain attributes (scales, slots), and every parameter the same storage.
+// the same submodules, parameters and plain attributes (scales of experts), and every parameter the same storage. Plain
+// attributes of the module itself come with the call: a binding that held its module's dictionary would keep the
+// module, and the memory of its weights, until the garbage collector ran.
 //
 // Lifetime: a bound call owns every buffer whose address it has (plan, workspaces, merged weights): the Python side may
 // replace its own, and the parameters may leave and come back (weights exchanged for an evaluation) with the binding
@@ -247,6 +249,8 @@ struct MergedUse {
   std::shared_ptr<Merged> merged;
   std::vector<double> scales;
   size_t first = 0;       // place of the first expert's parameters among the call's
+
+  bool has_scale(double scale) const { return merged == nullptr || scales[0] == scale; }      // of the only expert
 
   int refresh(const WatchList& w, int dtype, void* stream) const {
     if (merged == nullptr) return 0;
@@ -712,7 +716,7 @@ PyObject* block_new(PyTypeObject* type, PyObject*, PyObject*) {
   return reinterpret_cast<PyObject*>(self);
 }
 
-// The watched tree of a module holds the module's own dictionary, and that the binding.
+// (A tree whose parts refer to the module is a cycle through the binding.)
 int block_traverse(PyObject* o, visitproc visit, void* arg) {
   Py_VISIT(Py_TYPE(o));
   const WatchList* w = reinterpret_cast<Block*>(o)->watch;
@@ -820,17 +824,19 @@ bool rows_match(const Tensor& t, int device, int dtype, int d, int64_t n) {
          t.size(-1) == d && t.numel() == n * d && t.is_contiguous();
 }
 
-// forward(tensor, residual or None, norm or None) -> (out, loss), or None: prepare again
+// forward(tensor, residual or None, norm or None, slots) -> (out, loss), or None: prepare again
 PyObject* block_forward(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   Block* self = reinterpret_cast<Block*>(o);
-  if (nargs != 3) {
-    PyErr_SetString(PyExc_TypeError, "forward(tensor, residual, norm)");
+  if (nargs != 4) {
+    PyErr_SetString(PyExc_TypeError, "forward(tensor, residual, norm, slots)");
     return nullptr;
   }
+  const long k = PyLong_AsLong(args[3]);
+  if (k == -1 && PyErr_Occurred()) return nullptr;
   if (self->watch->empty() || !THPVariable_CheckExact(args[0])) Py_RETURN_NONE;    // the result is of the input's class
   const Tensor& x = THPVariable_Unpack(args[0]);
-  if (self->N <= 0 || !rows_match(x, self->device, self->dtype, self->d, self->N)) Py_RETURN_NONE;
+  if (self->N <= 0 || k != self->k || !rows_match(x, self->device, self->dtype, self->d, self->N)) Py_RETURN_NONE;
   const void* res = nullptr;
   if (args[1] != Py_None) {
     if (!THPVariable_Check(args[1])) Py_RETURN_NONE;
@@ -864,21 +870,23 @@ PyObject* block_forward(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// train(tensor, residual or None, dropout p, parameters or None) -> (out, loss, seed), or None: prepare again.
+// train(tensor, residual or None, dropout p, parameters or None, slots) -> (out, loss, seed), or None: prepare again.
 // Without a list the parameters are the watched ones.
 PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   Block* self = reinterpret_cast<Block*>(o);
-  if (nargs != 4) {
-    PyErr_SetString(PyExc_TypeError, "train(tensor, residual, p, parameters)");
+  if (nargs != 5) {
+    PyErr_SetString(PyExc_TypeError, "train(tensor, residual, p, parameters, slots)");
     return nullptr;
   }
+  const long k = PyLong_AsLong(args[4]);
+  if (k == -1 && PyErr_Occurred()) return nullptr;
   if (*self->train == nullptr || !THPVariable_Check(args[0])) Py_RETURN_NONE;
   if (args[3] == Py_None && !THPVariable_CheckExact(args[0])) Py_RETURN_NONE;    // the result is of the input's class
   if (args[3] == Py_None && torch::jit::tracer::isTracing()) Py_RETURN_NONE;
   const std::shared_ptr<TrainCall> c = *self->train;
   const Tensor& x = THPVariable_Unpack(args[0]);
-  if (!rows_match(x, c->device, MOE_B200_BF16, c->d, c->N)) Py_RETURN_NONE;
+  if (k != c->k || !rows_match(x, c->device, MOE_B200_BF16, c->d, c->N)) Py_RETURN_NONE;
   const bool has_res = args[1] != Py_None;
   if (has_res && !THPVariable_Check(args[1])) Py_RETURN_NONE;
   Tensor res;
@@ -1099,20 +1107,22 @@ PyObject* ffn_bind_train(PyObject* o, PyObject* args) {
   END_HANDLE_TH_ERRORS
 }
 
-// train(tensor, dropout p, parameters or None) -> (y, seed), or None: prepare again
+// train(tensor, dropout p, parameters or None, LoRA scale) -> (y, seed), or None: prepare again
 PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   Ffn* self = reinterpret_cast<Ffn*>(o);
-  if (nargs != 3) {
-    PyErr_SetString(PyExc_TypeError, "train(tensor, p, parameters)");
+  if (nargs != 4) {
+    PyErr_SetString(PyExc_TypeError, "train(tensor, p, parameters, scale)");
     return nullptr;
   }
+  const double scale = PyFloat_AsDouble(args[3]);
+  if (PyErr_Occurred()) return nullptr;
   if (*self->train == nullptr || !THPVariable_Check(args[0])) Py_RETURN_NONE;
   // (under a tracer the module takes a way that the tracer sees)
   if (args[2] == Py_None && torch::jit::tracer::isTracing()) Py_RETURN_NONE;
   const std::shared_ptr<TrainCall> c = *self->train;
   const Tensor& x = THPVariable_Unpack(args[0]);
-  if (!rows_match(x, c->device, MOE_B200_BF16, c->d, c->N)) Py_RETURN_NONE;
+  if (!c->lora.has_scale(scale) || !rows_match(x, c->device, MOE_B200_BF16, c->d, c->N)) Py_RETURN_NONE;
   const double p = PyFloat_AsDouble(args[1]);
   if (PyErr_Occurred()) return nullptr;
   Edges edges;
@@ -1171,17 +1181,21 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// forward(tensor) -> y, or None: prepare again
+// forward(tensor, LoRA scale) -> y, or None: prepare again
 PyObject* ffn_forward(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   Ffn* self = reinterpret_cast<Ffn*>(o);
-  if (nargs != 1) {
-    PyErr_SetString(PyExc_TypeError, "forward(tensor)");
+  if (nargs != 2) {
+    PyErr_SetString(PyExc_TypeError, "forward(tensor, scale)");
     return nullptr;
   }
+  const double scale = PyFloat_AsDouble(args[1]);
+  if (PyErr_Occurred()) return nullptr;
   if (self->watch->empty() || self->M <= 0 || !THPVariable_Check(args[0])) Py_RETURN_NONE;
   const Tensor& x = THPVariable_Unpack(args[0]);
-  if (!rows_match(x, self->device, self->dtype, self->d, self->M) || !self->watch->unchanged()) Py_RETURN_NONE;
+  if (!self->lora->has_scale(scale) || !rows_match(x, self->device, self->dtype, self->d, self->M) ||
+      !self->watch->unchanged())
+    Py_RETURN_NONE;
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
   void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream();
   int rc = self->lora->refresh(*self->watch, self->dtype, stream);

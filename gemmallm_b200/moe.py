@@ -37,13 +37,11 @@ _LORA_NAMES = ("gate_and_up", "down", "lora_gate_and_up_a", "lora_gate_and_up_b"
 
 def _expert_watch(ex, fine_tuning: bool) -> list:
     """(dictionary, key) of everything in an expert's module tree that a prepared call uses: the
-    Linears, weight and bias of each in the order of _LORA_NAMES, and the scale of the LoRA branches."""
+    Linears, then weight and bias of each in the order of _LORA_NAMES."""
     names = _LORA_NAMES if fine_tuning else _LORA_NAMES[:2]
     watch = [(ex._modules, n) for n in names]
     for n in names:
         watch += [(getattr(ex, n)._parameters, "weight"), (getattr(ex, n)._parameters, "bias")]
-    if fine_tuning:
-        watch.append((ex.__dict__, "lora_scale"))
     return watch
 
 
@@ -191,13 +189,17 @@ class _Calls(nn.Module):
     """A module with state that belongs to its calls (plans, workspaces, bound calls: addresses of this object's own
     tensors). A copy of the module, by copy, pickle or replication, starts without any."""
 
-    _CALL_STATE: tuple = ()
-
-    def _reset_calls(self) -> None:
+    @staticmethod
+    def _fresh_calls() -> dict:
         raise NotImplementedError
 
+    def _reset_calls(self) -> None:
+        # one update: an nn.Module takes about 2 us to set an attribute, and a block has a hundred of these
+        self.__dict__.update(self._fresh_calls())
+
     def __getstate__(self):
-        return {n: v for n, v in self.__dict__.items() if n not in self._CALL_STATE}
+        drop = self._fresh_calls()
+        return {n: v for n, v in self.__dict__.items() if n not in drop}
 
     def __setstate__(self, state):
         super().__setstate__(state)
@@ -235,21 +237,15 @@ class FeedForward(_Calls):
         self.last_seed = None
         self._reset_calls()
 
-    _CALL_STATE = ("_calls", "_plan", "_plan_ft", "_lora", "_native", "_native_ft", "_native_train", "_native_train_ft",
-                   "_offsets", "_tws", "_tws_key", "_generation")
-
-    def _reset_calls(self) -> None:
-        self._calls = _Asked()
-        self._plan = _Plan()
-        self._plan_ft = _Plan()
-        self._lora = _MergedLora()
-        # native calls prepared for the last number of rows: plain, and with the LoRA branches merged
-        self._native, self._native_ft = _host.Ffn(), _host.Ffn()
-        self._native_train, self._native_train_ft = _host.Ffn(), _host.Ffn()
-        self._offsets = None   # ((rows, device), int32 [0, rows]) of the last call
-        self._tws = None
-        self._tws_key = None
-        self._generation = None   # counts the forwards on _tws
+    @staticmethod
+    def _fresh_calls() -> dict:
+        return dict(
+            _calls=_Asked(), _plan=_Plan(), _plan_ft=_Plan(), _lora=_MergedLora(),
+            # native calls prepared for the last number of rows: plain, and with the LoRA branches merged
+            _native=_host.Ffn(), _native_ft=_host.Ffn(), _native_train=_host.Ffn(), _native_train_ft=_host.Ffn(),
+            _offsets=None,      # ((rows, device), int32 [0, rows]) of the last call
+            _tws=None, _tws_key=None,
+            _generation=None)   # counts the forwards on _tws
 
     def _rows(self, tensor):
         x = tensor.reshape(-1, tensor.shape[-1]).contiguous()
@@ -291,7 +287,7 @@ class FeedForward(_Calls):
             raise ValueError(f"last dimension {tensor.shape[-1]} != hidden_size {d}")
         x, M, dev, offsets = self._rows(tensor)
         if not tensor.is_contiguous():
-            done = native.train(x, self.dropout.p, None)
+            done = native.train(x, self.dropout.p, None, self.lora_scale)
             if done is not None:
                 return done[0].reshape(tensor.shape), done[1]
         with torch.cuda.device(dev):
@@ -309,7 +305,7 @@ class FeedForward(_Calls):
             table = _lora_table([self], dev) if fine_tuning else None
             native.bind_train(buf, tbase, tbytes, table, _lora_ranks([self]) if fine_tuning else [], self._generation)
             # the tensors themselves, wherever the module tree keeps them
-            y, seed = native.train(x, float(self.dropout.p), _expert_params(self, fine_tuning))
+            y, seed = native.train(x, float(self.dropout.p), _expert_params(self, fine_tuning), self.lora_scale)
         return y.reshape(tensor.shape), seed
 
     def forward(self, tensor: torch.Tensor, fine_tuning: bool = False) -> torch.Tensor:
@@ -324,7 +320,7 @@ class FeedForward(_Calls):
             if tensor.dtype != torch.bfloat16:
                 raise NotImplementedError("training mode computes in bfloat16")
             native = self._native_train_ft if fine_tuning else self._native_train
-            done = native.train(tensor, self.dropout.p, None)
+            done = native.train(tensor, self.dropout.p, None, self.lora_scale)
             if done is None and torch.jit.is_tracing():
                 return _TracedFfn.apply(self, tensor, bool(fine_tuning), *_expert_params(self, fine_tuning))
             if done is None:
@@ -332,7 +328,7 @@ class FeedForward(_Calls):
             y, self.last_seed = done
             return y
         native = self._native_ft if fine_tuning else self._native
-        y = native.forward(tensor)
+        y = native.forward(tensor, self.lora_scale)
         return self._forward_prepared(tensor, bool(fine_tuning), native) if y is None else y
 
     def _forward_prepared(self, tensor, fine_tuning: bool, native):
@@ -343,7 +339,7 @@ class FeedForward(_Calls):
         x, M, dev, offsets = self._rows(tensor)
         d, f = self.hidden_size, self.d_ff
         if not tensor.is_contiguous():
-            y = native.forward(x)          # bound for these rows, contiguous
+            y = native.forward(x, self.lora_scale)          # bound for these rows, contiguous
             if y is not None:
                 return y.reshape(shape)
         with torch.cuda.device(dev):
@@ -389,23 +385,14 @@ class MOE(_Calls):
         self.top_k = top_k
         self._reset_calls()
 
-    _CALL_STATE = ("_calls", "_plan", "_plan_ft", "_lora", "_native", "_native_ft", "_native_train", "_native_train_ft",
-                   "_ws", "_ws_key", "_tws", "_tws_key", "_generation", "_last_seed")
-
-    def _reset_calls(self) -> None:
-        self._calls = _Asked()
-        self._plan = _Plan()
-        self._plan_ft = _Plan()
-        self._lora = _MergedLora()
-        self._ws = None
-        self._ws_key = None
-        self._tws = None
-        self._tws_key = None
-        self._generation = None   # counts the forwards on _tws
-        self._last_seed = None
-        # native calls prepared for the last input size: plain, and with the LoRA branches merged
-        self._native, self._native_ft = _host.Block(), _host.Block()
-        self._native_train, self._native_train_ft = _host.Block(), _host.Block()
+    @staticmethod
+    def _fresh_calls() -> dict:
+        return dict(
+            _calls=_Asked(), _plan=_Plan(), _plan_ft=_Plan(), _lora=_MergedLora(), _ws=None, _ws_key=None, _tws=None,
+            _tws_key=None, _generation=None,      # counts the forwards on _tws
+            _last_seed=None,
+            # native calls prepared for the last input size: plain, and with the LoRA branches merged
+            _native=_host.Block(), _native_ft=_host.Block(), _native_train=_host.Block(), _native_train_ft=_host.Block())
 
     @property
     def last(self) -> dict | None:
@@ -486,7 +473,7 @@ class MOE(_Calls):
             if tensor.dtype != torch.bfloat16:
                 raise NotImplementedError("training mode computes in bfloat16")
             native = self._native_train_ft if fine_tuning else self._native_train
-            done = native.train(tensor, residual, self.experts[0].dropout.p, None)
+            done = native.train(tensor, residual, self.experts[0].dropout.p, None, self.top_k)
             if done is None and torch.jit.is_tracing():
                 raise RuntimeError("the block's training forward cannot be traced")
             if done is None:
@@ -495,7 +482,7 @@ class MOE(_Calls):
             return out, aux
         native = self._native_ft if fine_tuning else self._native
         self._last_seed = None
-        done = native.forward(tensor, residual, norm)
+        done = native.forward(tensor, residual, norm, self.top_k)
         if done is None:
             done = self._forward_prepared(tensor, bool(fine_tuning), residual, norm, native)
         return done
@@ -522,7 +509,7 @@ class MOE(_Calls):
         if gw.device != dev or _dtype_code(gw) != dtype:
             raise ValueError("gate parameters must share the input's device and dtype")
         if not as_it_lies:
-            done = native.forward(x, residual, norm)      # bound for these rows, contiguous
+            done = native.forward(x, residual, norm, self.top_k)      # bound for these rows, contiguous
             if done is not None:
                 return done[0].reshape(shape), done[1]
         nw = nb = None
@@ -551,11 +538,13 @@ class MOE(_Calls):
     def _watch(self, fine_tuning: bool) -> list:
         """Everything in the module tree a prepared call depends on; empty for trees that do not hold
         their parameters under the usual names (those calls are prepared every time)."""
-        watch = [(self.__dict__, "top_k"), (self.__dict__, "num_experts"), (self._modules, "gate"), (self._modules, "experts"),
+        watch = [(self._modules, "gate"), (self._modules, "experts"),
                  (self.gate._parameters, "weight"), (self.gate._parameters, "bias")]
         for name, ex in self.experts._modules.items():
             watch.append((self.experts._modules, name))
             watch += _expert_watch(ex, fine_tuning)
+            if fine_tuning:
+                watch.append((ex.__dict__, "lora_scale"))
         usual = len(self.experts) == self.num_experts and all(name in table for table, name in watch)
         return watch if usual else []
 
@@ -606,7 +595,7 @@ class MOE(_Calls):
                 raise ValueError("residual must match the input's shape, dtype and device")
             residual = residual.reshape(-1, d).contiguous()
         if not as_it_lies:
-            done = native.train(x, residual, self.experts[0].dropout.p, None)
+            done = native.train(x, residual, self.experts[0].dropout.p, None, self.top_k)
             if done is not None:
                 return done[0].reshape(shape), done[1], done[2]
         with torch.cuda.device(dev):
@@ -623,7 +612,7 @@ class MOE(_Calls):
             params = [self.gate.weight, self.gate.bias]
             for ex in self.experts:
                 params += _expert_params(ex, fine_tuning)
-            out, aux, seed = native.train(x, residual, float(self.experts[0].dropout.p), params)
+            out, aux, seed = native.train(x, residual, float(self.experts[0].dropout.p), params, k)
         if type(tensor) not in (torch.Tensor, nn.Parameter):
             out = out.as_subclass(type(tensor))
         return out.reshape(shape), aux, seed

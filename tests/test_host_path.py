@@ -91,7 +91,7 @@ def test_nothing_is_bound_after_an_error():
     status = torch.zeros(16, dtype=torch.int32)
     with pytest.raises(KeyError):
         native.bind([(table, "weight"), (table, "bias")], None, [], 0, [status], status, status, 1, D, F, 1, 0)
-    assert native.forward(torch.zeros(1, D, dtype=DT)) is None
+    assert native.forward(torch.zeros(1, D, dtype=DT), 1.0) is None
 
 
 def exchange(params, others):
@@ -158,9 +158,13 @@ def test_a_module_that_ran_can_be_freed(cuda_device, kind):
                 forward(m.eval(), x, fine_tuning)
     ref = weakref.ref(m)
     weight = weakref.ref(next(m.parameters()))
-    del m
     gc.collect()
-    assert ref() is None and weight() is None
+    gc.disable()            # no cycle through a binding: the memory is free at once
+    try:
+        del m
+        assert ref() is None and weight() is None
+    finally:
+        gc.enable()
 
 
 # ---- a backward belongs to the last training forward of its module ---------------------------
@@ -582,7 +586,7 @@ def test_a_copy_of_a_module_that_ran(cuda_device, kind, fine_tuning):
 @pytest.mark.parametrize("kind", KINDS)
 def test_a_call_is_bound_when_it_comes_again(cuda_device, kind):
     m = build(kind, cuda_device).eval()
-    bound = lambda x: (m._native.forward(x, None, None) if kind == "moe" else m._native.forward(x)) is not None
+    bound = lambda x: (m._native.forward(x, None, None, 2) if kind == "moe" else m._native.forward(x, 1.0)) is not None
     with torch.no_grad():
         for n in (1, 2, 3, 48, 4):
             x = rows(n, cuda_device)
