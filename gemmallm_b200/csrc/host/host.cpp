@@ -429,10 +429,11 @@ struct ExpertGrads {
       for (int i = 0; i < per; ++i) need[i] |= wanted(e * per + i);
     bool with_lora = false;
     for (int i = 4; i < per; ++i) with_lora |= need[i];
-    if (need[0] || with_lora) w1 = at::empty({E, 2 * f, d}, opt);
-    if (need[1] || with_lora) b1 = at::empty({E, 2 * f}, opt);
-    if (need[2] || with_lora) w2 = at::empty({E, d, f}, opt);
-    if (need[3] || with_lora) b2 = at::empty({E, d}, opt);
+    // (what the LoRA gradients need of these and nobody wants lies in the training workspace)
+    if (need[0]) w1 = at::empty({E, 2 * f, d}, opt);
+    if (need[1]) b1 = at::empty({E, 2 * f}, opt);
+    if (need[2]) w2 = at::empty({E, d, f}, opt);
+    if (need[3]) b2 = at::empty({E, d}, opt);
     auto ptr = [](Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
     g->w1 = ptr(w1);
     g->b1 = ptr(b1);

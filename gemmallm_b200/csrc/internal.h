@@ -20,8 +20,8 @@ struct TrainGrads {
   void *w1, *b1, *w2, *b2;   // experts [E, 2f, d], [E, 2f], [E, d, f], [E, d]
 };
 
-// LoRA gradients of both Linears (0: gate_and_up, 1: down); they are formed from w1, b1, w2 and b2 of TrainGrads,
-// which are needed with them. A run: experts [first, first + count) of the same ranks and scale.
+// LoRA gradients of both Linears (0: gate_and_up, 1: down); they are formed from w1, b1, w2 and b2 of TrainGrads: those
+// that are not wanted are formed in the training workspace. A run: experts [first, first + count) of the same ranks and scale.
 struct LoraRun {
   int first, count, rank[2];
   float scale;

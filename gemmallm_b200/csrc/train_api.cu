@@ -98,7 +98,6 @@ int experts_backward(const void* perm, const void* h, const int32_t* offsets, co
     if (rc) return rc;
   }
   if (lora == nullptr) return 0;
-  if (!g.w1 || !g.b1 || !g.w2 || !g.b2) return set_error(MOE_B200_ERR_NULL, "LoRA gradients need those of the merged weights");
   const void* const G[2] = {g.w1, g.w2};
   const void* const gb[2] = {g.b1, g.b2};
   for (const LoraRun& run : lora->runs) {
@@ -112,6 +111,17 @@ int experts_backward(const void* perm, const void* h, const int32_t* offsets, co
 TrainGrads own_grads(char* tws, const size_t* to, void* grad_x) {
   return TrainGrads{grad_x, tws + to[MOE_B200_TWS_G_WG], tws + to[MOE_B200_TWS_G_BG], tws + to[MOE_B200_TWS_G_W1],
                     tws + to[MOE_B200_TWS_G_B1], tws + to[MOE_B200_TWS_G_W2], tws + to[MOE_B200_TWS_G_B2]};
+}
+
+// `g` with the workspace's own place for what LoRA gradients need besides
+TrainGrads with_own(TrainGrads g, const LoraGrads* lora, char* tws, const size_t* to) {
+  if (lora == nullptr) return g;
+  const TrainGrads own = own_grads(tws, to, nullptr);
+  if (g.w1 == nullptr) g.w1 = own.w1;
+  if (g.b1 == nullptr) g.b1 = own.b1;
+  if (g.w2 == nullptr) g.w2 = own.w2;
+  if (g.b2 == nullptr) g.b2 = own.b2;
+  return g;
 }
 
 }  // namespace
@@ -314,7 +324,7 @@ int backward_into(const void* x, const void* Wg, const void* plan, const void* g
     if (rc) return rc;
   }
   // the experts (model.py:174-184)
-  TrainGrads eg = grads;
+  TrainGrads eg = with_own(grads, lora, tws, to);
   eg.x = grads.x != nullptr ? dxs : nullptr;
   rc = experts_backward(perm, h, offsets, plan, dy, M, d, f, E, tr, eg, lora, status, s);
   if (rc || grads.x == nullptr) return rc;
@@ -346,7 +356,7 @@ int experts_backward_into(const void* x_sorted, const void* h, const int32_t* of
     MOE_CUDA_CHECK(cudaMemcpyAsync(tws + to[MOE_B200_TWS_DY], grad_y, bytes, cudaMemcpyDeviceToDevice, s));
     dy = tws + to[MOE_B200_TWS_DY];
   }
-  TrainGrads eg = grads;
+  TrainGrads eg = with_own(grads, lora, tws, to);
   if (!aligned16(grads.x)) eg.x = tws + to[MOE_B200_TWS_DXS];
   rc = experts_backward(x_sorted, h, offsets, plan, dy, M, d, f, E, tr, eg, lora, status, s);
   if (rc) return rc;
