@@ -419,7 +419,7 @@ struct ExpertGrads {
   moe::LoraGrads lora_args = {};
   int per = 4;
 
-  // the arguments of the pass; LoRA gradients are wanted if lora_args.tab is set
+  // the arguments of the pass; LoRA gradients are wanted if lora_args has runs
   template <typename Wanted>
   void prepare(const TrainCall& c, const at::TensorOptions& opt, moe::TrainGrads* g, Wanted wanted) {
     const int64_t E = c.E, d = c.d, f = c.f;
@@ -471,7 +471,7 @@ struct ExpertGrads {
     lora_args.tab = static_cast<const void* const*>(c.lora_tab.const_data_ptr());
     lora_args.scratch = scratch.data_ptr<float>();
   }
-  const moe::LoraGrads* lora_grads() const { return lora_args.tab != nullptr ? &lora_args : nullptr; }
+  const moe::LoraGrads* lora_grads() const { return per == 12 ? &lora_args : nullptr; }
   void zero() {
     for (Tensor* t : {&w1, &b1, &w2, &b2})
       if (t->defined()) t->zero_();

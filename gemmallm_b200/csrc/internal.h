@@ -27,6 +27,8 @@ struct LoraRun {
   float scale;
   void *dA[2], *da[2], *dB[2], *db[2];   // [count, rank, in], [count, rank], [count, out, rank], [count, out]
 };
+// Given for every fine-tuning step, without runs where no LoRA tensor is wanted: such a step rounds dh, and what is wanted
+// must not decide what the other gradients are.
 struct LoraGrads {
   const void* const* tab;    // device [2][E][3]: A, a, B of every expert
   float* scratch;            // as many floats as the largest run asks for

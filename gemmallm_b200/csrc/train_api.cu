@@ -115,7 +115,7 @@ TrainGrads own_grads(char* tws, const size_t* to, void* grad_x) {
 
 // `g` with the workspace's own place for what LoRA gradients need besides
 TrainGrads with_own(TrainGrads g, const LoraGrads* lora, char* tws, const size_t* to) {
-  if (lora == nullptr) return g;
+  if (lora == nullptr || lora->runs.empty()) return g;
   const TrainGrads own = own_grads(tws, to, nullptr);
   if (g.w1 == nullptr) g.w1 = own.w1;
   if (g.b1 == nullptr) g.b1 = own.b1;

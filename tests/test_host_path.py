@@ -642,3 +642,24 @@ def test_the_last_call_can_be_cleared(cuda_device):
             assert m.last is None and m.device_status() == 0
             with pytest.raises(ValueError):
                 m.last = {}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_gradients_that_are_wanted_are_those_of_all(cuda_device, kind):
+    """Frozen base weights, frozen adapters, a frozen router, a frozen expert: what is left gets the gradient it gets when
+    everything does."""
+    m, x = build(kind, cuda_device), rows(48, cuda_device)
+    for fine_tuning in (False, True):
+        m.requires_grad_(True)
+        train_step(m, x, fine_tuning)
+        want = {n: p.grad for n, p in m.named_parameters()}
+        for frozen in (lambda n: "lora" not in n, lambda n: "lora" in n, lambda n: "gate." in n, lambda n: "experts.1" in n,
+                       lambda n: "bias" in n, lambda n: "gate_and_up" in n, lambda n: True):
+            for n, p in m.named_parameters():
+                p.requires_grad_(not frozen(n))
+            for _ in range(2):
+                train_step(m, x, fine_tuning)
+                for n, p in m.named_parameters():
+                    assert (p.grad is None) == (frozen(n) or want[n] is None), n
+                    assert p.grad is None or torch.equal(p.grad, want[n]), n
