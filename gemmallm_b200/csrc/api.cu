@@ -472,10 +472,13 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   // between the decode and the prefill sizes: the streaming kernel on the sorted rows
   const bool rows_path = dtype == MOE_B200_BF16 && !small_n && N * k <= kRowsPathMaxRows &&
                          rows_supported(N * k, E);
-  // ... of which those with 192 rows an expert or more, as long as the down product is one round of 256 x 256
-  // tiles, take the prefill products behind the single-launch front: the streaming kernel reads an expert's weights
-  // once per 128 rows and is bound by L2 there. Experts and combine, d 1024, f 4096, 8 experts (us, streaming /
-  // tiles): 1024 rows 79 / 81, 1536 88 / 83, 2346 109 / 101, 3072 117 / 101, 4096 (two rounds) 134 / 157
+  // ... of which those with 192 rows an expert or more (1536 in all with fewer than four experts), as long as the down
+  // product is one round of 256 x 256 tiles, take the prefill products behind the single-launch front: the streaming
+  // kernel reads an expert's weights once per 128 rows and is bound by L2 there. Experts and combine, d 1024, f 4096,
+  // 8 experts (us, streaming / tiles): 1024 rows 79 / 81, 1536 88 / 83, 2346 109 / 101, 3072 117 / 101, 4096 (two
+  // rounds) 134 / 157. With one to three experts a few tiles take as long as a full round of them; whole calls:
+  // 1 expert, d 512, f 2048, 300 rows 38 / 44, 1500 46 / 48; d 1024, f 4096, 300 rows 44 / 52, 1500 68 / 71; d 2048,
+  // f 8192, 300 rows 72 / 86, 1500 171 / 162; 2 experts, d 1024, 500 rows 52 / 60, 1500 72 / 73; 3, 900 rows 62 / 69
   const bool tiles = rows_path && tiles_at_row_counts(N * k, d, E);
   const bool counters = small_n || rows_path;
   // status words, and the completion counters behind them where a kernel uses them, in one memset

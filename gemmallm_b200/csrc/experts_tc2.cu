@@ -708,7 +708,7 @@ int64_t max_tiles(int64_t M, int E, int Nout) {
 
 bool tiles_at_row_counts(int64_t M, int d, int E) {
   const int64_t tiles = ((M + kPairRows - 1) / kPairRows + E / 2) * ((d + BN - 1) / BN);
-  return M >= (int64_t)192 * E && tiles <= kNumSMs / 2;
+  return M >= (E >= 4 ? (int64_t)192 * E : 1536) && tiles <= kNumSMs / 2;
 }
 
 int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d,
