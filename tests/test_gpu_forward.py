@@ -122,6 +122,18 @@ def test_between_streaming_and_prefill(cuda_device, N, d, bias0):
         check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device, residual=res)
 
 
+# the same line with fewer than four experts: 1536 rows
+@pytest.mark.parametrize("N,E,k", [(1535, 1, 1), (1536, 1, 1), (767, 3, 2), (768, 3, 2), (300, 2, 1)])
+def test_between_streaming_and_prefill_with_few_experts(cuda_device, N, E, k):
+    d, f = 136, 264
+    params = helpers.rounded_params(synthetic.make_params(d, E, f, seed=N), torch.bfloat16)
+    x = synthetic.round_to(synthetic.make_input(N, d, seed=N + 1), torch.bfloat16)
+    res = synthetic.round_to(synthetic.make_input(N, d, seed=N + 2), torch.bfloat16)
+    m = build(params, d, E, f, k, torch.bfloat16, cuda_device)
+    for _ in range(2):
+        check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device, residual=res)
+
+
 def test_c0_full_size_fp32(cuda_device):
     wl = synthetic.WORKLOADS["c0"]
     pins = json.loads((GOLDEN / "routing_pins.json").read_text())["c0"]

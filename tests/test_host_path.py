@@ -663,3 +663,108 @@ def test_gradients_that_are_wanted_are_those_of_all(cuda_device, kind):
                 for n, p in m.named_parameters():
                     assert (p.grad is None) == (frozen(n) or want[n] is None), n
                     assert p.grad is None or torch.equal(p.grad, want[n]), n
+
+
+# ---- other ways to run a call ----------------------------------------------------------------------
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("warm", [1, 3])
+@pytest.mark.parametrize("n", [1, 48, 3000])
+@pytest.mark.parametrize("kind", KINDS)
+def test_calls_under_stream_capture(cuda_device, kind, n, warm):
+    """Captured after one warm-up call (not bound yet) or three, replayed on other inputs."""
+    m, x = build(kind, cuda_device).eval(), rows(n, cuda_device)
+    side = torch.cuda.Stream()
+    with torch.no_grad():
+        with torch.cuda.stream(side):
+            for _ in range(warm):
+                forward(m, x)
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = forward(m, x)
+        for seed in (5, 6):
+            x.copy_(rows(n, cuda_device, seed))
+            graph.replay()
+            same(out, forward(fresh_copy(m, kind, cuda_device).eval(), x))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fine_tuning", [False, True])
+def test_a_training_step_under_stream_capture(cuda_device, fine_tuning):
+    m, x = build("ffn", cuda_device, p=0.0).train(), rows(48, cuda_device).requires_grad_(True)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            m.zero_grad(set_to_none=True)
+            m(x, fine_tuning=fine_tuning).float().square().sum().backward()
+    torch.cuda.current_stream().wait_stream(side)
+    m.zero_grad(set_to_none=True)
+    x.grad = None
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = m(x, fine_tuning=fine_tuning)
+        y.float().square().sum().backward()
+    with torch.no_grad():
+        x.copy_(rows(48, cuda_device, 7))
+    graph.replay()
+    got = [y.detach(), x.grad, *(p.grad for p in m.parameters() if p.grad is not None)]
+    got = [t.clone() for t in got]
+    same(got, train_step(fresh_copy(m, "ffn", cuda_device, p=0.0), x, fine_tuning))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_calls_in_inference_mode(cuda_device, kind):
+    m, x = build(kind, cuda_device), rows(48, cuda_device)
+    for fine_tuning in (False, True):
+        with torch.no_grad():
+            want = forward(fresh_copy(m, kind, cuda_device).eval(), x, fine_tuning)
+        for _ in range(3):
+            with torch.inference_mode():
+                z = x.clone()
+                same(forward(m.eval(), z, fine_tuning), want)
+                torch.manual_seed(5)
+                trained = forward(m.train(), z, fine_tuning)
+            same(trained, train_step(fresh_copy(m, kind, cuda_device), x, fine_tuning)[:len(trained)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fine_tuning", [False, True])
+@pytest.mark.parametrize("kind", KINDS)
+def test_parts_replaced_and_sizes_back_and_forth(cuda_device, kind, fine_tuning):
+    """A Linear, a Parameter, and the storage of one replaced under bound calls, at two sizes in turn."""
+    m, xs = build(kind, cuda_device), [rows(n, cuda_device, n) for n in (48, 20)]
+    ex = m.experts[1] if kind == "moe" else m
+
+    def linear():
+        ex.down = torch.nn.Linear(F, D).to(device=cuda_device, dtype=DT)
+
+    def parameter():
+        ex.gate_and_up.weight = torch.nn.Parameter(torch.randn_like(ex.gate_and_up.weight) * 0.1)
+
+    def storage():
+        ex.lora_down_b.weight.data = torch.randn_like(ex.lora_down_b.weight)
+        ex.down.bias.data = torch.randn_like(ex.down.bias)
+
+    def router():
+        if kind == "moe":
+            m.gate = torch.nn.Linear(D, E).to(device=cuda_device, dtype=DT)
+
+    def written():
+        with torch.no_grad():
+            ex.lora_gate_and_up_a.weight.mul_(2.0)
+            ex.down.weight.mul_(0.5)
+
+    for change in (lambda: None, linear, parameter, storage, router, written):
+        change()
+        new = fresh_copy(m, kind, cuda_device)
+        want = [train_step(new, x, fine_tuning) for x in xs]
+        with torch.no_grad():
+            want_eval = [forward(new.eval(), x, fine_tuning) for x in xs]
+        for _ in range(3):
+            for x, a, b in zip(xs, want, want_eval):
+                same(train_step(m, x, fine_tuning), a)
+                with torch.no_grad():
+                    same(forward(m.eval(), x, fine_tuning), b)
+                    same(forward(m, x, fine_tuning), b)
