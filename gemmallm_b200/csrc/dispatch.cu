@@ -350,7 +350,7 @@ int launch_dispatch(const void* x, const int32_t* idx, int64_t N, int d, int E, 
 // inside a framework's forward hook with a frozen memory pool, a serving loop
 // whose allocator is locked while requests are in flight, or a host language
 // binding that only receives the tensors of the op's signature. For them the
-// per-chunk counters live in this file-scope device array instead. Every GPU
+// per-block counters live in this file-scope device array instead. Every GPU
 // that loads the library holds kStaticScratchInts * 4 bytes (1 MiB) for the
 // lifetime of the process.
 //

@@ -63,8 +63,9 @@ enum {
    * zeroed once, and every call on this workspace since then has ended with
    * device status 0 (such calls leave the region zero). Saves the memset in
    * front of the first kernel of calls of up to 4096 rows, which then overlaps
-   * the tail of the kernel before it; larger calls clear the status words anyway. After a non-zero device status the region
-   * has to be zeroed again by the caller. */
+   * the tail of the kernel before it; larger calls clear the status words
+   * anyway. After a non-zero device status the region has to be zeroed again by
+   * the caller. */
   MOE_B200_FLAG_WS_CLEAN = 1
 };
 
@@ -160,9 +161,9 @@ int64_t moe_b200_router_blocks(int64_t N);
  * token rows into one expert-contiguous buffer; replaces the per-slot argsort,
  * count loop, gather and split of model.py:226-253. Rows of one expert keep
  * token order (stable).
- *   scratch    moe_b200_dispatch_scratch_bytes(N,E,k) bytes: per-chunk and
- *              per-block expert counts, per-block per-slot counts; contents
- *              need no initialisation and are overwritten by every call
+ *   scratch    moe_b200_dispatch_scratch_bytes(N,E,k) bytes: per-block expert
+ *              counts and per-slot counts (and room that earlier versions used);
+ *              contents need no initialisation and are overwritten by every call
  *   cnt_slot   int32 [k,E]   (top_expert_counts, second_expert_counts, ...)
  *   offsets    int32 [E+1]
  *   row_of     int32 [N,k]
