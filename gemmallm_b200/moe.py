@@ -173,7 +173,7 @@ class _Asked:
     """How often the last call, plain and with LoRA branches, has had to be prepared. Binding a call to the native path
     costs about as much as it saves one call, so it is done the second, fourth, eighth ... time: not for a size seen once
     (generation without a cache has another length with every token), and seldom for calls that find the
-    binding unusable."""
+    binding unusable. Other weights, slots or scales are another call and count anew."""
 
     def __init__(self):
         self.last = {}
@@ -351,7 +351,7 @@ class FeedForward(_Calls):
             check(lib.moe_b200_experts(x.data_ptr(), offsets.data_ptr(), plan, M, d, f, 1, dtype, 0,
                                        h.data_ptr(), y.data_ptr(), status.data_ptr(), _stream(dev)),
                   "experts")
-        if not self._calls.bind_now(fine_tuning, (M, dtype, str(dev))):
+        if not self._calls.bind_now(fine_tuning, (M, dtype, str(dev), plan, self.lora_scale)):
             return y.reshape(shape)
         native.unbind()
         watch = _expert_watch(self, fine_tuning)
@@ -531,7 +531,8 @@ class MOE(_Calls):
                                        nw, nb, eps, N, d, f, E, k, dtype, _cabi.FLAG_WS_CLEAN, base, nbytes,
                                        out.data_ptr(), _stream(dev)), "forward")
         aux = self._view("aux", torch.float32, (1,))[0].clone()
-        if self._calls.bind_now(fine_tuning, (N, dtype, str(dev))):
+        scales = tuple(ex.lora_scale for ex in self.experts) if fine_tuning else ()
+        if self._calls.bind_now(fine_tuning, (N, dtype, str(dev), plan, gw.data_ptr(), gb.data_ptr(), k, scales)):
             self._bind(native, fine_tuning, plan, N, dtype, dev)
         return out.reshape(shape), aux
 

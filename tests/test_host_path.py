@@ -594,6 +594,13 @@ def test_a_call_is_bound_when_it_comes_again(cuda_device, kind):
             assert not bound(x)
         forward(m, x)
         assert bound(x)
+        for _ in range(5):       # other weights: another call
+            for p in m.parameters():
+                p.data = p.data * 0.5
+            forward(m, x)
+            assert not bound(x)
+            same(forward(m, x), forward(fresh_copy(m, kind, cuda_device).eval(), x))
+            assert bound(x)
 
 
 @pytest.mark.gpu
