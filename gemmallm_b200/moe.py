@@ -336,8 +336,10 @@ class FeedForward(_Calls):
         offsets and merged weights, runs, and binds the result."""
         dtype = _dtype_code(tensor)
         shape = tensor.shape
-        x, M, dev, offsets = self._rows(tensor)
         d, f = self.hidden_size, self.d_ff
+        if shape[-1] != d:
+            raise ValueError(f"last dimension {shape[-1]} != hidden_size {d}")
+        x, M, dev, offsets = self._rows(tensor)
         if not tensor.is_contiguous():
             y = native.forward(x, self.lora_scale)          # bound for these rows, contiguous
             if y is not None:
@@ -355,7 +357,7 @@ class FeedForward(_Calls):
             return y.reshape(shape)
         native.unbind()
         watch = _expert_watch(self, fine_tuning)
-        if x.shape[-1] == d and all(name in table for table, name in watch):
+        if all(name in table for table, name in watch):
             native.bind(watch, *self._bound(fine_tuning), plan, [self._plan_of(fine_tuning).buf], offsets, status, M, d, f,
                         dtype, dev.index)
         return y.reshape(shape)

@@ -775,3 +775,18 @@ def test_parts_replaced_and_sizes_back_and_forth(cuda_device, kind, fine_tuning)
                 with torch.no_grad():
                     same(forward(m.eval(), x, fine_tuning), b)
                     same(forward(m, x, fine_tuning), b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_rows_of_another_width_are_refused(cuda_device, kind):
+    """(The feed-forward in inference took them for rows of its own width, past the end of the input.)"""
+    m = build(kind, cuda_device)
+    for train in (True, False):
+        m.train(train)
+        for _ in range(3):
+            with torch.no_grad():
+                forward(m, rows(48, cuda_device))
+                for width in (D // 2, D * 2, D - 8):
+                    with pytest.raises(ValueError):
+                        forward(m, torch.zeros(48, width, dtype=DT, device=cuda_device))
