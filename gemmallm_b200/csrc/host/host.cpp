@@ -178,7 +178,8 @@ struct Held {
 };
 
 // Merged copies W' = W + s B A, b' = b + s (B a + b_lora) of the two Linears of a list of experts, and the one record of
-// what they hold: addresses, versions and scale of the last merge. Every call that reads them, bound or not, forward
+// what they hold: storages, addresses, versions and scale of the last merge (weak references: an address alone may have
+// been given to other weights since, and weights that were moved away must be freed). Every call that reads them, bound or not, forward
 // or backward, compares its own parameters with that record first, so that adapters that were exchanged in between, by
 // whichever call, are merged again. Parameters are counted as in moe.py: twelve an expert.
 class Merged {
@@ -201,7 +202,7 @@ class Merged {
     return true;
   }
   size_t num_params() const { return jobs_.size() * 6; }
-  // param(i) -> (address, version) of the i-th parameter; scale of every expert
+  // param(i) -> (address, version, storage) of the i-th parameter; scale of every expert
   template <typename Param>
   int refresh(Param param, const std::vector<double>& scales, int dtype, void* stream) {
     const std::lock_guard<std::mutex> lock(mutex_);      // a backward runs on another thread
@@ -213,10 +214,12 @@ class Merged {
                             first + 7 + 4 * l};
       const void* data[6];
       int64_t version[6];
+      const c10::Storage* storage[6];
       bool same = j.valid && j.scale == scales[i / 2];
       for (int q = 0; q < 6; ++q) {
-        std::tie(data[q], version[q]) = param(at[q]);
-        same = same && data[q] == j.data[q] && version[q] == j.version[q];
+        std::tie(data[q], version[q], storage[q]) = param(at[q]);
+        same = same && data[q] == j.data[q] && version[q] == j.version[q] &&
+               storage[q]->unsafeGetStorageImpl() == j.storage[q]._unsafe_get_target();
       }
       if (same) continue;
       j.valid = false;
@@ -225,6 +228,8 @@ class Merged {
       if (rc != 0) return rc;
       std::copy(data, data + 6, j.data);
       std::copy(version, version + 6, j.version);
+      j.storage.clear();
+      for (const c10::Storage* s : storage) j.storage.push_back(s->getWeakStorageImpl());
       j.scale = scales[i / 2];
       j.valid = true;
     }
@@ -238,6 +243,7 @@ class Merged {
     bool valid = false;
     const void* data[6];
     int64_t version[6];
+    std::vector<c10::weak_intrusive_ptr<c10::StorageImpl>> storage;
     double scale = 0.0;
   };
   std::vector<Job> jobs_;
@@ -257,15 +263,18 @@ struct MergedUse {
     return merged->refresh(
         [&](size_t i) {
           const Tensor& t = w.param((int)(first + i));
-          return std::make_pair(t.const_data_ptr(), (int64_t)t._version());
+          return std::make_tuple(t.const_data_ptr(), (int64_t)t._version(), &t.storage());
         },
         scales, dtype, stream);
   }
   int refresh(const std::vector<Held>& h, int dtype, void* stream) const {
     if (merged == nullptr) return 0;
     return merged->refresh(
-        [&](size_t i) { return std::make_pair(h[first + i].data, (int64_t)h[first + i].version.current_version()); }, scales,
-        dtype, stream);
+        [&](size_t i) {
+          const Held& p = h[first + i];
+          return std::make_tuple(p.data, (int64_t)p.version.current_version(), &p.storage);
+        },
+        scales, dtype, stream);
   }
 };
 
@@ -314,7 +323,8 @@ PyObject* merged_refresh(PyObject* o, PyObject* args) {
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
   void* stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
   const int rc = m.refresh(
-      [&](size_t i) { return std::make_pair(t[i].const_data_ptr(), (int64_t)t[i]._version()); }, s, dtype, stream);
+      [&](size_t i) { return std::make_tuple(t[i].const_data_ptr(), (int64_t)t[i]._version(), &t[i].storage()); }, s, dtype,
+      stream);
   if (rc != 0) return fail(rc, "lora_merge");
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS

@@ -790,3 +790,26 @@ def test_rows_of_another_width_are_refused(cuda_device, kind):
                 for width in (D // 2, D * 2, D - 8):
                     with pytest.raises(ValueError):
                         forward(m, torch.zeros(48, width, dtype=DT, device=cuda_device))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_adapters_at_an_address_that_others_had(cuda_device, kind):
+    """A tensor's storage replaced twice between two calls, the second time by one that lies where the first call's lay:
+    address and version are as before, the values are not."""
+    m, x = build(kind, cuda_device), rows(48, cuda_device)
+    ex = m.experts[2] if kind == "moe" else m
+    p = ex.lora_gate_and_up_b.weight
+    for _ in range(3):
+        with torch.no_grad():
+            want = forward(fresh_copy(m, kind, cuda_device).eval(), x, True)
+            for _ in range(3):
+                same(forward(m.eval(), x, True), want)
+            address, held = p.data_ptr(), []
+            p.data = torch.randn_like(p)
+            while len(held) < 1000 and p.data_ptr() != address:
+                new = torch.randn_like(p)
+                if new.data_ptr() == address:
+                    p.data = new
+                held.append(new)
+            assert p.data_ptr() == address
