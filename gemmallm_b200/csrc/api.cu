@@ -141,10 +141,8 @@ int moe_b200_plan_build(const void* const* h_W1, const void* const* h_b1, const 
     ptrs[2 * E + e] = h_W2[e];
     ptrs[3 * E + e] = h_b2[e];
   }
-  if (dtype == MOE_B200_BF16) {
-    rc = build_weight_tensor_maps(h_W1, h_W2, E, d, f, stage + plan_ptr_bytes(E));
-    if (rc) return rc;
-  }
+  rc = build_weight_tensor_maps(h_W1, h_W2, E, d, f, dtype, stage + plan_ptr_bytes(E));
+  if (rc) return rc;
   MOE_CUDA_CHECK(cudaMemcpyAsync(plan, stage, bytes, cudaMemcpyHostToDevice, (cudaStream_t)stream));
   // the staging buffer is reused by the next call on this thread
   MOE_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));
@@ -251,7 +249,7 @@ int moe_b200_experts(const void* perm, const int32_t* offsets, const void* plan,
   if (dtype == MOE_B200_BF16)
     return launch_experts_tc2(perm, offsets, plan, M, d, f, E, h, y, nullptr, status,
                               (cudaStream_t)stream);
-  return launch_experts_simt(perm, offsets, plan, M, d, f, E, h, y, (cudaStream_t)stream);
+  return launch_experts_f32(perm, offsets, plan, M, d, f, E, h, y, status, (cudaStream_t)stream);
 }
 
 int moe_b200_rows_splits(int64_t M, int d, int f, int E) { return M > 0 && f >= 8 && d >= 8 && E >= 1 ? rows_splits(M, d, f, E) : 0; }

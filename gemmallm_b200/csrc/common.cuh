@@ -119,10 +119,17 @@ __device__ __forceinline__ void from_f32(__nv_bfloat16& o, float v) { o = __floa
 
 // GELU, tanh form, exactly the expression of F.gelu(approximate="tanh")
 // (used at model.py:181): 0.5 g (1 + tanh(sqrt(2/pi) (g + 0.044715 g^3))).
+// 0.5 (1 + tanh z) = 1 / (1 + exp(-2 z)): fewer instructions than tanhf, no cancellation where the tanh nears -1, and
+// no branch: the quotient g / (1 + e) from the hardware's approximate reciprocal and one correction by its remainder
+// (Markstein, IBM J. Res. Dev. 34 (1990) 111), so that several of them run side by side.
 __device__ __forceinline__ float gelu_tanh_precise(float g) {
-  const float kBeta = 0.7978845608028654f;  // sqrt(2/pi)
-  float inner = kBeta * (g + 0.044715f * g * g * g);
-  return 0.5f * g * (1.0f + tanhf(inner));
+  const float k2Beta = 2.f * 0.7978845608028654f;  // 2 sqrt(2/pi)
+  const float den = 1.0f + expf(-g * fmaf(0.044715f * k2Beta, g * g, k2Beta));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
+  const float q = g * r;
+  // (the remainder would be NaN for g = inf, where den = 1, and for den = inf, where q is the limit too)
+  return den > 1.0f && den < 1e37f ? fmaf(fmaf(-q, den, g), r, q) : q;
 }
 __device__ __forceinline__ float tanh_approx(float x) {
   float y;
@@ -283,12 +290,12 @@ int launch_norm_fold(const void* Wg, const void* bg, const void* gamma, const vo
                      int d, int dtype, void* Wn, float* c, cudaStream_t s);
 int launch_layernorm_rows(const void* x, const void* gamma, const void* beta, float eps, int64_t N,
                           int d, int dtype, void* out, float* stats, cudaStream_t s);
-int launch_experts_simt(const void* perm, const int32_t* offsets, const void* plan, int64_t M,
-                        int d, int f, int E, void* h, void* y, cudaStream_t s);
+int launch_experts_f32(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d,
+                       int f, int E, void* h, void* y, int32_t* status, cudaStream_t s);
 int launch_combine(const void* y, const int32_t* row_of, const float* w, const void* residual,
                    int64_t N, int d, int k, int dtype, void* out, cudaStream_t s,
                    const EpSync* ep_wait = nullptr, int32_t* status = nullptr);
-int build_weight_tensor_maps(const void* const* h_W1, const void* const* h_W2, int E, int d, int f,
+int build_weight_tensor_maps(const void* const* h_W1, const void* const* h_W2, int E, int d, int f, int dtype,
                              void* h_tmaps /* kPlanMapsPerExpert*E*128 bytes */);
 int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d,
                        int f, int E, void* h, void* y, const EpScatter* sc, int32_t* status,
@@ -324,6 +331,7 @@ int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N,
                        int32_t* status = nullptr);
 int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
                    uint32_t box_cols = 64);
+int encode_tmap_2d_f32(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 int sm_count(int* sms);
 int decode_splits(int f);
 int decode_spec_rows(int64_t N);

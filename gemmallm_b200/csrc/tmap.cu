@@ -49,11 +49,35 @@ int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, ui
   return 0;
 }
 
-// Plan maps per expert: W1 and W2 with 128-row boxes (large-N path), then W1
-// and W2 with 64-row boxes (small-N path).
-int build_weight_tensor_maps(const void* const* h_W1, const void* const* h_W2, int E, int d, int f,
+// [rows, cols] row-major fp32, box = box_rows x 32 columns (128-byte swizzle).
+int encode_tmap_2d_f32(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  EncodeTiledFn enc = get_encode();
+  if (enc == nullptr) return set_error(MOE_B200_ERR_DRIVER, "cuTensorMapEncodeTiled unavailable");
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {cols * 4};
+  cuuint32_t box[2] = {32, box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(static_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims,
+                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(MOE_B200_ERR_DRIVER, "cuTensorMapEncodeTiled failed");
+  return 0;
+}
+
+// Plan maps per expert. bf16: W1 and W2 with 128-row boxes (large-N path), then W1 and W2 with 64-row boxes
+// (small-N path). fp32: W1 and W2 with 64-row boxes.
+int build_weight_tensor_maps(const void* const* h_W1, const void* const* h_W2, int E, int d, int f, int dtype,
                              void* h_tmaps) {
   char* maps = static_cast<char*>(h_tmaps);
+  if (dtype == MOE_B200_F32) {
+    for (int e = 0; e < E; ++e) {
+      int rc = encode_tmap_2d_f32(maps + 128 * (size_t)e, h_W1[e], (uint64_t)2 * f, (uint64_t)d, 64);
+      if (rc) return rc;
+      rc = encode_tmap_2d_f32(maps + 128 * (size_t)(E + e), h_W2[e], (uint64_t)d, (uint64_t)f, 64);
+      if (rc) return rc;
+    }
+    return 0;
+  }
   for (int e = 0; e < E; ++e) {
     int rc = encode_tmap_2d(maps + 128 * (size_t)e, h_W1[e], (uint64_t)2 * f, (uint64_t)d, 128);
     if (rc) return rc;

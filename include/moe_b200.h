@@ -207,8 +207,8 @@ int moe_b200_dispatch_static(const void* x, const int32_t* idx,
 /* Part 3 — experts: for every expert e and its rows [offsets[e], offsets[e+1])
  * of perm: h = gelu_tanh(x W1g^T + b1g) * (x W1u^T + b1u), y = h W2^T + b2
  * (FeedForward.forward, model.py:173-190 with fine_tuning=False, dropout in
- * eval mode). M = N*k rows. bf16 runs on tcgen05 tensor cores with fp32
- * accumulation; fp32 runs on CUDA cores. h [M,f] and y [M,d] are outputs.
+ * eval mode). M = N*k rows. Both run on tcgen05 tensor cores with fp32
+ * accumulation, fp32 operands as exact sums of three bf16 parts. h [M,f] and y [M,d] are outputs.
  * flags: reserved, pass 0. */
 int moe_b200_experts(const void* perm, const int32_t* offsets, const void* plan,
                      int64_t M, int d, int f, int E, int dtype, int flags,

@@ -224,6 +224,45 @@ def test_experts_fp32_tile_edges(cuda_device, rows, d, f):
     assert (y.cpu().double() - y_ref).norm() <= 4e-6 * y_ref.norm()
 
 
+# edges of the fp32 token tiles (16 and 160 tokens) and of the read-outs (64 and 256 of K), whole and with K over clusters
+# of two, four and eight CTAs, more tiles than SMs
+@pytest.mark.parametrize("rows,d,f", [([15, 16, 17, 159], 512, 2048), ([160, 161, 0, 321], 1024, 512), ([7], 1024, 136),
+                                      ([40, 3], 64, 1024), ([33] * 64, 288, 264), ([1] * 9, 264, 1096)])
+def test_experts_fp32_against_64_bits(cuda_device, rows, d, f):
+    params, x, offsets = expert_inputs(rows, d, f, torch.float32, seed=5 * len(rows) + d)
+    dp = helpers.device_params(params, torch.float32, cuda_device)
+    plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
+    h, y, status = helpers.experts(x.to(cuda_device), offsets.to(cuda_device), plan)
+    assert status.cpu()[0] == 0
+    p64 = {n: t.double() for n, t in params.items()}
+    h_ref, _ = oracle_experts(p64, x.double(), offsets)
+    assert (h.cpu().double() - h_ref).norm() <= 5e-7 * h_ref.norm()
+    # the second product of the h it was given; four truncated steps of 2^-23 per read-out, then rounded sums
+    y_ref = torch.cat([F.linear(h[offsets[e]:offsets[e + 1]].cpu().double(), p64["w2"][e], p64["b2"][e])
+                       for e in range(len(rows))])
+    assert (y.cpu().double() - y_ref).norm() <= 3e-7 * y_ref.norm()
+
+
+@pytest.mark.parametrize("rows,d,f", [([40, 170], 512, 2048), ([3, 2], 1024, 1024)])
+def test_experts_fp32_not_finite(cuda_device, rows, d, f):
+    """Infinities, NaN and sums that overflow come out as fp32 arithmetic gives them, and nowhere else."""
+    params, x, offsets = expert_inputs(rows, d, f, torch.float32, seed=d)
+    x[0, 3], x[1, d - 1], x[rows[0] + 1, 5], x[2, 7] = float("inf"), float("nan"), -float("inf"), 3e38
+    params["w1"][0, 9, 7], params["w2"][1, 11, 100], params["w1"][1, f + 2, 1] = 1e4, float("inf"), -float("inf")
+    dp = helpers.device_params(params, torch.float32, cuda_device)
+    plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
+    h, y, status = helpers.experts(x.to(cuda_device), offsets.to(cuda_device), plan)
+    assert status.cpu()[0] == 0
+    h_ref, _ = oracle_experts(params, x, offsets)
+    y_ref = torch.cat([F.linear(h[offsets[e]:offsets[e + 1]].cpu(), params["w2"][e], params["b2"][e])
+                       for e in range(len(rows))])
+    for got, ref in ((h.cpu(), h_ref), (y.cpu(), y_ref)):
+        assert torch.equal(got.isnan(), ref.isnan())
+        assert torch.equal(got.isinf(), ref.isinf()) and torch.equal(got[got.isinf()], ref[ref.isinf()])
+        ok = ref.isfinite() & (ref.abs() < 1e6)
+        assert torch.allclose(got[ok], ref[ok], atol=1e-4, rtol=1e-5)
+
+
 # the down product with its contraction split over the pairs of a cluster: four and two ranges, the last one shorter,
 # K that is no multiple of 64, a last tile of 8 columns, odd CTAs without rows, an expert without rows; 33 tiles: none
 @pytest.mark.parametrize("rows,d,f", [([700], 1024, 2056), ([300, 1, 0, 40], 520, 1032), ([2048], 1024, 1024),
