@@ -49,7 +49,7 @@ static void layout(int64_t N, int d, int f, int E, int k, int dtype, size_t* off
   sizes[MOE_B200_WS_PSUM] = (size_t)E * sizeof(float);
   sizes[MOE_B200_WS_AUX] = sizeof(float);
   sizes[MOE_B200_WS_SCRATCH] = (size_t)dispatch_scratch_ints(N, E, k) * sizeof(int32_t);
-  if (front_split_supported(N, E, k, dtype) &&
+  if ((dtype == MOE_B200_F32 ? front_f32_supported(N, E, k) : front_split_supported(N, E, k, dtype)) &&
       (size_t)front_small_exchange_ints(N, E, k) * sizeof(int32_t) > sizes[MOE_B200_WS_SCRATCH])
     sizes[MOE_B200_WS_SCRATCH] = (size_t)front_small_exchange_ints(N, E, k) * sizeof(int32_t);
   sizes[MOE_B200_WS_CNT_SLOT] = (size_t)k * E * sizeof(int32_t);
@@ -478,14 +478,16 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   // 1 expert, d 512, f 2048, 300 rows 38 / 44, 1500 46 / 48; d 1024, f 4096, 300 rows 44 / 52, 1500 68 / 71; d 2048,
   // f 8192, 300 rows 72 / 86, 1500 171 / 162; 2 experts, d 1024, 500 rows 52 / 60, 1500 72 / 73; 3, 900 rows 62 / 69
   const bool tiles = rows_path && tiles_at_row_counts(N * k, d, E);
-  const bool counters = small_n || rows_path;
+  // (a folded LayerNorm stays with the general kernels)
+  const bool front32 = dtype == MOE_B200_F32 && !norm && front_f32_supported(N, E, k);
+  const bool counters = small_n || rows_path || front32;
   // status words, and the completion counters behind them where a kernel uses them, in one memset
   // (above these sizes a call always clears the status words: they are those of the most recent call)
   if (!(counters && (flags & MOE_B200_FLAG_WS_CLEAN)))
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
-  const bool front = (small_n || rows_path) &&
-                     (front_small_supported(N, E, k, dtype) || front_split_supported(N, E, k, dtype));
+  const bool front = front32 || ((small_n || rows_path) && (front_small_supported(N, E, k, dtype) ||
+                                                            front_split_supported(N, E, k, dtype)));
   float* stats = reinterpret_cast<float*>(ws + off[MOE_B200_WS_STATS]);
   if (norm && N > 0 && (front || small_n || rows_path)) {
     // up to 4096 rows the kernels read x through TMA: normalise the few rows once
@@ -503,7 +505,7 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
     // (beyond 128 tokens its blocks share the work and meet at a counter behind the status words)
     rc = launch_front_small(x, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm,
                             psum, aux, s, scratch,
-                            status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status);
+                            status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, dtype);
     if (rc) return rc;
   } else {
     if (fold) {

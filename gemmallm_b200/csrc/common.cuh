@@ -328,7 +328,9 @@ int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
                        cudaStream_t s, int* xch = nullptr, int* counter = nullptr,
-                       int32_t* status = nullptr);
+                       int32_t* status = nullptr, int dtype = MOE_B200_BF16);
+// fp32, with the exchange buffer and the counter
+bool front_f32_supported(int64_t N, int E, int k);
 int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
                    uint32_t box_cols = 64);
 int encode_tmap_2d_f32(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);

@@ -11,46 +11,48 @@ constexpr int kMaxTok = kFrontMaxTok;
 constexpr int kMaxE = kFrontMaxE;
 constexpr int kMaxPairs = kFrontMaxPairs;
 
-template <int NT, bool SPLIT>
+template <int NT, bool SPLIT, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-front_small_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ Wg,
-                   const __nv_bfloat16* __restrict__ bg, int Ntotal, int d, int E, int k,
+front_small_kernel(const T* __restrict__ x, const T* __restrict__ Wg,
+                   const T* __restrict__ bg, int Ntotal, int d, int E, int k,
                    float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                    float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
                    int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
-                   __nv_bfloat16* __restrict__ perm, float* __restrict__ psum,
+                   T* __restrict__ perm, float* __restrict__ psum,
                    float* __restrict__ aux, int* __restrict__ xch, int* __restrict__ counter,
                    int32_t* __restrict__ status) {
   extern __shared__ float smem[];
   pdl_wait();                 // x may come from the kernel before this one
   pdl_launch_dependents();
-  front_small_body<NT, SPLIT>(smem, (int)blockIdx.x, (int)gridDim.x, x, Wg, bg, Ntotal, d, E, k,
+  front_small_body<NT, SPLIT, T>(smem, (int)blockIdx.x, (int)gridDim.x, x, Wg, bg, Ntotal, d, E, k,
                               out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux,
                               xch, counter, status);
 }
 
-template <int NT>
+template <int NT, typename T>
 int launch(const void* x, const void* Wg, const void* bg, int N, int d, int E, int k,
            float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot, int32_t* offsets,
            int32_t* row_of, void* perm, float* psum, float* aux, int* xch, int* counter,
            int32_t* status, cudaStream_t s) {
   // beyond 128 tokens repeating the routing in every block costs more than one exchange
-  const bool split = xch != nullptr && counter != nullptr && status != nullptr && N > 128;
+  constexpr bool F32 = sizeof(T) == 4;
+  const bool split = F32 || (xch != nullptr && counter != nullptr && status != nullptr && N > 128);
   const int ntok = split ? 16 : N;
   const size_t smem = front_small_smem_bytes(NT, ntok, E, k);
   static PerDeviceOnce once_whole, once_split;
-  int rc = ensure_dynamic_smem(once_whole, front_small_kernel<NT, false>, 160 * 1024);
+  auto fn = front_small_kernel<NT, true, T>;
+  int rc = ensure_dynamic_smem(once_split, fn, 160 * 1024);
   if (rc) return rc;
-  rc = ensure_dynamic_smem(once_split, front_small_kernel<NT, true>, 160 * 1024);
-  if (rc) return rc;
+  if constexpr (!F32) {
+    rc = ensure_dynamic_smem(once_whole, front_small_kernel<NT, false, T>, 160 * 1024);
+    if (rc) return rc;
+    if (!split) fn = front_small_kernel<NT, false, T>;
+  }
   // one block per 16 tokens
   const int blocks = N <= 16 ? 1 : (N + 15) / 16;
-  auto fn = split ? front_small_kernel<NT, true> : front_small_kernel<NT, false>;
-  MOE_CUDA_CHECK(launch_pdl(fn, dim3(blocks), dim3(kThreads), smem, s,
-                            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(Wg),
-                            static_cast<const __nv_bfloat16*>(bg), N, d, E, k, out_logits, out_idx,
-                            out_w, cnt_slot, offsets, row_of, static_cast<__nv_bfloat16*>(perm), psum,
-                            aux, xch, counter, status));
+  MOE_CUDA_CHECK(launch_pdl(fn, dim3(blocks), dim3(kThreads), smem, s, static_cast<const T*>(x),
+                            static_cast<const T*>(Wg), static_cast<const T*>(bg), N, d, E, k, out_logits, out_idx,
+                            out_w, cnt_slot, offsets, row_of, static_cast<T*>(perm), psum, aux, xch, counter, status));
   return 0;
 }
 
@@ -74,13 +76,30 @@ int64_t front_small_exchange_ints(int64_t N, int E, int k) {
   return nb * k * E + nb * E;
 }
 
+// fp32 calls: the general kernels took 36 us at 512 tokens (d 512, 8 experts: router 22, dispatch 14, with a memset in front);
+// beyond 2048 tokens the blocks would no longer all be resident.
+bool front_f32_supported(int64_t N, int E, int k) {
+  return N >= 1 && N <= 16 * 128 && E <= kMaxE && k <= kMaxTopK && N * k <= kRowsPathMaxRows;
+}
+
+namespace {
+template <typename T, typename... Args>
+int launch_by_experts(int E, Args... args) {
+  if (E <= 8) return launch<1, T>(args...);
+  if (E <= 16) return launch<2, T>(args...);
+  return launch<4, T>(args...);
+}
+}  // namespace
+
 int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E, int k,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
-                       cudaStream_t s, int* xch, int* counter, int32_t* status) {
-  if (E <= 8) return launch<1>(x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux, xch, counter, status, s);
-  if (E <= 16) return launch<2>(x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux, xch, counter, status, s);
-  return launch<4>(x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux, xch, counter, status, s);
+                       cudaStream_t s, int* xch, int* counter, int32_t* status, int dtype) {
+  if (dtype == MOE_B200_F32)
+    return launch_by_experts<float>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of,
+                                    perm, psum, aux, xch, counter, status, s);
+  return launch_by_experts<__nv_bfloat16>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
+                                          row_of, perm, psum, aux, xch, counter, status, s);
 }
 
 }  // namespace moe

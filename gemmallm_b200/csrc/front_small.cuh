@@ -4,11 +4,13 @@
 // each one derives the complete routing by itself (the same instructions on the
 // same data, so every block gets the same answer and no grid barrier is needed),
 // block 0 writes the routing results, and the row copies are split over the blocks.
-// Covers reference model.py:206-253 for N <= 512, N*k <= 1024, E <= 32, bf16:
+// Covers reference model.py:206-253 for N <= 512, N*k <= 1024, E <= 32, bf16 (blocks that share the work: up to 2048
+// tokens, bf16 and fp32):
 //   A. logits: 32 warps = (16-token group) x (slice of K); each warp forms its
 //      partial x Wg^T with mma.sync m16n8k16 exactly like router_mma_kernel
 //      (router.cu), all its loads in flight at once; partials are summed over
-//      the K slices in slice order, plus bias;
+//      the K slices in slice order, plus bias. fp32: a thread per (token,
+//      expert mod 8, eighth of K), eight sums of every eighth element there;
 //   B. 8, 16 or 32 lanes per token, lane e = expert e: fp32 softmax, k passes of
 //      arg-max ordered by (logit desc, index asc) with shuffle reductions
 //      on order-preserving keys, renormalise;
@@ -72,19 +74,21 @@ __host__ __device__ inline size_t front_small_smem_bytes(int NT, int ntok, int E
          sizeof(float) * (size_t)ntok * k;
 }
 
-template <int NT, bool SPLIT>  // n-tiles of 8 experts: E <= 8*NT
+template <int NT, bool SPLIT, typename T = __nv_bfloat16>  // n-tiles of 8 experts: E <= 8*NT
 __device__ __forceinline__ FrontSmallView
 front_small_body(float* smem, const int blk, const int nblk,
-                 const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ Wg,
-                 const __nv_bfloat16* __restrict__ bg, int Ntotal, int d, int E, int k,
+                 const T* __restrict__ x, const T* __restrict__ Wg, const T* __restrict__ bg, int Ntotal, int d, int E, int k,
                  float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                  float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
                  int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
-                 __nv_bfloat16* __restrict__ perm, float* __restrict__ psum,
+                 T* __restrict__ perm, float* __restrict__ psum,
                  float* __restrict__ aux, int* __restrict__ xch, int* __restrict__ counter,
                  int32_t* __restrict__ status) {
   constexpr int kThreads = kFrontThreads;
   constexpr int kMaxE = kFrontMaxE;
+  constexpr bool F32 = sizeof(T) == 4;
+  static_assert(!F32 || SPLIT, "fp32: blocks of 16 tokens");
+  constexpr int kPiece = 16 / sizeof(T);                   // elements of a 16-byte piece
   const int ld = E + 1;
   // SPLIT: this block's 16 tokens are "the problem" for the phases A and B below
   const int tok_base = SPLIT ? 16 * blk : 0;
@@ -100,7 +104,7 @@ front_small_body(float* smem, const int blk, const int nblk,
   const int ngroups = (N + 15) >> 4;                       // 16-token groups
   int gp2 = 1;
   while (gp2 < ngroups) gp2 <<= 1;                         // 1, 2, 4 or 8
-  const int nslices = 32 / gp2;                            // K slices
+  const int nslices = F32 ? 8 : 32 / gp2;                  // K slices
   float* s_part = smem;                                    // [nslices][16*gp2][8*NT]
   float* s_logit = s_part + (size_t)nslices * 16 * gp2 * 8 * NT;   // [N][E+1]
   int* s_idx = reinterpret_cast<int*>(s_logit + (size_t)N * ld);   // [N*k]
@@ -115,10 +119,44 @@ front_small_body(float* smem, const int blk, const int nblk,
   const int g = lane >> 2, t = lane & 3;
   constexpr int ET_C = 8 * NT;
   const int ET = ET_C;
-  if (tid < E) s_bias[tid] = __bfloat162float(bg[tid]);   // visible after the barrier behind part A
+  if (tid < E) s_bias[tid] = to_f32(bg[tid]);   // visible after the barrier behind part A
 
   // ---- A. partial logits -----------------------------------------------------
-  {
+  if constexpr (F32) {
+    // lane = (token of four, expert mod 8): a warp reads four rows of x and eight of Wg
+    const int tok = (warp & 3) * 4 + (lane >> 3), e0 = lane & 7, ks = warp >> 2;
+    const float4* xr = reinterpret_cast<const float4*>(x + (size_t)min(tok, N - 1) * d);
+    const float4* w4 = reinterpret_cast<const float4*>(Wg);
+    const int n4 = d >> 2, per = (n4 + nslices - 1) / nslices, end = min(n4, (ks + 1) * per);
+    float4 acc[2][NT];       // pieces of even and of odd place
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) acc[h][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](int c, float4 (&a)[NT]) {
+      const float4 v = __ldcg(xr + c);     // (x may be the output of the kernel before this one)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const float4 w = __ldg(w4 + (size_t)min(8 * j + e0, E - 1) * n4 + c);
+        a[j].x = fmaf(v.x, w.x, a[j].x);
+        a[j].y = fmaf(v.y, w.y, a[j].y);
+        a[j].z = fmaf(v.z, w.z, a[j].z);
+        a[j].w = fmaf(v.w, w.w, a[j].w);
+      }
+    };
+    int c = ks * per;
+#pragma unroll 2
+    for (; c + 1 < end; c += 2) {
+      add(c, acc[0]);
+      add(c + 1, acc[1]);
+    }
+    if (c < end) add(c, acc[0]);
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+      s_part[((size_t)ks * 16 + tok) * ET + 8 * j + e0] =
+          ((acc[0][j].x + acc[1][j].x) + (acc[0][j].y + acc[1][j].y)) +
+          ((acc[0][j].z + acc[1][j].z) + (acc[0][j].w + acc[1][j].w));
+  } else {
     const int tg = warp % gp2, ks = warp / gp2;
     if (tg < ngroups) {
       const int tok0 = tg * 16;
@@ -174,7 +212,7 @@ front_small_body(float* smem, const int blk, const int nblk,
   __syncthreads();
   // the first batch of row copies: the loads do not depend on the routing, so they are
   // issued now and wait in registers until the destination rows are known
-  const int pieces = d >> 3;
+  const int pieces = d / kPiece;
   const int items = N * pieces;
   const uint4* src = reinterpret_cast<const uint4*>(x);
   constexpr int kInFlight = 4;
@@ -193,7 +231,14 @@ front_small_body(float* smem, const int blk, const int nblk,
   for (int i = tid; i < N * E; i += kThreads) {
     const int tok = i / E, e = i - tok * E;
     float s = 0.f;
-    for (int ks = 0; ks < nslices; ++ks) s += s_part[((size_t)ks * 16 * gp2 + tok) * ET + e];
+    if constexpr (F32) {
+      float q[8];
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) q[ks] = s_part[((size_t)ks * 16 + tok) * ET + e];
+      s = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+    } else {
+      for (int ks = 0; ks < nslices; ++ks) s += s_part[((size_t)ks * 16 * gp2 + tok) * ET + e];
+    }
     s += s_bias[e];
     s_logit[tok * ld + e] = s;
     if (out_logits != nullptr && writer) out_logits[i] = s;

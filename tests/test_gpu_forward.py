@@ -72,6 +72,26 @@ def test_tiny_fixture_from_reference(cuda_device):
     assert abs(float(aux) - float(z["aux"])) <= 1e-6
 
 
+@pytest.mark.parametrize("N,d,E,k", [(1, 8, 5, 2), (16, 72, 8, 2), (17, 512, 9, 1), (129, 264, 16, 5), (300, 2048, 32, 4),
+                                     (2047, 64, 8, 2), (2048, 64, 17, 2)])
+def test_fp32_routing_in_one_launch(cuda_device, N, d, E, k):
+    """Rows, counts and copies as the dispatch kernel lays the same choices out, twice on one workspace; logits against
+    64 bits (chains of at most 32 products and a tree: 2^-24 times a few)."""
+    params = synthetic.make_params(d, E, 8, seed=N + E)
+    params["gate_b"] = torch.randn(E, generator=torch.Generator().manual_seed(E)) * 0.3
+    x = torch.randn(N, d, generator=torch.Generator().manual_seed(N))
+    m = build(params, d, E, 8, k, torch.float32, cuda_device)
+    for _ in range(2):
+        last, _ = check_against_oracle(m, params, x, k, torch.float32, cuda_device)
+    ref = torch.nn.functional.linear(x.double(), params["gate_w"].double(), params["gate_b"].double())
+    assert (last["logits"].double() - ref).norm() <= 3e-7 * ref.norm()
+    disp = helpers.dispatch(x.to(cuda_device), m.last["idx"], E)
+    perm = m._view("perm", torch.float32, (N * k, d))
+    assert torch.equal(perm, disp["perm"])
+    for name in ("offsets", "row_of", "cnt_slot"):
+        assert torch.equal(m.last[name], disp[name]), name
+
+
 SMALL = [
     # N, d, E, f, k
     (1, 64, 8, 128, 2), (2, 64, 8, 128, 2), (3, 64, 8, 128, 2), (127, 64, 8, 128, 2),
