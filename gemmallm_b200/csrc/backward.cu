@@ -11,16 +11,19 @@
 //                    same pass dWg = dlogits^T x, dbg = sum dlogits                 (model.py:206)
 //   combine_dx       dx[t] = the sum of its rows' gradients + dlogits[t] Wg    (model.py:248-253, 206)
 //   colsum           bias gradients per expert
+// They start under programmatic dependent launch (each launch cost 1.5 to 2.9 us behind the kernel before it) and read
+// what that kernel may have written through L2, behind pdl_wait.
 #include "common.cuh"
 
 namespace moe {
 
 namespace {
 
-__global__ void pair_of_kernel(const int32_t* __restrict__ row_of, int64_t M, int32_t* __restrict__ pair_of) {
+__global__ void pair_of_kernel(const int32_t* row_of, int64_t M, int32_t* __restrict__ pair_of) {
+  pdl_wait();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p < M) {
-    const int r = row_of[p];
+    const int r = __ldcg(&row_of[p]);
     if (r >= 0) pair_of[r] = (int32_t)p;
   }
 }
@@ -28,16 +31,16 @@ __global__ void pair_of_kernel(const int32_t* __restrict__ row_of, int64_t M, in
 // One warp per sorted row. Rows behind the last expert's (pairs whose router index was out of range, such as those of
 // a token with NaN logits, have none) belong to no pair, and pair_of says nothing about them.
 __global__ void __launch_bounds__(256)
-combine_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y,
-                   const int32_t* __restrict__ pair_of, const int32_t* __restrict__ offsets, int E,
-                   const float* __restrict__ w, int64_t M, int d, int k, __nv_bfloat16* __restrict__ dy,
+combine_bwd_kernel(const __nv_bfloat16* dout, const __nv_bfloat16* y, const int32_t* pair_of, const int32_t* offsets,
+                   int E, const float* w, int64_t M, int d, int k, __nv_bfloat16* __restrict__ dy,
                    float* __restrict__ dw) {
   const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (r >= M || r >= offsets[E]) return;
-  const int p = pair_of[r];
+  pdl_wait();
+  if (r >= M || r >= __ldcg(&offsets[E])) return;
+  const int p = __ldcg(&pair_of[r]);
   const int64_t t = p / k;
-  const float wp = w[p];
+  const float wp = __ldcg(&w[p]);
   float dot = 0.f;
   for (int c = lane * 8; c < d; c += 256) {
     float g[8], yv[8], o[8];
@@ -61,7 +64,7 @@ combine_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* 
 //   dl[e] = p[e] * (dp[e] - sum_e' p[e'] dp[e'])
 template <int PER>
 __device__ __forceinline__ void token_dlogits(const float* __restrict__ logits, const int32_t* __restrict__ idx,
-                                              const float* __restrict__ w, const float* __restrict__ dw,
+                                              const float* __restrict__ w, const float* dw,
                                               const int32_t* __restrict__ cnt0, float aux_c, int64_t t, int E, int k,
                                               int lane, float (&dl)[PER]) {
   float p[PER], dp[PER];
@@ -85,7 +88,7 @@ __device__ __forceinline__ void token_dlogits(const float* __restrict__ logits, 
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   // total of the chosen probabilities and sum_i dw_i w_i (every lane computes them: k <= 8)
   float total = 0.f, dww = 0.f;
-  for (int j = 0; j < k; ++j) dww = fmaf(dw[t * k + j], w[t * k + j], dww);
+  for (int j = 0; j < k; ++j) dww = fmaf(__ldcg(&dw[t * k + j]), w[t * k + j], dww);
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     const int e = lane + 32 * i;
@@ -103,7 +106,7 @@ __device__ __forceinline__ void token_dlogits(const float* __restrict__ logits, 
   }
   for (int j = 0; j < k; ++j) {
     const int e = idx[t * k + j];
-    const float dv = (dw[t * k + j] - dww) / total;
+    const float dv = (__ldcg(&dw[t * k + j]) - dww) / total;
     if ((e & 31) == lane) {
 #pragma unroll
       for (int i = 0; i < PER; ++i)
@@ -130,7 +133,7 @@ constexpr int kDlCols = 1024;    // columns of a block, four per thread
 template <int PER>
 __global__ void __launch_bounds__(256)
 router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ idx,
-                  const float* __restrict__ w, const float* __restrict__ dw,
+                  const float* __restrict__ w, const float* dw,
                   const int32_t* __restrict__ cnt0, float grad_aux_host, const float* __restrict__ grad_aux_dev,
                   const __nv_bfloat16* __restrict__ x, int64_t N, int d, int E, int k, int tokens_per_block,
                   float* __restrict__ dl_out, float* __restrict__ part, float* __restrict__ part_b) {
@@ -140,6 +143,7 @@ router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ 
   const int c = blockIdx.x * kDlCols + tid * 4;
   const int64_t t_begin = (int64_t)blockIdx.y * tokens_per_block;
   const int64_t t_end = min(t_begin + tokens_per_block, N);
+  pdl_wait();
   const float grad_aux = grad_aux_dev != nullptr ? __ldg(grad_aux_dev) : grad_aux_host;
   const float aux_c = grad_aux * (float)E / ((float)N * (float)N);
   const bool store_dl = blockIdx.x == 0 && blockIdx.z == 0;
@@ -199,18 +203,19 @@ router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ 
 
 // out[i] = sum over `ranges` of part[r][i], in order; eight groups of 32 threads take every eighth.
 __global__ void __launch_bounds__(256)
-router_bwd_finish_kernel(const float* __restrict__ part, const float* __restrict__ part_b, int ranges, int64_t n,
+router_bwd_finish_kernel(const float* part, const float* part_b, int ranges, int64_t n,
                          int E, __nv_bfloat16* __restrict__ dWg, __nv_bfloat16* __restrict__ dbg) {
   __shared__ float s_sum[8][33];
   const int grp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool bias = blockIdx.x == gridDim.x - 1;
+  pdl_wait();
   for (int64_t i0 = bias ? 0 : (int64_t)blockIdx.x * 32; i0 < (bias ? (int64_t)E : n); i0 += bias ? 32 : n) {
     const float* p = bias ? part_b : part;
     const int64_t len = bias ? (int64_t)E : n, i = i0 + lane;
     float sum = 0.f;
     if (i < len) {
 #pragma unroll 4
-      for (int r = grp; r < ranges; r += 8) sum += p[(size_t)r * len + i];
+      for (int r = grp; r < ranges; r += 8) sum += __ldcg(&p[(size_t)r * len + i]);
     }
     s_sum[grp][lane] = sum;
     __syncthreads();
@@ -295,19 +300,15 @@ combine_dx_kernel(const __nv_bfloat16* __restrict__ dxs, const int32_t* __restri
     if (t0 + u < N) store8(dx + (t0 + u) * d + c, acc[u]);
 }
 
-__global__ void iota_kernel(int32_t* __restrict__ p, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = (int32_t)i;
-}
-
 // Partial column sums: one block per 256-row tile of an expert (blockIdx.x, which alone counts beyond 65535: tiles over
 // the experts in order, as the grouped products count them) and 64 columns (blockIdx.y); eight threads cover a row's 128 bytes,
 // 32 such groups take every 32nd row, eight loads in flight each.
 __global__ void __launch_bounds__(256)
-colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__ offsets, int E, int C,
+colsum_kernel(const __nv_bfloat16* src, const int32_t* offsets, int E, int C,
               float* __restrict__ part) {
   __shared__ float s_part[32][65];
   __shared__ int s_row0, s_row1;
+  pdl_wait();
   if (threadIdx.x == 0) {
     int tile = blockIdx.x, r0 = 0, r1 = 0;
     for (int e = 0; e < E; ++e) {
@@ -335,7 +336,7 @@ colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int r = r0 + lane_r + 32 * q;
-      v[q] = r < r1 ? __ldg(reinterpret_cast<const uint4*>(src + (size_t)r * C + c)) : make_uint4(0, 0, 0, 0);
+      v[q] = r < r1 ? __ldcg(reinterpret_cast<const uint4*>(src + (size_t)r * C + c)) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -364,11 +365,12 @@ colsum_kernel(const __nv_bfloat16* __restrict__ src, const int32_t* __restrict__
 // db[e][c] = sum of the expert's slots of part (`slots` per 256-row tile), in order: eight groups of
 // 32 threads take every eighth slot.
 __global__ void __launch_bounds__(256)
-colsum_finish_kernel(const float* __restrict__ part, int slots, const int32_t* __restrict__ offsets, int C,
+colsum_finish_kernel(const float* part, int slots, const int32_t* offsets, int C,
                      __nv_bfloat16* __restrict__ db) {
   __shared__ float s_sum[8][33];
   __shared__ int s_first, s_count;
   const int e = blockIdx.y;
+  pdl_wait();
   if (threadIdx.x == 0) {
     int first = 0;
     for (int i = 0; i < e; ++i) first += (offsets[i + 1] - offsets[i] + 255) / 256;
@@ -381,7 +383,7 @@ colsum_finish_kernel(const float* __restrict__ part, int slots, const int32_t* _
   if (col < C) {
     const float* p = part + (size_t)s_first * C + col;
 #pragma unroll 4
-    for (int i = grp; i < s_count; i += 8) sum += p[(size_t)i * C];
+    for (int i = grp; i < s_count; i += 8) sum += __ldcg(&p[(size_t)i * C]);
   }
   s_sum[grp][threadIdx.x & 31] = sum;
   __syncthreads();
@@ -399,18 +401,16 @@ unsigned blocks_for(int64_t n, int per) { return (unsigned)((n + per - 1) / per)
 
 int launch_pair_of(const int32_t* row_of, int64_t M, int32_t* pair_of, cudaStream_t s) {
   if (M == 0) return 0;
-  pair_of_kernel<<<blocks_for(M, 256), 256, 0, s>>>(row_of, M, pair_of);
-  MOE_CUDA_CHECK(cudaGetLastError());
+  MOE_CUDA_CHECK(launch_pdl(pair_of_kernel, dim3(blocks_for(M, 256)), dim3(256), 0, s, row_of, M, pair_of));
   return 0;
 }
 
 int launch_combine_bwd(const void* dout, const void* y, const int32_t* pair_of, const int32_t* offsets, int E,
                        const float* w, int64_t M, int d, int k, void* dy, float* dw, cudaStream_t s) {
   if (M == 0) return 0;
-  combine_bwd_kernel<<<blocks_for(M, 8), 256, 0, s>>>(
-      static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(y), pair_of, offsets, E, w,
-      M, d, k, static_cast<__nv_bfloat16*>(dy), dw);
-  MOE_CUDA_CHECK(cudaGetLastError());
+  MOE_CUDA_CHECK(launch_pdl(combine_bwd_kernel, dim3(blocks_for(M, 8)), dim3(256), 0, s,
+                            static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(y), pair_of,
+                            offsets, E, w, M, d, k, static_cast<__nv_bfloat16*>(dy), dw));
   return 0;
 }
 
@@ -439,15 +439,12 @@ int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, c
   float* part_b = scratch + (size_t)ranges * E * d;
   auto fn = E <= 32 ? router_bwd_kernel<1> : (E <= 64 ? router_bwd_kernel<2> : router_bwd_kernel<kMaxExperts / 32>);
   const dim3 grid((d + kDlCols - 1) / kDlCols, (unsigned)ranges, (E + kDlExperts - 1) / kDlExperts);
-  fn<<<grid, 256, 0, s>>>(logits, idx, w, dw, cnt0, grad_aux, grad_aux_dev, static_cast<const __nv_bfloat16*>(x), N, d,
-                          E, k, (int)per, dl, scratch, part_b);
-  MOE_CUDA_CHECK(cudaGetLastError());
+  MOE_CUDA_CHECK(launch_pdl(fn, grid, dim3(256), 0, s, logits, idx, w, dw, cnt0, grad_aux, grad_aux_dev,
+                            static_cast<const __nv_bfloat16*>(x), N, d, E, k, (int)per, dl, scratch, part_b));
   if (dWg == nullptr && dbg == nullptr) return 0;
   const int64_t n = (int64_t)E * d;
-  router_bwd_finish_kernel<<<blocks_for(n, 32) + 1, 256, 0, s>>>(scratch, part_b, (int)ranges, n, E,
-                                                                static_cast<__nv_bfloat16*>(dWg),
-                                                                static_cast<__nv_bfloat16*>(dbg));
-  MOE_CUDA_CHECK(cudaGetLastError());
+  MOE_CUDA_CHECK(launch_pdl(router_bwd_finish_kernel, dim3(blocks_for(n, 32) + 1), dim3(256), 0, s, scratch, part_b,
+                            (int)ranges, n, E, static_cast<__nv_bfloat16*>(dWg), static_cast<__nv_bfloat16*>(dbg)));
   return 0;
 }
 
@@ -461,27 +458,18 @@ int launch_combine_dx(const void* dxs, const int32_t* row_of, const float* dl, c
   return 0;
 }
 
-int launch_iota(int32_t* p, int64_t n, cudaStream_t s) {
-  if (n == 0) return 0;
-  iota_kernel<<<blocks_for(n, 256), 256, 0, s>>>(p, n);
-  MOE_CUDA_CHECK(cudaGetLastError());
-  return 0;
-}
-
 int launch_colsum_finish(const float* part, int slots, const int32_t* offsets, int E, int C, void* db,
                          cudaStream_t s) {
-  colsum_finish_kernel<<<dim3((C + 31) / 32, E), 256, 0, s>>>(part, slots, offsets, C,
-                                                             static_cast<__nv_bfloat16*>(db));
-  MOE_CUDA_CHECK(cudaGetLastError());
+  MOE_CUDA_CHECK(launch_pdl(colsum_finish_kernel, dim3((C + 31) / 32, E), dim3(256), 0, s, part, slots, offsets, C,
+                            static_cast<__nv_bfloat16*>(db)));
   return 0;
 }
 
 int launch_colsum(const void* src, const int32_t* offsets, int64_t M, int E, int C, float* part, void* db,
                   cudaStream_t s) {
   const unsigned tiles = blocks_for(M, 256) + (unsigned)E;    // at least as many as there are
-  colsum_kernel<<<dim3(tiles, (C + 63) / 64), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(src), offsets, E, C,
-                                                            part);
-  MOE_CUDA_CHECK(cudaGetLastError());
+  MOE_CUDA_CHECK(launch_pdl(colsum_kernel, dim3(tiles, (C + 63) / 64), dim3(256), 0, s,
+                            static_cast<const __nv_bfloat16*>(src), offsets, E, C, part));
   return launch_colsum_finish(part, 1, offsets, E, C, db, s);
 }
 

@@ -270,7 +270,7 @@ struct TrainArgs {
   __nv_bfloat16* gu;
   uint8_t* mask;            // [M, f / 8] one bit per element of h, set = kept
   float* col_part;          // [2 * m-tiles, 2f], backward only
-  const int32_t* pair_of;   // [M] token * k + slot of every sorted row
+  const int32_t* pair_of;   // [M] token * k + slot of every sorted row; nullptr: the row itself
   uint32_t thresh;          // p * 2^32; 0 keeps everything
   float scale;
   uint32_t seed_lo, seed_hi;
@@ -378,7 +378,6 @@ int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, c
                       int64_t N, int d, int E, int k, float* dl, float* scratch, void* dWg, void* dbg, cudaStream_t s);
 int launch_combine_dx(const void* dxs, const int32_t* row_of, const float* dl, const void* Wg, int64_t N, int d, int E,
                       int k, void* dx, cudaStream_t s);
-int launch_iota(int32_t* p, int64_t n, cudaStream_t s);
 // Bias gradients: column sums of src [M, C] over every expert's rows; part as TrainArgs::col_part.
 int launch_colsum(const void* src, const int32_t* offsets, int64_t M, int E, int C, float* part, void* db,
                   cudaStream_t s);

@@ -6,14 +6,17 @@
 // the activations instead (two products with one side of the rank's width, no G where the base weights are frozen)
 // is as exact, but a step then rounds elsewhere, and after one SGD step the two ways are 1.0e-2 of the outputs
 // apart (2-norm, 14912 rows, d 1024, f 4096, rank 16), where a step repeated the same way differs by nothing.
-// Three launches for both Linears of a run of experts, bound by reading G twice:
-//   lora_rows_kernel    Q = G A^T, `in` cut into ranges (partial sums): rows of G are the 16-row operand of
-//                       mma.sync, straight from global memory; A waits in shared memory
-//   lora_cols_kernel    P = G^T B over segments of G's rows: G^T fragments by transposing ldmatrix
+// Two launches for both Linears of a run of experts, bound by reading G twice:
+//   lora_products_kernel  blocks of two kinds, side by side:
+//     rows  Q = G A^T, `in` cut into ranges (partial sums): rows of G are the 16-row operand of
+//           mma.sync, straight from global memory; A waits in shared memory
+//     cols  P = G^T B over segments of G's rows: G^T fragments by transposing ldmatrix, the next tile of G
+//           requested before the products of this one
 //   lora_finish_kernel  sums over ranges and segments in order, the bias terms, scale, rounding
-// (A step of the dense feed-forward at 1632 rows, d 1024, f 4096: 277 us, 246 us from the activations.)
+// (Two kernels one after the other, without the request ahead and with one thread a rank for B^T g, took 9 + 24 us
+// for both Linears at d 1024, f 4096, rank 16, with launches 11 + 26 + 10; now 15 + 7.)
+// (A step of the dense feed-forward at 1632 rows, d 1024, f 4096: 239 us.)
 // Products of bf16 are exact in fp32 and all sums are fp32, so the only rounding behind G is that of the results.
-#include <algorithm>
 #include "common.cuh"
 #include "internal.h"
 
@@ -23,8 +26,8 @@ namespace {
 
 constexpr int kRank = 16;          // ranks in steps of 16, padded with zeros
 constexpr int kRowTile = 64;
-constexpr int kRange = 512;        // contraction range of a block of lora_rows_kernel
-constexpr int kSegRows = 256;      // rows of G of a block of lora_cols_kernel
+constexpr int kRange = 512;        // contraction range of a block of rows
+constexpr int kSegRows = 256;      // rows of G of a block of columns
 constexpr int kColTile = 128;
 constexpr int kWPitch = kRange + 8;
 constexpr int kXPitch = kColTile + 8;
@@ -45,7 +48,8 @@ struct Linear {
 struct Jobs {
   Linear lin[2];
   int E;
-  unsigned first[2];               // blocks of Linear 0 and of both, for the kernel that gets this
+  unsigned db[2], da[2];            // the same for the finishing kernel: dB and db of both, then dA and da
+  unsigned cols[2], rows[2];       // where each Linear's blocks end: first all `cols` blocks (the longer ones), then `rows`
 };
 
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -64,16 +68,16 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* 
                : "memory");
 }
 
-// blocks (Linear, expert, row tile, range) x rank steps; q[range][e][row][r] = G[row, range] . A[r, range]
-__global__ void __launch_bounds__(256)
-lora_rows_kernel(const __grid_constant__ Jobs jobs) {
-  __shared__ __align__(16) __nv_bfloat16 s_w[kRank * kWPitch];
-  __shared__ float s_red[4][32][8];
-  const int l = blockIdx.x >= jobs.first[0] ? 1 : 0;
-  const Linear& L = jobs.lin[l];
+constexpr int kRowsSmem = kRank * kWPitch * 2 + 4 * 32 * 8 * 4;
+constexpr int kColsSmem = kRowTile * kXPitch * 2 + kRowTile * kSPitch * 2;
+constexpr int kProductsSmem = kRowsSmem > kColsSmem ? kRowsSmem : kColsSmem;
+
+// block b of a Linear's (expert, row tile, range) x rank steps; q[range][e][row][r] = G[row, range] . A[r, range]
+__device__ __forceinline__ void rows_block(const Linear& L, int E, unsigned b, unsigned char* smem) {
+  __nv_bfloat16* s_w = reinterpret_cast<__nv_bfloat16*>(smem);                             // [kRank][kWPitch]
+  float (*s_red)[32][8] = reinterpret_cast<float (*)[32][8]>(smem + kRank * kWPitch * 2);    // [4]
   const int n0 = blockIdx.y * kRank;
   if (n0 >= L.R) return;               // the other Linear's rank is larger
-  const unsigned b = blockIdx.x - (l ? jobs.first[0] : 0u);
   const int range = (int)(b % L.ranges), tile = (int)(b / L.ranges % L.row_tiles), e = (int)(b / L.ranges / L.row_tiles);
   const int C = L.in, k0 = range * kRange, row0 = tile * kRowTile, rows = min(kRowTile, L.out - row0);
   const int klen = min(kRange, C - k0);             // a multiple of 8
@@ -101,8 +105,8 @@ lora_rows_kernel(const __grid_constant__ Jobs jobs) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int p = 4 * (c0 + u) + t;
-      a[u] = p < pieces ? __ldg(xa + p) : zero;
-      b4[u] = p < pieces ? __ldg(xb + p) : zero;
+      a[u] = p < pieces ? __ldcg(xa + p) : zero;
+      b4[u] = p < pieces ? __ldcg(xb + p) : zero;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -123,7 +127,7 @@ lora_rows_kernel(const __grid_constant__ Jobs jobs) {
   }
   __syncthreads();
   if (half == 0) {
-    float* out = L.q + (((size_t)range * jobs.E + e) * L.out + row0) * L.R + n0;
+    float* out = L.q + (((size_t)range * E + e) * L.out + row0) * L.R + n0;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
 #pragma unroll
@@ -135,17 +139,13 @@ lora_rows_kernel(const __grid_constant__ Jobs jobs) {
   }
 }
 
-// blocks (Linear, expert, segment, column tile) x rank steps;
+// block b of a Linear's (expert, segment, column tile) x rank steps;
 // p[segment][e][c][r] = sum over the segment's rows of G[row, c] * B[row, r]
-__global__ void __launch_bounds__(256)
-lora_cols_kernel(const __grid_constant__ Jobs jobs) {
-  __shared__ __align__(16) __nv_bfloat16 s_x[kRowTile * kXPitch];
-  __shared__ __align__(16) __nv_bfloat16 s_s[kRowTile * kSPitch];
-  const int l = blockIdx.x >= jobs.first[0] ? 1 : 0;
-  const Linear& L = jobs.lin[l];
+__device__ __forceinline__ void cols_block(const Linear& L, int E, unsigned b, unsigned char* smem) {
+  __nv_bfloat16* s_x = reinterpret_cast<__nv_bfloat16*>(smem);       // [kRowTile][kXPitch]
+  __nv_bfloat16* s_s = s_x + kRowTile * kXPitch;                      // [kRowTile][kSPitch]
   const int n0 = blockIdx.y * kRank;
   if (n0 >= L.R) return;               // the other Linear's rank is larger
-  const unsigned b = blockIdx.x - (l ? jobs.first[0] : 0u);
   const int ct = (int)(b % L.col_tiles), seg = (int)(b / L.col_tiles % L.segs), e = (int)(b / L.col_tiles / L.segs);
   const int C = L.in, c0 = ct * kColTile, row0 = seg * kSegRows, rows = min(kSegRows, L.out - row0);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -154,30 +154,44 @@ lora_cols_kernel(const __grid_constant__ Jobs jobs) {
   const __nv_bfloat16* gb = L.g + (size_t)e * L.out + row0;
   float acc[2][4] = {};
   float psum = 0.f;
+  // G: 64 rows x 128 columns at a time, 16 bytes of four rows a thread
+  uint4 v[4];
+  auto request = [&](int r0) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = tid + u * 256, rr = i >> 4, c = (i & 15) * 8;
+      v[u] = r0 + rr < rows && c0 + c < C ? __ldcg(reinterpret_cast<const uint4*>(G + (size_t)(r0 + rr) * C + c))
+                                          : make_uint4(0, 0, 0, 0);
+    }
+  };
+  request(0);
   for (int r0 = 0; r0 < rows; r0 += kRowTile) {
     __syncthreads();
     // B: four threads per row, four ranks each (rows of B are as wide as the rank: no wider loads)
     {
       const int rr = tid >> 2, q = (tid & 3) * 4;
-      __nv_bfloat16 v[4];
+      __nv_bfloat16 w[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        v[i] = r0 + rr < rows && n0 + q + i < L.rank ? B[(size_t)(r0 + rr) * L.rank + q + i] : __float2bfloat16_rn(0.f);
+        w[i] = r0 + rr < rows && n0 + q + i < L.rank ? B[(size_t)(r0 + rr) * L.rank + q + i] : __float2bfloat16_rn(0.f);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) s_s[rr * kSPitch + q + i] = v[i];
+      for (int i = 0; i < 4; ++i) s_s[rr * kSPitch + q + i] = w[i];
     }
-    // G: 64 rows x 128 columns
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int i = tid + u * 256, rr = i >> 4, c = (i & 15) * 8;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r0 + rr < rows && c0 + c < C) v = __ldg(reinterpret_cast<const uint4*>(G + (size_t)(r0 + rr) * C + c));
-      *reinterpret_cast<uint4*>(s_x + rr * kXPitch + c) = v;
+      const int i = tid + u * 256;
+      *reinterpret_cast<uint4*>(s_x + (i >> 4) * kXPitch + (i & 15) * 8) = v[u];
     }
+    if (r0 + kRowTile < rows) request(r0 + kRowTile);
     __syncthreads();
-    if (ct == 0 && tid < kRank)        // this block also forms B^T g
-      for (int rr = 0; rr < kRowTile && r0 + rr < rows; ++rr)
-        psum = fmaf(__bfloat162float(s_s[rr * kSPitch + tid]), __bfloat162float(gb[r0 + rr]), psum);
+    if (ct == 0) {       // this block also forms B^T g: sixteen threads a rank, four rows each
+      const int r = tid & 15, q = (tid >> 4) * 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (r0 + q + i < rows)
+          psum = fmaf(__bfloat162float(s_s[(q + i) * kSPitch + r]),
+                      __bfloat162float(__ushort_as_bfloat16(__ldcg(reinterpret_cast<const unsigned short*>(gb + r0 + q + i)))), psum);
+    }
 #pragma unroll
     for (int kk = 0; kk < kRowTile / 16; ++kk) {
       uint32_t a[4], w[4];
@@ -191,7 +205,7 @@ lora_cols_kernel(const __grid_constant__ Jobs jobs) {
     }
   }
   const int g = lane >> 2, t = lane & 3;
-  float* out = L.p + (((size_t)seg * jobs.E + e) * C + c0 + warp * 16) * L.R + n0;
+  float* out = L.p + (((size_t)seg * E + e) * C + c0 + warp * 16) * L.R + n0;
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     if (c0 + warp * 16 + g < C)
@@ -199,38 +213,84 @@ lora_cols_kernel(const __grid_constant__ Jobs jobs) {
     if (c0 + warp * 16 + g + 8 < C)
       *reinterpret_cast<float2*>(out + (size_t)(g + 8) * L.R + 8 * j + 2 * t) = make_float2(acc[j][2], acc[j][3]);
   }
-  if (ct == 0 && tid < kRank) L.pb[((size_t)seg * jobs.E + e) * L.R + n0 + tid] = psum;
+  if (ct == 0) {
+    __syncthreads();
+    float* s_psum = reinterpret_cast<float*>(smem);
+    s_psum[tid] = psum;
+    __syncthreads();
+    if (tid < kRank) {
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sum += s_psum[i * 16 + tid];
+      L.pb[((size_t)seg * E + e) * L.R + n0 + tid] = sum;
+    }
+  }
 }
 
-// blocks over the larger of out * rank and in * rank x (Linear, dB or dA) x experts
+__global__ void __launch_bounds__(256)
+lora_products_kernel(const __grid_constant__ Jobs jobs) {
+  __shared__ __align__(16) unsigned char smem[kProductsSmem];
+  pdl_wait();
+  const unsigned b = blockIdx.x;
+  if (b < jobs.cols[0]) cols_block(jobs.lin[0], jobs.E, b, smem);
+  else if (b < jobs.cols[1]) cols_block(jobs.lin[1], jobs.E, b - jobs.cols[0], smem);
+  else if (b < jobs.rows[0]) rows_block(jobs.lin[0], jobs.E, b - jobs.cols[1], smem);
+  else rows_block(jobs.lin[1], jobs.E, b - jobs.rows[0], smem);
+}
+
+constexpr int kFinishCols = 16;
+
+// `n` values `step` apart, added in order, eight requested at a time.
+__device__ __forceinline__ float sum_of(const float* p, int n, size_t step) {
+  float sum = 0.f;
+  for (int k = 0; k < n; k += 8) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __ldcg(p + (size_t)min(k + i, n - 1) * step);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (k + i < n) sum += v[i];
+  }
+  return sum;
+}
+
+// blocks: 256 elements of dB, or 16 columns x 16 ranks of dA (its partial sums lie by column, dA by rank: through shared
+// memory), of one expert
 __global__ void __launch_bounds__(256)
 lora_finish_kernel(const __grid_constant__ Jobs jobs, float scale) {
-  const Linear& L = jobs.lin[blockIdx.y >> 1];
-  const int e = blockIdx.z;
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if ((blockIdx.y & 1) == 0) {         // dB [out][rank], db [out]
+  __shared__ float s_t[kRank][kFinishCols + 1];
+  const unsigned bx = blockIdx.x;
+  const bool is_a = bx >= jobs.db[1];
+  const int l = is_a ? (bx >= jobs.da[0] ? 1 : 0) : (bx >= jobs.db[0] ? 1 : 0);
+  const Linear& L = jobs.lin[l];
+  const unsigned at = bx - (is_a ? (l ? jobs.da[0] : jobs.db[1]) : (l ? jobs.db[0] : 0u));
+  const int tid = threadIdx.x;
+  pdl_wait();
+  if (!is_a) {                         // dB [out][rank], db [out]
+    const unsigned per = ((unsigned)(L.out * L.rank) + 255) / 256;
+    const int e = (int)(at / per);
+    const int64_t i = (int64_t)(at % per) * 256 + tid;
     if (i >= (int64_t)L.out * L.rank) return;
     const int c = (int)(i / L.rank), r = (int)(i % L.rank);
     const size_t step = (size_t)jobs.E * L.out * L.R;
-    const float* q = L.q + ((size_t)e * L.out + c) * L.R + r;
-    float sum = 0.f;
-    for (int k = 0; k < L.ranges; ++k) sum += q[k * step];
+    const float sum = sum_of(L.q + ((size_t)e * L.out + c) * L.R + r, L.ranges, step);
     const float gc = __bfloat162float(L.g[(size_t)e * L.out + c]);
     const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(L.tab[(size_t)e * 3 + 1]);
     L.dB[(size_t)e * L.out * L.rank + i] = __float2bfloat16_rn(scale * fmaf(gc, __bfloat162float(a[r]), sum));
     if (r == 0) L.db[(size_t)e * L.out + c] = __float2bfloat16_rn(scale * gc);
   } else {                             // dA [rank][in], da [rank]
-    if (i >= (int64_t)L.in * L.rank) return;
-    const int c = (int)(i % L.in), r = (int)(i / L.in);
+    const int tiles = (L.in + kFinishCols - 1) / kFinishCols, steps = L.R / kRank;
+    const int c0 = (int)(at % tiles) * kFinishCols, n0 = (int)(at / tiles % steps) * kRank, e = (int)(at / tiles / steps);
     const size_t step = (size_t)jobs.E * L.in * L.R;
-    const float* p = L.p + ((size_t)e * L.in + c) * L.R + r;
-    float sum = 0.f;
-    for (int k = 0; k < L.segs; ++k) sum += p[k * step];
-    L.dA[(size_t)e * L.in * L.rank + i] = __float2bfloat16_rn(scale * sum);
-    if (c == 0) {
-      float ps = 0.f;
-      for (int k = 0; k < L.segs; ++k) ps += L.pb[((size_t)k * jobs.E + e) * L.R + r];
-      L.da[(size_t)e * L.rank + r] = __float2bfloat16_rn(scale * ps);
+    const int r = tid & 15, cc = tid >> 4;
+    s_t[r][cc] = sum_of(L.p + ((size_t)e * L.in + min(c0 + cc, L.in - 1)) * L.R + n0 + r, L.segs, step);
+    __syncthreads();
+    const int rr = tid / kFinishCols, c = tid % kFinishCols;
+    if (n0 + rr < L.rank && c0 + c < L.in)
+      L.dA[((size_t)e * L.rank + n0 + rr) * L.in + c0 + c] = __float2bfloat16_rn(scale * s_t[rr][c]);
+    if (c0 == 0 && tid < kRank && n0 + tid < L.rank) {
+      const float ps = sum_of(L.pb + (size_t)e * L.R + n0 + tid, L.segs, (size_t)jobs.E * L.R);
+      L.da[(size_t)e * L.rank + n0 + tid] = __float2bfloat16_rn(scale * ps);
     }
   }
 }
@@ -283,18 +343,16 @@ int launch_lora_grads(const void* const* tab, int d, int f, int all, const LoraR
   }
   const Linear &a = jobs.lin[0], &b = jobs.lin[1];
   const unsigned steps = (unsigned)((a.R > b.R ? a.R : b.R) / kRank);
-  jobs.first[0] = (unsigned)(a.row_tiles * a.ranges * E);
-  jobs.first[1] = jobs.first[0] + (unsigned)(b.row_tiles * b.ranges * E);
-  lora_rows_kernel<<<dim3(jobs.first[1], steps), 256, 0, s>>>(jobs);
-  MOE_CUDA_CHECK(cudaGetLastError());
-  jobs.first[0] = (unsigned)(a.segs * a.col_tiles * E);
-  jobs.first[1] = jobs.first[0] + (unsigned)(b.segs * b.col_tiles * E);
-  lora_cols_kernel<<<dim3(jobs.first[1], steps), 256, 0, s>>>(jobs);
-  MOE_CUDA_CHECK(cudaGetLastError());
-  int64_t widest = 0;
-  for (const Linear& L : jobs.lin) widest = std::max(widest, (int64_t)std::max(L.out, L.in) * L.rank);
-  lora_finish_kernel<<<dim3((unsigned)((widest + 255) / 256), 4, (unsigned)E), 256, 0, s>>>(jobs, run.scale);
-  MOE_CUDA_CHECK(cudaGetLastError());
+  jobs.cols[0] = (unsigned)(a.segs * a.col_tiles * E);
+  jobs.cols[1] = jobs.cols[0] + (unsigned)(b.segs * b.col_tiles * E);
+  jobs.rows[0] = jobs.cols[1] + (unsigned)(a.row_tiles * a.ranges * E);
+  jobs.rows[1] = jobs.rows[0] + (unsigned)(b.row_tiles * b.ranges * E);
+  MOE_CUDA_CHECK(launch_pdl(lora_products_kernel, dim3(jobs.rows[1], steps), dim3(256), 0, s, jobs));
+  unsigned at = 0;
+  for (int l = 0; l < 2; ++l) jobs.db[l] = at += (unsigned)((jobs.lin[l].out * jobs.lin[l].rank + 255) / 256 * E);
+  for (int l = 0; l < 2; ++l)
+    jobs.da[l] = at += (unsigned)((jobs.lin[l].in + kFinishCols - 1) / kFinishCols * (jobs.lin[l].R / kRank) * E);
+  MOE_CUDA_CHECK(launch_pdl(lora_finish_kernel, dim3(at), dim3(256), 0, s, jobs, run.scale));
   return 0;
 }
 

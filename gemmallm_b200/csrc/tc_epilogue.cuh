@@ -252,7 +252,7 @@ struct GegluTrain {
 // shared memory for the epilogue and to global memory for the backward pass.
 __device__ __forceinline__ void draw_mask(const TrainArgs& tr, int64_t row, bool row_ok, int n0, int Nout,
                                           uint32_t* s_row) {
-  const uint32_t pair = row_ok ? (uint32_t)__ldg(&tr.pair_of[row]) : 0u;
+  const uint32_t pair = tr.pair_of == nullptr ? (uint32_t)row : row_ok ? (uint32_t)__ldg(&tr.pair_of[row]) : 0u;
   uint32_t w[4];
 #pragma unroll
   for (int p = 0; p < 4; ++p) {

@@ -200,10 +200,8 @@ int moe_b200_experts_train(const void* x_sorted, const int32_t* offsets, const v
   if ((uintptr_t)train_ws & 1023) return set_error(MOE_B200_ERR_ALIGN, "training workspace must be 1024-byte aligned");
   char* tws = static_cast<char*>(train_ws);
   cudaStream_t s = (cudaStream_t)stream;
-  // row r is pair r: the dropout mask of element (r, c) depends on the row's position only
-  rc = launch_iota(reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]), M, s);
-  if (rc) return rc;
-  const TrainArgs tr = train_args(tws, to, dropout_p, seed);
+  TrainArgs tr = train_args(tws, to, dropout_p, seed);
+  tr.pair_of = nullptr;     // row r is pair r: the dropout mask of element (r, c) depends on the row's position only
   return launch_experts_tc2(x_sorted, offsets, plan, M, d, f, E, h, y, nullptr, status, s, &tr);
 }
 

@@ -224,6 +224,25 @@ def test_experts_fp32_tile_edges(cuda_device, rows, d, f):
     assert (y.cpu().double() - y_ref).norm() <= 4e-6 * y_ref.norm()
 
 
+# tiles of 64 rows x 256 columns that end early, one tile and several, ranks up to the largest
+@pytest.mark.parametrize("out_f,in_f,rank", [(1, 8, 1), (64, 256, 16), (65, 264, 5), (200, 520, 24), (63, 1032, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_lora_merge(cuda_device, out_f, in_f, rank, dtype):
+    g = torch.Generator().manual_seed(out_f + rank)
+    rnd = lambda *s: synthetic.round_to(torch.randn(*s, generator=g), dtype)
+    W, b, A, a, B, bl = rnd(out_f, in_f), rnd(out_f), rnd(rank, in_f), rnd(rank), rnd(out_f, rank), rnd(out_f)
+    dev = [t.to(dtype).to(cuda_device) for t in (W, b, A, a, B, bl)]
+    oW, ob = torch.full_like(dev[0], float("nan")), torch.full_like(dev[1], float("nan"))
+    check(lib.moe_b200_lora_merge(*[t.data_ptr() for t in dev], 1.3, out_f, in_f, rank, helpers.CODE[dtype],
+                                  oW.data_ptr(), ob.data_ptr(), helpers.stream(cuda_device)), "lora_merge")
+    scale = float(torch.tensor(1.3))
+    ref, refb = W.double() + scale * (B.double() @ A.double()), b.double() + scale * (B.double() @ a.double() + bl.double())
+    # fp32 sums of at most 65 products of size 1, then one rounding
+    eps = 2.0 ** -9 if dtype == torch.bfloat16 else 0.0
+    for got, want in ((oW, ref), (ob, refb)):
+        assert ((got.cpu().double() - want).abs() <= eps * want.abs() + 2e-5).all()
+
+
 # edges of the fp32 token tiles (16 and 160 tokens) and of the read-outs (64 and 256 of K), whole and with K over clusters
 # of two, four and eight CTAs, more tiles than SMs
 @pytest.mark.parametrize("rows,d,f", [([15, 16, 17, 159], 512, 2048), ([160, 161, 0, 321], 1024, 512), ([7], 1024, 136),
