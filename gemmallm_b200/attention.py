@@ -16,7 +16,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import _cabi
+from . import _cabi, _host
 from ._cabi import lib, check
 from .moe import _stream
 
@@ -92,16 +92,20 @@ class Attention(nn.Module):
         else:
             wq, bq, wo, bo = self.qkv.weight, self.qkv.bias, self.o.weight, self.o.bias
         x = tensor.contiguous()
+        mask = attention_mask
+        if mask is not None:
+            if mask.numel() != S * S:
+                raise NotImplementedError("one additive [S, S] mask for the whole batch is supported")
+            if mask.dtype != torch.float32 or mask.device != dev or not mask.is_contiguous():
+                mask = mask.reshape(S, S).to(device=dev, dtype=torch.float32).contiguous()
+        table = self._pos_table(dev)
+        done = _host.attention(x, wq, bq, self.gate.weight, self.gate.bias, wo, bo, table, mask, self.q_head, self.kv_head,
+                               self.head_dim, self.scaler)
+        if done is not None:
+            return done
         qkv = F.linear(x, wq, bq)
         gate = F.linear(x, self.gate.weight, self.gate.bias)          # [B,S,q_head] logits (model.py:139)
-        mask_ptr = None
-        if attention_mask is not None:
-            m = attention_mask
-            if m.numel() != S * S:
-                raise NotImplementedError("one additive [S, S] mask for the whole batch is supported")
-            mask = m.reshape(S, S).to(device=dev, dtype=torch.float32).contiguous()
-            mask_ptr = mask.data_ptr()
-        table = self._pos_table(dev)
+        mask_ptr = None if mask is None else mask.data_ptr()
         if table.shape[0] < S or table.shape[1] != 2 * self.head_dim:
             raise ValueError("the RoPE table is shorter than the sequence or has another head_dim")
         out = torch.empty(B, S, self.q_head * self.head_dim, dtype=tensor.dtype, device=dev)

@@ -17,6 +17,8 @@
 // does, from its forward to its backward, because the plan that it will use has their addresses.
 #include <Python.h>
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/autocast_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -24,6 +26,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/pybind.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include <algorithm>
@@ -1251,7 +1254,100 @@ PyType_Slot ffn_slots[] = {{Py_tp_new, reinterpret_cast<void*>(ffn_new)},
                            {0, nullptr}};
 PyType_Spec ffn_spec = {"gemmallm_b200._host.Ffn", sizeof(Ffn), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC, ffn_slots};
 
-PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
+// ---- the decoder layer's attention and first LayerNorm in inference --------------------------------
+// Nothing is bound or kept: every tensor comes with the call. None for what is left to the Python side (other classes of
+// tensors, modes that see Python calls, tracing, autocast). A layer call of one short sequence is 90 us of GPU work; with
+// its ten launches made from Python it took 119.
+
+bool plain_call() {
+  return !at::impl::torch_function_mode_enabled() && !torch::jit::tracer::isTracing() &&
+         !at::autocast::is_autocast_enabled(at::kCUDA);
+}
+
+// attention(x, qkv weight, bias, gate weight, bias, o weight, bias, table, mask or None, q heads, kv heads, head_dim, scaler)
+PyObject* host_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 13) {
+    PyErr_SetString(PyExc_TypeError, "attention() takes 13 arguments");
+    return nullptr;
+  }
+  const bool masked = args[8] != Py_None;
+  for (int i = 0; i < (masked ? 9 : 8); ++i)
+    if (!THPVariable_CheckExact(args[i])) Py_RETURN_NONE;
+  const long heads = PyLong_AsLong(args[9]), kv = PyLong_AsLong(args[10]), hd = PyLong_AsLong(args[11]);
+  const double scaler = PyFloat_AsDouble(args[12]);
+  if (PyErr_Occurred()) return nullptr;
+  auto t = [&](int i) -> const Tensor& { return THPVariable_Unpack(args[i]); };
+  const Tensor &x = t(0), &table = t(7);
+  if (!plain_call() || !x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() != 3 || !x.is_contiguous() || heads < 1 ||
+      kv < 1 || hd < 1)
+    Py_RETURN_NONE;
+  const int64_t B = x.size(0), S = x.size(1);
+  for (int i = 1; i < 7; ++i)
+    if (t(i).device() != x.device() || t(i).scalar_type() != at::kBFloat16) Py_RETURN_NONE;
+  if (t(1).dim() != 2 || t(1).size(0) != (heads + 2 * kv) * hd || t(3).dim() != 2 || t(3).size(0) != heads) Py_RETURN_NONE;
+  if (table.device() != x.device() || table.scalar_type() != at::kFloat || !table.is_contiguous() || table.dim() != 2 ||
+      table.size(0) < S || table.size(1) != 2 * hd)
+    Py_RETURN_NONE;
+  const float* mask = nullptr;
+  if (masked) {
+    if (t(8).device() != x.device() || t(8).scalar_type() != at::kFloat || !t(8).is_contiguous() || t(8).numel() != S * S)
+      Py_RETURN_NONE;
+    mask = t(8).const_data_ptr<float>();
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor result;
+  int rc = 0;
+  {
+    pybind11::gil_scoped_release no_gil;
+    const Tensor qkv = at::linear(x, t(1), t(2)), gate = at::linear(x, t(3), t(4));
+    const Tensor out = at::empty({B, S, heads * hd}, x.options());
+    void* stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+    rc = moe_b200_attention(qkv.const_data_ptr(), gate.const_data_ptr(), table.const_data_ptr<float>(), mask, B, (int)S,
+                            (int)heads, (int)kv, (int)hd, (float)scaler, out.data_ptr(), stream);
+    if (rc == 0) result = at::linear(out, t(5), t(6));
+  }
+  if (rc != 0) return fail(rc, "attention");
+  return THPVariable_Wrap(std::move(result));
+  END_HANDLE_TH_ERRORS
+}
+
+// layernorm(x, weight, bias, eps) by the library's row kernel, over the last dimension
+PyObject* host_layernorm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 4) {
+    PyErr_SetString(PyExc_TypeError, "layernorm(x, weight, bias, eps)");
+    return nullptr;
+  }
+  for (int i = 0; i < 3; ++i)
+    if (!THPVariable_CheckExact(args[i])) Py_RETURN_NONE;
+  const double eps = PyFloat_AsDouble(args[3]);
+  if (PyErr_Occurred()) return nullptr;
+  const Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]), &b = THPVariable_Unpack(args[2]);
+  const auto type = x.scalar_type();
+  if (!plain_call() || !x.is_cuda() || (type != at::kBFloat16 && type != at::kFloat) || x.dim() < 1 || !x.is_contiguous())
+    Py_RETURN_NONE;
+  const int64_t d = x.size(-1);
+  if (d < 8 || d % 8 != 0 || x.numel() == 0) Py_RETURN_NONE;
+  for (const Tensor* p : {&w, &b})
+    if (p->device() != x.device() || p->scalar_type() != type || !p->is_contiguous() || p->numel() != d) Py_RETURN_NONE;
+  if (at::GradMode::is_enabled() && (x.requires_grad() || w.requires_grad() || b.requires_grad())) Py_RETURN_NONE;
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = at::empty_like(x);
+  const int rc = moe_b200_layernorm(x.const_data_ptr(), w.const_data_ptr(), b.const_data_ptr(), (float)eps, x.numel() / d,
+                                    (int)d, type == at::kFloat ? MOE_B200_F32 : MOE_B200_BF16, out.data_ptr(),
+                                    c10::cuda::getCurrentCUDAStream(x.device().index()).stream());
+  if (rc == MOE_B200_ERR_ALIGN) Py_RETURN_NONE;      // tensors at an odd place
+  if (rc != 0) return fail(rc, "layernorm");
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef module_methods[] = {
+    {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(host_attention)), METH_FASTCALL, nullptr},
+    {"layernorm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(host_layernorm)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
 bool add_type(PyObject* m, const char* name, PyType_Spec* spec, PyTypeObject** keep = nullptr) {
   PyObject* t = PyType_FromSpec(spec);

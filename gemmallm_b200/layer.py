@@ -15,28 +15,19 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import _cabi
-from ._cabi import lib, check
+from . import _host
 from .attention import Attention
-from .moe import MOE, FeedForward, _stream
+from .moe import MOE, FeedForward
 
 
 def _layernorm(norm: nn.LayerNorm, x: torch.Tensor) -> torch.Tensor:
-    """norm(x) by the library's row kernel (moe_b200_layernorm) for contiguous bf16/fp32 CUDA
+    """norm(x) by the library's row kernel (moe_b200_layernorm) for bf16/fp32 CUDA
     tensors outside autograd; torch's own LayerNorm otherwise (training)."""
-    d = x.shape[-1]
-    if (not x.is_cuda or x.dtype not in (torch.bfloat16, torch.float32) or d % 8 != 0
-            or norm.weight is None or norm.bias is None or norm.weight.dtype != x.dtype
-            or (torch.is_grad_enabled() and (x.requires_grad or norm.weight.requires_grad))):
-        return norm(x)
-    xc = x.contiguous()
-    out = torch.empty_like(xc)
-    code = _cabi.BF16 if x.dtype == torch.bfloat16 else _cabi.F32
-    with torch.cuda.device(x.device):
-        check(lib.moe_b200_layernorm(xc.data_ptr(), norm.weight.data_ptr(), norm.bias.data_ptr(),
-                                     float(norm.eps), xc.numel() // d, d, code, out.data_ptr(),
-                                     _stream(x.device)), "layernorm")
-    return out
+    if x.is_cuda and norm.weight is not None and norm.bias is not None:
+        out = _host.layernorm(x.contiguous(), norm.weight, norm.bias, float(norm.eps))
+        if out is not None:
+            return out
+    return norm(x)
 
 
 class LLMLayer(nn.Module):

@@ -7,7 +7,7 @@ import weakref
 import pytest
 import torch
 
-from gemmallm_b200 import MOE, FeedForward, _host
+from gemmallm_b200 import MOE, Attention, FeedForward, _host
 from gemmallm_b200._cabi import MoeB200Error
 
 DT = torch.bfloat16
@@ -813,3 +813,54 @@ def test_adapters_at_an_address_that_others_had(cuda_device, kind):
                     p.data = new
                 held.append(new)
             assert p.data_ptr() == address
+
+
+# ---- the decoder layer's attention and LayerNorm ----------------------------------------------
+
+class Table(torch.nn.Module):
+    def __init__(self, n, hd):
+        super().__init__()
+        self.register_buffer("pos_emb", torch.randn(n, 2 * hd, generator=torch.Generator().manual_seed(2)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,S,heads,kv,ft", [(1, 1, 2, 1, False), (2, 37, 4, 4, True), (3, 128, 4, 2, False)])
+def test_attention_native_and_python_paths_agree(cuda_device, monkeypatch, B, S, heads, kv, ft):
+    torch.manual_seed(S)
+    m = Attention(D, 64, heads, kv, Table(128, 64)).to(device=cuda_device, dtype=DT).eval()
+    m.embedding.float()
+    x = rows(B * S, cuda_device).view(B, S, D)
+    causal = torch.full((S, S), float("-inf"), device=cuda_device).triu(1)
+    masks = [None, causal, causal.view(1, 1, S, S), causal.double(), causal.t().contiguous().t(), causal.cpu()]
+    inputs = [x, x.transpose(0, 1).contiguous().transpose(0, 1)]
+    with torch.no_grad():
+        native = [m(i, mask, ft) for i in inputs for mask in masks]
+        monkeypatch.setattr(_host, "attention", lambda *a: None)
+        same(native, [m(i, mask, ft) for i in inputs for mask in masks])
+        monkeypatch.undo()
+        with pytest.raises(NotImplementedError):
+            m(x, torch.zeros(S, S + 1, device=cuda_device))
+        with pytest.raises(ValueError):                                     # a table that is too short
+            m.embedding = Table(S - 1, 64).to(cuda_device)
+            m(x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [DT, torch.float32])
+def test_layernorm_native_and_left_alone(cuda_device, dtype):
+    norm = torch.nn.LayerNorm(72).to(device=cuda_device, dtype=dtype)
+    torch.nn.init.normal_(norm.weight)
+    x = torch.randn(5, 3, 72, generator=torch.Generator().manual_seed(3)).to(device=cuda_device, dtype=dtype)
+    args = (norm.weight, norm.bias, norm.eps)
+    assert _host.layernorm(x, *args) is None                                # gradients are wanted
+    with torch.no_grad():
+        got, want = _host.layernorm(x, *args), norm(x)
+        # a rounding of the result, and of the statistics
+        assert (got.float() - want.float()).abs().max() <= (2.0 ** -7 if dtype == DT else 1e-5) * want.abs().max()
+        assert _host.layernorm(x[..., :64], *args) is None                  # another width
+        assert _host.layernorm(x.half(), *args) is None
+        assert _host.layernorm(x[:0], *args) is None
+        odd = torch.empty(15 * 72 + 1, device=cuda_device, dtype=dtype)[1:].view(5, 3, 72).copy_(x)
+        assert _host.layernorm(odd, *args) is None                          # not on a 16-byte boundary
+        with torch.autocast("cuda"):
+            assert _host.layernorm(x, *args) is None
