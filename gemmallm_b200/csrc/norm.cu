@@ -53,9 +53,36 @@ norm_fold_kernel(const T* __restrict__ Wg, const T* __restrict__ bg, const T* __
 }
 
 // One warp per row: mean, biased variance around the mean, y = (x - mean) * rstd * gamma + beta,
-// as torch.nn.LayerNorm. Rows of up to 2048 elements stay in the lanes' registers between the
-// three steps (one pass over memory); longer rows are re-read (from L1).
-template <typename T>
+// as torch.nn.LayerNorm. Rows of up to 256 * KEEP elements stay in the lanes' registers between the
+// three steps, as they lie in memory (one pass over memory); longer rows (KEEP = 0) are re-read (from L1).
+// What bounds it is the loads in flight: kept as floats, and with room for 2048 at every width, a row took registers
+// for two blocks an SM (32768 rows of 1024 bf16: 41 us, now 24).
+template <typename T> struct RawPiece;      // eight elements
+template <> struct RawPiece<__nv_bfloat16> {
+  uint4 v;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void get(float (&o)[8]) const {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      o[2 * i] = bf16_lo(w[i]);
+      o[2 * i + 1] = bf16_hi(w[i]);
+    }
+  }
+};
+template <> struct RawPiece<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* p) {
+    a = *reinterpret_cast<const float4*>(p);
+    b = *reinterpret_cast<const float4*>(p + 4);
+  }
+  __device__ __forceinline__ void get(float (&o)[8]) const {
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+    o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+  }
+};
+
+template <typename T, int KEEP>
 __global__ void __launch_bounds__(256)
 layernorm_rows_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
                       const T* __restrict__ beta, float eps, int64_t N, int d, T* __restrict__ out,
@@ -65,78 +92,70 @@ layernorm_rows_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
   const int lane = threadIdx.x & 31;
   if (row >= N) return;
   const T* xr = x + row * d;
-  constexpr int kKeep = 8;                 // 8 x 8 elements per lane = rows of up to 2048
-  const bool keep = d <= kKeep * 256;
-  float r[kKeep][8];
-  float sum = 0.f;
-  if (keep) {
+  RawPiece<T> r[KEEP > 0 ? KEEP : 1];
+  // f(column, the row's eight elements from there), column after column of this lane
+  auto each = [&](auto f) {
+    if constexpr (KEEP > 0) {
 #pragma unroll
-    for (int i = 0; i < kKeep; ++i) {
-      const int c = lane * 8 + i * 256;
-      if (c < d) {
-        load8(xr + c, r[i]);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) sum += r[i][q];
+      for (int i = 0; i < KEEP; ++i) {
+        const int c = lane * 8 + i * 256;
+        if (c < d) {
+          float v[8];
+          r[i].get(v);
+          f(c, v);
+        }
+      }
+    } else {
+      for (int c = lane * 8; c < d; c += 256) {
+        float v[8];
+        load8(xr + c, v);
+        f(c, v);
       }
     }
-  } else {
-    for (int c = lane * 8; c < d; c += 256) {
-      float v[8];
-      load8(xr + c, v);
+  };
+  if constexpr (KEEP > 0) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) sum += v[i];
-    }
+    for (int i = 0; i < KEEP; ++i)
+      if (lane * 8 + i * 256 < d) r[i].load(xr + lane * 8 + i * 256);
   }
+  float sum = 0.f;
+  each([&](int, const float (&v)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) sum += v[q];
+  });
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float mean = sum / (float)d;
   float sq = 0.f;
-  if (keep) {
+  each([&](int, const float (&v)[8]) {
 #pragma unroll
-    for (int i = 0; i < kKeep; ++i)
-      if (lane * 8 + i * 256 < d) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) sq = fmaf(r[i][q] - mean, r[i][q] - mean, sq);
-      }
-  } else {
-    for (int c = lane * 8; c < d; c += 256) {
-      float v[8];
-      load8(xr + c, v);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) sq = fmaf(v[i] - mean, v[i] - mean, sq);
-    }
-  }
+    for (int q = 0; q < 8; ++q) sq = fmaf(v[q] - mean, v[q] - mean, sq);
+  });
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
   const float rstd = rsqrtf(sq / (float)d + eps);
-  if (keep) {
+  each([&](int c, const float (&v)[8]) {
+    float g[8], b[8], o[8];
+    load8_ldg(gamma + c, g);
+    load8_ldg(beta + c, b);
 #pragma unroll
-    for (int i = 0; i < kKeep; ++i) {
-      const int c = lane * 8 + i * 256;
-      if (c < d) {
-        float g[8], b[8], o[8];
-        load8_ldg(gamma + c, g);
-        load8_ldg(beta + c, b);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) o[q] = fmaf((r[i][q] - mean) * rstd, g[q], b[q]);
-        store8(out + row * d + c, o);
-      }
-    }
-  } else {
-    for (int c = lane * 8; c < d; c += 256) {
-      float v[8], g[8], b[8], o[8];
-      load8(xr + c, v);
-      load8_ldg(gamma + c, g);
-      load8_ldg(beta + c, b);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = fmaf((v[i] - mean) * rstd, g[i], b[i]);
-      store8(out + row * d + c, o);
-    }
-  }
+    for (int q = 0; q < 8; ++q) o[q] = fmaf((v[q] - mean) * rstd, g[q], b[q]);
+    store8(out + row * d + c, o);
+  });
   if (stats != nullptr && lane == 0) {
     stats[2 * row] = mean;
     stats[2 * row + 1] = rstd;
   }
+}
+
+template <typename T>
+int launch_rows(const void* x, const void* gamma, const void* beta, float eps, int64_t N, int d, void* out, float* stats,
+                cudaStream_t s) {
+  auto fn = d <= 1024 ? layernorm_rows_kernel<T, 4> : d <= 2048 ? layernorm_rows_kernel<T, 8> : layernorm_rows_kernel<T, 0>;
+  MOE_CUDA_CHECK(launch_pdl(fn, dim3((unsigned)((N + 7) / 8)), dim3(256), 0, s, static_cast<const T*>(x),
+                            static_cast<const T*>(gamma), static_cast<const T*>(beta), eps, N, d, static_cast<T*>(out),
+                            stats));
+  return 0;
 }
 
 }  // namespace
@@ -161,19 +180,8 @@ int launch_norm_fold(const void* Wg, const void* bg, const void* gamma, const vo
 int launch_layernorm_rows(const void* x, const void* gamma, const void* beta, float eps, int64_t N,
                           int d, int dtype, void* out, float* stats, cudaStream_t s) {
   if (N == 0) return 0;
-  const unsigned blocks = (unsigned)((N + 7) / 8);
-  if (dtype == MOE_B200_BF16)
-    MOE_CUDA_CHECK(launch_pdl(layernorm_rows_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, s,
-                              static_cast<const __nv_bfloat16*>(x),
-                              static_cast<const __nv_bfloat16*>(gamma),
-                              static_cast<const __nv_bfloat16*>(beta), eps, N, d,
-                              static_cast<__nv_bfloat16*>(out), stats));
-  else
-    MOE_CUDA_CHECK(launch_pdl(layernorm_rows_kernel<float>, dim3(blocks), dim3(256), 0, s,
-                              static_cast<const float*>(x), static_cast<const float*>(gamma),
-                              static_cast<const float*>(beta), eps, N, d, static_cast<float*>(out),
-                              stats));
-  return 0;
+  if (dtype == MOE_B200_BF16) return launch_rows<__nv_bfloat16>(x, gamma, beta, eps, N, d, out, stats, s);
+  return launch_rows<float>(x, gamma, beta, eps, N, d, out, stats, s);
 }
 
 }  // namespace moe
