@@ -6,8 +6,12 @@
 // one token at d=1024, f=4096, k=2: under 8 us at the HBM rate) and everything else is
 // latency: four dependent launches cost more than the stream itself. Here one grid of one
 // block per SM does it all:
-//   0. every block derives the routing by itself (front_small_body: same instructions on the
-//      same data in every block, so no exchange is needed); block 0 writes the routing results;
+//   0. every block derives the routing by itself (same instructions on the same data in every
+//      block, so no exchange is needed): 32 warps share d, then one warp per token does softmax
+//      and top-k in registers, and the first warp lists the hit experts. Two block barriers with one
+//      token, where the routing written for 512 tokens (front_small_body) took five and two
+//      more for the list, 6.2 of a call's 24.6 us; what the call records of the routing is
+//      written while the blocks meet at the grid barrier (the call: 21.0 us);
 //   1. every block requests its share of the down weights into shared memory (one bulk copy
 //      per weight row, completing on an mbarrier): the block owns d/gridDim output columns of
 //      EVERY hit expert, and these bytes do not depend on the hidden activations, so they
@@ -23,6 +27,7 @@
 //      rounds to bf16, weights, sums in slot order, adds the residual and writes the output:
 //      no partial sums in global memory and no combine kernel.
 #include <cooperative_groups.h>
+#include <utility>
 #include "front_small.cuh"
 #include "tc_ptx.cuh"
 
@@ -46,6 +51,104 @@ __host__ __device__ inline int w2_pitch_bytes(int f) {
   return row + ((64 - (row & 127)) + 128) % 128;
 }
 
+// The routing in shared memory (E <= 8 NT).
+template <int NT>
+struct Routing {
+  float part[kWarps][kTinyMaxTok][8 * NT];    // a warp's share of d
+  float logit[kTinyMaxTok][8 * NT], prob[kTinyMaxTok][8 * NT];
+  float wgt[kMaxPairs];        // renormalised weight of (token, slot)
+  int idx[kMaxPairs];          // its expert
+  int row[kMaxPairs];          // its row in the expert-sorted order
+  int off[kFrontMaxE + 1];     // first row of every expert
+  int tok[kMaxPairs];          // token of a sorted row
+  int hit[kFrontMaxE], nhit;   // experts with rows
+};
+
+// Softmax, top-k and renormalisation of token `tok` by one warp; lane e of a group of 8 NT lanes = expert e, the groups
+// do the same (reference model.py:207-223; order of the choices and of the sums as in front_small.cuh).
+template <int NT>
+__device__ __forceinline__ void route_token(Routing<NT>* rt, int tok, float bias, int E, int k, int lane) {
+  constexpr int ET = 8 * NT, P = 32 / ET;
+  const int e = lane % ET;
+  float v = 0.f;
+#pragma unroll
+  for (int q = 0; q < kWarps / P; ++q) v += rt->part[q * P + lane / ET][tok][e];
+#pragma unroll
+  for (int o = ET; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  v += bias;
+  if (lane < ET) rt->logit[tok][e] = v;
+  const bool live = e < E;
+  v = live ? v + 0.f : -INFINITY;      // + 0: no negative zero
+  // order-preserving map float -> unsigned: the maximum and its first position by integer compares
+  const unsigned u = __float_as_uint(v);
+  unsigned key = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+  unsigned kmax = key;
+#pragma unroll
+  for (int o = ET / 2; o > 0; o >>= 1) kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
+  const float m = __uint_as_float((kmax & 0x80000000u) ? (kmax & 0x7fffffffu) : ~kmax);
+  const float p = live ? expf(v - m) : 0.f;
+  float sum = p;
+#pragma unroll
+  for (int o = ET / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const float inv_sum = __frcp_rn(sum);
+  if (lane < ET) rt->prob[tok][e] = p * inv_sum;
+  int my_sel = 0;
+  float my_val = 0.f, total = 0.f;
+#pragma unroll 1
+  for (int j = 0; j < k; ++j) {
+    unsigned km = key;
+#pragma unroll
+    for (int o = ET / 2; o > 0; o >>= 1) km = max(km, __shfl_xor_sync(0xffffffffu, km, o));
+    const int winner = __ffs(__ballot_sync(0xffffffffu, key == km)) - 1;      // in the first group
+    const float bv = __uint_as_float((km & 0x80000000u) ? (km & 0x7fffffffu) : ~km);
+    const float val = expf(bv - m) * inv_sum;
+    total += val;
+    if (lane == j) { my_sel = winner; my_val = val; }
+    if (e == winner) key = 0u;     // below every real key
+  }
+  if (lane < k) {
+    rt->idx[tok * k + lane] = my_sel;
+    rt->wgt[tok * k + lane] = my_val * __frcp_rn(total);
+  }
+}
+
+// The routing results and the loss (model.py:213-216), by one block.
+template <int NT>
+__device__ __forceinline__ void record(const Routing<NT>* rt, int N, int E, int k, float* out_logits, int32_t* out_idx,
+                                       float* out_w, int32_t* row_of, int32_t* offsets, int32_t* cnt_slot, float* psum,
+                                       float* aux) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (out_logits != nullptr)
+    for (int i = tid; i < N * E; i += kThreads) out_logits[i] = rt->logit[i / E][i % E];
+  for (int p = tid; p < N * k; p += kThreads) {
+    out_idx[p] = rt->idx[p];
+    out_w[p] = rt->wgt[p];
+    row_of[p] = rt->row[p];
+  }
+  for (int i = tid; i <= E; i += kThreads) offsets[i] = rt->off[i];
+  for (int i = tid; i < k * E; i += kThreads) {
+    int c = 0;
+    for (int tok = 0; tok < N; ++tok) c += rt->idx[tok * k + i / E] == i % E;
+    cnt_slot[i] = c;
+  }
+  if (tid >> 5 == kWarps - 1) {
+    float term = 0.f;
+    if (lane < E) {
+      float ps = 0.f;
+      int c = 0;
+      for (int tok = 0; tok < N; ++tok) {
+        ps += rt->prob[tok][lane];
+        c += rt->idx[tok * k] == lane;
+      }
+      psum[lane] = ps;
+      term = (ps / (float)N) * ((float)c / (float)N);
+    }
+    float a = 0.f;
+    for (int e = 0; e < E; ++e) a += __shfl_sync(0xffffffffu, term, e);
+    if (lane == 0) aux[0] = a / (float)E * (float)(E * E);
+  }
+}
+
 template <int NT>
 __global__ void __launch_bounds__(kThreads, 1)
 decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ Wg,
@@ -64,14 +167,13 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   const int G = (int)gridDim.x, b = (int)blockIdx.x;
-  // the experts' parameter pointers do not depend on the routing: fetched first, so that their
-  // latency hides behind it
+  Routing<NT>* rt = reinterpret_cast<Routing<NT>*>(smem);
+  // the experts' parameter pointers and the router's weights do not depend on anything before: fetched first
   const void** s_ptr = reinterpret_cast<const void**>(reinterpret_cast<char*>(smem) + front_bytes);
-  const void* my_ptr = nullptr;      // requested now, stored after the routing
   if (tid < 4 * E) {
     const int which = tid / E, e = tid - which * E;
     const void* const* tab = which == 0 ? W1 : which == 1 ? b1 : which == 2 ? W2 : b2;
-    my_ptr = tab[e];
+    s_ptr[which * kFrontMaxE + e] = tab[e];
   }
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_ptr + 4 * kFrontMaxE);   // the down weights' arrival
   int* s_abort = reinterpret_cast<int*>(s_bar + 1);
@@ -80,20 +182,54 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  const float gate_bias = lane % (8 * NT) < E ? __bfloat162float(bg[lane % (8 * NT)]) : 0.f;
+  const int row_pieces = d >> 3, nchunk = (d + 31) >> 5;
+  auto gate_weights = [&](int c, uint4 (&w)[NT]) {
+    const int piece = 4 * c + t;
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+      w[j] = 8 * j + g < E && piece < row_pieces
+                 ? __ldg(reinterpret_cast<const uint4*>(Wg) + (size_t)(8 * j + g) * row_pieces + piece)
+                 : make_uint4(0, 0, 0, 0);
+  };
+  uint4 first_w[NT];
+  gate_weights(warp, first_w);
   pdl_wait();                 // x may come from the kernel before this one
   pdl_launch_dependents();
   // ---- 0. routing ------------------------------------------------------------------
-  const FrontSmallView rt = front_small_body<NT, false>(
-      smem, b, G, x, Wg, bg, N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm,
-      psum, aux, nullptr, nullptr, nullptr);
-  if (tid < 4 * E) s_ptr[(tid / E) * kFrontMaxE + tid % E] = my_ptr;
+  {
+    // partial logits: warp = chunks warp, warp + 32, ... of 32 elements, the contraction index inside a chunk permuted
+    // alike for x and Wg; tokens are rows 0..7 of the A tile
+    float acc[NT][4] = {};
+    for (int c = warp; c < nchunk; c += kWarps) {
+      const int piece = 4 * c + t;
+      uint4 w[NT];
+      if (c == warp) {
+#pragma unroll
+        for (int j = 0; j < NT; ++j) w[j] = first_w[j];
+      } else {
+        gate_weights(c, w);
+      }
+      const uint4 A = g < N && piece < row_pieces ? __ldcg(reinterpret_cast<const uint4*>(x + (size_t)g * d) + piece)
+                                                  : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        mma_bf16_16816(acc[j], A.x, 0u, A.y, 0u, w[j].x, w[j].y);
+        mma_bf16_16816(acc[j], A.z, 0u, A.w, 0u, w[j].z, w[j].w);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+      *reinterpret_cast<float2*>(&rt->part[warp][g][8 * j + 2 * t]) = make_float2(acc[j][0], acc[j][1]);
+  }
+  __syncthreads();
+  if (warp < N) route_token<NT>(rt, warp, gate_bias, E, k, lane);
+  if (N > 1) __syncthreads(); else __syncwarp();
   char* extra = reinterpret_cast<char*>(s_bar + 2);                // 16-byte aligned by the launcher
-  int* s_hit = reinterpret_cast<int*>(extra);                      // [32] experts with rows
-  int* s_tok = s_hit + 32;                                         // [kMaxPairs] token of a sorted row
-  int* s_nhit = s_tok + kMaxPairs;                                 // [4]
-  float* s_y = reinterpret_cast<float*>(s_nhit + 4);               // [kMaxPairs][8] down outputs
+  float* s_y = reinterpret_cast<float*>(extra);                    // [kMaxPairs][8] down outputs
   float* s_red = s_y + kMaxPairs * 8;                              // [kWarps][32][4] partial sums
   char* s_w2 = reinterpret_cast<char*>(s_red + kWarps * 32 * 4);   // down weights waiting for h
+  const int* s_hit = rt->hit;
 
   // this block's columns of the down weights
   const int c_lo = (int)((int64_t)d * b / G), c_hi = (int)((int64_t)d * (b + 1) / G);
@@ -101,17 +237,27 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   const int pitch = w2_pitch_bytes(f);
   const int ncol0 = min(8, c_hi - c_lo);
   const int M = N * k;
-  for (int p = tid; p < M; p += kThreads) {
-    const int r = rt.row[p];
-    if (r >= 0 && r < kMaxPairs) s_tok[r] = p / k;
-  }
-  __syncthreads();
   if (warp == 0) {
-    const bool hit = lane < E && rt.off[lane + 1] > rt.off[lane];
+    // rows in the expert-sorted order (stable), first rows and list of the experts that were hit
+    for (int p = lane; p < M; p += 32) {
+      const int e = rt->idx[p];
+      int row = 0;
+      for (int q = 0; q < M; ++q) row += rt->idx[q] < e || (rt->idx[q] == e && q < p);
+      rt->row[p] = row;
+      rt->tok[row] = p / k;
+    }
+    int before = 0, rows = 0;
+    for (int q = 0; q < M; ++q) {
+      before += rt->idx[q] < lane;
+      rows += rt->idx[q] == lane;
+    }
+    if (lane <= E) rt->off[lane] = before;
+    if (E == 32 && lane == 31) rt->off[32] = M;
+    const bool hit = lane < E && rows > 0;
     const unsigned mask = __ballot_sync(0xffffffffu, hit);
-    if (hit) s_hit[__popc(mask & ((1u << lane) - 1u))] = lane;
+    if (hit) rt->hit[__popc(mask & ((1u << lane) - 1u))] = lane;
     const int nh = __popc(mask);
-    if (lane == 0) s_nhit[0] = nh;
+    if (lane == 0) rt->nhit = nh;
     __syncwarp();
     // ---- 1. the first group of (up to) 8 columns of as many hit experts as fit, one bulk copy
     // per weight row, on their way to shared memory ----
@@ -131,7 +277,7 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     }
   }
   __syncthreads();
-  const int nhit = s_nhit[0];
+  const int nhit = rt->nhit;
   int n_pref = ncol0 > 0 ? min(nhit, w2_bytes / (8 * pitch)) : 0;
   // ---- 2. GEGLU product ------------------------------------------------------------
   {
@@ -162,12 +308,12 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
       if (tile < T1) {
         const int hi = tile / tiles_e, j0 = (tile - hi * tiles_e) << 3;
         const int e = s_hit[hi];
-        const int row0 = rt.off[e], rows = rt.off[e + 1] - row0;
+        const int row0 = rt->off[e], rows = rt->off[e + 1] - row0;
         const __nv_bfloat16* W = static_cast<const __nv_bfloat16*>(s_ptr[e]);
         const int ja = min(j0 + g, f - 1);                      // clamped: masked at the store
         const uint4* wa = reinterpret_cast<const uint4*>(W + (size_t)ja * d);        // gate row
         const uint4* wb = reinterpret_cast<const uint4*>(W + (size_t)(f + ja) * d);  // up row
-        const uint4* xr = g < rows ? reinterpret_cast<const uint4*>(x + (size_t)s_tok[row0 + g] * d)
+        const uint4* xr = g < rows ? reinterpret_cast<const uint4*>(x + (size_t)rt->tok[row0 + g] * d)
                                    : nullptr;
         for (int p0 = pb; p0 < pe; p0 += 16) {
           uint4 A[2][4];
@@ -197,7 +343,7 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
         if (tl < T1) {
           const int hi = tl / tiles_e, feat = ((tl - hi * tiles_e) << 3) + (ln >> 2);
           const int e = s_hit[hi];
-          const int row0 = rt.off[e], rows = rt.off[e + 1] - row0;
+          const int row0 = rt->off[e], rows = rt->off[e + 1] - row0;
           const int r = 2 * (ln & 3) + h2;
           if (feat < f && r < rows) {
             float gs = 0.f, us = 0.f;
@@ -229,8 +375,23 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   if (residual != nullptr && tid < N * 8 && (tid & 7) < ncol0)
     pre_res = __bfloat162float(residual[(size_t)(tid >> 3) * d + c_lo + (tid & 7)]);
   // ---- 3. every block's h is complete ------------------------------------------------
+  // (a row piece that this thread copies into the sorted buffer: read before the barrier, after which `out` is written)
+  const int copies = M * row_pieces, my_copy = b * kThreads + tid;
+  uint4 piece_x = make_uint4(0, 0, 0, 0);
+  if (my_copy < copies)
+    piece_x = __ldcg(reinterpret_cast<const uint4*>(x + (size_t)(my_copy / row_pieces / k) * d) + my_copy % row_pieces);
+  for (int i = my_copy + G * kThreads; i < copies; i += G * kThreads) {       // (rows of more than 16384 elements)
+    const int p = i / row_pieces, pc = i - p * row_pieces;
+    reinterpret_cast<uint4*>(perm + (size_t)rt->row[p] * d)[pc] =
+        __ldcg(reinterpret_cast<const uint4*>(x + (size_t)(p / k) * d) + pc);
+  }
   __threadfence();
-  grid.sync();
+  auto arrived = grid.barrier_arrive();
+  // what the call records of the routing, while the other blocks arrive
+  if (my_copy < copies)
+    reinterpret_cast<uint4*>(perm + (size_t)rt->row[my_copy / row_pieces] * d)[my_copy % row_pieces] = piece_x;
+  if (b == 0) record<NT>(rt, N, E, k, out_logits, out_idx, out_w, row_of, offsets, cnt_slot, psum, aux);
+  grid.barrier_wait(std::move(arrived));
   if (n_pref > 0) {
     // every thread observes the arrival itself (the copies were written by the async proxy)
     const bool ok = tc::mbar_wait(s_bar, 0, s_abort, status, 61);
@@ -248,7 +409,7 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     const int pb = min(pieces_f, ks * per), pe = min(pieces_f, (ks + 1) * per);
     const uint4 zero = make_uint4(0, 0, 0, 0);
     const int e = live ? s_hit[hi] : 0;
-    const int row0 = rt.off[e], rows = live ? rt.off[e + 1] - row0 : 0;
+    const int row0 = rt->off[e], rows = live ? rt->off[e + 1] - row0 : 0;
     const uint4* hr = g < rows ? reinterpret_cast<const uint4*>(h + (size_t)(row0 + g) * f) : nullptr;
     for (int c0 = c_lo; c0 < c_hi; c0 += 8) {
       const int ncol = min(8, c_hi - c0);
@@ -301,7 +462,7 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
       for (int item = tid; item < nhit * 64; item += kThreads) {
         const int xh = item >> 6, ln = (item >> 1) & 31, h2 = item & 1;
         const int xe = s_hit[xh];
-        const int xrow0 = rt.off[xe], xrows = rt.off[xe + 1] - xrow0;
+        const int xrow0 = rt->off[xe], xrows = rt->off[xe + 1] - xrow0;
         const int r = ln >> 2, col = 2 * (ln & 3) + h2;
         if (r < xrows && col < ncol) {
           float sum = 0.f;
@@ -321,9 +482,9 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
         if (col < ncol) {
           float o = 0.f;
           for (int j = 0; j < k; ++j) {
-            const int r = rt.row[tok * k + j];
+            const int r = rt->row[tok * k + j];
             if (r < 0) continue;
-            o = __fadd_rn(o, __fmul_rn(rt.wgt[tok * k + j], s_y[r * 8 + col]));
+            o = __fadd_rn(o, __fmul_rn(rt->wgt[tok * k + j], s_y[r * 8 + col]));
           }
           const size_t at = (size_t)tok * d + c0 + col;
           if (residual != nullptr)
@@ -337,8 +498,7 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 }
 
 size_t tiny_extra_bytes() {
-  return sizeof(void*) * 4 * kFrontMaxE + 16 + sizeof(int) * (32 + kMaxPairs + 4) +
-         sizeof(float) * (kMaxPairs * 8 + kWarps * 32 * 4);
+  return sizeof(void*) * 4 * kFrontMaxE + 16 + sizeof(float) * (kMaxPairs * 8 + kWarps * 32 * 4);
 }
 
 template <int NT>
@@ -350,7 +510,7 @@ int launch(const void* x, const void* Wg, const void* bg, int N, int d, int f, i
   static PerDeviceOnce once;
   int rc = ensure_dynamic_smem(once, decode_tiny_kernel<NT>, kSmemMax);
   if (rc) return rc;
-  int front_bytes = (int)((front_small_smem_bytes(NT, N, E, k) + 15) & ~(size_t)15);
+  int front_bytes = (int)((sizeof(Routing<NT>) + 15) & ~(size_t)15);
   const int fixed = front_bytes + (int)tiny_extra_bytes();
   // room for the down weights: all hit experts (at most N*k of them) if they fit
   const int want = (N * k < E ? N * k : E) * 8 * w2_pitch_bytes(f);

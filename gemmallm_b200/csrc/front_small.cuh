@@ -57,26 +57,14 @@ using front_detail::ld_acquire_gpu_i32;
 //   `status`), and each block places and copies its own rows. Same results as the other form
 //   except for the order in which the logits' partial sums are added.
 //
-// A device function so that a kernel which goes on to use the routing (experts_tiny.cu) can run
-// it in its own blocks: `blk` of `nblk` is the calling block's place among the blocks that run
-// it, `smem` front_small_smem_bytes() of shared memory. On return (after a block barrier) the
-// block's shared memory holds the routing: see FrontSmallView.
-struct FrontSmallView {
-  const int* idx;      // [N*k] expert of (token, slot)
-  const int* row;      // [N*k] row of (token, slot) in the expert-sorted order
-  const int* off;      // [E+1] first row of every expert
-  const float* wgt;    // [N*k] renormalised routing weight of (token, slot)
-};
-
+// `blk` of `nblk`: the calling block's place; `smem`: front_small_smem_bytes() of shared memory.
 __host__ __device__ inline size_t front_small_smem_bytes(int NT, int ntok, int E, int k) {
   return sizeof(float) * ((size_t)32 * 16 * 8 * NT + (size_t)ntok * (E + 1)) +
-         sizeof(int) * (2 * (size_t)ntok * k + 2 * kMaxTopK * kFrontMaxE + 4 * kFrontMaxE + 1) +
-         sizeof(float) * (size_t)ntok * k;
+         sizeof(int) * (2 * (size_t)ntok * k + 2 * kMaxTopK * kFrontMaxE + 4 * kFrontMaxE + 1);
 }
 
 template <int NT, bool SPLIT, typename T = __nv_bfloat16>  // n-tiles of 8 experts: E <= 8*NT
-__device__ __forceinline__ FrontSmallView
-front_small_body(float* smem, const int blk, const int nblk,
+__device__ __forceinline__ void front_small_body(float* smem, const int blk, const int nblk,
                  const T* __restrict__ x, const T* __restrict__ Wg, const T* __restrict__ bg, int Ntotal, int d, int E, int k,
                  float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                  float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
@@ -113,7 +101,6 @@ front_small_body(float* smem, const int blk, const int nblk,
   int* s_off = s_cnt + kMaxTopK * kMaxE;                   // [kMaxE+1]
   int* s_run = s_off + kMaxE + 1;                          // [kMaxE]
   float* s_bias = reinterpret_cast<float*>(s_run + kMaxE); // [kMaxE], then s_base, s_tot (SPLIT)
-  float* s_wgt = s_bias + 2 * kMaxE + kMaxTopK * kMaxE;    // [N*k]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -295,7 +282,6 @@ front_small_body(float* smem, const int blk, const int nblk,
           out_w[tok * k + e] = my_val * __frcp_rn(total);
         }
         s_idx[tok * k + e] = my_sel;
-        s_wgt[tok * k + e] = my_val * __frcp_rn(total);
         atomicAdd(&s_cnt[e * kMaxE + my_sel], 1);
       }
     }
@@ -452,8 +438,6 @@ front_small_body(float* smem, const int blk, const int nblk,
     __syncthreads();
     if (tid == 0 && atomicAdd(counter, 1) == 2 * nblk - 1) *counter = 0;
   }
-  __syncthreads();
-  return FrontSmallView{s_idx, s_row, s_off, s_wgt};
 }
 
 }  // namespace moe
