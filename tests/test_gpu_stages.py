@@ -150,6 +150,20 @@ def test_dispatch_is_a_stable_counting_sort(cuda_device, N, d, E, k, dtype):
     assert abs(float(out["aux"][0]) - float(aux)) <= 1e-5 * abs(float(aux)) + 1e-7
 
 
+# rows of one 16-byte piece, of odd counts of pieces, and on both sides of 8192 pieces
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 8), (torch.bfloat16, 24), (torch.float32, 8), (torch.float32, 1016),
+                                     (torch.bfloat16, 8 * 8191), (torch.bfloat16, 8 * 8192), (torch.float32, 4 * 8190)])
+def test_dispatch_copies_rows_of_any_width(cuda_device, dtype, d):
+    N, E, k = (20000, 8, 2) if d < 2000 else (150, 8, 2)     # chunks of more than four tokens where rows are short
+    g = torch.Generator().manual_seed(d)
+    x = torch.randn(N, d, generator=g).to(dtype).to(cuda_device)
+    idx = torch.rand(N, E, generator=g).topk(k, dim=1).indices.to(torch.int32).to(cuda_device)
+    out = helpers.dispatch(x, idx, E)
+    flat = out["row_of"].long().flatten()
+    assert torch.equal(flat.sort().values, torch.arange(N * k, device=cuda_device))
+    assert torch.equal(out["perm"][flat].view(N, k, d), x[:, None, :].expand(N, k, d))
+
+
 def test_dispatch_reports_bad_index(cuda_device):
     x = torch.randn(10, 64, device=cuda_device)
     idx = torch.zeros(10, 2, dtype=torch.int32, device=cuda_device)
