@@ -480,14 +480,18 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   const bool tiles = rows_path && tiles_at_row_counts(N * k, d, E);
   // (a folded LayerNorm stays with the general kernels)
   const bool front32 = dtype == MOE_B200_F32 && !norm && front_f32_supported(N, E, k);
+  const bool front = front32 || ((small_n || rows_path) && (front_small_supported(N, E, k, dtype) ||
+                                                            front_split_supported(N, E, k, dtype)));
+  // The small calls launch their kernels below without the entry points that test this, and a LayerNorm reads x before
+  // they do. (The folded LayerNorm of the large calls reads Wg an element at a time.)
+  if (N > 0 && (!aligned16(x) || ((tiny || front) && !aligned16(Wg))))
+    return set_error(MOE_B200_ERR_ALIGN, "x and Wg must be 16-byte aligned");
   const bool counters = small_n || rows_path || front32;
   // status words, and the completion counters behind them where a kernel uses them, in one memset
   // (above these sizes a call always clears the status words: they are those of the most recent call)
   if (!(counters && (flags & MOE_B200_FLAG_WS_CLEAN)))
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
-  const bool front = front32 || ((small_n || rows_path) && (front_small_supported(N, E, k, dtype) ||
-                                                            front_split_supported(N, E, k, dtype)));
   float* stats = reinterpret_cast<float*>(ws + off[MOE_B200_WS_STATS]);
   if (norm && N > 0 && (front || small_n || rows_path)) {
     // up to 4096 rows the kernels read x through TMA: normalise the few rows once

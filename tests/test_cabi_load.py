@@ -4,6 +4,9 @@ import ctypes as C
 import re
 from pathlib import Path
 
+import pytest
+import torch
+
 from gemmallm_b200 import _cabi
 from gemmallm_b200._cabi import lib
 
@@ -91,6 +94,24 @@ def test_small_and_mid_size_entry_points_check_their_arguments():
     assert tiny(4, 1024, 4096, 33, 2) == -7
     assert tiny(4, 1024, 4096, 8, 2, out=None) == -1
     assert tiny(4, 1024, 4096, 8, 2, x=a + 8) == -3
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="no address here is one of a device")
+@pytest.mark.parametrize("N,E,k,dtype", [(512, 8, 2, _cabi.F32), (2048, 8, 2, _cabi.F32), (1, 8, 2, _cabi.F32),
+                                         (1, 8, 2, _cabi.BF16), (48, 8, 2, _cabi.BF16), (300, 8, 2, _cabi.BF16),
+                                         (1500, 8, 2, _cabi.BF16), (20, 64, 2, _cabi.BF16)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_rows_and_router_weights_off_a_16_byte_boundary_are_refused_before_any_launch(N, E, k, dtype, norm):
+    """The small calls' kernels read both 16 bytes at a time: an error of the host's checks, not of CUDA, comes back."""
+    a = 1 << 20
+    ws = _cabi.workspace_bytes(N, 64, 128, E, k, dtype)
+    call = lambda x, wg: lib.moe_b200_forward(x, wg, a, a, None, a if norm else None, a if norm else None, 1e-5, N, 64, 128,
+                                              E, k, dtype, 0, a, ws, a, None)
+    for off in (4, 8):
+        assert call(a + off, a) == -3 and b"16-byte" in lib.moe_b200_last_error_string()
+    # (with a LayerNorm folded in, the large calls' kernels read the weights an element at a time: not refused there)
+    if E <= 32 and not (norm and dtype == _cabi.F32):
+        assert call(a, a + 4) == -3 and b"16-byte" in lib.moe_b200_last_error_string()
 
 
 def test_host_extension_is_rebuilt_for_another_torch(tmp_path, monkeypatch):
