@@ -11,7 +11,7 @@
 //      and top-k in registers, and the first warp lists the hit experts. Two block barriers with one
 //      token, where the routing written for 512 tokens (front_small_body) took five and two
 //      more for the list, 6.2 of a call's 24.6 us; what the call records of the routing is
-//      written while the blocks meet at the grid barrier (the call: 21.0 us);
+//      written while the blocks meet at the grid barrier (the call: 21.1 us);
 //   1. every block requests its share of the down weights into shared memory (one bulk copy
 //      per weight row, completing on an mbarrier): the block owns d/gridDim output columns of
 //      EVERY hit expert, and these bytes do not depend on the hidden activations, so they
@@ -168,7 +168,7 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   const int g = lane >> 2, t = lane & 3;
   const int G = (int)gridDim.x, b = (int)blockIdx.x;
   Routing<NT>* rt = reinterpret_cast<Routing<NT>*>(smem);
-  // the experts' parameter pointers and the router's weights do not depend on anything before: fetched first
+  // the experts' parameter pointers do not depend on anything before: fetched first
   const void** s_ptr = reinterpret_cast<const void**>(reinterpret_cast<char*>(smem) + front_bytes);
   if (tid < 4 * E) {
     const int which = tid / E, e = tid - which * E;
@@ -182,20 +182,15 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  const float gate_bias = lane % (8 * NT) < E ? __bfloat162float(bg[lane % (8 * NT)]) : 0.f;
   const int row_pieces = d >> 3, nchunk = (d + 31) >> 5;
-  auto gate_weights = [&](int c, uint4 (&w)[NT]) {
-    const int piece = 4 * c + t;
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-      w[j] = 8 * j + g < E && piece < row_pieces
-                 ? __ldg(reinterpret_cast<const uint4*>(Wg) + (size_t)(8 * j + g) * row_pieces + piece)
-                 : make_uint4(0, 0, 0, 0);
+  auto gate_piece = [&](int j, int piece) {
+    return reinterpret_cast<const uint4*>(Wg) + (size_t)(8 * j + g) * row_pieces + piece;
   };
-  uint4 first_w[NT];
-  gate_weights(warp, first_w);
-  pdl_wait();                 // x may come from the kernel before this one
+  // x, and the router's weights and biases too (an optimizer step, a copy), may come from the kernel before this one.
+  // (Asking for the weights in L2 ahead of the wait costs more than it gives: one token 22.1 us, without 21.1.)
+  pdl_wait();
   pdl_launch_dependents();
+  const float gate_bias = lane % (8 * NT) < E ? __bfloat162float(__ldcg(bg + lane % (8 * NT))) : 0.f;
   // ---- 0. routing ------------------------------------------------------------------
   {
     // partial logits: warp = chunks warp, warp + 32, ... of 32 elements, the contraction index inside a chunk permuted
@@ -204,12 +199,9 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     for (int c = warp; c < nchunk; c += kWarps) {
       const int piece = 4 * c + t;
       uint4 w[NT];
-      if (c == warp) {
 #pragma unroll
-        for (int j = 0; j < NT; ++j) w[j] = first_w[j];
-      } else {
-        gate_weights(c, w);
-      }
+      for (int j = 0; j < NT; ++j)
+        w[j] = 8 * j + g < E && piece < row_pieces ? __ldcg(gate_piece(j, piece)) : make_uint4(0, 0, 0, 0);
       const uint4 A = g < N && piece < row_pieces ? __ldcg(reinterpret_cast<const uint4*>(x + (size_t)g * d) + piece)
                                                   : make_uint4(0, 0, 0, 0);
 #pragma unroll
