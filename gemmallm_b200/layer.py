@@ -15,19 +15,35 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import _host
+from . import _cabi, _host
+from ._cabi import check, lib
 from .attention import Attention
-from .moe import MOE, FeedForward
+from .moe import MOE, FeedForward, _stream
 
 
 def _layernorm(norm: nn.LayerNorm, x: torch.Tensor) -> torch.Tensor:
     """norm(x) by the library's row kernel (moe_b200_layernorm) for bf16/fp32 CUDA
-    tensors outside autograd; torch's own LayerNorm otherwise (training)."""
-    if x.is_cuda and norm.weight is not None and norm.bias is not None:
-        out = _host.layernorm(x.contiguous(), norm.weight, norm.bias, float(norm.eps))
-        if out is not None:
-            return out
-    return norm(x)
+    tensors outside autograd; torch's own LayerNorm otherwise (training). What the native call
+    declines (autocast, under which torch's LayerNorm would hand on fp32, torch function modes,
+    tracing, other classes of tensors) takes the same kernel from here."""
+    if not x.is_cuda or norm.weight is None or norm.bias is None:
+        return norm(x)
+    out = _host.layernorm(x.contiguous(), norm.weight, norm.bias, float(norm.eps))
+    if out is not None:
+        return out
+    xc, d, params = x.contiguous(), x.shape[-1], (norm.weight, norm.bias)
+    if (x.dtype not in (torch.bfloat16, torch.float32) or d % 8 != 0 or xc.data_ptr() % 16 != 0
+            or any(p.dtype != x.dtype or p.device != x.device or p.numel() != d or not p.is_contiguous()
+                   or p.data_ptr() % 16 != 0 for p in params)
+            or (torch.is_grad_enabled() and any(t.requires_grad for t in (x, *params)))):
+        return norm(x)
+    out = torch.empty_like(xc)
+    code = _cabi.BF16 if x.dtype == torch.bfloat16 else _cabi.F32
+    with torch.cuda.device(x.device):
+        check(lib.moe_b200_layernorm(xc.data_ptr(), norm.weight.data_ptr(), norm.bias.data_ptr(),
+                                     float(norm.eps), xc.numel() // d, d, code, out.data_ptr(),
+                                     _stream(x.device)), "layernorm")
+    return out
 
 
 class LLMLayer(nn.Module):

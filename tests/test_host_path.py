@@ -7,8 +7,9 @@ import weakref
 import pytest
 import torch
 
-from gemmallm_b200 import MOE, Attention, FeedForward, _host
+from gemmallm_b200 import MOE, Attention, FeedForward, LLMLayer, _host
 from gemmallm_b200._cabi import MoeB200Error
+from gemmallm_b200.layer import _layernorm
 
 DT = torch.bfloat16
 D, F, E, RANK = 64, 128, 4, 16
@@ -864,3 +865,39 @@ def test_layernorm_native_and_left_alone(cuda_device, dtype):
         assert _host.layernorm(odd, *args) is None                          # not on a 16-byte boundary
         with torch.autocast("cuda"):
             assert _host.layernorm(x, *args) is None
+
+
+@pytest.mark.gpu
+def test_decoder_layer_in_the_modes_that_see_its_calls(cuda_device):
+    """Under autocast and torch function modes the layer runs the same kernels."""
+    from torch.overrides import TorchFunctionMode
+
+    class Watching(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    torch.manual_seed(4)
+    layer = LLMLayer(D, 64, 2, 1, Table(128, 64), expansion_factor=2, use_moe=True, num_experts=E, device="cuda")
+    layer = layer.to(device=cuda_device, dtype=DT).eval()
+    layer.mqa.embedding.float()
+    torch.nn.init.normal_(layer.norm1.weight)
+    x = rows(2 * 37, cuda_device).view(2, 37, D)
+    mask = torch.full((37, 37), float("-inf"), device=cuda_device).triu(1)
+    with torch.no_grad():
+        want = layer(x, mask)
+        with torch.autocast("cuda", dtype=DT):
+            same(layer(x, mask), want)
+        with torch.device("cuda"):
+            same(layer(x, mask), want)
+        with Watching():
+            same(layer(x, mask), want)
+        norm = layer.norm1
+        native = _host.layernorm(x, norm.weight, norm.bias, norm.eps)
+        for args in ((x,), (x.transpose(0, 1).contiguous().transpose(0, 1),)):
+            with torch.autocast("cuda", dtype=DT):
+                assert torch.equal(_layernorm(norm, *args), native)
+            assert torch.equal(_layernorm(norm, *args), native)
+        # what the row kernel cannot read stays torch's: rows at an odd place, none at all
+        odd = torch.empty(x.numel() + 1, device=cuda_device, dtype=DT)[1:].view_as(x).copy_(x)
+        same([_layernorm(norm, odd), _layernorm(norm, x[:0])], [norm(odd), norm(x[:0])])
+    assert _layernorm(norm, x).requires_grad
