@@ -479,13 +479,18 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   // f 8192, 300 rows 72 / 86, 1500 171 / 162; 2 experts, d 1024, 500 rows 52 / 60, 1500 72 / 73; 3, 900 rows 62 / 69
   const bool tiles = rows_path && tiles_at_row_counts(N * k, d, E);
   // (a folded LayerNorm stays with the general kernels)
-  const bool front32 = dtype == MOE_B200_F32 && !norm && front_f32_supported(N, E, k);
-  const bool front = front32 || ((small_n || rows_path) && (front_small_supported(N, E, k, dtype) ||
+  bool front32 = dtype == MOE_B200_F32 && !norm && front_f32_supported(N, E, k);
+  bool front = front32 || ((small_n || rows_path) && (front_small_supported(N, E, k, dtype) ||
                                                             front_split_supported(N, E, k, dtype)));
   // The small calls launch their kernels below without the entry points that test this, and a LayerNorm reads x before
   // they do. (The folded LayerNorm of the large calls reads Wg an element at a time.)
   if (N > 0 && (!aligned16(x) || ((tiny || front) && !aligned16(Wg))))
     return set_error(MOE_B200_ERR_ALIGN, "x and Wg must be 16-byte aligned");
+  if (front32) {
+    rc = front_f32_resident(N, &front32);
+    if (rc) return rc;
+    front = front32;
+  }
   const bool counters = small_n || rows_path || front32;
   // status words, and the completion counters behind them where a kernel uses them, in one memset
   // (above these sizes a call always clears the status words: they are those of the most recent call)

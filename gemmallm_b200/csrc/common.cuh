@@ -167,30 +167,42 @@ __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// cluster: blocks per cluster along x, 0 for none (or a compile-time __cluster_dims__)
+// cluster: blocks per cluster along x, 0 for none (or a compile-time __cluster_dims__); whole: a cooperative launch, all
+// blocks resident at once
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster, size_t smem,
-                                      cudaStream_t s, Args... args) {
+inline cudaError_t launch_pdl_as(void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster, bool whole, size_t smem,
+                                 cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 0 ? 2 : 1;
+  cfg.numAttrs = 1;
+  if (cluster > 0) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  if (whole) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeCooperative;
+    attr[cfg.numAttrs++].val.cooperative = 1;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster, size_t smem,
+                                      cudaStream_t s, Args... args) {
+  return launch_pdl_as(kernel, grid, block, cluster, false, smem, s, args...);
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                               cudaStream_t s, Args... args) {
-  return launch_pdl_cluster(kernel, grid, block, 0, smem, s, args...);
+  return launch_pdl_as(kernel, grid, block, 0, false, smem, s, args...);
 }
 
 // Plan buffer layout (device memory owned by the caller).
@@ -329,8 +341,9 @@ int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
                        cudaStream_t s, int* xch = nullptr, int* counter = nullptr,
                        int32_t* status = nullptr, int dtype = MOE_B200_BF16);
-// fp32, with the exchange buffer and the counter
+// fp32, with the exchange buffer; on this device only if its blocks are all resident at once
 bool front_f32_supported(int64_t N, int E, int k);
+int front_f32_resident(int64_t N, bool* yes);
 int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
                    uint32_t box_cols = 64);
 int encode_tmap_2d_f32(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);

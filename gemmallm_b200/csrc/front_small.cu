@@ -50,9 +50,9 @@ int launch(const void* x, const void* Wg, const void* bg, int N, int d, int E, i
   }
   // one block per 16 tokens
   const int blocks = N <= 16 ? 1 : (N + 15) / 16;
-  MOE_CUDA_CHECK(launch_pdl(fn, dim3(blocks), dim3(kThreads), smem, s, static_cast<const T*>(x),
-                            static_cast<const T*>(Wg), static_cast<const T*>(bg), N, d, E, k, out_logits, out_idx,
-                            out_w, cnt_slot, offsets, row_of, static_cast<T*>(perm), psum, aux, xch, counter, status));
+  MOE_CUDA_CHECK(launch_pdl_as(fn, dim3(blocks), dim3(kThreads), 0, F32 && blocks > 1, smem, s, static_cast<const T*>(x),
+                               static_cast<const T*>(Wg), static_cast<const T*>(bg), N, d, E, k, out_logits, out_idx,
+                               out_w, cnt_slot, offsets, row_of, static_cast<T*>(perm), psum, aux, xch, counter, status));
   return 0;
 }
 
@@ -76,10 +76,17 @@ int64_t front_small_exchange_ints(int64_t N, int E, int k) {
   return nb * k * E + nb * E;
 }
 
-// fp32 calls: the general kernels took 36 us at 512 tokens (d 512, 8 experts: router 22, dispatch 14, with a memset in front);
-// beyond 2048 tokens the blocks would no longer all be resident.
+// fp32 calls: the general kernels took 36 us at 512 tokens (d 512, 8 experts: router 22, dispatch 14, with a memset in front).
+// One block an SM, 16 tokens a block: up to 2048 tokens on a whole GPU, fewer where a part of one is at hand.
 bool front_f32_supported(int64_t N, int E, int k) {
   return N >= 1 && N <= 16 * 128 && E <= kMaxE && k <= kMaxTopK && N * k <= kRowsPathMaxRows;
+}
+
+int front_f32_resident(int64_t N, bool* yes) {
+  int sms = 0;
+  int rc = N > 16 ? sm_count(&sms) : 0;
+  *yes = rc == 0 && (N <= 16 || (N + 15) / 16 <= sms);
+  return rc;
 }
 
 namespace {

@@ -92,6 +92,37 @@ def test_fp32_routing_in_one_launch(cuda_device, N, d, E, k):
         assert torch.equal(m.last[name], disp[name]), name
 
 
+def test_fp32_calls_on_two_streams_and_in_a_graph(cuda_device):
+    """Two calls at once, each with a grid whose blocks wait on one another and nearly as many blocks as there are SMs; then
+    both from one graph."""
+    N, d, E, f, k = 2048, 64, 8, 128, 2
+    params = synthetic.make_params(d, E, f, seed=3)
+    mods = [build(params, d, E, f, k, torch.float32, cuda_device) for _ in range(2)]
+    xs = [torch.randn(1, N, d, generator=torch.Generator().manual_seed(i)).to(cuda_device) for i in range(2)]
+    with torch.no_grad():
+        want = [m(x)[0] for m, x in zip(mods, xs)]
+        torch.cuda.synchronize()
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        got = [[], []]
+        for _ in range(50):
+            for i, st in enumerate(streams):
+                with torch.cuda.stream(st):
+                    got[i].append(mods[i](xs[i])[0])
+        torch.cuda.synchronize()
+        for i in range(2):
+            assert mods[i].device_status() == 0
+            assert all(torch.equal(o, want[i]) for o in got[i])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = [m(x)[0] for m, x in zip(mods, xs)]
+        for _ in range(3):
+            for o in captured:
+                o.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert all(torch.equal(o, w) for o, w in zip(captured, want))
+
+
 SMALL = [
     # N, d, E, f, k
     (1, 64, 8, 128, 2), (2, 64, 8, 128, 2), (3, 64, 8, 128, 2), (127, 64, 8, 128, 2),
