@@ -491,10 +491,11 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
     if (rc) return rc;
     front = front32;
   }
-  const bool counters = small_n || rows_path || front32;
+  const bool counters = small_n || rows_path;
   // status words, and the completion counters behind them where a kernel uses them, in one memset
-  // (above these sizes a call always clears the status words: they are those of the most recent call)
-  if (!(counters && (flags & MOE_B200_FLAG_WS_CLEAN)))
+  // (above these sizes a call always clears the status words: they are those of the most recent call; the fp32 front
+  // clears them itself)
+  if (!front32 && !(counters && (flags & MOE_B200_FLAG_WS_CLEAN)))
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
   float* stats = reinterpret_cast<float*>(ws + off[MOE_B200_WS_STATS]);

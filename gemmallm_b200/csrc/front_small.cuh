@@ -249,6 +249,9 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
       // order-preserving map float -> unsigned: the maximum and its first position by integer compares
       const unsigned u = __float_as_uint(v);
       unsigned key = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+      // fp32: as in router_kernel, which takes the larger calls, NaN is never chosen, and slots that are left without an
+      // expert have an index out of range; the dispatch reports them and gives them no row
+      if (F32 && !(live && v == v)) key = 0u;
       unsigned kmax = key;
 #pragma unroll
       for (int o = G / 2; o > 0; o >>= 1) kmax = max(kmax, __shfl_xor_sync(gmask, kmax, o));
@@ -274,9 +277,10 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
         const unsigned hit = __ballot_sync(gmask, key == km) & gmask;
         const int winner = __ffs(hit) - 1;
         const float bv = __uint_as_float((km & 0x80000000u) ? (km & 0x7fffffffu) : ~km);
-        const float val = expf(bv - m) * inv_sum;
+        const bool none = F32 && km == 0u;
+        const float val = none ? 0.f : expf(bv - m) * inv_sum;
         total += val;
-        if (e == j) { my_sel = winner - grp * G; my_val = val; }
+        if (e == j) { my_sel = none ? 0x7fffffff : winner - grp * G; my_val = val; }
         if (lane == winner) key = 0u;     // below every real key
       }
       if (e < k && tok < N) {
@@ -285,7 +289,7 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
           out_w[tok * k + e] = my_val * __frcp_rn(total);
         }
         s_idx[tok * k + e] = my_sel;
-        atomicAdd(&s_cnt[e * kMaxE + my_sel], 1);
+        if (!F32 || my_sel < E) atomicAdd(&s_cnt[e * kMaxE + my_sel], 1);
       }
     }
   }
@@ -304,6 +308,8 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
       xps[b * E + tid] = ps;
     }
     for (int i = tid; i < kMaxE + kMaxTopK * kMaxE; i += kThreads) s_base[i] = 0;   // s_base, s_tot
+    // fp32: the status words are this call's; what a block has to say it says behind the barrier
+    if (F32 && b == 0 && tid < MOE_B200_STATUS_INTS) status[tid] = 0;
     __threadfence();
     if constexpr (F32) {
       if (nblk > 1) cooperative_groups::this_grid().sync();
@@ -370,7 +376,8 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
     for (int p0 = 0; p0 < npair; p0 += 32) {
       const int p = p0 + lane;
       const int e = p < npair ? s_idx[p] : -1;
-      const bool ok = e >= 0;
+      const bool ok = F32 ? (unsigned)e < (unsigned)E : e >= 0;
+      if (F32 && p < npair && !ok) atomicMax(&status[0], MOE_B200_DEV_BAD_INDEX);
       const unsigned grp = __match_any_sync(0xffffffffu, ok ? e : -1 - lane);
       int row = -1;
       if (ok) row = s_off[e] + s_run[e] + __popc(grp & ((1u << lane) - 1u));
@@ -399,8 +406,10 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
       const int i = i0 + u * kThreads;
       if (i < items) {
         const int tok = i / pieces, pc = i - tok * pieces;
-        for (int j = 0; j < k; ++j)
-          reinterpret_cast<uint4*>(perm + (size_t)s_row[tok * k + j] * d)[pc] = v[u];
+        for (int j = 0; j < k; ++j) {
+          const int row = s_row[tok * k + j];
+          if (!F32 || row >= 0) reinterpret_cast<uint4*>(perm + (size_t)row * d)[pc] = v[u];
+        }
       }
     }
   }

@@ -52,7 +52,11 @@ enum {
 enum {
   MOE_B200_DEV_OK = 0,
   MOE_B200_DEV_TIMEOUT = 1,   /* a bounded wait inside a kernel ran out */
-  MOE_B200_DEV_BAD_INDEX = 2  /* an expert index outside [0,E) was seen */
+  /* an expert index outside [0,E) was seen: a token with fewer than k logits that are not NaN
+   * (a row of x with a NaN has none). Such a slot has no row and adds nothing to the output. The
+   * bf16 kernels of small calls (moe_b200_front_small, moe_b200_decode_tiny) take NaN for the
+   * largest logit instead: the token's output is NaN and nothing is reported. */
+  MOE_B200_DEV_BAD_INDEX = 2
 };
 
 /* flags for moe_b200_forward */
@@ -62,8 +66,8 @@ enum {
    * (MOE_B200_WS_STATUS, status words and counters) is all zero on entry: it was
    * zeroed once, and every call on this workspace since then has ended with
    * device status 0 (such calls leave the region zero). Saves the memset in
-   * front of the first kernel of calls of up to 4096 rows, which then overlaps
-   * the tail of the kernel before it; larger calls clear the status words
+   * front of the first kernel of bf16 calls of up to 4096 rows, which then overlaps
+   * the tail of the kernel before it; larger calls and fp32 calls clear the status words
    * anyway. After a non-zero device status the region has to be zeroed again by
    * the caller. */
   MOE_B200_FLAG_WS_CLEAN = 1

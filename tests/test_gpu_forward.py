@@ -92,6 +92,59 @@ def test_fp32_routing_in_one_launch(cuda_device, N, d, E, k):
         assert torch.equal(m.last[name], disp[name]), name
 
 
+@pytest.mark.parametrize("N,fold", [(1, False), (40, False), (2048, False), (2049, False), (300, True), (2049, True)])
+def test_fp32_tokens_of_nan(cuda_device, N, fold):
+    """On both sides of 2048 tokens, with and without a folded LayerNorm: a token of NaN has no expert, its output is the
+    residual, the status says so, and the other tokens are as without it. The status is that of the last call."""
+    d, E, f, k = 64, 8, 128, 2
+    params = synthetic.make_params(d, E, f, seed=N)
+    m = build(params, d, E, f, k, torch.float32, cuda_device)
+    x = torch.randn(1, N, d, generator=torch.Generator().manual_seed(N)).to(cuda_device)
+    norm = torch.nn.LayerNorm(d, device=cuda_device) if fold else None
+    bad = x.clone()
+    rows = sorted({0, N // 3, N - 1})
+    bad[0, rows, 5] = float("nan")
+    other = torch.ones(N, dtype=torch.bool, device=cuda_device)
+    other[rows] = False
+    with torch.no_grad():
+        for _ in range(2):
+            want, _ = m(x, residual=x, norm=norm)
+            m(bad, residual=x, norm=norm)
+            m(x, residual=x, norm=norm)
+            assert m.device_status() == 0
+            got, aux = m(bad, residual=x, norm=norm)
+            assert m.device_status() == 2 and m.device_status() == 0
+            assert torch.equal(got[0, rows], x[0, rows]) and aux.isnan()
+            assert m.last["row_of"][rows].eq(-1).all() and int(m.last["offsets"][-1]) == (N - len(rows)) * k
+            assert torch.allclose(got[0, other], want[0, other], atol=1e-5, rtol=0)
+            assert m(bad, norm=norm)[0][0, rows].eq(0).all() and m.device_status() == 2
+
+
+@pytest.mark.parametrize("E,k", [(8, 2), (9, 8), (17, 3), (32, 4)])
+def test_fp32_logits_that_are_not_finite(cuda_device, E, k):
+    """Routing in one launch as the general kernel gives it: gate biases of NaN and both infinities, for some experts up
+    to all of them."""
+    d, f, N = 64, 8, 50
+    x = torch.randn(N, d, generator=torch.Generator().manual_seed(E)).to(cuda_device)
+    nan, inf = float("nan"), float("inf")
+    for i, values in enumerate([(nan,), (inf,), (-inf,), (nan, inf, -inf), (-inf,) * (E - 1), (nan,) * (E - 1),
+                                (nan,) * (E - k // 2), (nan,) * E, (inf,) * E, (-inf,) * E, (-nan, nan, -inf) * (E // 3)]):
+        params = synthetic.make_params(d, E, f, seed=i)
+        at = torch.randperm(E, generator=torch.Generator().manual_seed(i))[:len(values)]
+        params["gate_b"][at] = torch.tensor(values)
+        m = build(params, d, E, f, k, torch.float32, cuda_device)
+        with torch.no_grad():
+            m(x.view(1, N, d))
+        _, idx, w, _ = helpers.router(x, m.gate.weight.detach(), m.gate.bias.detach(), k)
+        last = m.last
+        assert torch.equal(last["idx"], idx), values
+        assert torch.allclose(last["w"], w, atol=2e-6, rtol=0, equal_nan=True), values
+        disp = helpers.dispatch(x, idx, E)
+        for name in ("offsets", "row_of", "cnt_slot"):
+            assert torch.equal(last[name], disp[name]), (values, name)
+        assert m.device_status() == int(disp["status"][0])
+
+
 def test_fp32_calls_on_two_streams_and_in_a_graph(cuda_device):
     """Two calls at once, each with a grid whose blocks wait on one another and nearly as many blocks as there are SMs; then
     both from one graph."""
