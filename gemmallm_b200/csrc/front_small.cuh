@@ -109,7 +109,9 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
   const int g = lane >> 2, t = lane & 3;
   constexpr int ET_C = 8 * NT;
   const int ET = ET_C;
-  if (tid < E) s_bias[tid] = to_f32(bg[tid]);   // visible after the barrier behind part A
+  // the router's weights and biases may have been written by the kernel before this one: read behind the wait, never as
+  // data that is constant over the kernel's life
+  if (tid < E) s_bias[tid] = to_f32(__ldcg(bg + tid));   // visible after the barrier behind part A
 
   // ---- A. partial logits -----------------------------------------------------
   if constexpr (F32) {
@@ -127,7 +129,7 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
       const float4 v = __ldcg(xr + c);     // (x may be the output of the kernel before this one)
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
-        const float4 w = __ldg(w4 + (size_t)min(8 * j + e0, E - 1) * n4 + c);
+        const float4 w = ld_behind_wait(w4 + (size_t)min(8 * j + e0, E - 1) * n4 + c);
         a[j].x = fmaf(v.x, w.x, a[j].x);
         a[j].y = fmaf(v.y, w.y, a[j].y);
         a[j].z = fmaf(v.z, w.z, a[j].z);
@@ -181,7 +183,7 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
           for (int j = 0; j < NT; ++j) {
             const int row = 8 * j + g;
             const uint4 w = (row < E && c < nchunk && piece < row_pieces)
-                                ? __ldg(w4 + (size_t)row * row_pieces + piece) : zero;
+                                ? ld_behind_wait(w4 + (size_t)row * row_pieces + piece) : zero;
             mma_bf16_16816(acc[j], A[u].x, B[u].x, A[u].y, B[u].y, w.x, w.y);
             mma_bf16_16816(acc[j], A[u].z, B[u].z, A[u].w, B[u].w, w.z, w.w);
           }

@@ -447,29 +447,42 @@ def test_decode_tiny_entry_point(cuda_device, N, d, f, E, k):
         assert (got - ref)[ok].norm() <= 2e-2 * ref[ok].norm()
 
 
-@pytest.mark.parametrize("N,d,E", [(1, 1024, 8), (3, 2048, 16), (2, 264, 32)])
-def test_decode_tiny_behind_the_kernel_that_writes_the_router_weights(cuda_device, N, d, E):
-    """The kernel in front writes the weights and lets its dependents go early: the routing is that of the new weights.
-    (A kernel that spins in front of both has them in the queue together.)"""
+@pytest.mark.parametrize("N,d,E", [(1, 1024, 8), (3, 2048, 16), (2, 264, 32), (20, 1024, 8), (100, 264, 32)])
+def test_routing_behind_the_kernel_that_writes_the_router_weights(cuda_device, N, d, E):
+    """The kernel in front writes the weights and lets its dependents go early: the routing (one-launch decode, and beyond
+    eight tokens the single-launch front) is that of the new weights. (A kernel that spins in front of both has them in
+    the queue together.)"""
     dt, f, k = torch.bfloat16, 64, 2
     params = helpers.rounded_params(synthetic.make_params(d, E, f, seed=d), dt)
     dp = helpers.device_params(params, dt, cuda_device)
     plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
     x = synthetic.make_input(N, d, seed=N).to(dt).to(cuda_device)
+
+    def route(gate):
+        if N <= 8:
+            return helpers.decode_tiny(x, gate, dp["gate_b"], plan, k, f)["logits"]
+        i32, f32 = dict(dtype=torch.int32, device=cuda_device), dict(dtype=torch.float32, device=cuda_device)
+        outs = [torch.empty(N, E, **f32), torch.empty(N, k, **i32), torch.empty(N, k, **f32), torch.empty(k, E, **i32),
+                torch.empty(E + 1, **i32), torch.empty(N, k, **i32), torch.empty(N * k, d, dtype=dt, device=cuda_device),
+                torch.empty(E, **f32), torch.empty(1, **f32)]
+        check(lib.moe_b200_front_small(x.data_ptr(), gate.data_ptr(), dp["gate_b"].data_ptr(), N, d, E, k, _cabi.BF16,
+                                       *(t.data_ptr() for t in outs), helpers.stream(cuda_device)), "front_small")
+        return outs[0]
+
     row_of = torch.arange(E, dtype=torch.int32, device=cuda_device).view(E, 1)
     idx, w = torch.zeros_like(row_of), torch.ones(E, 1, device=cuda_device)
     g = torch.Generator().manual_seed(E)
     parts = [torch.randn(1, E, d, generator=g).to(cuda_device) for _ in range(8)]
-    want = [helpers.combine_decode(p, row_of, idx, w, plan) for p in parts]
+    gates = [helpers.combine_decode(p, row_of, idx, w, plan) for p in parts]
     torch.cuda.synchronize()
-    want = [helpers.decode_tiny(x, gate, dp["gate_b"], plan, k, f) for gate in want]
+    want = [route(gate) for gate in gates]
     torch.cuda.synchronize()
     for i, p in enumerate(parts):
         torch.cuda._sleep(2_000_000)
         gate = helpers.combine_decode(p, row_of, idx, w, plan)
-        got = helpers.decode_tiny(x, gate, dp["gate_b"], plan, k, f)
+        got = route(gate)
         torch.cuda.synchronize()
-        assert torch.equal(got["logits"], want[i]["logits"]) and torch.equal(got["out"], want[i]["out"]), i
+        assert torch.equal(got, want[i]), i
         gate.zero_()          # what the next round's weights, at this address, hold before they are written
 
 
