@@ -156,10 +156,11 @@ __device__ __forceinline__ void split8(const float (&x)[8], uint32_t (&p0)[4], u
   }
 }
 
+// (a: the rows may come from the kernel before this one, so they are not read as constant data)
 __device__ __forceinline__ float dot_f32(const float* a, const float* w, int K) {
   float s = 0.f;
 #pragma unroll 1
-  for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
+  for (int k = 0; k < K; ++k) s = fmaf(__ldcg(a + k), w[k], s);
   return s;
 }
 __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= FLT_MAX; }
