@@ -10,8 +10,12 @@
 // products a0 b0 stay in its accumulator for 64 of K only and are then added, rounded to nearest, to fp32 registers;
 // the five small ones, 2^-8 of them, are summed apart over all of K.
 //
-// Infinities and NaN do not survive the split (inf - inf). Every output whose sum is not finite is therefore formed
-// again by an fp32 loop over K, which gives what fp32 arithmetic gives.
+// Infinities and NaN survive in the first parts only (the others are inf - inf): the large products say what becomes of
+// them. Small products that are not finite are therefore left out and noted (an infinity times a value under bf16's
+// smallest, 2^-133, so counts as one times zero). Where a sum is finite without them, with operands near the end of fp32's
+// range, it is formed again by an fp32 loop over K, which gives what fp32 arithmetic gives. Forming every sum that was not
+// finite that way made calls slow that hold infinities: 512 tokens, d 512, f 2048, 8 experts, top-2 took 8500 us with one
+// infinite weight and 19800 with an infinity in every token, now 105 and 110; without any 101.3 and now 102.9, for looking.
 //
 // Tile: 128 weight rows (the GEGLU pass: 64 gate and the 64 up rows of the same features) are the A operand, up to 160
 // tokens of one expert the B operand, N = their number rounded up to 16: the pipe's time is in proportion to N from 64
@@ -122,6 +126,11 @@ __device__ __forceinline__ void ld_tmem8(uint32_t taddr, uint32_t (&u)[8]) {
                : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
                : "r"(taddr));
 }
+__device__ __forceinline__ void st_tmem8(uint32_t taddr, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
 template <int N>
 __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
@@ -141,12 +150,18 @@ __device__ __forceinline__ uint64_t desc64(uint32_t saddr) {
          (uint64_t)4 << 61;
 }
 
+// Two values cut off to bf16, NaN to NaN (whose upper half alone may be an infinity's).
+__device__ __forceinline__ uint32_t cut_bf16x2(float lo, float hi) {
+  uint32_t v;
+  asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+  return v;
+}
 // Eight values into their three bf16 parts, exactly (where they are finite).
 __device__ __forceinline__ void split8(const float (&x)[8], uint32_t (&p0)[4], uint32_t (&p1)[4], uint32_t (&p2)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const uint32_t u0 = __float_as_uint(x[2 * i]), u1 = __float_as_uint(x[2 * i + 1]);
-    p0[i] = __byte_perm(u0, u1, 0x7632);
+    p0[i] = cut_bf16x2(x[2 * i], x[2 * i + 1]);
     float r0 = x[2 * i] - __uint_as_float(u0 & 0xffff0000u);
     float r1 = x[2 * i + 1] - __uint_as_float(u1 & 0xffff0000u);
     p1[i] = pack_bf16x2(r0, r1);
@@ -157,10 +172,10 @@ __device__ __forceinline__ void split8(const float (&x)[8], uint32_t (&p0)[4], u
 }
 
 // (a: the rows may come from the kernel before this one, so they are not read as constant data)
-__device__ __forceinline__ float dot_f32(const float* a, const float* w, int K) {
+__device__ __forceinline__ float dot_f32(const float* a, const float* w, int k0, int k1) {
   float s = 0.f;
 #pragma unroll 1
-  for (int k = 0; k < K; ++k) s = fmaf(__ldcg(a + k), w[k], s);
+  for (int k = k0; k < k1; ++k) s = fmaf(__ldcg(a + k), w[k], s);
   return s;
 }
 __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= FLT_MAX; }
@@ -417,6 +432,8 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
       for (int g = 0; g < kGroups; ++g)
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
+      uint64_t again = 0;      // a bit per sum of this thread whose small products were not finite, ...
+      uint32_t again_hi = 0;   // ... from the ninth group on
       auto add = [&](int col) {
         // (groups past n hold old sums; they are not used)
 #pragma unroll
@@ -435,6 +452,36 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
             }
         }
       };
+      // Small products that are not finite become zero, in tensor memory, and are noted.
+      auto keep_finite = [&]() {
+        static_assert(kGroups % 2 == 0 && kGroups <= 12, "two groups at a time, 96 bits");
+#pragma unroll 1
+        for (int g0 = 0; (g0 * 2 + part) * 8 < tl.n; g0 += 2) {
+          uint32_t v[2][8];
+          ld_tmem8(ta + kSmallCol + g0 * 16, v[0]);
+          ld_tmem8(ta + kSmallCol + g0 * 16 + 16, v[1]);
+          tc_ld_wait();
+          float probe[2] = {0.f, 0.f};      // times zero: NaN where one is not finite
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            probe[0] = fmaf(__uint_as_float(v[0][i]), 0.f, probe[0]);
+            probe[1] = fmaf(__uint_as_float(v[1][i]), 0.f, probe[1]);
+          }
+          if (__any_sync(0xffffffffu, probe[0] + probe[1] != 0.f)) {
+            uint32_t bits = 0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (!finite(__uint_as_float(v[i >> 3][i & 7]))) {
+                v[i >> 3][i & 7] = 0u;
+                bits |= 1u << i;
+              }
+            st_tmem8(ta + kSmallCol + g0 * 16, v[0]);
+            st_tmem8(ta + kSmallCol + g0 * 16 + 16, v[1]);
+            st_tmem_wait();
+            if (g0 < 8) again |= (uint64_t)bits << (g0 * 8); else again_hi |= bits << (g0 * 8 - 64);
+          }
+        }
+      };
       for (int i = 1; i <= kn; ++i) {
         if (i % kLargeSteps == 0 || i == kn) {
           if (!warp_wait(&ctl->main_full, larges & 1u, ctl, status, 47)) { ok = false; break; }
@@ -449,12 +496,37 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           if (!warp_wait(&ctl->small_full, smalls & 1u, ctl, status, 48)) { ok = false; break; }
           ++smalls;
           tc_fence_after();
+          keep_finite();
           add(kSmallCol);
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl->small_empty);
         }
       }
+      if (!ok && splits <= 1) break;
+      const float* W = static_cast<const float*>(Wp[tl.e]);
+      const int feat = tl.m * kFeatures + (GEGLU ? quad * 16 + (lane & 15) : quad * 32 + lane);
+      const bool feat_ok = feat < Nout;
+      // The sums at hand, of eight tokens from c0 on: those that lack their small products and are finite without them are
+      // formed again, over this CTA's range of K.
+      auto form_again = [&](int c0) {
+        const uint32_t bits = (uint32_t)again & 0xffu;
+        again = again >> 8 | (uint64_t)again_hi << 56;
+        again_hi >>= 8;
+        if (bits != 0u && feat_ok) {
+          float v[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = acc[0][i];
+          const float* w = W + (int64_t)(GEGLU && lane >= 16 ? Nout + feat : feat) * K;
+#pragma unroll 1
+          for (int i = 0; i < 8 && c0 + i < tl.rows; ++i)
+            if ((bits >> i & 1u) != 0u && finite(v[i]))
+              v[i] = dot_f32(A + (int64_t)(tl.row0 + c0 + i) * K, w, kb0 * BK, min(K, (kb0 + kn) * BK));
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[0][i] = v[i];
+        }
+        __syncwarp();
+      };
       if (splits > 1) {
         // Eight tokens at a time go to the CTAs in turn, which keep them as [eight][source][128 rows][8 tokens] in
         // their raw stages.
@@ -463,6 +535,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
         const uint32_t mine = smem_u32(smem) + (uint32_t)((rank * kRowsA + quad * 32 + lane) * 32);
 #pragma unroll 1
         for (int g = part; g * 8 < tl.n; g += 2, next_group(acc)) {
+          form_again(g * 8);
           const uint32_t to = map_to_cta(mine, g & (splits - 1)) + (uint32_t)((g & -splits) * kRowsA * 32);
           st_cluster4(to, acc[0][0], acc[0][1], acc[0][2], acc[0][3]);
           st_cluster4(to + 16, acc[0][4], acc[0][5], acc[0][6], acc[0][7]);
@@ -470,32 +543,13 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
         sent = true;
         break;
       }
-      if (!ok) break;
-      const float* W = static_cast<const float*>(Wp[tl.e]);
       const float* bias = static_cast<const float*>(bp[tl.e]);
-      const int feat = tl.m * kFeatures + (GEGLU ? quad * 16 + (lane & 15) : quad * 32 + lane);
-      const bool feat_ok = feat < Nout;
       const float b0 = feat_ok ? __ldg(bias + feat) : 0.f;
       const float b1 = GEGLU && feat_ok ? __ldg(bias + Nout + feat) : 0.f;
       // rolled, and the sums moved up: unrolled, 60 KB of code that runs from a cold instruction cache took 30000 clk
 #pragma unroll 1
       for (int c0 = part * 8; c0 < tl.rows; c0 += 16, next_group(acc)) {
-        // sums that are not finite are formed again (see the top)
-        bool fine = true;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) fine = fine && finite(acc[0][i]);
-        if (!fine && feat_ok) {
-          float v[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = acc[0][i];
-          const float* w = W + (int64_t)(GEGLU && lane >= 16 ? Nout + feat : feat) * K;
-#pragma unroll 1
-          for (int i = 0; i < 8 && c0 + i < tl.rows; ++i)
-            if (!finite(v[i])) v[i] = dot_f32(A + (int64_t)(tl.row0 + c0 + i) * K, w, K);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc[0][i] = v[i];
-        }
-        __syncwarp();
+        form_again(c0);
         float* o = out + (int64_t)(tl.row0 + c0) * Nout + feat;
         if (GEGLU) {
           // lanes 0-15 (gate) take tokens c0 + i, lanes 16-31 (up) tokens c0 + i + 1, i even
@@ -523,7 +577,6 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
       cluster_sync();                // the sums of all ranges are there (or a wait ran out, and the status says so)
       if (first < total) {
         const Tile tl = tile_of(ctl, E, m_tiles, first);
-        const float* W = static_cast<const float*>(Wp[tl.e]);
         const float* bias = static_cast<const float*>(bp[tl.e]);
         auto sum4 = [&](const float* p, float (&v)[4]) {
 #pragma unroll
@@ -545,20 +598,6 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
             float v[8];
             sum4(p, reinterpret_cast<float(&)[4]>(v[0]));
             if (GEGLU) sum4(p + 16 * 8, reinterpret_cast<float(&)[4]>(v[4]));
-            bool fine = true;
-#pragma unroll
-            for (int i = 0; i < (GEGLU ? 8 : 4); ++i) fine = fine && finite(v[i]);
-            if (!fine) {
-              float s8[8];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) s8[i] = GEGLU || i < 4 ? v[i] : 0.f;
-#pragma unroll 1
-              for (int i = 0; i < 8; ++i)
-                if (c0 + (i & 3) < tl.rows && !finite(s8[i]))
-                  s8[i] = dot_f32(A + (int64_t)(tl.row0 + c0 + (i & 3)) * K, W + (int64_t)(feat + (i >> 2) * Nout) * K, K);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) v[i] = s8[i];
-            }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
               if (c0 + i < tl.rows)

@@ -282,6 +282,9 @@ def test_experts_fp32_not_finite(cuda_device, rows, d, f):
     params, x, offsets = expert_inputs(rows, d, f, torch.float32, seed=d)
     x[0, 3], x[1, d - 1], x[rows[0] + 1, 5], x[2, 7] = float("inf"), float("nan"), -float("inf"), 3e38
     params["w1"][0, 9, 7], params["w2"][1, 11, 100], params["w1"][1, f + 2, 1] = 1e4, float("inf"), -float("inf")
+    # NaN whose upper half alone would be an infinity
+    for t, at in ((x, (rows[0], d // 2)), (params["w2"], (0, 13, 5))):
+        t.view(torch.int32)[at] = 0x7F800001
     dp = helpers.device_params(params, torch.float32, cuda_device)
     plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
     h, y, status = helpers.experts(x.to(cuda_device), offsets.to(cuda_device), plan)
@@ -294,6 +297,58 @@ def test_experts_fp32_not_finite(cuda_device, rows, d, f):
         assert torch.equal(got.isinf(), ref.isinf()) and torch.equal(got[got.isinf()], ref[ref.isinf()])
         ok = ref.isfinite() & (ref.abs() < 1e6)
         assert torch.allclose(got[ok], ref[ok], atol=1e-4, rtol=1e-5)
+
+
+@pytest.mark.parametrize("E,K", [(80, 256), (40, 512), (1, 1024)])        # K in one CTA, over two and over eight
+def test_experts_fp32_near_the_end_of_the_range(cuda_device, E, K):
+    """Products whose first parts cancel while the others, 2^-6 of them, sum up to more than the largest number: finite as
+    fp32 arithmetic is. Terms of one sign (1 + 2^-7 - 2^-23)^2 2^127, of the other two that outweigh them."""
+    f, top = 64, 2.0 ** 127
+    near = 1 + 2.0 ** -7 - 2.0 ** -23
+    a = torch.tensor([1.9921875 * top, near * top, near * top, 0.03125 * top] * 64)
+    b = torch.tensor([-1.0, near, near, -1.0] * 64)
+    params = synthetic.make_params(K, E, f, seed=1)
+    for t in params.values():
+        t.zero_()
+    params["b1"][:, :f] = 1.0                                   # gelu(1) as the factor of the up sums
+    params["w1"][:, f:, :256] = b
+    x = torch.zeros(2 * E, K)
+    x[:, :256] = a
+    offsets = torch.arange(E + 1, dtype=torch.int32) * 2
+    dp = helpers.device_params(params, torch.float32, cuda_device)
+    plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
+    h, _, status = helpers.experts(x.to(cuda_device), offsets.to(cuda_device), plan)
+    assert status.cpu()[0] == 0
+    want = float(F.gelu(torch.tensor(1.0, dtype=torch.float64), approximate="tanh") * (a.double() @ b.double()))
+    # 256 sums of at most 2^128, each rounded: 2^9 2^-24 2^127, where the result is 2^126
+    assert (h.cpu().double() - want).abs().max() <= 6.2e-5 * abs(want)
+
+
+def test_experts_fp32_infinities_take_no_longer(cuda_device):
+    """With an infinite weight, and an infinity in every token, within a few times the time without (85 and 200 times as
+    long when each sum that was not finite was formed again)."""
+    rows, d, f = [128] * 8, 512, 2048
+    params, x, offsets = expert_inputs(rows, d, f, torch.float32, seed=4)
+    offsets = offsets.to(cuda_device)
+
+    def best(params, x):
+        dp = helpers.device_params(params, torch.float32, cuda_device)
+        plan, xd, times = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"]), x.to(cuda_device), []
+        for _ in range(6):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            helpers.experts(xd, offsets, plan)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times)
+
+    clean = best(params, x)
+    params["w1"][:, 9, 7] = float("inf")
+    assert best(params, x) < 8 * clean
+    params["w1"][:, 9, 7] = 0.5
+    x[:, 5] = float("inf")
+    assert best(params, x) < 8 * clean
 
 
 # the down product with its contraction split over the pairs of a cluster: four and two ranges, the last one shorter,
