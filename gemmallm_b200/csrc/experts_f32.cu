@@ -3,12 +3,14 @@
 //   h = gelu_tanh(x W1[:f]^T + b1[:f]) * (x W1[f:]^T + b1[f:])   (model.py:174,180-182)
 //   y = h W2^T + b2                                               (model.py:184)
 //
-// Every fp32 operand is the exact sum of three bf16 values (24 = 8 + 8 + 8 bits of mantissa; bf16 has fp32's range),
-// and six of the nine products of parts make up the fp32 product to 2^-24 of it: a0 b0, a0 b1, a1 b0, a1 b1, a0 b2,
-// a2 b0. a0 is cut off, not rounded, so that nothing overflows; a1 and a2 are rounded, so that what is left out has
-// either sign. The tensor core adds with truncation, which would make long sums drift towards zero: the large
-// products a0 b0 stay in its accumulator for 64 of K only and are then added, rounded to nearest, to fp32 registers;
-// the five small ones, 2^-8 of them, are summed apart over all of K.
+// Every fp32 operand of 2^-110 or more is the exact sum of three bf16 values (24 = 8 + 8 + 8 bits of mantissa; the third of
+// a smaller one falls under bf16's smallest, and up to 2^-133 is left out), and six of the nine products of parts make up
+// the fp32 product to 2^-24 of it: a0 b0, a0 b1, a1 b0, a1 b1, a0 b2, a2 b0 (after Henry, Tang and Heinecke, "Leveraging the
+// bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", ARITH 2019). a0 is cut off, not rounded, so
+// that nothing overflows; a1 and a2 are rounded, so that what is left out has either sign. The tensor core adds with
+// truncation, which would make long sums drift towards zero: the large products a0 b0 stay in its accumulator for 64 of K
+// only and are then added, rounded to nearest, to fp32 registers; the five small ones, 2^-8 of them, are summed apart over
+// 256 of K.
 //
 // Infinities and NaN survive in the first parts only (the others are inf - inf): the large products say what becomes of
 // them. Small products that are not finite are therefore left out and noted (an infinity times a value under bf16's

@@ -351,6 +351,54 @@ def test_experts_fp32_infinities_take_no_longer(cuda_device):
     assert best(params, x) < 8 * clean
 
 
+def test_experts_fp32_small_operands(cuda_device):
+    """Down to 2^-110 an operand is the sum of its three parts; below, what is left out is under 2^-133 of one. Rows around
+    2^-104 and 2^-112, results normal numbers."""
+    d, f, n = 256, 64, 48
+    params, x, offsets = expert_inputs([n, n], d, f, torch.float32, seed=2)
+    for t in (params["w1"][:, :f], params["b1"], params["b2"]):
+        t.zero_()
+    params["b1"][:, :f] = 1.0
+    scale = torch.cat([torch.full((n, 1), 2.0 ** -104), torch.full((n, 1), 2.0 ** -112)])
+    x *= scale
+    dp = helpers.device_params(params, torch.float32, cuda_device)
+    plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
+    h, _, status = helpers.experts(x.to(cuda_device), offsets.to(cuda_device), plan)
+    assert status.cpu()[0] == 0
+    up = torch.cat([F.linear(x[:n].double(), params["w1"][0, f:].double()), F.linear(x[n:].double(), params["w1"][1, f:].double())])
+    want = F.gelu(torch.ones_like(up), approximate="tanh") * up
+    weight = torch.cat([params["w1"][e, f:].double().abs().sum(1).expand(n, f) for e in range(2)])
+    err = (h.cpu().double() - want).abs()
+    # the sums' rounding (as in test_experts_fp32_against_64_bits, elementwise and not in the 2-norm), and 2^-133 an operand
+    assert (err <= 2e-6 * want.abs().mean(1, keepdim=True) + 2.0 ** -133 * weight).all()
+
+
+def test_gelu_of_the_fp32_experts(cuda_device):
+    """Element by element against 64 bits: where the exponential underflows, where it no longer counts beside 1, where the
+    quotient's correction ends (a denominator of 1e37), very large arguments, infinities and NaN."""
+    inf = float("inf")
+    g = torch.cat([torch.linspace(-15, 15, 6001), torch.linspace(-10.2, -9.2, 4001), torch.linspace(4, 7, 2001),
+                   torch.logspace(-42, 2, 500), -torch.logspace(-42, 2, 500),
+                   torch.tensor([0.0, -0.0, 1e30, -1e30, 3e38, -3e38, inf, -inf, float("nan")])])
+    f = (g.numel() + 7) // 8 * 8
+    b1 = torch.ones(1, 2 * f)
+    b1[0, :g.numel()] = g
+    dev = [t.to(cuda_device) for t in (torch.zeros(1, 2 * f, 8), b1, torch.zeros(1, 8, f), torch.zeros(1, 8))]
+    h, _, status = helpers.experts(torch.zeros(1, 8, device=cuda_device),
+                                   torch.tensor([0, 1], dtype=torch.int32, device=cuda_device), helpers.Plan(*dev))
+    assert status.cpu()[0] == 0
+    got, g = h[0, :g.numel()].cpu().double(), g.double()
+    t = 2 * (2 / torch.pi) ** 0.5 * (g + 0.044715 * g ** 3)
+    want = g * torch.sigmoid(t)          # g / 2 (1 + tanh(t / 2)) without its cancellation
+    want[g == -inf] = float("nan")       # -inf * 0, as torch's own
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    ok = want.isfinite()
+    # t is rounded five times (and its constants), which the exponential turns into |t| times that of its value; then the
+    # exponential (2 ulp), the sum, the quotient; under 2^-120 the approximate reciprocal has become zero
+    bound = (5 * t.abs().clamp(max=100) + 6) * 2.0 ** -24 * want.abs() + 2.0 ** -120
+    assert ((got - want).abs() <= bound)[ok].all()
+
+
 # the down product with its contraction split over the pairs of a cluster: four and two ranges, the last one shorter,
 # K that is no multiple of 64, a last tile of 8 columns, odd CTAs without rows, an expert without rows; 33 tiles: none
 @pytest.mark.parametrize("rows,d,f", [([700], 1024, 2056), ([300, 1, 0, 40], 520, 1032), ([2048], 1024, 1024),
