@@ -289,7 +289,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
         const CUtensorMap* tw = tmap_w + tl.e;
         const int r0 = tl.m * kFeatures, r1 = GEGLU ? Nout + r0 : r0 + 64;
         for (int i = 0; i < kn; ++i) {
-          if (!mbar_wait(&ctl->raw_empty[s], phase ^ 1u, &ctl->abort, status, 41)) { ok = false; break; }
+          if (!mbar_wait(&ctl->raw_empty[s], phase ^ 1u, &ctl->abort, status, 51)) { ok = false; break; }
           uint8_t* dst = smem + (size_t)s * kRawBytes;
           const int k = (kb0 + i) * BK;
           mbar_expect_tx(&ctl->raw_full[s], (uint32_t)(kRawA + tl.n * BK * 4));
@@ -309,9 +309,9 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
         const Tile tl = tile_of(ctl, E, m_tiles, t);
         const uint32_t idesc = make_idesc(tl.n);
         for (int i = 0; i < kn; ++i) {
-          if (!warp_wait(&ctl->conv_full[c], phase, ctl, status, 43)) { ok = false; break; }
+          if (!warp_wait(&ctl->conv_full[c], phase, ctl, status, 53)) { ok = false; break; }
           if (i % kLargeSteps == 0) {
-            if (!warp_wait(&ctl->main_empty, (larges & 1u) ^ 1u, ctl, status, 44)) { ok = false; break; }
+            if (!warp_wait(&ctl->main_empty, (larges & 1u) ^ 1u, ctl, status, 54)) { ok = false; break; }
             ++larges;
           }
           tc_fence_after();
@@ -328,7 +328,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           }
           __syncwarp();
           if (i % kSmallSteps == 0) {
-            if (!warp_wait(&ctl->small_empty, (smalls & 1u) ^ 1u, ctl, status, 42)) { ok = false; break; }
+            if (!warp_wait(&ctl->small_empty, (smalls & 1u) ^ 1u, ctl, status, 52)) { ok = false; break; }
             tc_fence_after();
             ++smalls;
           }
@@ -374,8 +374,8 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
         if (turn != group) continue;
         // In this order: boxes may land out of order, and with the other group's last turn on this stage still to come its
         // barrier would be a phase behind and this parity would look done. The products of that turn are done first.
-        if (!warp_wait(&ctl->conv_empty[c], ph ^ 1u, ctl, status, 46)) { ok = false; break; }
-        if (!warp_wait(&ctl->raw_full[c], ph, ctl, status, 45)) { ok = false; break; }
+        if (!warp_wait(&ctl->conv_empty[c], ph ^ 1u, ctl, status, 56)) { ok = false; break; }
+        if (!warp_wait(&ctl->raw_full[c], ph, ctl, status, 55)) { ok = false; break; }
         tc_fence_after();
         const uint8_t* raw = smem + (size_t)c * kRawBytes;
         const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + kACol + c * kACols + part * 8;
@@ -486,7 +486,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
       };
       for (int i = 1; i <= kn; ++i) {
         if (i % kLargeSteps == 0 || i == kn) {
-          if (!warp_wait(&ctl->main_full, larges & 1u, ctl, status, 47)) { ok = false; break; }
+          if (!warp_wait(&ctl->main_full, larges & 1u, ctl, status, 57)) { ok = false; break; }
           ++larges;
           tc_fence_after();
           add(kMainCol);
@@ -495,7 +495,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           if (lane == 0) mbar_arrive(&ctl->main_empty);
         }
         if (i % kSmallSteps == 0 || i == kn) {
-          if (!warp_wait(&ctl->small_full, smalls & 1u, ctl, status, 48)) { ok = false; break; }
+          if (!warp_wait(&ctl->small_full, smalls & 1u, ctl, status, 58)) { ok = false; break; }
           ++smalls;
           tc_fence_after();
           keep_finite();
