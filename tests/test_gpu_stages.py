@@ -164,6 +164,55 @@ def test_dispatch_copies_rows_of_any_width(cuda_device, dtype, d):
     assert torch.equal(out["perm"][flat].view(N, k, d), x[:, None, :].expand(N, k, d))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_dispatch_normalises_with_weights_at_any_address(cuda_device, dtype, aligned):
+    """The folded LayerNorm with gamma and beta on and off a 16-byte boundary; statistics as given."""
+    N, d, E, k = 700, 136, 8, 2
+    g = torch.Generator().manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(dtype)
+    x, gamma, beta = rnd(N, d), rnd(d), rnd(d)
+    stats = torch.stack([torch.randn(N, generator=g), torch.rand(N, generator=g) + 0.5], dim=1)
+    at = 0 if aligned else 1
+    place = lambda t: torch.cat([torch.zeros(at, dtype=dtype), t]).to(cuda_device)[at:]
+    gd, bd, xd, sd = place(gamma), place(beta), x.to(cuda_device), stats.to(cuda_device)
+    assert (gd.data_ptr() % 16 == 0) == aligned
+    idx = torch.rand(N, E, generator=g).topk(k, dim=1).indices.to(torch.int32).to(cuda_device)
+    i32 = dict(dtype=torch.int32, device=cuda_device)
+    scratch = torch.empty(lib.moe_b200_dispatch_scratch_bytes(N, E, k) // 4, **i32)
+    cnt, offsets, row_of = torch.empty(k, E, **i32), torch.empty(E + 1, **i32), torch.empty(N, k, **i32)
+    perm, status = torch.empty(N * k, d, dtype=dtype, device=cuda_device), torch.zeros(16, **i32)
+    check(lib.moe_b200_dispatch_norm(xd.data_ptr(), idx.data_ptr(), sd.data_ptr(), gd.data_ptr(), bd.data_ptr(), N, d, E, k,
+                                     helpers.CODE[dtype], scratch.data_ptr(), cnt.data_ptr(), offsets.data_ptr(),
+                                     row_of.data_ptr(), perm.data_ptr(), None, None, None, status.data_ptr(),
+                                     helpers.stream(cuda_device)), "dispatch_norm")
+    assert status.cpu()[0] == 0
+    want = (x.double() - stats[:, :1].double()) * stats[:, 1:].double() * gamma.double() + beta.double()
+    got = perm[row_of.long().flatten()].view(N, k, d).cpu().double()
+    # three rounded operations, and the rounding of the result
+    size = ((x.double() - stats[:, :1].double()) * stats[:, 1:].double() * gamma.double()).abs() + beta.double().abs()
+    bound = 2.0 ** -22 * size + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs()
+    assert ((got - want[:, None]).abs() <= bound[:, None]).all()
+
+
+# rows kept in registers (up to 1024, up to 2048 wide) and read again, a lane's last piece missing
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("N,d", [(9, 8), (3, 1024), (17, 1032), (8, 2040), (5, 2048), (3, 2056), (2, 8200)])
+def test_layernorm_rows_of_any_width(cuda_device, dtype, N, d):
+    g = torch.Generator().manual_seed(d)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(dtype)
+    x, gamma, beta = rnd(N, d) * 2 + 1, rnd(d), rnd(d)
+    dev = [t.to(cuda_device) for t in (x, gamma, beta)]
+    out = torch.full_like(dev[0], float("nan"))
+    check(lib.moe_b200_layernorm(*[t.data_ptr() for t in dev], 1e-5, N, d, helpers.CODE[dtype], out.data_ptr(),
+                                 helpers.stream(cuda_device)), "layernorm")
+    want = F.layer_norm(x.double(), (d,), gamma.double(), beta.double(), 1e-5)
+    # sums of d / 32 terms a lane and five of the lanes' in fp32, against a deviation of 2: 2^-24 (d / 32 + 5) of the values
+    eps = (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+    bound = eps * want.abs() + 2.0 ** -24 * (d / 32 + 16) * (want.abs() + gamma.double().abs() + 1)
+    assert ((out.cpu().double() - want).abs() <= bound).all()
+
+
 def test_dispatch_reports_bad_index(cuda_device):
     x = torch.randn(10, 64, device=cuda_device)
     idx = torch.zeros(10, 2, dtype=torch.int32, device=cuda_device)
@@ -548,6 +597,24 @@ def test_decode_tiny_entry_point(cuda_device, N, d, f, E, k):
         got = r["out"].float().cpu()
         assert (got - ref)[ok].abs().max() <= 2e-2 * ref.abs().max()
         assert (got - ref)[ok].norm() <= 2e-2 * ref[ok].norm()
+
+
+def test_decode_tiny_copies_rows_wider_than_the_grid(cuda_device):
+    """More 16-byte pieces of rows than the grid has threads: the rest is copied ahead of the grid barrier."""
+    N, d, f, E, k, dt = 4, 43304, 8, 32, 7, torch.bfloat16
+    params = helpers.rounded_params(synthetic.make_params(d, E, f, seed=7), dt)
+    dp = helpers.device_params(params, dt, cuda_device)
+    x = synthetic.round_to(synthetic.make_input(N, d, seed=8), dt)
+    r = helpers.decode_tiny(x.to(dt).to(cuda_device), dp["gate_w"], dp["gate_b"],
+                            helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"]), k, f)
+    torch.cuda.synchronize()
+    assert N * k * d // 8 > torch.cuda.get_device_properties(cuda_device).multi_processor_count * 1024
+    rows = r["row_of"].long()
+    assert int(r["status"][0]) == 0 and torch.equal(rows.flatten().sort().values, torch.arange(N * k, device=cuda_device))
+    assert torch.equal(r["perm"][rows].cpu(), x.to(dt)[:, None, :].expand(N, k, d))
+    o = moe_oracle.moe_forward(x, params, k, logits=r["logits"].cpu())
+    assert torch.equal(r["idx"].cpu().long(), o["idx"])
+    assert (r["out"].float().cpu() - o["out"]).norm() <= 2e-2 * o["out"].norm()
 
 
 @pytest.mark.parametrize("N,d,E", [(1, 1024, 8), (3, 2048, 16), (2, 264, 32), (20, 1024, 8), (100, 264, 32)])
