@@ -24,9 +24,8 @@ front_small_kernel(const T* __restrict__ x, const T* __restrict__ Wg,
   extern __shared__ float smem[];
   pdl_wait();                 // x may come from the kernel before this one
   pdl_launch_dependents();
-  front_small_body<NT, SPLIT, T>(smem, (int)blockIdx.x, (int)gridDim.x, x, Wg, bg, Ntotal, d, E, k,
-                              out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux,
-                              xch, counter, status);
+  front_small_body<NT, SPLIT, T>(smem, x, Wg, bg, Ntotal, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
+                                 row_of, perm, psum, aux, xch, counter, status);
 }
 
 template <int NT, typename T>

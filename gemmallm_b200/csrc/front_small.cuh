@@ -60,14 +60,14 @@ using front_detail::ld_acquire_gpu_i32;
 //   98.0 with the barrier). Same results as the other form
 //   except for the order in which the logits' partial sums are added.
 //
-// `blk` of `nblk`: the calling block's place; `smem`: front_small_smem_bytes() of shared memory.
+// `smem`: front_small_smem_bytes() of shared memory.
 __host__ __device__ inline size_t front_small_smem_bytes(int NT, int ntok, int E, int k) {
   return sizeof(float) * ((size_t)32 * 16 * 8 * NT + (size_t)ntok * (E + 1)) +
          sizeof(int) * (2 * (size_t)ntok * k + 2 * kMaxTopK * kFrontMaxE + 4 * kFrontMaxE + 1);
 }
 
 template <int NT, bool SPLIT, typename T = __nv_bfloat16>  // n-tiles of 8 experts: E <= 8*NT
-__device__ __forceinline__ void front_small_body(float* smem, const int blk, const int nblk,
+__device__ __forceinline__ void front_small_body(float* smem,
                  const T* __restrict__ x, const T* __restrict__ Wg, const T* __restrict__ bg, int Ntotal, int d, int E, int k,
                  float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                  float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
@@ -78,6 +78,7 @@ __device__ __forceinline__ void front_small_body(float* smem, const int blk, con
   constexpr int kThreads = kFrontThreads;
   constexpr int kMaxE = kFrontMaxE;
   constexpr bool F32 = sizeof(T) == 4;
+  const int blk = (int)blockIdx.x, nblk = (int)gridDim.x;
   static_assert(!F32 || SPLIT, "fp32: blocks of 16 tokens");
   constexpr int kPiece = 16 / sizeof(T);                   // elements of a 16-byte piece
   const int ld = E + 1;
