@@ -475,6 +475,7 @@ decode_tiny_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
           float o = 0.f;
           for (int j = 0; j < k; ++j) {
             const int r = rt->row[tok * k + j];
+            if (r < 0) continue;      // (never; without the test the kernel spills 104 bytes instead of 68: one token 22.6 us, not 21.1)
             o = __fadd_rn(o, __fmul_rn(rt->wgt[tok * k + j], s_y[r * 8 + col]));
           }
           const size_t at = (size_t)tok * d + c0 + col;
