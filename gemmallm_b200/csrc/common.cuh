@@ -166,17 +166,6 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// 16 bytes that the kernel before this one may have written and that several warps of a block read: an ordinary load
-// (L1 serves it again), which stays behind pdl_wait()
-__device__ __forceinline__ uint4 ld_behind_wait(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 ld_behind_wait(const float4* p) {
-  const uint4 v = ld_behind_wait(reinterpret_cast<const uint4*>(p));
-  return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
-}
 
 // cluster: blocks per cluster along x, 0 for none (or a compile-time __cluster_dims__); whole: a cooperative launch, all
 // blocks resident at once

@@ -13,8 +13,7 @@ constexpr int kMaxPairs = kFrontMaxPairs;
 
 template <int NT, bool SPLIT, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-front_small_kernel(const T* __restrict__ x, const T* __restrict__ Wg,
-                   const T* __restrict__ bg, int Ntotal, int d, int E, int k,
+front_small_kernel(const T* __restrict__ x, const T* Wg, const T* bg, int Ntotal, int d, int E, int k,
                    float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                    float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
                    int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,

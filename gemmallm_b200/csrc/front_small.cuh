@@ -68,7 +68,7 @@ __host__ __device__ inline size_t front_small_smem_bytes(int NT, int ntok, int E
 
 template <int NT, bool SPLIT, typename T = __nv_bfloat16>  // n-tiles of 8 experts: E <= 8*NT
 __device__ __forceinline__ void front_small_body(float* smem,
-                 const T* __restrict__ x, const T* __restrict__ Wg, const T* __restrict__ bg, int Ntotal, int d, int E, int k,
+                 const T* __restrict__ x, const T* Wg, const T* bg, int Ntotal, int d, int E, int k,
                  float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                  float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
                  int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
@@ -110,9 +110,9 @@ __device__ __forceinline__ void front_small_body(float* smem,
   const int g = lane >> 2, t = lane & 3;
   constexpr int ET_C = 8 * NT;
   const int ET = ET_C;
-  // the router's weights and biases may have been written by the kernel before this one: read behind the wait, never as
-  // data that is constant over the kernel's life
-  if (tid < E) s_bias[tid] = to_f32(__ldcg(bg + tid));   // visible after the barrier behind part A
+  // (the router's weights and biases may have been written by the kernel before this one: ordinary loads behind the wait,
+  // and no __restrict__, which would make them loads of constant data)
+  if (tid < E) s_bias[tid] = to_f32(bg[tid]);   // visible after the barrier behind part A
 
   // ---- A. partial logits -----------------------------------------------------
   if constexpr (F32) {
@@ -130,7 +130,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
       const float4 v = __ldcg(xr + c);     // (x may be the output of the kernel before this one)
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
-        const float4 w = ld_behind_wait(w4 + (size_t)min(8 * j + e0, E - 1) * n4 + c);
+        const float4 w = w4[(size_t)min(8 * j + e0, E - 1) * n4 + c];
         a[j].x = fmaf(v.x, w.x, a[j].x);
         a[j].y = fmaf(v.y, w.y, a[j].y);
         a[j].z = fmaf(v.z, w.z, a[j].z);
@@ -184,7 +184,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
           for (int j = 0; j < NT; ++j) {
             const int row = 8 * j + g;
             const uint4 w = (row < E && c < nchunk && piece < row_pieces)
-                                ? ld_behind_wait(w4 + (size_t)row * row_pieces + piece) : zero;
+                                ? w4[(size_t)row * row_pieces + piece] : zero;
             mma_bf16_16816(acc[j], A[u].x, B[u].x, A[u].y, B[u].y, w.x, w.y);
             mma_bf16_16816(acc[j], A[u].z, B[u].z, A[u].w, B[u].w, w.z, w.w);
           }
