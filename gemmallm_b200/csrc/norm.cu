@@ -55,8 +55,9 @@ norm_fold_kernel(const T* __restrict__ Wg, const T* __restrict__ bg, const T* __
 // One warp per row: mean, biased variance around the mean, y = (x - mean) * rstd * gamma + beta,
 // as torch.nn.LayerNorm. Rows of up to 256 * KEEP elements stay in the lanes' registers between the
 // three steps, as they lie in memory (one pass over memory); longer rows (KEEP = 0) are re-read (from L1).
-// What bounds it is the loads in flight: kept as floats, and with room for 2048 at every width, a row took registers
-// for two blocks an SM (32768 rows of 1024 bf16: 41 us, now 24).
+// Kept as floats, and with room for 2048 at every width, a row took registers for two blocks an SM, and the loads in
+// flight bounded it (32768 rows of 1024 bf16, nothing in L2: 39 us, now 23); now its instructions do (issue slots 79 %
+// busy, HBM 3.5 TB/s). Of a decoder layer of 32768 tokens, 1.8 ms, that is 1 %.
 template <typename T> struct RawPiece;      // eight elements
 template <> struct RawPiece<__nv_bfloat16> {
   uint4 v;
