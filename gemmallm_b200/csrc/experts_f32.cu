@@ -34,8 +34,9 @@
 // What bounds it: shared-memory bandwidth (per step of 32 at N 128: 32 KiB in by TMA, 32 read and 24 written by the
 // split, 48 read by the products, about 1060 clk of 128 bytes) and the issue slots of the split (600 clk) against 768 clk
 // of products; a step takes 1400 to 1600. 1024 rows of 8 experts, d 512, f 2048, nothing in L2: gate_and_up 160 -> 46 us,
-// both products 250 -> 77 us (packed FMA on the CUDA cores before; 45 and 75 without the look for infinities). Error of h and y against 64 bits, in the 2-norm, at 2 to
-// 4096 rows: 1.8e-7 and 0.9e-7 to 1.4e-7 (before: 2.3e-7 to 4.2e-7 and 1.6e-7).
+// both products 250 -> 77 us (packed FMA on the CUDA cores before; 45 and 75 without the look for infinities). Error of h
+// and y against 64 bits, in the 2-norm, at 2 to 4096 rows: 1.8e-7 and 0.9e-7 to 1.4e-7 (before: 2.3e-7 to 4.2e-7 and
+// 1.6e-7).
 #include <cuda.h>
 #include <cfloat>
 #include "common.cuh"
