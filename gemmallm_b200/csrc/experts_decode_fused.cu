@@ -192,7 +192,7 @@ decode_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -235,7 +235,7 @@ decode_fused_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       uint32_t acc_phase = 0;

@@ -111,11 +111,6 @@ __device__ __forceinline__ void st_tmem4(uint32_t taddr, const uint32_t (&v)[4])
                "r"(v[2]), "r"(v[3])
                : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
 // For warps that stay together: all lanes have the same answer.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, Control* ctl, int32_t* status, int where) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, &ctl->abort, status, where)) != 0;
@@ -280,7 +275,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
 
   if (warp < 4) {
     fewer_registers<kRegsLoad>();
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
       // ---------------- TMA producer ----------------
       int s = 0;
       uint32_t phase = 0;

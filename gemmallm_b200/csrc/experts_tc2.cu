@@ -307,7 +307,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ---------------- TMA producer (each CTA loads its own rows and its half of B) -------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int e = 0;
@@ -355,7 +355,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (even CTA only) ----------------
-    if (lane == 0 && cta == 0) {
+    if (cta == 0 && elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       uint32_t acc_phase = 0;
@@ -453,7 +453,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (T::DH && warp == 2 + kEpiWarps) {
     // ---------------- gate and up values: two chunks ahead, stored again as gradients ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       struct Place { int col, row; bool boxes; } place[2];
       int ci = 0, e = 0;
       auto put_back = [&](int b, int use) {      // use: how many times the buffer has been filled before
