@@ -470,14 +470,9 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   // between the decode and the prefill sizes: the streaming kernel on the sorted rows
   const bool rows_path = dtype == MOE_B200_BF16 && !small_n && N * k <= kRowsPathMaxRows &&
                          rows_supported(N * k, E);
-  // ... of which those with 192 rows an expert or more (1536 in all with fewer than four experts), as long as the down
-  // product is one round of 256 x 256 tiles, take the prefill products behind the single-launch front: the streaming
-  // kernel reads an expert's weights once per 128 rows and is bound by L2 there. Experts and combine, d 1024, f 4096,
-  // 8 experts (us, streaming / tiles): 1024 rows 79 / 81, 1536 88 / 83, 2346 109 / 101, 3072 117 / 101, 4096 (two
-  // rounds) 134 / 157. With one to three experts a few tiles take as long as a full round of them; whole calls:
-  // 1 expert, d 512, f 2048, 300 rows 38 / 44, 1500 46 / 48; d 1024, f 4096, 300 rows 44 / 52, 1500 68 / 71; d 2048,
-  // f 8192, 300 rows 72 / 86, 1500 171 / 162; 2 experts, d 1024, 500 rows 52 / 60, 1500 72 / 73; 3, 900 rows 62 / 69
-  const bool tiles = rows_path && tiles_at_row_counts(N * k, d, E);
+  // both products in one launch on tiles that fit an expert's rows: from 64 rows an expert on, and beyond these sizes to
+  // 2048 rows an expert (experts_mid.cu); with more than 32 experts, which neither kernel for few rows takes, at any number
+  const bool mid = dtype == MOE_B200_BF16 && experts_mid_chosen(N * k, E);
   // (a folded LayerNorm stays with the general kernels)
   bool front32 = dtype == MOE_B200_F32 && !norm && front_f32_supported(N, E, k);
   bool front = front32 || ((small_n || rows_path) && (front_small_supported(N, E, k, dtype) ||
@@ -491,11 +486,12 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
     if (rc) return rc;
     front = front32;
   }
-  const bool counters = small_n || rows_path;
+  const bool counters = small_n || rows_path || mid;
+  const bool clean = (small_n || rows_path) && (flags & MOE_B200_FLAG_WS_CLEAN);
   // status words, and the completion counters behind them where a kernel uses them, in one memset
   // (above these sizes a call always clears the status words: they are those of the most recent call; the fp32 front
   // clears them itself)
-  if (!front32 && !(counters && (flags & MOE_B200_FLAG_WS_CLEAN)))
+  if (!front32 && !clean)
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
   float* stats = reinterpret_cast<float*>(ws + off[MOE_B200_WS_STATS]);
@@ -537,6 +533,11 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
       if (rc) return rc;
     }
   }
+  if (mid) {
+    rc = launch_experts_mid(perm, offsets, plan, N * k, d, f, E, h, y, status + MOE_B200_READY_OFFSET, status, s);
+    if (rc) return rc;
+    return moe_b200_combine(y, row_of, w, residual, N, d, k, dtype, out, stream);
+  }
   if (small_n) {
     // few tokens per expert: weight streaming with narrow tiles and split-K
     if (spec)
@@ -548,7 +549,7 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
     return moe_b200_combine_decode(part, decode_splits(f), N * k, row_of, idx, w, plan, E, residual,
                                    N, d, k, out, stream);
   }
-  if (rows_path && !tiles) {
+  if (rows_path) {
     const int ks = rows_splits(N * k, d, f, E);
     rc = launch_experts_tc_rows(perm, offsets, plan, N * k, d, f, E, ks, h, part,
                                 status + MOE_B200_READY_OFFSET, status, s);

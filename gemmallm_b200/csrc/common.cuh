@@ -208,7 +208,8 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 // Plan buffer layout (device memory owned by the caller).
 //   [0, 4*E*8)            : W1[E], b1[E], W2[E], b2[E] device pointers
 //   then, 128-byte aligned: tensor maps (128 bytes each) W1[E], W2[E] with
-//   128-row boxes, then W1[E], W2[E] with 64-row boxes for the small-N path
+//   128-row boxes, then W1[E], W2[E] with 64-row boxes for the small-N path, then W1[E] with
+//   gate and up rows in turn (boxes of 64 columns x 2 x 64 features)
 struct PlanView {
   const void* const* W1;
   const void* const* b1;
@@ -218,8 +219,9 @@ struct PlanView {
   const void* tmap_W2;  // CUtensorMap[E]
   const void* tmap_W1_dec;
   const void* tmap_W2_dec;
+  const void* tmap_W1_pairs;
 };
-constexpr int kPlanMapsPerExpert = 4;
+constexpr int kPlanMapsPerExpert = 5;
 __host__ __device__ inline size_t plan_ptr_bytes(int E) {
   return ((size_t)4 * E * sizeof(void*) + 127) & ~(size_t)127;
 }
@@ -234,6 +236,7 @@ __host__ __device__ inline PlanView plan_view(const void* plan, int E) {
   v.tmap_W2 = p + plan_ptr_bytes(E) + (size_t)128 * E;
   v.tmap_W1_dec = p + plan_ptr_bytes(E) + (size_t)128 * 2 * E;
   v.tmap_W2_dec = p + plan_ptr_bytes(E) + (size_t)128 * 3 * E;
+  v.tmap_W1_pairs = p + plan_ptr_bytes(E) + (size_t)128 * 4 * E;
   return v;
 }
 
@@ -313,8 +316,11 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
                        int f, int E, void* h, void* y, const EpScatter* sc, int32_t* status,
                        cudaStream_t s, const TrainArgs* train = nullptr, const EpSync* ep_wait = nullptr,
                        const EpSync* ep_signal = nullptr);
-// Whether a call between the decode and the prefill sizes (M sorted rows) is better off with launch_experts_tc2.
-bool tiles_at_row_counts(int64_t M, int d, int E);
+// Both products in one launch, for calls between the decode and the prefill sizes (experts_mid.cu); `ready` as for
+// launch_experts_tc_decode_spec.
+bool experts_mid_chosen(int64_t M, int E);
+int launch_experts_mid(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d, int f, int E, void* h,
+                       void* y, int* ready, int32_t* status, cudaStream_t s);
 // Input gradient of a grouped Linear: out[rows of e] = A[rows of e] . B_e, B_e [K, Nout] row-major, given by
 // the e-th tensor map of tmaps_b (64-row boxes). With geglu_bwd the product is dh (Nout = f) and is not
 // stored: the epilogue carries it back to gu (see TrainArgs); round_dh rounds it to bf16 in between.

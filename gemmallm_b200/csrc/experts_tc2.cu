@@ -39,6 +39,7 @@
 #include <cuda.h>
 #include "common.cuh"
 #include "tc_ptx.cuh"
+#include "tc_pair.cuh"
 #include "tc_epilogue.cuh"
 #include "ep_sync.cuh"
 
@@ -118,95 +119,6 @@ template <int KIND>
 constexpr size_t smem_bytes() {
   using T = Traits<KIND>;
   return 1024 + (size_t)T::kStages * kStageBytes + T::kBoxes + kControlBytes + T::kExtra;
-}
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// shared::cluster address of the same shared-memory offset in CTA `cta` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t cta) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tmap, uint32_t bar_cluster,
-                                                 int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster), "r"(c0),
-      "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   bar_cluster)
-               : "memory");
-}
-__device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                            uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// mbar_wait for a barrier the peer CTA arrives on
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* abort_flag, int32_t* status,
-                                                  int where) {
-  const unsigned long long t0 = global_ns();
-  for (uint32_t it = 1;; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if ((it & 255u) == 0) {
-      if (*reinterpret_cast<volatile int*>(abort_flag)) return false;
-      if (global_ns() - t0 > kWaitLimitNs) {
-        *reinterpret_cast<volatile int*>(abort_flag) = 1;
-        atomicMax(&status[0], MOE_B200_DEV_TIMEOUT);
-        status[1] = where;
-        status[2] = (int)blockIdx.x;
-        return false;
-      }
-    }
-  }
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster)
-               : "memory");
-}
-// The same without ordering this thread's earlier writes before it: a release at cluster scope waits for
-// all of the warp's global stores, and an epilogue warp that only hands its accumulator back (whose
-// reads tcgen05.wait::ld has completed) publishes nothing.
-__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-
-// Barrier of `threads` threads (all of them in whole warps) that also tells whether all of them agree.
-__device__ __forceinline__ bool barrier_and(int id, int threads, bool ok) {
-  int all;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.s32 p, %3, 0;\n\t"
-      "barrier.cta.red.and.pred q, %1, %2, p;\n\t"
-      "selp.s32 %0, 1, 0, q;\n\t}"
-      : "=r"(all)
-      : "r"(id), "r"(threads), "r"((int)ok)
-      : "memory");
-  return all != 0;
 }
 
 // COLS = false: groups are row ranges [offsets[e], offsets[e+1]) of A; B_e = tmap_b[e]; K fixed.
@@ -705,11 +617,6 @@ int64_t max_tiles(int64_t M, int E, int Nout) {
 }
 
 }  // namespace
-
-bool tiles_at_row_counts(int64_t M, int d, int E) {
-  const int64_t tiles = ((M + kPairRows - 1) / kPairRows + E / 2) * ((d + BN - 1) / BN);
-  return M >= (E >= 4 ? (int64_t)192 * E : 1536) && tiles <= kNumSMs / 2;
-}
 
 int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d,
                        int f, int E, void* h, void* y, const EpScatter* sc, int32_t* status,

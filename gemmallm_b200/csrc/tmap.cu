@@ -64,8 +64,23 @@ int encode_tmap_2d_f32(void* out, const void* base, uint64_t rows, uint64_t cols
   return 0;
 }
 
+// gate_and_up.weight [2 f, d] as [f][gate, up][d]: a box holds 64 columns of gate and up rows in turn, 64 features.
+static int encode_tmap_pairs(void* out, const void* base, uint64_t f, uint64_t d) {
+  EncodeTiledFn enc = get_encode();
+  if (enc == nullptr) return set_error(MOE_B200_ERR_DRIVER, "cuTensorMapEncodeTiled unavailable");
+  cuuint64_t dims[3] = {d, 2, f};
+  cuuint64_t strides[2] = {f * d * 2, d * 2};
+  cuuint32_t box[3] = {64, 2, 64};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(static_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides,
+                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(MOE_B200_ERR_DRIVER, "cuTensorMapEncodeTiled failed");
+  return 0;
+}
+
 // Plan maps per expert. bf16: W1 and W2 with 128-row boxes (large-N path), then W1 and W2 with 64-row boxes
-// (small-N path). fp32: W1 and W2 with 64-row boxes.
+// (small-N path), then W1 in pairs. fp32: W1 and W2 with 64-row boxes.
 int build_weight_tensor_maps(const void* const* h_W1, const void* const* h_W2, int E, int d, int f, int dtype,
                              void* h_tmaps) {
   char* maps = static_cast<char*>(h_tmaps);
@@ -86,6 +101,8 @@ int build_weight_tensor_maps(const void* const* h_W1, const void* const* h_W2, i
     rc = encode_tmap_2d(maps + 128 * (size_t)(2 * E + e), h_W1[e], (uint64_t)2 * f, (uint64_t)d, 64);
     if (rc) return rc;
     rc = encode_tmap_2d(maps + 128 * (size_t)(3 * E + e), h_W2[e], (uint64_t)d, (uint64_t)f, 64);
+    if (rc) return rc;
+    rc = encode_tmap_pairs(maps + 128 * (size_t)(4 * E + e), h_W1[e], (uint64_t)f, (uint64_t)d);
     if (rc) return rc;
   }
   return 0;

@@ -314,6 +314,46 @@ def test_mid_sizes_rows_path(cuda_device, N, d, E, f, k):
         check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device, residual=res)
 
 
+# both products in one launch: either side of its lines (96 and 2048 rows an expert, 1536 rows of one or two experts, 33
+# experts); blocks of 256 tokens and a token more, remainders of 32; more blocks than take turns on a tile of weights (16);
+# experts without rows; widths that are no multiple of a tile; K of one block; one token; 200 experts
+@pytest.mark.parametrize("N,d,E,f,k,bias0", [
+    (383, 264, 8, 136, 2, 0.0), (384, 264, 8, 136, 2, 0.0), (512, 64, 2, 264, 1, 9.0), (1537, 136, 2, 264, 1, 0.7),
+    (256 * 5 + 1, 72, 4, 200, 1, 40.0), (4400, 128, 8, 72, 1, 40.0), (8193, 64, 4, 64, 1, 0.0), (1, 256, 33, 136, 4, 0.0),
+    (40, 136, 64, 264, 4, 3.0), (700, 64, 200, 72, 8, 0.0), (1100, 1024, 8, 1032, 2, 0.0)])
+def test_both_products_in_one_launch(cuda_device, N, d, E, f, k, bias0):
+    params = helpers.rounded_params(synthetic.make_params(d, E, f, seed=N), torch.bfloat16)
+    params["w1"] *= 2.0
+    params["gate_b"][0] = bias0
+    m = build(params, d, E, f, k, torch.bfloat16, cuda_device)
+    for call in range(2):
+        x = synthetic.round_to(synthetic.make_input(N, d, seed=N + call), torch.bfloat16)
+        res = synthetic.round_to(synthetic.make_input(N, d, seed=N + 7), torch.bfloat16) if call else None
+        check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device, residual=res)
+
+
+def test_calls_in_one_launch_on_two_streams(cuda_device):
+    """Two such calls at once: tiles are claimed by pairs of CTAs that run, so that neither waits for one that does not.
+    The outputs are those of the calls one after the other, to the bit."""
+    N, d, E, f, k = 1200, 512, 8, 1024, 2
+    ms = []
+    for seed in (1, 2):
+        params = helpers.rounded_params(synthetic.make_params(d, E, f, seed=seed), torch.bfloat16)
+        x = synthetic.round_to(synthetic.make_input(N, d, seed=seed + 5), torch.bfloat16).bfloat16().to(cuda_device)
+        ms.append((build(params, d, E, f, k, torch.bfloat16, cuda_device), x.view(1, N, d), torch.cuda.Stream()))
+    with torch.no_grad():
+        want = [m(x)[0].clone() for m, x, _ in ms]
+        torch.cuda.synchronize()
+        for _ in range(20):
+            got = []
+            for m, x, s in ms:
+                with torch.cuda.stream(s):
+                    got.append(m(x)[0])
+            torch.cuda.synchronize()
+            assert all(torch.equal(g, w) for g, w in zip(got, want))
+    assert all(m.device_status() == 0 for m, _, _ in ms)
+
+
 def test_small_n_fresh_workspace_and_changing_inputs(cuda_device):
     """The small-N expert kernel runs while the routing kernel is still writing idx/offsets, and
     the combine may become resident before either has finished: every call on a fresh, zeroed
