@@ -275,20 +275,22 @@ struct EpScatter {
 };
 
 // Training-mode extras of the GEGLU pass (reference model.py:164,183: nn.Dropout on h, and
-// what the backward pass needs): the pre-activations gate/up with their biases go to
-// gu [M, 2f] (columns [0,f) gate, [f,2f) up), and h is multiplied by the dropout mask of its
-// (token, slot) pair: element (pair, c) is kept iff its Philox word (philox.cuh) is >= thresh,
-// and scaled by `scale` = 1 / (1 - p). The backward pass reads the mask back and replaces gu by
-// its gradient; col_part receives the column sums of that gradient, one row per 128-row half
+// what the backward pass needs): h is multiplied by the dropout mask of its (token, slot) pair:
+// element (pair, c) is kept iff its Philox word (philox.cuh) is >= thresh, and scaled by
+// `scale` = 1 / (1 - p). The derivatives of h after the gate and up values, mask and scale
+// included, go to gu [M, 2f] (columns [0,f) gate, [f,2f) up); with keep_pre (LoRA steps, whose
+// rounding is that of the pre-activations) those go there, with their biases, and the mask to
+// `mask`. The backward pass replaces gu by the gradients of gate and up; col_part receives the column sums of that gradient, one row per 128-row half
 // of a 256-row tile (tiles counted over the experts in order).
 struct TrainArgs {
   __nv_bfloat16* gu;
-  uint8_t* mask;            // [M, f / 8] one bit per element of h, set = kept
+  uint8_t* mask;            // keep_pre: [M, f / 8] one bit per element of h, set = kept
   float* col_part;          // [2 * m-tiles, 2f], backward only
   const int32_t* pair_of;   // [M] token * k + slot of every sorted row; nullptr: the row itself
   uint32_t thresh;          // p * 2^32; 0 keeps everything
   float scale;
   uint32_t seed_lo, seed_hi;
+  bool keep_pre;
 };
 
 // ---- launchers implemented in the other translation units -----------------

@@ -64,34 +64,37 @@ constexpr int kHalfTile = 64 * BK * 2;   // one 64 x 64 box of an MN-major opera
 // What a launch computes. Rows of A are grouped by expert except in kWgrad.
 enum Kind {
   kGeglu,        // h = gelu(x Wg^T + bg) * (x Wu^T + bu)
-  kGegluTrain,   // the same with dropout, keeping pre-activations and mask (TrainArgs)
+  kGegluTrain,   // the same with dropout, keeping the derivatives of h (TrainArgs)
+  kGegluTrainPre,   // ... keeping pre-activations and mask (LoRA steps)
   kPlain,        // y = h W2^T + b2
   kScatter,      // the same into the token owners' buffers (expert parallelism)
   kDx,           // out = A B, B [K, Nout] as it lies in memory
-  kDhGeglu,      // dh = dy W2 as kDx, then back through dropout, product and GELU in the epilogue
-  kDhGegluBf16,  // the same with dh rounded to bf16 and the column sums over rounded values (LoRA steps)
+  kDhGeglu,      // dh = dy W2 as kDx, times the derivatives of h in the epilogue
+  kDhGegluBf16,  // from pre-activations and mask, with dh rounded to bf16 and the column sums over rounded values (LoRA steps)
   kWgrad         // out_e [Ra, Nout] = A[rows of e]^T B[rows of e]
 };
 template <int KIND>
 struct Traits {
-  static constexpr bool GEGLU = KIND == kGeglu || KIND == kGegluTrain;
+  static constexpr bool TRAIN = KIND == kGegluTrain || KIND == kGegluTrainPre;
+  static constexpr bool PRE = KIND == kGegluTrainPre;
+  static constexpr bool GEGLU = KIND == kGeglu || TRAIN;
   static constexpr bool COLS = KIND == kWgrad;
   static constexpr bool DH = KIND == kDhGeglu || KIND == kDhGegluBf16;
   static constexpr bool A_MN = COLS;
   static constexpr bool B_MN = KIND == kDx || DH || COLS;
   // The training epilogues do 10 to 20 instructions per accumulator element and move as much again as the
   // products' operands: sixteen warps, and further ones for what does not need the accumulator.
-  static constexpr int kEpiWarps = KIND == kGegluTrain || DH ? 16 : 8;
-  static constexpr int kHelpers = KIND == kGegluTrain ? 4 : (DH || COLS ? 1 : 0);
+  static constexpr int kEpiWarps = TRAIN || DH ? 16 : 8;
+  static constexpr int kHelpers = TRAIN ? 4 : (DH || COLS ? 1 : 0);
   static constexpr int kThreads = 64 + 32 * (kEpiWarps + kHelpers);
   // (kGegluTrain at 16384 tokens, d 1024, f 4096: 149 / 126 / 116 us above the inference pass with 3 / 4 / 5
   // stages, so one box per epilogue warp and a fifth stage instead of two boxes)
-  static constexpr int kStages = KIND == kGegluTrain ? 5 : (DH ? 4 : 6);
+  static constexpr int kStages = TRAIN ? 5 : (DH ? 4 : 6);
   // room behind the stages (boxes want 1 KiB alignment): a box for each epilogue warp, or two chunks of gate and up
-  static constexpr int kBoxes = KIND == kGegluTrain ? 16 * kBoxBytes : (DH ? 2 * 2 * GegluBwd::kBoxBytes : 0);
+  static constexpr int kBoxes = TRAIN ? 16 * kBoxBytes : (DH ? 2 * 2 * GegluBwd::kBoxBytes : 0);
   // and behind Control: staging of the epilogue warps; biases and mask bits; column sums of the lane quadrants
   static constexpr int kExtra =
-      KIND == kGegluTrain ? 16 * 256 + 2 * BM * 16 : (DH ? 4 * 2 * BN * 4 : 8 * kStgBytes);
+      TRAIN ? 16 * 256 + 2 * BM * 16 : (DH ? 4 * 2 * BN * 4 : 8 * kStgBytes);
 };
 
 // M = 256 across the pair: M/16 at bit 24
@@ -103,7 +106,7 @@ struct Control {
   uint64_t empty[kMaxStages];
   uint64_t tail[kMaxStages];   // COLS: this CTA's half of a block that has to be cut has arrived
   uint64_t peer_cut[kMaxStages];   // COLS, even CTA: the odd CTA's half has been cut
-  uint64_t aux_full[2];    // kGegluTrain: mask bits of a tile drawn; kDhGeglu: a chunk of gate and up values there
+  uint64_t aux_full[2];    // kGegluTrain: mask bits of a tile drawn; kDhGeglu: a chunk of derivatives there
   uint64_t aux_empty[2];   // kGegluTrain: they have been read; kDhGeglu: replaced by their gradients
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
@@ -176,7 +179,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
     for (int a = 0; a < 2; ++a) {
       mbar_init(&ctl->tmem_full[a], 1);
       mbar_init(&ctl->tmem_empty[a], 2 * kEpiWarps);
-      mbar_init(&ctl->aux_full[a], KIND == kGegluTrain ? T::kHelpers : 1);
+      mbar_init(&ctl->aux_full[a], T::TRAIN ? T::kHelpers : 1);
       mbar_init(&ctl->aux_empty[a], kEpiWarps);
     }
     ctl->abort = 0;
@@ -347,7 +350,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       }
       parity ^= 1u << s;
     }
-  } else if (KIND == kGegluTrain && warp >= 2 + kEpiWarps) {
+  } else if (T::TRAIN && warp >= 2 + kEpiWarps) {
     // ---------------- dropout mask: four warps, 32 rows of the tile each ----------------
     int it = 0, e = 0;
     for (int t = pair; tr.thresh != 0u && t < total_tiles; t += num_pairs, ++it) {
@@ -359,12 +362,12 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (!mbar_wait(&ctl->aux_empty[a], ((uint32_t)(it >> 1) & 1u) ^ 1u, &ctl->abort, status, 37)) break;
       uint32_t* s_mask = reinterpret_cast<uint32_t*>(extra + kEpiWarps * 256) + a * BM * 4;
       const int rl = (warp - 2 - kEpiWarps) * 32 + lane;
-      draw_mask(tr, row_cta + rl, row_cta + rl < ctl->offsets[e + 1], nt * kTileN, Nout, s_mask + rl * 4);
+      draw_mask<T::PRE>(tr, row_cta + rl, row_cta + rl < ctl->offsets[e + 1], nt * kTileN, Nout, s_mask + rl * 4);
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->aux_full[a]);
     }
   } else if (T::DH && warp == 2 + kEpiWarps) {
-    // ---------------- gate and up values: two chunks ahead, stored again as gradients ----------------
+    // ---------------- derivatives after gate and up: two chunks ahead, stored again as gradients ----------------
     if (elect_one()) {
       struct Place { int col, row; bool boxes; } place[2];
       int ci = 0, e = 0;
@@ -433,9 +436,9 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       }
       const int a = it & 1;
       float* s_bias = reinterpret_cast<float*>(extra + (warp - 2) * 256);
-      if constexpr (KIND == kGegluTrain) GegluTrain::start(n0, Nout, bias, s_bias, lane, part);
+      if constexpr (T::TRAIN) GegluTrain<T::PRE>::start(n0, Nout, bias, s_bias, lane, part);
       uint32_t keep[4];
-      if constexpr (T::DH) {
+      if constexpr (KIND == kDhGegluBf16) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           keep[c] = GegluBwd::mask_bits(tr, row_warp + lane, lane < rows, n0 + c * 64 + part * 16, Nout);
@@ -449,7 +452,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(&ctl->tmem_empty[a]), lead));
       };
-      if constexpr (KIND == kGegluTrain) {
+      if constexpr (T::TRAIN) {
         uint32_t bits = 0xffffffffu;
         if (tr.thresh != 0u) {
           ok = mbar_wait(&ctl->aux_full[a], acc_phase, &ctl->abort, status, 39);
@@ -458,7 +461,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl->aux_empty[a]);
         }
-        GegluTrain::finish(taddr, row_warp, rows, n0, Nout, out_e, tr, &tmap_h, &tmap_gu, s_bias, bits, box, lane, part,
+        GegluTrain<T::PRE>::finish(taddr, row_warp, rows, n0, Nout, out_e, tr, &tmap_h, &tmap_gu, s_bias, bits, box, lane, part,
                            release);
       } else if constexpr (T::DH) {
         float* s_col = reinterpret_cast<float*>(extra);
@@ -475,12 +478,15 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           if (c == 3) release();
           const bool as_boxes = row_end - row_cta >= BM && n0 + c * 64 + 64 <= Nout;
           __nv_bfloat16* direct = as_boxes ? nullptr : tr.gu + (int64_t)(row_warp + lane) * 2 * Nout + n;
-          uint32_t bits = keep[0];
-          bits = c == 1 ? keep[1] : bits;
-          bits = c == 2 ? keep[2] : bits;
-          bits = c == 3 ? keep[3] : bits;
-          GegluBwd::chunk<KIND == kDhGegluBf16>(v, boxes + b * 2 * GegluBwd::kBoxBytes, bits, tr.scale, lane < rows, direct, Nout, Nout - n,
-                          s_col + quad * 2 * BN + c * 64 + part * 16, BN, quad, part, lane);
+          uint32_t bits = 0;
+          if constexpr (KIND == kDhGegluBf16) {
+            bits = keep[0];
+            bits = c == 1 ? keep[1] : bits;
+            bits = c == 2 ? keep[2] : bits;
+            bits = c == 3 ? keep[3] : bits;
+          }
+          GegluBwd::chunk<KIND == kDhGegluBf16>(v, boxes + b * 2 * GegluBwd::kBoxBytes, bits, tr.scale, lane < rows, direct,
+                          Nout, Nout - n, s_col + quad * 2 * BN + c * 64 + part * 16, BN, quad, part, lane);
           fence_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl->aux_empty[b]);
@@ -515,7 +521,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       if (a == 1) acc_phase ^= 1u;
       ++it;
     }
-    if (KIND == kGegluTrain && lane == 0) bulk_wait_all();
+    if (T::TRAIN && lane == 0) bulk_wait_all();
     if (KIND == kScatter) __threadfence_system();
   }
   if constexpr (SPLIT > 1) {
@@ -645,8 +651,11 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
     if (rc) return rc;
     rc = encode_tmap_2d(&tm_gu, train->gu, rows, (uint64_t)2 * f, 32, 32);
     if (rc) return rc;
-    rc = launch_pair<kGegluTrain>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, *train, sy1, 0, status,
-                                  sms, s, &tm_hb, &tm_gu);
+    rc = train->keep_pre
+             ? launch_pair<kGegluTrainPre>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, *train, sy1, 0, status,
+                                           sms, s, &tm_hb, &tm_gu)
+             : launch_pair<kGegluTrain>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, *train, sy1, 0, status,
+                                        sms, s, &tm_hb, &tm_gu);
   } else {
     rc = launch_pair<kGeglu>(tm_x, tm_x, pv.tmap_W1, offsets, pv.b1, E, d, f, h, none, eval, sy1, 0, status, sms, s);
   }

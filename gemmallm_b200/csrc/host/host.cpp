@@ -952,7 +952,7 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     const int rc = moe::forward_train_into(
         x.const_data_ptr(), gate_w.const_data_ptr(), gate_b.const_data_ptr(), c->plan,
         has_res ? res.const_data_ptr() : nullptr, c->N, c->d, c->f, c->E, c->k, MOE_B200_BF16, (float)p, seed, c->ws_base,
-        c->ws_bytes, c->tws_base, c->tws_bytes, out.data_ptr(), aux.data_ptr<float>(), stream);
+        c->ws_bytes, c->tws_base, c->tws_bytes, out.data_ptr(), aux.data_ptr<float>(), !c->ranks.empty(), stream);
     if (rc != 0) return fail(rc, "forward_train");
   }
   ++*c->gen;
@@ -1169,9 +1169,9 @@ PyObject* ffn_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     at::AutoGradMode no_grad(false);
     h = at::empty({c->N, c->f}, x.options());
     y = at::empty(x.sizes(), x.options());
-    const int rc = moe_b200_experts_train(x.const_data_ptr(), c->offsets.const_data_ptr<int32_t>(), c->plan, c->N, c->d,
-                                          c->f, 1, (float)p, seed, c->tws_base, c->tws_bytes, h.data_ptr(), y.data_ptr(),
-                                          c->status.data_ptr<int32_t>(), stream);
+    const int rc = moe::experts_train_into(x.const_data_ptr(), c->offsets.const_data_ptr<int32_t>(), c->plan, c->N, c->d,
+                                           c->f, 1, (float)p, seed, c->tws_base, c->tws_bytes, h.data_ptr(), y.data_ptr(),
+                                           !c->ranks.empty(), c->status.data_ptr<int32_t>(), stream);
     if (rc != 0) return fail(rc, "experts_train");
   }
   ++*c->gen;

@@ -186,10 +186,19 @@ struct BoxOut {
 };
 
 // GEGLU pass in training mode (TrainArgs in common.cuh), 16 epilogue warps: this one takes output
-// columns [32 part, 32 part + 32) of its 32 rows. The gate/up pre-activations are kept for the backward
-// pass and h gets its dropout mask: s_mask[row][part], bits drawn by four other warps while the products of the
-// tile run (draw_mask). start() fetches the biases into this warp's 64 floats of shared memory before the
-// products are awaited.
+// columns [32 part, 32 part + 32) of its 32 rows. h gets its dropout mask (s_mask[row][part], bits drawn by four other
+// warps while the products of the tile run, draw_mask), and what the backward pass multiplies dh by is kept, the
+// derivatives of h after the gate and the up value, mask and scale included:
+//   h = m gelu(g) u,   h_g = m u gelu'(g),   h_u = m gelu(g),   m = scale where the element is kept, else 0
+//   with s = 1 / (1 + exp(-2 z)), z = b (g + a g^3):  gelu(g) = g s,
+//   gelu'(g) = s + 2 g s (1 - s) b (1 + 3 a g^2)       (0.5 (1 + tanh z) = s)
+// (Keeping g and u instead left GELU, its derivative and the mask to the backward epilogue, which had twice the elements
+// per product and was bound by them, and rounded g and u before they went through the GELU. 32768 rows, d 1024, f 4096, 8
+// experts: that product 385 -> 302 us, now bound by the column sums' shuffles and its boxes' way through shared memory;
+// this one 438 -> 443; whole training step 2472 -> 2413.)
+// PRE, LoRA steps: g, u and the mask are kept all the same, whose rounding such a step repeats (lora_bwd.cu says why).
+// start() fetches the biases into this warp's 64 floats of shared memory before the products are awaited.
+template <bool PRE>
 struct GegluTrain {
   __device__ __forceinline__ static void start(int n0, int Nout, const __nv_bfloat16* __restrict__ bias, float* s_bias,
                                                int lane, int part) {
@@ -226,8 +235,21 @@ struct GegluTrain {
         for (int i = 0; i < 8; ++i) {
           gv[i] += __uint_as_float(g[q * 8 + i]);
           uv[i] += __uint_as_float(u[q * 8 + i]);
-          const float hv = gelu_tanh_fast(gv[i]) * uv[i];
-          o[i] = (keep >> (c + i)) & 1u ? hv * tr.scale : 0.f;
+          if constexpr (PRE) {
+            const float hv = gelu_tanh_fast(gv[i]) * uv[i];
+            o[i] = (keep >> (c + i)) & 1u ? hv * tr.scale : 0.f;
+            continue;
+          }
+          constexpr float kB = 0.7978845608028654f, kA = 0.044715f, kL = -2.f * 1.4426950408889634f;
+          const float x = gv[i], x2 = x * x;
+          const float sg = __fdividef(1.f, 1.f + exp2f_fast(x * fmaf(kL * kB * kA, x2, kL * kB)));
+          const float gs = x * sg;
+          const float dgelu = fmaf(fmaf(-gs, sg, gs), fmaf(6.f * kA * kB, x2, 2.f * kB), sg);
+          const bool kept = (keep >> (c + i)) & 1u;
+          gv[i] = kept ? uv[i] * dgelu * tr.scale : 0.f;
+          const float hu = kept ? gs * tr.scale : 0.f;
+          o[i] = kept ? hu * uv[i] : 0.f;
+          uv[i] = hu;
         }
         pg[c / 8] = pack8(gv);
         pu[c / 8] = pack8(uv);
@@ -249,7 +271,8 @@ struct GegluTrain {
 };
 
 // The dropout mask of one row's 128 columns from n0 (bit i of word w: column n0 + 32 w + i, set = kept), to
-// shared memory for the epilogue and to global memory for the backward pass.
+// shared memory for the epilogue and, where it is kept (PRE), to global memory for the backward pass.
+template <bool PRE>
 __device__ __forceinline__ void draw_mask(const TrainArgs& tr, int64_t row, bool row_ok, int n0, int Nout,
                                           uint32_t* s_row) {
   const uint32_t pair = tr.pair_of == nullptr ? (uint32_t)row : row_ok ? (uint32_t)__ldg(&tr.pair_of[row]) : 0u;
@@ -266,7 +289,7 @@ __device__ __forceinline__ void draw_mask(const TrainArgs& tr, int64_t row, bool
     w[p] = keep;
   }
   *reinterpret_cast<uint4*>(s_row) = make_uint4(w[0], w[1], w[2], w[3]);
-  if (row_ok) {
+  if (PRE && row_ok) {
     uint8_t* m = tr.mask + row * (Nout >> 3) + (n0 >> 3);
     if ((Nout & 127) == 0) {
       *reinterpret_cast<uint4*>(m) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -277,13 +300,13 @@ __device__ __forceinline__ void draw_mask(const TrainArgs& tr, int64_t row, bool
 }
 
 // Epilogue of dh = dy W2 in the backward pass (model.py:180-183), 16 epilogue warps, one accumulator row per
-// thread, back through dropout, product and GELU in place over the pre-activations gu:
+// thread, back through dropout, product and GELU in place over the derivatives the forward kept (GegluTrain):
+//   dg = dh h_g;  du = dh h_u
+// LoRA steps (ROUND) form them from the pre-activations and the mask, in one rounding:
 //   dhe = dh * mask * scale;  du = dhe * gelu(g);  dg = dhe * u * gelu'(g)
-//   with s = 1 / (1 + exp(-2 z)), z = b (g + a g^3):  gelu(g) = g s,
-//   gelu'(g) = s + 2 g s (1 - s) b (1 + 3 a g^2)       (0.5 (1 + tanh z) = s)
-// The tile is worked on in chunks of 64 columns: another warp (gu_warp in the kernel) brings a chunk of gate and up
+// The tile is worked on in chunks of 64 columns: another warp (gu_warp in the kernel) brings a chunk of the two
 // values (two boxes of 128 rows x 64 columns, 128-byte swizzle) to shared memory two chunks ahead, the epilogue
-// replaces them by their gradients there, and the boxes are stored again. (With the loads issued by the epilogue
+// replaces them by the gradients there, and the boxes are stored again. (With the loads issued by the epilogue
 // warps themselves, however far ahead registers allowed, their latency made the kernel 2.3 times as long.)
 // This warp takes columns [16 part, 16 part + 16) of the chunk for its 32 rows; it also sums dg and du over the
 // rows (the bias gradient of gate_and_up) into s_col[0..15] and s_col[du_off ..].
@@ -301,33 +324,42 @@ struct GegluBwd {
   // direct: the row's place in gu for a chunk that cannot be stored as boxes, else nullptr; cols: columns that exist;
   // ROUND: dh is rounded to bf16 first, and the sums take the rounded dg and du (lora_bwd.cu says why)
   template <bool ROUND>
-  __device__ __forceinline__ static void chunk(const uint32_t (&v)[16], uint8_t* box, uint32_t keep, float scale,
-                                               bool row_ok, __nv_bfloat16* direct, int f, int cols, float* s_col,
-                                               int du_off, int quad, int part, int lane) {
+  __device__ __forceinline__ static void chunk(uint32_t (&v)[16], uint8_t* box, uint32_t keep, float scale, bool row_ok,
+                                               __nv_bfloat16* direct, int f, int cols, float* s_col, int du_off, int quad,
+                                               int part, int lane) {
     float dg[16], du[16];
     const int r = quad * 32 + lane;
+    if (!ROUND && !row_ok) {      // rows of other experts: nothing of them in the sums
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = 0u;
+    }
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       uint4* gp = reinterpret_cast<uint4*>(box + r * 128 + (((part * 2 + j) ^ (r & 7)) << 4));
       uint4* up = gp + kBoxBytes / 16;
-      const uint4 g4 = *gp, u4 = *up;
+      uint4 g4 = *gp, u4 = *up;
+      if (!ROUND && !row_ok) g4 = u4 = make_uint4(0, 0, 0, 0);
       const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w};
       const uint32_t uw[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        constexpr float kB = 0.7978845608028654f, kA = 0.044715f, kL = -2.f * 1.4426950408889634f;
         const int c = j * 8 + i;
-        float dh = __uint_as_float(v[c]);
-        if (ROUND) dh = __bfloat162float(__float2bfloat16_rn(dh));
-        const float dv = (keep >> c) & 1u ? dh * scale : 0.f;
         const float x = (i & 1) ? bf16_hi(gw[i >> 1]) : bf16_lo(gw[i >> 1]);
         const float uv = (i & 1) ? bf16_hi(uw[i >> 1]) : bf16_lo(uw[i >> 1]);
-        const float x2 = x * x;
-        const float s = __fdividef(1.f, 1.f + exp2f_fast(x * fmaf(kL * kB * kA, x2, kL * kB)));
-        const float gs = x * s;
-        const float dgelu = fmaf(fmaf(-gs, s, gs), fmaf(6.f * kA * kB, x2, 2.f * kB), s);
-        du[c] = row_ok ? dv * gs : 0.f;
-        dg[c] = row_ok ? dv * uv * dgelu : 0.f;
+        if constexpr (!ROUND) {
+          dg[c] = __uint_as_float(v[c]) * x;
+          du[c] = __uint_as_float(v[c]) * uv;
+        } else {
+          constexpr float kB = 0.7978845608028654f, kA = 0.044715f, kL = -2.f * 1.4426950408889634f;
+          const float dh = __bfloat162float(__float2bfloat16_rn(__uint_as_float(v[c])));
+          const float dv = (keep >> c) & 1u ? dh * scale : 0.f;
+          const float x2 = x * x;
+          const float s = __fdividef(1.f, 1.f + exp2f_fast(x * fmaf(kL * kB * kA, x2, kL * kB)));
+          const float gs = x * s;
+          const float dgelu = fmaf(fmaf(-gs, s, gs), fmaf(6.f * kA * kB, x2, 2.f * kB), s);
+          du[c] = row_ok ? dv * gs : 0.f;
+          dg[c] = row_ok ? dv * uv * dgelu : 0.f;
+        }
       }
       const uint4 og = make_uint4(pack_bf16x2(dg[j * 8], dg[j * 8 + 1]), pack_bf16x2(dg[j * 8 + 2], dg[j * 8 + 3]),
                                   pack_bf16x2(dg[j * 8 + 4], dg[j * 8 + 5]), pack_bf16x2(dg[j * 8 + 6], dg[j * 8 + 7]));

@@ -49,7 +49,8 @@ void tws_layout(int64_t N, int d, int f, int E, int k, size_t* off, size_t* tota
   *total = pos;
 }
 
-TrainArgs train_args(char* tws, const size_t* to, float p, uint64_t seed) {
+// lora: of a LoRA step, forward and backward alike
+TrainArgs train_args(char* tws, const size_t* to, float p, uint64_t seed, bool lora) {
   TrainArgs tr;
   tr.gu = reinterpret_cast<__nv_bfloat16*>(tws + to[MOE_B200_TWS_GU]);
   tr.mask = reinterpret_cast<uint8_t*>(tws + to[MOE_B200_TWS_MASK]);
@@ -60,6 +61,7 @@ TrainArgs train_args(char* tws, const size_t* to, float p, uint64_t seed) {
   tr.scale = 1.0f / (1.0f - p);
   tr.seed_lo = (uint32_t)seed;
   tr.seed_hi = (uint32_t)(seed >> 32);
+  tr.keep_pre = lora;
   return tr;
 }
 
@@ -165,7 +167,7 @@ int moe_b200_forward_train(const void* x, const void* Wg, const void* bg, const 
                            float dropout_p, uint64_t seed, void* workspace, size_t workspace_bytes,
                            void* train_ws, size_t train_ws_bytes, void* out, void* stream) {
   return forward_train_into(x, Wg, bg, plan, residual, N, d, f, E, k, dtype, dropout_p, seed, workspace,
-                            workspace_bytes, train_ws, train_ws_bytes, out, nullptr, stream);
+                            workspace_bytes, train_ws, train_ws_bytes, out, nullptr, false, stream);
 }
 
 int moe_b200_backward(const void* x, const void* Wg, const void* plan, const void* grad_out,
@@ -189,20 +191,8 @@ int moe_b200_backward(const void* x, const void* Wg, const void* plan, const voi
 int moe_b200_experts_train(const void* x_sorted, const int32_t* offsets, const void* plan, int64_t M,
                            int d, int f, int E, float dropout_p, uint64_t seed, void* train_ws,
                            size_t train_ws_bytes, void* h, void* y, int32_t* status, void* stream) {
-  int rc = train_check(M, d, f, E, 1, MOE_B200_BF16, dropout_p);
-  if (rc) return rc;
-  if (M == 0) return 0;
-  if (!x_sorted || !offsets || !plan || !train_ws || !h || !y || !status)
-    return set_error(MOE_B200_ERR_NULL, "NULL argument");
-  size_t to[MOE_B200_TWS_NUM], ttotal;
-  tws_layout(M, d, f, E, 1, to, &ttotal);
-  if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
-  if ((uintptr_t)train_ws & 1023) return set_error(MOE_B200_ERR_ALIGN, "training workspace must be 1024-byte aligned");
-  char* tws = static_cast<char*>(train_ws);
-  cudaStream_t s = (cudaStream_t)stream;
-  TrainArgs tr = train_args(tws, to, dropout_p, seed);
-  tr.pair_of = nullptr;     // row r is pair r: the dropout mask of element (r, c) depends on the row's position only
-  return launch_experts_tc2(x_sorted, offsets, plan, M, d, f, E, h, y, nullptr, status, s, &tr);
+  return experts_train_into(x_sorted, offsets, plan, M, d, f, E, dropout_p, seed, train_ws, train_ws_bytes, h, y, false,
+                            status, stream);
 }
 
 int moe_b200_experts_backward(const void* x_sorted, const void* h, const int32_t* offsets,
@@ -224,10 +214,29 @@ int moe_b200_experts_backward(const void* x_sorted, const void* h, const int32_t
 
 namespace moe {
 
+int experts_train_into(const void* x_sorted, const int32_t* offsets, const void* plan, int64_t M, int d, int f, int E,
+                       float dropout_p, uint64_t seed, void* train_ws, size_t train_ws_bytes, void* h, void* y, bool lora,
+                       int32_t* status, void* stream) {
+  int rc = train_check(M, d, f, E, 1, MOE_B200_BF16, dropout_p);
+  if (rc) return rc;
+  if (M == 0) return 0;
+  if (!x_sorted || !offsets || !plan || !train_ws || !h || !y || !status)
+    return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  size_t to[MOE_B200_TWS_NUM], ttotal;
+  tws_layout(M, d, f, E, 1, to, &ttotal);
+  if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
+  if ((uintptr_t)train_ws & 1023) return set_error(MOE_B200_ERR_ALIGN, "training workspace must be 1024-byte aligned");
+  char* tws = static_cast<char*>(train_ws);
+  cudaStream_t s = (cudaStream_t)stream;
+  TrainArgs tr = train_args(tws, to, dropout_p, seed, lora);
+  tr.pair_of = nullptr;     // row r is pair r: the dropout mask of element (r, c) depends on the row's position only
+  return launch_experts_tc2(x_sorted, offsets, plan, M, d, f, E, h, y, nullptr, status, s, &tr);
+}
+
 int forward_train_into(const void* x, const void* Wg, const void* bg, const void* plan, const void* residual,
                        int64_t N, int d, int f, int E, int k, int dtype, float dropout_p, uint64_t seed,
                        void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes, void* out,
-                       float* aux, void* stream) {
+                       float* aux, bool lora, void* stream) {
   int rc = train_check(N, d, f, E, k, dtype, dropout_p);
   if (rc) return rc;
   if (!workspace || !train_ws) return set_error(MOE_B200_ERR_NULL, "workspace is NULL");
@@ -268,7 +277,7 @@ int forward_train_into(const void* x, const void* Wg, const void* bg, const void
   if (rc) return rc;
   rc = launch_pair_of(row_of, M, reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]), s);
   if (rc) return rc;
-  const TrainArgs tr = train_args(tws, to, dropout_p, seed);
+  const TrainArgs tr = train_args(tws, to, dropout_p, seed, lora);
   rc = launch_experts_tc2(perm, offsets, plan, M, d, f, E, h, y, nullptr, status, s, &tr);
   if (rc) return rc;
   return moe_b200_combine(y, row_of, w, residual, N, d, k, dtype, out, stream);
@@ -311,7 +320,7 @@ int backward_into(const void* x, const void* Wg, const void* plan, const void* g
   float* dl = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DL]);
   float* dw = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DW]);
   float* dwg32 = reinterpret_cast<float*>(tws + to[MOE_B200_TWS_DWG_F32]);
-  const TrainArgs tr = train_args(tws, to, dropout_p, seed);
+  const TrainArgs tr = train_args(tws, to, dropout_p, seed, lora != nullptr);
 
   // combine (model.py:271) and router (model.py:206-223)
   rc = launch_combine_bwd(grad_out, y, tr.pair_of, offsets, E, w, M, d, k, dy, dw, s);
@@ -345,7 +354,7 @@ int experts_backward_into(const void* x_sorted, const void* h, const int32_t* of
   if (train_ws_bytes < ttotal) return set_error(MOE_B200_ERR_WORKSPACE, "training workspace too small");
   char* tws = static_cast<char*>(train_ws);
   cudaStream_t s = (cudaStream_t)stream;
-  const TrainArgs tr = train_args(tws, to, dropout_p, seed);
+  const TrainArgs tr = train_args(tws, to, dropout_p, seed, lora != nullptr);
   // gradients come as they come (a slice of a concatenation starts anywhere): those that TMA and 16-byte accesses cannot
   // take go through the workspace
   const size_t bytes = (size_t)M * d * 2;

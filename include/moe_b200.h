@@ -416,9 +416,9 @@ int moe_b200_attention(const void* qkv, const void* gate, const float* pos_emb, 
  * that forward and its backward pass for bf16. Both work on the block's ordinary
  * workspace (which the forward fills and the backward reads: call the backward before
  * the next forward on the same workspace) plus a training workspace for the saved
- * pre-activations, the dropout mask and the parameter gradients. */
+ * derivatives of h and the parameter gradients. */
 enum {
-  MOE_B200_TWS_GU = 0,   /* bf16 [N*k, 2f] gate/up pre-activations; (dg, du) after the backward */
+  MOE_B200_TWS_GU = 0,   /* bf16 [N*k, 2f] derivatives of h after gate and up; (dg, du) after the backward */
   MOE_B200_TWS_PAIR_OF,  /* int32 [N*k]    token * k + slot of every sorted row */
   MOE_B200_TWS_KOFF,     /* empty, as DH, W1T .. DGUT, ONES and DXR below: the products read their
                           * operands as they lie in memory and dh never leaves the chip */
@@ -437,7 +437,8 @@ enum {
   MOE_B200_TWS_G_B1,     /* [E,2f]     experts.e.gate_and_up.bias */
   MOE_B200_TWS_G_W2,     /* [E,d,f]    experts.e.down.weight */
   MOE_B200_TWS_G_B2,     /* [E,d]      experts.e.down.bias */
-  MOE_B200_TWS_MASK,     /* uint8 [N*k, f/8] dropout mask of h, one bit per element */
+  MOE_B200_TWS_MASK,     /* uint8 [N*k, f/8], LoRA steps of the modules: the dropout mask of h, one bit per element,
+                          * whose GU holds the pre-activations; else the mask is part of GU and this is not used */
   MOE_B200_TWS_COL_PART, /* float      partial column sums of the bias gradients */
   MOE_B200_TWS_NUM
 };
