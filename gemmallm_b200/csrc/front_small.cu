@@ -36,7 +36,7 @@ int launch(const void* x, const void* Wg, const void* bg, int N, int d, int E, i
   constexpr bool F32 = sizeof(T) == 4;
   const bool split = F32 || (xch != nullptr && counter != nullptr && status != nullptr && N > 128);
   const int ntok = split ? 16 : N;
-  const size_t smem = front_small_smem_bytes(NT, ntok, E, k);
+  const size_t smem = front_small_smem_bytes(NT, ntok, E, k) + (F32 ? front_f32_chunk_bytes(NT) : 0);
   static PerDeviceOnce once_whole, once_split;
   auto fn = front_small_kernel<NT, true, T>;
   int rc = ensure_dynamic_smem(once_split, fn, 160 * 1024);

@@ -17,7 +17,7 @@
 //   C. warp 0: per-slot counts, offsets (scan over E), stable ranks in (token,
 //      slot) order; then row copies into the sorted buffer with 16-byte accesses
 //      (their loads were issued before B);
-//   E. block 0, after its copies: probabilities summed per expert in token order; loss.
+//   E. block 0: probabilities summed per expert in token order; loss.
 #pragma once
 #include <cooperative_groups.h>
 #include "common.cuh"
@@ -61,9 +61,17 @@ using front_detail::ld_acquire_gpu_i32;
 //   the logits' partial sums are added.
 //
 // `smem`: front_small_smem_bytes() of shared memory.
+// The partial logits' area also takes the blocks' probability sums (SPLIT, up to 128 blocks) once the logits are summed.
+// fp32: behind the rest, kFrontChunk elements of K of 16 tokens and 8 NT experts.
+template <int NT>
+constexpr int kFrontChunk = NT == 1 ? 512 : 256;
+constexpr int kFrontPad = 4;        // floats: rows 16 bytes apart modulo the banks
 __host__ __device__ inline size_t front_small_smem_bytes(int NT, int ntok, int E, int k) {
   return sizeof(float) * ((size_t)32 * 16 * 8 * NT + (size_t)ntok * (E + 1)) +
          sizeof(int) * (2 * (size_t)ntok * k + 2 * kMaxTopK * kFrontMaxE + 4 * kFrontMaxE + 1);
+}
+__host__ __device__ constexpr size_t front_f32_chunk_bytes(int NT) {
+  return (size_t)(16 + 8 * NT) * ((NT == 1 ? 512 : 256) + kFrontPad) * sizeof(float) + 16;
 }
 
 template <int NT, bool SPLIT, typename T = __nv_bfloat16>  // n-tiles of 8 experts: E <= 8*NT
@@ -116,34 +124,55 @@ __device__ __forceinline__ void front_small_body(float* smem,
 
   // ---- A. partial logits -----------------------------------------------------
   if constexpr (F32) {
-    // lane = (token of four, expert mod 8): a warp reads four rows of x and eight of Wg
+    // A chunk of K of the block's tokens and of all experts is brought to shared memory, all its loads in flight at once
+    // (read where they lie, 16 bytes at a time, they took 9.7 us of this kernel's 17 at d 512; a call of 512
+    // tokens 102.5 -> 94.7). Lane = (token
+    // of four, expert mod 8), warps also take an eighth of K each: its pieces in order, even and odd places apart.
+    constexpr int KC = kFrontChunk<NT>, KP = KC + kFrontPad;
     const int tok = (warp & 3) * 4 + (lane >> 3), e0 = lane & 7, ks = warp >> 2;
-    const float4* xr = reinterpret_cast<const float4*>(x + (size_t)min(tok, N - 1) * d);
-    const float4* w4 = reinterpret_cast<const float4*>(Wg);
-    const int n4 = d >> 2, per = (n4 + nslices - 1) / nslices, end = min(n4, (ks + 1) * per);
+    const int n4 = d >> 2, per = (n4 + nslices - 1) / nslices;
+    float* s_x = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(smem) + front_small_smem_bytes(NT, 16, E, k) + 15) &
+                                          ~(uintptr_t)15);          // [16][KP], then [8 NT][KP]
+    float* s_w = s_x + 16 * KP;
+    // a chunk holds the same part of every eighth
+    const int step = KC / 4 / 8;
     float4 acc[2][NT];       // pieces of even and of odd place
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
-      for (int j = 0; j < NT; ++j) acc[h][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto add = [&](int c, float4 (&a)[NT]) {
-      const float4 v = __ldcg(xr + c);     // (x may be the output of the kernel before this one)
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const float4 w = w4[(size_t)min(8 * j + e0, E - 1) * n4 + c];
-        a[j].x = fmaf(v.x, w.x, a[j].x);
-        a[j].y = fmaf(v.y, w.y, a[j].y);
-        a[j].z = fmaf(v.z, w.z, a[j].z);
-        a[j].w = fmaf(v.w, w.w, a[j].w);
+      for (int j = 0; j < NT; ++j) acc[hh][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c0 = 0; c0 < per; c0 += step) {
+      if (c0 > 0) __syncthreads();
+      const int rows = 16 + min(8 * NT, E);
+      for (int i = tid; i < rows * (KC / 4); i += kThreads) {
+        const int r = i / (KC / 4), q = i - r * (KC / 4);
+        const int slice = q / step, c = slice * per + c0 + (q - slice * step);      // piece of the row
+        const bool ok = c0 + (q - slice * step) < per && c < n4;
+        const T* src = r < 16 ? x + (size_t)min(r, N - 1) * d : Wg + (size_t)(r - 16) * d;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared((r < 16 ? s_x + r * KP : s_w + (r - 16) * KP) + q * 4);
+        if (ok)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + (size_t)c * 4) : "memory");
       }
-    };
-    int c = ks * per;
-#pragma unroll 2
-    for (; c + 1 < end; c += 2) {
-      add(c, acc[0]);
-      add(c + 1, acc[1]);
+      asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      const int n = min(step, min(per - c0, n4 - (ks * per + c0)));
+      const float4* xr = reinterpret_cast<const float4*>(s_x + tok * KP) + ks * step;
+      const float4* wr = reinterpret_cast<const float4*>(s_w) + ks * step;
+#pragma unroll 4
+      for (int c = 0; c < n; ++c) {
+        const float4 v = xr[c];
+        // (a chunk has an even number of pieces of a slice: even places stay even)
+        float4 (&s)[NT] = acc[c & 1];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const float4 w = wr[min(8 * j + e0, E - 1) * (KP / 4) + c];
+          s[j].x = fmaf(v.x, w.x, s[j].x);
+          s[j].y = fmaf(v.y, w.y, s[j].y);
+          s[j].z = fmaf(v.z, w.z, s[j].z);
+          s[j].w = fmaf(v.w, w.w, s[j].w);
+        }
+      }
     }
-    if (c < end) add(c, acc[0]);
 #pragma unroll
     for (int j = 0; j < NT; ++j)
       s_part[((size_t)ks * 16 + tok) * ET + 8 * j + e0] =
@@ -304,6 +333,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
   if constexpr (SPLIT) {
     const int nb = nblk, b = blk;
     float* xps = reinterpret_cast<float*>(xch + nb * k * E);    // [nb][E] probability sums
+    static_assert(32 * 16 * 8 * NT >= 128 * 8 * NT, "128 blocks' sums of 8 NT experts");
     if (tid < k * E) xch[b * k * E + tid] = s_cnt[(tid / E) * kMaxE + tid % E];
     if (tid < E) {
       float ps = 0.f;
@@ -348,7 +378,25 @@ __device__ __forceinline__ void front_small_body(float* smem,
         if (bb < b) atomicAdd(&s_base[e], c);
       }
     }
+    // the blocks' probability sums, for the loss
+    if (b == 0)
+      for (int i = tid; i < nb * E; i += kThreads) s_part[i] = __ldcg(&xps[i]);
     __syncthreads();
+    // ---- E. the loss (model.py:213-216), beside the ranks: behind the copies it kept the kernels that wait for this one
+    // waiting (1173 tokens: 3.3 us) ----
+    if (b == 0 && warp == 1) {
+      float part = 0.f;
+      if (lane < E) {
+        float ps = 0.f;
+#pragma unroll 8
+        for (int bb = 0; bb < nb; ++bb) ps += s_part[bb * E + lane];      // in block order
+        psum[lane] = ps;
+        part = (ps / (float)Ntotal) * ((float)s_tot[lane] / (float)Ntotal);
+      }
+      float a = 0.f;
+      for (int e = 0; e < E; ++e) a += __shfl_sync(0xffffffffu, part, e);
+      if (lane == 0) aux[0] = a / (float)E * (float)(E * E);
+    }
   }
   if (warp == 0) {
     int tot = 0;
@@ -417,34 +465,22 @@ __device__ __forceinline__ void front_small_body(float* smem,
     }
   }
 
-  // ---- E. the loss, off the path of the kernels that wait for the rows (model.py:213-216) ----
-  if (blk == 0) {
+  // ---- E. the loss of the form in which every block has all tokens (model.py:213-216) ----
+  if (!SPLIT && blk == 0) {
     __syncthreads();       // the partial-logit area is free again: every thread is past the reduction
-    if constexpr (SPLIT) {
-      // the blocks' probability sums, added in block order
-      const int nb = nblk;
-      const float* xps = reinterpret_cast<const float*>(xch + nb * k * E);
-      if (tid < E) {
-        float ps = 0.f;
-        for (int bb = 0; bb < nb; ++bb) ps += __ldcg(&xps[bb * E + tid]);
-        psum[tid] = ps;
-        s_part[1024 + tid] = (ps / (float)Ntotal) * ((float)s_tot[tid] / (float)Ntotal);
-      }
-    } else {
-      // probabilities summed per expert: warp w takes tokens w, w + 32, ...; the 32 partial sums
-      // of an expert are then added in warp order
-      if (lane < E) {
-        float ps = 0.f;
-        for (int tok = warp; tok < N; tok += kThreads / 32) ps += s_logit[tok * ld + lane];
-        s_part[warp * 32 + lane] = ps;
-      }
-      __syncthreads();
-      if (tid < E) {
-        float ps = 0.f;
-        for (int w = 0; w < kThreads / 32; ++w) ps += s_part[w * 32 + tid];
-        psum[tid] = ps;
-        s_part[1024 + tid] = (ps / (float)N) * ((float)s_cnt[tid] / (float)N);
-      }
+    // probabilities summed per expert: warp w takes tokens w, w + 32, ...; the 32 partial sums
+    // of an expert are then added in warp order
+    if (lane < E) {
+      float ps = 0.f;
+      for (int tok = warp; tok < N; tok += kThreads / 32) ps += s_logit[tok * ld + lane];
+      s_part[warp * 32 + lane] = ps;
+    }
+    __syncthreads();
+    if (tid < E) {
+      float ps = 0.f;
+      for (int w = 0; w < kThreads / 32; ++w) ps += s_part[w * 32 + tid];
+      psum[tid] = ps;
+      s_part[1024 + tid] = (ps / (float)N) * ((float)s_cnt[tid] / (float)N);
     }
     __syncthreads();
     if (tid == 0) {
