@@ -58,66 +58,67 @@ combine_bwd_kernel(const __nv_bfloat16* dout, const __nv_bfloat16* y, const int3
   if (lane == 0) dw[p] = dot;
 }
 
-// Gradient of a token's logits by one warp; lane l holds experts l, l + 32, ... (PER of them).
+// Gradient of a token's logits by G lanes; lane l of them holds experts l, l + G, ... (PER of them).
 //   w_j = v_j / total, v_j = p[idx_j]:  dv_j = (dw_j - sum_i dw_i w_i) / total
 //   aux = E * sum_e mean_n p[n,e] * cnt0_e / N:  dp[e] += grad_aux * E * cnt0_e / N^2
 //   dl[e] = p[e] * (dp[e] - sum_e' p[e'] dp[e'])
-template <int PER>
+template <int PER, int G>
 __device__ __forceinline__ void token_dlogits(const float* __restrict__ logits, const int32_t* __restrict__ idx,
                                               const float* __restrict__ w, const float* dw,
                                               const int32_t* __restrict__ cnt0, float aux_c, int64_t t, int E, int k,
                                               int lane, float (&dl)[PER]) {
+  static_assert(G == 32 || PER == 1, "experts of a token over part of a warp");
   float p[PER], dp[PER];
   float m = -INFINITY;
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
-    const int e = lane + 32 * i;
+    const int e = lane + G * i;
     p[i] = e < E ? logits[t * E + e] : -INFINITY;
     m = fmaxf(m, p[i]);
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  for (int o = G / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
-    const int e = lane + 32 * i;
+    const int e = lane + G * i;
     p[i] = e < E ? expf(p[i] - m) : 0.f;
     sum += p[i];
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   // total of the chosen probabilities and sum_i dw_i w_i (every lane computes them: k <= 8)
   float total = 0.f, dww = 0.f;
   for (int j = 0; j < k; ++j) dww = fmaf(__ldcg(&dw[t * k + j]), w[t * k + j], dww);
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
-    const int e = lane + 32 * i;
+    const int e = lane + G * i;
     p[i] = p[i] / sum;
     dp[i] = e < E ? aux_c * (float)cnt0[e] : 0.f;
   }
   for (int j = 0; j < k; ++j) {
-    // p[e] lives in lane e & 31, slice e >> 5
+    // p[e] lives in lane e mod G, slice e / G
     const int e = idx[t * k + j];
     float v = 0.f;
 #pragma unroll
     for (int i = 0; i < PER; ++i)
-      if (i == (e >> 5)) v = p[i];
-    total += __shfl_sync(0xffffffffu, v, e & 31);
+      if (i == e / G) v = p[i];
+    total += __shfl_sync(0xffffffffu, v, e % G, G);
   }
   for (int j = 0; j < k; ++j) {
     const int e = idx[t * k + j];
     const float dv = (__ldcg(&dw[t * k + j]) - dww) / total;
-    if ((e & 31) == lane) {
+    if (e % G == lane) {
 #pragma unroll
       for (int i = 0; i < PER; ++i)
-        if (i == (e >> 5)) dp[i] += dv;
+        if (i == e / G) dp[i] += dv;
     }
   }
   float pdp = 0.f;
 #pragma unroll
   for (int i = 0; i < PER; ++i) pdp = fmaf(p[i], dp[i], pdp);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) pdp += __shfl_xor_sync(0xffffffffu, pdp, o);
+  for (int o = G / 2; o > 0; o >>= 1) pdp += __shfl_xor_sync(0xffffffffu, pdp, o);
 #pragma unroll
   for (int i = 0; i < PER; ++i) dl[i] = p[i] * (dp[i] - pdp);
 }
@@ -129,8 +130,10 @@ constexpr int kDlCols = 1024;    // columns of a block, four per thread
 // grid: (column blocks, token ranges, expert groups). Every block forms the logits' gradients of its tokens (the
 // first column block and expert group store them) and the products of its eight experts with its columns of
 // x; the partial sums of a token range go to part [range][E][d] and part_b [range][E] (no atomics: the same
-// result every time). What bounds it is one pass over x.
-template <int PER>
+// result every time). What bounds it is latency: a step's loads of x are under way while its logits' gradients are formed,
+// and up to 16 experts a warp takes four or two tokens side by side (16384 tokens, d 1024, 8 experts: 40 -> 20 us,
+// 1024 tokens 17 -> 8).
+template <int PER, int G>
 __global__ void __launch_bounds__(256)
 router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ idx,
                   const float* __restrict__ w, const float* dw,
@@ -155,31 +158,40 @@ router_bwd_kernel(const float* __restrict__ logits, const int32_t* __restrict__ 
   float bsum = 0.f;
   for (int64_t t0 = t_begin; t0 < t_end; t0 += kDlTokens) {
     const int nt = (int)min((int64_t)kDlTokens, t_end - t0);
+    const uint2* xp = reinterpret_cast<const uint2*>(x + t0 * d + c);
+    const size_t pitch = (size_t)d >> 2;
+    uint2 v[8];
+    auto request = [&](int tb) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        v[u] = c < d && tb + u < nt ? __ldg(xp + (size_t)(tb + u) * pitch) : make_uint2(0, 0);
+    };
+    request(0);
     __syncthreads();
-    for (int tl = warp; tl < nt; tl += 8) {
+    for (int tb = warp * (32 / G); tb < nt; tb += 8 * (32 / G)) {      // (whole warps stay together)
+      const int tl = tb + lane / G, l = lane % G;
       float dl[PER];
-      token_dlogits<PER>(logits, idx, w, dw, cnt0, aux_c, t0 + tl, E, k, lane, dl);
+      token_dlogits<PER, G>(logits, idx, w, dw, cnt0, aux_c, t0 + min(tl, nt - 1), E, k, l, dl);
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
-        const int e = lane + 32 * i;
-        if (e < E && store_dl) dl_out[(t0 + tl) * E + e] = dl[i];
-        if (e >= e0 && e < e0 + kDlExperts) s_dl[tl][e - e0] = e < E ? dl[i] : 0.f;
+        const int e = l + G * i;
+        if (tl < nt && e < E && store_dl) dl_out[(t0 + tl) * E + e] = dl[i];
+        if (tl < nt && e >= e0 && e < e0 + kDlExperts) s_dl[tl][e - e0] = e < E ? dl[i] : 0.f;
       }
     }
     __syncthreads();
     if (blockIdx.x == 0 && tid < kDlExperts)
       for (int tl = 0; tl < nt; ++tl) bsum += s_dl[tl][tid];
     if (c < d) {
-      const uint2* xp = reinterpret_cast<const uint2*>(x + t0 * d + c);
-      const size_t pitch = (size_t)d >> 2;
       for (int tb = 0; tb < nt; tb += 8) {
-        uint2 v[8];
+        uint2 now[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = tb + u < nt ? __ldg(xp + (size_t)(tb + u) * pitch) : make_uint2(0, 0);
+        for (int u = 0; u < 8; ++u) now[u] = v[u];
+        if (tb + 8 < nt) request(tb + 8);
 #pragma unroll
         for (int u = 0; u < 8; ++u)
           if (tb + u < nt) {
-            const float xv[4] = {bf16_lo(v[u].x), bf16_hi(v[u].x), bf16_lo(v[u].y), bf16_hi(v[u].y)};
+            const float xv[4] = {bf16_lo(now[u].x), bf16_hi(now[u].x), bf16_lo(now[u].y), bf16_hi(now[u].y)};
             const float4 ga = *reinterpret_cast<const float4*>(&s_dl[tb + u][0]);
             const float4 gb = *reinterpret_cast<const float4*>(&s_dl[tb + u][4]);
             const float g[kDlExperts] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
@@ -284,6 +296,7 @@ combine_dx_kernel(const __nv_bfloat16* __restrict__ dxs, const int32_t* __restri
         }
     }
   }
+#pragma unroll 4
   for (int e = 0; e < E; ++e) {
     float wv[8];
     load8_ldg(Wg + (size_t)e * d + c, wv);
@@ -437,7 +450,10 @@ int launch_router_bwd(const float* logits, const int32_t* idx, const float* w, c
   const int64_t per = router_bwd_tokens(N, d, E);
   const int64_t ranges = (N + per - 1) / per;
   float* part_b = scratch + (size_t)ranges * E * d;
-  auto fn = E <= 32 ? router_bwd_kernel<1> : (E <= 64 ? router_bwd_kernel<2> : router_bwd_kernel<kMaxExperts / 32>);
+  auto fn = E <= 8 ? router_bwd_kernel<1, 8>
+                   : (E <= 16 ? router_bwd_kernel<1, 16>
+                              : (E <= 32 ? router_bwd_kernel<1, 32>
+                                         : (E <= 64 ? router_bwd_kernel<2, 32> : router_bwd_kernel<kMaxExperts / 32, 32>)));
   const dim3 grid((d + kDlCols - 1) / kDlCols, (unsigned)ranges, (E + kDlExperts - 1) / kDlExperts);
   MOE_CUDA_CHECK(launch_pdl(fn, grid, dim3(256), 0, s, logits, idx, w, dw, cnt0, grad_aux, grad_aux_dev,
                             static_cast<const __nv_bfloat16*>(x), N, d, E, k, (int)per, dl, scratch, part_b));

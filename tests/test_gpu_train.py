@@ -142,6 +142,14 @@ def test_backward_of_token_counts_that_are_no_multiple_of_four(cuda_device, N, k
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,E,k", [(33, 3, 2), (31, 9, 3), (70, 16, 2), (40, 17, 2), (40, 33, 4)])
+def test_backward_by_the_number_of_experts(cuda_device, N, E, k):
+    """A warp of the router's backward pass takes four tokens of up to 8 experts, two of up to 16, else one: same comparison
+    and tolerance as above."""
+    test_backward_matches_autograd_on_the_oracle(cuda_device, N, 72, E, 136, k, 0.1)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("N,d,E,f,k,p", [(600, 128, 8, 256, 2, 0.1), (900, 256, 4, 264, 2, 0.0)])
 def test_fine_tuning_trains_the_lora_tensors(cuda_device, N, d, E, f, k, p):
     """fine_tuning=True under .train() (what the reference's fine-tuning loop runs,
