@@ -306,6 +306,12 @@ def test_lora_merge(cuda_device, out_f, in_f, rank, dtype):
         assert ((got.cpu().double() - want).abs() <= eps * want.abs() + 2e-5).all()
 
 
+# bf16: units of 16 rows x 128 columns, more of them than warps, ranks in steps of 16
+@pytest.mark.parametrize("out_f,in_f,rank", [(16, 128, 16), (17, 136, 17), (5000, 1032, 33)])
+def test_lora_merge_by_units(cuda_device, out_f, in_f, rank):
+    test_lora_merge(cuda_device, out_f, in_f, rank, torch.bfloat16)
+
+
 # edges of the fp32 token tiles (16 and 160 tokens) and of the read-outs (64 and 256 of K), whole and with K over clusters
 # of two, four and eight CTAs, more tiles than SMs
 @pytest.mark.parametrize("rows,d,f", [([15, 16, 17, 159], 512, 2048), ([160, 161, 0, 321], 1024, 512), ([7], 1024, 136),
