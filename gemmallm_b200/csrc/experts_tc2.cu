@@ -30,9 +30,8 @@
 // block stop, and passes the stage on. (Only there do the two CTAs arrive on a common barrier: an
 // arrival across the pair for every block halved the rate, 680 instead of 1280 TFLOP/s.)
 //
-// SPLIT > 1 (kPlain, kDx): products of few tiles and a long contraction. A tile of 256 x 256 takes 0.39 us per
-// 64 of K however few of them run (the tensor pipe's own rate: 1630 TFLOP/s if all 74 pairs had one), so 28 tiles
-// of K = 4096 left 46 pairs idle for 27 us. SPLIT pairs in one cluster take a range of K each, put their fp32
+// SPLIT > 1 (kPlain, kDx): products of few tiles and a long contraction. A tile of 256 x 256 takes 0.31 us per
+// 64 of K however few of them run (shared memory's rate: 580 clk), so 28 tiles of K = 4096 left 46 pairs idle for 20 us. SPLIT pairs in one cluster take a range of K each, put their fp32
 // accumulators into shared memory (the stages are free by then: a cluster has one tile) and each adds up and
 // stores 256 / SPLIT columns, in the order of the ranges. (128-column tiles instead gained nothing: a product of
 // half the columns takes the same time.)

@@ -385,8 +385,9 @@ int moe_b200_layernorm(const void* x, const void* norm_weight, const void* norm_
  * call selects the kernels (bf16): one to eight tokens with fewer than E rows
  * moe_b200_decode_tiny; up to moe_b200_decode_max_rows() rows the single-launch
  * front and a weight-streaming expert kernel; up to 4096 rows the front and the
- * streaming kernel on sorted rows; beyond that router, dispatch, the two grouped
- * GEMM passes and combine. */
+ * streaming kernel on sorted rows; from 96 to 2048 rows per expert (and, with more
+ * than 32 experts, below) both products in one launch; beyond that router, dispatch,
+ * the two grouped GEMM passes and combine. */
 int moe_b200_forward(const void* x, const void* Wg, const void* bg,
                      const void* plan, const void* residual,
                      const void* norm_weight, const void* norm_bias, float norm_eps,
