@@ -186,7 +186,7 @@ experts_mid_kernel(const __grid_constant__ CUtensorMap tmap_x64, const __grid_co
                    const __grid_constant__ CUtensorMap tmap_h64, const __grid_constant__ CUtensorMap tmap_h16,
                    const CUtensorMap* __restrict__ tmap_w1, const CUtensorMap* __restrict__ tmap_w2,
                    const int32_t* __restrict__ offsets, const void* const* __restrict__ b1, const void* const* __restrict__ b2,
-                   int E, int d, int f, __nv_bfloat16* __restrict__ h, __nv_bfloat16* __restrict__ y,
+                   int E, int d, int f, int ahead, __nv_bfloat16* __restrict__ h, __nv_bfloat16* __restrict__ y,
                    int* __restrict__ ready, int32_t* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -221,7 +221,7 @@ experts_mid_kernel(const __grid_constant__ CUtensorMap tmap_x64, const __grid_co
                  "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  if (warp == 2 && elect_one()) {
+  if (ahead && warp == 2 && elect_one()) {
     // the first weights into L2 while the routing still runs, which they do not depend on: 28 MiB in all
     for (int i = 0, t = blockIdx.x >> 1; i < 12 && t < E * w.n1; t += gridDim.x >> 1) {
       const int e = t / w.n1, nt = t - e * w.n1;
@@ -599,9 +599,12 @@ int launch_experts_mid(const void* perm, const int32_t* offsets, const void* pla
   if (!rc) rc = encode_tmap_2d(&h64, h, (uint64_t)M, (uint64_t)f, 64);
   if (!rc) rc = encode_tmap_2d(&h16, h, (uint64_t)M, (uint64_t)f, 16);
   if (rc) return rc;
+  // with fewer rows many experts have none, and their weights would come for nothing (64 experts: 1 token 102.2 -> 99.7 us,
+  // 12 tokens 148.3 -> 147.2; the same at 64)
+  const int ahead = M >= 2 * (int64_t)E ? 1 : 0;
   MOE_CUDA_CHECK(launch_pdl_cluster(experts_mid_kernel, dim3((unsigned)(sms & ~1)), dim3(kThreads), 2, kSmemBytes, s, x64,
                                     x16, h64, h16, static_cast<const CUtensorMap*>(pv.tmap_W1_pairs),
-                                    static_cast<const CUtensorMap*>(pv.tmap_W2), offsets, pv.b1, pv.b2, E, d, f,
+                                    static_cast<const CUtensorMap*>(pv.tmap_W2), offsets, pv.b1, pv.b2, E, d, f, ahead,
                                     static_cast<__nv_bfloat16*>(h), static_cast<__nv_bfloat16*>(y), ready, status));
   return 0;
 }
