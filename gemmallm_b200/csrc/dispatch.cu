@@ -292,7 +292,18 @@ dispatch_kernel(const T* __restrict__ x, const int32_t* __restrict__ idx, int64_
     if (lane == 0) cnt_slot[i] = acc;
   }
   if (psum_part == nullptr) return;
-  for (int e = blockIdx.x; e < E; e += G) {
+  // up to 32 partial sums an expert: a warp each, in the order of the block's tree below (which took 64 experts in turn where
+  // one block has all tokens: calls of 1 token 99.6 -> 60.7 us, of 12 147 -> 134)
+  const bool few = router_blocks <= 32;
+  if (few) {
+    for (int e = blockIdx.x * (kThreads / 32) + warp; e < E; e += G * (kThreads / 32)) {
+      float acc = lane < router_blocks ? psum_part[(int64_t)lane * E + e] : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+      if (lane == 0) psum[e] = acc;
+    }
+  }
+  for (int e = few ? E : (int)blockIdx.x; e < E; e += G) {
     float acc = 0.f;
     for (int64_t b = tid; b < router_blocks; b += kThreads) acc += psum_part[b * E + e];
     s_red[tid] = acc;

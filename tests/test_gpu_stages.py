@@ -852,3 +852,19 @@ def test_attention_core(cuda_device, B, S, H, KV, masked, shift):
     # probabilities by as much of themselves; probabilities and outputs are rounded once more: about 2^-7 in the
     # 2-norm, twice that allowed
     assert (out.float().cpu() - want).norm() <= 2 ** -6 * want.norm()
+
+
+# up to 32 router blocks of 64 tokens a warp sums an expert's partial probabilities, beyond them a block
+@pytest.mark.parametrize("N,E", [(1, 64), (64, 200), (2048, 17), (2049, 17), (2049, 64)])
+def test_dispatch_probability_sums(cuda_device, N, E):
+    g = torch.Generator().manual_seed(N + E)
+    blocks = (N + 63) // 64
+    part = torch.rand(blocks, E, generator=g)
+    idx = torch.randint(E, (N, 1), generator=g, dtype=torch.int32)
+    got = helpers.dispatch(torch.zeros(N, 8, device=cuda_device).bfloat16(), idx.to(cuda_device), E, part.to(cuda_device))
+    want = part.double().sum(0)
+    # sums of at most 33 terms in fp32: six roundings on a path of the tree, 2^-24 each
+    assert ((got["psum"].cpu().double() - want).abs() <= 6 * 2.0 ** -24 * want).all()
+    freq = torch.bincount(idx[:, 0].long(), minlength=E).double() / N
+    aux = float((want / N * freq).sum() * E)
+    assert abs(float(got["aux"]) - aux) <= 1e-5 * aux
