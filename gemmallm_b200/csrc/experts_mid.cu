@@ -24,8 +24,8 @@
 // last tiles, 7 us. Block, d 1024, f 4096, 8 experts, two slots, weights not in L2, whole calls, us, with the streaming
 // kernel (up to 1024 tokens) or the 256-row tiles / with this one: 384 tokens 62 / 63, 512 72.7 / 64.7, 640 86.7 / 67.0, 1024
 // 97.3 / 79.9, 1173 110.5 / 88.0, 2048 151.5 / 125.8, 4096 233.8 / 224.0, 8192 385 / 390. 64 experts, d 2048, f 1408, four
-// slots: 1 token 146 / 100 (61 with a shorter dispatch), 16 1211 / 153, 64 942 / 207, 512 242 / 218, 4096 448 / 377, 16384 (popularity after Zipf)
-// 1202-1254 / 1155.
+// slots: 1 token 146 / 100 (61 with a shorter dispatch), 16 1211 / 153, 64 942 / 207, 512 242 / 218, 4096 448 / 377, 16384
+// (popularity after Zipf) 1202-1254 / 1155.
 // Tried and taken back: prefetches of weights into L2 ahead of their load (the SM's TMA unit takes as long for one as for a
 // load: 94 -> 100 us at 1173 tokens); the down product cut into equal ranges of K for all pairs, with partial sums handed
 // on through L2 (64 tiles for 74 pairs: the exchange took 5 us, as much as it gave; 1024 tokens 81 -> 87 us).
