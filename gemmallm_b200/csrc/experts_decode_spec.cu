@@ -128,9 +128,10 @@ decode_spec_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 
   int* tile_counter = ready + (MOE_B200_READY_INTS - 1);
 
-  // first tile: the claim is in flight while the barriers and the tensor memory are set up
+  // first tile: the claim is in flight while the barriers and the tensor memory are set up (by the lane that is elected
+  // again for the role that uses it: no other lane has it)
   int first_tile = 0;
-  if (threadIdx.x == 0) first_tile = atomicAdd(tile_counter, 1);
+  if (warp == 0 && elect_one()) first_tile = atomicAdd(tile_counter, 1);
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&ctl->full[s], 1); mbar_init(&ctl->empty[s], 1); }
     for (int a = 0; a < 2; ++a) {

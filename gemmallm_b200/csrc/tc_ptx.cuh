@@ -36,11 +36,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// One lane of a whole warp, the same one every time. The roles that issue TMA loads and products enter their loops by this
-// and not by `lane == 0`: only so does the compiler know that one lane is left, and keeps the operands of those instructions
-// in uniform registers. A load loop of three boxes a stage took 640 clk an iteration by `lane == 0` and takes 445 this way;
-// the issue of loads, not the tensor pipe, was what the grouped products waited for (32768 rows, d 1024, f 4096, 8 experts,
-// us: gate_and_up 407 -> 359, down 206 -> 196).
+// One lane of a whole warp, the same one every time but not known to be lane 0: what a role entered by this has in registers
+// from before must be in all lanes, or come from an elected lane as well. The roles that issue TMA loads and products enter
+// their loops by this and not by `lane == 0`: only so does the compiler know that one lane is left, and keeps the operands of
+// those instructions in uniform registers. A load loop of three boxes a stage took 640 clk an iteration by `lane == 0` and
+// takes 445 this way; the issue of loads, not the tensor pipe, was what the grouped products waited for (32768 rows, d 1024,
+// f 4096, 8 experts, us: gate_and_up 407 -> 359, down 206 -> 196).
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));

@@ -114,6 +114,19 @@ def test_rows_and_router_weights_off_a_16_byte_boundary_are_refused_before_any_l
         assert call(a, a + 4) == -3 and b"16-byte" in lib.moe_b200_last_error_string()
 
 
+def test_a_claimed_tile_belongs_to_the_lane_whose_role_uses_it():
+    """elect.sync does not say which lane it picks: a tile that another lane claims before the roles part would be lost, and a
+    kernel whose blocks wait for its rows with it. Read from the source: on hardware that picks lane 0 nothing shows it."""
+    csrc = HEADER.parent.parent / "gemmallm_b200" / "csrc"
+    claims = {}
+    for src in sorted(csrc.glob("experts_*.cu")):
+        text = src.read_text()
+        if "if (elect_one())" in text:
+            claims.update({(src.name, i): line for i, line in enumerate(text.splitlines())
+                           if re.search(r"if \(.*\) *\w+ = atomicAdd\(", line)})
+    assert len(claims) == 2 and all("elect_one()" in line for line in claims.values()), claims
+
+
 def test_host_extension_is_rebuilt_for_another_torch(tmp_path, monkeypatch):
     """Same sources, same dates: what counts besides them is the torch it was built against."""
     from gemmallm_b200 import build
