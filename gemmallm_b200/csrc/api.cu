@@ -254,6 +254,10 @@ int moe_b200_experts(const void* perm, const int32_t* offsets, const void* plan,
 
 int moe_b200_rows_splits(int64_t M, int d, int f, int E) { return M > 0 && f >= 8 && d >= 8 && E >= 1 ? rows_splits(M, d, f, E) : 0; }
 
+int moe_b200_one_launch(int64_t M, int d, int f, int E) {
+  return check_shape(0, d, f, E, 1, MOE_B200_BF16) == 0 && M < (int64_t)1 << 31 && experts_mid_chosen(M, d, f, E);
+}
+
 int moe_b200_experts_rows(const void* perm, const int32_t* offsets, const void* plan, int64_t M,
                           int d, int f, int E, int ksplit, void* h, float* part, int32_t* ready,
                           int32_t* status, void* stream) {
@@ -470,9 +474,8 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   // between the decode and the prefill sizes: the streaming kernel on the sorted rows
   const bool rows_path = dtype == MOE_B200_BF16 && !small_n && N * k <= kRowsPathMaxRows &&
                          rows_supported(N * k, E);
-  // both products in one launch on tiles that fit an expert's rows: from 64 rows an expert on, and beyond these sizes to
-  // 2048 rows an expert (experts_mid.cu); with more than 32 experts, which neither kernel for few rows takes, at any number
-  const bool mid = dtype == MOE_B200_BF16 && experts_mid_chosen(N * k, E);
+  // both products in one launch on tiles that fit an expert's rows, where that is the faster (experts_mid.cu)
+  const bool mid = dtype == MOE_B200_BF16 && experts_mid_chosen(N * k, d, f, E);
   // (a folded LayerNorm stays with the general kernels)
   bool front32 = dtype == MOE_B200_F32 && !norm && front_f32_supported(N, E, k);
   bool front = front32 || ((small_n || rows_path) && (front_small_supported(N, E, k, dtype) ||

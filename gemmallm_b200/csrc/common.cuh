@@ -320,7 +320,7 @@ int launch_experts_tc2(const void* perm, const int32_t* offsets, const void* pla
                        const EpSync* ep_signal = nullptr);
 // Both products in one launch, for calls between the decode and the prefill sizes (experts_mid.cu); `ready` as for
 // launch_experts_tc_decode_spec.
-bool experts_mid_chosen(int64_t M, int E);
+bool experts_mid_chosen(int64_t M, int d, int f, int E);
 int launch_experts_mid(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d, int f, int E, void* h,
                        void* y, int* ready, int32_t* status, cudaStream_t s);
 // Input gradient of a grouped Linear: out[rows of e] = A[rows of e] . B_e, B_e [K, Nout] row-major, given by
@@ -362,6 +362,7 @@ bool decode_spec_supported(int64_t N, int E, int k);
 int launch_experts_tc_decode_spec(const void* x, const int32_t* idx, const int32_t* offsets,
                                   const void* plan, int64_t N, int k, int d, int f, int E, void* h_all,
                                   float* part, int* ready, int32_t* status, cudaStream_t s);
+int rows_block(int64_t M, int E);
 int rows_splits(int64_t M, int d, int f, int E);
 bool rows_supported(int64_t M, int E);
 int launch_experts_tc_rows(const void* perm, const int32_t* offsets, const void* plan, int64_t M,

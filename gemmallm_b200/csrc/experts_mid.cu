@@ -21,15 +21,15 @@
 // What bounds it: from some 150 rows an expert on, shared memory: a step of 64 of K brings in 16 KiB of weights and n/2 x 128
 // bytes of tokens a CTA and the products read both again; 500 clk at N = 160 and 580 at 256, for 320 and 512 of products.
 // Below, the stream of the weights. Kept from the two launches it replaces: nothing of the second's start and of the first's
-// last tiles, 7 us. Block, d 1024, f 4096, 8 experts, two slots, weights not in L2, whole calls, us, with the streaming
-// kernel (up to 1024 tokens) or the 256-row tiles / with this one: 384 tokens 62 / 63, 512 72.7 / 64.7, 640 86.7 / 67.0, 1024
-// 97.3 / 79.9, 1173 110.5 / 88.0, 2048 151.5 / 125.8, 4096 233.8 / 224.0, 8192 385 / 390. 64 experts, d 2048, f 1408, four
-// slots: 1 token 146 / 100 (61 with a shorter dispatch), 16 1211 / 153, 64 942 / 207, 512 242 / 218, 4096 448 / 377, 16384
-// (popularity after Zipf) 1202-1254 / 1155.
+// last tiles, 7 us. Block, d 1024, f 4096, 8 experts, two slots, weights not in L2, whole calls one after the other, us, with
+// the streaming kernel (up to 2048 tokens) or the 256-row tiles / with this one: 384 tokens 62.2 / 62.2, 512 70.7 / 63.2, 640
+// 79.7 / 64.6, 1024 94.1 / 74.9, 2048 127 / 104, 4096 193 / 180, 8192 349 / 319. 64 experts, d 2048, f 1408, four slots: 1
+// token 99 / 58, 16 1163 / 147, 64 929 / 207, 512 225 / 219, 4096 396 / 332, 16384 998 / 999.
 // Tried and taken back: prefetches of weights into L2 ahead of their load (the SM's TMA unit takes as long for one as for a
 // load: 94 -> 100 us at 1173 tokens); the down product cut into equal ranges of K for all pairs, with partial sums handed
 // on through L2 (64 tiles for 74 pairs: the exchange took 5 us, as much as it gave; 1024 tokens 81 -> 87 us).
 #include <cuda.h>
+#include <cmath>
 #include "common.cuh"
 #include "tc_ptx.cuh"
 #include "tc_pair.cuh"
@@ -573,14 +573,41 @@ experts_mid_kernel(const __grid_constant__ CUtensorMap tmap_x64, const __grid_co
 
 }  // namespace
 
-// From 96 rows an expert on (at 75, 300 tokens, the streaming kernel takes 60 us and this one 62) to 2048, where remainders
-// no longer count and the 256-row tiles are as fast. With one or two experts tiles are few, and the streaming kernel, which
-// cuts K, is the faster up to 1536 rows (1 expert, d 1024, f 4096: 600 rows 46 / 50 us). With more than 32 experts, which the
-// kernels for few rows do not take, from one row on.
-bool experts_mid_chosen(int64_t M, int E) {
-  if (E > 32) return M > 0 && M <= (int64_t)2048 * E;
+// Whether a call of M rows is better off here than with the kernels it would take else.
+// More than 32 experts, up to 256 rows: the matrix-vector kernel goes row by row (64 experts, d 2048, f 1408, four slots, us:
+// 4 rows 99 / here 58, 64 rows 1163 / 147). Up to 32 experts the streaming kernel is as fast below 96 rows an expert (600 rows of
+// 8 experts 60 / 62) and, with one or two experts, below 1536 rows.
+// Up to 4096 rows the streaming kernel remains (experts_decode_spec.cu, sorted rows), which cuts the down product's K into
+// ranges for all SMs. Here that product takes whole rounds of all K on pairs of SMs, and where d is small and f large its
+// few tiles are the longest part of the call (d 256, f 8192, 8 experts, 768 rows: 51.8 / here 68.3 us, 3 experts 45.4 /
+// 67.9), while the streaming kernel's GEGLU product reads weights once per 128 rows. So the two are compared by what
+// differs, rounds x steps of 64 of K under balanced routing, in us: a step of the down product here, up to 0.31 with 256
+// tokens, and 0.75 a round of GEGLU epilogues; there 0.30 a step of GEGLU with 128 rows, 0.27 one of a range of down's K, and
+// what the fp32 sums of the ranges cost. Fitted to whole calls of both kernels: 1 to 200 experts, d 64 to 4096, f 264 to
+// 16384, 2012 sizes. The kernel that is chosen takes 0.4 % longer than the faster one on average (always here: 4 %), and is
+// the slower one by more than 3 % at 118 sizes (by 4.5 % in the middle of them, by 15 % at most).
+// Beyond, the 256-row tiles remain (experts_tc2.cu), to which remainders no longer count at 2048 rows an expert (8 experts,
+// d 1024, f 4096 there: 349 / here 319). With K of the down product more than four times that of gate_and_up a tile's
+// epilogue is the bound, and theirs is the faster: up to 2 d rows an expert this one is still ahead (d 256, f 2048, 24
+// experts, 320 rows each 93.9 / 87.3; d 256, f 8192, 8 experts, 2048 rows each 262 / 292).
+bool experts_mid_chosen(int64_t M, int d, int f, int E) {
+  if (M <= kDecodeMaxRows) return E > 32 && M > 0;
+  const int64_t least = E > 32 ? 0 : E > 2 ? (int64_t)96 * E : 1536;
   const int64_t most = E > 2 ? (int64_t)2048 * E : kRowsPathMaxRows;
-  return M > kDecodeMaxRows && M >= (E > 2 ? (int64_t)96 * E : 1536) && M <= most;
+  if (M < least || M > most) return false;
+  if (M > kRowsPathMaxRows || !rows_supported(M, E)) return f <= 4 * d + 64 || M <= (int64_t)2 * d * E;
+  auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+  auto rounds = [](int64_t tiles, int units) { return fmax(1., (double)tiles / units + .5); };
+  const int64_t hit = M < E ? M : E, share = up(M, hit);          // experts with rows, rows of one
+  const int64_t cut = up(share, kMaxTok), n = up(up(share, cut), 32) * 32;
+  const int64_t n1 = up(f, 128), n2 = up(d, 256), kb1 = up(d, BK), kb2 = up(f, BK);
+  const int NP = rows_block(M, E), ks = rows_splits(M, d, f, E);
+  const int64_t blocks = hit * up(share, NP);                     // of the streaming kernel
+  const double here = rounds(hit * cut * n2, kNumSMs / 2) * kb2 * (0.078 + 0.232 * n / kMaxTok) +
+                      0.75 * rounds(hit * cut * n1, kNumSMs / 2) - 1.3;
+  const double there = 0.30 * rounds(blocks * n1, kNumSMs) * kb1 * NP / 128 +
+                       0.27 * rounds(blocks * n2 * ks, kNumSMs) * up(kb2, ks) + 1.5e-6 * M * d * ks;
+  return here < there;
 }
 
 int launch_experts_mid(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d, int f, int E, void* h,

@@ -234,6 +234,10 @@ int moe_b200_experts_rows(const void* perm, const int32_t* offsets, const void* 
                           int32_t* ready, int32_t* status, void* stream);
 int moe_b200_rows_splits(int64_t M, int d, int f, int E);
 
+/* 1 if moe_b200_forward computes both products of a bf16 call of M = N*k rows in one launch on tiles that fit an
+ * expert's rows, 0 if it takes one of the other kernels. */
+int moe_b200_one_launch(int64_t M, int d, int f, int E);
+
 /* Parts 1+2 for a handful of tokens in ONE single-block launch: same results as
  * moe_b200_router followed by moe_b200_dispatch (model.py:206-253), for bf16,
  * 1 <= N <= 512, N*k <= 1024, E <= 32; other shapes return
@@ -386,8 +390,8 @@ int moe_b200_layernorm(const void* x, const void* norm_weight, const void* norm_
  * moe_b200_decode_tiny; up to moe_b200_decode_max_rows() rows the single-launch
  * front and a weight-streaming expert kernel; up to 4096 rows the front and the
  * streaming kernel on sorted rows; from 96 to 2048 rows per expert (and, with more
- * than 32 experts, below) both products in one launch; beyond that router, dispatch,
- * the two grouped GEMM passes and combine. */
+ * than 32 experts, below) both products in one launch where moe_b200_one_launch says so;
+ * beyond that router, dispatch, the two grouped GEMM passes and combine. */
 int moe_b200_forward(const void* x, const void* Wg, const void* bg,
                      const void* plan, const void* residual,
                      const void* norm_weight, const void* norm_bias, float norm_eps,

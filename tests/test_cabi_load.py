@@ -114,6 +114,24 @@ def test_rows_and_router_weights_off_a_16_byte_boundary_are_refused_before_any_l
         assert call(a, a + 4) == -3 and b"16-byte" in lib.moe_b200_last_error_string()
 
 
+def test_which_calls_compute_both_products_in_one_launch():
+    """Its lines, and the calls with few tiles of a long down product, which stay with the kernels that split its K."""
+    one = lib.moe_b200_one_launch
+    # the workloads' shapes, from 96 rows an expert to 2048
+    for d, f, E in ((1024, 4096, 8), (512, 2048, 8), (2048, 1408, 8), (1024, 512, 4), (4096, 1024, 32)):
+        assert [one(r, d, f, E) for r in (96 * E - 1, 96 * E, 512 * E, 2048 * E, 2048 * E + 1)] == [0, 1, 1, 1, 0]
+    assert [one(r, 1024, 4096, 2) for r in (1535, 1536, 4096, 4097)] == [0, 1, 1, 0]
+    # down products of 128 steps of K in 3 to 16 tiles: 68 us against 45 to 52 of the streaming kernel, and K in ranges there
+    assert [one(M, 256, 8192, E) for M, E in ((288, 3), (768, 3), (768, 8), (1536, 8), (1800, 1), (2048, 2), (896, 8))] == [0] * 7
+    assert one(768, 512, 8192, 4) == 0 and one(1280, 1024, 8192, 8) == 1
+    # beyond 4096 rows: the epilogue's share where K of gate_and_up is short
+    assert one(16384, 256, 8192, 8) == 0 and one(7680, 256, 2048, 24) == 1 and one(16384, 512, 2048, 8) == 1
+    # more than 32 experts: up to 256 rows whatever the shape, and where row blocks outnumber the streaming kernel's counters
+    assert [one(r, 256, 8192, 64) for r in (0, 1, 256, 257, 4096)] == [0, 1, 1, 0, 0]
+    assert one(4096, 256, 8192, 200) == 1 and one(256, 1024, 4096, 32) == 0
+    assert one(1024, 1020, 4096, 8) == 0 and one(1 << 31, 1024, 4096, 256) == 0      # no such call
+
+
 def test_a_claimed_tile_belongs_to_the_lane_whose_role_uses_it():
     """elect.sync does not say which lane it picks: a tile that another lane claims before the roles part would be lost, and a
     kernel whose blocks wait for its rows with it. Read from the source: on hardware that picks lane 0 nothing shows it."""
