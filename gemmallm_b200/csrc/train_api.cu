@@ -66,7 +66,7 @@ TrainArgs train_args(char* tws, const size_t* to, float p, uint64_t seed, bool l
 }
 
 // Backward of the grouped expert feed-forward (model.py:174-184) on sorted rows: given dy (gradient of y),
-// h (the dropped h of the forward), the saved pre-activations and the sorted inputs, writes g.x (gradient of the
+// h (the dropped h of the forward), what the forward kept in gu and mask (TrainArgs) and the sorted inputs, writes g.x (gradient of the
 // sorted inputs) and the four parameter gradients.
 int experts_backward(const void* perm, const void* h, const int32_t* offsets, const void* plan, const void* dy,
                      int64_t M, int d, int f, int E, const TrainArgs& tr, const TrainGrads& g, const LoraGrads* lora,

@@ -32,7 +32,9 @@
 extern "C" {
 #endif
 
-#define MOE_B200_ABI_VERSION 2
+/* 3: plans hold a fifth tensor map an expert; after a training forward MOE_B200_TWS_GU holds derivatives of h instead of
+ * pre-activations, and MOE_B200_TWS_MASK is written in LoRA steps only. */
+#define MOE_B200_ABI_VERSION 3
 
 enum { MOE_B200_F32 = 0, MOE_B200_BF16 = 1 };
 
@@ -443,7 +445,8 @@ enum {
   MOE_B200_TWS_G_W2,     /* [E,d,f]    experts.e.down.weight */
   MOE_B200_TWS_G_B2,     /* [E,d]      experts.e.down.bias */
   MOE_B200_TWS_MASK,     /* uint8 [N*k, f/8], LoRA steps of the modules: the dropout mask of h, one bit per element,
-                          * whose GU holds the pre-activations; else the mask is part of GU and this is not used */
+                          * whose GU holds the pre-activations. Else the mask is part of GU and this, laid out for every
+                          * step alike, is not written */
   MOE_B200_TWS_COL_PART, /* float      partial column sums of the bias gradients */
   MOE_B200_TWS_NUM
 };

@@ -44,6 +44,13 @@ def test_version_and_sizes():
     assert lib.moe_b200_dispatch_scratch_bytes(1000, 8, 2) > 0
 
 
+def test_version_goes_with_the_plan_and_the_training_workspace():
+    """A caller built against another layout of a plan, or against other contents of GU and MASK, sees another version."""
+    maps = [(lib.moe_b200_plan_bytes(E) - (32 * E + 127) // 128 * 128) / (128 * E) for E in (1, 8, 256)]
+    assert (lib.moe_b200_version(), maps) == (3, [5, 5, 5])
+    assert re.search(r"ABI_VERSION 3\b", HEADER.read_text())
+
+
 def test_bad_shapes_are_rejected_on_the_host():
     assert lib.moe_b200_workspace_bytes(16, 1020, 4096, 8, 2, _cabi.BF16) == 0   # d % 8
     assert lib.moe_b200_workspace_bytes(16, 1024, 4096, 300, 2, _cabi.BF16) == 0  # E > 256
