@@ -598,7 +598,9 @@ def run_ours(args, wl):
             gbs_experts = wbytes / (stage_ms["experts"] * 1e-3) / 1e9
             line["roofline"] = {
                 "kernel": ("decode_spec_kernel (GEGLU + split-K down tiles, one launch) / geglu_gemv + down_gemv"
-                           if small_n else "decode_spec_kernel<SORTED> (GEGLU + split-K down tiles on sorted rows)"),
+                           if small_n else "experts_mid_kernel (GEGLU + down tiles on blocks of an expert's rows, one launch)"
+                           if _cabi.lib.moe_b200_one_launch(N * k, d, f, E)
+                           else "decode_spec_kernel<SORTED> (GEGLU + split-K down tiles on sorted rows)"),
                 "bound": "hbm", "achieved": gbs_experts, "peak": hbm, "unit": "GB/s",
                 "frac": gbs_experts / hbm, "traffic": traffic, "traffic_source": traffic_source,
                 "peak_source": f"{peak_kind} copy",
@@ -1402,11 +1404,12 @@ def time_stages(m, x2d, wl, dev, small_n: bool = False, reps: int = 20, mid_n: b
             p["part"], splits, N * k, p["row_of"], p["idx"], p["w"], plan, E, None, N, d, k,
             out.data_ptr(), s)
     if mid_n:
-        # single-launch front (blocks share the routing), streaming kernel on the sorted rows,
-        # the small-N combine
+        # single-launch front (blocks share the routing), then the streaming kernel on the sorted rows and the
+        # small-N combine, or both products in one launch and the combine of bf16 rows
         ks = lib.moe_b200_rows_splits(N * k, d, f, E)
         ready = p["status"] + 4 * _cabi.READY_OFFSET
         counter = ready + 4 * (_cabi.READY_INTS - 4)
+        combine = calls["combine"]
         calls = {
             "front": lambda: lib.moe_b200_front_small_split(
                 x2d.data_ptr(), gw.data_ptr(), gb.data_ptr(), N, d, E, k, code, p["logits"], p["idx"],
@@ -1419,6 +1422,10 @@ def time_stages(m, x2d, wl, dev, small_n: bool = False, reps: int = 20, mid_n: b
                 p["part"], ks, N * k, p["row_of"], p["idx"], p["w"], plan, E, None, N, d, k,
                 out.data_ptr(), s),
         }
+        if lib.moe_b200_one_launch(N * k, d, f, E):
+            calls["experts"] = lambda: lib.moe_b200_experts_mid(
+                p["perm"], p["offsets"], plan, N * k, d, f, E, p["h"], p["y"], ready, p["status"], s)
+            calls["combine"] = combine
     res = {}
     for name, fn in calls.items():
         for _ in range(3):

@@ -258,6 +258,18 @@ int moe_b200_one_launch(int64_t M, int d, int f, int E) {
   return check_shape(0, d, f, E, 1, MOE_B200_BF16) == 0 && M < (int64_t)1 << 31 && experts_mid_chosen(M, d, f, E);
 }
 
+int moe_b200_experts_mid(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d, int f, int E,
+                         void* h, void* y, int32_t* ready, int32_t* status, void* stream) {
+  int rc = check_shape(0, d, f, E, 1, MOE_B200_BF16);
+  if (rc) return rc;
+  if (M < 0 || M >= (int64_t)1 << 31) return set_error(MOE_B200_ERR_SHAPE, "M out of range");
+  if (M == 0) return 0;
+  if (!perm || !offsets || !plan || !h || !y || !ready || !status) return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  if (!aligned16(perm) || !aligned16(h) || !aligned16(y)) return set_error(MOE_B200_ERR_ALIGN, "buffers must be 16-byte aligned");
+  MOE_CUDA_CHECK(cudaMemsetAsync(ready, 0, MOE_B200_READY_INTS * sizeof(int32_t), (cudaStream_t)stream));
+  return launch_experts_mid(perm, offsets, plan, M, d, f, E, h, y, ready, status, (cudaStream_t)stream);
+}
+
 int moe_b200_experts_rows(const void* perm, const int32_t* offsets, const void* plan, int64_t M,
                           int d, int f, int E, int ksplit, void* h, float* part, int32_t* ready,
                           int32_t* status, void* stream) {

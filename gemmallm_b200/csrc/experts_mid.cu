@@ -595,7 +595,7 @@ bool experts_mid_chosen(int64_t M, int d, int f, int E) {
   const int64_t least = E > 32 ? 0 : E > 2 ? (int64_t)96 * E : 1536;
   const int64_t most = E > 2 ? (int64_t)2048 * E : kRowsPathMaxRows;
   if (M < least || M > most) return false;
-  if (M > kRowsPathMaxRows || !rows_supported(M, E)) return f <= 4 * d + 64 || M <= (int64_t)2 * d * E;
+  if (M > kRowsPathMaxRows || !rows_supported(M, E)) return f <= 4 * (int64_t)d + 64 || M <= (int64_t)2 * d * E;
   auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
   auto rounds = [](int64_t tiles, int units) { return fmax(1., (double)tiles / units + .5); };
   const int64_t hit = M < E ? M : E, share = up(M, hit);          // experts with rows, rows of one

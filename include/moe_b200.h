@@ -236,8 +236,14 @@ int moe_b200_experts_rows(const void* perm, const int32_t* offsets, const void* 
                           int32_t* ready, int32_t* status, void* stream);
 int moe_b200_rows_splits(int64_t M, int d, int f, int E);
 
-/* 1 if moe_b200_forward computes both products of a bf16 call of M = N*k rows in one launch on tiles that fit an
- * expert's rows, 0 if it takes one of the other kernels. */
+/* Part 3 in one launch (bf16): h [M,f] and y [M,d] as moe_b200_experts. An expert's rows are cut into equal blocks of at
+ * most 256 on tiles that fit them, the down product's tiles follow the GEGLU product's in the order in which running CTA
+ * pairs claim them, so that its blocks need not all be resident. ready: int32[MOE_B200_READY_INTS], zeroed by this call;
+ * time-out behaviour as for moe_b200_experts_decode_fused. */
+int moe_b200_experts_mid(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d, int f, int E,
+                         void* h, void* y, int32_t* ready, int32_t* status, void* stream);
+/* 1 if moe_b200_forward computes both products of a bf16 call of M = N*k rows so, 0 if by one of the other
+ * kernels. */
 int moe_b200_one_launch(int64_t M, int d, int f, int E);
 
 /* Parts 1+2 for a handful of tokens in ONE single-block launch: same results as

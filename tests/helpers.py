@@ -110,6 +110,18 @@ def experts_rows(perm, offsets, plan: Plan, ksplit: int):
     return h, part, status
 
 
+def experts_mid(perm, offsets, plan: Plan):
+    M, d = perm.shape
+    dev = perm.device
+    h = torch.full((M, plan.f), float("nan"), dtype=perm.dtype, device=dev)
+    y = torch.full((M, d), float("nan"), dtype=perm.dtype, device=dev)
+    status = torch.zeros(16, dtype=torch.int32, device=dev)
+    ready = torch.full((_cabi.READY_INTS,), 7, dtype=torch.int32, device=dev)
+    check(lib.moe_b200_experts_mid(perm.data_ptr(), offsets.data_ptr(), plan.ptr, M, d, plan.f, plan.E, h.data_ptr(),
+                                   y.data_ptr(), ready.data_ptr(), status.data_ptr(), stream(dev)), "experts_mid")
+    return h, y, status, ready
+
+
 def experts_decode_fused(perm, offsets, plan: Plan):
     M, d = perm.shape
     dev = perm.device

@@ -83,6 +83,9 @@ def test_small_and_mid_size_entry_points_check_their_arguments():
     assert lib.moe_b200_experts_rows(a, a, a, 512, 1024, 64, 8, 2, a, a, a, a, None) == -2
     assert lib.moe_b200_experts_rows(a, a, a, 512, 1024, 4096, 8, 4, a, a, None, a, None) == -1
     assert lib.moe_b200_experts_rows(a + 8, a, a, 512, 1024, 4096, 8, 4, a, a, a, a, None) == -3
+    # both products in one launch: any number of rows, no NULL buffer, aligned rows
+    mid = lambda M=512, d=1024, x=a, y=a: lib.moe_b200_experts_mid(x, a, a, M, d, 4096, 8, a, y, a, a, None)
+    assert (mid(M=0), mid(M=-1), mid(d=1020), mid(y=None), mid(x=a + 8), mid(y=a + 4)) == (0, -2, -2, -1, -3, -3)
     # one counter per row block: far too many rows
     assert lib.moe_b200_experts_rows(a, a, a, 1 << 20, 1024, 4096, 8, 4, a, a, a, a, None) == -7
     # sizes the forward uses

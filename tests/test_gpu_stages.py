@@ -737,6 +737,29 @@ def test_experts_rows_matches_prefill_kernels(cuda_device, rows, d, f, ksplit):
         assert (y - y2.float().cpu()).abs().max() <= 1e-2 * y_ref.abs().max()
 
 
+# 18 blocks of an expert, more than the 16 that take turns on a tile of weights, with several tiles of features in both
+# products; blocks of 256 and a row more; one row; few tiles of a long down product; experts without rows
+@pytest.mark.parametrize("rows,d,f", [([4400, 3], 520, 264), ([513, 1, 255, 256, 0, 700, 31, 64], 512, 1024),
+                                      ([1], 72, 200), ([96, 0, 300], 256, 4096), ([0, 2] * 40, 136, 264)])
+def test_experts_mid_matches_prefill_kernels(cuda_device, rows, d, f):
+    """Both products in one launch against the prefill kernels and the oracle, twice in a row; the counters are left zero."""
+    params, x, offsets = expert_inputs(rows, d, f, torch.bfloat16, seed=len(rows) + f)
+    dp = helpers.device_params(params, torch.bfloat16, cuda_device)
+    plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
+    xd, od = x.to(torch.bfloat16).to(cuda_device), offsets.to(cuda_device)
+    h2, y2, _ = helpers.experts(xd, od, plan)
+    h_ref, y_ref = oracle_experts(params, x, offsets)
+    for _ in range(2):
+        h, y, status, ready = helpers.experts_mid(xd, od, plan)
+        torch.cuda.synchronize()
+        assert status.cpu().tolist()[0] == 0 and not ready.any()
+        # where a sum was formed in another order a last bit of bf16 (2^-7) apart; y by that of h and by its own
+        assert (h.float() - h2.float()).abs().max() <= 2 ** -7 * h2.float().abs().max()
+        assert (y.float() - y2.float()).abs().max() <= 2 ** -6 * y2.float().abs().max()
+        assert (h.float().cpu() - h_ref).abs().max() <= 2e-2 * h_ref.abs().max()
+        assert (y.float().cpu() - y_ref).abs().max() <= 2e-2 * y_ref.abs().max()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("N,d,k", [(1, 64, 2), (130, 128, 2), (1000, 512, 4), (33, 72, 1)])
 def test_combine_is_exact(cuda_device, N, d, k, dtype):
