@@ -211,8 +211,8 @@ def test_empty_expert_and_one_hot_expert(cuda_device, dtype):
     assert last["cnt_slot"][1].tolist() == [0, N, 0, 0, 0, 0, 0, 0]
 
 
-# where calls of up to 4096 rows leave the streaming kernel for the prefill products: 192 rows an expert, and the tiles
-# of the down product in one round (74); 1534 and 1536 rows, an uneven routing, and 4096 rows of too many tiles
+# calls of 192 and more rows an expert, up to 4096 in all: widths that are no multiple of a tile, an uneven routing, and 64
+# tiles of the down product in one round
 @pytest.mark.parametrize("N,d,bias0", [(767, 264, 0.0), (768, 264, 0.0), (1000, 72, 2.0), (2048, 1024, 0.0)])
 def test_between_streaming_and_prefill(cuda_device, N, d, bias0):
     E, f, k = 8, 136, 2
@@ -226,7 +226,7 @@ def test_between_streaming_and_prefill(cuda_device, N, d, bias0):
         check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device, residual=res)
 
 
-# the same line with fewer than four experts: 1536 rows
+# one to three experts: 1536 rows, where one or two leave the streaming kernel, and below
 @pytest.mark.parametrize("N,E,k", [(1535, 1, 1), (1536, 1, 1), (767, 3, 2), (768, 3, 2), (300, 2, 1)])
 def test_between_streaming_and_prefill_with_few_experts(cuda_device, N, E, k):
     d, f = 136, 264
@@ -314,13 +314,15 @@ def test_mid_sizes_rows_path(cuda_device, N, d, E, f, k):
         check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device, residual=res)
 
 
-# both products in one launch: either side of its lines (96 and 2048 rows an expert, 1536 rows of one or two experts, 33
-# experts); blocks of 256 tokens and a token more, remainders of 32; more blocks than take turns on a tile of weights (16);
-# experts without rows; widths that are no multiple of a tile; K of one block; one token; 200 experts
+# both products in one launch: either side of its lines (96 and 2048 rows an expert, 1536 and 4096 rows of one or two
+# experts, 33 experts); blocks of 256 tokens and a token more, remainders of 32; more blocks than take turns on a tile of
+# weights (16); experts without rows; widths that are no multiple of a tile; K of one block; one token; 200 experts
 @pytest.mark.parametrize("N,d,E,f,k,bias0", [
     (383, 264, 8, 136, 2, 0.0), (384, 264, 8, 136, 2, 0.0), (512, 64, 2, 264, 1, 9.0), (1537, 136, 2, 264, 1, 0.7),
     (256 * 5 + 1, 72, 4, 200, 1, 40.0), (4400, 128, 8, 72, 1, 40.0), (8193, 64, 4, 64, 1, 0.0), (1, 256, 33, 136, 4, 0.0),
-    (40, 136, 64, 264, 4, 3.0), (700, 64, 200, 72, 8, 0.0), (1100, 1024, 8, 1032, 2, 0.0)])
+    (40, 136, 64, 264, 4, 3.0), (700, 64, 200, 72, 8, 0.0), (1100, 1024, 8, 1032, 2, 0.0),
+    (143, 136, 3, 264, 2, 0.0), (144, 136, 3, 264, 2, 0.0), (8192, 64, 4, 64, 1, 0.0), (4096, 136, 2, 264, 1, 0.0),
+    (4097, 136, 2, 264, 1, 0.0), (384, 256, 8, 4096, 2, 0.0), (2049, 136, 8, 1032, 2, 0.0)])
 def test_both_products_in_one_launch(cuda_device, N, d, E, f, k, bias0):
     params = helpers.rounded_params(synthetic.make_params(d, E, f, seed=N), torch.bfloat16)
     params["w1"] *= 2.0
@@ -330,6 +332,17 @@ def test_both_products_in_one_launch(cuda_device, N, d, E, f, k, bias0):
         x = synthetic.round_to(synthetic.make_input(N, d, seed=N + call), torch.bfloat16)
         res = synthetic.round_to(synthetic.make_input(N, d, seed=N + 7), torch.bfloat16) if call else None
         check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device, residual=res)
+
+
+def test_calls_of_every_size_share_their_counters(cuda_device):
+    """The kernels of small calls and the one that takes both products count in the same words of a workspace, and each finds
+    them zero: sizes in turn on one module, up to one whose call clears them itself."""
+    d, E, f, k = 128, 8, 264, 2
+    params = helpers.rounded_params(synthetic.make_params(d, E, f, seed=3), torch.bfloat16)
+    m = build(params, d, E, f, k, torch.bfloat16, cuda_device)
+    for N in (2300, 64, 512, 1, 300, 512, 40, 2300, 512, 512, 3, 2047, 64):
+        x = synthetic.round_to(synthetic.make_input(N, d, seed=N), torch.bfloat16)
+        check_against_oracle(m, params, x, k, torch.bfloat16, cuda_device)
 
 
 def test_calls_in_one_launch_on_two_streams(cuda_device):
