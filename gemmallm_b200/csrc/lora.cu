@@ -2,11 +2,14 @@
 // model.py:175-179 and 185-189, fine_tuning=True):
 //   x W^T + b + s * (B (A x + a) + b_lora)  =  x (W + s B A)^T + (b + s (B a + b_lora))
 // so the grouped GEMM kernels run unchanged on W' = W + s B A and b' = b + s (B a + b_lora).
-// W [out,in], A [r,in], B [out,r]; fp32 arithmetic, one rounding to the parameter dtype.
+// W [out,in], A [r,in], B [out,r]; sums in fp32, one rounding to the parameter dtype.
 // W is read once and W' written once. bf16: B A by mma.sync, the rest is the stream of W and W' (4 KiB units a warp, the
-// next one under way): [8192,1024] and [1024,4096], rank 16, nothing in L2: 16 + 9 us with the sums on the CUDA cores (packed
-// FMA, which bound it), now 10.7 + 6.9; a LoRA step of the dense feed-forward, 1632 rows, 223 -> 215 us. fp32: the sums on
-// the CUDA cores, a thread owning 8 rows x 8 columns, A and B in shared memory.
+// next one asked for before this one is stored): [8192,1024] and [1024,4096], rank 16, nothing in L2: 16 + 9 us with the
+// sums on the CUDA cores (packed FMA, which bound it), now 10.7 + 6.9; a LoRA step of the dense feed-forward, 1632 rows, 223
+// -> 215 us. The tensor core cuts its fp32 sums off where FMA rounds them, but adds 16 products at once and takes B
+// unscaled: fewer W' are not the nearest bf16 to their 64-bit value than with FMA ([8192,1024], rank 16, N(0, 0.02^2): 11 of
+// 8388608 against 42; rank 64 37 against 147; rank 33, A and B five times as large, [2816,2048]: 101 of 5767168 against 513).
+// fp32: the sums on the CUDA cores, a thread owning 8 rows x 8 columns, A and B in shared memory.
 #include "common.cuh"
 
 namespace moe {
@@ -43,56 +46,52 @@ __device__ __forceinline__ float hi_float(uint64_t v) { return __uint_as_float((
 
 // fp32. One block per 64 x 256 tile of W: the tile's slice of A [rank][256] and the scaled rows of
 // B [rank][64] wait in shared memory, every thread owns 8 rows x 8 columns, and W streams through once.
-template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 2 : 1)
-lora_merge_kernel(const T* W, const T* b, const T* A, const T* a_bias, const T* B, const T* b_lora,
-                  float scale, int out_f, int in_f, int rank, T* out_W, T* out_b) {
-  constexpr int kRaw = sizeof(T) / 2;      // 16-byte pieces of eight elements
+__global__ void __launch_bounds__(256, 1)
+lora_merge_f32_kernel(const float* W, const float* b, const float* A, const float* a_bias, const float* B, const float* b_lora,
+                      float scale, int out_f, int in_f, int rank, float* out_W, float* out_b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* s_a = reinterpret_cast<T*>(smem_raw);                                                  // [rank][256]
-  float* s_b = reinterpret_cast<float*>(smem_raw + (size_t)rank * kTileCols * sizeof(T));   // [rank][kBPitch]
+  float* s_a = reinterpret_cast<float*>(smem_raw);       // [rank][256]
+  float* s_b = s_a + (size_t)rank * kTileCols;           // [rank][kBPitch]
   const int c0 = blockIdx.x * kTileCols, r0 = blockIdx.y * kTileRows;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = c0 + tx * 8;
   pdl_wait();
   // W first: its loads are in flight while the tables are filled
-  uint4 raw[8][kRaw];
+  uint4 raw[8][2];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int row = r0 + ty * 8 + i;
     if (row < out_f && c < in_f) {
       raw8(W + (size_t)row * in_f + c, raw[i]);
     } else {
-#pragma unroll
-      for (int q = 0; q < kRaw; ++q) raw[i][q] = make_uint4(0, 0, 0, 0);
+      raw[i][0] = raw[i][1] = make_uint4(0, 0, 0, 0);
     }
   }
   const int rows = min(kTileRows, out_f - r0);
 #pragma unroll 4
   for (int i = threadIdx.x; i < kTileRows * rank; i += 256) {      // neighbours in memory are ranks of a row
     const int rr = i / rank, r = i - rr * rank;
-    s_b[r * kBPitch + rr] = rr < rows ? scale * to_f32(B[(size_t)r0 * rank + i]) : 0.f;
+    s_b[r * kBPitch + rr] = rr < rows ? scale * B[(size_t)r0 * rank + i] : 0.f;
   }
   for (int i = threadIdx.x; i < rank * (kTileCols / 8); i += 256) {
     const int r = i / (kTileCols / 8), pc = i - r * (kTileCols / 8);
-    uint4 v[kRaw];
+    uint4 v[2];
     if (c0 + pc * 8 < in_f) {
       raw8(A + (size_t)r * in_f + c0 + pc * 8, v);
     } else {
-#pragma unroll
-      for (int q = 0; q < kRaw; ++q) v[q] = make_uint4(0, 0, 0, 0);
+      v[0] = v[1] = make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
-    for (int q = 0; q < kRaw; ++q) reinterpret_cast<uint4*>(s_a + (size_t)r * kTileCols + pc * 8)[q] = v[q];
+    for (int q = 0; q < 2; ++q) reinterpret_cast<uint4*>(s_a + (size_t)r * kTileCols + pc * 8)[q] = v[q];
   }
   __syncthreads();
   uint64_t acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i) unpack8(raw[i], acc[i]);
   for (int r = 0; r < rank; ++r) {
-    uint4 v[kRaw];
+    uint4 v[2];
 #pragma unroll
-    for (int q = 0; q < kRaw; ++q) v[q] = reinterpret_cast<const uint4*>(s_a + (size_t)r * kTileCols + tx * 8)[q];
+    for (int q = 0; q < 2; ++q) v[q] = reinterpret_cast<const uint4*>(s_a + (size_t)r * kTileCols + tx * 8)[q];
     uint64_t a[4];
     unpack8(v, a);
     float br[8];
@@ -120,17 +119,16 @@ lora_merge_kernel(const T* W, const T* b, const T* A, const T* a_bias, const T* 
   if (blockIdx.x == 0 && (int)threadIdx.x < rows) {
     const int row = r0 + threadIdx.x;
     float sum = 0.f;
-    for (int r = 0; r < rank; ++r) sum = fmaf(s_b[r * kBPitch + threadIdx.x], to_f32(a_bias[r]), sum);
-    T v;
-    from_f32(v, to_f32(b[row]) + sum + scale * to_f32(b_lora[row]));
-    out_b[row] = v;
+    for (int r = 0; r < rank; ++r) sum = fmaf(s_b[r * kBPitch + threadIdx.x], a_bias[r], sum);
+    out_b[row] = b[row] + sum + scale * b_lora[row];
   }
 }
 
-// bf16: B A on the tensor cores (products of bf16 are exact in fp32, the sums are fp32), so that one pass over W is left.
+// bf16: B A on the tensor cores (products of bf16 are exact in fp32, the sums fp32, cut off), so that one pass over W is left.
 // A warp takes units of 16 rows x 128 columns of its block's 128 columns; the slice of A [rank][128] waits in shared
-// memory with its columns in the order that gives a thread eight neighbouring ones: tile j, place n of a group of 32 columns is
-// column 8 (n / 2) + 2 j + n % 2. The next unit of W is requested before the products of this one.
+// memory with its columns in the order that gives a thread eight neighbouring ones: tile j, place n of a group of 32 columns
+// is column 8 (n / 2) + 2 j + n % 2. The next unit of W is requested when this one's products have been added, before the
+// result is stored.
 constexpr int kMergeCols = 128;
 constexpr int kMergePitch = kMergeCols + 8;      // elements: rows 16 bytes apart modulo the banks
 constexpr int kMergeWarps = 8;
@@ -250,21 +248,19 @@ int launch_merge_bf16(const void* W, const void* b, const void* A, const void* a
   return 0;
 }
 
-template <typename T>
-int launch_merge(const void* W, const void* b, const void* A, const void* a_bias, const void* B,
-                 const void* b_lora, float scale, int out_f, int in_f, int rank, void* out_W,
-                 void* out_b, cudaStream_t s) {
-  const size_t smem = (size_t)rank * (kTileCols * sizeof(T) + kBPitch * sizeof(float));
+int launch_merge_f32(const void* W, const void* b, const void* A, const void* a_bias, const void* B, const void* b_lora,
+                     float scale, int out_f, int in_f, int rank, void* out_W, void* out_b, cudaStream_t s) {
+  typedef const float* In;
+  const size_t smem = (size_t)rank * (kTileCols + kBPitch) * sizeof(float);
   static PerDeviceOnce once;
   if (smem > 48 * 1024) {
-    int rc = ensure_dynamic_smem(once, lora_merge_kernel<T>, 96 * 1024);
+    int rc = ensure_dynamic_smem(once, lora_merge_f32_kernel, 96 * 1024);
     if (rc) return rc;
   }
-  MOE_CUDA_CHECK(launch_pdl(lora_merge_kernel<T>, dim3((in_f + kTileCols - 1) / kTileCols, (out_f + kTileRows - 1) / kTileRows),
-                            dim3(256), smem, s, static_cast<const T*>(W), static_cast<const T*>(b),
-                            static_cast<const T*>(A), static_cast<const T*>(a_bias), static_cast<const T*>(B),
-                            static_cast<const T*>(b_lora), scale, out_f, in_f, rank, static_cast<T*>(out_W),
-                            static_cast<T*>(out_b)));
+  MOE_CUDA_CHECK(launch_pdl(lora_merge_f32_kernel, dim3((in_f + kTileCols - 1) / kTileCols, (out_f + kTileRows - 1) / kTileRows),
+                            dim3(256), smem, s, static_cast<In>(W), static_cast<In>(b), static_cast<In>(A),
+                            static_cast<In>(a_bias), static_cast<In>(B), static_cast<In>(b_lora), scale, out_f, in_f, rank,
+                            static_cast<float*>(out_W), static_cast<float*>(out_b)));
   return 0;
 }
 
@@ -288,6 +284,5 @@ extern "C" int moe_b200_lora_merge(const void* W, const void* b, const void* A, 
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == MOE_B200_BF16)
     return launch_merge_bf16(W, b, A, a_bias, B, b_lora, scale, out_features, in_features, rank, out_W, out_b, s);
-  return launch_merge<float>(W, b, A, a_bias, B, b_lora, scale, out_features, in_features, rank, out_W,
-                             out_b, s);
+  return launch_merge_f32(W, b, A, a_bias, B, b_lora, scale, out_features, in_features, rank, out_W, out_b, s);
 }
