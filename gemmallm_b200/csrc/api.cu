@@ -483,7 +483,7 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   // a handful of tokens, a row or two per expert: routing, both products and the weighted sum
   // in one cooperative launch
   const bool tiny = small_n && !spec && decode_tiny_supported(N, d, f, E, k, dtype);
-  // between the decode and the prefill sizes: the streaming kernel on the sorted rows
+  // between the decode and the prefill sizes: the streaming kernel on the sorted rows, or
   const bool rows_path = dtype == MOE_B200_BF16 && !small_n && N * k <= kRowsPathMaxRows &&
                          rows_supported(N * k, E);
   // both products in one launch on tiles that fit an expert's rows, where that is the faster (experts_mid.cu)

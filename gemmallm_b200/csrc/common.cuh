@@ -20,7 +20,9 @@ constexpr int kDispatchChunk = 64;
 
 // The small-N (weight-streaming) expert path is taken up to this many sorted rows (N*k).
 constexpr int64_t kDecodeMaxRows = 256;
-constexpr int64_t kRowsPathMaxRows = 4096;   // above: the prefill kernels (256-row tiles)
+// ... and the streaming kernel on sorted rows up to this many, where both products in one launch (experts_mid.cu) are not the
+// faster; above: those, or the prefill kernels (256-row tiles).
+constexpr int64_t kRowsPathMaxRows = 4096;
 
 int set_error(int code, const char* msg);
 int cuda_error(cudaError_t e, const char* where);
@@ -280,8 +282,8 @@ struct EpScatter {
 // `scale` = 1 / (1 - p). The derivatives of h after the gate and up values, mask and scale
 // included, go to gu [M, 2f] (columns [0,f) gate, [f,2f) up); with keep_pre (LoRA steps, whose
 // rounding is that of the pre-activations) those go there, with their biases, and the mask to
-// `mask`. The backward pass replaces gu by the gradients of gate and up; col_part receives the column sums of that gradient, one row per 128-row half
-// of a 256-row tile (tiles counted over the experts in order).
+// `mask`. The backward pass replaces gu by the gradients of gate and up; col_part receives the column sums of that gradient,
+// one row per 128-row half of a 256-row tile (tiles counted over the experts in order).
 struct TrainArgs {
   __nv_bfloat16* gu;
   uint8_t* mask;            // keep_pre: [M, f / 8] one bit per element of h, set = kept

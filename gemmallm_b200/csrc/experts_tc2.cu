@@ -31,10 +31,11 @@
 // arrival across the pair for every block halved the rate, 680 instead of 1280 TFLOP/s.)
 //
 // SPLIT > 1 (kPlain, kDx): products of few tiles and a long contraction. A tile of 256 x 256 takes 0.31 us per
-// 64 of K however few of them run (shared memory's rate: 580 clk), so 28 tiles of K = 4096 left 46 pairs idle for 20 us. SPLIT pairs in one cluster take a range of K each, put their fp32
-// accumulators into shared memory (the stages are free by then: a cluster has one tile) and each adds up and
-// stores 256 / SPLIT columns, in the order of the ranges. (128-column tiles instead gained nothing: a product of
-// half the columns takes the same time.)
+// 64 of K however few of them run (shared memory's rate: 580 clk), so 28 tiles of K = 4096 left 46 pairs idle for 20 us.
+// SPLIT pairs in one cluster take a range of K each, put their fp32 accumulators into shared memory (the stages are free by
+// then: a cluster has one tile) and each adds up and stores 256 / SPLIT columns, in the order of the ranges. (128-column
+// tiles instead gained nothing when the load loop still set the pace, 640 clk a step whatever the columns; they have not
+// been measured since it does not.)
 #include <cuda.h>
 #include "common.cuh"
 #include "tc_ptx.cuh"

@@ -333,7 +333,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
   if constexpr (SPLIT) {
     const int nb = nblk, b = blk;
     float* xps = reinterpret_cast<float*>(xch + nb * k * E);    // [nb][E] probability sums
-    static_assert(32 * 16 * 8 * NT >= 128 * 8 * NT, "128 blocks' sums of 8 NT experts");
+    static_assert((F32 ? 8 : 32) * 16 * 8 * NT >= 128 * 8 * NT, "128 blocks' sums of 8 NT experts in [nslices][16][8 NT]");
     if (tid < k * E) xch[b * k * E + tid] = s_cnt[(tid / E) * kMaxE + tid % E];
     if (tid < E) {
       float ps = 0.f;
