@@ -37,7 +37,7 @@ sys.path.insert(0, str(ROOT))
 # down pass) from the ncu captures summarised under profiles/: a static figure, not measured by
 # this run
 NCU_TRAFFIC = {
-    "c1_uniform": (429.7e6 + 405.7e6, "profiles/grouped_gemm_tc2_c1_uniform.md (static, ncu capture)"),
+    "c1_uniform": (437.4e6 + 412.2e6, "profiles/grouped_gemm_tc2_c1_uniform.md (static, ncu capture)"),
     "c2_t64": (204.8e6 + 3.8e6, "profiles/decode_spec_kernel_c2_t64.md (static, ncu capture)"),
 }
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
@@ -1260,10 +1260,10 @@ def run_train(args, wl):
         "e2e": {"value": N / (e2e_ms * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": N * d * es,
                 "d2h_bytes_per_step": N * d * es + 4, "ms_per_step": e2e_ms,
                 "mode": "input copied in, input gradient and loss copied out, every step, one stream"},
-        "gpu_launches": 26 * args.steps,   # the library's kernels per step (launch list in profiles/)
+        "gpu_launches": 17 * args.steps,   # the library's kernels per step (launch list in profiles/)
         "clocks": clocks.summary(),
         "roofline": {"kernel": "whole step: six grouped_gemm_tc2_kernel launches (two forward, four backward) "
-                               "plus router, dispatch, combine, their backward kernels and the transposes",
+                               "plus router, dispatch, combine, their backward kernels and column sums",
                      "bound": "tensor", "achieved": flops / (ms_step * 1e-3) / 1e12, "peak": peak,
                      "unit": "TFLOP/s", "frac": flops / (ms_step * 1e-3) / 1e12 / peak, "traffic": None,
                      "peak_source": f"{peak_kind} bf16 sustained (the step is a seconds-long loop of GEMMs)",
