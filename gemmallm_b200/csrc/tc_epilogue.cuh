@@ -197,7 +197,9 @@ struct BoxOut {
 // experts: that product 385 -> 302 us, now bound by the column sums' shuffles and its boxes' way through shared memory;
 // this one 438 -> 443; whole training step 2472 -> 2413. Gradients against 64 bits, 2-norm, 13 sizes of 99 to 16384 tokens with
 // dropout 0.1: of x 3.75e-3 to 3.81e-3 -> 3.65e-3 to 3.73e-3, w1 3.44e-3 -> 3.32e-3, b1 3.00e-3 -> 2.87e-3, the router's and
-// the down Linear's as before.)
+// the down Linear's as before. A dropped element's derivatives are zeros that dh is multiplied by: with dh infinite or NaN
+// its gradients are NaN, as autograd's through a product with the mask, where they were 0; with g beyond 1e19 they are 0,
+// where they were NaN.)
 // PRE, LoRA steps: g, u and the mask are kept all the same, whose rounding such a step repeats (lora_bwd.cu says why).
 // start() fetches the biases into this warp's 64 floats of shared memory before the products are awaited.
 template <bool PRE>
