@@ -575,8 +575,8 @@ experts_mid_kernel(const __grid_constant__ CUtensorMap tmap_x64, const __grid_co
 
 // Whether a call of M rows is better off here than with the kernels it would take else.
 // More than 32 experts, up to 256 rows: the matrix-vector kernel goes row by row (64 experts, d 2048, f 1408, four slots, us:
-// 4 rows 99 / here 58, 64 rows 1163 / 147). Up to 32 experts the streaming kernel is as fast below 96 rows an expert (600 rows of
-// 8 experts 60 / 62) and, with one or two experts, below 1536 rows.
+// 4 rows 99 / here 58, 64 rows 1163 / 147). Up to 32 experts the streaming kernel is as fast below 96 rows an expert (600
+// rows of 8 experts 60 / 62) and, with one or two experts, below 1536 rows.
 // Up to 4096 rows the streaming kernel remains (experts_decode_spec.cu, sorted rows), which cuts the down product's K into
 // ranges for all SMs. Here that product takes whole rounds of all K on pairs of SMs, and where d is small and f large its
 // few tiles are the longest part of the call (d 256, f 8192, 8 experts, 768 rows: 51.8 / here 68.3 us, 3 experts 45.4 /
@@ -585,7 +585,9 @@ experts_mid_kernel(const __grid_constant__ CUtensorMap tmap_x64, const __grid_co
 // tokens, and 0.75 a round of GEGLU epilogues; there 0.30 a step of GEGLU with 128 rows, 0.27 one of a range of down's K, and
 // what the fp32 sums of the ranges cost. Fitted to whole calls of both kernels: 1 to 200 experts, d 64 to 4096, f 264 to
 // 16384, 2012 sizes. The kernel that is chosen takes 0.4 % longer than the faster one on average (always here: 4 %), and is
-// the slower one by more than 3 % at 118 sizes (by 4.5 % in the middle of them, by 15 % at most).
+// the slower one by more than 3 % at 106 sizes (by 4.4 % in the middle of them, by 15 % at most). One or two experts with f
+// beyond 4 d are told apart by d alone, where the estimate is least good (3000 rows of two: d 512, f 8192 105 / here 118, d
+// 1024, f 8192 174 / 148).
 // Beyond, the 256-row tiles remain (experts_tc2.cu), to which remainders no longer count at 2048 rows an expert (8 experts,
 // d 1024, f 4096 there: 349 / here 319). With K of the down product more than four times that of gate_and_up a tile's
 // epilogue is the bound, and theirs is the faster: up to 2 d rows an expert this one is still ahead (d 256, f 2048, 24
@@ -595,6 +597,7 @@ bool experts_mid_chosen(int64_t M, int d, int f, int E) {
   const int64_t least = E > 32 ? 0 : E > 2 ? (int64_t)96 * E : 1536;
   const int64_t most = E > 2 ? (int64_t)2048 * E : kRowsPathMaxRows;
   if (M < least || M > most) return false;
+  if (E <= 2 && f > 4 * (int64_t)d + 64) return d >= 1024;
   if (M > kRowsPathMaxRows || !rows_supported(M, E)) return f <= 4 * (int64_t)d + 64 || M <= (int64_t)2 * d * E;
   auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
   auto rounds = [](int64_t tiles, int units) { return fmax(1., (double)tiles / units + .5); };

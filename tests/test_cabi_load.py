@@ -134,6 +134,9 @@ def test_which_calls_compute_both_products_in_one_launch():
     # down products of 128 steps of K in 3 to 16 tiles: 68 us against 45 to 52 of the streaming kernel, and K in ranges there
     assert [one(M, 256, 8192, E) for M, E in ((288, 3), (768, 3), (768, 8), (1536, 8), (1800, 1), (2048, 2), (896, 8))] == [0] * 7
     assert one(768, 512, 8192, 4) == 0 and one(1280, 1024, 8192, 8) == 1
+    # one or two experts with such a product: by d
+    assert [one(M, d, 8 * d, E) for d in (512, 1024) for M, E in ((1536, 2), (3000, 1), (4096, 2))] == [0] * 3 + [1] * 3
+    assert one(3000, 512, 8192, 2) == 0
     # beyond 4096 rows: the epilogue's share where K of gate_and_up is short
     assert one(16384, 256, 8192, 8) == 0 and one(7680, 256, 2048, 24) == 1 and one(16384, 512, 2048, 8) == 1
     # more than 32 experts: up to 256 rows whatever the shape, and where row blocks outnumber the streaming kernel's counters
