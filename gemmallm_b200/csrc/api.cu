@@ -34,6 +34,8 @@ static int check_shape(int64_t N, int d, int f, int E, int k, int dtype) {
   return 0;
 }
 
+// (16-byte aligned: f is a multiple of 8)
+static size_t h_planes_bytes(size_t M, int f) { return M * f * 6; }
 static size_t align_up(size_t v) { return (v + 1023) & ~(size_t)1023; }
 
 static void layout(int64_t N, int d, int f, int E, int k, int dtype, size_t* off, size_t* total) {
@@ -57,6 +59,8 @@ static void layout(int64_t N, int d, int f, int E, int k, int dtype, size_t* off
   sizes[MOE_B200_WS_ROW_OF] = M * sizeof(int32_t);
   sizes[MOE_B200_WS_PERM] = M * d * es;
   sizes[MOE_B200_WS_H] = M * f * es;
+  // fp32 calls of the single-launch front: three bf16 planes of h, then of the sorted rows
+  if (dtype == MOE_B200_F32 && front_f32_supported(N, E, k)) sizes[MOE_B200_WS_H] = h_planes_bytes(M, f) + M * d * 6;
   if (dtype == MOE_B200_BF16 && decode_spec_supported(N, E, k)) {
     // the routing-independent small-N kernel keeps one slab of h per expert
     const size_t slabs = (size_t)E * decode_spec_rows(N) * f * es;
@@ -67,6 +71,8 @@ static void layout(int64_t N, int d, int f, int E, int k, int dtype, size_t* off
       (dtype == MOE_B200_BF16 && M <= kDecodeMaxRows) ? (size_t)decode_splits(f) * M * d * sizeof(float) : 0;
   if (dtype == MOE_B200_BF16 && (int64_t)M > kDecodeMaxRows && (int64_t)M <= kRowsPathMaxRows)
     sizes[MOE_B200_WS_PART] = (size_t)rows_splits((int64_t)M, d, f, E) * M * d * sizeof(float);
+  if (dtype == MOE_B200_F32 && front_f32_supported(N, E, k) && f32_down_splits((int64_t)M, d, f, E) > 1)
+    sizes[MOE_B200_WS_PART] = (size_t)f32_down_splits((int64_t)M, d, f, E) * M * d * sizeof(float);
   sizes[MOE_B200_WS_NORM_W] = (size_t)E * d * es;
   sizes[MOE_B200_WS_NORM_C] = (size_t)2 * E * sizeof(float);
   sizes[MOE_B200_WS_STATS] = (size_t)N * 2 * sizeof(float);
@@ -524,10 +530,22 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   if (front) {
     // router and dispatch of up to a few hundred tokens in one launch
     // (beyond 128 tokens its blocks share the work and meet at a counter behind the status words)
+    void* planes = front32 ? static_cast<char*>(h) + h_planes_bytes((size_t)N * k, f) : nullptr;
     rc = launch_front_small(x, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm,
                             psum, aux, s, scratch,
-                            status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, dtype);
+                            status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, dtype, planes);
     if (rc) return rc;
+    if (front32) {
+      const int parts = f32_down_splits(N * k, d, f, E);
+      rc = launch_experts_f32_planes(perm, planes, offsets, plan, N * k, d, f, E, h, parts > 1 ? static_cast<void*>(part) : y,
+                                     status, s);
+      if (rc) return rc;
+      if (parts > 1 && (!aligned16(out) || !aligned16(residual)))
+        return set_error(MOE_B200_ERR_ALIGN, "buffers must be 16-byte aligned");
+      if (parts > 1)
+        return launch_combine_parts_f32(part, parts, N * k, row_of, idx, w, plan, E, residual, N, d, k, out, s);
+      return moe_b200_combine(y, row_of, w, residual, N, d, k, dtype, out, stream);
+    }
   } else {
     if (fold) {
       void* wn = ws + off[MOE_B200_WS_NORM_W];

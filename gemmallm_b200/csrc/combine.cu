@@ -160,7 +160,57 @@ combine_decode_kernel(const float* __restrict__ part, int ksplit, int64_t part_s
   store8(out + t * d + c, acc);
 }
 
+// fp32: the down product as `splits` partial sums part[s][M][d] without bias, added in order, with the expert's down.bias,
+// then weighted as above. A thread: four elements of a token. 512 tokens, d 512, four parts, two slots: 8 MB that lie in L2.
+__global__ void __launch_bounds__(128)
+combine_parts_f32_kernel(const float* __restrict__ part, int splits, int64_t part_stride, const int32_t* __restrict__ row_of,
+                         const int32_t* __restrict__ idx, const float* __restrict__ w, const void* const* __restrict__ b2,
+                         const float* __restrict__ residual, int64_t N, int d, int k, float* __restrict__ out) {
+  const int pieces = d >> 2;
+  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
+  if (item >= N * pieces) return;
+  const int64_t t = item / pieces;
+  const int c = (int)(item - t * pieces) << 2;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int j = 0; j < k; ++j) {
+    const int row = __ldcg(&row_of[t * k + j]);
+    if (row < 0) continue;
+    const float wj = __ldcg(&w[t * k + j]);
+    const float* b = static_cast<const float*>(b2[__ldcg(&idx[t * k + j])]) + c;    // (of any alignment)
+    const float bias[4] = {__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3)};
+    const float* p = part + (int64_t)row * d + c;
+    float4 u[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < splits) u[q] = __ldcg(reinterpret_cast<const float4*>(p + q * part_stride));
+    float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < splits) { y[0] += u[q].x; y[1] += u[q].y; y[2] += u[q].z; y[3] += u[q].w; }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(wj, y[i] + bias[i]));
+  }
+  if (residual != nullptr) {
+    const float4 r = *reinterpret_cast<const float4*>(residual + t * d + c);
+    acc[0] = __fadd_rn(acc[0], r.x); acc[1] = __fadd_rn(acc[1], r.y);
+    acc[2] = __fadd_rn(acc[2], r.z); acc[3] = __fadd_rn(acc[3], r.w);
+  }
+  *reinterpret_cast<float4*>(out + t * d + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
 }  // namespace
+
+int launch_combine_parts_f32(const float* part, int splits, int64_t M, const int32_t* row_of, const int32_t* idx,
+                             const float* w, const void* plan, int E, const void* residual, int64_t N, int d, int k,
+                             void* out, cudaStream_t s) {
+  if (N == 0) return 0;
+  const int64_t blocks = (N * (d >> 2) + 127) / 128;
+  MOE_CUDA_CHECK(launch_pdl(combine_parts_f32_kernel, dim3((unsigned)blocks), dim3(128), 0, s, part, splits, M * (int64_t)d,
+                            row_of, idx, w, plan_view(plan, E).b2, static_cast<const float*>(residual), N, d, k,
+                            static_cast<float*>(out)));
+  return 0;
+}
 
 int launch_combine_decode(const float* part, int ksplit, int64_t M, const int32_t* row_of,
                           const int32_t* idx, const float* w, const void* plan, int E,

@@ -73,6 +73,23 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Two values cut off to bf16, NaN to NaN (whose upper half alone may be an infinity's).
+__device__ __forceinline__ uint32_t cut_bf16x2(float lo, float hi) {
+  uint32_t v;
+  asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+  return v;
+}
+// Two values into their three bf16 parts, exactly (where they are finite): see experts_f32.cu.
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  p0 = cut_bf16x2(x0, x1);
+  float r0 = x0 - __uint_as_float(__float_as_uint(x0) & 0xffff0000u);
+  float r1 = x1 - __uint_as_float(__float_as_uint(x1) & 0xffff0000u);
+  p1 = pack_bf16x2(r0, r1);
+  r0 -= bf16_lo(p1);
+  r1 -= bf16_hi(p1);
+  p2 = pack_bf16x2(r0, r1);
+}
+
 // Load 8 consecutive elements starting at p (16-byte aligned for bf16,
 // 32-byte aligned pairs of float4 for fp32) into fp32 registers.
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
@@ -311,6 +328,9 @@ int launch_layernorm_rows(const void* x, const void* gamma, const void* beta, fl
                           int d, int dtype, void* out, float* stats, cudaStream_t s);
 int launch_experts_f32(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d,
                        int f, int E, void* h, void* y, int32_t* status, cudaStream_t s);
+int f32_down_splits(int64_t M, int d, int f, int E);
+int launch_experts_f32_planes(const void* perm, const void* perm_planes, const int32_t* offsets, const void* plan, int64_t M,
+                              int d, int f, int E, void* h_planes, void* y, int32_t* status, cudaStream_t s);
 int launch_combine(const void* y, const int32_t* row_of, const float* w, const void* residual,
                    int64_t N, int d, int k, int dtype, void* out, cudaStream_t s,
                    const EpSync* ep_wait = nullptr, int32_t* status = nullptr);
@@ -350,12 +370,15 @@ int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
                        cudaStream_t s, int* xch = nullptr, int* counter = nullptr,
-                       int32_t* status = nullptr, int dtype = MOE_B200_BF16);
-// fp32, with the exchange buffer; on this device only if its blocks are all resident at once
+                       int32_t* status = nullptr, int dtype = MOE_B200_BF16, void* planes = nullptr);
+// fp32, with the exchange buffer and room for the rows' bf16 planes [3][N k][d]; on this device only if its blocks are all
+// resident at once
 bool front_f32_supported(int64_t N, int E, int k);
 int front_f32_resident(int64_t N, bool* yes);
 int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
                    uint32_t box_cols = 64);
+// [3][rows, cols] bf16, boxes of 32 columns x box_rows x 3
+int encode_tmap_planes(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 int encode_tmap_2d_f32(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 int sm_count(int* sms);
 int decode_splits(int f);
@@ -373,6 +396,10 @@ int launch_experts_tc_rows(const void* perm, const int32_t* offsets, const void*
 int launch_experts_tc_decode_fused(const void* perm, const int32_t* offsets, const void* plan,
                                    int64_t M, int d, int f, int E, void* h, float* part, int* ready,
                                    int32_t* status, cudaStream_t s, int spec = -1);
+// fp32: out from partial sums of fp32 calls (f32_down_splits)
+int launch_combine_parts_f32(const float* part, int splits, int64_t M, const int32_t* row_of, const int32_t* idx,
+                             const float* w, const void* plan, int E, const void* residual, int64_t N, int d, int k,
+                             void* out, cudaStream_t s);
 int launch_combine_decode(const float* part, int ksplit, int64_t M, const int32_t* row_of,
                           const int32_t* idx, const float* w, const void* plan, int E,
                           const void* residual, int64_t N, int d, int k, void* out, cudaStream_t s);

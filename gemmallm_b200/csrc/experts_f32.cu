@@ -23,20 +23,24 @@
 // tokens of one expert the B operand, N = their number rounded up to 16: the pipe's time is in proportion to N from 64
 // on (64 clk per K = 16 at N 128, 46 at N 16 to 64), so that an expert's last rows cost what they are. K in
 // steps of 32.
-//   warp 0       loads fp32 boxes by TMA, three stages ahead
-//   warp 1       issues the products (A from tensor memory, B from shared memory)
-//   warps 4-19   split, eight on even and eight on odd steps: their row of A into tensor memory (tcgen05.st), tokens of
-//                B into three bf16 tiles
-//   warps 20-27  add up the products, then bias, GELU and the store
-// A cluster of up to eight CTAs shares a tile and splits K where tiles are few; every CTA sends each other one its
-// sums of that one's tokens through distributed shared memory, and they are added in rank order.
+//   warp 0       loads boxes by TMA, three or four stages ahead
+//   warp 1       one lane issues the products (A from tensor memory, B from shared memory), two steps at a time
+//   then split warps, half of them on even and half on odd steps: their row of A into tensor memory (tcgen05.st)
+//   and epilogue warps, which add up the products, then bias, GELU and the store
+// In whole calls (PLANES) the tokens come as three bf16 planes, split once by the kernel in front (front_small.cuh) and by
+// the GEGLU pass's epilogue: one box a step brings all three, and 8 split and 16 epilogue warps are at work. Where h is the
+// caller's fp32 tensor, or the rows come from the dispatch kernel, 16 split warps also turn the tokens' boxes into three bf16
+// tiles, and 8 warps are left for the epilogue.
+// Where tiles are few K is split: the GEGLU pass over a cluster of up to eight CTAs, every one of which sends each other one
+// its sums of that one's tokens through distributed shared memory, to be added in rank order; the down pass on planes over
+// blocks that leave partial sums to the combine kernel (the exchange took 6 of that pass's 26 us).
 //
-// What bounds it: shared-memory bandwidth (per step of 32 at N 128: 32 KiB in by TMA, 32 read and 24 written by the
-// split, 48 read by the products, about 1060 clk of 128 bytes) and the issue slots of the split (600 clk) against 768 clk
-// of products; a step takes 1400 to 1600. 1024 rows of 8 experts, d 512, f 2048, nothing in L2: gate_and_up 160 -> 46 us,
-// both products 250 -> 77 us (packed FMA on the CUDA cores before; 45 and 75 without the look for infinities). Error of h
-// and y against 64 bits, in the 2-norm, at 2 to 4096 rows: 1.8e-7 and 0.9e-7 to 1.4e-7 (before: 2.3e-7 to 4.2e-7 and
-// 1.6e-7).
+// What bounds it (clk of 1.9 GHz, 512 tokens, d 512, f 2048, 8 experts, top-2): a step takes 1000 to 1100 for 768 of products
+// at N 128; a pass's first step is done 7000 to 9000 after the routing is known, most of it code that runs for the first time;
+// the epilogue 5000 to 8000, stores and again code that is cold. The call 95.4 -> 81.8 us: a step 1500 -> 1100 (tokens split
+// once, 1024 tokens 145.9 -> 134; the issuing lane looking at half as many barriers), epilogue warps and partial sums the
+// rest; 1 / 16 / 128 / 2048 tokens 38.1 -> 35.2, 61.5 -> 57.2, 71.3 -> 65.6, 243 -> 228. Error of h and y against 64 bits, in
+// the 2-norm, at 2 to 4096 rows: 1.8e-7 and 0.9e-7 to 1.4e-7.
 #include <cuda.h>
 #include <cfloat>
 #include "common.cuh"
@@ -51,34 +55,53 @@ using namespace tc;
 constexpr int kRowsA = 128;      // weight rows per tile = accumulator lanes
 constexpr int kMaxN = 160;       // tokens per tile; 2 * 160 + 3 * 48 columns of tensor memory
 constexpr int BK = 32;
-constexpr int kRawStages = 3, kConvStages = 3;
 constexpr int kRawA = kRowsA * BK * 4;            // 16 KiB, rows of 128 bytes
-constexpr int kRawBytes = kRawA + kMaxN * BK * 4;
+constexpr int kRawB = kMaxN * BK * 4;
 constexpr int kPlane = kMaxN * BK * 2;            // one bf16 tile of the tokens, rows of 64 bytes
-constexpr int kSplitWarps = 8, kEpiWarps = 8;       // split warps of a step
-constexpr int kEpiFirst = 4 + 2 * kSplitWarps;
-constexpr int kThreads = 32 * (kEpiFirst + kEpiWarps);
-// Registers: 896 threads start with 72 each, 504 for the seven warps of a thread index
-constexpr int kRegsLoad = 40, kRegsSplit = 48, kRegsEpi = 136;
-static_assert(kRegsLoad + 4 * kRegsSplit + 2 * kRegsEpi <= 7 * 72, "a share above the launch's registers would wait for good");
+constexpr int kThreads = 896;
+constexpr int kMaxStages = 4;
+// PLANES: the tokens come as three bf16 planes, and only the weights are split here: half as many warps do, and the others
+// are epilogue warps.
+template <bool PLANES>
+struct Cfg {
+  static constexpr int kStages = PLANES ? 4 : 3;
+  static constexpr int kRawBytes = kRawA + (PLANES ? 0 : kRawB);
+  static constexpr int kSplitWarps = PLANES ? 4 : 8;        // of a step; as many on even as on odd steps
+  static constexpr int kEpiFirst = 4 + 2 * kSplitWarps;
+  static constexpr int kEpiWarps = kThreads / 32 - kEpiFirst;
+  static constexpr int kParts = kEpiWarps / 4;              // warps that share the tile's tokens, eight at a time in turn
+  static constexpr int kGroups = (kMaxN / 8 + kParts - 1) / kParts;   // groups of eight tokens per epilogue warp
+  // Registers: 896 threads start with 72 each, 504 for the seven warps of a thread index
+  static constexpr int kRegsLoad = PLANES ? 56 : 40, kRegsSplit = 48, kRegsEpi = PLANES ? 88 : 136;
+  static_assert(kRegsLoad + kSplitWarps / 2 * kRegsSplit + kParts * kRegsEpi <= 7 * 72,
+                "a share above the launch's registers would wait for good");
+  static constexpr size_t kStageBytes = (size_t)kStages * (kRawBytes + 3 * kPlane);
+};
 constexpr int kMainCol = 0, kSmallCol = kMaxN, kACol = 2 * kMaxN;   // tensor memory columns
 constexpr int kACols = 3 * BK / 2;                                  // of one stage of A
 constexpr int kLargeSteps = 2, kSmallSteps = 8;   // steps of K after which an accumulator is read out and started again
-constexpr int kGroups = kMaxN / 8 / 2;            // groups of eight tokens per epilogue warp
-static_assert(kACol + kConvStages * kACols <= 512, "tensor memory");
-static_assert((kMaxN / 8 + 4) * kRowsA * 32 <= kRawStages * kRawBytes, "sums of all ranges reuse the raw stages");
+static_assert(kACol + kMaxStages * kACols <= 512, "tensor memory");
+static_assert((kMaxN / 8 + 4) * kRowsA * 32 <= Cfg<false>::kStages * Cfg<false>::kRawBytes &&
+              (kMaxN / 8 + 4) * kRowsA * 32 <= Cfg<true>::kStageBytes, "sums of all ranges reuse the stages");
 
 struct Control {
-  uint64_t raw_full[kRawStages], raw_empty[kRawStages];
-  uint64_t conv_full[kConvStages], conv_empty[kConvStages];
+  uint64_t raw_full[kMaxStages], raw_empty[kMaxStages];
+  uint64_t conv_full[kMaxStages], conv_empty[kMaxStages];
   uint64_t main_full, main_empty, small_full, small_empty;
   uint32_t tmem_base;
   int abort;
   int offsets[kMaxExperts + 1];
   int block_start[kMaxExperts + 1];   // token blocks of the experts before
 };
-constexpr size_t kSmemBytes = 1024 + (size_t)kRawStages * kRawBytes + kConvStages * 3 * kPlane + sizeof(Control);
-static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
+template <bool PLANES>
+constexpr size_t kSmemBytes = 1024 + Cfg<PLANES>::kStageBytes + sizeof(Control);
+static_assert(kSmemBytes<false> <= 227 * 1024 && kSmemBytes<true> <= 227 * 1024, "shared memory of one CTA");
+
+// The activations. Split in the kernel: 16-row boxes of 32 columns in rows[0]. PLANES: [3][M][K] bf16, boxes of 32 columns
+// of 32, 64, ..., 160 rows of all planes.
+struct TokenMaps {
+  CUtensorMap rows[kMaxN / 32];
+};
 
 struct Tile {
   int e, m;            // expert, tile of weight rows
@@ -148,25 +171,9 @@ __device__ __forceinline__ uint64_t desc64(uint32_t saddr) {
          (uint64_t)4 << 61;
 }
 
-// Two values cut off to bf16, NaN to NaN (whose upper half alone may be an infinity's).
-__device__ __forceinline__ uint32_t cut_bf16x2(float lo, float hi) {
-  uint32_t v;
-  asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
-  return v;
-}
-// Eight values into their three bf16 parts, exactly (where they are finite).
 __device__ __forceinline__ void split8(const float (&x)[8], uint32_t (&p0)[4], uint32_t (&p1)[4], uint32_t (&p2)[4]) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t u0 = __float_as_uint(x[2 * i]), u1 = __float_as_uint(x[2 * i + 1]);
-    p0[i] = cut_bf16x2(x[2 * i], x[2 * i + 1]);
-    float r0 = x[2 * i] - __uint_as_float(u0 & 0xffff0000u);
-    float r1 = x[2 * i + 1] - __uint_as_float(u1 & 0xffff0000u);
-    p1[i] = pack_bf16x2(r0, r1);
-    r0 -= bf16_lo(p1[i]);
-    r1 -= bf16_hi(p1[i]);
-    p2[i] = pack_bf16x2(r0, r1);
-  }
+  for (int i = 0; i < 4; ++i) split2(x[2 * i], x[2 * i + 1], p0[i], p1[i], p2[i]);
 }
 
 // (a: the rows may come from the kernel before this one, so they are not read as constant data)
@@ -178,7 +185,20 @@ __device__ __forceinline__ float dot_f32(const float* a, const float* w, int k0,
 }
 __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= FLT_MAX; }
 
+// Row `a` of three bf16 planes: what they are the parts of (an infinity's other parts are NaN).
+__device__ __forceinline__ float join(const __nv_bfloat16* a, int64_t plane) {
+  const float p0 = __bfloat162float(__ldcg(a));
+  return fabsf(p0) <= FLT_MAX ? p0 + (__bfloat162float(__ldcg(a + plane)) + __bfloat162float(__ldcg(a + 2 * plane))) : p0;
+}
+__device__ __forceinline__ float dot_planes(const __nv_bfloat16* a, int64_t plane, const float* w, int k0, int k1) {
+  float s = 0.f;
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) s = fmaf(join(a + k, plane), w[k], s);
+  return s;
+}
+
 // The sums of eight tokens have been used: those of the next eight take their place.
+template <int kGroups>
 __device__ __forceinline__ void next_group(float (&acc)[kGroups][8]) {
 #pragma unroll
   for (int g = 0; g + 1 < kGroups; ++g)
@@ -204,42 +224,62 @@ __device__ __forceinline__ void st_cluster4(uint32_t addr, float a, float b, flo
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// A: [rows, K] activations (sorted buffer); W_e: [Nw, K]; out [rows, Nout].
+__device__ __forceinline__ void tma_load_planes(void* dst, const void* tmap, uint64_t* bar, int k, int row) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(k), "r"(row), "r"(0)
+      : "memory");
+}
+
+// A: [M, K] activations (sorted buffer); W_e: [Nw, K]; out [M, Nout].
 // GEGLU: Nw = 2 * Nout, gate rows [0, Nout), up rows [Nout, 2 * Nout).
+// PLANES: the activations are read as bf16 planes, and the GEGLU pass writes its own so; A is read again where a sum is
+// formed again, fp32 rows in the GEGLU pass, planes in the down pass.
 // splits: CTAs of a cluster; with more than one a cluster has one tile at most.
-template <bool GEGLU>
+template <bool GEGLU, bool PLANES>
 __global__ void __launch_bounds__(kThreads, 1)
-ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activations, 16-row boxes of 32 columns
-               const CUtensorMap* __restrict__ tmap_w,              // [E], 64-row boxes of 32 columns
-               const float* __restrict__ A, const int32_t* __restrict__ offsets, const void* const* __restrict__ Wp,
-               const void* const* __restrict__ bp, int E, int K, int Nout, int splits, float* __restrict__ out,
+ffn_f32_kernel(const __grid_constant__ TokenMaps tmap_a, const CUtensorMap* __restrict__ tmap_w,   // [E], 64-row boxes of 32
+               const void* __restrict__ A, const int32_t* __restrict__ offsets, const void* const* __restrict__ Wp,
+               const void* const* __restrict__ bp, int64_t M, int E, int K, int Nout, int splits, void* __restrict__ out_raw,
                int32_t* __restrict__ status) {
+  using C = Cfg<PLANES>;
+  constexpr int kStages = C::kStages, kRawBytes = C::kRawBytes, kEpiFirst = C::kEpiFirst, kParts = C::kParts, kGroups = C::kGroups;
+  float* out = static_cast<float*>(out_raw);
+  __nv_bfloat16* out_planes = static_cast<__nv_bfloat16*>(out_raw);     // PLANES && GEGLU: [3][M][Nout]
+  const int64_t plane_out = M * Nout;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* planes = smem + (size_t)kRawStages * kRawBytes;      // [kConvStages][3] bf16 tiles of the tokens
-  Control* ctl = reinterpret_cast<Control*>(planes + kConvStages * 3 * kPlane);
+  uint8_t* planes = smem + (size_t)kStages * kRawBytes;         // [kStages][3] bf16 tiles of the tokens
+  Control* ctl = reinterpret_cast<Control*>(planes + kStages * 3 * kPlane);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kFeatures = GEGLU ? 64 : 128;                    // output columns of a tile
   const int m_tiles = (Nout + kFeatures - 1) / kFeatures;
-  const int rank = splits > 1 ? (int)cluster_rank() : 0;
+  // K over a cluster that adds its sums up, or (the down pass on planes) over blocks that leave them to the combine kernel
+  constexpr bool kParted = PLANES && !GEGLU;
+  const bool clustered = !kParted && splits > 1;
+  const int rank = kParted ? (int)(blockIdx.x % splits) : clustered ? (int)cluster_rank() : 0;
   const int first = blockIdx.x / splits, step = gridDim.x / splits;
   const int kb_all = (K + BK - 1) / BK;
   const int kb_per = (kb_all + splits - 1) / splits;
   const int kb0 = min(kb_all, rank * kb_per), kn = min(kb_all, kb0 + kb_per) - kb0;   // this CTA's steps of K
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kRawStages; ++s) { mbar_init(&ctl->raw_full[s], 1); mbar_init(&ctl->raw_empty[s], kSplitWarps); }
-    for (int c = 0; c < kConvStages; ++c) { mbar_init(&ctl->conv_full[c], kSplitWarps); mbar_init(&ctl->conv_empty[c], 1); }
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&ctl->raw_full[s], 1);
+      mbar_init(&ctl->raw_empty[s], C::kSplitWarps);
+      mbar_init(&ctl->conv_full[s], C::kSplitWarps + (PLANES ? 1 : 0));   // and the planes
+      mbar_init(&ctl->conv_empty[s], 1);
+    }
     mbar_init(&ctl->main_full, 1);
-    mbar_init(&ctl->main_empty, kEpiWarps);
+    mbar_init(&ctl->main_empty, C::kEpiWarps);
     mbar_init(&ctl->small_full, 1);
-    mbar_init(&ctl->small_empty, kEpiWarps);
+    mbar_init(&ctl->small_empty, C::kEpiWarps);
     ctl->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
   if (warp == 2) {
-    if (lane == 0) prefetch_tmap(&tmap_a);
+    if (lane < (PLANES ? kMaxN / 32 : 1)) prefetch_tmap(&tmap_a.rows[lane]);
     for (int e = lane; e < E; e += 32) prefetch_tmap(tmap_w + e);
   }
   if (warp == 1) {
@@ -274,7 +314,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
   const int total = ctl->block_start[E] * m_tiles;
 
   if (warp < 4) {
-    fewer_registers<kRegsLoad>();
+    fewer_registers<C::kRegsLoad>();
     if (warp == 0 && elect_one()) {
       // ---------------- TMA producer ----------------
       int s = 0;
@@ -288,76 +328,92 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           if (!mbar_wait(&ctl->raw_empty[s], phase ^ 1u, &ctl->abort, status, 51)) { ok = false; break; }
           uint8_t* dst = smem + (size_t)s * kRawBytes;
           const int k = (kb0 + i) * BK;
-          mbar_expect_tx(&ctl->raw_full[s], (uint32_t)(kRawA + tl.n * BK * 4));
+          mbar_expect_tx(&ctl->raw_full[s], (uint32_t)(kRawA + (PLANES ? 0 : tl.n * BK * 4)));
           tma_load_2d(dst, tw, &ctl->raw_full[s], k, r0);
           tma_load_2d(dst + kRawA / 2, tw, &ctl->raw_full[s], k, r1);
-          for (int j = 0; j < tl.n; j += 16) tma_load_2d(dst + kRawA + j * BK * 4, &tmap_a, &ctl->raw_full[s], k, tl.row0 + j);
-          if (++s == kRawStages) { s = 0; phase ^= 1u; }
+          if constexpr (PLANES) {
+            if (!mbar_wait(&ctl->conv_empty[s], phase ^ 1u, &ctl->abort, status, 59)) { ok = false; break; }
+            const int boxes = (tl.n + 31) >> 5;
+            mbar_expect_tx(&ctl->conv_full[s], (uint32_t)(boxes * 32 * 3 * BK * 2));
+            tma_load_planes(planes + (size_t)s * 3 * kPlane, &tmap_a.rows[boxes - 1], &ctl->conv_full[s], k, tl.row0);
+          } else {
+            for (int j = 0; j < tl.n; j += 16)
+              tma_load_2d(dst + kRawA + j * BK * 4, &tmap_a.rows[0], &ctl->raw_full[s], k, tl.row0 + j);
+          }
+          if (++s == kStages) { s = 0; phase ^= 1u; }
         }
       }
-    } else if (warp == 1) {
-      // ---------------- products: the whole warp keeps step, so that addresses stay in uniform registers ----------------
-      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    } else if (warp == 1 && elect_one()) {
+      // ---------------- products ----------------
       uint32_t phase = 0, larges = 0, smalls = 0;
       int c = 0;
       bool ok = true;
       for (int t = first; ok && t < total; t += step) {
         const Tile tl = tile_of(ctl, E, m_tiles, t);
         const uint32_t idesc = make_idesc(tl.n);
-        for (int i = 0; i < kn; ++i) {
-          if (!warp_wait(&ctl->conv_full[c], phase, ctl, status, 53)) { ok = false; break; }
-          if (i % kLargeSteps == 0) {
-            if (!warp_wait(&ctl->main_empty, (larges & 1u) ^ 1u, ctl, status, 54)) { ok = false; break; }
-            ++larges;
-          }
+        // 16-byte units from one plane of the tokens to the next
+        const uint64_t kP = PLANES ? (uint64_t)((tl.n + 31) >> 5) * (32 * BK * 2 / 16) : (uint64_t)(kPlane / 16);
+        // Two steps at a time, their large products first: those sums are read out while the small products run, and the
+        // thread that issues has to look at barriers half as often (46 clk a product, 60 to 100 a barrier or commit).
+        static_assert(kLargeSteps == 2 && kSmallSteps % 2 == 0, "steps go in pairs");
+        for (int i = 0; i < kn; i += 2) {
+          const bool two = i + 1 < kn;
+          const int c1 = c + 1 == kStages ? 0 : c + 1;
+          const uint32_t phase1 = c + 1 == kStages ? phase ^ 1u : phase;
+          if (!mbar_wait(&ctl->conv_full[c], phase, &ctl->abort, status, 53)) { ok = false; break; }
+          if (!mbar_wait(&ctl->main_empty, (larges++ & 1u) ^ 1u, &ctl->abort, status, 54)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a = tm + kACol + c * kACols;
-          const uint64_t b = desc64(smem_u32(planes) + (uint32_t)(c * 3 * kPlane));
-          constexpr uint64_t kP = kPlane / 16;
-          const bool large_ends = (i + 1) % kLargeSteps == 0 || i == kn - 1;
-          const bool small_ends = (i + 1) % kSmallSteps == 0 || i == kn - 1;
-          // the large products first: their sums are read out while the small products run
-          if (elect_one()) {
-            mma_ts(tm + kMainCol, a, b, idesc, i % kLargeSteps != 0 ? 1u : 0u);
-            mma_ts(tm + kMainCol, a + 8, b + 2, idesc, 1u);
-            if (large_ends) tc_commit(&ctl->main_full);
-          }
-          __syncwarp();
-          if (i % kSmallSteps == 0) {
-            if (!warp_wait(&ctl->small_empty, (smalls & 1u) ^ 1u, ctl, status, 52)) { ok = false; break; }
+          const uint32_t a0 = tmem + kACol + c * kACols, a1 = tmem + kACol + c1 * kACols;
+          const uint64_t b0 = desc64(smem_u32(planes) + (uint32_t)(c * 3 * kPlane));
+          const uint64_t b1 = desc64(smem_u32(planes) + (uint32_t)(c1 * 3 * kPlane));
+          mma_ts(tmem + kMainCol, a0, b0, idesc, 0u);
+          mma_ts(tmem + kMainCol, a0 + 8, b0 + 2, idesc, 1u);
+          if (two) {
+            if (!mbar_wait(&ctl->conv_full[c1], phase1, &ctl->abort, status, 53)) { ok = false; break; }
             tc_fence_after();
-            ++smalls;
+            mma_ts(tmem + kMainCol, a1, b1, idesc, 1u);
+            mma_ts(tmem + kMainCol, a1 + 8, b1 + 2, idesc, 1u);
           }
-          if (elect_one()) {
+          tc_commit(&ctl->main_full);
+          if (i % kSmallSteps == 0) {
+            if (!mbar_wait(&ctl->small_empty, (smalls++ & 1u) ^ 1u, &ctl->abort, status, 52)) { ok = false; break; }
+            tc_fence_after();
+          }
+          auto small_products = [&](uint32_t a, uint64_t b, bool more) {
 #pragma unroll
             for (int kk = 0; kk < 2; ++kk) {
               const uint32_t ak = a + kk * 8;
               const uint64_t bk = b + kk * 2;
-              mma_ts(tm + kSmallCol, ak + 32, bk, idesc, (i % kSmallSteps | kk) != 0 ? 1u : 0u);   // a2 b0
-              mma_ts(tm + kSmallCol, ak, bk + 2 * kP, idesc, 1u);                                  // a0 b2
-              mma_ts(tm + kSmallCol, ak + 16, bk + kP, idesc, 1u);                                 // a1 b1
-              mma_ts(tm + kSmallCol, ak + 16, bk, idesc, 1u);                                      // a1 b0
-              mma_ts(tm + kSmallCol, ak, bk + kP, idesc, 1u);                                      // a0 b1
+              mma_ts(tmem + kSmallCol, ak + 32, bk, idesc, more || kk != 0 ? 1u : 0u);   // a2 b0
+              mma_ts(tmem + kSmallCol, ak, bk + 2 * kP, idesc, 1u);                      // a0 b2
+              mma_ts(tmem + kSmallCol, ak + 16, bk + kP, idesc, 1u);                     // a1 b1
+              mma_ts(tmem + kSmallCol, ak + 16, bk, idesc, 1u);                          // a1 b0
+              mma_ts(tmem + kSmallCol, ak, bk + kP, idesc, 1u);                          // a0 b1
             }
-            if (small_ends) tc_commit(&ctl->small_full);
-            tc_commit(&ctl->conv_empty[c]);
+          };
+          small_products(a0, b0, i % kSmallSteps != 0);
+          tc_commit(&ctl->conv_empty[c]);
+          if (two) {
+            small_products(a1, b1, true);
+            tc_commit(&ctl->conv_empty[c1]);
           }
-          __syncwarp();
-          if (++c == kConvStages) { c = 0; phase ^= 1u; }
+          if ((i + 2) % kSmallSteps == 0 || i + 2 >= kn) tc_commit(&ctl->small_full);
+          if (two) { c = c1; phase = phase1; }
+          if (++c == kStages) { c = 0; phase ^= 1u; }
         }
       }
     }
     __syncwarp();
-    if (splits > 1) { cluster_sync(); cluster_sync(); }
+    if (clustered) { cluster_sync(); cluster_sync(); }
   } else if (warp < kEpiFirst) {
     // ---------------- split ----------------
-    fewer_registers<kRegsSplit>();
-    const int quad = warp & 3, part = ((warp - 4) >> 2) & 1;   // lanes of tensor memory; half of the step's K
+    fewer_registers<C::kRegsSplit>();
+    constexpr int kSplitWarps = C::kSplitWarps;
+    const int quad = warp & 3, part = PLANES ? 0 : ((warp - 4) >> 2) & 1;   // lanes of tensor memory; half of the step's K
     const int group = (warp - 4) / kSplitWarps;
     const int et = (threadIdx.x - 128) % (32 * kSplitWarps);
     // the row of the raw tile that goes to this lane. GEGLU: gate and up of a feature in one warp, 16 lanes apart
     const int r = GEGLU ? (lane & 15) + quad * 16 + (lane >> 4) * 64 : quad * 32 + lane;
-    static_assert(kRawStages == kConvStages, "one stage counter for both");
     int s = 0, turn = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -366,7 +422,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
       for (int i = 0; i < kn; ++i, turn ^= 1) {
         const int c = s;
         const uint32_t ph = phase;
-        if (++s == kRawStages) { s = 0; phase ^= 1u; }
+        if (++s == kStages) { s = 0; phase ^= 1u; }
         if (turn != group) continue;
         // In this order: boxes may land out of order, and with the other group's last turn on this stage still to come its
         // barrier would be a phase behind and this parity would look done. The products of that turn are done first.
@@ -383,7 +439,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
         };
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < 16 / kSplitWarps; ++j) {
           float x[8];
           uint32_t p0[4], p1[4], p2[4];
           load8_at(raw + r * 128, r, part * 4 + j * 2, x);
@@ -393,7 +449,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           st_tmem4(ta + 32 + j * 4, p2);
         }
         uint8_t* pl = planes + (size_t)c * 3 * kPlane;
-        for (int q = et; q < tl.n * 4; q += 32 * kSplitWarps) {      // a token's eight values at a time
+        for (int q = et; !PLANES && q < tl.n * 4; q += 32 * kSplitWarps) {      // a token's eight values at a time
           const int rr = q >> 2, p = q & 3;
           float x[8];
           uint32_t p0[4], p1[4], p2[4];
@@ -405,7 +461,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           *reinterpret_cast<uint4*>(d + 2 * kPlane) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
         }
         st_tmem_wait();
-        fence_async_smem();
+        if (!PLANES) fence_async_smem();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
@@ -415,11 +471,11 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
       }
     }
     __syncwarp();
-    if (splits > 1) { cluster_sync(); cluster_sync(); }
+    if (clustered) { cluster_sync(); cluster_sync(); }
   } else {
     // ---------------- sums and epilogue: lane = weight row, columns = tokens ----------------
-    more_registers<kRegsEpi>();
-    const int quad = warp & 3, part = (warp - kEpiFirst) >> 2;   // this warp: token groups part, part + 2, ...
+    more_registers<C::kRegsEpi>();
+    const int quad = warp & 3, part = (warp - kEpiFirst) >> 2;   // this warp: token groups part, part + kParts, ...
     const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + part * 8;
     uint32_t larges = 0, smalls = 0;
     bool ok = true, sent = false;
@@ -430,54 +486,95 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
       for (int g = 0; g < kGroups; ++g)
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
+      const int feat = tl.m * kFeatures + (GEGLU ? quad * 16 + (lane & 15) : quad * 32 + lane);
+      const bool feat_ok = feat < Nout;
+      // (asked for here: behind the products their way from memory took longer than the rest of the epilogue)
+      const bool biased = !clustered && !(kParted && splits > 1);
+      const float* bias = biased && feat_ok ? static_cast<const float*>(bp[tl.e]) : nullptr;
+      const float b0 = bias != nullptr ? __ldg(bias + feat) : 0.f;
+      const float b1 = GEGLU && bias != nullptr ? __ldg(bias + Nout + feat) : 0.f;
       uint64_t again = 0;      // a bit per sum of this thread whose small products were not finite, ...
       uint32_t again_hi = 0;   // ... from the ninth group on
       auto add = [&](int col) {
         // (groups past n hold old sums; they are not used)
+        constexpr int kAtOnce = PLANES ? 3 : 4;
 #pragma unroll
-        for (int g0 = 0; g0 < kGroups; g0 += 4) {
-          if ((g0 * 2 + part) * 8 >= tl.n) break;
-          uint32_t v[4][8];
+        for (int g0 = 0; g0 < kGroups; g0 += kAtOnce) {
+          if ((g0 * kParts + part) * 8 >= tl.n) break;
+          uint32_t v[kAtOnce][8];
 #pragma unroll
-          for (int g = 0; g < 4; ++g)
-            if (g0 + g < kGroups) ld_tmem8(ta + col + (g0 + g) * 16, v[g]);
+          for (int g = 0; g < kAtOnce; ++g)
+            if (g0 + g < kGroups) ld_tmem8(ta + col + (g0 + g) * 8 * kParts, v[g]);
           tc_ld_wait();
 #pragma unroll
-          for (int g = 0; g < 4; ++g)
+          for (int g = 0; g < kAtOnce; ++g)
             if (g0 + g < kGroups) {
 #pragma unroll
               for (int i = 0; i < 8; ++i) acc[g0 + g][i] += __uint_as_float(v[g][i]);
             }
         }
       };
-      // Small products that are not finite become zero, in tensor memory, and are noted.
-      auto keep_finite = [&]() {
-        static_assert(kGroups % 2 == 0 && kGroups <= 12, "two groups at a time, 96 bits");
-#pragma unroll 1
-        for (int g0 = 0; (g0 * 2 + part) * 8 < tl.n; g0 += 2) {
-          uint32_t v[2][8];
-          ld_tmem8(ta + kSmallCol + g0 * 16, v[0]);
-          ld_tmem8(ta + kSmallCol + g0 * 16 + 16, v[1]);
-          tc_ld_wait();
-          float probe[2] = {0.f, 0.f};      // times zero: NaN where one is not finite
+      // Small products that are not finite become zero and are noted.
+      auto add_small = [&]() {
+        if constexpr (PLANES) {
+          constexpr int kAtOnce = 3;
+          static_assert(kGroups <= 8, "bits of `again`");
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            probe[0] = fmaf(__uint_as_float(v[0][i]), 0.f, probe[0]);
-            probe[1] = fmaf(__uint_as_float(v[1][i]), 0.f, probe[1]);
-          }
-          if (__any_sync(0xffffffffu, probe[0] + probe[1] != 0.f)) {
-            uint32_t bits = 0;
+          for (int g0 = 0; g0 < kGroups; g0 += kAtOnce) {
+            if ((g0 * kParts + part) * 8 >= tl.n) break;
+            uint32_t v[kAtOnce][8];
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (!finite(__uint_as_float(v[i >> 3][i & 7]))) {
-                v[i >> 3][i & 7] = 0u;
-                bits |= 1u << i;
+            for (int g = 0; g < kAtOnce; ++g)
+              if (g0 + g < kGroups) ld_tmem8(ta + kSmallCol + (g0 + g) * 8 * kParts, v[g]);
+            tc_ld_wait();
+#pragma unroll
+            for (int g = 0; g < kAtOnce; ++g)
+              if (g0 + g < kGroups) {
+                float probe[2] = {0.f, 0.f};      // times zero: NaN where one is not finite
+#pragma unroll
+                for (int i = 0; i < 8; ++i) probe[i & 1] = fmaf(__uint_as_float(v[g][i]), 0.f, probe[i & 1]);
+                if (probe[0] + probe[1] != 0.f) {
+#pragma unroll
+                  for (int i = 0; i < 8; ++i)
+                    if (!finite(__uint_as_float(v[g][i]))) {
+                      v[g][i] = 0u;
+                      again |= 1ull << ((g0 + g) * 8 + i);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[g0 + g][i] += __uint_as_float(v[g][i]);
               }
-            st_tmem8(ta + kSmallCol + g0 * 16, v[0]);
-            st_tmem8(ta + kSmallCol + g0 * 16 + 16, v[1]);
-            st_tmem_wait();
-            if (g0 < 8) again |= (uint64_t)bits << (g0 * 8); else again_hi |= bits << (g0 * 8 - 64);
           }
+        } else {
+          // (in tensor memory: twenty groups in registers leave no room to do it on the way)
+          static_assert(PLANES || (kGroups % 2 == 0 && kGroups <= 12), "two groups at a time, 96 bits");
+#pragma unroll 1
+          for (int g0 = 0; (g0 * kParts + part) * 8 < tl.n; g0 += 2) {
+            uint32_t v[2][8];
+            ld_tmem8(ta + kSmallCol + g0 * 8 * kParts, v[0]);
+            ld_tmem8(ta + kSmallCol + (g0 + 1) * 8 * kParts, v[1]);
+            tc_ld_wait();
+            float probe[2] = {0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              probe[0] = fmaf(__uint_as_float(v[0][i]), 0.f, probe[0]);
+              probe[1] = fmaf(__uint_as_float(v[1][i]), 0.f, probe[1]);
+            }
+            if (__any_sync(0xffffffffu, probe[0] + probe[1] != 0.f)) {
+              uint32_t bits = 0;
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (!finite(__uint_as_float(v[i >> 3][i & 7]))) {
+                  v[i >> 3][i & 7] = 0u;
+                  bits |= 1u << i;
+                }
+              st_tmem8(ta + kSmallCol + g0 * 8 * kParts, v[0]);
+              st_tmem8(ta + kSmallCol + (g0 + 1) * 8 * kParts, v[1]);
+              st_tmem_wait();
+              if (g0 < 8) again |= (uint64_t)bits << (g0 * 8); else again_hi |= bits << (g0 * 8 - 64);
+            }
+          }
+          add(kSmallCol);
         }
       };
       for (int i = 1; i <= kn; ++i) {
@@ -494,20 +591,17 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           if (!warp_wait(&ctl->small_full, smalls & 1u, ctl, status, 58)) { ok = false; break; }
           ++smalls;
           tc_fence_after();
-          keep_finite();
-          add(kSmallCol);
+          add_small();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl->small_empty);
         }
       }
-      if (!ok && splits <= 1) break;
-      const float* W = static_cast<const float*>(Wp[tl.e]);
-      const int feat = tl.m * kFeatures + (GEGLU ? quad * 16 + (lane & 15) : quad * 32 + lane);
-      const bool feat_ok = feat < Nout;
+      if (!ok && !clustered) break;
       // The sums at hand, of eight tokens from c0 on: those that lack their small products and are finite without them are
       // formed again, over this CTA's range of K.
       auto form_again = [&](int c0) {
+        if ((again | again_hi) == 0) return;       // none of this thread's; nothing below needs the warp
         const uint32_t bits = (uint32_t)again & 0xffu;
         again = again >> 8 | (uint64_t)again_hi << 56;
         again_hi >>= 8;
@@ -515,25 +609,30 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
           float v[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = acc[0][i];
-          const float* w = W + (int64_t)(GEGLU && lane >= 16 ? Nout + feat : feat) * K;
+          const float* w = static_cast<const float*>(Wp[tl.e]) + (int64_t)(GEGLU && lane >= 16 ? Nout + feat : feat) * K;
 #pragma unroll 1
           for (int i = 0; i < 8 && c0 + i < tl.rows; ++i)
             if ((bits >> i & 1u) != 0u && finite(v[i]))
-              v[i] = dot_f32(A + (int64_t)(tl.row0 + c0 + i) * K, w, kb0 * BK, min(K, (kb0 + kn) * BK));
+            {
+              const int64_t at = (int64_t)(tl.row0 + c0 + i) * K;
+              const int k0 = kb0 * BK, k1 = min(K, (kb0 + kn) * BK);
+              v[i] = PLANES && !GEGLU ? dot_planes(static_cast<const __nv_bfloat16*>(A) + at, M * K, w, k0, k1)
+                                      : dot_f32(static_cast<const float*>(A) + at, w, k0, k1);
+            }
 #pragma unroll
           for (int i = 0; i < 8; ++i) acc[0][i] = v[i];
         }
-        __syncwarp();
       };
-      if (splits > 1) {
+      if (clustered) {
         // Eight tokens at a time go to the CTAs in turn, which keep them as [eight][source][128 rows][8 tokens] in
         // their raw stages.
         __syncwarp();
         cluster_sync();    // no CTA reads its raw stages any more
         const uint32_t mine = smem_u32(smem) + (uint32_t)((rank * kRowsA + quad * 32 + lane) * 32);
 #pragma unroll 1
-        for (int g = part; g * 8 < tl.n; g += 2, next_group(acc)) {
+        for (int g = part; g * 8 < tl.n; g += kParts, next_group(acc)) {
           form_again(g * 8);
+          __syncwarp();
           const uint32_t to = map_to_cta(mine, g & (splits - 1)) + (uint32_t)((g & -splits) * kRowsA * 32);
           st_cluster4(to, acc[0][0], acc[0][1], acc[0][2], acc[0][3]);
           st_cluster4(to + 16, acc[0][4], acc[0][5], acc[0][6], acc[0][7]);
@@ -541,14 +640,12 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
         sent = true;
         break;
       }
-      const float* bias = static_cast<const float*>(bp[tl.e]);
-      const float b0 = feat_ok ? __ldg(bias + feat) : 0.f;
-      const float b1 = GEGLU && feat_ok ? __ldg(bias + Nout + feat) : 0.f;
       // rolled, and the sums moved up: unrolled, 60 KB of code that runs from a cold instruction cache took 30000 clk
 #pragma unroll 1
-      for (int c0 = part * 8; c0 < tl.rows; c0 += 16, next_group(acc)) {
+      for (int c0 = part * 8; c0 < tl.rows; c0 += 8 * kParts, next_group(acc)) {
         form_again(c0);
-        float* o = out + (int64_t)(tl.row0 + c0) * Nout + feat;
+        __syncwarp();
+        float* o = out + ((kParted ? rank * M : 0) + tl.row0 + c0) * Nout + feat;
         if (GEGLU) {
           // lanes 0-15 (gate) take tokens c0 + i, lanes 16-31 (up) tokens c0 + i + 1, i even
           const int upper = lane >> 4;
@@ -559,9 +656,29 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
             const float gate = upper ? other : acc[0][2 * i], up = upper ? acc[0][2 * i + 1] : other;
             v[i] = gelu_tanh_precise(gate + b0) * (up + b1);
           }
+          if constexpr (PLANES) {
+            // lanes of even features take the first two of their tokens for both features, the others the last two
+            const int odd = lane & 1;
+            const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[2], 1);
+            const float r1 = __shfl_xor_sync(0xffffffffu, odd ? v[1] : v[3], 1);
+            const float pair[2][2] = {{odd ? r0 : v[0], odd ? v[2] : r0}, {odd ? r1 : v[1], odd ? v[3] : r1}};
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (c0 + 2 * i + upper < tl.rows && feat_ok) o[(int64_t)(2 * i + upper) * Nout] = v[i];
+            for (int i = 0; i < 2; ++i) {
+              const int token = c0 + 4 * odd + 2 * i + upper;
+              if (token < tl.rows && feat_ok) {
+                uint32_t p0, p1, p2;
+                split2(pair[i][0], pair[i][1], p0, p1, p2);
+                __nv_bfloat16* q = out_planes + (int64_t)(tl.row0 + token) * Nout + (feat - odd);
+                *reinterpret_cast<uint32_t*>(q) = p0;
+                *reinterpret_cast<uint32_t*>(q + plane_out) = p1;
+                *reinterpret_cast<uint32_t*>(q + 2 * plane_out) = p2;
+              }
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (c0 + 2 * i + upper < tl.rows && feat_ok) o[(int64_t)(2 * i + upper) * Nout] = v[i];
+          }
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i)
@@ -569,7 +686,7 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
         }
       }
     }
-    if (splits > 1) {
+    if (clustered) {
       __syncwarp();
       if (!sent) cluster_sync();     // (a cluster without a tile)
       cluster_sync();                // the sums of all ranges are there (or a wait ran out, and the status says so)
@@ -584,13 +701,16 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
             v[0] += u.x; v[1] += u.y; v[2] += u.z; v[3] += u.w;
           }
         };
-        // a thread: one feature of four tokens
-        const int et = threadIdx.x - 32 * kEpiFirst, j = et & (kFeatures - 1), half = et / kFeatures;
+        // a thread: one feature of four tokens at a time
+        constexpr int kUnits = 32 * C::kEpiWarps / kFeatures;
+        const int et = threadIdx.x - 32 * kEpiFirst, j = et & (kFeatures - 1);
         const int feat = tl.m * kFeatures + j;
         const int r = GEGLU ? (j >> 4) * 32 + (j & 15) : j;
-        if (half < 2 && feat < Nout) {
+        if (feat < Nout) {
           const float b0 = __ldg(bias + feat), b1 = GEGLU ? __ldg(bias + Nout + feat) : 0.f;
-          for (int g = rank; g * 8 < tl.rows; g += splits) {
+          for (int u = et / kFeatures;; u += kUnits) {
+            const int g = rank + (u >> 1) * splits, half = u & 1;
+            if (g * 8 >= tl.rows) break;
             const int c0 = g * 8 + half * 4;
             const float* p = reinterpret_cast<const float*>(smem) + ((g & -splits) * kRowsA + r) * 8 + half * 4;
             float v[8];
@@ -598,9 +718,19 @@ ffn_f32_kernel(const __grid_constant__ CUtensorMap tmap_a,          // activatio
             if (GEGLU) sum4(p + 16 * 8, reinterpret_cast<float(&)[4]>(v[4]));
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              if (c0 + i < tl.rows)
-                out[(int64_t)(tl.row0 + c0 + i) * Nout + feat] =
-                    GEGLU ? gelu_tanh_precise(v[i] + b0) * (v[4 + i] + b1) : v[i] + b0;
+              if (c0 + i < tl.rows) {
+                const float o = GEGLU ? gelu_tanh_precise(v[i] + b0) * (v[4 + i] + b1) : v[i] + b0;
+                const int64_t at = (int64_t)(tl.row0 + c0 + i) * Nout + feat;
+                if constexpr (GEGLU && PLANES) {
+                  uint32_t p0, p1, p2;
+                  split2(o, 0.f, p0, p1, p2);
+                  reinterpret_cast<uint16_t*>(out_planes)[at] = (uint16_t)p0;
+                  reinterpret_cast<uint16_t*>(out_planes)[at + plane_out] = (uint16_t)p1;
+                  reinterpret_cast<uint16_t*>(out_planes)[at + 2 * plane_out] = (uint16_t)p2;
+                } else {
+                  out[at] = o;
+                }
+              }
           }
         }
       }
@@ -629,26 +759,56 @@ int pick_splits(int64_t tiles, int K) {
   return 1;
 }
 
-template <bool GEGLU>
-int launch(const float* A, const int32_t* offsets, const void* tmaps_w, const void* const* W, const void* const* b,
-           int64_t M, int K, int Nout, int E, float* out, int32_t* status, cudaStream_t s) {
+}  // namespace
+
+// Ranges of K of the down pass on planes, a part of the sums each: those with which the rounds of tiles take the fewest
+// steps, a tile's start, epilogue and partial sums counted as five. (The host does not know the routing: every expert that
+// can have rows is taken to have them.)
+int f32_down_splits(int64_t M, int d, int f, int E) {
+  const int64_t hit = M < E ? M : E, full = (M + kMaxN - 1) / kMaxN, kb = (f + BK - 1) / BK;
+  const int64_t tiles = (hit > full ? hit : full) * ((d + 127) / 128);
+  int best = 1;
+  int64_t least = 0;
+  for (int s = 1; s <= 8 && (s == 1 || kb >= 4 * s); ++s) {
+    const int64_t cost = (tiles * s + kNumSMs - 1) / kNumSMs * ((kb + s - 1) / s + 5);
+    if (s == 1 || cost < least) { best = s; least = cost; }
+  }
+  return best;
+}
+
+namespace {
+
+// A: fp32 rows; planes: [3][M][K] bf16, or nullptr and A is split in the kernel.
+template <bool GEGLU, bool PLANES>
+int launch(const void* A, const void* planes, const int32_t* offsets, const void* tmaps_w, const void* const* W,
+           const void* const* b, int64_t M, int K, int Nout, int E, void* out,
+           int32_t* status, cudaStream_t s) {
   static PerDeviceOnce once;
-  int rc = ensure_dynamic_smem(once, ffn_f32_kernel<GEGLU>, kSmemBytes);
+  auto kernel = ffn_f32_kernel<GEGLU, PLANES>;
+  int rc = ensure_dynamic_smem(once, kernel, kSmemBytes<PLANES>);
   if (rc) return rc;
-  alignas(64) CUtensorMap tm;
-  rc = encode_tmap_2d_f32(&tm, A, (uint64_t)M, (uint64_t)K, 16);
+  alignas(64) TokenMaps tm;
+  if (PLANES) {
+    for (int i = 0; i < kMaxN / 32 && rc == 0; ++i)
+      if (i * 32 < M) rc = encode_tmap_planes(&tm.rows[i], planes, (uint64_t)M, (uint64_t)K, 32 * (i + 1));
+      else tm.rows[i] = tm.rows[0];         // no block has more tokens than there are rows
+  } else {
+    rc = encode_tmap_2d_f32(&tm.rows[0], A, (uint64_t)M, (uint64_t)K, 16);
+  }
   if (rc) return rc;
   int sms = 0;
   rc = sm_count(&sms);
   if (rc) return rc;
   const int64_t m_tiles = (Nout + (GEGLU ? 64 : 128) - 1) / (GEGLU ? 64 : 128);
   const int64_t hit = M < E ? M : E, full = (M + kMaxN - 1) / kMaxN;
-  const int splits = pick_splits((hit > full ? hit : full) * m_tiles, K);
+  constexpr bool kParted = PLANES && !GEGLU;
+  const int splits = kParted ? f32_down_splits(M, Nout, K, E) : pick_splits((hit > full ? hit : full) * m_tiles, K);
   const int64_t most = (M / kMaxN + hit) * m_tiles;        // tiles there can be
-  const unsigned grid = splits > 1 ? (unsigned)(most * splits) : (unsigned)(most < sms ? most : sms);
-  MOE_CUDA_CHECK(launch_pdl_cluster(ffn_f32_kernel<GEGLU>, dim3(grid), dim3(kThreads), splits, kSmemBytes, s, tm,
-                                    static_cast<const CUtensorMap*>(tmaps_w), A, offsets, W, b, E, K, Nout, splits, out,
-                                    status));
+  const int64_t at_once = kParted ? sms / splits : splits > 1 ? most : sms;     // a cluster has one tile at most
+  const unsigned grid = (unsigned)((most < at_once || at_once < 1 ? most : at_once) * splits);
+  MOE_CUDA_CHECK(launch_pdl_cluster(kernel, dim3(grid), dim3(kThreads), kParted ? 1 : splits, kSmemBytes<PLANES>, s, tm,
+                                    static_cast<const CUtensorMap*>(tmaps_w), PLANES && !GEGLU ? planes : A, offsets, W, b, M,
+                                    E, K, Nout, splits, out, status));
   return 0;
 }
 
@@ -658,11 +818,20 @@ int launch_experts_f32(const void* perm, const int32_t* offsets, const void* pla
                        void* y, int32_t* status, cudaStream_t s) {
   if (M == 0) return 0;
   PlanView pv = plan_view(plan, E);
-  int rc = launch<true>(static_cast<const float*>(perm), offsets, pv.tmap_W1, pv.W1, pv.b1, M, d, f, E,
-                        static_cast<float*>(h), status, s);
+  int rc = launch<true, false>(perm, nullptr, offsets, pv.tmap_W1, pv.W1, pv.b1, M, d, f, E, h, status, s);
   if (rc) return rc;
-  return launch<false>(static_cast<const float*>(h), offsets, pv.tmap_W2, pv.W2, pv.b2, M, f, d, E,
-                       static_cast<float*>(y), status, s);
+  return launch<false, false>(h, nullptr, offsets, pv.tmap_W2, pv.W2, pv.b2, M, f, d, E, y, status, s);
+}
+
+// The same with perm in three bf16 planes [3][M, d] as well, and h [3][M, f] kept in planes only. y: [M, d], or with more
+// than one of f32_down_splits() the partial sums [splits][M, d] without down.bias.
+int launch_experts_f32_planes(const void* perm, const void* perm_planes, const int32_t* offsets, const void* plan, int64_t M,
+                              int d, int f, int E, void* h_planes, void* y, int32_t* status, cudaStream_t s) {
+  if (M == 0) return 0;
+  PlanView pv = plan_view(plan, E);
+  int rc = launch<true, true>(perm, perm_planes, offsets, pv.tmap_W1, pv.W1, pv.b1, M, d, f, E, h_planes, status, s);
+  if (rc) return rc;
+  return launch<false, true>(nullptr, h_planes, offsets, pv.tmap_W2, pv.W2, pv.b2, M, f, d, E, y, status, s);
 }
 
 }  // namespace moe

@@ -17,20 +17,20 @@ front_small_kernel(const T* __restrict__ x, const T* Wg, const T* bg, int Ntotal
                    float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                    float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
                    int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
-                   T* __restrict__ perm, float* __restrict__ psum,
+                   T* __restrict__ perm, __nv_bfloat16* __restrict__ planes, float* __restrict__ psum,
                    float* __restrict__ aux, int* __restrict__ xch, int* __restrict__ counter,
                    int32_t* __restrict__ status) {
   extern __shared__ float smem[];
   pdl_wait();                 // x may come from the kernel before this one
   pdl_launch_dependents();
   front_small_body<NT, SPLIT, T>(smem, x, Wg, bg, Ntotal, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
-                                 row_of, perm, psum, aux, xch, counter, status);
+                                 row_of, perm, planes, psum, aux, xch, counter, status);
 }
 
 template <int NT, typename T>
 int launch(const void* x, const void* Wg, const void* bg, int N, int d, int E, int k,
            float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot, int32_t* offsets,
-           int32_t* row_of, void* perm, float* psum, float* aux, int* xch, int* counter,
+           int32_t* row_of, void* perm, void* planes, float* psum, float* aux, int* xch, int* counter,
            int32_t* status, cudaStream_t s) {
   // beyond 128 tokens repeating the routing in every block costs more than one exchange
   constexpr bool F32 = sizeof(T) == 4;
@@ -50,7 +50,8 @@ int launch(const void* x, const void* Wg, const void* bg, int N, int d, int E, i
   const int blocks = N <= 16 ? 1 : (N + 15) / 16;
   MOE_CUDA_CHECK(launch_pdl_as(fn, dim3(blocks), dim3(kThreads), 0, F32 && blocks > 1, smem, s, static_cast<const T*>(x),
                                static_cast<const T*>(Wg), static_cast<const T*>(bg), N, d, E, k, out_logits, out_idx,
-                               out_w, cnt_slot, offsets, row_of, static_cast<T*>(perm), psum, aux, xch, counter, status));
+                               out_w, cnt_slot, offsets, row_of, static_cast<T*>(perm),
+                               static_cast<__nv_bfloat16*>(planes), psum, aux, xch, counter, status));
   return 0;
 }
 
@@ -99,12 +100,12 @@ int launch_by_experts(int E, Args... args) {
 int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E, int k,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
-                       cudaStream_t s, int* xch, int* counter, int32_t* status, int dtype) {
+                       cudaStream_t s, int* xch, int* counter, int32_t* status, int dtype, void* planes) {
   if (dtype == MOE_B200_F32)
     return launch_by_experts<float>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of,
-                                    perm, psum, aux, xch, counter, status, s);
+                                    perm, planes, psum, aux, xch, counter, status, s);
   return launch_by_experts<__nv_bfloat16>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
-                                          row_of, perm, psum, aux, xch, counter, status, s);
+                                          row_of, perm, nullptr, psum, aux, xch, counter, status, s);
 }
 
 }  // namespace moe

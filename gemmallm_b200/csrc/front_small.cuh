@@ -16,7 +16,7 @@
 //      on order-preserving keys, renormalise;
 //   C. warp 0: per-slot counts, offsets (scan over E), stable ranks in (token,
 //      slot) order; then row copies into the sorted buffer with 16-byte accesses
-//      (their loads were issued before B);
+//      (their loads were issued before B; fp32: also as planes, three bf16 parts of every value, [3][N k][d]);
 //   E. block 0: probabilities summed per expert in token order; loss.
 #pragma once
 #include <cooperative_groups.h>
@@ -80,7 +80,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
                  float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                  float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
                  int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
-                 T* __restrict__ perm, float* __restrict__ psum,
+                 T* __restrict__ perm, __nv_bfloat16* __restrict__ planes, float* __restrict__ psum,
                  float* __restrict__ aux, int* __restrict__ xch, int* __restrict__ counter,
                  int32_t* __restrict__ status) {
   constexpr int kThreads = kFrontThreads;
@@ -457,9 +457,22 @@ __device__ __forceinline__ void front_small_body(float* smem,
       const int i = i0 + u * kThreads;
       if (i < items) {
         const int tok = i / pieces, pc = i - tok * pieces;
-        for (int j = 0; j < k; ++j) {
-          const int row = s_row[tok * k + j];
-          if (!F32 || row >= 0) reinterpret_cast<uint4*>(perm + (size_t)row * d)[pc] = v[u];
+        if constexpr (F32) {
+          // the rows as they are, and as the three bf16 planes the products read (split once here, not by every tile)
+          uint2 part[3];
+          split2(__uint_as_float(v[u].x), __uint_as_float(v[u].y), part[0].x, part[1].x, part[2].x);
+          split2(__uint_as_float(v[u].z), __uint_as_float(v[u].w), part[0].y, part[1].y, part[2].y);
+          for (int j = 0; j < k; ++j) {
+            const int row = s_row[tok * k + j];
+            if (row < 0) continue;
+            reinterpret_cast<uint4*>(perm + (size_t)row * d)[pc] = v[u];
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+              reinterpret_cast<uint2*>(planes + ((size_t)q * Ntotal * k + row) * d)[pc] = part[q];
+          }
+        } else {
+          for (int j = 0; j < k; ++j)
+            reinterpret_cast<uint4*>(perm + (size_t)s_row[tok * k + j] * d)[pc] = v[u];
         }
       }
     }

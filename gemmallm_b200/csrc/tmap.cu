@@ -64,6 +64,20 @@ int encode_tmap_2d_f32(void* out, const void* base, uint64_t rows, uint64_t cols
   return 0;
 }
 
+int encode_tmap_planes(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  EncodeTiledFn enc = get_encode();
+  if (enc == nullptr) return set_error(MOE_B200_ERR_DRIVER, "cuTensorMapEncodeTiled unavailable");
+  cuuint64_t dims[3] = {cols, rows, 3};
+  cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
+  cuuint32_t box[3] = {32, box_rows, 3};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(static_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides,
+                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(MOE_B200_ERR_DRIVER, "cuTensorMapEncodeTiled failed");
+  return 0;
+}
+
 // gate_and_up.weight [2 f, d] as [f][gate, up][d]: a box holds 64 columns of gate and up rows in turn, 64 features.
 static int encode_tmap_pairs(void* out, const void* base, uint64_t f, uint64_t d) {
   EncodeTiledFn enc = get_encode();

@@ -96,10 +96,12 @@ enum {
   MOE_B200_WS_OFFSETS,    /* int32 [E+1]   start row of each expert in the sorted buffers */
   MOE_B200_WS_ROW_OF,     /* int32 [N,k]   sorted-buffer row of (token, slot) */
   MOE_B200_WS_PERM,       /* T [N*k, d]    tokens sorted by expert (model.py:248-253) */
-  MOE_B200_WS_H,          /* T [N*k, f]    gelu_tanh(gate)*up (model.py:180-182) */
+  MOE_B200_WS_H,          /* T [N*k, f]    gelu_tanh(gate)*up (model.py:180-182); fp32 calls of up to 2048 tokens and
+                           * 4096 rows: scratch of h and the sorted rows as bf16 parts */
   MOE_B200_WS_Y,          /* T [N*k, d]    expert outputs, sorted order (model.py:184) */
   MOE_B200_WS_PART,       /* float [splits, N*k, d] split-K partial sums of the small-N path
-                           * (present when N*k <= moe_b200_decode_max_rows(), bf16) */
+                           * (bf16 calls of up to 4096 rows; fp32 calls as above whose down product
+                           * is split over K) */
   MOE_B200_WS_NORM_W,     /* T [E,d]       gate.weight * norm weight (moe_b200_norm_fold) */
   MOE_B200_WS_NORM_C,     /* float [2E]    constants of the folded router */
   MOE_B200_WS_STATS,      /* float [N,2]   mean and 1/std of every row of x */

@@ -92,6 +92,53 @@ def test_fp32_routing_in_one_launch(cuda_device, N, d, E, k):
         assert torch.equal(m.last[name], disp[name]), name
 
 
+# Tokens in planes: one to 160 tokens a tile (and an expert of more), the down product whole and in two to eight ranges of K
+# that end early, boxes of 32 to 160 rows, widths that are no multiple of 32, 64 or 128.
+@pytest.mark.parametrize("N,d,f,E,k,special", [(1, 64, 264, 8, 2, ""), (7, 264, 1096, 4, 3, ""), (80, 512, 2048, 1, 1, ""),
+                                               (161, 72, 1024, 2, 1, ""), (160, 1032, 200, 2, 2, ""), (400, 264, 512, 3, 2, ""),
+                                               (2048, 128, 72, 17, 2, ""), (1300, 1024, 136, 8, 3, ""),
+                                               (50, 264, 1024, 4, 2, "inf"), (700, 512, 2048, 8, 2, "inf"),
+                                               (40, 264, 1024, 4, 2, "end"), (512, 512, 2048, 8, 2, "end")])
+def test_fp32_calls_on_planes(cuda_device, N, d, f, E, k, special):
+    """The whole call against the products that split their own activations, on the same routing: the products are the same,
+    the sums of the ranges of K are added in another order."""
+    params = synthetic.make_params(d, E, f, seed=N + f)
+    g = torch.Generator().manual_seed(N)
+    x = torch.randn(N, d, generator=g)
+    if special == "inf":
+        params["w1"][0, 9, 7], params["w2"][1, 11, 100], params["w1"][1, f + 2, 1] = 1e4, float("inf"), -float("inf")
+        params["w2"].view(torch.int32)[0, 13, 5] = 0x7F800001      # NaN whose upper half alone would be an infinity
+    if special == "end":
+        # h = 64 up: products of h and w2 whose first parts cancel while the others sum up to more than the largest number
+        top, near = 2.0 ** 127, 1 + 2.0 ** -7 - 2.0 ** -23
+        params["w1"].zero_(), params["b1"].zero_(), params["w2"].zero_()
+        params["b1"][:, :f] = 64.0
+        params["b1"][:, f:f + 256] = torch.tensor([1.9921875 * top, near * top, near * top, 0.03125 * top] * 64) / 64
+        params["w2"][:, ::2, :256] = torch.tensor([-1.0, near, near, -1.0] * 64)
+    m = build(params, d, E, f, k, torch.float32, cuda_device)
+    with torch.no_grad():
+        out, _ = m(x.to(cuda_device).view(1, N, d))
+    assert m.device_status() == 0
+    dp = helpers.device_params(params, torch.float32, cuda_device)
+    plan = helpers.Plan(dp["w1"], dp["b1"], dp["w2"], dp["b2"])
+    disp = helpers.dispatch(x.to(cuda_device), m.last["idx"], E)
+    _, y, status = helpers.experts(disp["perm"], disp["offsets"], plan)
+    assert status.cpu()[0] == 0
+    want = helpers.combine(y, disp["row_of"], m.last["w"]).cpu()
+    got = out.view(N, d).cpu()
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    ok = want.isfinite()
+    assert ok.any()
+    if special == "end":
+        # 256 sums of at most 2^128, each rounded, on both sides: 2^10 2^-24 2^127, where the result is 2^126
+        assert want[:, ::2].abs().max() > 1e37
+        assert (got[ok] - want[ok]).abs().max() <= 1.3e-4 * want[ok].abs().max()
+    else:
+        # sums of at most eight ranges and a read-out per 64 of K, each rounded to 2^-24
+        assert (got[ok].double() - want[ok].double()).norm() <= 5e-7 * want[ok].double().norm()
+
+
 @pytest.mark.parametrize("N,fold", [(1, False), (40, False), (2048, False), (2049, False), (300, True), (2049, True)])
 def test_fp32_tokens_of_nan(cuda_device, N, fold):
     """On both sides of 2048 tokens, with and without a folded LayerNorm: a token of NaN has no expert, its output is the
