@@ -1,6 +1,7 @@
 """Drop-in for the reference's ``Attention`` (model.py:59-152): same constructor, attribute
 and parameter names, ``state_dict`` layout and ``forward`` signature. The two Linears
-(fused QKV, output) and the head-gate Linear are plain library GEMMs; everything between
+(fused QKV, output) and the head-gate Linear are plain library GEMMs, for the rows of a few short
+sequences the library's own (``moe_b200_linear_rows``); everything between
 them — head split, shared KV heads, RoPE from the model's own table, scores, mask, softmax,
 the product with V and the sigmoid head gate — is one kernel of libmoe_b200
 (``moe_b200_attention``), so the [B, H, S, S] score tensor is never materialised.
@@ -78,6 +79,23 @@ class Attention(nn.Module):
             self._table = (key, pe.detach().to(device=device, dtype=torch.float32).contiguous())
         return self._table[1]
 
+    def _arguments(self, tensor, attention_mask, fine_tuning):
+        """What the native call takes: input, weights (merged ones when fine-tuning), table and mask."""
+        S, dev = tensor.shape[1], tensor.device
+        if fine_tuning:
+            wq, bq = self._merged_qkv.get(self.qkv, self.lora_qkv_a, self.lora_qkv_b, self.lora_scale)
+            wo, bo = self._merged_o.get(self.o, self.lora_o_a, self.lora_o_b, self.lora_scale)
+        else:
+            wq, bq, wo, bo = self.qkv.weight, self.qkv.bias, self.o.weight, self.o.bias
+        mask = attention_mask
+        if mask is not None:
+            if mask.numel() != S * S:
+                raise NotImplementedError("one additive [S, S] mask for the whole batch is supported")
+            if mask.dtype != torch.float32 or mask.device != dev or not mask.is_contiguous():
+                mask = mask.reshape(S, S).to(device=dev, dtype=torch.float32).contiguous()
+        return (tensor.contiguous(), wq, bq, self.gate.weight, self.gate.bias, wo, bo, self._pos_table(dev), mask, self.q_head,
+                self.kv_head, self.head_dim, self.scaler)
+
     def forward(self, tensor: torch.Tensor, attention_mask: torch.Tensor = None,
                 fine_tuning: bool = False) -> torch.Tensor:
         if not tensor.is_cuda or tensor.dtype != torch.bfloat16:
@@ -86,31 +104,47 @@ class Attention(nn.Module):
             raise NotImplementedError("the attention kernel has no backward pass; use torch.no_grad()")
         B, S, hid = tensor.shape
         dev = tensor.device
-        if fine_tuning:
-            wq, bq = self._merged_qkv.get(self.qkv, self.lora_qkv_a, self.lora_qkv_b, self.lora_scale)
-            wo, bo = self._merged_o.get(self.o, self.lora_o_a, self.lora_o_b, self.lora_scale)
-        else:
-            wq, bq, wo, bo = self.qkv.weight, self.qkv.bias, self.o.weight, self.o.bias
-        x = tensor.contiguous()
-        mask = attention_mask
-        if mask is not None:
-            if mask.numel() != S * S:
-                raise NotImplementedError("one additive [S, S] mask for the whole batch is supported")
-            if mask.dtype != torch.float32 or mask.device != dev or not mask.is_contiguous():
-                mask = mask.reshape(S, S).to(device=dev, dtype=torch.float32).contiguous()
-        table = self._pos_table(dev)
-        done = _host.attention(x, wq, bq, self.gate.weight, self.gate.bias, wo, bo, table, mask, self.q_head, self.kv_head,
-                               self.head_dim, self.scaler)
+        args = self._arguments(tensor, attention_mask, fine_tuning)
+        done = _host.attention(*args)
         if done is not None:
             return done
-        qkv = F.linear(x, wq, bq)
-        gate = F.linear(x, self.gate.weight, self.gate.bias)          # [B,S,q_head] logits (model.py:139)
+        x, wq, bq, wg, bg, wo, bo, table, mask = args[:9]
+        inner = self.q_head * self.head_dim
+        few = self._few_rows(args, B * S, hid, inner)
+        if few:
+            qkv, gate = _linear_rows(x, wq, bq, wg, bg)
+        else:
+            qkv = F.linear(x, wq, bq)
+            gate = F.linear(x, wg, bg)                                # [B,S,q_head] logits (model.py:139)
         mask_ptr = None if mask is None else mask.data_ptr()
         if table.shape[0] < S or table.shape[1] != 2 * self.head_dim:
             raise ValueError("the RoPE table is shorter than the sequence or has another head_dim")
-        out = torch.empty(B, S, self.q_head * self.head_dim, dtype=tensor.dtype, device=dev)
+        out = torch.empty(B, S, inner, dtype=tensor.dtype, device=dev)
         with torch.cuda.device(dev):
             check(lib.moe_b200_attention(qkv.data_ptr(), gate.data_ptr(), table.data_ptr(), mask_ptr, B, S,
                                          self.q_head, self.kv_head, self.head_dim, float(self.scaler),
                                          out.data_ptr(), _stream(dev)), "attention")
-        return F.linear(out, wo, bo)
+        return _linear_rows(out, wo, bo)[0] if few else F.linear(out, wo, bo)
+
+    def _few_rows(self, args, N, hid, inner):
+        """Whether the Linears go through moe_b200_linear_rows: the same answer as the native call's."""
+        x, wq, bq, wg, bg, wo, bo = args[:7]
+        rows = (self.q_head + 2 * self.kv_head) * self.head_dim
+        return (1 <= N <= lib.moe_b200_linear_rows_max() and hid % 8 == 0 and inner % 8 == 0 and self.head_dim == 64
+                and x.shape[1] <= 128 and x.data_ptr() % 16 == 0
+                and all(w.shape == (r, c) and w.is_contiguous() and w.data_ptr() % 16 == 0 and b is not None and b.numel() == r
+                        and b.is_contiguous() and all(p.dtype == torch.bfloat16 and p.device == x.device for p in (w, b))
+                        for w, b, r, c in ((wq, bq, rows, hid), (wg, bg, self.q_head, hid), (wo, bo, hid, inner))))
+
+
+def _linear_rows(x, w, b, w2=None, b2=None):
+    """x W^T + b, and with the second Linear its output too, by the library's kernel for few rows."""
+    N, K, dev = x.numel() // x.shape[-1], x.shape[-1], x.device
+    out = torch.empty(*x.shape[:-1], w.shape[0], dtype=x.dtype, device=dev)
+    out2 = None if w2 is None else torch.empty(*x.shape[:-1], w2.shape[0], dtype=x.dtype, device=dev)
+    ptr = lambda t: None if t is None else t.data_ptr()
+    with torch.cuda.device(dev):
+        check(lib.moe_b200_linear_rows(x.data_ptr(), w.data_ptr(), b.data_ptr(), w.shape[0], ptr(w2), ptr(b2),
+                                       0 if w2 is None else w2.shape[0], N, K, out.data_ptr(), ptr(out2), _stream(dev)),
+              "linear_rows")
+    return out, out2

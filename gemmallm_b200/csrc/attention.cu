@@ -53,8 +53,7 @@ __device__ __forceinline__ uint2 rope4(uint2 x, const float* __restrict__ pe) {
 // pos_emb [S][128] f32, mask [S][S + 8] f32 (optional).
 template <int S_TILES>   // ceil(S / 16), 1..8
 __global__ void __launch_bounds__(kWarpsAtt * 32)
-attention_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ gate,
-                 const float* __restrict__ pos_emb, const float* __restrict__ mask, int S, int H,
+attention_kernel(const __nv_bfloat16* qkv, const __nv_bfloat16* gate, const float* pos_emb, const float* mask, int S, int H,
                  int KV, float scaler, __nv_bfloat16* __restrict__ out) {
   constexpr int SP = S_TILES * 16;        // padded context
   constexpr int KP = HD + 8;              // K / Q row pitch (bf16): conflict-free fragment loads
@@ -79,32 +78,20 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __r
     for (int i = threadIdx.x; i < SP * 2 * HD / 4; i += blockDim.x) {
       const int r = i / (2 * HD / 4);
       reinterpret_cast<float4*>(sPE)[i] =
-          r < S ? __ldg(reinterpret_cast<const float4*>(pos_emb) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+          r < S ? reinterpret_cast<const float4*>(pos_emb)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   } else {      // a table that is a view at an odd place
-    for (int i = threadIdx.x; i < SP * 2 * HD; i += blockDim.x) sPE[i] = i < S * 2 * HD ? __ldg(pos_emb + i) : 0.f;
+    for (int i = threadIdx.x; i < SP * 2 * HD; i += blockDim.x) sPE[i] = i < S * 2 * HD ? pos_emb[i] : 0.f;
   }
   if (mask != nullptr)
     for (int i = threadIdx.x; i < SP * SP; i += blockDim.x) {
       const int r = i / SP, c = i - r * SP;
-      sM[r * MP + c] = (r < S && c < S) ? __ldg(mask + r * S + c) : (c < S ? 0.f : -INFINITY);
+      sM[r * MP + c] = (r < S && c < S) ? mask[r * S + c] : (c < S ? 0.f : -INFINITY);
     }
-  __syncthreads();
-  for (int i = threadIdx.x; i < SP * (HD / 4); i += blockDim.x) {
-    const int s = i / (HD / 4), c = (i - s * (HD / 4)) * 4;
-    uint2 k4 = make_uint2(0u, 0u), v4 = make_uint2(0u, 0u);
-    if (s < S) {
-      k4 = __ldg(reinterpret_cast<const uint2*>(base + (size_t)s * row_elems + (H + kvh) * HD + c));
-      v4 = __ldg(reinterpret_cast<const uint2*>(base + (size_t)s * row_elems + (H + KV + kvh) * HD + c));
-      k4 = rope4(k4, sPE + s * 2 * HD + c);
-    }
-    *reinterpret_cast<uint2*>(sK + s * KP + c) = k4;
-    const __nv_bfloat16* v = reinterpret_cast<const __nv_bfloat16*>(&v4);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) sVt[(c + q) * VP + s] = v[q];
-  }
-  __syncthreads();
-
+  // (table and mask are older than the kernel in front, which may still run where this one is its dependent; qkv and gate
+  // come from it: ordinary loads behind the wait)
+  pdl_wait();
+  pdl_launch_dependents();
   __nv_bfloat16* myQ = sQ + warp * 16 * KP;
   // A warp's work: (query head, 16-row tile) items, one in kWarpsAtt of the block's. The rows of
   // the next item and its gate values are requested before the products of the current one, so
@@ -121,8 +108,8 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __r
     for (int q = 0; q < 4; ++q) {
       const int s = mt * 16 + (lane >> 3) + 4 * q;
       const __nv_bfloat16* p = base + (size_t)s * row_elems + h * HD + lc;
-      raw[2 * q] = s < S ? __ldg(reinterpret_cast<const uint2*>(p)) : zero2;
-      raw[2 * q + 1] = s < S ? __ldg(reinterpret_cast<const uint2*>(p + 32)) : zero2;
+      raw[2 * q] = s < S ? __ldcg(reinterpret_cast<const uint2*>(p)) : zero2;
+      raw[2 * q + 1] = s < S ? __ldcg(reinterpret_cast<const uint2*>(p + 32)) : zero2;
     }
     const int r0 = mt * 16 + g;
     ga = r0 < S ? __bfloat162float(gate[((size_t)b * S + r0) * H + h]) : 0.f;
@@ -131,6 +118,22 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __r
   uint2 raw[8];
   float gate_a = 0.f, gate_b = 0.f;
   if (warp < items) fetch(warp, raw, gate_a, gate_b);
+  __syncthreads();
+  for (int i = threadIdx.x; i < SP * (HD / 4); i += blockDim.x) {
+    const int s = i / (HD / 4), c = (i - s * (HD / 4)) * 4;
+    uint2 k4 = make_uint2(0u, 0u), v4 = make_uint2(0u, 0u);
+    if (s < S) {
+      k4 = __ldcg(reinterpret_cast<const uint2*>(base + (size_t)s * row_elems + (H + kvh) * HD + c));
+      v4 = __ldcg(reinterpret_cast<const uint2*>(base + (size_t)s * row_elems + (H + KV + kvh) * HD + c));
+      k4 = rope4(k4, sPE + s * 2 * HD + c);
+    }
+    *reinterpret_cast<uint2*>(sK + s * KP + c) = k4;
+    const __nv_bfloat16* v = reinterpret_cast<const __nv_bfloat16*>(&v4);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sVt[(c + q) * VP + s] = v[q];
+  }
+  __syncthreads();
+
   for (int item = warp; item < items; item += kWarpsAtt) {
     {
       const int h = kvh * heads_per_kv + head0 + item / S_TILES, mt = item % S_TILES;
@@ -248,7 +251,7 @@ attention_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __r
 
 template <int ST>
 int launch_att(const void* qkv, const void* gate, const float* pos_emb, const float* mask, int B, int S,
-               int H, int KV, float scaler, void* out, cudaStream_t s) {
+               int H, int KV, float scaler, void* out, bool chained, cudaStream_t s) {
   constexpr int SP = ST * 16;
   const size_t smem = (size_t)(SP * (HD + 8) + HD * (SP + 8) + kWarpsAtt * 16 * (HD + 8)) * 2 +
                       (size_t)SP * 2 * HD * 4 + (mask != nullptr ? (size_t)SP * (SP + 8) * 4 : 0);
@@ -262,21 +265,23 @@ int launch_att(const void* qkv, const void* gate, const float* pos_emb, const fl
   const int64_t blocks = (int64_t)B * KV, heads = H / KV;
   const int64_t want = blocks < 2 * kNumSMs ? (2 * kNumSMs + blocks - 1) / blocks : 1;
   const dim3 grid((unsigned)blocks, (unsigned)(want < heads ? want : heads));
-  attention_kernel<ST><<<grid, kWarpsAtt * 32, smem, s>>>(
-      static_cast<const __nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(gate), pos_emb, mask, S,
-      H, KV, scaler, static_cast<__nv_bfloat16*>(out));
+  const __nv_bfloat16 *q = static_cast<const __nv_bfloat16*>(qkv), *gt = static_cast<const __nv_bfloat16*>(gate);
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
+  if (chained) {
+    MOE_CUDA_CHECK(launch_pdl(attention_kernel<ST>, grid, dim3(kWarpsAtt * 32), smem, s, q, gt, pos_emb, mask, S, H, KV,
+                              scaler, o));
+    return 0;
+  }
+  attention_kernel<ST><<<grid, kWarpsAtt * 32, smem, s>>>(q, gt, pos_emb, mask, S, H, KV, scaler, o);
   MOE_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
 
 }  // namespace
-}  // namespace moe
 
-using namespace moe;
 
-extern "C" int moe_b200_attention(const void* qkv, const void* gate, const float* pos_emb,
-                                  const float* mask, int64_t B, int S, int q_heads, int kv_heads,
-                                  int head_dim, float scaler, void* out, void* stream) {
+int launch_attention(const void* qkv, const void* gate, const float* pos_emb, const float* mask, int64_t B, int S, int q_heads,
+                     int kv_heads, int head_dim, float scaler, void* out, bool chained, cudaStream_t s) {
   if (head_dim != HD) return set_error(MOE_B200_ERR_UNSUPPORTED, "head_dim must be 64");
   if (S < 1 || S > kMaxS) return set_error(MOE_B200_ERR_UNSUPPORTED, "context must be in [1,128]");
   if (B < 0 || B > (1 << 24) || q_heads < 1 || kv_heads < 1 || q_heads % kv_heads != 0)
@@ -284,15 +289,25 @@ extern "C" int moe_b200_attention(const void* qkv, const void* gate, const float
   if (B == 0) return 0;
   if (!qkv || !gate || !pos_emb || !out) return set_error(MOE_B200_ERR_NULL, "NULL argument");
   if (!aligned16(qkv) || !aligned16(out)) return set_error(MOE_B200_ERR_ALIGN, "buffers must be 16-byte aligned");
-  cudaStream_t s = (cudaStream_t)stream;
   switch ((S + 15) / 16) {
-    case 1: return launch_att<1>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, s);
-    case 2: return launch_att<2>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, s);
-    case 3: return launch_att<3>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, s);
-    case 4: return launch_att<4>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, s);
-    case 5: return launch_att<5>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, s);
-    case 6: return launch_att<6>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, s);
-    case 7: return launch_att<7>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, s);
-    default: return launch_att<8>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, s);
+    case 1: return launch_att<1>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, chained, s);
+    case 2: return launch_att<2>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, chained, s);
+    case 3: return launch_att<3>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, chained, s);
+    case 4: return launch_att<4>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, chained, s);
+    case 5: return launch_att<5>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, chained, s);
+    case 6: return launch_att<6>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, chained, s);
+    case 7: return launch_att<7>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, chained, s);
+    default: return launch_att<8>(qkv, gate, pos_emb, mask, (int)B, S, q_heads, kv_heads, scaler, out, chained, s);
   }
+}
+
+}  // namespace moe
+
+using namespace moe;
+
+extern "C" int moe_b200_attention(const void* qkv, const void* gate, const float* pos_emb,
+                                  const float* mask, int64_t B, int S, int q_heads, int kv_heads,
+                                  int head_dim, float scaler, void* out, void* stream) {
+  return launch_attention(qkv, gate, pos_emb, mask, B, S, q_heads, kv_heads, head_dim, scaler, out, false,
+                          (cudaStream_t)stream);
 }

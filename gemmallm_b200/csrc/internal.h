@@ -58,4 +58,21 @@ int experts_backward_into(const void* x_sorted, const void* h, const int32_t* of
                           void* train_ws, size_t train_ws_bytes, const TrainGrads& grads, const LoraGrads* lora,
                           int32_t* status, void* stream);
 
+// The attention of a few short sequences (bf16, B S <= moe_b200_linear_rows_max()): QKV projection and head gate, on
+// LayerNorm(x) where norm_weight is given, the core of moe_b200_attention, the output projection, plus skip where given.
+// Three launches. Buffers: qkv [B S, (q + 2 kv) 64], gate [B S, q], core [B S, q 64]; x, out, skip [B S, hidden].
+struct AttentionRows {
+  const void *x, *norm_weight, *norm_bias;
+  float eps;
+  const void *wqkv, *bqkv, *wgate, *bgate, *wo, *bo;
+  const float *pos_emb, *mask;
+  const void* skip;
+  int64_t B;
+  int S, hidden, q_heads, kv_heads, head_dim;
+  float scaler;
+  void *qkv, *gate, *core, *out;
+};
+bool linear_rows_supported(int64_t N, int K, bool norm);
+int attention_rows(const AttentionRows& p, void* stream);
+
 }  // namespace moe

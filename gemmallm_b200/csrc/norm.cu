@@ -89,6 +89,7 @@ layernorm_rows_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
                       const T* __restrict__ beta, float eps, int64_t N, int d, T* __restrict__ out,
                       float* __restrict__ stats /* nullable [N][2] */) {
   pdl_wait();
+  pdl_launch_dependents();
   const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= N) return;

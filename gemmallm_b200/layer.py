@@ -8,7 +8,8 @@ in inference the second LayerNorm (model.py:298,312) is folded into the block's 
 dispatch kernels and the second skip connection (model.py:319) into its combine kernel, so
 neither is a pass over the activations of its own; the first LayerNorm runs the library's row
 kernel (``moe_b200_layernorm``). The attention's Linears and the first skip connection stay
-library code around ``moe_b200_attention``.
+library code around ``moe_b200_attention``, but for a few short sequences: there LayerNorm, QKV and head gate are one
+launch, the attention core the second, output Linear and skip connection the third (``csrc/linear_rows.cu``).
 """
 from __future__ import annotations
 
@@ -19,6 +20,17 @@ from . import _cabi, _host
 from ._cabi import check, lib
 from .attention import Attention
 from .moe import MOE, FeedForward, _stream
+
+
+_FEW_ROWS = lib.moe_b200_linear_rows_max()
+_module = nn.modules.module
+
+
+def _watched(m: nn.Module) -> bool:
+    """Hooks that a call of the module would run."""
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                or _module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks
+                or _module._global_backward_pre_hooks)
 
 
 def _layernorm(norm: nn.LayerNorm, x: torch.Tensor) -> torch.Tensor:
@@ -64,11 +76,23 @@ class LLMLayer(nn.Module):
                                    lora_rank=lora_rank, lora_alpha=lora_alpha)
         self.device = device
 
+    def _attend(self, tensor, attention_mask, fine_tuning):
+        """First LayerNorm, attention and first skip connection (model.py:297-308): in three launches for a few short
+        sequences, else as four steps, whose results are the same to the bit at those sizes."""
+        mqa, norm = self.mqa, self.norm1
+        if (type(mqa) is Attention and "forward" not in mqa.__dict__ and not _watched(mqa) and tensor.is_cuda
+                and tensor.dtype == torch.bfloat16 and tensor.dim() == 3
+                and tensor.shape[0] * tensor.shape[1] <= _FEW_ROWS and norm.weight is not None and norm.bias is not None
+                and not (torch.is_grad_enabled() and (tensor.requires_grad or mqa.qkv.weight.requires_grad))):
+            done = _host.attention(*mqa._arguments(tensor, attention_mask, fine_tuning), norm.weight, norm.bias,
+                                   float(norm.eps))
+            if done is not None:
+                return done
+        out = mqa(_layernorm(norm, tensor), attention_mask=attention_mask, fine_tuning=fine_tuning)
+        return out + tensor                                    # model.py:308
+
     def forward(self, tensor: torch.Tensor, attention_mask: torch.Tensor = None, fine_tuning: bool = False):
-        skip_connection = tensor
-        tensor = _layernorm(self.norm1, tensor)
-        tensor = self.mqa(tensor, attention_mask=attention_mask, fine_tuning=fine_tuning)
-        tensor = tensor + skip_connection                      # model.py:308
+        tensor = self._attend(tensor, attention_mask, fine_tuning)
         if self.use_moe:
             if self.moe.training:
                 # training mode has no backward pass for the folded LayerNorm

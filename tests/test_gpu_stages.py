@@ -312,6 +312,31 @@ def test_lora_merge_by_units(cuda_device, out_f, in_f, rank):
     test_lora_merge(cuda_device, out_f, in_f, rank, torch.bfloat16)
 
 
+# blocks of 16 rows and 16 or 32 tokens that end early, K that ends within a chunk of 32, a round of chunks more, one Linear
+# and two, the most tokens there can be
+@pytest.mark.parametrize("N,K,r,r2", [(1, 8, 1, 0), (15, 40, 17, 2), (16, 1024, 1152, 16), (17, 1032, 72, 5), (33, 264, 2400, 1),
+                                      (160, 3080, 48, 31)])
+def test_linear_rows(cuda_device, N, K, r, r2):
+    g = torch.Generator().manual_seed(N + K)
+    rnd = lambda *s: (torch.randn(*s, generator=g) / 4).to(torch.bfloat16)
+    x, W, b, W2, b2 = rnd(N, K), rnd(r, K), rnd(r), rnd(max(r2, 1), K), rnd(max(r2, 1))
+    dev = [t.to(cuda_device) for t in (x, W, b, W2, b2)]
+    out = torch.full((N + 1, r), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    out2 = torch.full((N + 1, max(r2, 1)), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    ptr = [t.data_ptr() for t in dev]
+    check(lib.moe_b200_linear_rows(ptr[0], ptr[1], ptr[2], r, ptr[3], ptr[4], r2, N, K, out.data_ptr(), out2.data_ptr(),
+                                   helpers.stream(cuda_device)), "linear_rows")
+    for got, w, bias, wanted in ((out, W, b, True), (out2, W2, b2, r2 > 0)):
+        assert (got[N:] == 7.0).all()
+        if wanted:
+            want = x.double() @ w.double().t() + bias.double()
+            # K products of size 1/16 in fp32, in whatever order: 2^-24 K of their sum of sizes; half an ulp of bf16
+            slack = 2.0 ** -24 * K * (x.double().abs() @ w.double().abs().t() + bias.double().abs())
+            assert ((got[:N].cpu().double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()
+        else:
+            assert (got == 7.0).all()
+
+
 # edges of the fp32 token tiles (16 and 160 tokens) and of the read-outs (64 and 256 of K), whole and with K over clusters
 # of two, four and eight CTAs, more tiles than SMs
 @pytest.mark.parametrize("rows,d,f", [([15, 16, 17, 159], 512, 2048), ([160, 161, 0, 321], 1024, 512), ([7], 1024, 136),

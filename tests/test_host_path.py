@@ -847,6 +847,39 @@ def test_attention_native_and_python_paths_agree(cuda_device, monkeypatch, B, S,
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("B,S,hidden,heads,kv,ft", [(1, 1, 64, 2, 1, False), (1, 16, 200, 4, 2, True), (17, 1, 1024, 16, 1, False),
+                                                    (1, 65, 1032, 2, 2, False), (5, 32, 2048, 4, 1, False),
+                                                    (7, 23, 256, 2, 1, False)])
+def test_attention_of_a_layer_in_one_call(cuda_device, B, S, hidden, heads, kv, ft):
+    """LayerNorm, attention and skip connection in three launches, and step by step: the same to the bit, on both sides of
+    the most rows there can be. What the one call cannot do is left to the steps."""
+    torch.manual_seed(S)
+    layer = LLMLayer(hidden, 64, heads, kv, Table(128, 64), expansion_factor=1, use_moe=False, device="cuda")
+    layer = layer.to(device=cuda_device, dtype=DT).eval()
+    layer.mqa.embedding.float()
+    torch.nn.init.normal_(layer.norm1.weight)
+    torch.nn.init.normal_(layer.norm1.bias)
+    x = torch.randn(B, S, hidden, generator=torch.Generator().manual_seed(B)).to(device=cuda_device, dtype=DT)
+    mask = torch.full((S, S), float("-inf"), device=cuda_device).triu(1)
+    with torch.no_grad():
+        want = layer.mqa(_layernorm(layer.norm1, x), mask, ft) + x
+        args = (*layer.mqa._arguments(x, mask, ft), layer.norm1.weight, layer.norm1.bias, layer.norm1.eps)
+        one = _host.attention(*args)
+        assert (one is None) == (B * S > 160)
+        if one is not None:
+            assert torch.equal(one, want)
+        assert torch.equal(layer._attend(x, mask, ft), want)
+        seen = []
+        handle = layer.mqa.register_forward_hook(lambda *a: seen.append(a))
+        assert torch.equal(layer._attend(x, mask, ft), want) and len(seen) == 1
+        handle.remove()
+        odd = torch.empty(x.numel() + 1, device=cuda_device, dtype=DT)[1:].view_as(x).copy_(x)
+        assert _host.attention(odd, *args[1:]) is None
+        assert _host.attention(*args[:13], layer.norm1.weight[:8], *args[14:]) is None
+    assert _host.attention(*args) is None                                   # gradients are wanted
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [DT, torch.float32])
 def test_layernorm_native_and_left_alone(cuda_device, dtype):
     norm = torch.nn.LayerNorm(72).to(device=cuda_device, dtype=dtype)
