@@ -1,7 +1,7 @@
 """Drop-in for the reference's ``Attention`` (model.py:59-152): same constructor, attribute
-and parameter names, ``state_dict`` layout and ``forward`` signature. The two Linears
-(fused QKV, output) and the head-gate Linear are plain library GEMMs, for the rows of a few short
-sequences the library's own (``moe_b200_linear_rows``); everything between
+and parameter names, ``state_dict`` layout and ``forward`` signature. The fused QKV Linear and the
+head gate are one launch (``moe_b200_linear_rows``), the output Linear another (torch's Linears where sizes or
+places are not those it takes: a number of heads that is no multiple of 8, from 129 rows on); everything between
 them — head split, shared KV heads, RoPE from the model's own table, scores, mask, softmax,
 the product with V and the sigmoid head gate — is one kernel of libmoe_b200
 (``moe_b200_attention``), so the [B, H, S, S] score tensor is never materialised.
@@ -70,7 +70,16 @@ class Attention(nn.Module):
             self.multi_query_attention = False
         self.gate = nn.Linear(hidden_dim, q_head)
         self._merged_qkv, self._merged_o = _MergedLinear(), _MergedLinear()
-        self._table = None
+        self._table, self._status = None, None
+
+    def _status_words(self, device):
+        if self._status is None or self._status.device != device:
+            self._status = torch.zeros(16, dtype=torch.int32, device=device)
+        return self._status
+
+    def device_status(self) -> int:
+        """Status word of the calls so far (0 = ok; see moe_b200.h); synchronises."""
+        return 0 if self._status is None else int(self._status[0])
 
     def _pos_table(self, device):
         pe = self.embedding.pos_emb
@@ -94,7 +103,7 @@ class Attention(nn.Module):
             if mask.dtype != torch.float32 or mask.device != dev or not mask.is_contiguous():
                 mask = mask.reshape(S, S).to(device=dev, dtype=torch.float32).contiguous()
         return (tensor.contiguous(), wq, bq, self.gate.weight, self.gate.bias, wo, bo, self._pos_table(dev), mask, self.q_head,
-                self.kv_head, self.head_dim, self.scaler)
+                self.kv_head, self.head_dim, self.scaler, self._status_words(dev))
 
     def forward(self, tensor: torch.Tensor, attention_mask: torch.Tensor = None,
                 fine_tuning: bool = False) -> torch.Tensor:
@@ -110,9 +119,9 @@ class Attention(nn.Module):
             return done
         x, wq, bq, wg, bg, wo, bo, table, mask = args[:9]
         inner = self.q_head * self.head_dim
-        few = self._few_rows(args, B * S, hid, inner)
-        if few:
-            qkv, gate = _linear_rows(x, wq, bq, wg, bg)
+        own = self._own_linears(args, B * S, hid, inner)
+        if own:
+            qkv, gate = _linear_rows(args[13], x, wq, bq, wg, bg)
         else:
             qkv = F.linear(x, wq, bq)
             gate = F.linear(x, wg, bg)                                # [B,S,q_head] logits (model.py:139)
@@ -124,27 +133,29 @@ class Attention(nn.Module):
             check(lib.moe_b200_attention(qkv.data_ptr(), gate.data_ptr(), table.data_ptr(), mask_ptr, B, S,
                                          self.q_head, self.kv_head, self.head_dim, float(self.scaler),
                                          out.data_ptr(), _stream(dev)), "attention")
-        return _linear_rows(out, wo, bo)[0] if few else F.linear(out, wo, bo)
+        return _linear_rows(args[13], out, wo, bo)[0] if own else F.linear(out, wo, bo)
 
-    def _few_rows(self, args, N, hid, inner):
+    def _own_linears(self, args, N, hid, inner):
         """Whether the Linears go through moe_b200_linear_rows: the same answer as the native call's."""
         x, wq, bq, wg, bg, wo, bo = args[:7]
-        rows = (self.q_head + 2 * self.kv_head) * self.head_dim
-        return (1 <= N <= lib.moe_b200_linear_rows_max() and hid % 8 == 0 and inner % 8 == 0 and self.head_dim == 64
-                and x.shape[1] <= 128 and x.data_ptr() % 16 == 0
+        rows, many = (self.q_head + 2 * self.kv_head) * self.head_dim, N > lib.moe_b200_linear_rows_max()
+        return (1 <= N <= 1 << 28 and hid % 8 == 0 and self.head_dim == 64 and self.q_head % self.kv_head == 0
+                and x.shape[1] <= 128 and x.data_ptr() % 16 == 0 and not (many and self.q_head % 8 != 0)
                 and all(w.shape == (r, c) and w.is_contiguous() and w.data_ptr() % 16 == 0 and b is not None and b.numel() == r
-                        and b.is_contiguous() and all(p.dtype == torch.bfloat16 and p.device == x.device for p in (w, b))
+                        and b.is_contiguous() and not (many and b.data_ptr() % 16 != 0)
+                        and all(p.dtype == torch.bfloat16 and p.device == x.device for p in (w, b))
                         for w, b, r, c in ((wq, bq, rows, hid), (wg, bg, self.q_head, hid), (wo, bo, hid, inner))))
 
 
-def _linear_rows(x, w, b, w2=None, b2=None):
-    """x W^T + b, and with the second Linear its output too, by the library's kernel for few rows."""
+def _linear_rows(status, x, w, b, w2=None, b2=None):
+    """x W^T + b, and with the second Linear its output too, by the library's kernels."""
     N, K, dev = x.numel() // x.shape[-1], x.shape[-1], x.device
     out = torch.empty(*x.shape[:-1], w.shape[0], dtype=x.dtype, device=dev)
     out2 = None if w2 is None else torch.empty(*x.shape[:-1], w2.shape[0], dtype=x.dtype, device=dev)
     ptr = lambda t: None if t is None else t.data_ptr()
     with torch.cuda.device(dev):
         check(lib.moe_b200_linear_rows(x.data_ptr(), w.data_ptr(), b.data_ptr(), w.shape[0], ptr(w2), ptr(b2),
-                                       0 if w2 is None else w2.shape[0], N, K, out.data_ptr(), ptr(out2), _stream(dev)),
+                                       0 if w2 is None else w2.shape[0], N, K, out.data_ptr(), ptr(out2), status.data_ptr(),
+                                       _stream(dev)),
               "linear_rows")
     return out, out2

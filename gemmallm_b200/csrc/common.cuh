@@ -419,15 +419,16 @@ int launch_decode_tiny(const void* x, const void* Wg, const void* bg, int64_t N,
 int launch_experts_gemv(const void* perm, const int32_t* offsets, const void* plan, int64_t M, int d,
                         int f, int E, int ksplit, void* h, float* part, cudaStream_t s);
 
-// ---- linear_rows.cu, attention.cu ----
-// bf16 Linears on a few rows: out [N, rows] = x W^T + b, W [rows, K]; rows = 0: none. With gamma and beta on LayerNorm(x);
-// skip [N, first.rows] is added to the first one's rounded output. chained: no kernel that may still run writes weights or
-// biases.
+// ---- linear_rows.cu, experts_tc2.cu, attention.cu ----
+// bf16 Linears: out [N, rows] = x W^T + b, W [rows, K]; rows = 0: none. skip [N, first.rows] is added to the first one's
+// rounded output. Up to kLinearRowsMax rows of x: with gamma and beta on LayerNorm(x); chained: no kernel that may still run
+// writes weights or biases. As tiles of the tensor cores: all buffers 16-byte aligned, rows multiples of 8.
 struct LinearRows { const void *W, *b; void* out; int rows; };
-constexpr int64_t kLinearRowsMax = 160;
-bool linear_rows_supported(int64_t N, int K, bool norm);
+constexpr int64_t kLinearRowsMax = 128;
 int launch_linear_rows(const void* x, const void* gamma, const void* beta, float eps, const LinearRows& first,
                        const LinearRows& second, const void* skip, int64_t N, int K, bool chained, cudaStream_t s);
+int launch_linear_tiles(const void* x, const LinearRows& first, const LinearRows& second, const void* skip, int64_t N, int K,
+                        int32_t* status, cudaStream_t s);
 // chained: launched as a dependent of the kernel that writes qkv and gate, which waited for what was before it
 int launch_attention(const void* qkv, const void* gate, const float* pos_emb, const float* mask, int64_t B, int S, int q_heads,
                      int kv_heads, int head_dim, float scaler, void* out, bool chained, cudaStream_t s);

@@ -36,6 +36,12 @@
 // then: a cluster has one tile) and each adds up and stores 256 / SPLIT columns, in the order of the ranges. (128-column
 // tiles instead gained nothing when the load loop still set the pace, 640 clk a step whatever the columns; they have not
 // been measured since it does not.)
+//
+// kLinear, kLinearSkip: the Linears around the attention core (model.py:104, 139, 150), QKV and head gate as one product, the
+// output Linear with the skip connection behind it (model.py:308), whose pieces are asked for before a tile's accumulator is
+// awaited (in the epilogue's stores they made it the bound: 100 us, now 60 to 75). 32768 tokens, d 1024, 16 heads, one KV
+// head: QKV and gate 75 us as two library products, 56 here; output Linear and addition 87, 65. A decoder layer, 8 experts:
+// 512 tokens 109.7 -> 103.1 us, 1024 128.4 -> 119.5, 4096 279 -> 267, 6528 393 -> 388, 32768 1729 -> 1680 (two runs each).
 #include <cuda.h>
 #include "common.cuh"
 #include "tc_ptx.cuh"
@@ -71,7 +77,33 @@ enum Kind {
   kDx,           // out = A B, B [K, Nout] as it lies in memory
   kDhGeglu,      // dh = dy W2 as kDx, times the derivatives of h in the epilogue
   kDhGegluBf16,  // from pre-activations and mask, with dh rounded to bf16 and the column sums over rounded values (LoRA steps)
-  kWgrad         // out_e [Ra, Nout] = A[rows of e]^T B[rows of e]
+  kWgrad,        // out_e [Ra, Nout] = A[rows of e]^T B[rows of e]
+  kLinear,       // one group of rows, one or two weights: out = A W^T + b of both, column after column (LinearArgs)
+  kLinearSkip    // ... of one, plus the skip connection
+};
+// The Linears around the attention core. 128 columns, a CTA's share of a tile's weights and an epilogue warp's of its
+// columns, belong to one of the two.
+struct LinearArgs {
+  const __nv_bfloat16* bias[2];
+  __nv_bfloat16* out[2];       // [rows, cols]
+  int cols[2];
+  int rows;
+  const __nv_bfloat16* skip;   // kLinearSkip: [rows, cols[0]]
+  __host__ __device__ int halves(int i) const { return (cols[i] + 127) / 128; }
+  // (no index: parameters that are indexed are copied to local memory)
+  __device__ __forceinline__ const __nv_bfloat16* bias_of(int i) const { return i ? bias[1] : bias[0]; }
+  __device__ __forceinline__ __nv_bfloat16* out_of(int i) const { return i ? out[1] : out[0]; }
+  __device__ __forceinline__ int cols_of(int i) const { return i ? cols[1] : cols[0]; }
+};
+// Where the 128 columns `half` of the tiles lie.
+struct LinearHalf {
+  int which, col, limit;       // limit: columns of the output; 0: none of these exist
+  __device__ __forceinline__ LinearHalf(const LinearArgs& la, int half) {
+    const int h0 = la.halves(0);
+    which = half < h0 || la.cols[1] == 0 ? 0 : 1;
+    col = (which ? half - h0 : half) * 128;
+    limit = col < la.cols_of(which) ? la.cols_of(which) : 0;
+  }
 };
 template <int KIND>
 struct Traits {
@@ -80,6 +112,7 @@ struct Traits {
   static constexpr bool GEGLU = KIND == kGeglu || TRAIN;
   static constexpr bool COLS = KIND == kWgrad;
   static constexpr bool DH = KIND == kDhGeglu || KIND == kDhGegluBf16;
+  static constexpr bool LIN = KIND == kLinear || KIND == kLinearSkip;
   static constexpr bool A_MN = COLS;
   static constexpr bool B_MN = KIND == kDx || DH || COLS;
   // The training epilogues do 10 to 20 instructions per accumulator element and move as much again as the
@@ -137,7 +170,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
                         const int32_t* __restrict__ offsets,
                         const void* const* __restrict__ bias_ptrs, int E, int K, int Nout,
                         __nv_bfloat16* __restrict__ out, const EpScatter sc, const TrainArgs tr,
-                        const EpSync sy, int Ra, int32_t* __restrict__ status) {
+                        const EpSync sy, int Ra, const LinearArgs la, int32_t* __restrict__ status) {
   using T = Traits<KIND>;
   constexpr bool GEGLU = T::GEGLU, COLS = T::COLS, A_MN = T::A_MN, B_MN = T::B_MN;
   constexpr int kStages = T::kStages, kEpiWarps = T::kEpiWarps;
@@ -153,7 +186,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  static_assert(SPLIT == 1 || KIND == kPlain || KIND == kDx, "kinds with a split form");
+  static_assert(SPLIT == 1 || KIND == kPlain || KIND == kDx || T::LIN, "kinds with a split form");
   static_assert(SPLIT == 1 || BM * kPartPitch * 4 <= kStages * kStageBytes, "the partial tile reuses the stages");
   const uint32_t rank = cluster_ctarank();
   const uint32_t cta = rank & 1u;           // 0 = even CTA: issues the MMAs, owns full/tmem_empty
@@ -162,7 +195,7 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int pair = blockIdx.x / (2 * SPLIT);
   const int num_pairs = gridDim.x / (2 * SPLIT);
   constexpr int kTileN = GEGLU ? BN / 2 : BN;
-  const int n_tiles = (Nout + kTileN - 1) / kTileN;
+  const int n_tiles = T::LIN ? (la.halves(0) + la.halves(1) + 1) / 2 : (Nout + kTileN - 1) / kTileN;
   const int k_blocks_all = (K + BK - 1) / BK;
   const int k_blocks_per = (k_blocks_all + SPLIT - 1) / SPLIT;
   const int kb_first = SPLIT > 1 ? (int)(rank >> 1) * k_blocks_per : 0;       // this pair's range of K
@@ -200,11 +233,11 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (sy.wait_flags != nullptr) asm volatile("fence.proxy.async;" ::: "memory");
   if (threadIdx.x == 0) {
     int acc = 0;
-    int beg = offsets[0];
+    int beg = T::LIN ? 0 : offsets[0];
     ctl->offsets[0] = beg;
     for (int e = 0; e < E; ++e) {
       ctl->tile_start[e] = acc;
-      const int end = offsets[e + 1];
+      const int end = T::LIN ? la.rows : offsets[e + 1];
       ctl->offsets[e + 1] = end;
       acc += (COLS ? m_tiles_cols : (end - beg + kPairRows - 1) / kPairRows) * n_tiles;
       beg = end;
@@ -232,9 +265,14 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int local = t - ctl->tile_start[e];
         const int mt = local / n_tiles, nt = local - mt * n_tiles;
         const int row0 = (COLS ? 0 : ctl->offsets[e]) + mt * kPairRows + (int)cta * BM;
-        const int brow = GEGLU ? (cta == 0 ? nt * kTileN : Nout + nt * kTileN)
-                               : nt * kTileN + (int)cta * (BN / 2);
+        int brow = GEGLU ? (cta == 0 ? nt * kTileN : Nout + nt * kTileN)
+                         : nt * kTileN + (int)cta * (BN / 2);
         const CUtensorMap* tb = COLS ? &tmap_bc : tmap_b + e;
+        if constexpr (T::LIN) {
+          const LinearHalf lh(la, nt * 2 + (int)cta);
+          tb = lh.which ? &tmap_h : &tmap_bc;
+          brow = lh.col;
+        }
         const int k0 = COLS ? ctl->offsets[e] : 0;
         const int k_rows = COLS ? ctl->offsets[e + 1] - k0 : 0;
         const int k_blocks = COLS ? (k_rows + BK - 1) / BK : k_blocks_rows;
@@ -443,6 +481,12 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
         for (int c = 0; c < 4; ++c)
           keep[c] = GegluBwd::mask_bits(tr, row_warp + lane, lane < rows, n0 + c * 64 + part * 16, Nout);
       }
+      uint4 skip[KIND == kLinearSkip ? 2 : 1][8];
+      if constexpr (KIND == kLinearSkip) {
+        const LinearHalf lh(la, nt * 2 + part);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) load_skip64(skip[q], la.skip, row_warp, rows, la.cols[0], lh.col + q * 64, lh.limit, lane);
+      }
       ok = mbar_wait(&ctl->tmem_full[a], acc_phase, &ctl->abort, status, 34);
       if (!T::DH && !ok) break;
       tc_fence_after();
@@ -514,6 +558,11 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
           for (int q = 0; q < 32; q += 4)
             *reinterpret_cast<uint4*>(mine + c + q) = make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]);
         }
+      } else if constexpr (T::LIN) {
+        const LinearHalf lh(la, nt * 2 + part);
+        store_tile<false, false, KIND == kLinearSkip>(
+            taddr, row_cta + r, row_cta + r < row_end, lh.col - part * 128, lh.limit, la.bias_of(lh.which), la.out_of(lh.which), sc,
+            extra + (warp - 2) * kStgBytes, lane, part, release, la.cols_of(lh.which), skip);
       } else {
         store_tile<GEGLU, KIND == kScatter>(taddr, row_cta + r, row_cta + r < row_end, n0, Nout, bias, out_e, sc,
                                             extra + (warp - 2) * kStgBytes, lane, part, release);
@@ -535,11 +584,23 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int row_cta = ctl->offsets[e] + mt * kPairRows + (int)cta * BM;
       const int rows = min(BM, ctl->offsets[e + 1] - row_cta);
       const __nv_bfloat16* bias = bias_ptrs != nullptr ? static_cast<const __nv_bfloat16*>(bias_ptrs[e]) : nullptr;
+      __nv_bfloat16* to = out;
+      int width = Nout;
       constexpr int kPieces = BN / SPLIT / 8;          // of eight columns, per row
       const int c0 = (int)(rank >> 1) * (BN / SPLIT);
       for (int i = threadIdx.x; i < rows * kPieces; i += T::kThreads) {
-        const int rr = i / kPieces, c = c0 + (i % kPieces) * 8, n = nt * kTileN + c;
-        if (n >= Nout) continue;
+        const int rr = i / kPieces, c = c0 + (i % kPieces) * 8;
+        int n = nt * kTileN + c;
+        if constexpr (T::LIN) {
+          const LinearHalf lh(la, nt * 2 + (c >> 7));
+          n = lh.col + (c & 127);
+          if (n >= lh.limit) continue;
+          bias = la.bias_of(lh.which);
+          to = la.out_of(lh.which);
+          width = la.cols_of(lh.which);
+        } else if (n >= Nout) {
+          continue;
+        }
         const uint32_t at = smem_u32(smem) + (uint32_t)(rr * kPartPitch + c) * 4;
         float o[8] = {};
 #pragma unroll
@@ -559,7 +620,14 @@ grouped_gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
           for (int q = 0; q < 8; ++q) o[q] += b[q];
         }
-        store8(out + (int64_t)(row_cta + rr) * Nout + n, o);
+        const int64_t at_out = (int64_t)(row_cta + rr) * width + n;
+        if constexpr (KIND == kLinearSkip) {
+          float k[8];
+          load8(la.skip + at_out, k);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) o[q] = __bfloat162float(__float2bfloat16_rn(o[q])) + k[q];
+        }
+        store8(to + at_out, o);
       }
     }
   }
@@ -589,7 +657,8 @@ template <int KIND, int SPLIT = 1>
 int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_bc, const void* tmap_b, const int32_t* offsets,
                 const void* const* bias, int E, int K, int Nout, void* out, const EpScatter& sc,
                 const TrainArgs& tr, const EpSync& sy, int Ra, int32_t* status, int sms, cudaStream_t s,
-                const CUtensorMap* tm_h = nullptr, const CUtensorMap* tm_gu = nullptr, int64_t max_tiles = 0) {
+                const CUtensorMap* tm_h = nullptr, const CUtensorMap* tm_gu = nullptr, int64_t max_tiles = 0,
+                const LinearArgs& la = {}) {
   static PerDeviceOnce once;
   auto fn = grouped_gemm_tc2_kernel<KIND, SPLIT>;
   constexpr size_t smem = smem_bytes<KIND>();
@@ -600,7 +669,7 @@ int launch_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_bc, const void* t
   MOE_CUDA_CHECK(launch_pdl_cluster(fn, dim3(grid), dim3(Traits<KIND>::kThreads), 2 * SPLIT, smem, s, tm_a, tm_bc,
                                     tm_h != nullptr ? *tm_h : tm_a, tm_gu != nullptr ? *tm_gu : tm_a,
                                     static_cast<const CUtensorMap*>(tmap_b), offsets, bias, E, K, Nout,
-                                    static_cast<__nv_bfloat16*>(out), sc, tr, sy, Ra, status));
+                                    static_cast<__nv_bfloat16*>(out), sc, tr, sy, Ra, la, status));
   return 0;
 }
 
@@ -704,6 +773,52 @@ int launch_grouped_dx(const void* A, int64_t M, int K, const void* tmaps_b, cons
                                sms, s, nullptr, nullptr, max_tiles(M, E, Nout));
   return launch_pair<kDx>(tm_a, tm_a, tmaps_b, offsets, nullptr, E, K, Nout, out, none, eval, nosync, 0, status, sms,
                           s);
+}
+
+namespace {
+template <int KIND>
+int linear_tiles(const CUtensorMap& a, const CUtensorMap& w0, const CUtensorMap& w1, int64_t N, int K, const LinearArgs& la,
+                 int32_t* status, int sms, cudaStream_t s) {
+  const int cols = (la.halves(0) + la.halves(1)) * 128;
+  const EpScatter none = {};
+  const TrainArgs eval = {};
+  const EpSync nosync = {};
+  const int64_t tiles = max_tiles(N, 1, cols);
+  switch (k_splits(N, 1, K, cols)) {
+    case 4: return launch_pair<KIND, 4>(a, w0, nullptr, nullptr, nullptr, 1, K, cols, nullptr, none, eval, nosync, 0, status,
+                                        sms, s, &w1, nullptr, tiles, la);
+    case 2: return launch_pair<KIND, 2>(a, w0, nullptr, nullptr, nullptr, 1, K, cols, nullptr, none, eval, nosync, 0, status,
+                                        sms, s, &w1, nullptr, tiles, la);
+    default: return launch_pair<KIND, 1>(a, w0, nullptr, nullptr, nullptr, 1, K, cols, nullptr, none, eval, nosync, 0, status,
+                                         sms, s, &w1, nullptr, 0, la);
+  }
+}
+}  // namespace
+
+// All buffers 16-byte aligned, K and the numbers of rows of W multiples of 8.
+int launch_linear_tiles(const void* x, const LinearRows& first, const LinearRows& second, const void* skip, int64_t N, int K,
+                        int32_t* status, cudaStream_t s) {
+  if (N == 0) return 0;
+  alignas(64) CUtensorMap a, w0, w1;
+  int rc = encode_tmap_2d(&a, x, (uint64_t)N, (uint64_t)K, BM);
+  if (!rc) rc = encode_tmap_2d(&w0, first.W, (uint64_t)first.rows, (uint64_t)K, BN / 2);
+  if (!rc && second.rows > 0) rc = encode_tmap_2d(&w1, second.W, (uint64_t)second.rows, (uint64_t)K, BN / 2);
+  if (rc) return rc;
+  if (second.rows == 0) w1 = w0;
+  int sms = 0;
+  rc = sm_count(&sms);
+  if (rc) return rc;
+  LinearArgs la = {};
+  int i = 0;
+  for (const LinearRows* l : {&first, &second}) {
+    la.bias[i] = static_cast<const __nv_bfloat16*>(l->b);
+    la.out[i] = static_cast<__nv_bfloat16*>(l->out);
+    la.cols[i++] = l->rows;
+  }
+  la.rows = (int)N;
+  la.skip = static_cast<const __nv_bfloat16*>(skip);
+  return skip != nullptr ? linear_tiles<kLinearSkip>(a, w0, w1, N, K, la, status, sms, s)
+                         : linear_tiles<kLinear>(a, w0, w1, N, K, la, status, sms, s);
 }
 
 int launch_grouped_wgrad(const void* A, const void* B, int64_t M, int Ra, int Rb, const int32_t* offsets, void* out,

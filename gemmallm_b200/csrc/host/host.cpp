@@ -1264,59 +1264,76 @@ bool plain_call() {
          !at::autocast::is_autocast_enabled(at::kCUDA);
 }
 
-// attention(x, qkv weight, bias, gate weight, bias, o weight, bias, table, mask or None, q heads, kv heads, head_dim, scaler
-//           [, norm weight, bias, eps]). With the LayerNorm: on its output, and x is added (the skip connection); only for the
-// few rows that moe_b200_linear_rows takes, None for more.
+// attention(x, qkv weight, bias, gate weight, bias, o weight, bias, table, mask or None, q heads, kv heads, head_dim, scaler,
+//           status [, norm weight, bias, eps]). With the LayerNorm: on its output, and x is added (the skip connection); None
+// where attention_supported() says no.
 PyObject* host_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 13 && nargs != 16) {
-    PyErr_SetString(PyExc_TypeError, "attention() takes 13 or 16 arguments");
+  if (nargs != 14 && nargs != 17) {
+    PyErr_SetString(PyExc_TypeError, "attention() takes 14 or 17 arguments");
     return nullptr;
   }
-  const bool masked = args[8] != Py_None, layer = nargs == 16;
+  const bool masked = args[8] != Py_None, layer = nargs == 17;
   for (int i = 0; i < (masked ? 9 : 8); ++i)
     if (!THPVariable_CheckExact(args[i])) Py_RETURN_NONE;
-  if (layer && (!THPVariable_CheckExact(args[13]) || !THPVariable_CheckExact(args[14]))) Py_RETURN_NONE;
+  if (!THPVariable_CheckExact(args[13])) Py_RETURN_NONE;
+  if (layer && (!THPVariable_CheckExact(args[14]) || !THPVariable_CheckExact(args[15]))) Py_RETURN_NONE;
   const long heads = PyLong_AsLong(args[9]), kv = PyLong_AsLong(args[10]), hd = PyLong_AsLong(args[11]);
-  const double scaler = PyFloat_AsDouble(args[12]), eps = layer ? PyFloat_AsDouble(args[15]) : 0.;
+  const double scaler = PyFloat_AsDouble(args[12]), eps = layer ? PyFloat_AsDouble(args[16]) : 0.;
   if (PyErr_Occurred()) return nullptr;
   auto t = [&](int i) -> const Tensor& { return THPVariable_Unpack(args[i]); };
-  const Tensor &x = t(0), &table = t(7);
+  const Tensor &x = t(0), &table = t(7), &status = t(13);
   if (!plain_call() || !x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() != 3 || !x.is_contiguous() || heads < 1 ||
       kv < 1 || hd < 1)
     Py_RETURN_NONE;
-  const int64_t B = x.size(0), S = x.size(1), hidden = x.size(2);
+  const int64_t B = x.size(0), S = x.size(1), hidden = x.size(2), inner = heads * hd;
   for (int i = 1; i < 7; ++i)
     if (t(i).device() != x.device() || t(i).scalar_type() != at::kBFloat16) Py_RETURN_NONE;
   if (t(1).dim() != 2 || t(1).size(0) != (heads + 2 * kv) * hd || t(3).dim() != 2 || t(3).size(0) != heads) Py_RETURN_NONE;
   if (table.device() != x.device() || table.scalar_type() != at::kFloat || !table.is_contiguous() || table.dim() != 2 ||
       table.size(0) < S || table.size(1) != 2 * hd)
     Py_RETURN_NONE;
+  if (status.device() != x.device() || status.scalar_type() != at::kInt || status.numel() < MOE_B200_STATUS_INTS) Py_RETURN_NONE;
   const float* mask = nullptr;
   if (masked) {
     if (t(8).device() != x.device() || t(8).scalar_type() != at::kFloat || !t(8).is_contiguous() || t(8).numel() != S * S)
       Py_RETURN_NONE;
     mask = t(8).const_data_ptr<float>();
   }
-  // few rows: three launches of the library's own (the sizes and places that attention.py asks for as well)
-  const int64_t inner = heads * hd;
-  auto placed = [](const Tensor& p) { return (reinterpret_cast<uintptr_t>(p.const_data_ptr()) & 15u) == 0; };
-  auto matrix = [&](const Tensor& w, int64_t rows, int64_t cols) {
-    return w.dim() == 2 && w.size(0) == rows && w.size(1) == cols && w.is_contiguous() && placed(w);
+  // the library's own launches throughout, where sizes and places allow (attention.py asks for the same)
+  auto matrix = [](const Tensor& w, int64_t rows, int64_t cols) {
+    return w.dim() == 2 && w.size(0) == rows && w.size(1) == cols && w.is_contiguous();
   };
   auto vector = [](const Tensor& b, int64_t n) { return b.numel() == n && b.is_contiguous(); };
-  const bool few = moe::linear_rows_supported(B * S, (int)std::min<int64_t>(hidden, 1 << 24), layer) &&
-                   moe::linear_rows_supported(B * S, (int)std::min<int64_t>(inner, 1 << 24), false) && hd == 64 && S <= 128 &&
-                   heads % kv == 0 && placed(x) && matrix(t(1), (heads + 2 * kv) * hd, hidden) &&
-                   vector(t(2), (heads + 2 * kv) * hd) && matrix(t(3), heads, hidden) && vector(t(4), heads) &&
-                   matrix(t(5), hidden, inner) && vector(t(6), hidden);
+  moe::AttentionArgs p = {};
+  bool own = hidden <= 1 << 24 && inner <= 1 << 24 && B <= 1 << 24 && S <= 128 && matrix(t(1), (heads + 2 * kv) * hd, hidden) &&
+             vector(t(2), (heads + 2 * kv) * hd) && matrix(t(3), heads, hidden) && vector(t(4), heads) &&
+             matrix(t(5), hidden, inner) && vector(t(6), hidden);
+  if (own) {
+    p.x = x.const_data_ptr();
+    if (layer) {
+      for (int i = 14; i < 16; ++i)
+        if (t(i).device() != x.device() || t(i).scalar_type() != at::kBFloat16 || !vector(t(i), hidden)) Py_RETURN_NONE;
+      p.norm_weight = t(14).const_data_ptr();
+      p.norm_bias = t(15).const_data_ptr();
+      p.eps = (float)eps;
+      p.skip = p.x;
+    }
+    p.wqkv = t(1).const_data_ptr(); p.bqkv = t(2).const_data_ptr();
+    p.wgate = t(3).const_data_ptr(); p.bgate = t(4).const_data_ptr();
+    p.wo = t(5).const_data_ptr(); p.bo = t(6).const_data_ptr();
+    p.pos_emb = table.const_data_ptr<float>();
+    p.mask = mask;
+    p.B = B; p.S = (int)S; p.hidden = (int)hidden;
+    p.q_heads = (int)heads; p.kv_heads = (int)kv; p.head_dim = (int)hd;
+    p.scaler = (float)scaler;
+    p.status = status.data_ptr<int32_t>();
+    own = moe::attention_supported(p);
+  }
   if (layer) {
-    if (!few) Py_RETURN_NONE;
-    for (int i = 13; i < 15; ++i)
-      if (t(i).device() != x.device() || t(i).scalar_type() != at::kBFloat16 || !vector(t(i), hidden) || !placed(t(i)))
-        Py_RETURN_NONE;
+    if (!own) Py_RETURN_NONE;
     if (at::GradMode::is_enabled()) {
-      if (x.requires_grad() || t(13).requires_grad() || t(14).requires_grad()) Py_RETURN_NONE;
+      if (x.requires_grad() || t(14).requires_grad() || t(15).requires_grad()) Py_RETURN_NONE;
       for (int i = 1; i < 7; ++i)
         if (t(i).requires_grad()) Py_RETURN_NONE;
     }
@@ -1327,33 +1344,18 @@ PyObject* host_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   {
     pybind11::gil_scoped_release no_gil;
     void* stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
-    if (few) {
-      moe::AttentionRows p = {};
-      // qkv, gate and the core's output in one piece (rows of heads * 64 elements, the gate last)
-      const int64_t N = B * S;
-      const Tensor scratch = at::empty({N * (2 * (heads + kv) * hd + heads)}, x.options());
+    if (own) {
+      // qkv, the core's output, the normalised rows and the gate in one piece (rows of 16-byte multiples, the gate last)
+      const int64_t N = B * S, qkv = N * (heads + 2 * kv) * hd, apart = moe::attention_normalises_apart(p) ? N * hidden : 0;
+      const Tensor scratch = at::empty({qkv + N * inner + apart + N * heads}, x.options());
       result = at::empty({B, S, hidden}, x.options());
       char* at_byte = static_cast<char*>(scratch.data_ptr());
-      p.x = x.const_data_ptr();
-      if (layer) {
-        p.norm_weight = t(13).const_data_ptr();
-        p.norm_bias = t(14).const_data_ptr();
-        p.eps = (float)eps;
-        p.skip = p.x;
-      }
-      p.wqkv = t(1).const_data_ptr(); p.bqkv = t(2).const_data_ptr();
-      p.wgate = t(3).const_data_ptr(); p.bgate = t(4).const_data_ptr();
-      p.wo = t(5).const_data_ptr(); p.bo = t(6).const_data_ptr();
-      p.pos_emb = table.const_data_ptr<float>();
-      p.mask = mask;
-      p.B = B; p.S = (int)S; p.hidden = (int)hidden;
-      p.q_heads = (int)heads; p.kv_heads = (int)kv; p.head_dim = (int)hd;
-      p.scaler = (float)scaler;
       p.qkv = at_byte;
-      p.core = at_byte + N * (heads + 2 * kv) * hd * 2;
-      p.gate = at_byte + N * 2 * (heads + kv) * hd * 2;
+      p.core = at_byte + qkv * 2;
+      p.xn = at_byte + (qkv + N * inner) * 2;
+      p.gate = at_byte + (qkv + N * inner + apart) * 2;
       p.out = result.data_ptr();
-      rc = moe::attention_rows(p, stream);
+      rc = moe::attention_layer(p, stream);
     } else {
       const Tensor qkv = at::linear(x, t(1), t(2)), gate = at::linear(x, t(3), t(4));
       const Tensor out = at::empty({B, S, inner}, x.options());

@@ -58,10 +58,11 @@ int experts_backward_into(const void* x_sorted, const void* h, const int32_t* of
                           void* train_ws, size_t train_ws_bytes, const TrainGrads& grads, const LoraGrads* lora,
                           int32_t* status, void* stream);
 
-// The attention of a few short sequences (bf16, B S <= moe_b200_linear_rows_max()): QKV projection and head gate, on
-// LayerNorm(x) where norm_weight is given, the core of moe_b200_attention, the output projection, plus skip where given.
-// Three launches. Buffers: qkv [B S, (q + 2 kv) 64], gate [B S, q], core [B S, q 64]; x, out, skip [B S, hidden].
-struct AttentionRows {
+// The attention of the decoder layer (bf16): QKV projection and head gate, on LayerNorm(x) where norm_weight is given, the core
+// of moe_b200_attention, the output projection, plus skip where given. Three launches up to moe_b200_linear_rows_max() rows,
+// beyond a fourth for the LayerNorm. Buffers: qkv [B S, (q + 2 kv) 64], gate [B S, q], core [B S, q 64]; x, out, skip and, where
+// attention_normalises_apart() says so, xn [B S, hidden]; status: 16 words.
+struct AttentionArgs {
   const void *x, *norm_weight, *norm_bias;
   float eps;
   const void *wqkv, *bqkv, *wgate, *bgate, *wo, *bo;
@@ -70,9 +71,12 @@ struct AttentionRows {
   int64_t B;
   int S, hidden, q_heads, kv_heads, head_dim;
   float scaler;
-  void *qkv, *gate, *core, *out;
+  void *xn, *qkv, *gate, *core, *out;
+  int32_t* status;
 };
-bool linear_rows_supported(int64_t N, int K, bool norm);
-int attention_rows(const AttentionRows& p, void* stream);
+// Whether sizes and places are those that these launches take (and moe_b200_linear_rows): not all are the library's Linears'.
+bool attention_supported(const AttentionArgs& p);
+bool attention_normalises_apart(const AttentionArgs& p);
+int attention_layer(const AttentionArgs& p, void* stream);
 
 }  // namespace moe

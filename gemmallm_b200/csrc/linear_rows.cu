@@ -11,8 +11,8 @@
 // and that each has its first loads under way when the kernel before it ends: weights are asked for before the wait where
 // the launch says that nothing in flight writes them. A decoder layer of 37 tokens (d 1024, 16 heads, 8 experts) took 93.4 us
 // with six launches around the attention (LayerNorm, three library products, the core, the addition) and takes 69.5 with
-// three; one token 84 -> 39.6, 102 tokens 92.6 -> 79.7, 160 tokens 97.0 -> 94.5. At 192 tokens both take 100, at 256 the
-// library's products are ahead (102, here 107): the line is at 160.
+// three; one token 84 -> 39.6, 102 tokens 92.6 -> 79.6, 128 tokens 93.9 -> 80.7. Beyond 128 rows the Linears are tiles of
+// experts_tc2.cu (kLinear): 64 tokens 81.8 so and 72.3 here, 128 86.9 and 80.7, 140 89.9 and 91.3, 160 91.8 and 94.8.
 #include "common.cuh"
 #include "internal.h"
 
@@ -223,10 +223,6 @@ int launch_by_norm(bool norm, int K, Args... args) {
 
 }  // namespace
 
-bool linear_rows_supported(int64_t N, int K, bool norm) {
-  return N >= 1 && N <= kLinearRowsMax && K >= 8 && (K & 7) == 0 && (!norm || K <= 2048);
-}
-
 int launch_linear_rows(const void* x, const void* gamma, const void* beta, float eps, const LinearRows& first,
                        const LinearRows& second, const void* skip, int64_t N, int K, bool chained, cudaStream_t s) {
   auto op = [](const LinearRows& l) {
@@ -241,18 +237,47 @@ int launch_linear_rows(const void* x, const void* gamma, const void* beta, float
   return launch_by_norm<32>(gamma != nullptr, K, x, gamma, beta, eps, a, b, skip, N, K, chained, s);
 }
 
-int attention_rows(const AttentionRows& p, void* stream) {
+// K up to which the rows kernel keeps rows for their LayerNorm
+constexpr int kNormMaxK = 2048;
+
+bool attention_normalises_apart(const AttentionArgs& p) {
+  return p.norm_weight != nullptr && (p.B * p.S > kLinearRowsMax || p.hidden > kNormMaxK);
+}
+
+bool attention_supported(const AttentionArgs& p) {
+  const int64_t N = p.B * p.S;
+  if (N < 1 || N > (int64_t)1 << 28 || p.S > 128 || p.head_dim != 64 || p.kv_heads < 1 || p.q_heads % p.kv_heads != 0 ||
+      (p.hidden & 7) != 0 || p.hidden < 8)
+    return false;
+  for (const void* q : {p.x, p.wqkv, p.wgate, p.wo, p.norm_weight, p.norm_bias, p.skip})
+    if (!aligned16(q)) return false;
+  // as tiles the head gate's rows are stored, and biases loaded, 16 bytes at a time
+  return N <= kLinearRowsMax || ((p.q_heads & 7) == 0 && aligned16(p.bqkv) && aligned16(p.bgate) && aligned16(p.bo));
+}
+
+int attention_layer(const AttentionArgs& p, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t N = p.B * p.S;
-  const int heads = (p.q_heads + 2 * p.kv_heads) * p.head_dim, inner = p.q_heads * p.head_dim;
-  int rc = launch_linear_rows(p.x, p.norm_weight, p.norm_bias, p.eps, {p.wqkv, p.bqkv, p.qkv, heads},
-                              {p.wgate, p.bgate, p.gate, p.q_heads}, nullptr, N, p.hidden, false, s);
+  const LinearRows qkv = {p.wqkv, p.bqkv, p.qkv, (p.q_heads + 2 * p.kv_heads) * p.head_dim};
+  const LinearRows gate = {p.wgate, p.bgate, p.gate, p.q_heads}, out = {p.wo, p.bo, p.out, p.hidden}, none = {};
+  const int inner = p.q_heads * p.head_dim;
+  const bool few = N <= kLinearRowsMax;
+  const void *x = p.x, *gamma = p.norm_weight;
+  int rc = 0;
+  if (attention_normalises_apart(p)) {
+    rc = launch_layernorm_rows(x, gamma, p.norm_bias, p.eps, N, p.hidden, MOE_B200_BF16, p.xn, nullptr, s);
+    if (rc) return rc;
+    x = p.xn;
+    gamma = nullptr;
+  }
+  rc = few ? launch_linear_rows(x, gamma, p.norm_bias, p.eps, qkv, gate, nullptr, N, p.hidden, false, s)
+           : launch_linear_tiles(x, qkv, gate, nullptr, N, p.hidden, p.status, s);
   if (rc) return rc;
   rc = launch_attention(p.qkv, p.gate, p.pos_emb, p.mask, p.B, p.S, p.q_heads, p.kv_heads, p.head_dim, p.scaler, p.core, true,
                         s);
   if (rc) return rc;
-  return launch_linear_rows(p.core, nullptr, nullptr, 0.f, {p.wo, p.bo, p.out, p.hidden}, {nullptr, nullptr, nullptr, 0},
-                            p.skip, N, inner, true, s);
+  return few ? launch_linear_rows(p.core, nullptr, nullptr, 0.f, out, none, p.skip, N, inner, true, s)
+             : launch_linear_tiles(p.core, out, none, p.skip, N, inner, p.status, s);
 }
 
 }  // namespace moe
@@ -262,13 +287,19 @@ using namespace moe;
 extern "C" int64_t moe_b200_linear_rows_max(void) { return kLinearRowsMax; }
 
 extern "C" int moe_b200_linear_rows(const void* x, const void* W, const void* b, int rows, const void* W2, const void* b2,
-                                    int rows2, int64_t N, int K, void* out, void* out2, void* stream) {
-  if (N < 0 || N > kLinearRowsMax) return set_error(MOE_B200_ERR_SHAPE, "N out of range");
+                                    int rows2, int64_t N, int K, void* out, void* out2, int32_t* status, void* stream) {
+  if (N < 0 || N > (int64_t)1 << 28) return set_error(MOE_B200_ERR_SHAPE, "N out of range");
   if (K < 8 || (K & 7) || rows < 1 || rows2 < 0) return set_error(MOE_B200_ERR_SHAPE, "K must be a positive multiple of 8, rows positive");
   if (N == 0) return 0;
-  if (!x || !W || !b || !out || (rows2 > 0 && (!W2 || !b2 || !out2))) return set_error(MOE_B200_ERR_NULL, "NULL argument");
+  if (!x || !W || !b || !out || !status || (rows2 > 0 && (!W2 || !b2 || !out2)))
+    return set_error(MOE_B200_ERR_NULL, "NULL argument");
   if (!aligned16(x) || !aligned16(W) || (rows2 > 0 && !aligned16(W2)))
     return set_error(MOE_B200_ERR_ALIGN, "x and the weights must be 16-byte aligned");
-  return launch_linear_rows(x, nullptr, nullptr, 0.f, {W, b, out, rows}, {W2, b2, out2, rows2}, nullptr, N, K, false,
-                            (cudaStream_t)stream);
+  const LinearRows first = {W, b, out, rows}, second = {W2, b2, out2, rows2};
+  if (N <= kLinearRowsMax)
+    return launch_linear_rows(x, nullptr, nullptr, 0.f, first, second, nullptr, N, K, false, (cudaStream_t)stream);
+  if ((rows & 7) || (rows2 & 7)) return set_error(MOE_B200_ERR_SHAPE, "rows must be multiples of 8 at this N");
+  if (!aligned16(b) || !aligned16(out) || (rows2 > 0 && (!aligned16(b2) || !aligned16(out2))))
+    return set_error(MOE_B200_ERR_ALIGN, "buffers must be 16-byte aligned");
+  return launch_linear_tiles(x, first, second, nullptr, N, K, status, (cudaStream_t)stream);
 }

@@ -21,9 +21,10 @@ constexpr int kStg32Bytes = kStgRows * kStg32Pitch;
 // instruction): an eighth of the memory requests a one-row-per-thread store would make,
 // which compete with the TMA loads for the SM's path to L2, and the run length NVLink wants
 // for the expert-parallel scatter. dst = this thread's row (nullptr: nothing to store),
-// n = first column, Nlimit = number of valid columns of the row.
+// n = first column, Nlimit = number of valid columns of the row. skip: what this lane adds to the pieces it
+// stores, in fp32, rounded again (load_skip64), or nullptr.
 __device__ __forceinline__ void flush64(const uint4 (&packed)[8], __nv_bfloat16* dst, int n,
-                                        int Nlimit, uint8_t* stg, int lane) {
+                                        int Nlimit, uint8_t* stg, int lane, const uint4 (*skip)[8] = nullptr) {
 #pragma unroll
   for (int hr = 0; hr < 2; ++hr) {
     if ((lane >> 4) == hr) {
@@ -38,11 +39,32 @@ __device__ __forceinline__ void flush64(const uint4 (&packed)[8], __nv_bfloat16*
       __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(
           __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst), hr * 16 + rr));
       const int nn = n + piece * 8;
-      if (d != nullptr && nn < Nlimit)
-        *reinterpret_cast<uint4*>(d + nn) =
-            *reinterpret_cast<const uint4*>(stg + rr * kStgPitch + piece * 16);
+      if (d != nullptr && nn < Nlimit) {
+        uint4 v = *reinterpret_cast<const uint4*>(stg + rr * kStgPitch + piece * 16);
+        if (skip != nullptr) {
+          const uint4 k = (*skip)[hr * 4 + i];
+          uint32_t w[4] = {v.x, v.y, v.z, v.w};
+          const uint32_t o[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(bf16_lo(w[q]) + bf16_lo(o[q]), bf16_hi(w[q]) + bf16_hi(o[q]));
+          v = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        *reinterpret_cast<uint4*>(d + nn) = v;
+      }
     }
     __syncwarp();
+  }
+}
+
+// The pieces of a skip connection [rows, pitch] that a lane adds in flush64: rows of this warp from `row` on, `rows` of them
+// exist, 64 columns from n on of Nlimit.
+__device__ __forceinline__ void load_skip64(uint4 (&k)[8], const __nv_bfloat16* skip, int row, int rows, int pitch, int n,
+                                            int Nlimit, int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int rr = i * 4 + (lane >> 3), nn = n + (lane & 7) * 8;
+    k[i] = rr < rows && nn < Nlimit ? *reinterpret_cast<const uint4*>(skip + (int64_t)(row + rr) * pitch + nn)
+                                    : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -59,11 +81,14 @@ __device__ __forceinline__ uint4 pack8(const float (&o)[8]) {
 //   SCATTER: plain, but the row goes to sc.ret_y[meta >> 24] + (meta & 0xffffff) * Nout
 //            (the token owner's buffer, possibly on another GPU)
 //   release(): called once the warp has read its part of the accumulator
-template <bool GEGLU, bool SCATTER, typename Release>
+//   pitch  : elements from one output row to the next, where it is not Nout (0)
+//   SKIP   : plain, plus skip[pass], asked for before the accumulator was awaited
+template <bool GEGLU, bool SCATTER, bool SKIP = false, typename Release>
 __device__ __forceinline__ void store_tile(uint32_t taddr, int row, bool row_ok, int n0, int Nout,
                                            const __nv_bfloat16* __restrict__ bias,
                                            __nv_bfloat16* __restrict__ out, const EpScatter& sc,
-                                           uint8_t* stg, int lane, int half, Release release) {
+                                           uint8_t* stg, int lane, int half, Release release, int pitch = 0,
+                                           const uint4 (*skip)[8] = nullptr) {
   constexpr int BN = 256;
   constexpr int kTileN = GEGLU ? BN / 2 : BN;
   constexpr int kPasses = kTileN / 128;        // 64-column passes per warp
@@ -74,10 +99,10 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, int row, bool row_ok,
       const int meta = __ldg(&sc.meta[row]);
       dst = static_cast<__nv_bfloat16*>(sc.ret_y[(meta >> 24) & 7]) + (int64_t)(meta & 0xffffff) * Nout;
     } else {
-      dst = out + (int64_t)row * Nout;
+      dst = out + (int64_t)row * (pitch > 0 ? pitch : Nout);
     }
   }
-#pragma unroll 1
+#pragma unroll(SKIP ? kPasses : 1)
   for (int p = 0; p < kPasses; ++p) {
     const int col0 = (half * kPasses + p) * 64;   // first output column of this pass inside the tile
     uint4 packed[8];
@@ -129,7 +154,7 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, int row, bool row_ok,
         }
       }
     }
-    flush64(packed, dst, n0 + col0, Nout, stg, lane);
+    flush64(packed, dst, n0 + col0, Nout, stg, lane, SKIP ? skip + p : nullptr);
   }
 }
 

@@ -7,9 +7,9 @@ What the layer adds over assigning ``layer.moe`` / ``layer.mqa`` in the referenc
 in inference the second LayerNorm (model.py:298,312) is folded into the block's router and
 dispatch kernels and the second skip connection (model.py:319) into its combine kernel, so
 neither is a pass over the activations of its own; the first LayerNorm runs the library's row
-kernel (``moe_b200_layernorm``). The attention's Linears and the first skip connection stay
-library code around ``moe_b200_attention``, but for a few short sequences: there LayerNorm, QKV and head gate are one
-launch, the attention core the second, output Linear and skip connection the third (``csrc/linear_rows.cu``).
+kernel (``moe_b200_layernorm``); QKV and head gate are one launch, the attention core the next, output Linear and first
+skip connection the last, and for a few short sequences the first LayerNorm is part of the first one
+(``csrc/linear_rows.cu``).
 """
 from __future__ import annotations
 
@@ -22,7 +22,6 @@ from .attention import Attention
 from .moe import MOE, FeedForward, _stream
 
 
-_FEW_ROWS = lib.moe_b200_linear_rows_max()
 _module = nn.modules.module
 
 
@@ -77,12 +76,11 @@ class LLMLayer(nn.Module):
         self.device = device
 
     def _attend(self, tensor, attention_mask, fine_tuning):
-        """First LayerNorm, attention and first skip connection (model.py:297-308): in three launches for a few short
-        sequences, else as four steps, whose results are the same to the bit at those sizes."""
+        """First LayerNorm, attention and first skip connection (model.py:297-308): in one native call, or step by step,
+        whose results are the same to the bit."""
         mqa, norm = self.mqa, self.norm1
         if (type(mqa) is Attention and "forward" not in mqa.__dict__ and not _watched(mqa) and tensor.is_cuda
-                and tensor.dtype == torch.bfloat16 and tensor.dim() == 3
-                and tensor.shape[0] * tensor.shape[1] <= _FEW_ROWS and norm.weight is not None and norm.bias is not None
+                and tensor.dtype == torch.bfloat16 and tensor.dim() == 3 and norm.weight is not None and norm.bias is not None
                 and not (torch.is_grad_enabled() and (tensor.requires_grad or mqa.qkv.weight.requires_grad))):
             done = _host.attention(*mqa._arguments(tensor, attention_mask, fine_tuning), norm.weight, norm.bias,
                                    float(norm.eps))

@@ -424,11 +424,12 @@ int moe_b200_attention(const void* qkv, const void* gate, const float* pos_emb, 
                        int64_t B, int S, int q_heads, int kv_heads, int head_dim, float scaler,
                        void* out, void* stream);
 
-/* The Linears around it (model.py:104, 139, 150) on the rows of a few short sequences, bf16, N <= moe_b200_linear_rows_max():
- * out [N, rows] = x W^T + b and, where rows2 > 0, out2 [N, rows2] = x W2^T + b2 in the same launch; x [N,K], W [rows,K],
- * K a multiple of 8; fp32 sums, one rounding. x, W and W2 16-byte aligned. */
+/* The Linears around it (model.py:104, 139, 150), bf16: out [N, rows] = x W^T + b and, where rows2 > 0, out2 [N, rows2] =
+ * x W2^T + b2 in the same launch; x [N,K], W [rows,K], K a multiple of 8; fp32 sums, one rounding. x, W and W2 16-byte
+ * aligned; beyond moe_b200_linear_rows_max() rows of x, which are tiles of the tensor cores, rows and rows2 multiples of 8
+ * and the other buffers aligned as well. status: int32[16], written when a wait runs out. */
 int moe_b200_linear_rows(const void* x, const void* W, const void* b, int rows, const void* W2, const void* b2, int rows2,
-                         int64_t N, int K, void* out, void* out2, void* stream);
+                         int64_t N, int K, void* out, void* out2, int32_t* status, void* stream);
 int64_t moe_b200_linear_rows_max(void);
 
 /* ---- Training mode ---------------------------------------------------------------

@@ -313,9 +313,10 @@ def test_lora_merge_by_units(cuda_device, out_f, in_f, rank):
 
 
 # blocks of 16 rows and 16 or 32 tokens that end early, K that ends within a chunk of 32, a round of chunks more, one Linear
-# and two, the most tokens there can be
+# and two; from 129 tokens on tiles of 256 x 2 times 128, the second Linear in either half, K whole and in two and four ranges
 @pytest.mark.parametrize("N,K,r,r2", [(1, 8, 1, 0), (15, 40, 17, 2), (16, 1024, 1152, 16), (17, 1032, 72, 5), (33, 264, 2400, 1),
-                                      (160, 3080, 48, 31)])
+                                      (128, 3080, 48, 31), (129, 8, 8, 0), (255, 264, 128, 8), (300, 1032, 1152, 16),
+                                      (257, 2056, 264, 136), (5000, 72, 1152, 16), (3000, 1024, 1024, 0)])
 def test_linear_rows(cuda_device, N, K, r, r2):
     g = torch.Generator().manual_seed(N + K)
     rnd = lambda *s: (torch.randn(*s, generator=g) / 4).to(torch.bfloat16)
@@ -323,9 +324,10 @@ def test_linear_rows(cuda_device, N, K, r, r2):
     dev = [t.to(cuda_device) for t in (x, W, b, W2, b2)]
     out = torch.full((N + 1, r), 7.0, dtype=torch.bfloat16, device=cuda_device)
     out2 = torch.full((N + 1, max(r2, 1)), 7.0, dtype=torch.bfloat16, device=cuda_device)
-    ptr = [t.data_ptr() for t in dev]
+    ptr, status = [t.data_ptr() for t in dev], torch.zeros(16, dtype=torch.int32, device=cuda_device)
     check(lib.moe_b200_linear_rows(ptr[0], ptr[1], ptr[2], r, ptr[3], ptr[4], r2, N, K, out.data_ptr(), out2.data_ptr(),
-                                   helpers.stream(cuda_device)), "linear_rows")
+                                   status.data_ptr(), helpers.stream(cuda_device)), "linear_rows")
+    assert status.cpu()[0] == 0
     for got, w, bias, wanted in ((out, W, b, True), (out2, W2, b2, r2 > 0)):
         assert (got[N:] == 7.0).all()
         if wanted:

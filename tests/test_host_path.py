@@ -9,6 +9,7 @@ import torch
 
 from gemmallm_b200 import MOE, Attention, FeedForward, LLMLayer, _host
 from gemmallm_b200._cabi import MoeB200Error
+from gemmallm_b200.attention import _linear_rows
 from gemmallm_b200.layer import _layernorm
 
 DT = torch.bfloat16
@@ -848,11 +849,12 @@ def test_attention_native_and_python_paths_agree(cuda_device, monkeypatch, B, S,
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,S,hidden,heads,kv,ft", [(1, 1, 64, 2, 1, False), (1, 16, 200, 4, 2, True), (17, 1, 1024, 16, 1, False),
-                                                    (1, 65, 1032, 2, 2, False), (5, 32, 2048, 4, 1, False),
-                                                    (7, 23, 256, 2, 1, False)])
+                                                    (1, 65, 1032, 2, 2, False), (4, 32, 2048, 4, 1, False), (3, 7, 2056, 8, 8, False),
+                                                    (3, 43, 256, 2, 1, False), (3, 43, 200, 8, 1, False), (4, 64, 1024, 16, 1, True),
+                                                    (3, 100, 1032, 24, 2, False), (40, 63, 512, 8, 4, False)])
 def test_attention_of_a_layer_in_one_call(cuda_device, B, S, hidden, heads, kv, ft):
-    """LayerNorm, attention and skip connection in three launches, and step by step: the same to the bit, on both sides of
-    the most rows there can be. What the one call cannot do is left to the steps."""
+    """LayerNorm, attention and skip connection in one call, and step by step: the same to the bit, on both sides of 128 rows,
+    where the Linears become tiles (whole, and with K in two or four ranges). What the call cannot do is left to the steps."""
     torch.manual_seed(S)
     layer = LLMLayer(hidden, 64, heads, kv, Table(128, 64), expansion_factor=1, use_moe=False, device="cuda")
     layer = layer.to(device=cuda_device, dtype=DT).eval()
@@ -862,10 +864,17 @@ def test_attention_of_a_layer_in_one_call(cuda_device, B, S, hidden, heads, kv, 
     x = torch.randn(B, S, hidden, generator=torch.Generator().manual_seed(B)).to(device=cuda_device, dtype=DT)
     mask = torch.full((S, S), float("-inf"), device=cuda_device).triu(1)
     with torch.no_grad():
+        args = layer.mqa._arguments(x, mask, ft)
+        norm = (layer.norm1.weight, layer.norm1.bias, layer.norm1.eps)
         want = layer.mqa(_layernorm(layer.norm1, x), mask, ft) + x
-        args = (*layer.mqa._arguments(x, mask, ft), layer.norm1.weight, layer.norm1.bias, layer.norm1.eps)
-        one = _host.attention(*args)
-        assert (one is None) == (B * S > 160)
+        # torch's Linears around the same core: sums in another order, and bf16 between the steps
+        xn = _layernorm(layer.norm1, x)
+        lib_qkv, own_qkv = torch.nn.functional.linear(xn, args[1], args[2]), _linear_rows(args[13], xn, *args[1:5])[0] \
+            if layer.mqa._own_linears(args, B * S, hidden, heads * 64) else None
+        if own_qkv is not None:
+            assert (lib_qkv.float() - own_qkv.float()).norm() <= 2.0 ** -8 * lib_qkv.float().norm()
+        one = _host.attention(*args, *norm)
+        assert (one is None) == (B * S > 128 and heads % 8 != 0)
         if one is not None:
             assert torch.equal(one, want)
         assert torch.equal(layer._attend(x, mask, ft), want)
@@ -873,10 +882,11 @@ def test_attention_of_a_layer_in_one_call(cuda_device, B, S, hidden, heads, kv, 
         handle = layer.mqa.register_forward_hook(lambda *a: seen.append(a))
         assert torch.equal(layer._attend(x, mask, ft), want) and len(seen) == 1
         handle.remove()
+        assert layer.mqa.device_status() == 0
         odd = torch.empty(x.numel() + 1, device=cuda_device, dtype=DT)[1:].view_as(x).copy_(x)
-        assert _host.attention(odd, *args[1:]) is None
-        assert _host.attention(*args[:13], layer.norm1.weight[:8], *args[14:]) is None
-    assert _host.attention(*args) is None                                   # gradients are wanted
+        assert _host.attention(odd, *args[1:], *norm) is None
+        assert _host.attention(*args, norm[0][:8], *norm[1:]) is None
+    assert _host.attention(*args, *norm) is None                            # gradients are wanted
 
 
 @pytest.mark.gpu
