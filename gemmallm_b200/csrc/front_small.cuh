@@ -10,7 +10,7 @@
 //      partial x Wg^T with mma.sync m16n8k16 exactly like router_mma_kernel
 //      (router.cu), all its loads in flight at once; partials are summed over
 //      the K slices in slice order, plus bias. fp32: a thread per (token,
-//      expert mod 8, eighth of K), eight sums of every eighth element there;
+//      expert mod 8, slice of K), eight sums of every eighth element there;
 //   B. 8, 16 or 32 lanes per token, lane e = expert e: fp32 softmax, k passes of
 //      arg-max ordered by (logit desc, index asc) with shuffle reductions
 //      on order-preserving keys, renormalise;
@@ -52,7 +52,7 @@ using front_detail::mma_bf16_16816;
 using front_detail::ld_acquire_gpu_i32;
 
 // SPLIT = false: every block derives the complete routing (fastest up to about a hundred tokens).
-// SPLIT = true: block b routes tokens 16b .. 16b+15 only; the blocks then exchange their per-slot
+// SPLIT = true: block b routes tokens per*b .. per*b+per-1 only (at most 16); the blocks then exchange their per-slot
 //   expert counts and probability sums through `xch` and meet, and each block places and copies its
 //   own rows. They meet at a counter (bf16: at most 128 blocks on an otherwise idle GPU; the wait is
 //   bounded and reports a time-out in `status`) or at a grid barrier (fp32: a cooperative launch, as
@@ -82,7 +82,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
                  int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
                  T* __restrict__ perm, __nv_bfloat16* __restrict__ planes, float* __restrict__ psum,
                  float* __restrict__ aux, int* __restrict__ xch, int* __restrict__ counter,
-                 int32_t* __restrict__ status) {
+                 int32_t* __restrict__ status, int per_given) {
   constexpr int kThreads = kFrontThreads;
   constexpr int kMaxE = kFrontMaxE;
   constexpr bool F32 = sizeof(T) == 4;
@@ -90,9 +90,10 @@ __device__ __forceinline__ void front_small_body(float* smem,
   static_assert(!F32 || SPLIT, "fp32: blocks of 16 tokens");
   constexpr int kPiece = 16 / sizeof(T);                   // elements of a 16-byte piece
   const int ld = E + 1;
-  // SPLIT: this block's 16 tokens are "the problem" for the phases A and B below
-  const int tok_base = SPLIT ? 16 * blk : 0;
-  const int N = SPLIT ? min(16, Ntotal - tok_base) : Ntotal;
+  // SPLIT: this block's tokens are "the problem" for the phases A and B below
+  const int per = F32 ? per_given : 16;
+  const int tok_base = SPLIT ? per * blk : 0;
+  const int N = SPLIT ? min(per, Ntotal - tok_base) : Ntotal;
   const bool writer = SPLIT || blk == 0;     // this block writes the per-token results
   if (SPLIT) {
     x += (size_t)tok_base * d;
@@ -104,9 +105,12 @@ __device__ __forceinline__ void front_small_body(float* smem,
   const int ngroups = (N + 15) >> 4;                       // 16-token groups
   int gp2 = 1;
   while (gp2 < ngroups) gp2 <<= 1;                         // 1, 2, 4 or 8
-  const int nslices = F32 ? 8 : 32 / gp2;                  // K slices
-  float* s_part = smem;                                    // [nslices][16*gp2][8*NT]
-  float* s_logit = s_part + (size_t)nslices * 16 * gp2 * 8 * NT;   // [N][E+1]
+  // fp32: a warp has four tokens; 1, 2 or 4 of them side by side
+  const int tg4 = per <= 4 ? 1 : per <= 8 ? 2 : 4;
+  const int nslices = F32 ? 32 / tg4 : 32 / gp2;           // K slices
+  const int tok_pitch = F32 ? 4 * tg4 : 16 * gp2;          // tokens of a slice
+  float* s_part = smem;                                    // [nslices][tok_pitch][8*NT]
+  float* s_logit = s_part + (size_t)nslices * tok_pitch * 8 * NT;   // [N][E+1]
   int* s_idx = reinterpret_cast<int*>(s_logit + (size_t)N * ld);   // [N*k]
   int* s_row = s_idx + N * k;                              // [N*k]
   int* s_cnt = s_row + N * k;                              // [kMaxTopK][kMaxE]
@@ -127,35 +131,35 @@ __device__ __forceinline__ void front_small_body(float* smem,
     // A chunk of K of the block's tokens and of all experts is brought to shared memory, all its loads in flight at once
     // (read where they lie, 16 bytes at a time, they took 9.7 us of this kernel's 17 at d 512; a call of 512
     // tokens 102.5 -> 94.7). Lane = (token
-    // of four, expert mod 8), warps also take an eighth of K each: its pieces in order, even and odd places apart.
+    // of four, expert mod 8), warps also take a slice of K each: its pieces in order, even and odd places apart.
     constexpr int KC = kFrontChunk<NT>, KP = KC + kFrontPad;
-    const int tok = (warp & 3) * 4 + (lane >> 3), e0 = lane & 7, ks = warp >> 2;
-    const int n4 = d >> 2, per = (n4 + nslices - 1) / nslices;
-    float* s_x = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(smem) + front_small_smem_bytes(NT, 16, E, k) + 15) &
+    const int tok = (warp % tg4) * 4 + (lane >> 3), e0 = lane & 7, ks = warp / tg4;
+    const int n4 = d >> 2, each = (n4 + nslices - 1) / nslices;
+    float* s_x = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(smem) + front_small_smem_bytes(NT, per, E, k) + 15) &
                                           ~(uintptr_t)15);          // [16][KP], then [8 NT][KP]
     float* s_w = s_x + 16 * KP;
-    // a chunk holds the same part of every eighth
-    const int step = KC / 4 / 8;
+    // a chunk holds the same part of every slice
+    const int step = KC / 4 / nslices;
     float4 acc[2][NT];       // pieces of even and of odd place
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
       for (int j = 0; j < NT; ++j) acc[hh][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int c0 = 0; c0 < per; c0 += step) {
+    for (int c0 = 0; c0 < each; c0 += step) {
       if (c0 > 0) __syncthreads();
-      const int rows = 16 + min(8 * NT, E);
+      const int rows = N + min(8 * NT, E);
       for (int i = tid; i < rows * (KC / 4); i += kThreads) {
         const int r = i / (KC / 4), q = i - r * (KC / 4);
-        const int slice = q / step, c = slice * per + c0 + (q - slice * step);      // piece of the row
-        const bool ok = c0 + (q - slice * step) < per && c < n4;
-        const T* src = r < 16 ? x + (size_t)min(r, N - 1) * d : Wg + (size_t)(r - 16) * d;
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared((r < 16 ? s_x + r * KP : s_w + (r - 16) * KP) + q * 4);
+        const int slice = q / step, c = slice * each + c0 + (q - slice * step);     // piece of the row
+        const bool ok = c0 + (q - slice * step) < each && c < n4;
+        const T* src = r < N ? x + (size_t)r * d : Wg + (size_t)(r - N) * d;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared((r < N ? s_x + r * KP : s_w + (r - N) * KP) + q * 4);
         if (ok)
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + (size_t)c * 4) : "memory");
       }
       asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
       __syncthreads();
-      const int n = min(step, min(per - c0, n4 - (ks * per + c0)));
+      const int n = min(step, min(each - c0, n4 - (ks * each + c0)));
       const float4* xr = reinterpret_cast<const float4*>(s_x + tok * KP) + ks * step;
       const float4* wr = reinterpret_cast<const float4*>(s_w) + ks * step;
 #pragma unroll 4
@@ -175,7 +179,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
     }
 #pragma unroll
     for (int j = 0; j < NT; ++j)
-      s_part[((size_t)ks * 16 + tok) * ET + 8 * j + e0] =
+      s_part[((size_t)ks * tok_pitch + tok) * ET + 8 * j + e0] =
           ((acc[0][j].x + acc[1][j].x) + (acc[0][j].y + acc[1][j].y)) +
           ((acc[0][j].z + acc[1][j].z) + (acc[0][j].w + acc[1][j].w));
   } else {
@@ -240,11 +244,16 @@ __device__ __forceinline__ void front_small_body(float* smem,
   constexpr int kInFlight = 4;
   const int first_item = (SPLIT ? 0 : blk * kThreads * kInFlight) + tid;
   const int item_stride = (SPLIT ? 1 : nblk) * kThreads * kInFlight;
+  // fp32: 2^lg warps (32 over the block's tokens, those rounded up to a power of two) share a token's row, which is stored
+  // five times as wide: no division per piece (bf16 is the slower so, 59.2 -> 61 us at 300 tokens: registers)
+  const int lg = F32 ? min(5, __clz(N - 1) - 27) : 0;
+  const int copy_tok = warp >> lg, copy_pc = ((warp & ((1 << lg) - 1)) << 5) + lane, copy_stride = 32 << lg;
   uint4 pre[kInFlight];
 #pragma unroll
   for (int u = 0; u < kInFlight; ++u) {
-    const int i = first_item + u * kThreads;
-    if (i < items)
+    const int p = copy_pc + u * copy_stride;
+    const int i = F32 ? copy_tok * pieces + p : first_item + u * kThreads;
+    if (F32 ? copy_tok < N && p < pieces : i < items)
       asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
                    : "=r"(pre[u].x), "=r"(pre[u].y), "=r"(pre[u].z), "=r"(pre[u].w)
                    : "l"(src + i)
@@ -254,10 +263,12 @@ __device__ __forceinline__ void front_small_body(float* smem,
     const int tok = i / E, e = i - tok * E;
     float s = 0.f;
     if constexpr (F32) {
-      float q[8];
+      for (int k0 = 0; k0 < nslices; k0 += 8) {
+        float q[8];
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) q[ks] = s_part[((size_t)ks * 16 + tok) * ET + e];
-      s = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+        for (int ks = 0; ks < 8; ++ks) q[ks] = s_part[((size_t)(k0 + ks) * tok_pitch + tok) * ET + e];
+        s += ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+      }
     } else {
       for (int ks = 0; ks < nslices; ++ks) s += s_part[((size_t)ks * 16 * gp2 + tok) * ET + e];
     }
@@ -334,7 +345,8 @@ __device__ __forceinline__ void front_small_body(float* smem,
     const int nb = nblk, b = blk;
     float* xps = reinterpret_cast<float*>(xch + nb * k * E);    // [nb][E] probability sums
     static_assert((F32 ? 8 : 32) * 16 * 8 * NT >= 128 * 8 * NT, "128 blocks' sums of 8 NT experts in [nslices][16][8 NT]");
-    if (tid < k * E) xch[b * k * E + tid] = s_cnt[(tid / E) * kMaxE + tid % E];
+    // (fp32: a count's blocks side by side, for a warp to add)
+    if (tid < k * E) xch[F32 ? tid * nb + b : b * k * E + tid] = s_cnt[(tid / E) * kMaxE + tid % E];
     if (tid < E) {
       float ps = 0.f;
       for (int tok = 0; tok < N; ++tok) ps += s_logit[tok * ld + tid];
@@ -369,7 +381,23 @@ __device__ __forceinline__ void front_small_body(float* smem,
       __syncthreads();
     }
     // totals per (slot, expert) and the rows that earlier blocks put in front of this block's
-    for (int i = tid; i < nb * k * E; i += kThreads) {
+    if constexpr (F32) {
+      for (int je = warp; je < k * E; je += kThreads / 32) {
+        unsigned sum = 0;      // both, 16 bits each: 2048 tokens at most
+        for (int bb = lane; bb < nb; bb += 32) {
+          const unsigned c = (unsigned)__ldcg(&xch[je * nb + bb]);
+          sum += c | (bb < b ? c << 16 : 0u);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) {
+          const int j = je / E, e = je - j * E;
+          s_tot[j * kMaxE + e] = (int)(sum & 0xffffu);
+          if (sum >> 16) atomicAdd(&s_base[e], (int)(sum >> 16));
+        }
+      }
+    }
+    for (int i = tid; !F32 && i < nb * k * E; i += kThreads) {
       const int c = __ldcg(&xch[i]);
       const int bb = i / (k * E), je = i - bb * (k * E);
       const int j = je / E, e = je - j * E;
@@ -423,12 +451,11 @@ __device__ __forceinline__ void front_small_body(float* smem,
       if (blk == 0) offsets[E] = incl;
     }
     __syncwarp();
-    const int npair = N * k;
+    const int npair = F32 ? 0 : N * k;
     for (int p0 = 0; p0 < npair; p0 += 32) {
       const int p = p0 + lane;
       const int e = p < npair ? s_idx[p] : -1;
-      const bool ok = F32 ? (unsigned)e < (unsigned)E : e >= 0;
-      if (F32 && p < npair && !ok) atomicMax(&status[0], MOE_B200_DEV_BAD_INDEX);
+      const bool ok = e >= 0;
       const unsigned grp = __match_any_sync(0xffffffffu, ok ? e : -1 - lane);
       int row = -1;
       if (ok) row = s_off[e] + s_run[e] + __popc(grp & ((1u << lane) - 1u));
@@ -443,8 +470,61 @@ __device__ __forceinline__ void front_small_body(float* smem,
   }
   __syncthreads();
 
+  if constexpr (F32) {
+    // ranks: a warp per expert, 32 pairs at a time; slots without an expert have no row
+    const int npair = N * k;
+    if (warp < E) {
+      int next = s_off[warp];
+      for (int p0 = 0; p0 < npair; p0 += 32) {
+        const int p = p0 + lane;
+        const bool mine = p < npair && s_idx[p] == warp;
+        const unsigned hit = __ballot_sync(0xffffffffu, mine);
+        if (mine) {
+          const int row = next + __popc(hit & ((1u << lane) - 1u));
+          s_row[p] = row;
+          row_of[p] = row;
+        }
+        next += __popc(hit);
+      }
+    }
+    for (int p = tid; p < npair; p += kThreads)
+      if ((unsigned)s_idx[p] >= (unsigned)E) {
+        atomicMax(&status[0], MOE_B200_DEV_BAD_INDEX);
+        s_row[p] = -1;
+        row_of[p] = -1;
+      }
+    __syncthreads();
+    for (int tok = copy_tok; tok < N; tok += 32 >> lg)
+      for (int p0 = copy_pc; p0 < pieces; p0 += copy_stride * kInFlight) {
+        uint4 v[kInFlight];
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u) {
+          const int p = p0 + u * copy_stride;
+          if (tok == copy_tok && p0 == copy_pc) v[u] = pre[u];
+          else if (p < pieces) v[u] = __ldcg(src + (size_t)tok * pieces + p);
+        }
+        for (int j = 0; j < k; ++j) {
+          const int row = s_row[tok * k + j];
+          if (row < 0) continue;
+#pragma unroll
+          for (int u = 0; u < kInFlight; ++u) {
+            const int p = p0 + u * copy_stride;
+            if (p >= pieces) break;
+            // the rows as they are, and as the three bf16 planes the products read (split once here, not by every tile)
+            reinterpret_cast<uint4*>(perm + (size_t)row * d)[p] = v[u];
+            uint2 part[3];
+            split2(__uint_as_float(v[u].x), __uint_as_float(v[u].y), part[0].x, part[1].x, part[2].x);
+            split2(__uint_as_float(v[u].z), __uint_as_float(v[u].w), part[0].y, part[1].y, part[2].y);
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+              reinterpret_cast<uint2*>(planes + ((size_t)q * Ntotal * k + row) * d)[p] = part[q];
+          }
+        }
+      }
+  }
+
   // ---- D. copy the token rows into the sorted buffer (split over the blocks) -----
-  for (int i0 = first_item; i0 < items; i0 += item_stride) {
+  for (int i0 = first_item; !F32 && i0 < items; i0 += item_stride) {
     uint4 v[kInFlight];
 #pragma unroll
     for (int u = 0; u < kInFlight; ++u) {
@@ -457,23 +537,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
       const int i = i0 + u * kThreads;
       if (i < items) {
         const int tok = i / pieces, pc = i - tok * pieces;
-        if constexpr (F32) {
-          // the rows as they are, and as the three bf16 planes the products read (split once here, not by every tile)
-          uint2 part[3];
-          split2(__uint_as_float(v[u].x), __uint_as_float(v[u].y), part[0].x, part[1].x, part[2].x);
-          split2(__uint_as_float(v[u].z), __uint_as_float(v[u].w), part[0].y, part[1].y, part[2].y);
-          for (int j = 0; j < k; ++j) {
-            const int row = s_row[tok * k + j];
-            if (row < 0) continue;
-            reinterpret_cast<uint4*>(perm + (size_t)row * d)[pc] = v[u];
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-              reinterpret_cast<uint2*>(planes + ((size_t)q * Ntotal * k + row) * d)[pc] = part[q];
-          }
-        } else {
-          for (int j = 0; j < k; ++j)
-            reinterpret_cast<uint4*>(perm + (size_t)s_row[tok * k + j] * d)[pc] = v[u];
-        }
+        for (int j = 0; j < k; ++j) reinterpret_cast<uint4*>(perm + (size_t)s_row[tok * k + j] * d)[pc] = v[u];
       }
     }
   }

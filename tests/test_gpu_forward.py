@@ -139,6 +139,13 @@ def test_fp32_calls_on_planes(cuda_device, N, d, f, E, k, special):
         assert (got[ok].double() - want[ok].double()).norm() <= 5e-7 * want[ok].double().norm()
 
 
+# four, six and nine tokens a block, the last block with fewer, one to four of a warp's tokens side by side, a row's pieces over
+# two to eight warps
+@pytest.mark.parametrize("N,d,E,k", [(18, 8, 3, 2), (513, 1032, 8, 2), (645, 72, 9, 3), (1150, 264, 24, 1)])
+def test_fp32_routing_by_tokens_of_a_block(cuda_device, N, d, E, k):
+    test_fp32_routing_in_one_launch(cuda_device, N, d, E, k)
+
+
 @pytest.mark.parametrize("N,fold", [(1, False), (40, False), (2048, False), (2049, False), (300, True), (2049, True)])
 def test_fp32_tokens_of_nan(cuda_device, N, fold):
     """On both sides of 2048 tokens, with and without a folded LayerNorm: a token of NaN has no expert, its output is the
