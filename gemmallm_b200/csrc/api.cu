@@ -531,7 +531,8 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
     // router and dispatch of up to a few hundred tokens in one launch
     // (beyond 128 tokens its blocks share the work and meet at a counter behind the status words)
     void* planes = front32 ? static_cast<char*>(h) + h_planes_bytes((size_t)N * k, f) : nullptr;
-    rc = launch_front_small(x, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm,
+    // (spec reads the tokens where they lie, and waits for this kernel: 128 tokens 54.8 us with their copies, 52.1 without)
+    rc = launch_front_small(x, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, spec ? nullptr : perm,
                             psum, aux, s, scratch,
                             status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, dtype, planes);
     if (rc) return rc;

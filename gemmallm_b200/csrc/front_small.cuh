@@ -239,7 +239,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
   // the first batch of row copies: the loads do not depend on the routing, so they are
   // issued now and wait in registers until the destination rows are known
   const int pieces = d / kPiece;
-  const int items = N * pieces;
+  const int items = perm != nullptr ? N * pieces : 0;      // nullptr: the next kernel reads x itself
   const uint4* src = reinterpret_cast<const uint4*>(x);
   constexpr int kInFlight = 4;
   const int first_item = (SPLIT ? 0 : blk * kThreads * kInFlight) + tid;
