@@ -4,8 +4,8 @@
 // each one derives the complete routing by itself (the same instructions on the
 // same data, so every block gets the same answer and no grid barrier is needed),
 // block 0 writes the routing results, and the row copies are split over the blocks.
-// Covers reference model.py:206-253 for N <= 512, N*k <= 1024, E <= 32, bf16 (blocks that share the work: up to 2048
-// tokens, bf16 and fp32):
+// Covers reference model.py:206-253 for N <= 512, N*k <= 1024, E <= 32, bf16 (fp32, whose blocks share the work: up to 2048
+// tokens):
 //   A. logits: 32 warps = (16-token group) x (slice of K); each warp forms its
 //      partial x Wg^T with mma.sync m16n8k16 exactly like router_mma_kernel
 //      (router.cu), all its loads in flight at once; partials are summed over
@@ -51,15 +51,12 @@ __device__ __forceinline__ int ld_acquire_gpu_i32(const int* p) {
 using front_detail::mma_bf16_16816;
 using front_detail::ld_acquire_gpu_i32;
 
-// SPLIT = false: every block derives the complete routing (fastest up to about a hundred tokens).
-// SPLIT = true: block b routes tokens per*b .. per*b+per-1 only (at most 16); the blocks then exchange their per-slot
-//   expert counts and probability sums through `xch` and meet, and each block places and copies its
-//   own rows. They meet at a counter (bf16: at most 128 blocks on an otherwise idle GPU; the wait is
-//   bounded and reports a time-out in `status`) or at a grid barrier (fp32: a cooperative launch, as
-//   the dispatch kernel's that these calls took before; the launch, not the barrier, costs 2.3 us of a
-//   call of 512 tokens, 101.3 us without). Same results as the other form except for the order in which
-//   the logits' partial sums are added.
-//
+// bf16: every block derives the complete routing (fastest up to about a hundred tokens; beyond, front_mid_kernel in
+//   front_small.cu).
+// fp32 (SPLIT): block b routes tokens per*b .. per*b+per-1 only (at most 16); the blocks then exchange their per-slot
+//   expert counts and probability sums through `xch` and meet at a grid barrier (a cooperative launch, as the dispatch kernel's
+//   that these calls took before; the launch, not the barrier, costs 2.3 us of a call of 512 tokens, 101.3 us without),
+//   and each block places and copies its own rows.
 // `smem`: front_small_smem_bytes() of shared memory.
 // The partial logits' area also takes the blocks' probability sums (SPLIT, up to 128 blocks) once the logits are summed.
 // fp32: behind the rest, kFrontChunk elements of K of 16 tokens and 8 NT experts.
@@ -74,24 +71,21 @@ __host__ __device__ constexpr size_t front_f32_chunk_bytes(int NT) {
   return (size_t)(16 + 8 * NT) * ((NT == 1 ? 512 : 256) + kFrontPad) * sizeof(float) + 16;
 }
 
-template <int NT, bool SPLIT, typename T = __nv_bfloat16>  // n-tiles of 8 experts: E <= 8*NT
+template <int NT, typename T>  // n-tiles of 8 experts: E <= 8*NT
 __device__ __forceinline__ void front_small_body(float* smem,
                  const T* __restrict__ x, const T* Wg, const T* bg, int Ntotal, int d, int E, int k,
                  float* __restrict__ out_logits, int32_t* __restrict__ out_idx,
                  float* __restrict__ out_w, int32_t* __restrict__ cnt_slot,
                  int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
                  T* __restrict__ perm, __nv_bfloat16* __restrict__ planes, float* __restrict__ psum,
-                 float* __restrict__ aux, int* __restrict__ xch, int* __restrict__ counter,
-                 int32_t* __restrict__ status, int per_given) {
+                 float* __restrict__ aux, int* __restrict__ xch, int32_t* __restrict__ status, int per) {
   constexpr int kThreads = kFrontThreads;
   constexpr int kMaxE = kFrontMaxE;
-  constexpr bool F32 = sizeof(T) == 4;
+  constexpr bool F32 = sizeof(T) == 4, SPLIT = F32;
   const int blk = (int)blockIdx.x, nblk = (int)gridDim.x;
-  static_assert(!F32 || SPLIT, "fp32: blocks of 16 tokens");
   constexpr int kPiece = 16 / sizeof(T);                   // elements of a 16-byte piece
   const int ld = E + 1;
   // SPLIT: this block's tokens are "the problem" for the phases A and B below
-  const int per = F32 ? per_given : 16;
   const int tok_base = SPLIT ? per * blk : 0;
   const int N = SPLIT ? min(per, Ntotal - tok_base) : Ntotal;
   const bool writer = SPLIT || blk == 0;     // this block writes the per-token results
@@ -245,7 +239,7 @@ __device__ __forceinline__ void front_small_body(float* smem,
   const int first_item = (SPLIT ? 0 : blk * kThreads * kInFlight) + tid;
   const int item_stride = (SPLIT ? 1 : nblk) * kThreads * kInFlight;
   // fp32: 2^lg warps (32 over the block's tokens, those rounded up to a power of two) share a token's row, which is stored
-  // five times as wide: no division per piece (bf16 is the slower so, 59.2 -> 61 us at 300 tokens: registers)
+  // in five pieces: no division for each
   const int lg = F32 ? min(5, __clz(N - 1) - 27) : 0;
   const int copy_tok = warp >> lg, copy_pc = ((warp & ((1 << lg) - 1)) << 5) + lane, copy_stride = 32 << lg;
   uint4 pre[kInFlight];
@@ -344,66 +338,33 @@ __device__ __forceinline__ void front_small_body(float* smem,
   if constexpr (SPLIT) {
     const int nb = nblk, b = blk;
     float* xps = reinterpret_cast<float*>(xch + nb * k * E);    // [nb][E] probability sums
-    static_assert((F32 ? 8 : 32) * 16 * 8 * NT >= 128 * 8 * NT, "128 blocks' sums of 8 NT experts in [nslices][16][8 NT]");
-    // (fp32: a count's blocks side by side, for a warp to add)
-    if (tid < k * E) xch[F32 ? tid * nb + b : b * k * E + tid] = s_cnt[(tid / E) * kMaxE + tid % E];
+    static_assert(32 * 4 >= 128, "128 blocks' sums of 8 NT experts in [nslices][tok_pitch][8 NT]");
+    // (a count's blocks side by side, for a warp to add)
+    if (tid < k * E) xch[tid * nb + b] = s_cnt[(tid / E) * kMaxE + tid % E];
     if (tid < E) {
       float ps = 0.f;
       for (int tok = 0; tok < N; ++tok) ps += s_logit[tok * ld + tid];
       xps[b * E + tid] = ps;
     }
     for (int i = tid; i < kMaxE + kMaxTopK * kMaxE; i += kThreads) s_base[i] = 0;   // s_base, s_tot
-    // fp32: the status words are this call's; what a block has to say it says behind the barrier
-    if (F32 && b == 0 && tid < MOE_B200_STATUS_INTS) status[tid] = 0;
+    // the status words are this call's; what a block has to say it says behind the barrier
+    if (b == 0 && tid < MOE_B200_STATUS_INTS) status[tid] = 0;
     __threadfence();
-    if constexpr (F32) {
-      if (nblk > 1) cooperative_groups::this_grid().sync();
-      else __syncthreads();
-    } else {
-      __syncthreads();
-      if (tid == 0) {
-        atomicAdd(counter, 1);
-        unsigned long long t0 = 0;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-        for (uint32_t it = 0; ld_acquire_gpu_i32(counter) < nb; ++it) {
-          if ((it & 63u) == 63u) {
-            unsigned long long t1;
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-            if (t1 - t0 > 2000000000ull) {     // 2 s: some block of the grid never arrived
-              atomicMax(&status[0], MOE_B200_DEV_TIMEOUT);
-              status[1] = 41;
-              status[2] = b;
-              break;
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
+    if (nblk > 1) cooperative_groups::this_grid().sync();
+    else __syncthreads();
     // totals per (slot, expert) and the rows that earlier blocks put in front of this block's
-    if constexpr (F32) {
-      for (int je = warp; je < k * E; je += kThreads / 32) {
-        unsigned sum = 0;      // both, 16 bits each: 2048 tokens at most
-        for (int bb = lane; bb < nb; bb += 32) {
-          const unsigned c = (unsigned)__ldcg(&xch[je * nb + bb]);
-          sum += c | (bb < b ? c << 16 : 0u);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) {
-          const int j = je / E, e = je - j * E;
-          s_tot[j * kMaxE + e] = (int)(sum & 0xffffu);
-          if (sum >> 16) atomicAdd(&s_base[e], (int)(sum >> 16));
-        }
+    for (int je = warp; je < k * E; je += kThreads / 32) {
+      unsigned sum = 0;      // both, 16 bits each: 2048 tokens at most
+      for (int bb = lane; bb < nb; bb += 32) {
+        const unsigned c = (unsigned)__ldcg(&xch[je * nb + bb]);
+        sum += c | (bb < b ? c << 16 : 0u);
       }
-    }
-    for (int i = tid; !F32 && i < nb * k * E; i += kThreads) {
-      const int c = __ldcg(&xch[i]);
-      const int bb = i / (k * E), je = i - bb * (k * E);
-      const int j = je / E, e = je - j * E;
-      if (c != 0) {
-        atomicAdd(&s_tot[j * kMaxE + e], c);
-        if (bb < b) atomicAdd(&s_base[e], c);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0) {
+        const int j = je / E, e = je - j * E;
+        s_tot[j * kMaxE + e] = (int)(sum & 0xffffu);
+        if (sum >> 16) atomicAdd(&s_base[e], (int)(sum >> 16));
       }
     }
     // the blocks' probability sums, for the loss
@@ -565,11 +526,6 @@ __device__ __forceinline__ void front_small_body(float* smem,
       for (int e = 0; e < E; ++e) a += s_part[1024 + e];
       aux[0] = a / (float)E * (float)(E * E);
     }
-  }
-  if constexpr (SPLIT && !F32) {
-    // the last block to leave puts the meeting counter back to zero for the next call
-    __syncthreads();
-    if (tid == 0 && atomicAdd(counter, 1) == 2 * nblk - 1) *counter = 0;
   }
 }
 

@@ -110,6 +110,13 @@ def test_front_small_equals_router_plus_dispatch(cuda_device, N, d, E, k, split)
         assert torch.equal(got["cnt_slot"].cpu().long(), r["cnt_slot"])
 
 
+# more than 128 tokens: a last block of one token, rows of fewer and more pieces than a warp has under way, chunks of K for a few
+# warps and for several rounds, one expert and as many as there can be, all slots
+@pytest.mark.parametrize("N,d,E,k", [(129, 8, 1, 1), (145, 4104, 8, 2), (600, 1032, 9, 8), (1041, 40, 32, 8), (2047, 2048, 17, 1)])
+def test_front_of_many_tokens(cuda_device, N, d, E, k):
+    test_front_small_equals_router_plus_dispatch(cuda_device, N, d, E, k, True)
+
+
 DISPATCH_CASES = [(1, 64, 8, 2), (2, 64, 8, 2), (63, 64, 8, 2), (64, 64, 8, 2), (65, 64, 8, 2),
                   (129, 128, 8, 2), (1000, 256, 64, 4), (5000, 512, 8, 2), (333, 72, 5, 3),
                   (4097, 64, 256, 8), (40000, 64, 8, 2)]
