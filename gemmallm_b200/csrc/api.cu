@@ -51,7 +51,7 @@ static void layout(int64_t N, int d, int f, int E, int k, int dtype, size_t* off
   sizes[MOE_B200_WS_PSUM] = (size_t)E * sizeof(float);
   sizes[MOE_B200_WS_AUX] = sizeof(float);
   sizes[MOE_B200_WS_SCRATCH] = (size_t)dispatch_scratch_ints(N, E, k) * sizeof(int32_t);
-  if ((dtype == MOE_B200_F32 ? front_f32_supported(N, E, k) : front_split_supported(N, E, k, dtype)) &&
+  if ((dtype == MOE_B200_F32 ? front_f32_supported(N, E, k) : front_split_supported(N, d, E, k, dtype)) &&
       (size_t)front_small_exchange_ints(N, E, k) * sizeof(int32_t) > sizes[MOE_B200_WS_SCRATCH])
     sizes[MOE_B200_WS_SCRATCH] = (size_t)front_small_exchange_ints(N, E, k) * sizeof(int32_t);
   sizes[MOE_B200_WS_CNT_SLOT] = (size_t)k * E * sizeof(int32_t);
@@ -320,7 +320,7 @@ int moe_b200_front_small_split(const void* x, const void* Wg, const void* bg, in
                                int32_t* status, void* stream) {
   int rc = check_shape(N, d, 8, E, k, dtype);
   if (rc) return rc;
-  if (!front_split_supported(N, E, k, dtype))
+  if (E > 32 || !front_split_supported(N, d, E, k, dtype))
     return set_error(MOE_B200_ERR_UNSUPPORTED,
                      "moe_b200_front_small_split needs bf16, 1 <= N <= 2048, E <= 32");
   if (!x || !Wg || !bg || !out_idx || !out_w || !cnt_slot || !offsets || !row_of || !perm || !psum ||
@@ -497,15 +497,15 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   // (a folded LayerNorm stays with the general kernels)
   bool front32 = dtype == MOE_B200_F32 && !norm && front_f32_supported(N, E, k);
   bool front = front32 || ((small_n || rows_path) && (front_small_supported(N, E, k, dtype) ||
-                                                            front_split_supported(N, E, k, dtype)));
+                                                            front_split_supported(N, d, E, k, dtype)));
   // The small calls launch their kernels below without the entry points that test this, and a LayerNorm reads x before
   // they do. (The folded LayerNorm of the large calls reads Wg an element at a time.)
   if (N > 0 && (!aligned16(x) || ((tiny || front) && !aligned16(Wg))))
     return set_error(MOE_B200_ERR_ALIGN, "x and Wg must be 16-byte aligned");
-  if (front32) {
-    rc = front_f32_resident(N, &front32);
+  if (front32 || (front && (N > 128 || E > 32))) {      // blocks that meet
+    rc = front_resident(N, dtype, &front);
     if (rc) return rc;
-    front = front32;
+    front32 = front32 && front;
   }
   const bool counters = small_n || rows_path || mid;
   const bool clean = (small_n || rows_path) && (flags & MOE_B200_FLAG_WS_CLEAN);

@@ -365,7 +365,7 @@ int launch_ep_dispatch(const void* x, const int32_t* idx, int64_t N, int d, int 
                        int64_t n_total, int32_t* status, cudaStream_t s);
 bool front_small_supported(int64_t N, int E, int k, int dtype);
 int64_t front_small_exchange_ints(int64_t N, int E, int k);
-bool front_split_supported(int64_t N, int E, int k, int dtype);
+bool front_split_supported(int64_t N, int d, int E, int k, int dtype);
 int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E, int k,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
@@ -374,7 +374,7 @@ int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N,
 // fp32, with the exchange buffer and room for the rows' bf16 planes [3][N k][d]; on this device only if its blocks are all
 // resident at once
 bool front_f32_supported(int64_t N, int E, int k);
-int front_f32_resident(int64_t N, bool* yes);
+int front_resident(int64_t N, int dtype, bool* yes);
 int encode_tmap_2d(void* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
                    uint32_t box_cols = 64);
 // [3][rows, cols] bf16, boxes of 32 columns x box_rows x 3

@@ -40,8 +40,11 @@ front_small_kernel(const T* __restrict__ x, const T* Wg, const T* bg, int Ntotal
 // at a counter (up to 128 of them, one an SM, on an otherwise idle GPU); the wait is bounded and reports a time-out.
 // (front_small_body did it with 32 warps: 9.4 us from the wait to the end at 300 tokens, where this kernel takes 7.2. Whole
 // calls, d 1024, f 4096, 8 experts: 130 tokens 53.1 -> 51.6 us, 300 59.3 -> 57.9, 400 62.0 -> 60.9, 1173 88.0 -> 86.8.)
-constexpr int kMidWarps = 16, kMidTok = 16;
+constexpr int kMidWarps = 16, kMidTok = 16, kMidMaxE = 64;
 
+// More than 32 experts, two a lane: calls of up to 2048 tokens and 4096 rows, from one token on (d 2048, 64 experts of f 1408,
+// four slots, whole calls against the general router and dispatch: 1 token 60.4 -> 48.2 us, 8 111 -> 98.5, 100 206 -> 198,
+// 1000 213 -> 200).
 template <int NT>      // 8 NT >= E
 __global__ void __launch_bounds__(32 * kMidWarps, 1)
 front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfloat16* bg, int Ntotal, int d, int E, int k,
@@ -49,12 +52,15 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
                  int32_t* __restrict__ cnt_slot, int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
                  __nv_bfloat16* __restrict__ perm, float* __restrict__ psum, float* __restrict__ aux, int* __restrict__ xch,
                  int* __restrict__ counter, int32_t* __restrict__ status) {
-  constexpr int ET = 8 * NT, P = 32 / ET;
-  constexpr int kInFlight = 4;
-  __shared__ __align__(16) float s_part[kMidWarps][kMidTok][ET];    // then block 0's probability sums of all blocks
+  constexpr int ET = 8 * NT, EL = ET > 32 ? 2 : 1, GL = ET / EL, P = 32 / GL;      // experts a lane, lanes of a token
+  constexpr int kInFlight = 4, kChunks = NT > 4 ? 1 : 2;       // of a row to copy; of K
+  extern __shared__ __align__(16) float s_dyn[];
+  float (*s_part)[kMidTok][ET] = reinterpret_cast<float (*)[kMidTok][ET]>(s_dyn);   // [kMidWarps]; then block 0's probability
+                                                                                    // sums of all blocks
   __shared__ float s_prob[kMidTok][ET];
-  __shared__ int s_idx[kMidTok * kMaxTopK], s_row[kMidTok * kMaxTopK], s_tot[kMaxTopK * kMaxE], s_base[kMaxE];
-  static_assert(sizeof(s_part) >= 128 * ET * sizeof(float), "the sums of 128 blocks");
+  __shared__ int s_idx[kMidTok * kMaxTopK], s_row[kMidTok * kMaxTopK], s_tot[kMaxTopK * ET], s_base[ET];
+  static_assert(kMidWarps * kMidTok >= 128, "the sums of 128 blocks");
+  static_assert(EL == 1 || kMaxTopK * ET == 32 * kMidWarps, "a thread per count");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int b = (int)blockIdx.x, nb = (int)gridDim.x;
   const int N = min(kMidTok, Ntotal - b * kMidTok);
@@ -63,7 +69,8 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   out_idx += (size_t)b * kMidTok * k;
   out_w += (size_t)b * kMidTok * k;
   row_of += (size_t)b * kMidTok * k;
-  if (tid < kMaxE) s_base[tid] = 0;
+  if (tid < ET) s_base[tid] = 0;
+  if (EL > 1) s_tot[tid] = 0;      // (32 kMidWarps of them)
   pdl_wait();                 // x may come from the kernel before this one
   pdl_launch_dependents();
 
@@ -76,16 +83,18 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   const uint4* xa = reinterpret_cast<const uint4*>(x) + (size_t)min(g, N - 1) * pieces + t;
   const uint4* xb = reinterpret_cast<const uint4*>(x) + (size_t)min(g + 8, N - 1) * pieces + t;
   const uint4* wg = reinterpret_cast<const uint4*>(Wg) + t;
-  const float bias = lane % ET < E ? to_f32(bg[lane % ET]) : 0.f;
+  float bias[EL];
+#pragma unroll
+  for (int i = 0; i < EL; ++i) bias[i] = lane % GL + 32 * i < E ? to_f32(bg[lane % GL + 32 * i]) : 0.f;
   float acc[NT][4];
 #pragma unroll
   for (int j = 0; j < NT; ++j)
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
-  for (int c0 = warp; c0 < nchunk; c0 += 2 * kMidWarps) {
-    uint4 A[2], B[2], W[2][NT];
+  for (int c0 = warp; c0 < nchunk; c0 += kChunks * kMidWarps) {
+    uint4 A[kChunks], B[kChunks], W[kChunks][NT];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < kChunks; ++u) {
       const int p = 4 * (c0 + u * kMidWarps);
       const bool ok = p + t < pieces;
       A[u] = ok ? __ldcg(xa + p) : zero;
@@ -94,7 +103,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
       for (int j = 0; j < NT; ++j) W[u][j] = ok ? wg[(size_t)min(8 * j + g, E - 1) * pieces + p] : zero;
     }
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+    for (int u = 0; u < kChunks; ++u)
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
         mma_bf16_16816(acc[j], A[u].x, B[u].x, A[u].y, B[u].y, W[u][j].x, W[u][j].y);
@@ -110,37 +119,55 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
 
   // ---- softmax, top-k, renormalise: a warp per token; lane = expert, groups of lanes share the sum over the slices ----
   if (warp < N) {
-    const int e = lane % ET;
-    float v = 0.f;
+    const int e0 = lane % GL;
+    float v[EL], p[EL], sum = 0.f;
+    unsigned key[EL], kmax = 0u;
 #pragma unroll
-    for (int q = 0; q < kMidWarps / P; ++q) v += s_part[q * P + lane / ET][warp][e];
+    for (int i = 0; i < EL; ++i) {
+      const int e = e0 + 32 * i;
+      v[i] = 0.f;
 #pragma unroll
-    for (int o = ET; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    v += bias;
-    const bool live = e < E;
-    if (out_logits != nullptr && lane < E) out_logits[((size_t)b * kMidTok + warp) * E + lane] = v;
-    v = live ? v + 0.f : -INFINITY;      // + 0: no negative zero
-    const unsigned u = __float_as_uint(v);
-    unsigned key = (u & 0x80000000u) ? ~u : (u | 0x80000000u);      // order-preserving; NaN is the largest
-    const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
+      for (int q = 0; q < kMidWarps / P; ++q) v[i] += s_part[q * P + lane / GL][warp][e];
+#pragma unroll
+      for (int o = GL; o < 32; o <<= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+      v[i] += bias[i];
+      if (out_logits != nullptr && lane < GL && e < E) out_logits[((size_t)b * kMidTok + warp) * E + e] = v[i];
+      const bool live = e < E;
+      v[i] = live ? v[i] + 0.f : -INFINITY;      // + 0: no negative zero
+      const unsigned u = __float_as_uint(v[i]);
+      key[i] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);      // order-preserving; NaN is the largest
+      kmax = max(kmax, key[i]);
+    }
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
     const float m = __uint_as_float((kmax & 0x80000000u) ? (kmax & 0x7fffffffu) : ~kmax);
-    const float p = live ? expf(v - m) : 0.f;
-    float sum = p;
 #pragma unroll
-    for (int o = ET / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    for (int i = 0; i < EL; ++i) {
+      p[i] = e0 + 32 * i < E ? expf(v[i] - m) : 0.f;
+      sum += p[i];
+    }
+#pragma unroll
+    for (int o = GL / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const float inv_sum = __frcp_rn(sum);
-    if (lane < ET) s_prob[warp][lane] = p * inv_sum;
+#pragma unroll
+    for (int i = 0; i < EL; ++i)
+      if (lane < GL) s_prob[warp][lane + 32 * i] = p[i] * inv_sum;
     int my_sel = 0;
     float my_val = 0.f, total = 0.f;
 #pragma unroll 1
     for (int j = 0; j < k; ++j) {
-      const unsigned km = __reduce_max_sync(0xffffffffu, key);
-      const int winner = __ffs(__ballot_sync(0xffffffffu, key == km)) - 1;      // in the first group
+      unsigned km = key[0];
+      if (EL > 1) km = max(km, key[EL - 1]);
+      km = __reduce_max_sync(0xffffffffu, km);
+      const unsigned low = __ballot_sync(0xffffffffu, key[0] == km);      // (the first group's lanes come first)
+      const unsigned high = EL > 1 ? __ballot_sync(0xffffffffu, key[EL - 1] == km) : 0u;
+      const int winner = low != 0u ? __ffs(low) - 1 : 31 + __ffs(high);
       const float bv = __uint_as_float((km & 0x80000000u) ? (km & 0x7fffffffu) : ~km);
       const float val = expf(bv - m) * inv_sum;
       total += val;
       if (lane == j) { my_sel = winner; my_val = val; }
-      if (e == winner) key = 0u;     // below every real key
+#pragma unroll
+      for (int i = 0; i < EL; ++i)
+        if (e0 + 32 * i == winner) key[i] = 0u;     // below every real key
     }
     if (lane < k) {
       s_idx[warp * k + lane] = my_sel;
@@ -149,79 +176,107 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
     }
   } else {      // (no token: below, nothing has to ask)
     if (lane < k) s_idx[warp * k + lane] = -1;
-    if (lane < ET) s_prob[warp][lane] = 0.f;
+    for (int e = lane; e < ET; e += 32) s_prob[warp][e] = 0.f;
   }
   __syncthreads();
 
-  // ---- this block's counts per (slot, expert), a count's blocks side by side, and its probability sums ----
-  float* xps = reinterpret_cast<float*>(xch + nb * k * E);    // [nb][E]
-  if (tid < k * E) {
+  // ---- this block's counts per (slot, expert), a count's blocks side by side (a block's counts, with more than 32 experts),
+  // and its probability sums ----
+  float* s_sum = s_dyn;
+  const int ke = k * E;
+  float* xps = reinterpret_cast<float*>(xch + nb * ke);    // [nb][E]
+  for (int i = tid; i < ke; i += 32 * kMidWarps) {
     int c = 0;
-    const int j = tid / E, e = tid - j * E;
+    const int j = i / E, e = i - j * E;
 #pragma unroll
     for (int tok = 0; tok < kMidTok; ++tok) c += s_idx[tok * k + j] == e ? 1 : 0;
-    xch[tid * nb + b] = c;
-  } else if (tid >= 32 * kMidWarps - E) {
+    if (nb == 1) s_tot[i] = c;
+    else xch[EL > 1 ? b * ke + i : i * nb + b] = c;
+  }
+  if (tid >= 32 * kMidWarps - E) {
     const int e = tid - (32 * kMidWarps - E);
     float ps = 0.f;
 #pragma unroll
     for (int tok = 0; tok < kMidTok; ++tok) ps += s_prob[tok][e];
-    xps[b * E + e] = ps;
+    if (nb == 1) s_sum[e] = ps;
+    else xps[b * E + e] = ps;
   }
   __syncthreads();
   int left = 0;
-  if (tid == 0) {
-    __threadfence();
-    atomicAdd(counter, 1);
-    unsigned long long t0 = 0;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-    for (uint32_t it = 0; ld_acquire_gpu_i32(counter) < nb; ++it) {
-      if ((it & 63u) == 63u) {
-        unsigned long long t1;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-        if (t1 - t0 > 2000000000ull) {     // 2 s: some block of the grid never arrived
-          atomicMax(&status[0], MOE_B200_DEV_TIMEOUT);
-          status[1] = 41;
-          status[2] = b;
-          break;
+  if (nb > 1) {
+    if (tid == 0) {
+      __threadfence();
+      atomicAdd(counter, 1);
+      unsigned long long t0 = 0;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+      for (uint32_t it = 0; ld_acquire_gpu_i32(counter) < nb; ++it) {
+        if ((it & 63u) == 63u) {
+          unsigned long long t1;
+          asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+          if (t1 - t0 > 2000000000ull) {     // 2 s: some block of the grid never arrived
+            atomicMax(&status[0], MOE_B200_DEV_TIMEOUT);
+            status[1] = 41;
+            status[2] = b;
+            break;
+          }
         }
       }
+      left = atomicAdd(counter, 1);      // looked at in the end
     }
-    left = atomicAdd(counter, 1);      // looked at in the end
+    __syncthreads();
+    // totals, and the rows that earlier blocks put in front of this block's (16 bits: 2048 tokens)
+    if (EL == 1) {      // a warp per count
+      for (int je = warp; je < ke; je += kMidWarps) {
+        unsigned both = 0;
+        for (int bb = lane; bb < nb; bb += 32) {
+          const unsigned c = (unsigned)__ldcg(&xch[je * nb + bb]);
+          both += c | (bb < b ? c << 16 : 0u);
+        }
+        both = __reduce_add_sync(0xffffffffu, both);
+        if (lane == 0) {
+          s_tot[je] = (int)(both & 0xffffu);
+          if (both >> 16) atomicAdd(&s_base[je % E], (int)(both >> 16));
+        }
+      }
+    } else {            // a thread per count, or several (a warp per count: 16 rounds of loads one after the other)
+      const int per = 32 * kMidWarps / ke, q = tid / ke, je = tid - q * ke;
+      if (q < per) {
+        unsigned both = 0;
+#pragma unroll 8
+        for (int bb = q; bb < nb; bb += per) {
+          const unsigned c = (unsigned)__ldcg(&xch[bb * ke + je]);
+          both += c | (bb < b ? c << 16 : 0u);
+        }
+        if (both & 0xffffu) atomicAdd(&s_tot[je], (int)(both & 0xffffu));
+        if (both >> 16) atomicAdd(&s_base[je % E], (int)(both >> 16));
+      }
+    }
+    if (b == 0)
+      for (int i = tid; i < nb * E; i += 32 * kMidWarps) s_sum[i] = __ldcg(&xps[i]);
+    __syncthreads();
   }
-  __syncthreads();
-  // totals, and the rows that earlier blocks put in front of this block's: a warp each (16 bits: 2048 tokens)
-  for (int je = warp; je < k * E; je += kMidWarps) {
-    unsigned both = 0;
-    for (int bb = lane; bb < nb; bb += 32) {
-      const unsigned c = (unsigned)__ldcg(&xch[je * nb + bb]);
-      both += c | (bb < b ? c << 16 : 0u);
-    }
-    both = __reduce_add_sync(0xffffffffu, both);
-    if (lane == 0) {
-      s_tot[je] = (int)(both & 0xffffu);
-      if (both >> 16) atomicAdd(&s_base[je % E], (int)(both >> 16));
-    }
-  }
-  float* s_sum = &s_part[0][0][0];
-  if (b == 0)
-    for (int i = tid; i < nb * E; i += 32 * kMidWarps) s_sum[i] = __ldcg(&xps[i]);
-  __syncthreads();
 
   // ---- offsets (every warp), stable ranks in (token, slot) order: a warp per expert, 32 pairs at a time ----
-  int tot = 0;
-  if (lane < E)
-    for (int j = 0; j < k; ++j) tot += s_tot[j * E + lane];
-  int incl = tot;
+  int first[EL], mine0[EL], before = 0;      // of experts lane, 32 + lane: first row; first row of this block's tokens
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int up = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += up;
+  for (int i = 0; i < EL; ++i) {
+    const int e = lane + 32 * i;
+    int tot = 0;
+    if (e < E)
+      for (int j = 0; j < k; ++j) tot += s_tot[j * E + e];
+    int incl = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    first[i] = before + incl - tot;
+    mine0[i] = first[i] + (e < E ? s_base[e] : 0);
+    before += __shfl_sync(0xffffffffu, incl, 31);
   }
-  const int mine0 = incl - tot + (lane < E ? s_base[lane] : 0);      // first row of this block's tokens
   const int npair = N * k;
   for (int e = warp; e < E; e += kMidWarps) {
-    int next = __shfl_sync(0xffffffffu, mine0, e);
+    int next = __shfl_sync(0xffffffffu, EL > 1 && e >= 32 ? mine0[EL - 1] : mine0[0], e & 31);
     for (int p0 = 0; p0 < npair; p0 += 32) {
       const int p = p0 + lane;
       const bool mine = p < npair && s_idx[p] == e;
@@ -249,46 +304,58 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
     }
   if (b == 0) {
     if (warp == kMidWarps - 1) {
-      if (lane < E) {
-        for (int j = 0; j < k; ++j) cnt_slot[j * E + lane] = s_tot[j * E + lane];
-        offsets[lane] = incl - tot;
+#pragma unroll
+      for (int i = 0; i < EL; ++i) {
+        const int e = lane + 32 * i;
+        if (e < E) {
+          for (int j = 0; j < k; ++j) cnt_slot[j * E + e] = s_tot[j * E + e];
+          offsets[e] = first[i];
+        }
       }
-      if (lane == 31) offsets[E] = incl;
+      if (lane == 31) offsets[E] = before;
     }
     if (warp == kMidWarps - 2) {      // the loss (model.py:213-216)
-      float term = 0.f;
-      if (lane < E) {
-        float ps = 0.f;
-#pragma unroll 8
-        for (int bb = 0; bb < nb; ++bb) ps += s_sum[bb * E + lane];      // in block order
-        psum[lane] = ps;
-        term = (ps / (float)Ntotal) * ((float)s_tot[lane] / (float)Ntotal);
-      }
       float a = 0.f;
-      for (int e = 0; e < E; ++e) a += __shfl_sync(0xffffffffu, term, e);
+#pragma unroll
+      for (int i = 0; i < EL; ++i) {
+        const int e = lane + 32 * i;
+        float term = 0.f;
+        if (e < E) {
+          float ps = 0.f;
+#pragma unroll 8
+          for (int bb = 0; bb < nb; ++bb) ps += s_sum[bb * E + e];      // in block order
+          psum[e] = ps;
+          term = (ps / (float)Ntotal) * ((float)s_tot[e] / (float)Ntotal);
+        }
+        for (int q = 0; q < 32 && q + 32 * i < E; ++q) a += __shfl_sync(0xffffffffu, term, q);
+      }
       if (lane == 0) aux[0] = a / (float)E * (float)(E * E);
     }
   }
   // the last block to leave puts the meeting counter back to zero for the next call
-  if (tid == 0 && left == 2 * nb - 1) *counter = 0;
+  if (tid == 0 && nb > 1 && left == 2 * nb - 1) *counter = 0;
+}
+
+template <int NT>
+int launch_mid(const void* x, const void* Wg, const void* bg, int N, int d, int E, int k, float* out_logits, int32_t* out_idx,
+               float* out_w, int32_t* cnt_slot, int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux, int* xch,
+               int* counter, int32_t* status, cudaStream_t s) {
+  const size_t smem = sizeof(float) * kMidWarps * kMidTok * 8 * NT;
+  static PerDeviceOnce once;
+  int rc = ensure_dynamic_smem(once, front_mid_kernel<NT>, smem);
+  if (rc) return rc;
+  MOE_CUDA_CHECK(launch_pdl(front_mid_kernel<NT>, dim3((N + kMidTok - 1) / kMidTok), dim3(32 * kMidWarps), smem, s,
+                            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(Wg),
+                            static_cast<const __nv_bfloat16*>(bg), N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
+                            row_of, static_cast<__nv_bfloat16*>(perm), psum, aux, xch, counter, status));
+  return 0;
 }
 
 template <int NT, typename T>
 int launch(const void* x, const void* Wg, const void* bg, int N, int d, int E, int k,
            float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot, int32_t* offsets,
-           int32_t* row_of, void* perm, void* planes, float* psum, float* aux, int* xch, int* counter,
-           int32_t* status, cudaStream_t s) {
-  // beyond 128 tokens repeating the routing in every block costs more than one exchange
+           int32_t* row_of, void* perm, void* planes, float* psum, float* aux, int* xch, int32_t* status, cudaStream_t s) {
   constexpr bool F32 = sizeof(T) == 4;
-  if constexpr (!F32) {
-    if (xch != nullptr && counter != nullptr && status != nullptr && N > 128) {
-      MOE_CUDA_CHECK(launch_pdl(front_mid_kernel<NT>, dim3((N + kMidTok - 1) / kMidTok), dim3(32 * kMidWarps), 0, s,
-                                static_cast<const T*>(x), static_cast<const T*>(Wg), static_cast<const T*>(bg), N, d, E, k,
-                                out_logits, out_idx, out_w, cnt_slot, offsets, row_of, static_cast<T*>(perm), psum, aux, xch,
-                                counter, status));
-      return 0;
-    }
-  }
   const int per = F32 ? f32_tokens_per_block(N) : 16;
   const size_t smem = front_small_smem_bytes(NT, F32 ? per : N, E, k) + (F32 ? front_f32_chunk_bytes(NT) : 0);
   static PerDeviceOnce once;
@@ -311,8 +378,10 @@ bool front_small_supported(int64_t N, int E, int k, int dtype) {
 
 // With the exchange buffer and the counter (blocks share the work): as many tokens as give a grid
 // whose blocks are all resident at once with room to spare.
-bool front_split_supported(int64_t N, int E, int k, int dtype) {
-  return dtype == MOE_B200_BF16 && N >= 1 && N <= 16 * 128 && E <= kMaxE && k <= kMaxTopK;
+// (More than 32 experts where the general router is the tcgen05 kernel, whose choice among logits that are not finite is also
+// always an expert.)
+bool front_split_supported(int64_t N, int d, int E, int k, int dtype) {
+  return dtype == MOE_B200_BF16 && N >= 1 && N <= 16 * 128 && E <= kMidMaxE && (E <= kMaxE || d >= 64) && k <= kMaxTopK;
 }
 
 // xch: int32 scratch of at least front_small_exchange_ints(N, E, k) words and counter: one int32
@@ -330,10 +399,10 @@ bool front_f32_supported(int64_t N, int E, int k) {
   return N >= 1 && N <= 16 * 128 && E <= kMaxE && k <= kMaxTopK && N * k <= kRowsPathMaxRows;
 }
 
-int front_f32_resident(int64_t N, bool* yes) {
+int front_resident(int64_t N, int dtype, bool* yes) {
   int sms = 0;
   int rc = N > 16 ? sm_count(&sms) : 0;
-  const int per = f32_tokens_per_block(N);
+  const int per = dtype == MOE_B200_F32 ? f32_tokens_per_block(N) : kMidTok;
   *yes = rc == 0 && (N <= 16 || (N + per - 1) / per <= sms);
   return rc;
 }
@@ -353,9 +422,15 @@ int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N,
                        cudaStream_t s, int* xch, int* counter, int32_t* status, int dtype, void* planes) {
   if (dtype == MOE_B200_F32)
     return launch_by_experts<float>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of,
-                                    perm, planes, psum, aux, xch, counter, status, s);
+                                    perm, planes, psum, aux, xch, status, s);
+  // beyond 128 tokens repeating the routing in every block costs more than one exchange
+  if (xch != nullptr && counter != nullptr && status != nullptr && (N > 128 || E > kMaxE)) {
+    auto mid = E <= 8 ? launch_mid<1> : E <= 16 ? launch_mid<2> : E <= 32 ? launch_mid<4> : launch_mid<8>;
+    return mid(x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux, xch, counter,
+               status, s);
+  }
   return launch_by_experts<__nv_bfloat16>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
-                                          row_of, perm, nullptr, psum, aux, xch, counter, status, s);
+                                          row_of, perm, nullptr, psum, aux, xch, status, s);
 }
 
 }  // namespace moe

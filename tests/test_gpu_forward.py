@@ -174,6 +174,39 @@ def test_fp32_tokens_of_nan(cuda_device, N, fold):
             assert m(bad, norm=norm)[0][0, rows].eq(0).all() and m.device_status() == 2
 
 
+# a whole bf16 call of 33 to 64 experts: one token, a block of one and of all 16, streaming and sorted-row sizes, one slot and eight
+@pytest.mark.parametrize("N,d,E,k", [(1, 64, 33, 1), (16, 2056, 64, 4), (33, 72, 63, 8), (130, 1024, 40, 2), (511, 520, 64, 8),
+                                     (2048, 64, 64, 2)])
+def test_routing_of_many_experts(cuda_device, N, d, E, k):
+    """As the general router and dispatch give it; a token of NaN is routed to experts and its output is NaN."""
+    x = torch.randn(N, d, generator=torch.Generator().manual_seed(E + N)).bfloat16().to(cuda_device)
+    params = synthetic.make_params(d, E, 64, seed=N)
+    m = build(params, d, E, 64, k, torch.bfloat16, cuda_device)
+    gate = (m.gate.weight.detach(), m.gate.bias.detach())
+    with torch.no_grad():
+        out = m(x.view(1, N, d))[0]
+    last = {n: t.clone() for n, t in m.last.items()}
+    assert m.device_status() == 0 and bool(out.isfinite().all())
+    logits, idx, w, psum_part = helpers.router(x, *gate, k)
+    # fp32 sums of d products in another order: d 2^-24 of their sum of magnitudes, at the worst
+    mag = x.float().abs() @ gate[0].float().abs().T + gate[1].float().abs()
+    assert bool(((last["logits"] - logits).abs() <= 2 * d * 2.0 ** -24 * mag).all())
+    r = moe_oracle.route_from_logits(last["logits"].cpu(), k)
+    ok = ~moe_oracle.tie_rows(r["probs"], k)
+    assert torch.equal(last["idx"].cpu()[ok].long(), r["idx"][ok])
+    assert torch.allclose(last["w"].cpu()[ok], r["w"][ok], atol=2e-6, rtol=0)
+    disp = helpers.dispatch(x, last["idx"], E, psum_part)
+    for name in ("offsets", "row_of", "cnt_slot"):
+        assert torch.equal(last[name], disp[name]), name
+    bad = x.clone()
+    bad[N // 2, 3] = float("nan")
+    with torch.no_grad():
+        got = m(bad.view(1, N, d))[0][0]
+    assert m.device_status() == 0 and bool(got[N // 2].isnan().all())
+    others = torch.arange(N, device=cuda_device) != N // 2
+    assert bool(got[others].isfinite().all())
+
+
 @pytest.mark.parametrize("E,k", [(8, 2), (9, 8), (17, 3), (32, 4)])
 def test_fp32_logits_that_are_not_finite(cuda_device, E, k):
     """Routing in one launch as the general kernel gives it: gate biases of NaN and both infinities, for some experts up
