@@ -12,7 +12,8 @@ constexpr int kMaxE = kFrontMaxE;
 constexpr int kMaxPairs = kFrontMaxPairs;
 
 // fp32 tokens of a block: as few as 128 blocks allow, but four (their rows' copies and parts are the longest step of a block of
-// 16, which stores 160 KB at d 512: 512 tokens 81.8 -> 76.0 us, 51 tokens 58.5 -> 55.1, 1024 134 -> 130). Up to 16 are one block's, which need not meet any other.
+// 16, which stores 160 KB at d 512: 512 tokens 81.8 -> 76.0 us, 51 tokens 58.5 -> 55.1, 1024 134 -> 130). Up to 16 are one
+// block's, which need not meet any other.
 int f32_tokens_per_block(int64_t N) {
   if (N <= 16) return 16;
   const int64_t per = (N + 127) / 128;
@@ -34,13 +35,23 @@ front_small_kernel(const T* __restrict__ x, const T* Wg, const T* bg, int Ntotal
                           psum, aux, xch, status, per);
 }
 
-// bf16 calls of more than 128 tokens: blocks of 16 tokens that share the work, of 16 warps. What a warp does counts four
+// bf16 calls of more than 128 tokens: blocks of up to 16 tokens that share the work, of 16 warps. What a warp does counts four
 // times and not eight, its loads (both its chunks of the tokens and of the weights, its token's row for the copy) are in flight
 // together without spills, a token's softmax and top-k are a warp's and not a few lanes', and no step divides. Blocks meet
 // at a counter (up to 128 of them, one an SM, on an otherwise idle GPU); the wait is bounded and reports a time-out.
 // (front_small_body did it with 32 warps: 9.4 us from the wait to the end at 300 tokens, where this kernel takes 7.2. Whole
 // calls, d 1024, f 4096, 8 experts: 130 tokens 53.1 -> 51.6 us, 300 59.3 -> 57.9, 400 62.0 -> 60.9, 1173 88.0 -> 86.8.)
 constexpr int kMidWarps = 16, kMidTok = 16, kMidMaxE = 64;
+
+// Tokens of a block, a power of two: fewer of them shorten the row copies, which the block's warps then share, and more blocks
+// lengthen the meeting and read the router's weights more often. Best of 2, 4, 8 and 16 (64 experts, d 2048: 60 tokens 89.3,
+// 87.9, 88.4, 92.1 us a call; 100 192.5, 190.1, 189.5, 193.5; 300 202.6, 199.6, 196.7, 198.3; 1000 -, 202.9, 203.4, 199.9;
+// 8 experts, d 1024: 130 51.0, 50.7, 50.7, 51.6; 300 57.8, 57.7, 57.5, 58.2; 600 -, 64.9, 64.3, 64.1; 1173 -, -, 87.7, 87.2).
+// Up to 8 tokens stay one block's, which need not meet any other.
+int mid_tokens_per_block(int64_t N) {
+  if (N <= 64) return N > 4 && N <= 8 ? 8 : 4;
+  return N <= 512 ? 8 : kMidTok;
+}
 
 // More than 32 experts, two a lane: calls of up to 2048 tokens and 4096 rows, from one token on (d 2048, 64 experts of f 1408,
 // four slots, whole calls against the general router and dispatch: 1 token 60.4 -> 48.2 us, 8 111 -> 98.5, 100 206 -> 198,
@@ -51,7 +62,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
                  float* __restrict__ out_logits, int32_t* __restrict__ out_idx, float* __restrict__ out_w,
                  int32_t* __restrict__ cnt_slot, int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
                  __nv_bfloat16* __restrict__ perm, float* __restrict__ psum, float* __restrict__ aux, int* __restrict__ xch,
-                 int* __restrict__ counter, int32_t* __restrict__ status) {
+                 int* __restrict__ counter, int32_t* __restrict__ status, int per, int share) {
   constexpr int ET = 8 * NT, EL = ET > 32 ? 2 : 1, GL = ET / EL, P = 32 / GL;      // experts a lane, lanes of a token
   constexpr int kInFlight = 4, kChunks = NT > 4 ? 1 : 2;       // of a row to copy; of K
   extern __shared__ __align__(16) float s_dyn[];
@@ -63,12 +74,12 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   static_assert(EL == 1 || kMaxTopK * ET == 32 * kMidWarps, "a thread per count");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int b = (int)blockIdx.x, nb = (int)gridDim.x;
-  const int N = min(kMidTok, Ntotal - b * kMidTok);
+  const int N = min(per, Ntotal - b * per);
   const int pieces = d >> 3, nchunk = (d + 31) >> 5;
-  x += (size_t)b * kMidTok * d;
-  out_idx += (size_t)b * kMidTok * k;
-  out_w += (size_t)b * kMidTok * k;
-  row_of += (size_t)b * kMidTok * k;
+  x += (size_t)b * per * d;
+  out_idx += (size_t)b * per * k;
+  out_w += (size_t)b * per * k;
+  row_of += (size_t)b * per * k;
   if (tid < ET) s_base[tid] = 0;
   if (EL > 1) s_tot[tid] = 0;      // (32 kMidWarps of them)
   pdl_wait();                 // x may come from the kernel before this one
@@ -76,10 +87,11 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
 
   // ---- logits: a warp's chunks of 32 of K, as in the body above ----
   const uint4 zero = make_uint4(0, 0, 0, 0);
-  const uint4* row = reinterpret_cast<const uint4*>(x) + (size_t)min(warp, N - 1) * pieces;      // the one this warp copies
+  const int own = warp / share, step = 32 * share, first_p = lane + 32 * (warp - own * share);     // the row this warp copies, from which
+  const uint4* row = reinterpret_cast<const uint4*>(x) + (size_t)min(own, N - 1) * pieces;         // piece on
   uint4 pre[kInFlight];
 #pragma unroll
-  for (int u = 0; u < kInFlight; ++u) pre[u] = lane + 32 * u < pieces ? __ldcg(row + lane + 32 * u) : zero;
+  for (int u = 0; u < kInFlight; ++u) pre[u] = first_p + step * u < pieces ? __ldcg(row + first_p + step * u) : zero;
   const uint4* xa = reinterpret_cast<const uint4*>(x) + (size_t)min(g, N - 1) * pieces + t;
   const uint4* xb = reinterpret_cast<const uint4*>(x) + (size_t)min(g + 8, N - 1) * pieces + t;
   const uint4* wg = reinterpret_cast<const uint4*>(Wg) + t;
@@ -131,7 +143,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
 #pragma unroll
       for (int o = GL; o < 32; o <<= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
       v[i] += bias[i];
-      if (out_logits != nullptr && lane < GL && e < E) out_logits[((size_t)b * kMidTok + warp) * E + e] = v[i];
+      if (out_logits != nullptr && lane < GL && e < E) out_logits[((size_t)b * per + warp) * E + e] = v[i];
       const bool live = e < E;
       v[i] = live ? v[i] + 0.f : -INFINITY;      // + 0: no negative zero
       const unsigned u = __float_as_uint(v[i]);
@@ -291,16 +303,16 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   }
   __syncthreads();
 
-  // ---- row copies: a warp per token ----
-  if (warp < N)
+  // ---- row copies: `share` warps per token ----
+  if (own < N)
     for (int j = 0; j < k; ++j) {
-      const int r = s_row[warp * k + j];
+      const int r = s_row[own * k + j];
       if ((unsigned)r >= (unsigned)(Ntotal * k)) continue;      // (counts of a block that never arrived)
       uint4* to = reinterpret_cast<uint4*>(perm + (size_t)r * d);
 #pragma unroll
       for (int u = 0; u < kInFlight; ++u)
-        if (lane + 32 * u < pieces) to[lane + 32 * u] = pre[u];
-      for (int p = lane + 32 * kInFlight; p < pieces; p += 32) to[p] = __ldcg(row + p);
+        if (first_p + step * u < pieces) to[first_p + step * u] = pre[u];
+      for (int p = first_p + step * kInFlight; p < pieces; p += step) to[p] = __ldcg(row + p);
     }
   if (b == 0) {
     if (warp == kMidWarps - 1) {
@@ -344,10 +356,11 @@ int launch_mid(const void* x, const void* Wg, const void* bg, int N, int d, int 
   static PerDeviceOnce once;
   int rc = ensure_dynamic_smem(once, front_mid_kernel<NT>, smem);
   if (rc) return rc;
-  MOE_CUDA_CHECK(launch_pdl(front_mid_kernel<NT>, dim3((N + kMidTok - 1) / kMidTok), dim3(32 * kMidWarps), smem, s,
+  const int per = mid_tokens_per_block(N);
+  MOE_CUDA_CHECK(launch_pdl(front_mid_kernel<NT>, dim3((N + per - 1) / per), dim3(32 * kMidWarps), smem, s,
                             static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(Wg),
                             static_cast<const __nv_bfloat16*>(bg), N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
-                            row_of, static_cast<__nv_bfloat16*>(perm), psum, aux, xch, counter, status));
+                            row_of, static_cast<__nv_bfloat16*>(perm), psum, aux, xch, counter, status, per, kMidWarps / per));
   return 0;
 }
 
@@ -388,8 +401,7 @@ bool front_split_supported(int64_t N, int d, int E, int k, int dtype) {
 // that is zero on entry (both only used beyond 128 tokens; without them every block repeats the
 // whole routing at every size).
 int64_t front_small_exchange_ints(int64_t N, int E, int k) {
-  const int per = f32_tokens_per_block(N);      // no fewer blocks than bf16 has
-  const int64_t nb = (N + per - 1) / per;
+  const int64_t nb = N < 512 ? (N + 3) / 4 : 128;      // the most that either type has
   return nb * k * E + nb * E;
 }
 
@@ -401,9 +413,9 @@ bool front_f32_supported(int64_t N, int E, int k) {
 
 int front_resident(int64_t N, int dtype, bool* yes) {
   int sms = 0;
-  int rc = N > 16 ? sm_count(&sms) : 0;
-  const int per = dtype == MOE_B200_F32 ? f32_tokens_per_block(N) : kMidTok;
-  *yes = rc == 0 && (N <= 16 || (N + per - 1) / per <= sms);
+  int rc = N > 8 ? sm_count(&sms) : 0;
+  const int per = dtype == MOE_B200_F32 ? f32_tokens_per_block(N) : mid_tokens_per_block(N);
+  *yes = rc == 0 && (N + per - 1) / per <= (N > 8 ? sms : 1);
   return rc;
 }
 
