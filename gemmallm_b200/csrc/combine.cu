@@ -6,7 +6,8 @@
 // model.py:264-271, and the `tensor += skip_connection` of model.py:319.
 //
 // HBM-bound gather (no atomics, deterministic): each thread produces eight
-// consecutive output elements from k 16-byte (bf16) or 32-byte (fp32) loads.
+// consecutive output elements from k 16-byte (bf16) or 32-byte (fp32) loads, which for one, two and four slots are all under
+// way together with the skip connection's.
 #include "common.cuh"
 #include "ep_sync.cuh"
 
@@ -14,42 +15,97 @@ namespace moe {
 
 namespace {
 
+// Eight elements as they lie in memory.
 template <typename T>
+struct Eight {
+  uint4 raw[sizeof(T) / 2];
+  __device__ __forceinline__ void load(const T* p) {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T) / 2; ++i) raw[i] = reinterpret_cast<const uint4*>(p)[i];
+  }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+    if constexpr (sizeof(T) == 2) {
+      v[0] = bf16_lo(raw[0].x); v[1] = bf16_hi(raw[0].x);
+      v[2] = bf16_lo(raw[0].y); v[3] = bf16_hi(raw[0].y);
+      v[4] = bf16_lo(raw[0].z); v[5] = bf16_hi(raw[0].z);
+      v[6] = bf16_lo(raw[0].w); v[7] = bf16_hi(raw[0].w);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        v[4 * i] = __uint_as_float(raw[i].x); v[4 * i + 1] = __uint_as_float(raw[i].y);
+        v[4 * i + 2] = __uint_as_float(raw[i].z); v[4 * i + 3] = __uint_as_float(raw[i].w);
+      }
+    }
+  }
+};
+
+// K: the number of slots, 0 for any other. FEW: N * pieces < 2^31.
+template <typename T, int K, bool FEW>
 __global__ void __launch_bounds__(256)
 combine_kernel(const T* __restrict__ y, const int32_t* __restrict__ row_of,
                const float* __restrict__ w, const T* __restrict__ residual, int64_t N, int d,
                int k, T* __restrict__ out, const EpSync sy, int32_t* __restrict__ status) {
   const int pieces = d >> 3;
   const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = FEW ? (int64_t)((unsigned)item / (unsigned)pieces) : item / pieces;
+  const int c = (int)(item - t * pieces) << 3;
   pdl_wait();
   // expert-parallel: y is the return buffer the expert owners store into; wait for all of them
   if (!epsync::block_wait(sy, status, 25)) return;
   if (item >= N * pieces) return;
-  const int64_t t = item / pieces;
-  const int c = (int)(item - t * pieces) << 3;
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-  for (int j = 0; j < k; ++j) {
-    // row_of == nullptr: y is already in (token, slot) order (expert-parallel return buffer)
-    const int row = row_of != nullptr ? __ldg(&row_of[t * k + j]) : (int)(t * k + j);
-    if (row < 0) continue;
-    const float wj = __ldg(&w[t * k + j]);
-    float v[8];
-    load8(y + (int64_t)row * d + c, v);
-    // mul then add, not fma: the reference forms w0*a + w1*b from rounded products
+  Eight<T> res;
+  if (residual != nullptr) res.load(residual + t * d + c);
+  // row_of == nullptr: y is already in (token, slot) order (expert-parallel return buffer)
+  // mul then add, not fma: the reference forms w0*a + w1*b from rounded products
+  if constexpr (K > 0) {
+    int row[K];
+    float wj[K];
+    Eight<T> yj[K];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(wj, v[i]));
+    for (int j = 0; j < K; ++j) {
+      row[j] = row_of != nullptr ? __ldg(&row_of[t * K + j]) : (int)(t * K + j);
+      wj[j] = __ldg(&w[t * K + j]);
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+      if (row[j] >= 0) yj[j].load(y + (int64_t)row[j] * d + c);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      if (row[j] < 0) continue;
+      float v[8];
+      yj[j].get(v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(wj[j], v[i]));
+    }
+  } else {
+    for (int j = 0; j < k; ++j) {
+      const int row = row_of != nullptr ? __ldg(&row_of[t * k + j]) : (int)(t * k + j);
+      if (row < 0) continue;
+      const float wj = __ldg(&w[t * k + j]);
+      float v[8];
+      load8(y + (int64_t)row * d + c, v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(wj, v[i]));
+    }
   }
   if (residual != nullptr) {
     float r[8];
-    load8(residual + t * d + c, r);
+    res.get(r);
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = __fadd_rn(acc[i], r[i]);
   }
   store8(out + t * d + c, acc);
 }
 
+template <typename T>
+auto combine_kernel_of(int k, bool few) {
+  if (!few) return combine_kernel<T, 0, false>;
+  return k == 1 ? combine_kernel<T, 1, true> : k == 2 ? combine_kernel<T, 2, true>
+         : k == 4 ? combine_kernel<T, 4, true> : combine_kernel<T, 0, true>;
+}
 
 // Small-N variant: the down product arrives as `ksplit` fp32 partial buffers
 // part[s][M][d] without bias; sum them in order s = 0..ksplit-1, add the
@@ -240,13 +296,14 @@ int launch_combine(const void* y, const int32_t* row_of, const float* w, const v
   const EpSync& sy = ep_wait != nullptr ? *ep_wait : nosync;
   const int64_t items = N * (d >> 3);
   const int64_t blocks = (items + 255) / 256;
+  const bool few = blocks * 256 < (int64_t)1 << 31;
   if (dtype == MOE_B200_BF16) {
-    MOE_CUDA_CHECK(launch_pdl(combine_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(256), 0, s,
+    MOE_CUDA_CHECK(launch_pdl(combine_kernel_of<__nv_bfloat16>(k, few), dim3((unsigned)blocks), dim3(256), 0, s,
                               static_cast<const __nv_bfloat16*>(y), row_of, w,
                               static_cast<const __nv_bfloat16*>(residual), N, d, k,
                               static_cast<__nv_bfloat16*>(out), sy, status));
   } else {
-    MOE_CUDA_CHECK(launch_pdl(combine_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, s,
+    MOE_CUDA_CHECK(launch_pdl(combine_kernel_of<float>(k, few), dim3((unsigned)blocks), dim3(256), 0, s,
                               static_cast<const float*>(y), row_of, w,
                               static_cast<const float*>(residual), N, d, k, static_cast<float*>(out),
                               sy, status));
