@@ -507,7 +507,13 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
     if (rc) return rc;
     front32 = front32 && front;
   }
-  const bool counters = small_n || rows_path || mid;
+  // beyond, router and dispatch in one launch up to some thousand tokens
+  int many = 0;
+  if (!front && !tiny && !norm && aligned16(Wg)) {
+    rc = front_many_tokens(N, d, E, k, dtype, &many);
+    if (rc) return rc;
+  }
+  const bool counters = small_n || rows_path || mid || many > 0;
   const bool clean = (small_n || rows_path) && (flags & MOE_B200_FLAG_WS_CLEAN);
   // status words, and the completion counters behind them where a kernel uses them, in one memset
   // (above these sizes a call always clears the status words: they are those of the most recent call; the fp32 front
@@ -547,6 +553,10 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
         return launch_combine_parts_f32(part, parts, N * k, row_of, idx, w, plan, E, residual, N, d, k, out, s);
       return moe_b200_combine(y, row_of, w, residual, N, d, k, dtype, out, stream);
     }
+  } else if (many > 0) {
+    rc = launch_front_many(x, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm, nullptr, psum, aux, scratch,
+                           status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many, s);
+    if (rc) return rc;
   } else {
     if (fold) {
       void* wn = ws + off[MOE_B200_WS_NORM_W];

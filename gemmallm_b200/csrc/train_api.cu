@@ -267,16 +267,29 @@ int forward_train_into(const void* x, const void* Wg, const void* bg, const void
   const int64_t M = N * k;
   MOE_CUDA_CHECK(cudaMemsetAsync(status, 0, (MOE_B200_READY_OFFSET + MOE_B200_READY_INTS) * sizeof(int32_t), s));
   // training always takes the large-N kernels: the backward pass works on their sorted buffers
-  rc = moe_b200_router(x, Wg, bg, N, d, E, k, dtype, logits, idx, w, psum_part, status, stream);
-  if (rc) return rc;
-  rc = moe_b200_dispatch(x, idx, N, d, E, k, dtype, reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_SCRATCH]),
-                         reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_CNT_SLOT]), offsets, row_of, perm,
-                         psum_part, reinterpret_cast<float*>(ws + off[MOE_B200_WS_PSUM]),
-                         aux != nullptr ? aux : reinterpret_cast<float*>(ws + off[MOE_B200_WS_AUX]), status,
-                         stream);
-  if (rc) return rc;
-  rc = launch_pair_of(row_of, M, reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]), s);
-  if (rc) return rc;
+  int32_t* scratch = reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_SCRATCH]);
+  int32_t* cnt_slot = reinterpret_cast<int32_t*>(ws + off[MOE_B200_WS_CNT_SLOT]);
+  float* psum = reinterpret_cast<float*>(ws + off[MOE_B200_WS_PSUM]);
+  int32_t* pair_of = reinterpret_cast<int32_t*>(tws + to[MOE_B200_TWS_PAIR_OF]);
+  if (aux == nullptr) aux = reinterpret_cast<float*>(ws + off[MOE_B200_WS_AUX]);
+  int many = 0;
+  if (aligned16(x) && aligned16(Wg)) {
+    rc = front_many_tokens(N, d, E, k, dtype, &many);
+    if (rc) return rc;
+  }
+  if (many > 0) {
+    rc = launch_front_many(x, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm, pair_of, psum, aux, scratch,
+                           status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many, s);
+    if (rc) return rc;
+  } else {
+    rc = moe_b200_router(x, Wg, bg, N, d, E, k, dtype, logits, idx, w, psum_part, status, stream);
+    if (rc) return rc;
+    rc = moe_b200_dispatch(x, idx, N, d, E, k, dtype, scratch, cnt_slot, offsets, row_of, perm, psum_part, psum, aux, status,
+                           stream);
+    if (rc) return rc;
+    rc = launch_pair_of(row_of, M, pair_of, s);
+    if (rc) return rc;
+  }
   const TrainArgs tr = train_args(tws, to, dropout_p, seed, lora);
   rc = launch_experts_tc2(perm, offsets, plan, M, d, f, E, h, y, nullptr, status, s, &tr);
   if (rc) return rc;

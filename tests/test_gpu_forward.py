@@ -174,6 +174,43 @@ def test_fp32_tokens_of_nan(cuda_device, N, fold):
             assert m(bad, norm=norm)[0][0, rows].eq(0).all() and m.device_status() == 2
 
 
+# past the rows of the small calls: blocks of one group of 16 tokens and of one token more, a last block of one token, the most
+# tokens and one more, rows of one piece and of several rounds, one expert and 64, one slot and eight
+@pytest.mark.parametrize("N,d,E,k", [(2049, 8, 1, 1), (2500, 1032, 8, 2), (2369, 2056, 16, 8), (18944, 64, 9, 2), (18945, 64, 9, 2),
+                                     (4737, 520, 3, 3), (1025, 2056, 64, 4), (3001, 64, 40, 2), (6000, 72, 32, 1), (2200, 40, 17, 2)])
+def test_routing_of_thousands_of_tokens(cuda_device, N, d, E, k):
+    """As the general router and dispatch give it, also where tokens or logits are not finite (up to 16 experts)."""
+    x = torch.randn(N, d, generator=torch.Generator().manual_seed(E + N)).bfloat16().to(cuda_device)
+    params = synthetic.make_params(d, E, 8, seed=N)
+    m = build(params, d, E, 8, k, torch.bfloat16, cuda_device)
+    gate = (m.gate.weight.detach(), m.gate.bias.detach())
+    mag = x.float().abs() @ gate[0].float().abs().T + gate[1].float().abs()
+    nan, inf = float("nan"), float("inf")
+    for values in [(), (nan,), (-inf,), (inf, -inf), (nan,) * E, (-inf,) * (E - 1)][:6 if E <= 16 else 1]:
+        if len(values) <= E:
+            m.gate.bias.data.copy_(params["gate_b"])
+            m.gate.bias.data[:len(values)] = torch.tensor(values, dtype=torch.bfloat16)
+        with torch.no_grad():
+            m(x.view(1, N, d))
+        last = {n: t.clone() for n, t in m.last.items()}
+        status = m.device_status()
+        logits, idx, w, psum_part = helpers.router(x, *gate, k)
+        # fp32 sums of d products in another order: d 2^-24 of their sum of magnitudes, at the worst
+        diff = (last["logits"] - logits).abs()
+        assert bool(((diff <= 2 * d * 2.0 ** -24 * mag) | ~logits.isfinite()).all()), values
+        same = (last["idx"] == idx).all(1).cpu()
+        if not values:
+            r = moe_oracle.route_from_logits(last["logits"].cpu(), k)
+            assert bool(same[~moe_oracle.tie_rows(r["probs"], k)].all())
+        assert int((~same).sum()) <= N // 500, values      # near-ties
+        assert torch.allclose(last["w"].cpu()[same], w.cpu()[same], atol=4e-6, rtol=0, equal_nan=True), values
+        disp = helpers.dispatch(x, last["idx"], E, psum_part)
+        for name in ("offsets", "row_of", "cnt_slot"):
+            assert torch.equal(last[name], disp[name]), (values, name)
+        assert torch.allclose(last["psum"], disp["psum"], rtol=1e-5, atol=1e-6, equal_nan=True), values
+        assert status == int(disp["status"][0]), values
+
+
 # a whole bf16 call of 33 to 64 experts: one token, a block of one and of all 16, streaming and sorted-row sizes, one slot and eight
 @pytest.mark.parametrize("N,d,E,k", [(1, 64, 33, 1), (16, 2056, 64, 4), (33, 72, 63, 8), (130, 1024, 40, 2), (511, 520, 64, 8),
                                      (2048, 64, 64, 2)])
