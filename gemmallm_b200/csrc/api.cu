@@ -509,16 +509,17 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   }
   // beyond, router and dispatch in one launch up to some thousand tokens
   int many = 0;
-  if (!front && !tiny && !norm && aligned16(Wg)) {
-    rc = front_many_tokens(N, d, E, k, dtype, &many);
+  if (!front && !tiny && aligned16(Wg)) {
+    rc = front_many_tokens(N, d, E, k, dtype, norm, &many);
     if (rc) return rc;
   }
   const bool counters = small_n || rows_path || mid || many > 0;
   const bool clean = (small_n || rows_path) && (flags & MOE_B200_FLAG_WS_CLEAN);
   // status words, and the completion counters behind them where a kernel uses them, in one memset
-  // (above these sizes a call always clears the status words: they are those of the most recent call; the fp32 front
-  // clears them itself)
-  if (!front32 && !clean)
+  // (above these sizes a call always clears the status words: they are those of the most recent call; the fp32 front and,
+  // where the counters are known to be zero, the one of a few thousand tokens clear them themselves)
+  const bool clears = many > 0 && (flags & MOE_B200_FLAG_WS_CLEAN);
+  if (!front32 && !clean && !clears)
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
   float* stats = reinterpret_cast<float*>(ws + off[MOE_B200_WS_STATS]);
@@ -553,16 +554,22 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
         return launch_combine_parts_f32(part, parts, N * k, row_of, idx, w, plan, E, residual, N, d, k, out, s);
       return moe_b200_combine(y, row_of, w, residual, N, d, k, dtype, out, stream);
     }
-  } else if (many > 0) {
-    rc = launch_front_many(x, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm, nullptr, psum, aux, scratch,
-                           status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many, s);
-    if (rc) return rc;
   } else {
+    void* wn = ws + off[MOE_B200_WS_NORM_W];
+    float* nc = reinterpret_cast<float*>(ws + off[MOE_B200_WS_NORM_C]);
     if (fold) {
-      void* wn = ws + off[MOE_B200_WS_NORM_W];
-      float* nc = reinterpret_cast<float*>(ws + off[MOE_B200_WS_NORM_C]);
       rc = launch_norm_fold(Wg, bg, norm_weight, norm_bias, E, d, dtype, wn, nc, s);
       if (rc) return rc;
+    }
+    if (many > 0) {
+      // (the normalised rows lie where the down product's will: nothing reads them behind this launch)
+      if (fold) rc = launch_layernorm_rows(x, norm_weight, norm_bias, norm_eps, N, d, dtype, y, stats, s);
+      if (rc) return rc;
+      rc = launch_front_many(x, y, stats, fold ? nc : nullptr, fold ? wn : Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets,
+                             row_of, perm, nullptr, psum, aux, scratch,
+                             status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many, clears, s);
+      if (rc) return rc;
+    } else if (fold) {
       rc = moe_b200_router_norm(x, wn, nc, norm_eps, N, d, E, k, dtype, logits, idx, w, psum_part,
                                 stats, status, stream);
       if (rc) return rc;

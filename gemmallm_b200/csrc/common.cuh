@@ -366,10 +366,11 @@ int launch_ep_dispatch(const void* x, const int32_t* idx, int64_t N, int d, int 
 bool front_small_supported(int64_t N, int E, int k, int dtype);
 int64_t front_small_exchange_ints(int64_t N, int E, int k);
 bool front_split_supported(int64_t N, int d, int E, int k, int dtype);
-int front_many_tokens(int64_t N, int d, int E, int k, int dtype, int* per);
-int launch_front_many(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E, int k, float* logits, int32_t* idx,
-                      float* w, int32_t* cnt_slot, int32_t* offsets, int32_t* row_of, void* perm, int32_t* pair_of, float* psum,
-                      float* aux, int32_t* xch, int* counter, int32_t* status, int per, cudaStream_t s);
+int front_many_tokens(int64_t N, int d, int E, int k, int dtype, bool norm, int* per);
+int launch_front_many(const void* x, const void* xn, const float* stats, const float* norm_c, const void* Wg, const void* bg,
+                      int64_t N, int d, int E, int k, float* logits, int32_t* idx, float* w, int32_t* cnt_slot,
+                      int32_t* offsets, int32_t* row_of, void* perm, int32_t* pair_of, float* psum, float* aux, int32_t* xch,
+                      int* counter, int32_t* status, int per, bool clear, cudaStream_t s);
 int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E, int k,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,

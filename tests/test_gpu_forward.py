@@ -652,6 +652,12 @@ def test_layernorm_folded_into_the_block(cuda_device, N, d, E, f, k, dtype):
         assert (got - ref)[ok].norm() <= 2e-2 * ref[ok].norm()
 
 
+# routed in one launch: a block of one group of tokens and of one more, the most tokens, rows of several rounds
+@pytest.mark.parametrize("N,d,E,f,k", [(2305, 264, 16, 64, 8), (2500, 2056, 3, 64, 2), (18944, 72, 8, 64, 1)])
+def test_layernorm_folded_into_thousands_of_tokens(cuda_device, N, d, E, f, k):
+    test_layernorm_folded_into_the_block(cuda_device, N, d, E, f, k, torch.bfloat16)
+
+
 def test_state_survives_dtype_change_and_repeat_calls(cuda_device):
     d, E, f, k, N = 64, 8, 128, 2, 200
     params = synthetic.make_params(d, E, f, seed=9)
