@@ -209,6 +209,8 @@ class Merged {
   template <typename Param>
   int refresh(Param param, const std::vector<double>& scales, int dtype, void* stream) {
     const std::lock_guard<std::mutex> lock(mutex_);      // a backward runs on another thread
+    std::vector<moe::LoraMerge> todo;
+    std::vector<Job*> jobs;
     for (size_t i = 0; i < jobs_.size(); ++i) {
       Job& j = jobs_[i];
       const size_t first = i / 2 * 12, l = i % 2;
@@ -226,17 +228,19 @@ class Merged {
       }
       if (same) continue;
       j.valid = false;
-      const int rc = moe_b200_lora_merge(data[0], data[1], data[2], data[3], data[4], data[5], (float)scales[i / 2],
-                                         j.out_f, j.in_f, j.rank, dtype, j.w.data_ptr(), j.b.data_ptr(), stream);
-      if (rc != 0) return rc;
+      todo.push_back({data[0], data[1], data[2], data[3], data[4], data[5], j.w.data_ptr(), j.b.data_ptr(),
+                      (float)scales[i / 2], j.out_f, j.in_f, j.rank});
+      jobs.push_back(&j);
       std::copy(data, data + 6, j.data);
       std::copy(version, version + 6, j.version);
       j.storage.clear();
       for (const c10::Storage* s : storage) j.storage.push_back(s->getWeakStorageImpl());
       j.scale = scales[i / 2];
-      j.valid = true;
     }
-    return 0;
+    if (todo.empty()) return 0;
+    const int rc = moe::lora_merges(todo.data(), (int)todo.size(), dtype, stream);
+    for (Job* j : jobs) j->valid = rc == 0;
+    return rc;
   }
 
  private:

@@ -34,6 +34,14 @@ struct LoraGrads {
   float* scratch;            // as many floats as the largest run asks for
   std::vector<LoraRun> runs;
 };
+// Linears with their LoRA branches folded in (moe_b200_lora_merge), in as few launches as can be.
+struct LoraMerge {
+  const void *W, *b, *A, *a_bias, *B, *b_lora;
+  void *out_W, *out_b;
+  float scale;
+  int out_f, in_f, rank;
+};
+int lora_merges(const LoraMerge* merges, int n, int dtype, void* stream);
 size_t lora_grads_scratch_floats(int d, int f, const LoraRun& run);
 
 // moe_b200_forward_train with the load-balancing loss written to `aux` (nullptr: the workspace's word). lora: of a LoRA

@@ -11,6 +11,7 @@
 // 8388608 against 42; rank 64 37 against 147; rank 33, A and B five times as large, [2816,2048]: 101 of 5767168 against 513).
 // fp32: the sums on the CUDA cores, a thread owning 8 rows x 8 columns, A and B in shared memory.
 #include "common.cuh"
+#include "internal.h"
 
 namespace moe {
 
@@ -128,20 +129,38 @@ lora_merge_f32_kernel(const float* W, const float* b, const float* A, const floa
 // A warp takes units of 16 rows x 128 columns of its block's 128 columns; the slice of A [rank][128] waits in shared
 // memory with its columns in the order that gives a thread eight neighbouring ones: tile j, place n of a group of 32 columns
 // is column 8 (n / 2) + 2 j + n % 2. The next unit of W is requested when this one's products have been added, before the
-// result is stored.
+// result is stored. A launch takes several Linears, one after the other in its blocks (both of a feed-forward of d 1024, f 4096:
+// 17 us of a fine-tuning step with a launch each, which the second one's blocks could not begin before the first's end).
 constexpr int kMergeCols = 128;
 constexpr int kMergePitch = kMergeCols + 8;      // elements: rows 16 bytes apart modulo the banks
 constexpr int kMergeWarps = 8;
+constexpr int kMergeJobs = 32;      // of a launch: 3 KB of arguments
 
-__global__ void __launch_bounds__(32 * kMergeWarps, 2)
-lora_merge_tc_kernel(const __nv_bfloat16* W, const __nv_bfloat16* b, const __nv_bfloat16* A, const __nv_bfloat16* a_bias,
-                     const __nv_bfloat16* B, const __nv_bfloat16* b_lora, float scale, int out_f, int in_f, int rank,
-                     __nv_bfloat16* out_W, __nv_bfloat16* out_b) {
+struct MergeJob {
+  const __nv_bfloat16 *W, *b, *A, *a_bias, *B, *b_lora;
+  __nv_bfloat16 *out_W, *out_b;
+  float scale;
+  int out_f, in_f, rank;
+  int end, strips, sharing;      // blocks of the launch up to this Linear's last; strips of columns; blocks that share one
+};
+struct MergeJobs {
+  MergeJob job[kMergeJobs];
+};
+
+__global__ void __launch_bounds__(32 * kMergeWarps, 2) lora_merge_tc_kernel(const __grid_constant__ MergeJobs jobs) {
+  int which = 0, before = 0;
+  for (; (int)blockIdx.x >= jobs.job[which].end; ++which) before = jobs.job[which].end;
+  const MergeJob& job = jobs.job[which];
+  const __nv_bfloat16 *W = job.W, *b = job.b, *A = job.A, *a_bias = job.a_bias, *B = job.B, *b_lora = job.b_lora;
+  __nv_bfloat16 *out_W = job.out_W, *out_b = job.out_b;
+  const float scale = job.scale;
+  const int out_f = job.out_f, in_f = job.in_f, rank = job.rank;
+  const int share = ((int)blockIdx.x - before) / job.strips, strip = (int)blockIdx.x - before - share * job.strips;
   __shared__ __align__(16) __nv_bfloat16 s_a[kMaxRank][kMergePitch];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int c0 = blockIdx.x * kMergeCols;
+  const int c0 = strip * kMergeCols;
   const int ksteps = (rank + 15) >> 4;
-  const int units = (out_f + 15) >> 4, stride = gridDim.y * kMergeWarps;
+  const int units = (out_f + 15) >> 4, stride = job.sharing * kMergeWarps;
   pdl_wait();
   uint4 w[2][4];      // rows g and g + 8; columns 32 q + 8 t
   auto request = [&](int u) {
@@ -156,7 +175,7 @@ lora_merge_tc_kernel(const __nv_bfloat16* W, const __nv_bfloat16* b, const __nv_
       }
     }
   };
-  int u = blockIdx.y * kMergeWarps + warp;
+  int u = share * kMergeWarps + warp;
   if (u < units) request(u);
   for (int i = tid; i < ksteps * 16 * (kMergeCols / 8); i += 32 * kMergeWarps) {
     const int r = i / (kMergeCols / 8), p = i - r * (kMergeCols / 8);      // eight columns of a rank
@@ -227,7 +246,7 @@ lora_merge_tc_kernel(const __nv_bfloat16* W, const __nv_bfloat16* b, const __nv_
         if (row < out_f && c < in_f) *reinterpret_cast<uint4*>(out_W + (size_t)row * in_f + c) = o[h][q];
       }
     }
-    if (blockIdx.x == 0 && lane < 16 && row0 + lane < out_f) {
+    if (strip == 0 && lane < 16 && row0 + lane < out_f) {
       const int row = row0 + lane;
       float sum = 0.f;
       for (int r = 0; r < rank; ++r) sum = fmaf(scale * to_f32(B[(size_t)row * rank + r]), to_f32(a_bias[r]), sum);
@@ -236,15 +255,22 @@ lora_merge_tc_kernel(const __nv_bfloat16* W, const __nv_bfloat16* b, const __nv_
   }
 }
 
-int launch_merge_bf16(const void* W, const void* b, const void* A, const void* a_bias, const void* B, const void* b_lora,
-                      float scale, int out_f, int in_f, int rank, void* out_W, void* out_b, cudaStream_t s) {
+int launch_merges_bf16(const LoraMerge* merges, int n, cudaStream_t s) {
   typedef const __nv_bfloat16* In;
-  const unsigned strips = (unsigned)((in_f + kMergeCols - 1) / kMergeCols);
-  const unsigned blocks = (unsigned)(((out_f + 15) / 16 + kMergeWarps - 1) / kMergeWarps), most = (2 * kNumSMs + strips - 1) / strips;
-  MOE_CUDA_CHECK(launch_pdl(lora_merge_tc_kernel, dim3(strips, blocks < most ? blocks : most), dim3(32 * kMergeWarps), 0, s,
-                            static_cast<In>(W), static_cast<In>(b), static_cast<In>(A), static_cast<In>(a_bias),
-                            static_cast<In>(B), static_cast<In>(b_lora), scale, out_f, in_f, rank,
-                            static_cast<__nv_bfloat16*>(out_W), static_cast<__nv_bfloat16*>(out_b)));
+  typedef __nv_bfloat16* Out;
+  MergeJobs jobs;
+  unsigned grid = 0;
+  for (int i = 0; i < n; ++i) {
+    const LoraMerge& m = merges[i];
+    const unsigned strips = (unsigned)((m.in_f + kMergeCols - 1) / kMergeCols);
+    const unsigned blocks = (unsigned)(((m.out_f + 15) / 16 + kMergeWarps - 1) / kMergeWarps);
+    const unsigned most = (2 * kNumSMs + strips - 1) / strips, sharing = blocks < most ? blocks : most;
+    grid += strips * sharing;
+    jobs.job[i] = {static_cast<In>(m.W), static_cast<In>(m.b), static_cast<In>(m.A), static_cast<In>(m.a_bias),
+                   static_cast<In>(m.B), static_cast<In>(m.b_lora), static_cast<Out>(m.out_W), static_cast<Out>(m.out_b),
+                   m.scale, m.out_f, m.in_f, m.rank, (int)grid, (int)strips, (int)sharing};
+  }
+  MOE_CUDA_CHECK(launch_pdl(lora_merge_tc_kernel, dim3(grid), dim3(32 * kMergeWarps), 0, s, jobs));
   return 0;
 }
 
@@ -267,22 +293,42 @@ int launch_merge_f32(const void* W, const void* b, const void* A, const void* a_
 }  // namespace
 }  // namespace moe
 
+namespace moe {
+
+int lora_merges(const LoraMerge* merges, int n, int dtype, void* stream) {
+  if (dtype != MOE_B200_F32 && dtype != MOE_B200_BF16)
+    return set_error(MOE_B200_ERR_DTYPE, "dtype must be MOE_B200_F32 or MOE_B200_BF16");
+  for (int i = 0; i < n; ++i) {
+    const LoraMerge& m = merges[i];
+    if (m.out_f < 1 || m.in_f < 8 || (m.in_f & 7) || m.rank < 1 || m.rank > kMaxRank)
+      return set_error(MOE_B200_ERR_SHAPE, "in_features must be a multiple of 8 and rank in [1,64]");
+    if (!m.W || !m.b || !m.A || !m.a_bias || !m.B || !m.b_lora || !m.out_W || !m.out_b)
+      return set_error(MOE_B200_ERR_NULL, "NULL argument");
+    if (!aligned16(m.W) || !aligned16(m.A) || !aligned16(m.out_W))
+      return set_error(MOE_B200_ERR_ALIGN, "W, A and out_W must be 16-byte aligned");
+  }
+  cudaStream_t s = (cudaStream_t)stream;
+  int rc = 0;
+  if (dtype == MOE_B200_BF16) {
+    for (int i = 0; i < n && rc == 0; i += kMergeJobs)
+      rc = launch_merges_bf16(merges + i, n - i < kMergeJobs ? n - i : kMergeJobs, s);
+  } else {
+    for (int i = 0; i < n && rc == 0; ++i) {
+      const LoraMerge& m = merges[i];
+      rc = launch_merge_f32(m.W, m.b, m.A, m.a_bias, m.B, m.b_lora, m.scale, m.out_f, m.in_f, m.rank, m.out_W, m.out_b, s);
+    }
+  }
+  return rc;
+}
+
+}  // namespace moe
+
 using namespace moe;
 
 extern "C" int moe_b200_lora_merge(const void* W, const void* b, const void* A, const void* a_bias,
                                    const void* B, const void* b_lora, float scale, int out_features,
                                    int in_features, int rank, int dtype, void* out_W, void* out_b,
                                    void* stream) {
-  if (dtype != MOE_B200_F32 && dtype != MOE_B200_BF16)
-    return set_error(MOE_B200_ERR_DTYPE, "dtype must be MOE_B200_F32 or MOE_B200_BF16");
-  if (out_features < 1 || in_features < 8 || (in_features & 7) || rank < 1 || rank > kMaxRank)
-    return set_error(MOE_B200_ERR_SHAPE, "in_features must be a multiple of 8 and rank in [1,64]");
-  if (!W || !b || !A || !a_bias || !B || !b_lora || !out_W || !out_b)
-    return set_error(MOE_B200_ERR_NULL, "NULL argument");
-  if (!aligned16(W) || !aligned16(A) || !aligned16(out_W))
-    return set_error(MOE_B200_ERR_ALIGN, "W, A and out_W must be 16-byte aligned");
-  cudaStream_t s = (cudaStream_t)stream;
-  if (dtype == MOE_B200_BF16)
-    return launch_merge_bf16(W, b, A, a_bias, B, b_lora, scale, out_features, in_features, rank, out_W, out_b, s);
-  return launch_merge_f32(W, b, A, a_bias, B, b_lora, scale, out_features, in_features, rank, out_W, out_b, s);
+  const LoraMerge m = {W, b, A, a_bias, B, b_lora, out_W, out_b, scale, out_features, in_features, rank};
+  return lora_merges(&m, 1, dtype, stream);
 }

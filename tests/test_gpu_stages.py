@@ -319,6 +319,32 @@ def test_lora_merge_by_units(cuda_device, out_f, in_f, rank):
     test_lora_merge(cuda_device, out_f, in_f, rank, torch.bfloat16)
 
 
+@pytest.mark.parametrize("E", [1, 16, 17])      # 2, 32 and 34 Linears: one launch takes 32
+def test_lora_merges_of_many_experts(cuda_device, E):
+    """The merged weights of all experts are those of a call for each Linear, also when one adapter changed since."""
+    from gemmallm_b200 import FeedForward
+    from gemmallm_b200.moe import _MergedLora
+    with torch.device(cuda_device):
+        experts = [FeedForward(72, lora_rank=5, d_ff=264).bfloat16().requires_grad_(False) for _ in range(E)]
+    for ex in experts:
+        for p in ex.parameters():
+            p.normal_(0.0, 0.1)
+    lora = _MergedLora()
+    for change in (False, True):
+        if change:
+            experts[-1].lora_down_b.weight.mul_(2.0)
+        merged = lora.get(experts, _cabi.BF16, experts[0].gate_and_up.weight.device)
+        for ex, mg in zip(experts, merged):
+            for lin, a, b, out in ((ex.gate_and_up, ex.lora_gate_and_up_a, ex.lora_gate_and_up_b, mg.gate_and_up),
+                                   (ex.down, ex.lora_down_a, ex.lora_down_b, mg.down)):
+                W, bias = torch.empty_like(lin.weight), torch.empty_like(lin.bias)
+                check(lib.moe_b200_lora_merge(
+                    *[t.data_ptr() for m in (lin, a, b) for t in (m.weight, m.bias)], float(ex.lora_scale), lin.out_features,
+                    lin.in_features, a.out_features, _cabi.BF16, W.data_ptr(), bias.data_ptr(), helpers.stream(cuda_device)),
+                    "lora_merge")
+                assert torch.equal(out.weight, W) and torch.equal(out.bias, bias)
+
+
 # blocks of 16 rows and 16 or 32 tokens that end early, K that ends within a chunk of 32, a round of chunks more, one Linear
 # and two; from 129 tokens on tiles of 256 x 2 times 128, the second Linear in either half, K whole and in two and four ranges
 @pytest.mark.parametrize("N,K,r,r2", [(1, 8, 1, 0), (15, 40, 17, 2), (16, 1024, 1152, 16), (17, 1032, 72, 5), (33, 264, 2400, 1),
