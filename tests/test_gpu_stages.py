@@ -905,11 +905,12 @@ def test_layernorm_stage_entry_points(cuda_device, N, d, E, k, dtype):
         assert (perm.float().cpu()[ro[:, j]] - xn).abs().max() <= rtol * scale
 
 
-# query heads of one KV head over several blocks (few sequences) and in one block; contexts at the edges of the
+# rounds of two, four and eight tiles, blocks whose share ends within a sequence and of one round; contexts at the edges of the
 # 16-token tiles; a position table at an address that is no multiple of 16; masks with -inf, with none
 @pytest.mark.parametrize("B,S,H,KV,masked,shift", [(1, 37, 16, 1, True, 0), (1, 1, 16, 1, True, 0), (3, 16, 6, 2, False, 1),
                                                    (2, 17, 4, 4, True, 0), (400, 48, 3, 1, True, 0),
-                                                   (300, 15, 2, 1, False, 3), (1, 128, 5, 1, True, 0)])
+                                                   (300, 15, 2, 1, False, 3), (1, 128, 5, 1, True, 0),
+                                                   (97, 64, 16, 1, True, 0), (131, 50, 6, 3, False, 0), (37, 80, 9, 3, True, 1)])
 def test_attention_core(cuda_device, B, S, H, KV, masked, shift):
     hd, g = 64, torch.Generator().manual_seed(B + S)
     qkv = synthetic.round_to(torch.randn(B, S, H + 2 * KV, hd, generator=g), torch.bfloat16)
