@@ -95,7 +95,8 @@ enum {
   MOE_B200_WS_CNT_SLOT,   /* int32 [k,E]   per-slot expert counts (model.py:237-245) */
   MOE_B200_WS_OFFSETS,    /* int32 [E+1]   start row of each expert in the sorted buffers */
   MOE_B200_WS_ROW_OF,     /* int32 [N,k]   sorted-buffer row of (token, slot) */
-  MOE_B200_WS_PERM,       /* T [N*k, d]    tokens sorted by expert (model.py:248-253) */
+  MOE_B200_WS_PERM,       /* T [N*k, d]    tokens sorted by expert (model.py:248-253); not written by bf16 calls of up to 128
+                           * tokens with at least E pairs, which read the tokens where they lie */
   MOE_B200_WS_H,          /* T [N*k, f]    gelu_tanh(gate)*up (model.py:180-182); fp32 calls of up to 2048 tokens and
                            * 4096 rows: scratch of h and the sorted rows as bf16 parts */
   MOE_B200_WS_Y,          /* T [N*k, d]    expert outputs, sorted order (model.py:184) */
@@ -259,7 +260,7 @@ int moe_b200_front_small(const void* x, const void* Wg, const void* bg,
                          float* psum, float* aux, void* stream);
 
 /* The same results from blocks that share the work: beyond 128 tokens every block of
- * moe_b200_front_small would repeat the whole routing; here block b routes tokens 16b..16b+15,
+ * moe_b200_front_small would repeat the whole routing; here a block routes 8 or 16 tokens,
  * the blocks exchange their counts through `exchange` (int32, at least
  * moe_b200_front_exchange_ints(N,E,k) words) and meet at `counter` (one int32, zeroed by this
  * call; bounded wait, MOE_B200_DEV_TIMEOUT in `status` if a block never arrives). bf16,
