@@ -222,7 +222,8 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
           }
         }
       }
-      left = atomicAdd(counter, 1);      // looked at in the end
+      // looked at in the end; not counted where the wait gave up, so that nobody takes it for another block's arrival
+      if (!dead) left = atomicAdd(counter, 1);
     }
     dead = __syncthreads_or(dead);
     // totals, and the rows that earlier blocks put in front of this block's (16 bits: fewer than 65536 tokens)

@@ -216,6 +216,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   __syncthreads();
   int left = 0;
   if (nb > 1) {
+    bool dead = false;      // gave up: goes on as if nobody had any tokens, so that no row lies outside
     if (tid == 0) {
       __threadfence();
       atomicAdd(counter, 1);
@@ -229,19 +230,21 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
             atomicMax(&status[0], MOE_B200_DEV_TIMEOUT);
             status[1] = 41;
             status[2] = b;
+            dead = true;
             break;
           }
         }
       }
-      left = atomicAdd(counter, 1);      // looked at in the end
+      // looked at in the end; not counted where the wait gave up, so that nobody takes it for another block's arrival
+      if (!dead) left = atomicAdd(counter, 1);
     }
-    __syncthreads();
+    dead = __syncthreads_or(dead);
     // totals, and the rows that earlier blocks put in front of this block's (16 bits: 2048 tokens)
     if (EL == 1) {      // a warp per count
       for (int je = warp; je < ke; je += kMidWarps) {
         unsigned both = 0;
         for (int bb = lane; bb < nb; bb += 32) {
-          const unsigned c = (unsigned)__ldcg(&xch[je * nb + bb]);
+          const unsigned c = dead ? 0u : (unsigned)__ldcg(&xch[je * nb + bb]);
           both += c | (bb < b ? c << 16 : 0u);
         }
         both = __reduce_add_sync(0xffffffffu, both);
@@ -256,7 +259,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
         unsigned both = 0;
 #pragma unroll 8
         for (int bb = q; bb < nb; bb += per) {
-          const unsigned c = (unsigned)__ldcg(&xch[bb * ke + je]);
+          const unsigned c = dead ? 0u : (unsigned)__ldcg(&xch[bb * ke + je]);
           both += c | (bb < b ? c << 16 : 0u);
         }
         if (both & 0xffffu) atomicAdd(&s_tot[je], (int)(both & 0xffffu));
@@ -264,7 +267,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
       }
     }
     if (b == 0)
-      for (int i = tid; i < nb * E; i += 32 * kMidWarps) s_sum[i] = __ldcg(&xps[i]);
+      for (int i = tid; i < nb * E; i += 32 * kMidWarps) s_sum[i] = dead ? 0.f : __ldcg(&xps[i]);
     __syncthreads();
   }
 
@@ -307,7 +310,6 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   if (own < N)
     for (int j = 0; j < k; ++j) {
       const int r = s_row[own * k + j];
-      if ((unsigned)r >= (unsigned)(Ntotal * k)) continue;      // (counts of a block that never arrived)
       uint4* to = reinterpret_cast<uint4*>(perm + (size_t)r * d);
 #pragma unroll
       for (int u = 0; u < kInFlight; ++u)
