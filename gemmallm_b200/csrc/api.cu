@@ -310,7 +310,7 @@ int moe_b200_front_small(const void* x, const void* Wg, const void* bg, int64_t 
 }
 
 int64_t moe_b200_front_exchange_ints(int64_t N, int E, int k) {
-  return (N >= 1 && E >= 1 && k >= 1) ? front_small_exchange_ints(N, E, k) : 0;
+  return (N >= 1 && E >= 1 && k >= 1) ? (N + 15) / 16 * ((int64_t)k * E + E) : 0;      // 16 tokens a block
 }
 
 int moe_b200_front_small_split(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E,
@@ -330,7 +330,7 @@ int moe_b200_front_small_split(const void* x, const void* Wg, const void* bg, in
     return set_error(MOE_B200_ERR_ALIGN, "x, Wg and perm must be 16-byte aligned");
   MOE_CUDA_CHECK(cudaMemsetAsync(counter, 0, sizeof(int32_t), (cudaStream_t)stream));
   return launch_front_small(x, Wg, bg, N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
-                            row_of, perm, psum, aux, (cudaStream_t)stream, exchange, counter, status);
+                            row_of, perm, psum, aux, (cudaStream_t)stream, exchange, counter, status, dtype, nullptr, 16);
 }
 
 int moe_b200_decode_tiny(const void* x, const void* Wg, const void* bg, const void* plan,

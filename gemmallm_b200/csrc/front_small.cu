@@ -353,12 +353,11 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
 template <int NT>
 int launch_mid(const void* x, const void* Wg, const void* bg, int N, int d, int E, int k, float* out_logits, int32_t* out_idx,
                float* out_w, int32_t* cnt_slot, int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux, int* xch,
-               int* counter, int32_t* status, cudaStream_t s) {
+               int* counter, int32_t* status, int per, cudaStream_t s) {
   const size_t smem = sizeof(float) * kMidWarps * kMidTok * 8 * NT;
   static PerDeviceOnce once;
   int rc = ensure_dynamic_smem(once, front_mid_kernel<NT>, smem);
   if (rc) return rc;
-  const int per = mid_tokens_per_block(N);
   MOE_CUDA_CHECK(launch_pdl(front_mid_kernel<NT>, dim3((N + per - 1) / per), dim3(32 * kMidWarps), smem, s,
                             static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(Wg),
                             static_cast<const __nv_bfloat16*>(bg), N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
@@ -400,8 +399,9 @@ bool front_split_supported(int64_t N, int d, int E, int k, int dtype) {
 }
 
 // xch: int32 scratch of at least front_small_exchange_ints(N, E, k) words and counter: one int32
-// that is zero on entry (both only used beyond 128 tokens; without them every block repeats the
-// whole routing at every size).
+// that is zero on entry (both only used beyond 128 tokens or 32 experts; without them every block repeats the
+// whole routing at every size). per: tokens of a block that shares the work, 0 for the best number; with 16 the public
+// entry's smaller exchange buffer does.
 int64_t front_small_exchange_ints(int64_t N, int E, int k) {
   const int64_t nb = N < 512 ? (N + 3) / 4 : 128;      // the most that either type has
   return nb * k * E + nb * E;
@@ -433,7 +433,7 @@ int launch_by_experts(int E, Args... args) {
 int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E, int k,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
-                       cudaStream_t s, int* xch, int* counter, int32_t* status, int dtype, void* planes) {
+                       cudaStream_t s, int* xch, int* counter, int32_t* status, int dtype, void* planes, int per) {
   if (dtype == MOE_B200_F32)
     return launch_by_experts<float>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of,
                                     perm, planes, psum, aux, xch, status, s);
@@ -441,7 +441,7 @@ int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N,
   if (xch != nullptr && counter != nullptr && status != nullptr && (N > 128 || E > kMaxE)) {
     auto mid = E <= 8 ? launch_mid<1> : E <= 16 ? launch_mid<2> : E <= 32 ? launch_mid<4> : launch_mid<8>;
     return mid(x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux, xch, counter,
-               status, s);
+               status, per > 0 ? per : mid_tokens_per_block(N), s);
   }
   return launch_by_experts<__nv_bfloat16>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
                                           row_of, perm, nullptr, psum, aux, xch, status, s);

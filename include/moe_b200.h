@@ -260,7 +260,7 @@ int moe_b200_front_small(const void* x, const void* Wg, const void* bg,
                          float* psum, float* aux, void* stream);
 
 /* The same results from blocks that share the work: beyond 128 tokens every block of
- * moe_b200_front_small would repeat the whole routing; here a block routes 8 or 16 tokens,
+ * moe_b200_front_small would repeat the whole routing; here block b routes tokens 16b..16b+15,
  * the blocks exchange their counts through `exchange` (int32, at least
  * moe_b200_front_exchange_ints(N,E,k) words) and meet at `counter` (one int32, zeroed by this
  * call; bounded wait, MOE_B200_DEV_TIMEOUT in `status` if a block never arrives). bf16,
