@@ -544,6 +544,8 @@ def run_ours(args, wl):
 
     # ---- per-stage times through the stage entry points --------------------
     launches_per_step = 3 if streaming else 5
+    if wl.dtype == "bf16" and not streaming and N <= (18944 if wl.n_experts <= 16 else 9472 if wl.n_experts <= 32 else 3552):
+        launches_per_step = 4                  # router and dispatch in one launch
     if wl.dtype != "bf16" and wl.tokens <= 2048 and wl.tokens * wl.top_k <= 4096 and wl.n_experts <= 32:
         launches_per_step = 4                  # router and dispatch in one launch
     elif small_n and wl.tokens <= 8 and wl.tokens * wl.top_k < wl.n_experts <= 32:
@@ -1260,7 +1262,7 @@ def run_train(args, wl):
         "e2e": {"value": N / (e2e_ms * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": N * d * es,
                 "d2h_bytes_per_step": N * d * es + 4, "ms_per_step": e2e_ms,
                 "mode": "input copied in, input gradient and loss copied out, every step, one stream"},
-        "gpu_launches": 17 * args.steps,   # the library's kernels per step (launch list in profiles/)
+        "gpu_launches": 15 * args.steps,   # the library's kernels per step (launch list in profiles/)
         "clocks": clocks.summary(),
         "roofline": {"kernel": "whole step: six grouped_gemm_tc2_kernel launches (two forward, four backward) "
                                "plus router, dispatch, combine, their backward kernels and column sums",
