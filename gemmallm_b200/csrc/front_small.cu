@@ -358,7 +358,10 @@ int launch_mid(const void* x, const void* Wg, const void* bg, int N, int d, int 
   static PerDeviceOnce once;
   int rc = ensure_dynamic_smem(once, front_mid_kernel<NT>, smem);
   if (rc) return rc;
-  MOE_CUDA_CHECK(launch_pdl(front_mid_kernel<NT>, dim3((N + per - 1) / per), dim3(32 * kMidWarps), smem, s,
+  // beyond 32 experts cooperative, as the dispatch is that such calls had: they run beside those of any other streams (1.6 us a
+  // call; up to 32 experts the meeting has always assumed that the GPU has room for all blocks)
+  const int blocks = (N + per - 1) / per;
+  MOE_CUDA_CHECK(launch_pdl_as(front_mid_kernel<NT>, dim3(blocks), dim3(32 * kMidWarps), 0, NT > 4 && blocks > 1, smem, s,
                             static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(Wg),
                             static_cast<const __nv_bfloat16*>(bg), N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
                             row_of, static_cast<__nv_bfloat16*>(perm), psum, aux, xch, counter, status, per, kMidWarps / per));
