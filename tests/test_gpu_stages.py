@@ -839,6 +839,23 @@ def test_combine_is_exact(cuda_device, N, d, k, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 8])      # one, two and four slots have kernels of their own
+def test_combine_of_slots_without_rows(cuda_device, k, dtype):
+    """A slot whose row is -1 adds nothing; the others are added in order."""
+    N, d, g = 97, 72, torch.Generator().manual_seed(k)
+    y = torch.randn(N * k, d, generator=g).to(dtype)
+    row_of = torch.randperm(N * k, generator=g).view(N, k).to(torch.int32)
+    row_of[torch.rand(N, k, generator=g) < 0.3] = -1
+    w, res = torch.rand(N, k, generator=g), torch.randn(N, d, generator=g).to(dtype)
+    acc = torch.zeros(N, d)
+    for j in range(k):
+        has = row_of[:, j] >= 0
+        acc[has] = acc[has] + w[has, j:j + 1] * y[row_of[has, j].long()].float()
+    out = helpers.combine(y.to(cuda_device), row_of.to(cuda_device), w.to(cuda_device), res.to(cuda_device))
+    assert torch.equal(out.cpu(), (acc + res.float()).to(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("N,d,E,k", [(777, 256, 8, 2), (64, 1024, 64, 4), (4100, 72, 5, 3)])
 def test_layernorm_stage_entry_points(cuda_device, N, d, E, k, dtype):
     """moe_b200_norm_fold + moe_b200_router_norm + moe_b200_dispatch_norm against
