@@ -16,6 +16,7 @@ import math
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from . import _cabi, _host
 from ._cabi import lib, check
@@ -136,8 +137,11 @@ class Attention(nn.Module):
         return _linear_rows(args[13], out, wo, bo)[0] if own else F.linear(out, wo, bo)
 
     def _own_linears(self, args, N, hid, inner):
-        """Whether the Linears go through moe_b200_linear_rows: the same answer as the native call's."""
+        """Whether the Linears go through moe_b200_linear_rows: the same answer as the native call's. Not where derivatives are
+        asked for: torch's Linears give those of the output projection."""
         x, wq, bq, wg, bg, wo, bo = args[:7]
+        if any(_derived(p) for p in args[:7]):
+            return False
         rows, many = (self.q_head + 2 * self.kv_head) * self.head_dim, N > lib.moe_b200_linear_rows_max()
         return (1 <= N <= 1 << 28 and hid % 8 == 0 and self.head_dim == 64 and self.q_head % self.kv_head == 0
                 and x.shape[1] <= 128 and x.data_ptr() % 16 == 0 and not (many and self.q_head % 8 != 0)
@@ -145,6 +149,10 @@ class Attention(nn.Module):
                         and b.is_contiguous() and not (many and b.data_ptr() % 16 != 0)
                         and all(p.dtype == torch.bfloat16 and p.device == x.device for p in (w, b))
                         for w, b, r, c in ((wq, bq, rows, hid), (wg, bg, self.q_head, hid), (wo, bo, hid, inner))))
+
+
+def _derived(p):
+    return p is not None and ((torch.is_grad_enabled() and p.requires_grad) or forward_ad.unpack_dual(p).tangent is not None)
 
 
 def _linear_rows(status, x, w, b, w2=None, b2=None):

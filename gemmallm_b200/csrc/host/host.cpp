@@ -1304,13 +1304,18 @@ PyObject* host_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       Py_RETURN_NONE;
     mask = t(8).const_data_ptr<float>();
   }
-  // the library's own launches throughout, where sizes and places allow (attention.py asks for the same)
+  // the library's own launches throughout, where sizes and places allow (attention.py asks for the same) and nobody asks for
+  // derivatives: torch's Linears give those of the output projection (the core has none, so no other Linear has any)
+  bool derived = x._fw_grad(0).defined();
+  for (int i = 1; i < 7; ++i)
+    derived |= t(i)._fw_grad(0).defined() || (at::GradMode::is_enabled() && t(i).requires_grad());
+  // (has_storage: a batch of weights under vmap has none)
   auto matrix = [](const Tensor& w, int64_t rows, int64_t cols) {
-    return w.dim() == 2 && w.size(0) == rows && w.size(1) == cols && w.is_contiguous();
+    return w.dim() == 2 && w.size(0) == rows && w.size(1) == cols && w.is_contiguous() && w.has_storage();
   };
-  auto vector = [](const Tensor& b, int64_t n) { return b.numel() == n && b.is_contiguous(); };
+  auto vector = [](const Tensor& b, int64_t n) { return b.numel() == n && b.is_contiguous() && b.has_storage(); };
   moe::AttentionArgs p = {};
-  bool own = hidden <= 1 << 24 && inner <= 1 << 24 && B <= 1 << 24 && S <= 128 && matrix(t(1), (heads + 2 * kv) * hd, hidden) &&
+  bool own = !derived && x.has_storage() && hidden <= 1 << 24 && inner <= 1 << 24 && B <= 1 << 24 && S <= 128 && matrix(t(1), (heads + 2 * kv) * hd, hidden) &&
              vector(t(2), (heads + 2 * kv) * hd) && matrix(t(3), heads, hidden) && vector(t(4), heads) &&
              matrix(t(5), hidden, inner) && vector(t(6), hidden);
   if (own) {
@@ -1336,11 +1341,8 @@ PyObject* host_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   }
   if (layer) {
     if (!own) Py_RETURN_NONE;
-    if (at::GradMode::is_enabled()) {
-      if (x.requires_grad() || t(14).requires_grad() || t(15).requires_grad()) Py_RETURN_NONE;
-      for (int i = 1; i < 7; ++i)
-        if (t(i).requires_grad()) Py_RETURN_NONE;
-    }
+    for (int i : {0, 14, 15})
+      if (t(i)._fw_grad(0).defined() || (at::GradMode::is_enabled() && t(i).requires_grad())) Py_RETURN_NONE;
   }
   c10::cuda::CUDAGuard guard(x.device());
   Tensor result;

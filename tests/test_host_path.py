@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from gemmallm_b200 import MOE, Attention, FeedForward, LLMLayer, _host
-from gemmallm_b200._cabi import MoeB200Error
+from gemmallm_b200._cabi import MoeB200Error, check, lib
 from gemmallm_b200.attention import _linear_rows
 from gemmallm_b200.layer import _layernorm
 
@@ -887,6 +887,53 @@ def test_attention_of_a_layer_in_one_call(cuda_device, B, S, hidden, heads, kv, 
         assert _host.attention(odd, *args[1:], *norm) is None
         assert _host.attention(*args, norm[0][:8], *norm[1:]) is None
     assert _host.attention(*args, *norm) is None                            # gradients are wanted
+
+
+def test_own_linears_of_the_attention_give_no_derivatives():
+    """The attention's Linears are torch's where gradients or tangents of one of their tensors are wanted."""
+    import torch.autograd.forward_ad as fw
+    m = Attention(D, 64, 8, 1, Table(16, 64)).to(dtype=DT).eval().requires_grad_(False)
+    x = rows(32, "cpu").view(2, 16, D)
+    own = lambda: m._own_linears(m._arguments(x, None, False), 32, D, 8 * 64)
+    assert own()
+    for p in (m.o.weight, m.o.bias, m.gate.bias):
+        p.requires_grad_(True)
+        assert not own()
+        with torch.no_grad():
+            assert own()
+        p.requires_grad_(False)
+    with fw.dual_level():
+        x = fw.make_dual(x, torch.ones_like(x))
+        assert not own()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("B,S", [(1, 1), (3, 17), (5, 64)])
+def test_gradients_of_the_output_projection(cuda_device, monkeypatch, B, S, native):
+    """With all but the output projection frozen it receives torch's gradients, from the attention and from a layer."""
+    torch.manual_seed(S)
+    layer = LLMLayer(256, 64, 8, 2, Table(128, 64), expansion_factor=1, use_moe=False, device="cuda")
+    layer = layer.to(device=cuda_device, dtype=DT).eval().requires_grad_(False)
+    m = layer.mqa
+    m.embedding.float()
+    m.o.requires_grad_(True)
+    if not native:
+        monkeypatch.setattr(_host, "attention", lambda *a: None)
+    x = torch.randn(B, S, 256, generator=torch.Generator().manual_seed(B)).to(device=cuda_device, dtype=DT)
+    g = torch.randn(B, S, 256, generator=torch.Generator().manual_seed(9)).to(device=cuda_device, dtype=DT)
+    for whole in (False, True):
+        xn = _layernorm(layer.norm1, x) if whole else x
+        with torch.no_grad():
+            qkv, gate = [torch.nn.functional.linear(xn, lin.weight, lin.bias) for lin in (m.qkv, m.gate)]
+            core = torch.empty(B, S, 512, device=cuda_device, dtype=DT)
+            check(lib.moe_b200_attention(qkv.data_ptr(), gate.data_ptr(), m._pos_table(cuda_device).data_ptr(), None, B, S, 8, 2, 64,
+                                         float(m.scaler), core.data_ptr(), torch.cuda.current_stream().cuda_stream), "attention")
+        want = torch.nn.functional.linear(core, m.o.weight, m.o.bias)
+        want = want + x if whole else want
+        wanted = torch.autograd.grad(want, [m.o.weight, m.o.bias], g)
+        got = layer._attend(x, None, False) if whole else m(x)
+        same((got, *torch.autograd.grad(got, [m.o.weight, m.o.bias], g)), (want, *wanted))
 
 
 @pytest.mark.gpu
