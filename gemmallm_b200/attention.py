@@ -138,9 +138,10 @@ class Attention(nn.Module):
 
     def _own_linears(self, args, N, hid, inner):
         """Whether the Linears go through moe_b200_linear_rows: the same answer as the native call's. Not where derivatives are
-        asked for: torch's Linears give those of the output projection."""
+        asked for: torch's Linears give those of the output projection; and not for weights of a class of their own (quantised
+        ones, say), whose data may lie anywhere: they say themselves what a Linear is."""
         x, wq, bq, wg, bg, wo, bo = args[:7]
-        if any(_derived(p) for p in args[:7]):
+        if any(type(p) not in (torch.Tensor, nn.Parameter, type(None)) for p in args[1:7]) or any(_derived(p) for p in args[:7]):
             return False
         rows, many = (self.q_head + 2 * self.kv_head) * self.head_dim, N > lib.moe_b200_linear_rows_max()
         return (1 <= N <= 1 << 28 and hid % 8 == 0 and self.head_dim == 64 and self.q_head % self.kv_head == 0

@@ -907,6 +907,50 @@ def test_own_linears_of_the_attention_give_no_derivatives():
         assert not own()
 
 
+class Scaled(torch.Tensor):
+    """A weight that is half of what it stands for, and keeps it elsewhere."""
+
+    @staticmethod
+    def __new__(cls, half):
+        return torch.Tensor._make_wrapper_subclass(cls, half.shape, dtype=half.dtype, device=half.device)
+
+    def __init__(self, half):
+        self.half_ = half
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        if func is torch.nn.functional.linear:
+            x, w, b = args
+            return torch.nn.functional.linear(x, w.half_ * 2, b)
+        return super().__torch_function__(func, types, args, kwargs or {})
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        raise NotImplementedError(func)
+
+
+def test_own_linears_of_the_attention_leave_other_weights_alone():
+    m = Attention(D, 64, 8, 1, Table(16, 64)).to(dtype=DT).eval().requires_grad_(False)
+    args = m._arguments(rows(32, "cpu").view(2, 16, D), None, False)
+    assert m._own_linears(args, 32, D, 8 * 64)
+    for i in (1, 3, 5):
+        assert not m._own_linears((*args[:i], Scaled(args[i]), *args[i + 1:]), 32, D, 8 * 64)
+
+
+@pytest.mark.gpu
+def test_attention_with_weights_of_a_class_of_their_own(cuda_device):
+    m = Attention(D, 64, 8, 1, Table(16, 64)).to(device=cuda_device, dtype=DT).eval().requires_grad_(False)
+    m.embedding.float()
+    x = rows(32, cuda_device).view(2, 16, D)
+    want = m(x)
+    for lin in (m.qkv, m.gate, m.o):
+        half = lin.weight.detach() / 2
+        del lin.weight
+        lin.weight = Scaled(half)
+    # the library's Linears against torch's: sums in another order, rounded to bf16
+    assert (m(x).float() - want.float()).norm() <= 2.0 ** -7 * want.float().norm()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("native", [True, False])
 @pytest.mark.parametrize("B,S", [(1, 1), (3, 17), (5, 64)])
