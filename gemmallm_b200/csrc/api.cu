@@ -516,10 +516,9 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   const bool counters = small_n || rows_path || mid || many > 0;
   const bool clean = (small_n || rows_path) && (flags & MOE_B200_FLAG_WS_CLEAN);
   // status words, and the completion counters behind them where a kernel uses them, in one memset
-  // (above these sizes a call always clears the status words: they are those of the most recent call; the fp32 front and,
-  // where the counters are known to be zero, the one of a few thousand tokens clear them themselves)
-  const bool clears = many > 0 && (flags & MOE_B200_FLAG_WS_CLEAN);
-  if (!front32 && !clean && !clears)
+  // (above these sizes a call always clears both: the status words are those of the most recent call, and what a call that
+  // timed out left in the counters does not reach the next one; the fp32 front clears the status words itself)
+  if (!front32 && !clean)
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
   float* stats = reinterpret_cast<float*>(ws + off[MOE_B200_WS_STATS]);
@@ -567,7 +566,7 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
       if (rc) return rc;
       rc = launch_front_many(x, y, stats, fold ? nc : nullptr, fold ? wn : Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets,
                              row_of, perm, nullptr, psum, aux, scratch,
-                             status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many, clears, s);
+                             status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many, s);
       if (rc) return rc;
     } else if (fold) {
       rc = moe_b200_router_norm(x, wn, nc, norm_eps, N, d, E, k, dtype, logits, idx, w, psum_part,

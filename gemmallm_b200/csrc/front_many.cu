@@ -29,7 +29,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
                   int32_t* __restrict__ cnt_slot, int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
                   __nv_bfloat16* __restrict__ perm, int32_t* __restrict__ pair_of, float* __restrict__ psum,
                   float* __restrict__ aux, int* __restrict__ xch, int* __restrict__ counter, int32_t* __restrict__ status,
-                  int per, int share, bool clear) {
+                  int per, int share) {
   constexpr int ET = 8 * NT, EL = ET > 32 ? 2 : 1, GL = ET / EL, P = 32 / GL;      // experts a lane, lanes of a token
   constexpr bool STRICT = NT <= 2;
   static_assert(!NORM || STRICT, "with a folded LayerNorm the general router is the strict one at any number of experts");
@@ -55,7 +55,6 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
   if (tid < ET) s_base[tid] = 0;
   pdl_wait();                 // x may come from the kernel before this one
   pdl_launch_dependents();
-  if (clear && b == 0 && tid < MOE_B200_STATUS_INTS) status[tid] = 0;      // (before the exchange: nothing else is reported there)
   __syncthreads();
 
   // ---- routing, 16 tokens at a time: a warp's chunks of 32 of K for all of them, then a token for every warp ----
@@ -364,8 +363,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
 template <int NT, bool NORM>
 int launch(const void* x, const void* xn, const float* stats, const float* norm_c, const void* Wg, const void* bg, int N, int d,
            int E, int k, float* logits, int32_t* idx, float* w, int32_t* cnt_slot, int32_t* offsets, int32_t* row_of, void* perm,
-           int32_t* pair_of, float* psum, float* aux, int32_t* xch, int* counter, int32_t* status, int per, bool clear,
-           cudaStream_t s) {
+           int32_t* pair_of, float* psum, float* aux, int32_t* xch, int* counter, int32_t* status, int per, cudaStream_t s) {
   constexpr size_t part = sizeof(float) * 2 * kWarps * kGroup * 8 * NT;
   static PerDeviceOnce once;
   int rc = ensure_dynamic_smem(once, front_many_kernel<NT, NORM>, part + 2 * sizeof(int) * kMaxPer * kMaxTopK);
@@ -376,7 +374,7 @@ int launch(const void* x, const void* xn, const float* stats, const float* norm_
                                static_cast<const __nv_bfloat16*>(xn), stats, norm_c,
                                static_cast<const __nv_bfloat16*>(Wg), static_cast<const __nv_bfloat16*>(bg), N, d, E, k, logits,
                                idx, w, cnt_slot, offsets, row_of, static_cast<__nv_bfloat16*>(perm), pair_of, psum, aux, xch,
-                               counter, status, per, per < kWarps ? kWarps / per : 1, clear));
+                               counter, status, per, per < kWarps ? kWarps / per : 1));
   return 0;
 }
 
@@ -406,16 +404,15 @@ int front_many_tokens(int64_t N, int d, int E, int k, int dtype, bool norm, int*
 }
 
 // norm_c, or nullptr: a folded LayerNorm, with `stats` and the normalised rows `xn` of layernorm_rows.
-// clear: the status words are zeroed here first (a memset in front of the launch: 2.8 us of every call).
 // xch: int32 scratch, (k + 1) * E words for each of kNumSMs blocks; counter: one int32 that is zero on entry and on exit.
 int launch_front_many(const void* x, const void* xn, const float* stats, const float* norm_c, const void* Wg, const void* bg,
                       int64_t N, int d, int E, int k, float* logits, int32_t* idx, float* w, int32_t* cnt_slot,
                       int32_t* offsets, int32_t* row_of, void* perm, int32_t* pair_of, float* psum, float* aux, int32_t* xch,
-                      int* counter, int32_t* status, int per, bool clear, cudaStream_t s) {
+                      int* counter, int32_t* status, int per, cudaStream_t s) {
   auto fn = norm_c != nullptr ? (E <= 8 ? launch<1, true> : launch<2, true>)
             : E <= 8 ? launch<1, false> : E <= 16 ? launch<2, false> : E <= 32 ? launch<4, false> : launch<8, false>;
   return fn(x, norm_c != nullptr ? xn : x, stats, norm_c, Wg, bg, (int)N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of,
-            perm, pair_of, psum, aux, xch, counter, status, per, clear, s);
+            perm, pair_of, psum, aux, xch, counter, status, per, s);
 }
 
 }  // namespace moe

@@ -956,7 +956,7 @@ PyObject* block_train(PyObject* o, PyObject* const* args, Py_ssize_t nargs) {
     const int rc = moe::forward_train_into(
         x.const_data_ptr(), gate_w.const_data_ptr(), gate_b.const_data_ptr(), c->plan,
         has_res ? res.const_data_ptr() : nullptr, c->N, c->d, c->f, c->E, c->k, MOE_B200_BF16, (float)p, seed, c->ws_base,
-        c->ws_bytes, c->tws_base, c->tws_bytes, out.data_ptr(), aux.data_ptr<float>(), !c->ranks.empty(), true, stream);
+        c->ws_bytes, c->tws_base, c->tws_bytes, out.data_ptr(), aux.data_ptr<float>(), !c->ranks.empty(), stream);
     if (rc != 0) return fail(rc, "forward_train");
   }
   ++*c->gen;

@@ -45,11 +45,11 @@ int lora_merges(const LoraMerge* merges, int n, int dtype, void* stream);
 size_t lora_grads_scratch_floats(int d, int f, const LoraRun& run);
 
 // moe_b200_forward_train with the load-balancing loss written to `aux` (nullptr: the workspace's word). lora: of a LoRA
-// step, whose backward pass is given LoraGrads; it works on other saved values. clean: MOE_B200_FLAG_WS_CLEAN.
+// step, whose backward pass is given LoraGrads; it works on other saved values.
 int forward_train_into(const void* x, const void* Wg, const void* bg, const void* plan, const void* residual,
                        int64_t N, int d, int f, int E, int k, int dtype, float dropout_p, uint64_t seed,
                        void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes, void* out,
-                       float* aux, bool lora, bool clean, void* stream);
+                       float* aux, bool lora, void* stream);
 // moe_b200_experts_train likewise.
 int experts_train_into(const void* x_sorted, const int32_t* offsets, const void* plan, int64_t M, int d, int f, int E,
                        float dropout_p, uint64_t seed, void* train_ws, size_t train_ws_bytes, void* h, void* y, bool lora,

@@ -167,7 +167,7 @@ int moe_b200_forward_train(const void* x, const void* Wg, const void* bg, const 
                            float dropout_p, uint64_t seed, void* workspace, size_t workspace_bytes,
                            void* train_ws, size_t train_ws_bytes, void* out, void* stream) {
   return forward_train_into(x, Wg, bg, plan, residual, N, d, f, E, k, dtype, dropout_p, seed, workspace,
-                            workspace_bytes, train_ws, train_ws_bytes, out, nullptr, false, false, stream);
+                            workspace_bytes, train_ws, train_ws_bytes, out, nullptr, false, stream);
 }
 
 int moe_b200_backward(const void* x, const void* Wg, const void* plan, const void* grad_out,
@@ -236,7 +236,7 @@ int experts_train_into(const void* x_sorted, const int32_t* offsets, const void*
 int forward_train_into(const void* x, const void* Wg, const void* bg, const void* plan, const void* residual,
                        int64_t N, int d, int f, int E, int k, int dtype, float dropout_p, uint64_t seed,
                        void* workspace, size_t workspace_bytes, void* train_ws, size_t train_ws_bytes, void* out,
-                       float* aux, bool lora, bool clean, void* stream) {
+                       float* aux, bool lora, void* stream) {
   int rc = train_check(N, d, f, E, k, dtype, dropout_p);
   if (rc) return rc;
   if (!workspace || !train_ws) return set_error(MOE_B200_ERR_NULL, "workspace is NULL");
@@ -276,12 +276,11 @@ int forward_train_into(const void* x, const void* Wg, const void* bg, const void
     rc = front_many_tokens(N, d, E, k, dtype, false, &many);
     if (rc) return rc;
   }
-  const bool clears = many > 0 && clean;
-  if (!clears)
-    MOE_CUDA_CHECK(cudaMemsetAsync(status, 0, (MOE_B200_READY_OFFSET + MOE_B200_READY_INTS) * sizeof(int32_t), s));
+  MOE_CUDA_CHECK(cudaMemsetAsync(status, 0, (MOE_B200_READY_OFFSET + MOE_B200_READY_INTS) * sizeof(int32_t), s));
   if (many > 0) {
-    rc = launch_front_many(x, nullptr, nullptr, nullptr, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm, pair_of, psum, aux, scratch,
-                           status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many, clears, s);
+    rc = launch_front_many(x, nullptr, nullptr, nullptr, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm,
+                           pair_of, psum, aux, scratch, status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many,
+                           s);
     if (rc) return rc;
   } else {
     rc = moe_b200_router(x, Wg, bg, N, d, E, k, dtype, logits, idx, w, psum_part, status, stream);

@@ -69,8 +69,8 @@ enum {
    * zeroed once, and every call on this workspace since then has ended with
    * device status 0 (such calls leave the region zero). Saves the memset in
    * front of the first kernel of bf16 calls of up to 4096 rows, which then overlaps
-   * the tail of the kernel before it, and of larger ones whose router and dispatch are one
-   * launch; these, all larger calls and fp32 calls clear the status words anyway. After a non-zero device status the region has to be zeroed again by
+   * the tail of the kernel before it; larger calls and fp32 calls clear the status words
+   * anyway. After a non-zero device status the region has to be zeroed again by
    * the caller. */
   MOE_B200_FLAG_WS_CLEAN = 1
 };

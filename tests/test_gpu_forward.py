@@ -211,6 +211,29 @@ def test_routing_of_thousands_of_tokens(cuda_device, N, d, E, k):
         assert status == int(disp["status"][0]), values
 
 
+@pytest.mark.parametrize("N,E,k,norm", [(3000, 8, 2, False), (2300, 40, 2, False), (3000, 8, 2, True), (300, 8, 2, None)])
+def test_large_calls_take_nothing_from_a_call_that_timed_out(cuda_device, N, E, k, norm):
+    """Status words and counters as a wait that ran out leaves them: the next large call, and the next training step (norm:
+    None) of any size, gives what a call on a clean workspace gives, and its own status."""
+    d, f = 64, 128
+    m = build(synthetic.make_params(d, E, f, seed=N), d, E, f, k, torch.bfloat16, cuda_device).train(norm is None)
+    x = torch.randn(1, N, d, generator=torch.Generator().manual_seed(E)).bfloat16().to(cuda_device)
+    ln = torch.nn.LayerNorm(d).to(device=cuda_device, dtype=torch.bfloat16) if norm else None
+
+    def call():
+        torch.manual_seed(3)
+        with torch.set_grad_enabled(norm is None):
+            out, aux = m(x, norm=ln) if norm else m(x)
+        return out.detach().clone(), aux.detach().clone(), *(m.last[n].clone() for n in ("logits", "idx", "w", "row_of", "psum"))
+
+    want = call()
+    assert m.device_status() == 0
+    region = m._view("status", torch.int32, (_cabi.READY_OFFSET + _cabi.READY_INTS,))
+    for left in (1, 16, 1 << 20, -5):
+        region.fill_(left)
+        assert all(torch.equal(a, b) for a, b in zip(call(), want)) and m.device_status() == 0
+
+
 # a whole bf16 call of 33 to 64 experts: one token, a block of one and of all 16, streaming and sorted-row sizes, one slot and eight
 @pytest.mark.parametrize("N,d,E,k", [(1, 64, 33, 1), (16, 2056, 64, 4), (33, 72, 63, 8), (130, 1024, 40, 2), (511, 520, 64, 8),
                                      (2048, 64, 64, 2)])
