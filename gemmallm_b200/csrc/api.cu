@@ -330,7 +330,7 @@ int moe_b200_front_small_split(const void* x, const void* Wg, const void* bg, in
     return set_error(MOE_B200_ERR_ALIGN, "x, Wg and perm must be 16-byte aligned");
   MOE_CUDA_CHECK(cudaMemsetAsync(counter, 0, sizeof(int32_t), (cudaStream_t)stream));
   return launch_front_small(x, Wg, bg, N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
-                            row_of, perm, psum, aux, (cudaStream_t)stream, exchange, counter, status, dtype, nullptr, 16);
+                            row_of, perm, psum, aux, (cudaStream_t)stream, exchange, status, dtype, nullptr, 16);
 }
 
 int moe_b200_decode_tiny(const void* x, const void* Wg, const void* bg, const void* plan,
@@ -513,7 +513,7 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
     rc = front_many_tokens(N, d, E, k, dtype, norm, &many);
     if (rc) return rc;
   }
-  const bool counters = small_n || rows_path || mid || many > 0;
+  const bool counters = small_n || rows_path || mid;
   const bool clean = (small_n || rows_path) && (flags & MOE_B200_FLAG_WS_CLEAN);
   // status words, and the completion counters behind them where a kernel uses them, in one memset
   // (above these sizes a call always clears both: the status words are those of the most recent call, and what a call that
@@ -535,12 +535,11 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
                               offsets, row_of, perm, psum, aux, h, out, status, s);
   if (front) {
     // router and dispatch of up to a few hundred tokens in one launch
-    // (beyond 128 tokens its blocks share the work and meet at a counter behind the status words)
+    // (beyond 128 tokens its blocks share the work and meet at a grid barrier)
     void* planes = front32 ? static_cast<char*>(h) + h_planes_bytes((size_t)N * k, f) : nullptr;
     // (spec reads the tokens where they lie, and waits for this kernel: 128 tokens 54.8 us with their copies, 52.1 without)
     rc = launch_front_small(x, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, spec ? nullptr : perm,
-                            psum, aux, s, scratch,
-                            status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, dtype, planes);
+                            psum, aux, s, scratch, status, dtype, planes);
     if (rc) return rc;
     if (front32) {
       const int parts = f32_down_splits(N * k, d, f, E);
@@ -565,8 +564,7 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
       if (fold) rc = launch_layernorm_rows(x, norm_weight, norm_bias, norm_eps, N, d, dtype, y, stats, s);
       if (rc) return rc;
       rc = launch_front_many(x, y, stats, fold ? nc : nullptr, fold ? wn : Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets,
-                             row_of, perm, nullptr, psum, aux, scratch,
-                             status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many, s);
+                             row_of, perm, nullptr, psum, aux, scratch, status, many, s);
       if (rc) return rc;
     } else if (fold) {
       rc = moe_b200_router_norm(x, wn, nc, norm_eps, N, d, E, k, dtype, logits, idx, w, psum_part,

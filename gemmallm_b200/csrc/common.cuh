@@ -370,12 +370,12 @@ int front_many_tokens(int64_t N, int d, int E, int k, int dtype, bool norm, int*
 int launch_front_many(const void* x, const void* xn, const float* stats, const float* norm_c, const void* Wg, const void* bg,
                       int64_t N, int d, int E, int k, float* logits, int32_t* idx, float* w, int32_t* cnt_slot,
                       int32_t* offsets, int32_t* row_of, void* perm, int32_t* pair_of, float* psum, float* aux, int32_t* xch,
-                      int* counter, int32_t* status, int per, cudaStream_t s);
+                      int32_t* status, int per, cudaStream_t s);
 int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E, int k,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
-                       cudaStream_t s, int* xch = nullptr, int* counter = nullptr,
-                       int32_t* status = nullptr, int dtype = MOE_B200_BF16, void* planes = nullptr, int per = 0);
+                       cudaStream_t s, int* xch = nullptr, int32_t* status = nullptr,
+                       int dtype = MOE_B200_BF16, void* planes = nullptr, int per = 0);
 // fp32, with the exchange buffer and room for the rows' bf16 planes [3][N k][d]; on this device only if its blocks are all
 // resident at once
 bool front_f32_supported(int64_t N, int E, int k);

@@ -1,12 +1,11 @@
 // Router and dispatch of a few thousand tokens in ONE launch (bf16): logits, softmax, top-k, counts, offsets, ranks, the sorted
 // copies of the rows and the load-balancing loss (reference model.py:206-253), and for a training step the pair of every row.
 //
-// A block routes a range of tokens, 16 at a time, exchanges its counts with the other blocks at a counter in global memory and
+// A block routes a range of tokens, 16 at a time, exchanges its counts with the other blocks at a grid barrier and
 // copies its tokens' rows. What bounds it is latency, not bandwidth: a group of 16 tokens is one round trip for its rows, one
 // meeting of the block's warps and one chain of softmax and top-k, so the next group's rows are under way during that chain
 // (its partial sums go to the other half of a double buffer, one block barrier a group), and the first rows to copy during
-// the exchange. The blocks are at most one an SM and are launched cooperatively, since they wait for one another; the wait is
-// bounded, and a block that gave up reports it and goes on as if nobody had any tokens.
+// the exchange. The blocks are at most one an SM and are launched cooperatively, since they wait for one another.
 //
 // Logits that are not finite are treated as by the general kernels that take the larger calls: up to 16 experts neither NaN nor
 // minus infinity is ever chosen, a slot without an expert has the index 0x7fffffff and no row, and the status says so; beyond,
@@ -28,8 +27,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
                   float* __restrict__ out_logits, int32_t* __restrict__ out_idx, float* __restrict__ out_w,
                   int32_t* __restrict__ cnt_slot, int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
                   __nv_bfloat16* __restrict__ perm, int32_t* __restrict__ pair_of, float* __restrict__ psum,
-                  float* __restrict__ aux, int* __restrict__ xch, int* __restrict__ counter, int32_t* __restrict__ status,
-                  int per, int share) {
+                  float* __restrict__ aux, int* __restrict__ xch, int32_t* __restrict__ status, int per, int share) {
   constexpr int ET = 8 * NT, EL = ET > 32 ? 2 : 1, GL = ET / EL, P = 32 / GL;      // experts a lane, lanes of a token
   constexpr bool STRICT = NT <= 2;
   static_assert(!NORM || STRICT, "with a folded LayerNorm the general router is the strict one at any number of experts");
@@ -199,38 +197,16 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
     if (nb == 1) s_sum[e] = ps;
     else xps[b * E + e] = ps;
   }
-  __syncthreads();
-  int left = 0;
-  if (nb > 1) {
-    bool dead = false;
-    if (tid == 0) {
-      __threadfence();
-      atomicAdd(counter, 1);
-      unsigned long long since = 0;
-      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(since));
-      for (uint32_t it = 0; ld_acquire_gpu_i32(counter) < nb; ++it) {
-        if ((it & 63u) == 63u) {
-          unsigned long long now;
-          asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-          if (now - since > 2000000000ull) {     // 2 s: some block of the grid never arrived
-            atomicMax(&status[0], MOE_B200_DEV_TIMEOUT);
-            status[1] = 42;
-            status[2] = b;
-            dead = true;
-            break;
-          }
-        }
-      }
-      // looked at in the end; not counted where the wait gave up, so that nobody takes it for another block's arrival
-      if (!dead) left = atomicAdd(counter, 1);
-    }
-    dead = __syncthreads_or(dead);
+  if (nb == 1) {
+    __syncthreads();
+  } else {
+    cooperative_groups::this_grid().sync();
     // totals, and the rows that earlier blocks put in front of this block's (16 bits: fewer than 65536 tokens)
     if (EL == 1) {      // a warp per count
       for (int je = warp; je < ke; je += kWarps) {
         unsigned both = 0;
         for (int bb = lane; bb < nb; bb += 32) {
-          const unsigned c = dead ? 0u : (unsigned)__ldcg(&xch[je * nb + bb]);
+          const unsigned c = (unsigned)__ldcg(&xch[je * nb + bb]);
           both += c | (bb < b ? c << 16 : 0u);
         }
         both = __reduce_add_sync(0xffffffffu, both);
@@ -245,7 +221,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
         unsigned both = 0;
 #pragma unroll 8
         for (int bb = q; bb < nb; bb += shares) {
-          const unsigned c = dead ? 0u : (unsigned)__ldcg(&xch[bb * ke + je]);
+          const unsigned c = (unsigned)__ldcg(&xch[bb * ke + je]);
           both += c | (bb < b ? c << 16 : 0u);
         }
         if (both & 0xffffu) atomicAdd(&s_tot[je], (int)(both & 0xffffu));
@@ -253,7 +229,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
       }
     }
     if (b == 0)
-      for (int i = tid; i < nb * E; i += 32 * kWarps) s_sum[i] = dead ? 0.f : __ldcg(&xps[i]);
+      for (int i = tid; i < nb * E; i += 32 * kWarps) s_sum[i] = __ldcg(&xps[i]);
     __syncthreads();
   }
 
@@ -356,14 +332,12 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
       if (lane == 0) aux[0] = a / (float)E * (float)(E * E);
     }
   }
-  // the last block to leave puts the meeting counter back to zero for the next call
-  if (tid == 0 && nb > 1 && left == 2 * nb - 1) *counter = 0;
 }
 
 template <int NT, bool NORM>
 int launch(const void* x, const void* xn, const float* stats, const float* norm_c, const void* Wg, const void* bg, int N, int d,
            int E, int k, float* logits, int32_t* idx, float* w, int32_t* cnt_slot, int32_t* offsets, int32_t* row_of, void* perm,
-           int32_t* pair_of, float* psum, float* aux, int32_t* xch, int* counter, int32_t* status, int per, cudaStream_t s) {
+           int32_t* pair_of, float* psum, float* aux, int32_t* xch, int32_t* status, int per, cudaStream_t s) {
   constexpr size_t part = sizeof(float) * 2 * kWarps * kGroup * 8 * NT;
   static PerDeviceOnce once;
   int rc = ensure_dynamic_smem(once, front_many_kernel<NT, NORM>, part + 2 * sizeof(int) * kMaxPer * kMaxTopK);
@@ -374,7 +348,7 @@ int launch(const void* x, const void* xn, const float* stats, const float* norm_
                                static_cast<const __nv_bfloat16*>(xn), stats, norm_c,
                                static_cast<const __nv_bfloat16*>(Wg), static_cast<const __nv_bfloat16*>(bg), N, d, E, k, logits,
                                idx, w, cnt_slot, offsets, row_of, static_cast<__nv_bfloat16*>(perm), pair_of, psum, aux, xch,
-                               counter, status, per, per < kWarps ? kWarps / per : 1));
+                               status, per, per < kWarps ? kWarps / per : 1));
   return 0;
 }
 
@@ -404,15 +378,15 @@ int front_many_tokens(int64_t N, int d, int E, int k, int dtype, bool norm, int*
 }
 
 // norm_c, or nullptr: a folded LayerNorm, with `stats` and the normalised rows `xn` of layernorm_rows.
-// xch: int32 scratch, (k + 1) * E words for each of kNumSMs blocks; counter: one int32 that is zero on entry and on exit.
+// xch: int32 scratch, (k + 1) * E words for each of kNumSMs blocks.
 int launch_front_many(const void* x, const void* xn, const float* stats, const float* norm_c, const void* Wg, const void* bg,
                       int64_t N, int d, int E, int k, float* logits, int32_t* idx, float* w, int32_t* cnt_slot,
                       int32_t* offsets, int32_t* row_of, void* perm, int32_t* pair_of, float* psum, float* aux, int32_t* xch,
-                      int* counter, int32_t* status, int per, cudaStream_t s) {
+                      int32_t* status, int per, cudaStream_t s) {
   auto fn = norm_c != nullptr ? (E <= 8 ? launch<1, true> : launch<2, true>)
             : E <= 8 ? launch<1, false> : E <= 16 ? launch<2, false> : E <= 32 ? launch<4, false> : launch<8, false>;
   return fn(x, norm_c != nullptr ? xn : x, stats, norm_c, Wg, bg, (int)N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of,
-            perm, pair_of, psum, aux, xch, counter, status, per, s);
+            perm, pair_of, psum, aux, xch, status, per, s);
 }
 
 }  // namespace moe

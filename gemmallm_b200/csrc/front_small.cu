@@ -38,7 +38,7 @@ front_small_kernel(const T* __restrict__ x, const T* Wg, const T* bg, int Ntotal
 // bf16 calls of more than 128 tokens: blocks of up to 16 tokens that share the work, of 16 warps. What a warp does counts four
 // times and not eight, its loads (both its chunks of the tokens and of the weights, its token's row for the copy) are in flight
 // together without spills, a token's softmax and top-k are a warp's and not a few lanes', and no step divides. Blocks meet
-// at a counter (up to 128 of them, one an SM, on an otherwise idle GPU); the wait is bounded and reports a time-out.
+// at a grid barrier (up to 128 of them, one an SM, launched cooperatively).
 // (front_small_body did it with 32 warps: 9.4 us from the wait to the end at 300 tokens, where this kernel takes 7.2. Whole
 // calls, d 1024, f 4096, 8 experts: 130 tokens 53.1 -> 51.6 us, 300 59.3 -> 57.9, 400 62.0 -> 60.9, 1173 88.0 -> 86.8.)
 constexpr int kMidWarps = 16, kMidTok = 16, kMidMaxE = 64;
@@ -62,7 +62,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
                  float* __restrict__ out_logits, int32_t* __restrict__ out_idx, float* __restrict__ out_w,
                  int32_t* __restrict__ cnt_slot, int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
                  __nv_bfloat16* __restrict__ perm, float* __restrict__ psum, float* __restrict__ aux, int* __restrict__ xch,
-                 int* __restrict__ counter, int32_t* __restrict__ status, int per, int share) {
+                 int per, int share) {
   constexpr int ET = 8 * NT, EL = ET > 32 ? 2 : 1, GL = ET / EL, P = 32 / GL;      // experts a lane, lanes of a token
   constexpr int kInFlight = 4, kChunks = NT > 4 ? 1 : 2;       // of a row to copy; of K
   extern __shared__ __align__(16) float s_dyn[];
@@ -213,38 +213,16 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
     if (nb == 1) s_sum[e] = ps;
     else xps[b * E + e] = ps;
   }
-  __syncthreads();
-  int left = 0;
-  if (nb > 1) {
-    bool dead = false;      // gave up: goes on as if nobody had any tokens, so that no row lies outside
-    if (tid == 0) {
-      __threadfence();
-      atomicAdd(counter, 1);
-      unsigned long long t0 = 0;
-      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-      for (uint32_t it = 0; ld_acquire_gpu_i32(counter) < nb; ++it) {
-        if ((it & 63u) == 63u) {
-          unsigned long long t1;
-          asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-          if (t1 - t0 > 2000000000ull) {     // 2 s: some block of the grid never arrived
-            atomicMax(&status[0], MOE_B200_DEV_TIMEOUT);
-            status[1] = 41;
-            status[2] = b;
-            dead = true;
-            break;
-          }
-        }
-      }
-      // looked at in the end; not counted where the wait gave up, so that nobody takes it for another block's arrival
-      if (!dead) left = atomicAdd(counter, 1);
-    }
-    dead = __syncthreads_or(dead);
+  if (nb == 1) {
+    __syncthreads();
+  } else {
+    cooperative_groups::this_grid().sync();
     // totals, and the rows that earlier blocks put in front of this block's (16 bits: 2048 tokens)
     if (EL == 1) {      // a warp per count
       for (int je = warp; je < ke; je += kMidWarps) {
         unsigned both = 0;
         for (int bb = lane; bb < nb; bb += 32) {
-          const unsigned c = dead ? 0u : (unsigned)__ldcg(&xch[je * nb + bb]);
+          const unsigned c = (unsigned)__ldcg(&xch[je * nb + bb]);
           both += c | (bb < b ? c << 16 : 0u);
         }
         both = __reduce_add_sync(0xffffffffu, both);
@@ -259,7 +237,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
         unsigned both = 0;
 #pragma unroll 8
         for (int bb = q; bb < nb; bb += per) {
-          const unsigned c = dead ? 0u : (unsigned)__ldcg(&xch[bb * ke + je]);
+          const unsigned c = (unsigned)__ldcg(&xch[bb * ke + je]);
           both += c | (bb < b ? c << 16 : 0u);
         }
         if (both & 0xffffu) atomicAdd(&s_tot[je], (int)(both & 0xffffu));
@@ -267,7 +245,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
       }
     }
     if (b == 0)
-      for (int i = tid; i < nb * E; i += 32 * kMidWarps) s_sum[i] = dead ? 0.f : __ldcg(&xps[i]);
+      for (int i = tid; i < nb * E; i += 32 * kMidWarps) s_sum[i] = __ldcg(&xps[i]);
     __syncthreads();
   }
 
@@ -346,25 +324,22 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
       if (lane == 0) aux[0] = a / (float)E * (float)(E * E);
     }
   }
-  // the last block to leave puts the meeting counter back to zero for the next call
-  if (tid == 0 && nb > 1 && left == 2 * nb - 1) *counter = 0;
 }
 
 template <int NT>
 int launch_mid(const void* x, const void* Wg, const void* bg, int N, int d, int E, int k, float* out_logits, int32_t* out_idx,
                float* out_w, int32_t* cnt_slot, int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux, int* xch,
-               int* counter, int32_t* status, int per, cudaStream_t s) {
+               int per, cudaStream_t s) {
   const size_t smem = sizeof(float) * kMidWarps * kMidTok * 8 * NT;
   static PerDeviceOnce once;
   int rc = ensure_dynamic_smem(once, front_mid_kernel<NT>, smem);
   if (rc) return rc;
-  // beyond 32 experts cooperative, as the dispatch is that such calls had: they run beside those of any other streams (1.6 us a
-  // call; up to 32 experts the meeting has always assumed that the GPU has room for all blocks)
+  // cooperative, since its blocks wait for one another: beside those of other streams they start when all of them fit
   const int blocks = (N + per - 1) / per;
-  MOE_CUDA_CHECK(launch_pdl_as(front_mid_kernel<NT>, dim3(blocks), dim3(32 * kMidWarps), 0, NT > 4 && blocks > 1, smem, s,
+  MOE_CUDA_CHECK(launch_pdl_as(front_mid_kernel<NT>, dim3(blocks), dim3(32 * kMidWarps), 0, blocks > 1, smem, s,
                             static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(Wg),
                             static_cast<const __nv_bfloat16*>(bg), N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
-                            row_of, static_cast<__nv_bfloat16*>(perm), psum, aux, xch, counter, status, per, kMidWarps / per));
+                            row_of, static_cast<__nv_bfloat16*>(perm), psum, aux, xch, per, kMidWarps / per));
   return 0;
 }
 
@@ -393,7 +368,7 @@ bool front_small_supported(int64_t N, int E, int k, int dtype) {
   return dtype == MOE_B200_BF16 && N >= 1 && N <= kMaxTok && N * k <= kMaxPairs && E <= kMaxE;
 }
 
-// With the exchange buffer and the counter (blocks share the work): as many tokens as give a grid
+// With the exchange buffer (blocks share the work): as many tokens as give a grid
 // whose blocks are all resident at once with room to spare.
 // (More than 32 experts where the general router is the tcgen05 kernel, whose choice among logits that are not finite is also
 // always an expert.)
@@ -401,9 +376,8 @@ bool front_split_supported(int64_t N, int d, int E, int k, int dtype) {
   return dtype == MOE_B200_BF16 && N >= 1 && N <= 16 * 128 && E <= kMidMaxE && (E <= kMaxE || d >= 64) && k <= kMaxTopK;
 }
 
-// xch: int32 scratch of at least front_small_exchange_ints(N, E, k) words and counter: one int32
-// that is zero on entry (both only used beyond 128 tokens or 32 experts; without them every block repeats the
-// whole routing at every size). per: tokens of a block that shares the work, 0 for the best number; with 16 the public
+// xch: int32 scratch of at least front_small_exchange_ints(N, E, k) words (only used beyond 128 tokens or 32 experts; without
+// it every block repeats the whole routing at every size). per: tokens of a block that shares the work, 0 for the best number; with 16 the public
 // entry's smaller exchange buffer does.
 int64_t front_small_exchange_ints(int64_t N, int E, int k) {
   const int64_t nb = N < 512 ? (N + 3) / 4 : 128;      // the most that either type has
@@ -436,15 +410,15 @@ int launch_by_experts(int E, Args... args) {
 int launch_front_small(const void* x, const void* Wg, const void* bg, int64_t N, int d, int E, int k,
                        float* out_logits, int32_t* out_idx, float* out_w, int32_t* cnt_slot,
                        int32_t* offsets, int32_t* row_of, void* perm, float* psum, float* aux,
-                       cudaStream_t s, int* xch, int* counter, int32_t* status, int dtype, void* planes, int per) {
+                       cudaStream_t s, int* xch, int32_t* status, int dtype, void* planes, int per) {
   if (dtype == MOE_B200_F32)
     return launch_by_experts<float>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of,
                                     perm, planes, psum, aux, xch, status, s);
   // beyond 128 tokens repeating the routing in every block costs more than one exchange
-  if (xch != nullptr && counter != nullptr && status != nullptr && (N > 128 || E > kMaxE)) {
+  if (xch != nullptr && (N > 128 || E > kMaxE)) {
     auto mid = E <= 8 ? launch_mid<1> : E <= 16 ? launch_mid<2> : E <= 32 ? launch_mid<4> : launch_mid<8>;
-    return mid(x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux, xch, counter,
-               status, per > 0 ? per : mid_tokens_per_block(N), s);
+    return mid(x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets, row_of, perm, psum, aux, xch,
+               per > 0 ? per : mid_tokens_per_block(N), s);
   }
   return launch_by_experts<__nv_bfloat16>(E, x, Wg, bg, (int)N, d, E, k, out_logits, out_idx, out_w, cnt_slot, offsets,
                                           row_of, perm, nullptr, psum, aux, xch, status, s);

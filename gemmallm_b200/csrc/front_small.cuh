@@ -40,16 +40,9 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ int ld_acquire_gpu_i32(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 }  // namespace front_detail
 
 using front_detail::mma_bf16_16816;
-using front_detail::ld_acquire_gpu_i32;
 
 // bf16: every block derives the complete routing (fastest up to about a hundred tokens; beyond, front_mid_kernel in
 //   front_small.cu).

@@ -279,8 +279,7 @@ int forward_train_into(const void* x, const void* Wg, const void* bg, const void
   MOE_CUDA_CHECK(cudaMemsetAsync(status, 0, (MOE_B200_READY_OFFSET + MOE_B200_READY_INTS) * sizeof(int32_t), s));
   if (many > 0) {
     rc = launch_front_many(x, nullptr, nullptr, nullptr, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm,
-                           pair_of, psum, aux, scratch, status + MOE_B200_READY_OFFSET + MOE_B200_READY_INTS - 4, status, many,
-                           s);
+                           pair_of, psum, aux, scratch, status, many, s);
     if (rc) return rc;
   } else {
     rc = moe_b200_router(x, Wg, bg, N, d, E, k, dtype, logits, idx, w, psum_part, status, stream);

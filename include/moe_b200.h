@@ -262,8 +262,9 @@ int moe_b200_front_small(const void* x, const void* Wg, const void* bg,
 /* The same results from blocks that share the work: beyond 128 tokens every block of
  * moe_b200_front_small would repeat the whole routing; here block b routes tokens 16b..16b+15,
  * the blocks exchange their counts through `exchange` (int32, at least
- * moe_b200_front_exchange_ints(N,E,k) words) and meet at `counter` (one int32, zeroed by this
- * call; bounded wait, MOE_B200_DEV_TIMEOUT in `status` if a block never arrives). bf16,
+ * moe_b200_front_exchange_ints(N,E,k) words) and meet at a grid barrier (a cooperative launch: an
+ * error where the GPU cannot hold its blocks at once). `counter`, one int32, is zeroed; `status` is
+ * left alone. bf16,
  * 1 <= N <= 2048, E <= 32. Up to 128 tokens it runs exactly moe_b200_front_small. The logits differ from that function's in the
  * order their partial sums are added; everything derived from them is derived the same way. */
 int moe_b200_front_small_split(const void* x, const void* Wg, const void* bg,

@@ -267,6 +267,41 @@ def test_routing_of_many_experts(cuda_device, N, d, E, k):
     assert bool(got[others].isfinite().all())
 
 
+# fronts whose blocks meet: 8 and 16 tokens a block, up to 32 experts and more, and a block an SM
+@pytest.mark.parametrize("N,E,k", [(512, 8, 2), (2048, 8, 2), (1000, 40, 2), (3000, 8, 2), (2500, 40, 2)])
+def test_bf16_calls_on_three_streams_and_in_a_graph(cuda_device, N, E, k):
+    """Three calls at once, whose fronts together have more blocks than there are SMs; then all from one graph. Words of the
+    status region that no kernel of such a call uses may hold anything."""
+    d, f = 64, 128
+    params = synthetic.make_params(d, E, f, seed=3)
+    mods = [build(params, d, E, f, k, torch.bfloat16, cuda_device) for _ in range(3)]
+    xs = [torch.randn(1, N, d, generator=torch.Generator().manual_seed(i)).bfloat16().to(cuda_device) for i in range(3)]
+    with torch.no_grad():
+        want = [m(x)[0] for m, x in zip(mods, xs)]
+        for m in mods:      # (where the blocks met before: one left there let the next call's blocks pass at once)
+            m._view("status", torch.int32, (_cabi.READY_OFFSET + _cabi.READY_INTS,))[-4] = 7
+        torch.cuda.synchronize()
+        streams = [torch.cuda.Stream() for _ in range(3)]
+        got = [[], [], []]
+        for _ in range(50):
+            for i, st in enumerate(streams):
+                with torch.cuda.stream(st):
+                    got[i].append(mods[i](xs[i])[0])
+        torch.cuda.synchronize()
+        for i in range(3):
+            assert mods[i].device_status() == 0
+            assert all(torch.equal(o, want[i]) for o in got[i])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = [m(x)[0] for m, x in zip(mods, xs)]
+        for _ in range(3):
+            for o in captured:
+                o.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert all(torch.equal(o, w) for o, w in zip(captured, want))
+
+
 @pytest.mark.parametrize("E,k", [(8, 2), (9, 8), (17, 3), (32, 4)])
 def test_fp32_logits_that_are_not_finite(cuda_device, E, k):
     """Routing in one launch as the general kernel gives it: gate biases of NaN and both infinities, for some experts up
