@@ -22,7 +22,7 @@ struct Eight {
   uint4 raw[sizeof(T) / 2];
   __device__ __forceinline__ void load(const T* p) {
 #pragma unroll
-    for (int i = 0; i < (int)sizeof(T) / 2; ++i) raw[i] = reinterpret_cast<const uint4*>(p)[i];
+    for (int i = 0; i < (int)sizeof(T) / 2; ++i) raw[i] = __ldcg(reinterpret_cast<const uint4*>(p) + i);
   }
   __device__ __forceinline__ void get(float (&v)[8]) const {
     if constexpr (sizeof(T) == 2) {
@@ -40,11 +40,13 @@ struct Eight {
   }
 };
 
-// K: the number of slots, 0 for any other. FEW: N * pieces < 2^31.
+// K: the number of slots, 0 for any other (the workloads have one, two or four; unrolled, three slots of 32768 tokens, d 1024,
+// would take 47 us and not 54, six of 16384, d 2048, 85 and not 92, eight 113 as they do). FEW: N * pieces < 2^31.
+// (y comes from the kernel in front, which may still run where this one starts, row_of and w perhaps as well: no loads of
+// constant data, so no __restrict__)
 template <typename T, int K, bool FEW>
 __global__ void __launch_bounds__(256)
-combine_kernel(const T* __restrict__ y, const int32_t* __restrict__ row_of,
-               const float* __restrict__ w, const T* __restrict__ residual, int64_t N, int d,
+combine_kernel(const T* y, const int32_t* row_of, const float* w, const T* residual, int64_t N, int d,
                int k, T* __restrict__ out, const EpSync sy, int32_t* __restrict__ status) {
   const int pieces = d >> 3;
   const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -67,8 +69,8 @@ combine_kernel(const T* __restrict__ y, const int32_t* __restrict__ row_of,
     Eight<T> yj[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      row[j] = row_of != nullptr ? __ldg(&row_of[t * K + j]) : (int)(t * K + j);
-      wj[j] = __ldg(&w[t * K + j]);
+      row[j] = row_of != nullptr ? row_of[t * K + j] : (int)(t * K + j);
+      wj[j] = w[t * K + j];
     }
 #pragma unroll
     for (int j = 0; j < K; ++j)
@@ -83,11 +85,13 @@ combine_kernel(const T* __restrict__ y, const int32_t* __restrict__ row_of,
     }
   } else {
     for (int j = 0; j < k; ++j) {
-      const int row = row_of != nullptr ? __ldg(&row_of[t * k + j]) : (int)(t * k + j);
+      const int row = row_of != nullptr ? row_of[t * k + j] : (int)(t * k + j);
       if (row < 0) continue;
-      const float wj = __ldg(&w[t * k + j]);
+      const float wj = w[t * k + j];
+      Eight<T> yj;
+      yj.load(y + (int64_t)row * d + c);
       float v[8];
-      load8(y + (int64_t)row * d + c, v);
+      yj.get(v);
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(wj, v[i]));
     }
