@@ -10,7 +10,7 @@ import ctypes as C
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libmoe_b200.so"
-ABI_VERSION = 3
+ABI_VERSION = 4
 
 F32, BF16 = 0, 1
 FLAG_DEFAULT, FLAG_WS_CLEAN = 0, 1

@@ -32,9 +32,10 @@
 extern "C" {
 #endif
 
-/* 3: plans hold a fifth tensor map an expert; after a training forward MOE_B200_TWS_GU holds derivatives of h instead of
+/* 4: MOE_B200_WS_PSUM_PART, _PERM, _H and _Y are not what they were after every forward call (see there).
+ * 3: plans hold a fifth tensor map an expert; after a training forward MOE_B200_TWS_GU holds derivatives of h instead of
  * pre-activations, and MOE_B200_TWS_MASK is written in LoRA steps only. */
-#define MOE_B200_ABI_VERSION 3
+#define MOE_B200_ABI_VERSION 4
 
 enum { MOE_B200_F32 = 0, MOE_B200_BF16 = 1 };
 
@@ -88,7 +89,10 @@ enum {
   MOE_B200_WS_LOGITS,     /* float [N,E]   router logits (model.py:206) */
   MOE_B200_WS_IDX,        /* int32 [N,k]   chosen experts, slot 0 = best (model.py:210) */
   MOE_B200_WS_W,          /* float [N,k]   renormalised scores (model.py:219-223) */
-  MOE_B200_WS_PSUM_PART,  /* float [router blocks, E] partial sums of softmax */
+  MOE_B200_WS_PSUM_PART,  /* float [router blocks, E] partial sums of softmax; not written where router and
+                           * dispatch are one launch: bf16 calls of up to 4096 rows and of up to 18944 tokens (16
+                           * experts; 9472: 32, or 16 and a folded LayerNorm; 3552: 64), training forwards of as many
+                           * tokens, fp32 calls of up to 2048 tokens and 4096 rows */
   MOE_B200_WS_PSUM,       /* float [E]     sum over tokens of softmax (model.py:215) */
   MOE_B200_WS_AUX,        /* float [1]     load-balancing loss (model.py:216) */
   MOE_B200_WS_SCRATCH,    /* int32 [moe_b200_dispatch_scratch_bytes/4] dispatch scratch */
@@ -99,7 +103,8 @@ enum {
                            * tokens with at least E pairs, which read the tokens where they lie */
   MOE_B200_WS_H,          /* T [N*k, f]    gelu_tanh(gate)*up (model.py:180-182); fp32 calls of up to 2048 tokens and
                            * 4096 rows: scratch of h and the sorted rows as bf16 parts */
-  MOE_B200_WS_Y,          /* T [N*k, d]    expert outputs, sorted order (model.py:184) */
+  MOE_B200_WS_Y,          /* T [N*k, d]    expert outputs, sorted order (model.py:184); not written by calls that leave
+                           * the down product as partial sums in PART */
   MOE_B200_WS_PART,       /* float [splits, N*k, d] split-K partial sums of the small-N path
                            * (bf16 calls of up to 4096 rows; fp32 calls as above whose down product
                            * is split over K) */

@@ -45,10 +45,11 @@ def test_version_and_sizes():
 
 
 def test_version_goes_with_the_plan_and_the_training_workspace():
-    """A caller built against another layout of a plan, or against other contents of GU and MASK, sees another version."""
+    """A caller built against another layout of a plan, or against other contents of GU and MASK or of the forward's PSUM_PART,
+    PERM, H and Y, sees another version."""
     maps = [(lib.moe_b200_plan_bytes(E) - (32 * E + 127) // 128 * 128) / (128 * E) for E in (1, 8, 256)]
-    assert (lib.moe_b200_version(), maps) == (3, [5, 5, 5])
-    assert re.search(r"ABI_VERSION 3\b", HEADER.read_text())
+    assert (lib.moe_b200_version(), maps) == (4, [5, 5, 5])
+    assert re.search(r"ABI_VERSION 4\b", HEADER.read_text())
 
 
 def test_bad_shapes_are_rejected_on_the_host():
