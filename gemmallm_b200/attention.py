@@ -48,6 +48,8 @@ class _MergedLinear:
 
 
 class Attention(nn.Module):
+    _status = None          # (also of a module that was saved without it)
+
     def __init__(self, hidden_dim: int, head_dim: int, q_head: int, kv_head: int, embedding: nn.Module,
                  lora_rank: int = 16, lora_alpha: int = 32):
         super().__init__()
@@ -71,7 +73,7 @@ class Attention(nn.Module):
             self.multi_query_attention = False
         self.gate = nn.Linear(hidden_dim, q_head)
         self._merged_qkv, self._merged_o = _MergedLinear(), _MergedLinear()
-        self._table, self._status = None, None
+        self._table = None
 
     def _status_words(self, device):
         if self._status is None or self._status.device != device:
@@ -79,8 +81,14 @@ class Attention(nn.Module):
         return self._status
 
     def device_status(self) -> int:
-        """Status word of the calls so far (0 = ok; see moe_b200.h); synchronises."""
-        return 0 if self._status is None else int(self._status[0])
+        """Status word of the calls since it was last asked for (0 = ok; see moe_b200.h); synchronises. A non-zero status
+        is returned once, so that later calls start clean."""
+        if self._status is None:
+            return 0
+        code = int(self._status[0])
+        if code != 0:
+            self._status.zero_()
+        return code
 
     def _pos_table(self, device):
         pe = self.embedding.pos_emb

@@ -75,6 +75,13 @@ class LLMLayer(nn.Module):
                                    lora_rank=lora_rank, lora_alpha=lora_alpha)
         self.device = device
 
+    def device_status(self) -> int:
+        """Status word of the layer's own kernels (0 = ok): the attention's, or else the block's; synchronises. Both are
+        asked for and start clean again."""
+        parts = [self.mqa, self.moe] if self.use_moe else [self.mqa]
+        codes = [m.device_status() for m in parts if hasattr(m, "device_status")]
+        return next((c for c in codes if c != 0), 0)
+
     def _attend(self, tensor, attention_mask, fine_tuning):
         """First LayerNorm, attention and first skip connection (model.py:297-308): in one native call, or step by step,
         whose results are the same to the bit."""

@@ -907,6 +907,24 @@ def test_own_linears_of_the_attention_give_no_derivatives():
         assert not own()
 
 
+def test_status_of_a_layer():
+    """Of its attention or of its block, each returned once; and of an attention that was saved before it had any."""
+    layer = LLMLayer(D, 64, 2, 1, Table(16, 64), expansion_factor=1, use_moe=True, num_experts=E, device="cuda")
+    assert layer.device_status() == 0 and layer.mqa.device_status() == 0
+    words = layer.mqa._status_words(torch.device("cpu"))
+    words[:3] = torch.tensor([1, 34, 5], dtype=torch.int32)
+    assert layer.device_status() == 1 and layer.device_status() == 0 and not words.any()
+    words[0] = 1
+    layer.moe.device_status = lambda: 2
+    assert [layer.device_status(), layer.device_status()] == [1, 2]
+    old = Attention(D, 64, 2, 1, Table(16, 64))
+    old.__dict__.pop("_status", None)
+    assert old.device_status() == 0 and old._status_words(torch.device("cpu")).numel() == 16
+    plain = LLMLayer(D, 64, 2, 1, Table(16, 64), use_moe=False)
+    plain.mqa = torch.nn.Identity()
+    assert plain.device_status() == 0
+
+
 class Scaled(torch.Tensor):
     """A weight that is half of what it stands for, and keeps it elsewhere."""
 
