@@ -9,7 +9,8 @@
 //
 // Logits that are not finite are treated as by the general kernels that take the larger calls: up to 16 experts neither NaN nor
 // minus infinity is ever chosen, a slot without an expert has the index 0x7fffffff and no row, and the status says so; beyond,
-// every slot gets an expert.
+// every slot gets an expert, NaN after all others, and the weights are formed of the chosen logits alone: one expert whose
+// logits are NaN does not make those of the others NaN.
 #include "front_small.cuh"
 
 namespace moe {
@@ -128,6 +129,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
         const unsigned u = __float_as_uint(v[i]);
         key[i] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);      // order-preserving
         if (STRICT && !(v[i] > -INFINITY)) key[i] = 0u;           // never chosen
+        if (!STRICT && !(live && v[i] == v[i])) key[i] = live ? 1u : 0u;      // below every number's: chosen last; never
         kmax = max(kmax, key[i]);
       }
       kmax = __reduce_max_sync(0xffffffffu, kmax);
@@ -153,7 +155,8 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
         const int winner = low != 0u ? __ffs(low) - 1 : 31 + __ffs(high);
         const float bv = __uint_as_float((km & 0x80000000u) ? (km & 0x7fffffffu) : ~km);
         const bool none = STRICT && km == 0u;
-        const float val = (none ? 0.f : expf(bv - m)) / sum;
+        // (beyond 16 experts as router_tc_kernel: the denominator, which the sum of the chosen cancels, is left out)
+        const float val = STRICT ? (none ? 0.f : expf(bv - m)) / sum : expf(bv - m);
         total += val;                    // left-to-right sum, as model.py:221
         if (lane == j) { my_sel = none ? 0x7fffffff : winner; my_val = val; }
 #pragma unroll

@@ -53,7 +53,8 @@ int mid_tokens_per_block(int64_t N) {
   return N <= 512 ? 8 : kMidTok;
 }
 
-// More than 32 experts, two a lane: calls of up to 2048 tokens and 4096 rows, from one token on (d 2048, 64 experts of f 1408,
+// More than 32 experts, two a lane, logits that are not finite as in front_many.cu: calls of up to 2048 tokens and 4096 rows,
+// from one token on (d 2048, 64 experts of f 1408,
 // four slots, whole calls against the general router and dispatch: 1 token 60.4 -> 48.2 us, 8 111 -> 98.5, 100 206 -> 198,
 // 1000 213 -> 200).
 template <int NT>      // 8 NT >= E
@@ -147,7 +148,8 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
       const bool live = e < E;
       v[i] = live ? v[i] + 0.f : -INFINITY;      // + 0: no negative zero
       const unsigned u = __float_as_uint(v[i]);
-      key[i] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);      // order-preserving; NaN is the largest
+      key[i] = (u & 0x80000000u) ? ~u : (u | 0x80000000u);      // order-preserving
+      if (EL > 1 && !(live && v[i] == v[i])) key[i] = live ? 1u : 0u;      // below every number's: chosen last; never
       kmax = max(kmax, key[i]);
     }
     kmax = __reduce_max_sync(0xffffffffu, kmax);
@@ -174,7 +176,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
       const unsigned high = EL > 1 ? __ballot_sync(0xffffffffu, key[EL - 1] == km) : 0u;
       const int winner = low != 0u ? __ffs(low) - 1 : 31 + __ffs(high);
       const float bv = __uint_as_float((km & 0x80000000u) ? (km & 0x7fffffffu) : ~km);
-      const float val = expf(bv - m) * inv_sum;
+      const float val = EL > 1 ? expf(bv - m) : expf(bv - m) * inv_sum;      // (as router_tc_kernel: their sum cancels the denominator)
       total += val;
       if (lane == j) { my_sel = winner; my_val = val; }
 #pragma unroll
@@ -184,7 +186,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
     if (lane < k) {
       s_idx[warp * k + lane] = my_sel;
       out_idx[warp * k + lane] = my_sel;
-      out_w[warp * k + lane] = my_val * __frcp_rn(total);
+      out_w[warp * k + lane] = EL > 1 ? my_val / total : my_val * __frcp_rn(total);
     }
   } else {      // (no token: below, nothing has to ask)
     if (lane < k) s_idx[warp * k + lane] = -1;

@@ -57,8 +57,10 @@ enum {
   MOE_B200_DEV_TIMEOUT = 1,   /* a bounded wait inside a kernel ran out */
   /* an expert index outside [0,E) was seen: a token with fewer than k logits that are not NaN
    * (a row of x with a NaN has none). Such a slot has no row and adds nothing to the output. The
-   * bf16 kernels of small calls (moe_b200_front_small, moe_b200_decode_tiny) take NaN for the
-   * largest logit instead: the token's output is NaN and nothing is reported. */
+   * bf16 kernels of small calls (moe_b200_front_small, moe_b200_decode_tiny) route such a token
+   * all the same: its output is NaN and nothing is reported. So do all bf16 calls of 17 to 64 experts
+   * without a folded LayerNorm beyond them, where an expert whose logit is NaN is chosen after all others
+   * and takes nothing from the weights of those that are chosen. */
   MOE_B200_DEV_BAD_INDEX = 2
 };
 

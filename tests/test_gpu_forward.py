@@ -211,6 +211,41 @@ def test_routing_of_thousands_of_tokens(cuda_device, N, d, E, k):
         assert status == int(disp["status"][0]), values
 
 
+# router and dispatch in one launch, up to 2048 tokens and 4096 rows and beyond
+@pytest.mark.parametrize("N,d,E,k", [(1, 64, 64, 4), (130, 1024, 40, 2), (700, 64, 33, 8), (2048, 72, 64, 2), (2200, 64, 17, 2),
+                                     (3000, 128, 32, 4), (3001, 64, 40, 8), (1025, 2056, 64, 4)])
+def test_logits_of_many_experts_that_are_not_finite(cuda_device, N, d, E, k):
+    """As the general router of 17 to 64 experts has it: NaN is not chosen while there are numbers, and the weights are those of
+    the chosen alone. Where a token has fewer than k logits above minus infinity its slots still have experts of their own."""
+    x = torch.randn(N, d, generator=torch.Generator().manual_seed(E + N)).bfloat16().to(cuda_device)
+    params = synthetic.make_params(d, E, 8, seed=N)
+    m = build(params, d, E, 8, k, torch.bfloat16, cuda_device)
+    gate = (m.gate.weight.detach(), m.gate.bias.detach())
+    nan, inf = float("nan"), float("inf")
+    for values, token in [({0: nan}, 0.), ({E - 1: nan, 9: nan}, 0.), ({3: -inf}, 0.), ({0: inf, 1: -inf}, 0.), ({2: inf, 5: inf}, 0.),
+                          (dict.fromkeys(range(E), nan), 0.), (dict.fromkeys(range(E - 1), -inf), 0.),
+                          (dict.fromkeys(range(E), -inf), 0.), ({}, nan), ({}, inf)]:
+        m.gate.bias.data.copy_(params["gate_b"])
+        for e, v in values.items():
+            m.gate.bias.data[e] = v
+        xx = x.clone()
+        if token != 0.:
+            xx[N // 2, 3] = token
+        with torch.no_grad():
+            m(xx.view(1, N, d))
+        got_idx, got_w = m.last["idx"].cpu(), m.last["w"].cpu()
+        assert m.device_status() == 0, values
+        logits, idx, w = [t.cpu() for t in helpers.router(xx, *gate, k)[:3]]
+        enough = (logits > -inf).sum(1) >= k
+        same = (got_idx == idx).all(1)
+        assert int((enough & ~same).sum()) <= N // 500, values      # near-ties
+        assert got_idx.min() >= 0 and got_idx.max() < E
+        ordered = got_idx.sort(1).values
+        assert (ordered[:, 1:] != ordered[:, :-1]).all(), values
+        # fp32 sums of the logits in another order, as above; without k numbers the choice is another one, the weights are the same
+        assert torch.allclose(got_w[same | ~enough], w[same | ~enough], atol=4e-6, rtol=0, equal_nan=True), values
+
+
 @pytest.mark.parametrize("N,E,k,norm", [(3000, 8, 2, False), (2300, 40, 2, False), (3000, 8, 2, True), (300, 8, 2, None)])
 def test_large_calls_take_nothing_from_a_call_that_timed_out(cuda_device, N, E, k, norm):
     """Status words and counters as a wait that ran out leaves them: the next large call, and the next training step (norm:
