@@ -146,7 +146,9 @@ layernorm_rows_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
   });
   if (stats != nullptr && lane == 0) {
     stats[2 * row] = mean;
-    stats[2 * row + 1] = rstd;
+    // (as the general routers: for a row with an infinity, whose variance is NaN, of zero; its logits are then infinities or
+    // NaN, each as its expert's weights make them, and its normalised row is NaN)
+    stats[2 * row + 1] = rsqrtf(fmaxf(sq / (float)d, 0.f) + eps);
   }
 }
 

@@ -10,6 +10,7 @@ import torch
 
 import helpers
 from gemmallm_b200 import MOE, _cabi, synthetic
+from gemmallm_b200._cabi import check, lib
 from oracle import moe_oracle
 
 pytestmark = pytest.mark.gpu
@@ -267,6 +268,47 @@ def test_large_calls_take_nothing_from_a_call_that_timed_out(cuda_device, N, E, 
     for left in (1, 16, 1 << 20, -5):
         region.fill_(left)
         assert all(torch.equal(a, b) for a, b in zip(call(), want)) and m.device_status() == 0
+
+
+@pytest.mark.parametrize("N,E,k", [(2049, 8, 2), (2500, 16, 3), (5000, 9, 8)])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_tokens_that_are_not_finite_behind_a_folded_layernorm(cuda_device, N, E, k, value):
+    """Routed as by the general folded router, whichever experts that leaves: with any the output is NaN, and it is reported
+    where there are fewer than k. The other tokens are as without them."""
+    d, dev = 128, cuda_device
+    params = synthetic.make_params(d, E, 32, seed=N)
+    m = build(params, d, E, 32, k, torch.bfloat16, dev)
+    norm = torch.nn.LayerNorm(d).to(device=dev, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(E)
+    with torch.no_grad():
+        norm.weight.copy_(1 + torch.randn(d, generator=g) / 4), norm.bias.copy_(torch.randn(d, generator=g) / 4)
+    x = torch.randn(N, d, generator=g).bfloat16().to(dev)
+    rows = torch.arange(0, N, 97, device=dev)
+    bad = x.clone()
+    # (not the first column: the general kernels take a row's first element from all others, and no logit is left of an infinity)
+    bad[rows, 1 + torch.arange(len(rows), device=dev) % (d - 1)] = value
+    wn, c = torch.empty(E, d, dtype=torch.bfloat16, device=dev), torch.empty(2 * E, device=dev)
+    gate, s = (m.gate.weight.detach(), m.gate.bias.detach()), helpers.stream(dev)
+    check(lib.moe_b200_norm_fold(gate[0].data_ptr(), gate[1].data_ptr(), norm.weight.data_ptr(), norm.bias.data_ptr(), E, d,
+                                 _cabi.BF16, wn.data_ptr(), c.data_ptr(), s), "norm_fold")
+    logits, idx = torch.empty(N, E, device=dev), torch.empty(N, k, dtype=torch.int32, device=dev)
+    w, part = torch.empty(N, k, device=dev), torch.empty(lib.moe_b200_router_blocks(N), E, device=dev)
+    stats, status = torch.empty(N, 2, device=dev), torch.zeros(16, dtype=torch.int32, device=dev)
+    check(lib.moe_b200_router_norm(bad.data_ptr(), wn.data_ptr(), c.data_ptr(), float(norm.eps), N, d, E, k, _cabi.BF16,
+                                   logits.data_ptr(), idx.data_ptr(), w.data_ptr(), part.data_ptr(), stats.data_ptr(),
+                                   status.data_ptr(), s), "router_norm")
+    with torch.no_grad():
+        want = m(x.view(1, N, d), norm=norm)[0][0]
+        got = m(bad.view(1, N, d), norm=norm)[0][0]
+    assert torch.equal(m.last["idx"][rows], idx[rows])
+    new = m.last["logits"][rows]
+    assert torch.equal(new.isnan(), logits[rows].isnan()) and torch.equal(new.isposinf(), logits[rows].isposinf())
+    assert m.device_status() == (2 if (idx >= E).any() else 0)
+    routed = (idx[rows] < E).any(1)
+    assert got[rows[routed]].isnan().all() and (value != value or routed.any())
+    others = torch.ones(N, dtype=torch.bool, device=dev)
+    others[rows] = False
+    assert torch.equal(got[others], want[others])
 
 
 # a whole bf16 call of 33 to 64 experts: one token, a block of one and of all 16, streaming and sorted-row sizes, one slot and eight
