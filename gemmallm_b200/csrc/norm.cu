@@ -85,7 +85,7 @@ template <> struct RawPiece<float> {
 
 template <typename T, int KEEP>
 __global__ void __launch_bounds__(256)
-layernorm_rows_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
+layernorm_rows_kernel(const T* x /* may come from the kernel in front: no constant data */, const T* __restrict__ gamma,
                       const T* __restrict__ beta, float eps, int64_t N, int d, T* __restrict__ out,
                       float* __restrict__ stats /* nullable [N][2] */) {
   pdl_wait();
