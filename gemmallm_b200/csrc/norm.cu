@@ -145,9 +145,11 @@ layernorm_rows_kernel(const T* x /* may come from the kernel in front: no consta
     store8(out + row * d + c, o);
   });
   if (stats != nullptr && lane == 0) {
-    stats[2 * row] = mean;
-    // (as the general routers: for a row with an infinity, whose variance is NaN, of zero; its logits are then infinities or
-    // NaN, each as its expert's weights make them, and its normalised row is NaN)
+    // (a row with an infinity as in the general routers, which take its first element from all others and a variance of NaN for
+    // zero: its logits are infinities or NaN, each as its expert's weights make them, or all NaN where it is the first element;
+    // its normalised row is NaN)
+    const float x0 = to_f32(xr[0]);
+    stats[2 * row] = mean + (x0 - x0);
     stats[2 * row + 1] = rsqrtf(fmaxf(sq / (float)d, 0.f) + eps);
   }
 }

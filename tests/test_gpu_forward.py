@@ -285,8 +285,7 @@ def test_tokens_that_are_not_finite_behind_a_folded_layernorm(cuda_device, N, E,
     x = torch.randn(N, d, generator=g).bfloat16().to(dev)
     rows = torch.arange(0, N, 97, device=dev)
     bad = x.clone()
-    # (not the first column: the general kernels take a row's first element from all others, and no logit is left of an infinity)
-    bad[rows, 1 + torch.arange(len(rows), device=dev) % (d - 1)] = value
+    bad[rows, torch.arange(len(rows), device=dev) % d] = value      # (with an infinity in the first column no logit is left)
     wn, c = torch.empty(E, d, dtype=torch.bfloat16, device=dev), torch.empty(2 * E, device=dev)
     gate, s = (m.gate.weight.detach(), m.gate.bias.detach()), helpers.stream(dev)
     check(lib.moe_b200_norm_fold(gate[0].data_ptr(), gate[1].data_ptr(), norm.weight.data_ptr(), norm.bias.data_ptr(), E, d,
