@@ -1,7 +1,8 @@
 """Drop-in for the reference's ``Attention`` (model.py:59-152): same constructor, attribute
 and parameter names, ``state_dict`` layout and ``forward`` signature. The fused QKV Linear and the
 head gate are one launch (``moe_b200_linear_rows``), the output Linear another (torch's Linears where sizes or
-places are not those it takes: a number of heads that is no multiple of 8, from 129 rows on); everything between
+places are not those it takes — a number of heads that is no multiple of 8, from 129 rows on — and where their
+derivatives are asked for or their weights are of a class of their own); everything between
 them — head split, shared KV heads, RoPE from the model's own table, scores, mask, softmax,
 the product with V and the sigmoid head gate — is one kernel of libmoe_b200
 (``moe_b200_attention``), so the [B, H, S, S] score tensor is never materialised.

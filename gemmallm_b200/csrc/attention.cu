@@ -11,10 +11,11 @@
 // products. HBM traffic = QKV in, output out; what bounds it is the trips to shared memory and their latency with
 // two blocks an SM. Fragments come by ldmatrix (36 loads an item instead of 144), the position table 16 bytes a
 // lane, the mask 8 bytes a lane; queries and outputs do not go through shared memory. (Three blocks an SM, which then fit,
-// took longer: 110 us.)
+// took longer: 110 us in that trace.)
 // A block takes an equal share of all rounds of eight tiles, whatever sequence they are of, and stages table and mask once
-// (a block a sequence: 512 sequences were 1.7 waves of blocks, and took two). Sequences of 64 tokens, 16 heads, behind the QKV
-// product: 512 of them 99 -> 89.6 us, 100 30 -> 26.6; queries and outputs through shared memory before.
+// (a block a sequence: 512 sequences were 1.7 waves of blocks, and took two). Sequences of 64 tokens, 16 heads, queries and outputs
+// through shared memory before: 512 of them 79.7 -> 71.1 us, 100 25.9 -> 20.6 (behind the QKV product, in a trace: 99 -> 89.6 and
+// 30 -> 26.6).
 #include "common.cuh"
 
 namespace moe {

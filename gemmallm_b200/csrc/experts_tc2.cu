@@ -40,8 +40,9 @@
 // kLinear, kLinearSkip: the Linears around the attention core (model.py:104, 139, 150), QKV and head gate as one product, the
 // output Linear with the skip connection behind it (model.py:308), whose pieces are asked for before a tile's accumulator is
 // awaited (in the epilogue's stores they made it the bound: 100 us, now 60 to 75). 32768 tokens, d 1024, 16 heads, one KV
-// head: QKV and gate 75 us as two library products, 56 here; output Linear and addition 87, 65. A decoder layer, 8 experts:
-// 512 tokens 109.7 -> 103.1 us, 1024 128.4 -> 119.5, 4096 279 -> 267, 6528 393 -> 388, 32768 1729 -> 1680 (two runs each).
+// head: QKV and gate 75 us as two library products, 56 here; output Linear and addition 87, 65. A decoder layer, 8 experts,
+// torch's Linears -> these: 512 tokens 108.6 -> 104.7 us, 1024 125.4 -> 120.3, 4096 236 -> 225, 6528 341 -> 328, 32768 1560 to 1629
+// -> 1528 to 1591 (three runs each).
 #include <cuda.h>
 #include "common.cuh"
 #include "tc_ptx.cuh"

@@ -359,12 +359,13 @@ int launch(const void* x, const void* xn, const float* stats, const float* norm_
 
 // Tokens of a block for a call that this kernel takes, 0 for any other: as many as give every SM one block, a few (a power of
 // two) where that shortens the copies. A block reads the router's weights once per 16 tokens and has its groups one after the
-// other, which the general kernels do not: the more experts, the fewer tokens. Whole calls, general kernels -> this one:
-// 8 experts, d 1024: 2560 tokens 158.7 -> 144.6 us, 6400 319 -> 306, 16384 729 -> 718; 16 experts: 3840 135 -> 118, 15360
-// 384 -> 376; 32 experts, d 2048: 2560 135 -> 120, 7680 252 -> 242; 64 experts, d 2048, four slots: 1152 250 -> 232, 1920
-// 273 -> 263, 2880 310 -> 304, but 4096 378 -> 407. Training steps, 8 experts: 64 tokens 293 -> 277, d 512 with 2560 319 -> 278.
-// With a folded LayerNorm, whose rows a launch of their own normalises, from the memset to the products: 2560 tokens 34 -> 22 us,
-// 6400 36 -> 29, 9600 39 -> 37, 12800 44 -> 43, 16384 45 -> 49.
+// other, which the general kernels do not: the more experts, the fewer tokens. Whole calls, a memset in front of both, general
+// kernels -> this one (medians of three): 8 experts, d 1024, f 4096: 2100 tokens 143 -> 128 us, 4000 191 -> 178, 12000 551 -> 540,
+// 18000 780 -> 776; d 512, f 2048: 4000 85.5 -> 70.0, 12000 173 -> 165, 18000 243 -> 235; 16 experts, d 1024, f 2048: 2200 108 ->
+// 88, 8000 225 -> 207, 15360 380 -> 367; 32 experts, d 2048, f 1408: 2200 156 -> 139, 5000 240 -> 230, 9400 362 -> 365; 64 experts,
+// four slots: 1100 244 -> 228, 2000 277 -> 267, 3500 324 -> 324, but 4096 378 -> 407. Training steps, 8 experts, d 512 with 2560
+// tokens 325 -> 285; of a few hundred tokens they are as long on the host. With a folded LayerNorm, whose rows a launch of their own
+// normalises: 2100 tokens 146 -> 133, 4000 201 -> 193, 9400 451 -> 448; in front of the products 12800 44 -> 43, 16384 45 -> 49.
 int front_many_tokens(int64_t N, int d, int E, int k, int dtype, bool norm, int* per) {
   *per = 0;
   if (norm && E > 16) return 0;

@@ -39,14 +39,16 @@ front_small_kernel(const T* __restrict__ x, const T* Wg, const T* bg, int Ntotal
 // times and not eight, its loads (both its chunks of the tokens and of the weights, its token's row for the copy) are in flight
 // together without spills, a token's softmax and top-k are a warp's and not a few lanes', and no step divides. Blocks meet
 // at a grid barrier (up to 128 of them, one an SM, launched cooperatively).
-// (front_small_body did it with 32 warps: 9.4 us from the wait to the end at 300 tokens, where this kernel takes 7.2. Whole
-// calls, d 1024, f 4096, 8 experts: 130 tokens 53.1 -> 51.6 us, 300 59.3 -> 57.9, 400 62.0 -> 60.9, 1173 88.0 -> 86.8.)
+// (front_small_body did it with 32 warps: 9.4 us from the wait to the end at 300 tokens, where this kernel takes 7.2. The
+// cooperative launch takes 2 us of that again: front_small_body's blocks met under an ordinary launch, as if the GPU were
+// theirs. Whole calls, d 1024, f 4096, 8 experts, that one -> this one: 130 tokens 52.3 -> 51.5 us, 300 58.3 -> 58.7, 400 61.3 ->
+// 61.6, 600 64.4 -> 65.2, 1173 89.5 -> 90.3.)
 constexpr int kMidWarps = 16, kMidTok = 16, kMidMaxE = 64;
 
 // Tokens of a block, a power of two: fewer of them shorten the row copies, which the block's warps then share, and more blocks
-// lengthen the meeting and read the router's weights more often. Best of 2, 4, 8 and 16 (64 experts, d 2048: 60 tokens 89.3,
-// 87.9, 88.4, 92.1 us a call; 100 192.5, 190.1, 189.5, 193.5; 300 202.6, 199.6, 196.7, 198.3; 1000 -, 202.9, 203.4, 199.9;
-// 8 experts, d 1024: 130 51.0, 50.7, 50.7, 51.6; 300 57.8, 57.7, 57.5, 58.2; 600 -, 64.9, 64.3, 64.1; 1173 -, -, 87.7, 87.2).
+// lengthen the meeting and read the router's weights more often. 2, 4, 8 and 16 of them, us a call: 64 experts, d 2048, f 1408,
+// four slots, 60 tokens 189, 189, 190, 194; 100 200, 198, 198, 200; 300 203, 207, 205, 206; 1000 228, 226, 231, 230; 8 experts,
+// d 1024, f 4096, 130 tokens 51.7, 51.3, 51.6, 53.0; 300 59.3, 59.4, 58.6, 59.7; 600 65.7, 65.5, 65.4, 65.5.
 // Up to 8 tokens stay one block's, which need not meet any other.
 int mid_tokens_per_block(int64_t N) {
   if (N <= 64) return N > 4 && N <= 8 ? 8 : 4;
@@ -54,9 +56,8 @@ int mid_tokens_per_block(int64_t N) {
 }
 
 // More than 32 experts, two a lane, logits that are not finite as in front_many.cu: calls of up to 2048 tokens and 4096 rows,
-// from one token on (d 2048, 64 experts of f 1408,
-// four slots, whole calls against the general router and dispatch: 1 token 60.4 -> 48.2 us, 8 111 -> 98.5, 100 206 -> 198,
-// 1000 213 -> 200).
+// from one token on (d 2048, 64 experts of f 1408, four slots, whole calls against the general router and dispatch: 1 token
+// 58.6 -> 37.3 us, 8 112 -> 90, 100 212 -> 199, 1000 245 -> 229).
 template <int NT>      // 8 NT >= E
 __global__ void __launch_bounds__(32 * kMidWarps, 1)
 front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfloat16* bg, int Ntotal, int d, int E, int k,
