@@ -71,6 +71,7 @@ SIGNATURES = {
     "moe_b200_attention": (_i, [_vp, _vp, _vp, _vp, _i64, _i, _i, _i, _i, _f, _vp, _vp]),
     "moe_b200_linear_rows": (_i, [_vp, _vp, _vp, _i, _vp, _vp, _i, _i64, _i, _vp, _vp, _vp, _vp]),
     "moe_b200_linear_rows_max": (_i64, []),
+    "moe_b200_attention_linears": (_i, [_i64, _i, _i, _i, _i]),
     "moe_b200_train_workspace_bytes": (_sz, [_i64, _i, _i, _i, _i, _i]),
     "moe_b200_train_workspace_layout": (_i, [_i64, _i, _i, _i, _i, _i, C.POINTER(_sz)]),
     "moe_b200_train_setup": (_i, [_i64, _i, _i, _i, _i, _i, _vp, _sz, _vp]),

@@ -1,8 +1,9 @@
 """Drop-in for the reference's ``Attention`` (model.py:59-152): same constructor, attribute
 and parameter names, ``state_dict`` layout and ``forward`` signature. The fused QKV Linear and the
-head gate are one launch (``moe_b200_linear_rows``), the output Linear another (torch's Linears where sizes or
-places are not those it takes — a number of heads that is no multiple of 8, from 129 rows on — and where their
-derivatives are asked for or their weights are of a class of their own); everything between
+head gate are one launch (``moe_b200_linear_rows``), the output Linear another (torch's Linears where those are the
+faster ones, ``moe_b200_attention_linears``, where sizes or places are not those it takes — a number of heads that is no
+multiple of 8, from 129 rows on — and where their derivatives are asked for or their weights are of a class of their own);
+everything between
 them — head split, shared KV heads, RoPE from the model's own table, scores, mask, softmax,
 the product with V and the sigmoid head gate — is one kernel of libmoe_b200
 (``moe_b200_attention``), so the [B, H, S, S] score tensor is never materialised.
@@ -153,7 +154,8 @@ class Attention(nn.Module):
         if any(type(p) not in (torch.Tensor, nn.Parameter, type(None)) for p in args[1:7]) or any(_derived(p) for p in args[:7]):
             return False
         rows, many = (self.q_head + 2 * self.kv_head) * self.head_dim, N > lib.moe_b200_linear_rows_max()
-        return (1 <= N <= 1 << 28 and hid % 8 == 0 and self.head_dim == 64 and self.q_head % self.kv_head == 0
+        return (1 <= N <= 1 << 28 and lib.moe_b200_attention_linears(N, hid, self.q_head, self.kv_head, self.head_dim) != 0
+                and hid % 8 == 0 and self.head_dim == 64 and self.q_head % self.kv_head == 0
                 and x.shape[1] <= 128 and x.data_ptr() % 16 == 0 and not (many and self.q_head % 8 != 0)
                 and all(w.shape == (r, c) and w.is_contiguous() and w.data_ptr() % 16 == 0 and b is not None and b.numel() == r
                         and b.is_contiguous() and not (many and b.data_ptr() % 16 != 0)

@@ -82,7 +82,8 @@ struct AttentionArgs {
   void *xn, *qkv, *gate, *core, *out;
   int32_t* status;
 };
-// Whether sizes and places are those that these launches take (and moe_b200_linear_rows): not all are the library's Linears'.
+// Whether sizes and places are those that these launches take (and moe_b200_linear_rows) and the sizes are those where they are
+// the faster ones (moe_b200_attention_linears).
 bool attention_supported(const AttentionArgs& p);
 bool attention_normalises_apart(const AttentionArgs& p);
 int attention_layer(const AttentionArgs& p, void* stream);

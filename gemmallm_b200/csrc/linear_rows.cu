@@ -244,10 +244,35 @@ bool attention_normalises_apart(const AttentionArgs& p) {
   return p.norm_weight != nullptr && (p.B * p.S > kLinearRowsMax || p.hidden > kNormMaxK);
 }
 
+namespace {
+// Rounds of a launch's blocks (two an SM; one where 32 rows of more than 1024 elements wait in shared memory for their
+// LayerNorm) times what a block does, 1 for 16 tokens and K 1024.
+double rows_cost(int rows, int rows2, int64_t N, int K, bool norm) {
+  const int64_t b = (rows + kRowsW - 1) / kRowsW + (rows2 + kRowsW - 1) / kRowsW;
+  const int tok = b * ((N + 15) / 16) <= 2 * kNumSMs ? 16 : 32;
+  const int at_once = norm && K > 1024 && K <= kNormMaxK && tok == 32 ? kNumSMs : 2 * kNumSMs;
+  return (double)(b * ((N + tok - 1) / tok)) / at_once * tok / 16. * K / 1024.;
+}
+}  // namespace
+
+// Whether the Linears of an attention are launches of this library or torch's. Up to kLinearRowsMax rows a block reads its
+// tokens, and its share of W, once for every 16 or 32 of the others': a small product is over before a library's would have
+// begun, a large one is not. 336 sizes (hidden 256 to 4096, 4 to 32 heads, 1 to 128 rows) were timed, LayerNorm to skip connection,
+// both ways: up to a cost of 3 none is slower than with torch's Linears (2056, 8 heads, 128 rows: 39.5 us both; 1024, 16 heads, one KV
+// head, 37 rows 32 -> 16, 128 rows 38 -> 31), beyond it most are (2048, 32 heads, eight KV heads: 17 rows 33 -> 38, 128 rows 44 ->
+// 107), the best left out is 1.2 times as fast. Tiles (323 sizes, 129 to 8192 rows): 0.97 to 1.18 times as fast from 4096 rows on; below,
+// 0.93 to 1.15 with K of 1024 to 1536 (1024, 16 heads, 512 rows 32 / 32, 2048 39 -> 37; 520, 8 heads, 129 rows 25 -> 28), but with longer K, where
+// few tiles leave the chip idle however K is split, 0.81 to 1.15 (2056, 8 heads, 129 rows 32 -> 40; 4096, 32 heads, 640 rows 62 -> 73).
+bool attention_own_linears(int64_t N, int hidden, int q_heads, int kv_heads, int head_dim) {
+  const int inner = q_heads * head_dim;
+  if (N > kLinearRowsMax) return N >= 4096 || (hidden <= 1536 && inner <= 1536);
+  return rows_cost(inner + 2 * kv_heads * head_dim, q_heads, N, hidden, true) <= 3. && rows_cost(hidden, 0, N, inner, false) <= 3.;
+}
+
 bool attention_supported(const AttentionArgs& p) {
   const int64_t N = p.B * p.S;
   if (N < 1 || N > (int64_t)1 << 28 || p.S > 128 || p.head_dim != 64 || p.kv_heads < 1 || p.q_heads % p.kv_heads != 0 ||
-      (p.hidden & 7) != 0 || p.hidden < 8)
+      (p.hidden & 7) != 0 || p.hidden < 8 || !attention_own_linears(N, p.hidden, p.q_heads, p.kv_heads, p.head_dim))
     return false;
   for (const void* q : {p.x, p.wqkv, p.wgate, p.wo, p.norm_weight, p.norm_bias, p.skip})
     if (!aligned16(q)) return false;
@@ -285,6 +310,13 @@ int attention_layer(const AttentionArgs& p, void* stream) {
 using namespace moe;
 
 extern "C" int64_t moe_b200_linear_rows_max(void) { return kLinearRowsMax; }
+
+extern "C" int moe_b200_attention_linears(int64_t N, int hidden, int q_heads, int kv_heads, int head_dim) {
+  if (N < 1 || N > (int64_t)1 << 28 || hidden < 8 || hidden > 1 << 24 || q_heads < 1 || kv_heads < 1 || head_dim < 1 ||
+      (int64_t)(q_heads + 2 * (int64_t)kv_heads) * head_dim > 1 << 24)
+    return 0;
+  return attention_own_linears(N, hidden, q_heads, kv_heads, head_dim) ? 1 : 0;
+}
 
 extern "C" int moe_b200_linear_rows(const void* x, const void* W, const void* b, int rows, const void* W2, const void* b2,
                                     int rows2, int64_t N, int K, void* out, void* out2, int32_t* status, void* stream) {

@@ -440,6 +440,9 @@ int moe_b200_attention(const void* qkv, const void* gate, const float* pos_emb, 
 int moe_b200_linear_rows(const void* x, const void* W, const void* b, int rows, const void* W2, const void* b2, int rows2,
                          int64_t N, int K, void* out, void* out2, int32_t* status, void* stream);
 int64_t moe_b200_linear_rows_max(void);
+/* Whether the modules run an attention's Linears by these kernels at N rows (1) or leave them to torch, whose are the faster
+ * there (0). */
+int moe_b200_attention_linears(int64_t N, int hidden, int q_heads, int kv_heads, int head_dim);
 
 /* ---- Training mode ---------------------------------------------------------------
  * The reference trains through this block (loss.backward(), train.py:140-141): under

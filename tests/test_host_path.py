@@ -907,6 +907,42 @@ def test_own_linears_of_the_attention_give_no_derivatives():
         assert not own()
 
 
+def test_sizes_of_the_own_linears():
+    """Products that are over before a library's have begun, and tiles that fill the chip; the native call and the module
+    give the same answer."""
+    own = lambda N, *a: lib.moe_b200_attention_linears(N, *a, 64)
+    assert [own(N, 1024, 16, 1) for N in (1, 37, 64, 128, 129, 512, 32768)] == [1] * 7
+    assert [own(N, 2048, 32, 8) for N in (1, 16, 17, 128, 129, 4095, 4096)] == [1, 1, 0, 0, 0, 0, 1]
+    assert [own(N, 1024, 16, 16) for N in (64, 65, 128, 129)] == [1, 0, 0, 1]
+    assert [own(N, 1536, 24, 6) for N in (32, 33, 129)] == [1, 0, 1] and own(129, 1544, 24, 6) == 0 and own(129, 1536, 25, 5) == 0
+    assert own(0, 1024, 16, 1) == 0 and own(1, 1024, 0, 1) == 0 and own(1, 1 << 30, 1, 1) == 0
+    m = Attention(2048, 64, 32, 8, Table(128, 64)).to(dtype=DT).eval().requires_grad_(False)
+    for N in (16, 17):
+        x = torch.zeros(1, N, 2048, dtype=DT)
+        assert m._own_linears(m._arguments(x, None, False), N, 2048, 2048) is (N == 16)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,S", [(1, 17), (1, 128), (3, 50)])
+def test_large_attentions_keep_torchs_linears(cuda_device, monkeypatch, B, S):
+    torch.manual_seed(S)
+    layer = LLMLayer(2048, 64, 32, 8, Table(128, 64), expansion_factor=1, use_moe=False, device="cuda")
+    layer = layer.to(device=cuda_device, dtype=DT).eval().requires_grad_(False)
+    m, x = layer.mqa, torch.randn(B, S, 2048, generator=torch.Generator().manual_seed(B)).to(device=cuda_device, dtype=DT)
+    m.embedding.float()
+    qkv, gate = [torch.nn.functional.linear(x, lin.weight, lin.bias) for lin in (m.qkv, m.gate)]
+    core = torch.empty(B, S, 2048, device=cuda_device, dtype=DT)
+    check(lib.moe_b200_attention(qkv.data_ptr(), gate.data_ptr(), m._pos_table(cuda_device).data_ptr(), None, B, S, 32, 8, 64,
+                                 float(m.scaler), core.data_ptr(), torch.cuda.current_stream().cuda_stream), "attention")
+    want = torch.nn.functional.linear(core, m.o.weight, m.o.bias)
+    assert torch.equal(m(x), want)
+    args = m._arguments(x, None, False)
+    assert _host.attention(*args, layer.norm1.weight, layer.norm1.bias, layer.norm1.eps) is None
+    assert torch.equal(layer._attend(x, None, False), m(_layernorm(layer.norm1, x)) + x)
+    monkeypatch.setattr(_host, "attention", lambda *a: None)
+    assert torch.equal(m(x), want)
+
+
 def test_status_of_a_layer():
     """Of its attention or of its block, each returned once; and of an attention that was saved before it had any."""
     layer = LLMLayer(D, 64, 2, 1, Table(16, 64), expansion_factor=1, use_moe=True, num_experts=E, device="cuda")
