@@ -42,6 +42,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
   __shared__ int s_cnt[kMaxTopK * ET], s_tot[kMaxTopK * ET], s_base[ET];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int b = (int)blockIdx.x, nb = (int)gridDim.x, ke = k * E;
+  const bool wide = ke > 2 * kWarps;      // many counts
   const int N = min(per, Ntotal - b * per);
   const int pieces = d >> 3, nchunk = (d + 31) >> 5;
   x += (size_t)b * per * d;
@@ -190,7 +191,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
   float* xps = reinterpret_cast<float*>(xch + nb * ke);    // [nb][E]
   for (int i = tid; i < ke; i += 32 * kWarps) {
     if (nb == 1) s_tot[i] = s_cnt[i];
-    else xch[EL > 1 ? b * ke + i : i * nb + b] = s_cnt[i];
+    else xch[wide ? b * ke + i : i * nb + b] = s_cnt[i];
   }
   if (tid >= 32 * kWarps - E) {
     const int e = tid - (32 * kWarps - E);
@@ -205,7 +206,7 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
   } else {
     cooperative_groups::this_grid().sync();
     // totals, and the rows that earlier blocks put in front of this block's (16 bits: fewer than 65536 tokens)
-    if (EL == 1) {      // a warp per count
+    if (!wide) {      // a warp per count
       for (int je = warp; je < ke; je += kWarps) {
         unsigned both = 0;
         for (int bb = lane; bb < nb; bb += 32) {
@@ -218,11 +219,11 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
           if (both >> 16) atomicAdd(&s_base[je % E], (int)(both >> 16));
         }
       }
-    } else {            // a thread per count, or several
+    } else {          // a thread per count, or several
       const int shares = 32 * kWarps / ke, q = tid / ke, je = tid - q * ke;
       if (q < shares) {
         unsigned both = 0;
-#pragma unroll 8
+#pragma unroll 16
         for (int bb = q; bb < nb; bb += shares) {
           const unsigned c = (unsigned)__ldcg(&xch[bb * ke + je]);
           both += c | (bb < b ? c << 16 : 0u);

@@ -73,7 +73,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   __shared__ float s_prob[kMidTok][ET];
   __shared__ int s_idx[kMidTok * kMaxTopK], s_row[kMidTok * kMaxTopK], s_tot[kMaxTopK * ET], s_base[ET];
   static_assert(kMidWarps * kMidTok >= 128, "the sums of 128 blocks");
-  static_assert(EL == 1 || kMaxTopK * ET == 32 * kMidWarps, "a thread per count");
+  static_assert(kMaxTopK * ET <= 32 * kMidWarps, "a thread per count");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int b = (int)blockIdx.x, nb = (int)gridDim.x;
   const int N = min(per, Ntotal - b * per);
@@ -83,7 +83,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   out_w += (size_t)b * per * k;
   row_of += (size_t)b * per * k;
   if (tid < ET) s_base[tid] = 0;
-  if (EL > 1) s_tot[tid] = 0;      // (32 kMidWarps of them)
+  if (tid < kMaxTopK * ET) s_tot[tid] = 0;
   pdl_wait();                 // x may come from the kernel before this one
   pdl_launch_dependents();
 
@@ -195,10 +195,11 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   }
   __syncthreads();
 
-  // ---- this block's counts per (slot, expert), a count's blocks side by side (a block's counts, with more than 32 experts),
-  // and its probability sums ----
+  // ---- this block's counts per (slot, expert), a count's blocks side by side (where there are many counts, a block's), and its
+  // probability sums ----
   float* s_sum = s_dyn;
   const int ke = k * E;
+  const bool wide = ke > 2 * kMidWarps;
   float* xps = reinterpret_cast<float*>(xch + nb * ke);    // [nb][E]
   for (int i = tid; i < ke; i += 32 * kMidWarps) {
     int c = 0;
@@ -206,7 +207,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
 #pragma unroll
     for (int tok = 0; tok < kMidTok; ++tok) c += s_idx[tok * k + j] == e ? 1 : 0;
     if (nb == 1) s_tot[i] = c;
-    else xch[EL > 1 ? b * ke + i : i * nb + b] = c;
+    else xch[wide ? b * ke + i : i * nb + b] = c;
   }
   if (tid >= 32 * kMidWarps - E) {
     const int e = tid - (32 * kMidWarps - E);
@@ -221,7 +222,7 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
   } else {
     cooperative_groups::this_grid().sync();
     // totals, and the rows that earlier blocks put in front of this block's (16 bits: 2048 tokens)
-    if (EL == 1) {      // a warp per count
+    if (!wide) {      // a warp per count
       for (int je = warp; je < ke; je += kMidWarps) {
         unsigned both = 0;
         for (int bb = lane; bb < nb; bb += 32) {
@@ -234,11 +235,11 @@ front_mid_kernel(const __nv_bfloat16* x, const __nv_bfloat16* Wg, const __nv_bfl
           if (both >> 16) atomicAdd(&s_base[je % E], (int)(both >> 16));
         }
       }
-    } else {            // a thread per count, or several (a warp per count: 16 rounds of loads one after the other)
+    } else {          // a thread per count, or several (a warp per count: 16 rounds of loads one after the other)
       const int per = 32 * kMidWarps / ke, q = tid / ke, je = tid - q * ke;
       if (q < per) {
         unsigned both = 0;
-#pragma unroll 8
+#pragma unroll 16
         for (int bb = q; bb < nb; bb += per) {
           const unsigned c = (unsigned)__ldcg(&xch[bb * ke + je]);
           both += c | (bb < b ? c << 16 : 0u);
