@@ -355,8 +355,40 @@ ffn_f32_kernel(const __grid_constant__ TokenMaps tmap_a, const CUtensorMap* __re
         const uint64_t kP = PLANES ? (uint64_t)((tl.n + 31) >> 5) * (32 * BK * 2 / 16) : (uint64_t)(kPlane / 16);
         // Two steps at a time, their large products first: those sums are read out while the small products run, and the
         // thread that issues has to look at barriers half as often (46 clk a product, 60 to 100 a barrier or commit).
+        // (of three stages, which the split of tokens here leaves, two would be taken: there a step at a time; d 512, f 2048, 8 experts,
+        // 2049 / 4000 / 8000 tokens 267 / 443 / 746 us in pairs, 253 / 420 / 712 so)
         static_assert(kLargeSteps == 2 && kSmallSteps % 2 == 0, "steps go in pairs");
-        for (int i = 0; i < kn; i += 2) {
+        auto small_products = [&](uint32_t a, uint64_t b, bool more) {
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {
+            const uint32_t ak = a + kk * 8;
+            const uint64_t bk = b + kk * 2;
+            mma_ts(tmem + kSmallCol, ak + 32, bk, idesc, more || kk != 0 ? 1u : 0u);   // a2 b0
+            mma_ts(tmem + kSmallCol, ak, bk + 2 * kP, idesc, 1u);                      // a0 b2
+            mma_ts(tmem + kSmallCol, ak + 16, bk + kP, idesc, 1u);                     // a1 b1
+            mma_ts(tmem + kSmallCol, ak + 16, bk, idesc, 1u);                          // a1 b0
+            mma_ts(tmem + kSmallCol, ak, bk + kP, idesc, 1u);                          // a0 b1
+          }
+        };
+        for (int i = 0; !PLANES && i < kn; ++i) {
+          if (!mbar_wait(&ctl->conv_full[c], phase, &ctl->abort, status, 53)) { ok = false; break; }
+          if (i % kLargeSteps == 0 && !mbar_wait(&ctl->main_empty, (larges++ & 1u) ^ 1u, &ctl->abort, status, 54)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t a = tmem + kACol + c * kACols;
+          const uint64_t b = desc64(smem_u32(planes) + (uint32_t)(c * 3 * kPlane));
+          mma_ts(tmem + kMainCol, a, b, idesc, i % kLargeSteps != 0 ? 1u : 0u);
+          mma_ts(tmem + kMainCol, a + 8, b + 2, idesc, 1u);
+          if ((i + 1) % kLargeSteps == 0 || i + 1 == kn) tc_commit(&ctl->main_full);
+          if (i % kSmallSteps == 0) {
+            if (!mbar_wait(&ctl->small_empty, (smalls++ & 1u) ^ 1u, &ctl->abort, status, 52)) { ok = false; break; }
+            tc_fence_after();
+          }
+          small_products(a, b, i % kSmallSteps != 0);
+          if ((i + 1) % kSmallSteps == 0 || i + 1 == kn) tc_commit(&ctl->small_full);
+          tc_commit(&ctl->conv_empty[c]);
+          if (++c == kStages) { c = 0; phase ^= 1u; }
+        }
+        for (int i = 0; PLANES && i < kn; i += 2) {
           const bool two = i + 1 < kn;
           const int c1 = c + 1 == kStages ? 0 : c + 1;
           const uint32_t phase1 = c + 1 == kStages ? phase ^ 1u : phase;
@@ -379,18 +411,6 @@ ffn_f32_kernel(const __grid_constant__ TokenMaps tmap_a, const CUtensorMap* __re
             if (!mbar_wait(&ctl->small_empty, (smalls++ & 1u) ^ 1u, &ctl->abort, status, 52)) { ok = false; break; }
             tc_fence_after();
           }
-          auto small_products = [&](uint32_t a, uint64_t b, bool more) {
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {
-              const uint32_t ak = a + kk * 8;
-              const uint64_t bk = b + kk * 2;
-              mma_ts(tmem + kSmallCol, ak + 32, bk, idesc, more || kk != 0 ? 1u : 0u);   // a2 b0
-              mma_ts(tmem + kSmallCol, ak, bk + 2 * kP, idesc, 1u);                      // a0 b2
-              mma_ts(tmem + kSmallCol, ak + 16, bk + kP, idesc, 1u);                     // a1 b1
-              mma_ts(tmem + kSmallCol, ak + 16, bk, idesc, 1u);                          // a1 b0
-              mma_ts(tmem + kSmallCol, ak, bk + kP, idesc, 1u);                          // a0 b1
-            }
-          };
           small_products(a0, b0, i % kSmallSteps != 0);
           tc_commit(&ctl->conv_empty[c]);
           if (two) {
