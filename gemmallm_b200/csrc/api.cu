@@ -517,8 +517,10 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
   const bool clean = (small_n || rows_path) && (flags & MOE_B200_FLAG_WS_CLEAN);
   // status words, and the completion counters behind them where a kernel uses them, in one memset
   // (above these sizes a call always clears both: the status words are those of the most recent call, and what a call that
-  // timed out left in the counters does not reach the next one; the fp32 front clears the status words itself)
-  if (!front32 && !clean)
+  // timed out left in the counters does not reach the next one; the front of a few thousand tokens clears them itself, that of
+  // fp32 calls, which have no counters, the status words)
+  const bool clears = many > 0 && !small_n && !rows_path;
+  if (!front32 && !clean && !clears)
     MOE_CUDA_CHECK(cudaMemsetAsync(
         status, 0, (counters ? MOE_B200_READY_OFFSET + MOE_B200_READY_INTS : MOE_B200_STATUS_INTS) * sizeof(int32_t), s));
   float* stats = reinterpret_cast<float*>(ws + off[MOE_B200_WS_STATS]);
@@ -564,7 +566,7 @@ int forward_into(const void* x, const void* Wg, const void* bg, const void* plan
       if (fold) rc = launch_layernorm_rows(x, norm_weight, norm_bias, norm_eps, N, d, dtype, y, stats, s);
       if (rc) return rc;
       rc = launch_front_many(x, y, stats, fold ? nc : nullptr, fold ? wn : Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets,
-                             row_of, perm, nullptr, psum, aux, scratch, status, many, s);
+                             row_of, perm, nullptr, psum, aux, scratch, status, many, clears, s);
       if (rc) return rc;
     } else if (fold) {
       rc = moe_b200_router_norm(x, wn, nc, norm_eps, N, d, E, k, dtype, logits, idx, w, psum_part,

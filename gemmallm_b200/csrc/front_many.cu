@@ -28,7 +28,8 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
                   float* __restrict__ out_logits, int32_t* __restrict__ out_idx, float* __restrict__ out_w,
                   int32_t* __restrict__ cnt_slot, int32_t* __restrict__ offsets, int32_t* __restrict__ row_of,
                   __nv_bfloat16* __restrict__ perm, int32_t* __restrict__ pair_of, float* __restrict__ psum,
-                  float* __restrict__ aux, int* __restrict__ xch, int32_t* __restrict__ status, int per, int share) {
+                  float* __restrict__ aux, int* __restrict__ xch, int32_t* __restrict__ status, int per, int share,
+                  bool clear) {
   constexpr int ET = 8 * NT, EL = ET > 32 ? 2 : 1, GL = ET / EL, P = 32 / GL;      // experts a lane, lanes of a token
   constexpr bool STRICT = NT <= 2;
   static_assert(!NORM || STRICT, "with a folded LayerNorm the general router is the strict one at any number of experts");
@@ -55,6 +56,9 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
   if (tid < ET) s_base[tid] = 0;
   pdl_wait();                 // x may come from the kernel before this one
   pdl_launch_dependents();
+  // (in front of the exchange: nothing is reported or counted before it)
+  if (clear && b == 0)
+    for (int i = tid; i < MOE_B200_READY_OFFSET + MOE_B200_READY_INTS; i += 32 * kWarps) status[i] = 0;
   __syncthreads();
 
   // ---- routing, 16 tokens at a time: a warp's chunks of 32 of K for all of them, then a token for every warp ----
@@ -341,7 +345,8 @@ front_many_kernel(const __nv_bfloat16* x, const __nv_bfloat16* xn, const float* 
 template <int NT, bool NORM>
 int launch(const void* x, const void* xn, const float* stats, const float* norm_c, const void* Wg, const void* bg, int N, int d,
            int E, int k, float* logits, int32_t* idx, float* w, int32_t* cnt_slot, int32_t* offsets, int32_t* row_of, void* perm,
-           int32_t* pair_of, float* psum, float* aux, int32_t* xch, int32_t* status, int per, cudaStream_t s) {
+           int32_t* pair_of, float* psum, float* aux, int32_t* xch, int32_t* status, int per, bool clear,
+           cudaStream_t s) {
   constexpr size_t part = sizeof(float) * 2 * kWarps * kGroup * 8 * NT;
   static PerDeviceOnce once;
   int rc = ensure_dynamic_smem(once, front_many_kernel<NT, NORM>, part + 2 * sizeof(int) * kMaxPer * kMaxTopK);
@@ -352,7 +357,7 @@ int launch(const void* x, const void* xn, const float* stats, const float* norm_
                                static_cast<const __nv_bfloat16*>(xn), stats, norm_c,
                                static_cast<const __nv_bfloat16*>(Wg), static_cast<const __nv_bfloat16*>(bg), N, d, E, k, logits,
                                idx, w, cnt_slot, offsets, row_of, static_cast<__nv_bfloat16*>(perm), pair_of, psum, aux, xch,
-                               status, per, per < kWarps ? kWarps / per : 1));
+                               status, per, per < kWarps ? kWarps / per : 1, clear));
   return 0;
 }
 
@@ -360,8 +365,8 @@ int launch(const void* x, const void* xn, const float* stats, const float* norm_
 
 // Tokens of a block for a call that this kernel takes, 0 for any other: as many as give every SM one block, a few (a power of
 // two) where that shortens the copies. A block reads the router's weights once per 16 tokens and has its groups one after the
-// other, which the general kernels do not: the more experts, the fewer tokens. Whole calls, a memset in front of both, general
-// kernels -> this one (medians of three): 8 experts, d 1024, f 4096: 2100 tokens 143 -> 128 us, 4000 191 -> 178, 12000 551 -> 540,
+// other, which the general kernels do not: the more experts, the fewer tokens. Whole calls, general kernels -> this
+// one (medians of three, a memset in front of both, which this one has no more): 8 experts, d 1024, f 4096: 2100 tokens 143 -> 128 us, 4000 191 -> 178, 12000 551 -> 540,
 // 18000 780 -> 776; d 512, f 2048: 4000 85.5 -> 70.0, 12000 173 -> 165, 18000 243 -> 235; 16 experts, d 1024, f 2048: 2200 108 ->
 // 88, 8000 225 -> 207, 15360 380 -> 367; 32 experts, d 2048, f 1408: 2200 156 -> 139, 5000 240 -> 230, 9400 362 -> 365; 64 experts,
 // four slots: 1100 244 -> 228, 2000 277 -> 267, 3500 324 -> 324, but 4096 378 -> 407. Training steps, 8 experts, d 512 with 2560
@@ -383,15 +388,17 @@ int front_many_tokens(int64_t N, int d, int E, int k, int dtype, bool norm, int*
 }
 
 // norm_c, or nullptr: a folded LayerNorm, with `stats` and the normalised rows `xn` of layernorm_rows.
-// xch: int32 scratch, (k + 1) * E words for each of kNumSMs blocks.
+// xch: int32 scratch, (k + 1) * E words for each of kNumSMs blocks. clear: the status words and the counters behind them, none of
+// which this kernel uses itself, are zeroed here first, whatever they held (a memset in front of the launch takes 2.0 to 2.6 us:
+// 3000 tokens, d 256, f 64, 8 experts 32.3 us with it and 29.8 without).
 int launch_front_many(const void* x, const void* xn, const float* stats, const float* norm_c, const void* Wg, const void* bg,
                       int64_t N, int d, int E, int k, float* logits, int32_t* idx, float* w, int32_t* cnt_slot,
                       int32_t* offsets, int32_t* row_of, void* perm, int32_t* pair_of, float* psum, float* aux, int32_t* xch,
-                      int32_t* status, int per, cudaStream_t s) {
+                      int32_t* status, int per, bool clear, cudaStream_t s) {
   auto fn = norm_c != nullptr ? (E <= 8 ? launch<1, true> : launch<2, true>)
             : E <= 8 ? launch<1, false> : E <= 16 ? launch<2, false> : E <= 32 ? launch<4, false> : launch<8, false>;
   return fn(x, norm_c != nullptr ? xn : x, stats, norm_c, Wg, bg, (int)N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of,
-            perm, pair_of, psum, aux, xch, status, per, s);
+            perm, pair_of, psum, aux, xch, status, per, clear, s);
 }
 
 }  // namespace moe

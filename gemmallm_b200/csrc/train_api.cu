@@ -276,12 +276,12 @@ int forward_train_into(const void* x, const void* Wg, const void* bg, const void
     rc = front_many_tokens(N, d, E, k, dtype, false, &many);
     if (rc) return rc;
   }
-  MOE_CUDA_CHECK(cudaMemsetAsync(status, 0, (MOE_B200_READY_OFFSET + MOE_B200_READY_INTS) * sizeof(int32_t), s));
   if (many > 0) {
     rc = launch_front_many(x, nullptr, nullptr, nullptr, Wg, bg, N, d, E, k, logits, idx, w, cnt_slot, offsets, row_of, perm,
-                           pair_of, psum, aux, scratch, status, many, s);
+                           pair_of, psum, aux, scratch, status, many, true, s);
     if (rc) return rc;
   } else {
+    MOE_CUDA_CHECK(cudaMemsetAsync(status, 0, (MOE_B200_READY_OFFSET + MOE_B200_READY_INTS) * sizeof(int32_t), s));
     rc = moe_b200_router(x, Wg, bg, N, d, E, k, dtype, logits, idx, w, psum_part, status, stream);
     if (rc) return rc;
     rc = moe_b200_dispatch(x, idx, N, d, E, k, dtype, scratch, cnt_slot, offsets, row_of, perm, psum_part, psum, aux, status,
