@@ -12,7 +12,8 @@
 // the launch says that nothing in flight writes them. A decoder layer of 37 tokens (d 1024, 16 heads, 8 experts) took 93.4 us
 // with six launches around the attention (LayerNorm, three library products, the core, the addition) and takes 69.5 with
 // three; one token 84 -> 39.6, 102 tokens 92.6 -> 79.6, 128 tokens 93.9 -> 80.7. Beyond 128 rows the Linears are tiles of
-// experts_tc2.cu (kLinear), and large ones torch's (attention_own_linears below): 64 tokens 81.8 so and 72.3 here, 128 86.9 and 80.7, 140 89.9 and 91.3, 160 91.8 and 94.8.
+// experts_tc2.cu (kLinear): 64 tokens 81.8 so and 72.3 here, 128 86.9 and 80.7, 140 89.9 and 91.3, 160 91.8 and 94.8. Large
+// ones are torch's (attention_own_linears below).
 #include "common.cuh"
 #include "internal.h"
 

@@ -955,6 +955,12 @@ def test_attention_core(cuda_device, B, S, H, KV, masked, shift):
     assert (out.float().cpu() - want).norm() <= 2 ** -6 * want.norm()
 
 
+# 81 to 96 tokens: two blocks an SM without a mask, one with it; shares that end within a sequence
+@pytest.mark.parametrize("B,S,H,KV,masked", [(131, 96, 6, 3, False), (61, 81, 6, 3, True), (300, 90, 2, 2, False)])
+def test_attention_core_by_blocks_of_an_sm(cuda_device, B, S, H, KV, masked):
+    test_attention_core(cuda_device, B, S, H, KV, masked, 0)
+
+
 # up to 32 router blocks of 64 tokens a warp sums an expert's partial probabilities, beyond them a block
 @pytest.mark.parametrize("N,E", [(1, 64), (64, 200), (2048, 17), (2049, 17), (2049, 64)])
 def test_dispatch_probability_sums(cuda_device, N, E):
